@@ -67,6 +67,90 @@ __device__ __forceinline__ void gelu_fwd_bwd(float x, const GeluCoef& c, float& 
   dy = fmaf(hx * fmaf(-t, t, 1.0f), dq, fmaf(0.5f, t, 0.5f));
 }
 
+#ifdef __CUDACC__
+// The same functions on two values at once (sm_100 packed fp32 arithmetic: one instruction, two roundings identical to the
+// scalar ones).  The packed derivative carries the opposite sign through t^2 - 1 and -dq, which changes no rounding.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 f2_pack(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void f2_unpack(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 f2_fma(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 f2_mul(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 f2_add(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// eight fp32 values rounded to one 16-byte vector of bf16
+__device__ __forceinline__ uint4 f2_bf16x8(const f32x2 (&f)[4]) {
+  uint4 r;
+  uint32_t* w = reinterpret_cast<uint32_t*>(&r);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    float a, b;
+    f2_unpack(f[j], a, b);
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w[j]) : "f"(b), "f"(a));
+  }
+  return r;
+}
+// eight bf16 of one 16-byte vector as four pairs of fp32
+__device__ __forceinline__ void f2_unpack8(const uint4& v, f32x2 (&f)[4]) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) f[j] = f2_pack(__uint_as_float(w[j] << 16), __uint_as_float(w[j] & 0xffff0000u));
+}
+__device__ __forceinline__ f32x2 f2_clamp36(f32x2 u) {
+  float a, b;
+  f2_unpack(u, a, b);
+  return f2_pack(fminf(a, 36.f), fminf(b, 36.f));
+}
+__device__ __forceinline__ f32x2 f2_tanh(f32x2 u) {
+  float a, b;
+  f2_unpack(u, a, b);
+  return f2_pack(gelu_tanh_approx(a), gelu_tanh_approx(b));
+}
+__device__ __forceinline__ f32x2 gelu_fwd2(f32x2 x, const GeluCoef& c) {
+  const f32x2 u = f2_clamp36(f2_mul(x, x));
+  const f32x2 q = f2_fma(u, f2_fma(u, f2_pack(c.c2, c.c2), f2_pack(c.c1, c.c1)), f2_pack(c.c0, c.c0));
+  const f32x2 hx = f2_mul(x, f2_pack(0.5f, 0.5f));
+  return f2_fma(hx, f2_tanh(f2_mul(x, q)), hx);
+}
+__device__ __forceinline__ f32x2 gelu_bwd2(f32x2 x, const GeluCoef& c) {
+  const f32x2 u = f2_clamp36(f2_mul(x, x));
+  const f32x2 q = f2_fma(u, f2_fma(u, f2_pack(c.c2, c.c2), f2_pack(c.c1, c.c1)), f2_pack(c.c0, c.c0));
+  const float n2 = -5.f * c.c2, n1 = -3.f * c.c1, n0 = -c.c0;
+  const f32x2 ndq = f2_fma(u, f2_fma(u, f2_pack(n2, n2), f2_pack(n1, n1)), f2_pack(n0, n0));
+  const f32x2 t = f2_tanh(f2_mul(x, q));
+  const f32x2 half = f2_pack(0.5f, 0.5f);
+  const f32x2 s = f2_fma(t, t, f2_pack(-1.f, -1.f));
+  return f2_fma(f2_mul(f2_mul(x, half), s), ndq, f2_fma(t, half, half));
+}
+__device__ __forceinline__ void gelu_fwd_bwd2(f32x2 x, const GeluCoef& c, f32x2& y, f32x2& dy) {
+  const f32x2 u = f2_clamp36(f2_mul(x, x));
+  const f32x2 q = f2_fma(u, f2_fma(u, f2_pack(c.c2, c.c2), f2_pack(c.c1, c.c1)), f2_pack(c.c0, c.c0));
+  const float n2 = -5.f * c.c2, n1 = -3.f * c.c1, n0 = -c.c0;
+  const f32x2 ndq = f2_fma(u, f2_fma(u, f2_pack(n2, n2), f2_pack(n1, n1)), f2_pack(n0, n0));
+  const f32x2 t = f2_tanh(f2_mul(x, q));
+  const f32x2 half = f2_pack(0.5f, 0.5f);
+  const f32x2 hx = f2_mul(x, half);
+  const f32x2 s = f2_fma(t, t, f2_pack(-1.f, -1.f));
+  y = f2_fma(hx, t, hx);
+  dy = f2_fma(f2_mul(hx, s), ndq, f2_fma(t, half, half));
+}
+
+#endif  // __CUDACC__
+
 // Activation codes of the GEMM epilogue.  Odd codes act on the value itself (then an optional residual is added); even
 // codes multiply the value by the derivative of the matching activation, evaluated at the epilogue operand:
 //   1 GELU(x)               2 x * GELU'(aux)          aux = saved pre-activation

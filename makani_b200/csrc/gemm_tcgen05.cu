@@ -1,13 +1,13 @@
 // Persistent warp-specialised GEMM for sm_100a: TMA -> shared memory (128B swizzle) -> tcgen05.mma with
 // accumulators in tensor memory -> tcgen05.ld epilogue with fused bias / GELU / residual / scatter.
 //
-// Roles per CTA (320 threads, one CTA per SM):
-//   warp 0      : TMA producer (one elected lane)
-//   warp 1      : TMEM allocator + MMA issuer (one elected lane)
-//   warps 2..9  : epilogue; warp w reads TMEM lanes [32*(w%4), 32*(w%4)+32), the two warps that share a lane
-//                 quarter take alternating column chunks
-//   warp 10     : only in launches whose epilogue operand (residual, saved pre-activation) is prefetched by TMA
-//                 (352 threads): its producer, so that waiting for a free operand buffer never delays A and B
+// Roles per CTA (one CTA per SM; EW epilogue warps: one per 64-column box and lane quarter of the tile, see epi_warps):
+//   warp 0         : TMA producer (one elected lane)
+//   warp 1         : TMEM allocator + MMA issuer (one elected lane)
+//   warps 2..EW+1  : epilogue; warp w reads TMEM lanes [32*(w%4), 32*(w%4)+32) and the 64-column box (w-2)/4 (generic
+//                    epilogue: alternating 32-column chunks)
+//   warp EW+2      : only in launches whose epilogue operand (residual, saved pre-activation) is prefetched by TMA: its
+//                    producer, so that waiting for a free operand buffer never delays A and B
 // Two accumulator buffers in TMEM let the epilogue of tile i overlap the main loop of tile i+1.
 // Every mbarrier wait is bounded; on expiry the kernel records a code in *err and drains.
 //
@@ -41,8 +41,16 @@ namespace {
 
 constexpr int BM = 128;
 constexpr int A_STAGE_BYTES = BM * 128;
-constexpr int NUM_THREADS = 320;   // TMA warp + MMA warp + 8 epilogue warps
-constexpr int E_WARP = 10;         // launches with a TMA-fed epilogue operand run an eleventh warp: its producer
+// Epilogue warps of an instance.  The specialised epilogues give every 64-column box of every lane quarter a warp of its
+// own: 8 / 12 / 16 warps for 128- / 192- / 256-column tiles.  With eight warps for any width a warp of a wide tile worked
+// through its boxes one after the other, two warps per scheduler, at 50 % issue utilisation; the generic epilogue (fp32
+// outputs, atomics) needs its registers and stays at eight.
+__host__ __device__ constexpr int epi_warps(int bn, int epi) { return epi == 0 ? 8 : bn / 16; }
+// Register bound, given as a thread count: the warps of one scheduler's register bank (5, 4 or 3 of them) leave room for one
+// 64-register warp of the gradient all-reduce, which overlaps with these GEMMs in data-parallel training.
+__host__ __device__ constexpr int bound_threads(int bn, int epi) {
+  return epi == 0 || bn == 128 ? 352 : (bn == 192 ? 576 : 736);
+}
 constexpr int MAX_STAGES = 6;
 constexpr int MAX_SEG = 8;
 
@@ -70,6 +78,13 @@ struct DMaps {
 };
 constexpr uint64_t WAIT_LIMIT_NS = 2000000000ull;   // 2 s per barrier wait
 
+// Division of a 31-bit index by an invariant: q = (umulhi(n, mul) + n) >> shift (Granlund and Montgomery 1994).  Every
+// warp of a CTA decodes every tile; with 64-bit divisions that was a third of an epilogue warp's instructions.
+struct FastDiv {
+  uint32_t d, mul, shift;
+};
+__device__ __forceinline__ uint32_t fast_div(uint32_t n, const FastDiv& f) { return (__umulhi(n, f.mul) + n) >> f.shift; }
+
 struct KParams {
   int M, N, K;
   int zlo_n, zhi_n;
@@ -91,7 +106,8 @@ struct KParams {
   void* D;
   int out_f32, accumulate, vec_ok;
   int m_tiles, n_tiles;
-  long long total_tiles;
+  FastDiv dv_n, dv_m, dv_split, dv_zlo;
+  uint32_t total_tiles;           // below 2^31
   int stages, e_tma, plain_cols;
   int n_fast;                     // tile order: 1 = n-tile index fastest, 0 = m-tile index fastest
   int* err;
@@ -291,26 +307,27 @@ struct TileCoord {
 // CG = 2: `t` counts 256-row pair tiles (p.m_tiles is then the number of pair tiles) and `half` (0 / 1) selects this
 // CTA's 128 rows; skip decisions are taken for the pair as a whole because the MMA is issued once for both CTAs.
 template <int BK, int CG = 1>
-__device__ __forceinline__ TileCoord decode_tile(const KParams& p, long long t, int half = 0) {
+__device__ __forceinline__ TileCoord decode_tile(const KParams& p, uint32_t t, int half = 0) {
   TileCoord c;
   // The index that varies fastest walks over the tiles that share the larger operand, so that the CTAs of one wave
   // fetch that operand's tile from DRAM once and hit L2 for the rest (token-major convolutions: many m-tiles of
   // activations against two to six n-tiles of weights -> n fastest).
+  auto take = [&](const FastDiv& f) {
+    const uint32_t qt = fast_div(t, f);
+    const int rem = static_cast<int>(t - qt * f.d);
+    t = qt;
+    return rem;
+  };
   if (p.n_fast) {
-    c.nt = static_cast<int>(t % p.n_tiles);
-    t /= p.n_tiles;
-    c.mt = static_cast<int>(t % p.m_tiles);
-    t /= p.m_tiles;
+    c.nt = take(p.dv_n);
+    c.mt = take(p.dv_m);
   } else {
-    c.mt = static_cast<int>(t % p.m_tiles);
-    t /= p.m_tiles;
-    c.nt = static_cast<int>(t % p.n_tiles);
-    t /= p.n_tiles;
+    c.mt = take(p.dv_m);
+    c.nt = take(p.dv_n);
   }
-  c.split = static_cast<int>(t % p.splits);
-  t /= p.splits;
-  c.zlo = static_cast<int>(t % p.zlo_n);
-  c.zhi = static_cast<int>(t / p.zlo_n);
+  c.split = take(p.dv_split);
+  c.zlo = take(p.dv_zlo);
+  c.zhi = static_cast<int>(t);
   const int rmin = p.rmin_a * c.zhi + p.rmin_b;
   const int rmax = p.rmax_a * c.zhi + p.rmax_b;
   int kmin = p.kmin_a * c.zhi + p.kmin_b;
@@ -331,15 +348,18 @@ __device__ __forceinline__ TileCoord decode_tile(const KParams& p, long long t, 
   return c;
 }
 
-// Specialised epilogues stage their output for TMA stores in 32-row x 128-byte boxes, two per epilogue warp.  The
-// epilogues with a TMA-fed operand (3, 4) run 128-column tiles, where a warp writes one box per tile: its previous
-// store left the box a whole tile ago, so one box is enough and the other 32 KB go to a further operand stage.
-__host__ __device__ constexpr int stg_warp_bytes(int epi) { return (epi == 3 || epi == 4) ? 32 * 128 : 2 * 32 * 128; }
-__host__ __device__ constexpr int stg_bytes(int epi) { return epi == 0 ? 0 : 8 * stg_warp_bytes(epi); }
+// Specialised epilogues leave through TMA stores of 32-row x 128-byte boxes, one per epilogue warp and output.  Without an
+// epilogue operand (1, 2) the boxes are staged in a buffer of their own; with one (3, 4) the warp overwrites the operand's
+// box in place, element by element, and the store reads from there: no staging, so 192-column tiles fit.
+__host__ __device__ constexpr int stg_warp_bytes(int epi) { return epi == 2 ? 2 * 32 * 128 : (epi == 1 ? 32 * 128 : 0); }
+__host__ __device__ constexpr int stg_bytes(int bn, int epi) { return epi_warps(bn, epi) * stg_warp_bytes(epi); }
 
 // EPI selects a compile-time specialised epilogue (bf16 output, 16-byte vector stores, row bias only):
 //   0 generic (all options decided at run time)      1 plain store
 //   2 GELU + saved pre-activation                     3 + residual (TMA-prefetched)      4 * GELU'(aux) (TMA-prefetched)
+// rows of B per stage: whole MN-major boxes of 64 (a pair's half of a 192-wide tile is one and a half of them)
+__host__ __device__ constexpr int b_stage_rows(int bn, int cg) { return (bn / cg + 63) / 64 * 64; }
+
 // local k range [lb, le) of segment `sg` for tile `c` (multi-device B operand)
 template <int BK>
 __device__ __forceinline__ void seg_range(const KParams& p, const TileCoord& c, int sg, int& lb, int& le) {
@@ -356,19 +376,21 @@ __device__ __forceinline__ unsigned int ld_acquire_sys_u32(const unsigned int* p
 }
 
 template <int BN, int EB, int EPI, int CG>
-__global__ void __launch_bounds__(NUM_THREADS + 32, 1)
+__global__ void __launch_bounds__(bound_threads(BN, EPI), 1)
 gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ BMaps maps_b,
             const __grid_constant__ CUtensorMap map_e, const __grid_constant__ CUtensorMap map_d,
             const __grid_constant__ CUtensorMap map_p, const __grid_constant__ DMaps maps_dx, const KParams p) {
   const CUtensorMap& map_b = maps_b.m[0];
   constexpr int BK = 128 / EB;            // elements per 128-byte k-slab
   constexpr int UMMA_K = 32 / EB;         // elements per tcgen05.mma
-  constexpr int BNL = BN / CG;            // rows of the B tile this CTA loads (a pair splits the tile)
-  constexpr int B_STAGE_BYTES = BNL * 128;
+  constexpr int BNL = BN / CG;            // rows of the B tile this CTA contributes (a pair splits the tile)
+  constexpr int B_STAGE_BYTES = b_stage_rows(BN, CG) * 128;
+  constexpr int EW = epi_warps(BN, EPI);
+  constexpr int E_WARP = 2 + EW;
   constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
   constexpr int MN_BOX = 128 / EB;        // extent of an MN-major box along the contiguous dimension
-  constexpr uint32_t TMEM_COLS = 2 * BN;
-  constexpr int E_BYTES = BM * BN * 2;    // bf16 epilogue-operand tile
+  constexpr uint32_t TMEM_COLS = BN == 128 ? 256 : 512;   // two accumulators, rounded up to a power of two
+  constexpr uint32_t E_BYTES = BM * BN * 2;    // bf16 epilogue-operand tile
   const int STAGES = p.stages;
 
   extern __shared__ uint8_t smem_raw[];
@@ -380,7 +402,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
   // layout: [stages][E tile x2 (optional)][staging][barriers]
   const uint32_t e_off = STAGES * STAGE_BYTES;
   const uint32_t stg_off = e_off + (p.e_tma ? 2 * E_BYTES : 0);
-  const uint32_t bar_off = stg_off + stg_bytes(EPI);
+  const uint32_t bar_off = stg_off + stg_bytes(BN, EPI);
   uint8_t* bar_ptr = smem + bar_off;
   const uint32_t bar_base = smem_base + bar_off;
   auto full_bar = [&](int s) { return bar_base + 8u * s; };
@@ -395,8 +417,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
   const int lane = threadIdx.x & 31;
   // pair geometry: `crank` = rank inside the cluster (the leader is rank 0), tiles are dealt out per cluster
   const int crank = (CG == 2) ? static_cast<int>(cluster_ctarank()) : 0;
-  const long long tile0 = (CG == 2) ? (blockIdx.x >> 1) : blockIdx.x;
-  const long long tile_step = (CG == 2) ? (gridDim.x >> 1) : gridDim.x;
+  const uint32_t tile0 = (CG == 2) ? (blockIdx.x >> 1) : blockIdx.x;
+  const uint32_t tile_step = (CG == 2) ? (gridDim.x >> 1) : gridDim.x;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -405,9 +427,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(tfull_bar(b), 1);
-      mbar_init(tempty_bar(b), 8 * CG);
+      mbar_init(tempty_bar(b), EW * CG);
       mbar_init(efull_bar(b), 1);
-      mbar_init(eempty_bar(b), 8);
+      mbar_init(eempty_bar(b), EW);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -466,7 +488,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
       if (p.sync.nwait > 0) asm volatile("fence.proxy.async;" ::: "memory");   // flags acquired in the prologue order the TMA loads below
       // pair: every load of both CTAs is counted on the leader's "full" barrier
       const uint32_t leader_full0 = (CG == 2) ? mapa_u32(full_bar(0), 0) : 0u;
-      for (long long t = tile0; t < p.total_tiles && ok; t += tile_step) {
+      const uint32_t load_bytes = A_STAGE_BYTES + (p.b_mn ? B_STAGE_BYTES : BNL * 128);
+      for (uint32_t t = tile0; t < p.total_tiles && ok; t += tile_step) {
         const TileCoord c = decode_tile<BK, CG>(p, t, crank);
         const int m0 = c.mt * BM, n0 = c.nt * BN;
         if (c.skip) continue;
@@ -492,7 +515,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
             if constexpr (CG == 2) {
               // the leader announces the bytes of both CTAs; the partner's loads may land first (the barrier's byte
               // count goes negative for a moment, its phase cannot complete before the leader's arrival)
-              if (crank == 0) mbar_expect_tx(full_bar(s), 2 * STAGE_BYTES);
+              if (crank == 0) mbar_expect_tx(full_bar(s), 2 * load_bytes);
               const uint32_t lbar = leader_full0 + 8u * s;
               const int nb0 = n0 + crank * BNL;
               if (!p.a_mn) {
@@ -506,11 +529,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
                 tma_load_4d_pair(sb, mb, lbar, k, nb0, bzl, bzh);
               } else {
 #pragma unroll
-                for (int j = 0; j < BNL / MN_BOX; ++j)
+                for (int j = 0; j < B_STAGE_BYTES / (BK * 128); ++j)
                   tma_load_4d_pair(sb + j * (BK * 128), mb, lbar, nb0 + j * MN_BOX, k, bzl, bzh);
               }
             } else {
-              mbar_expect_tx(full_bar(s), STAGE_BYTES);
+              mbar_expect_tx(full_bar(s), load_bytes);
               if (!p.a_mn) {
                 tma_load_4d(sa, &map_a, full_bar(s), ka, m0, azl, azh);
               } else {
@@ -543,7 +566,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
     if (lane == 0 && p.e_tma && peers_ready) {
       if (p.sync.nwait > 0) asm volatile("fence.proxy.async;" ::: "memory");
       uint32_t epi_it = 0;
-      for (long long t = tile0; t < p.total_tiles; t += tile_step) {
+      for (uint32_t t = tile0; t < p.total_tiles; t += tile_step) {
         const TileCoord c = decode_tile<BK, CG>(p, t, crank);
         if (c.skip && p.accumulate) continue;
         const int eb = epi_it & 1;
@@ -574,7 +597,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
       int s = 0;
       uint32_t ph = 0, acc_it = 0;
       bool ok = peers_ready;
-      for (long long t = tile0; t < p.total_tiles && ok; t += tile_step) {
+      for (uint32_t t = tile0; t < p.total_tiles && ok; t += tile_step) {
         const TileCoord c = decode_tile<BK, CG>(p, t, crank);
         if (c.skip) continue;
         const int buf = acc_it & 1;
@@ -626,15 +649,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
     }
   } else {
     // ------------------------------------------------------------------ epilogue warps
-    // Eight warps: warp w serves TMEM lanes [32*(w%4), +32) (one accumulator row per thread) and the 32-column
-    // chunks with (chunk % 2) == (w-2)/4, so two warps per scheduler hide each other's latency.
+    // Warp w serves TMEM lanes [32*(w%4), +32), one accumulator row per thread.  Specialised epilogues: the 64-column box
+    // (w-2)/4.  Generic epilogue: the 32-column chunks with (chunk % 2) == (w-2)/4.
     const int q = warp & 3;
     const int half = (warp - 2) >> 2;
     uint32_t acc_it = 0, epi_it = 0;
     bool ok = peers_ready;
     // the "accumulator drained" barrier of a pair lives in the leader and counts the warps of both CTAs
     const uint32_t leader_tempty0 = (CG == 2) ? mapa_u32(tempty_bar(0), 0) : 0u;
-    for (long long t = tile0; t < p.total_tiles; t += tile_step) {
+    for (uint32_t t = tile0; t < p.total_tiles; t += tile_step) {
       const TileCoord c = decode_tile<BK, CG>(p, t, crank);
       if (c.skip && p.accumulate) continue;
       const int rt = q * 32 + lane;                 // row inside the tile
@@ -667,131 +690,131 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
       if constexpr (EPI != 0) {
         // ---------------- specialised bf16 epilogues: registers -> swizzled smem box -> TMA store (full lines, clipped
         // at the matrix edge by the tensor map)
-        constexpr bool ONE_BOX = (EPI == 3 || EPI == 4);
-        const uint32_t stg_base = smem_base + stg_off + (warp - 2) * stg_warp_bytes(EPI);
-        uint8_t* const stg_ptr = smem + stg_off + (warp - 2) * stg_warp_bytes(EPI);
-        int sb = 0;
-#pragma unroll 1
-        for (int bx = half; bx < BN / 64; bx += 2) {
-          const int nb = n0 + bx * 64;
-          if (nb >= p.N) break;
+        constexpr bool IN_PLACE = (EPI == 3 || EPI == 4);
+        const int bx = half;
+        const int nb = n0 + bx * 64;
+        // the box this warp's output is written to: staging (1, 2) or the operand's own box (3, 4)
+        const uint32_t box_off = IN_PLACE ? e_off + ebuf * E_BYTES + bx * (BM * 128) + q * (32 * 128)
+                                          : stg_off + (warp - 2) * stg_warp_bytes(EPI) + (EPI == 2 ? 32 * 128 : 0);
+        uint8_t* const box_d = smem + box_off + lane * 128;
+        uint8_t* const box_p = box_d - 32 * 128;      // second output (2)
+        if (nb < p.N) {     // uniform across the warp
           const uint32_t taddr = tmem_base + buf * BN + bx * 64 + (static_cast<uint32_t>(q * 32) << 16);
-          // the staging box written two stores ago (one for the two-output epilogue) must have been read out
-          if constexpr (EPI == 2 || ONE_BOX) tma_store_wait_read<0>();
-          else tma_store_wait_read<1>();
-          __syncwarp();
-          uint8_t* const box_d = stg_ptr + (EPI == 2 ? 32 * 128 : (ONE_BOX ? 0 : sb * 32 * 128));
-          uint8_t* const box_p = stg_ptr;
+          // the previous store of this warp must have read its box (the operand box was released after that already)
+          if constexpr (!IN_PLACE) {
+            tma_store_wait_read<0>();
+            __syncwarp();
+          }
+          const f32x2 alpha2 = f2_pack(p.alpha, p.alpha);
+          const f32x2 rbias2 = f2_pack(rbias, rbias);
           // The 64 columns of a box go through a ROLLED loop of four 16-column steps.  Unrolled, the body of one box ran
-          // to tens of KB of straight-line code per epilogue flavour, the eight epilogue warps (each at another place
+          // to tens of KB of straight-line code per epilogue flavour, the epilogue warps (each at another place
           // in it) missed the instruction caches on most fetches, and "no instruction" was their top stall reason.
+          // Arithmetic is on pairs of columns (fma / mul on f32x2): same roundings, half the instructions.
 #pragma unroll 1
           for (int it = 0; it < 4; ++it) {
-          uint32_t v[16];
-          if (!c.skip) {
-            tmem_ld16(taddr + it * 16, v);
-          } else {
+            uint32_t v[16];
+            if (!c.skip) {
+              tmem_ld16(taddr + it * 16, v);
+            } else {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = 0u;
+              for (int j = 0; j < 16; ++j) v[j] = 0u;
+            }
+#pragma unroll
+            for (int gg = 0; gg < 2; ++gg) {
+              const int g = it * 2 + gg;
+              const int n = nb + g * 8;
+              f32x2 f[4];
+#pragma unroll
+              for (int j = 0; j < 4; ++j) f[j] = rbias2;
+              if (p.bias_mode == 2) {      // the column bias rides on the scaling fma below
+                if (n + 8 <= p.N) {
+                  const ulonglong2 b0 = __ldg(reinterpret_cast<const ulonglong2*>(bias_z + n));
+                  const ulonglong2 b1 = __ldg(reinterpret_cast<const ulonglong2*>(bias_z + n) + 1);
+                  f[0] = b0.x; f[1] = b0.y; f[2] = b1.x; f[3] = b1.y;
+                } else {
+#pragma unroll
+                  for (int j = 0; j < 4; ++j)
+                    f[j] = f2_pack(n + 2 * j < p.N ? __ldg(bias_z + n + 2 * j) : 0.f,
+                                   n + 2 * j + 1 < p.N ? __ldg(bias_z + n + 2 * j + 1) : 0.f);
+                }
+              }
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+                f[j] = f2_fma(f2_pack(__uint_as_float(v[gg * 8 + 2 * j]), __uint_as_float(v[gg * 8 + 2 * j + 1])), alpha2, f[j]);
+              const uint32_t sw = static_cast<uint32_t>((g ^ (lane & 7)) << 4);
+              if constexpr (EPI == 1) {
+                if (p.act == 1) {
+#pragma unroll
+                  for (int j = 0; j < 4; ++j) f[j] = gelu_fwd2(f[j], p.gelu);
+                } else if (p.act != 0) {      // ReLU / soft shrinkage (uniform over the launch)
+#pragma unroll
+                  for (int j = 0; j < 4; ++j) {
+                    float x, y;
+                    f2_unpack(f[j], x, y);
+                    f[j] = f2_pack(act_fwd(x, p.act, p.act_param, p.gelu), act_fwd(y, p.act, p.act_param, p.gelu));
+                  }
+                }
+              }
+              if constexpr (EPI == 2) {
+                f32x2 s2[4];
+                if (p.save_deriv) {      // uniform over the launch: second output = GELU'(pre-activation)
+#pragma unroll
+                  for (int j = 0; j < 4; ++j) gelu_fwd_bwd2(f[j], p.gelu, f[j], s2[j]);
+                } else {
+#pragma unroll
+                  for (int j = 0; j < 4; ++j) {
+                    s2[j] = f[j];
+                    f[j] = gelu_fwd2(f[j], p.gelu);
+                  }
+                }
+                *reinterpret_cast<uint4*>(box_p + sw) = f2_bf16x8(s2);
+              }
+              if constexpr (IN_PLACE) {
+                const uint4 ev = *reinterpret_cast<const uint4*>(box_d + sw);
+                const uint32_t ew[4] = {ev.x, ev.y, ev.z, ev.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  const float e0 = __uint_as_float(ew[j] << 16), e1 = __uint_as_float(ew[j] & 0xffff0000u);
+                  if constexpr (EPI == 3) f[j] = f2_add(f[j], f2_pack(e0, e1));
+                  else if (p.act == 8) f[j] = f2_mul(f[j], f2_pack(e0, e1));      // uniform: the operand is the saved derivative
+                  else f[j] = f2_mul(f[j], f2_pack(act_bwd(e0, p.act, p.gelu), act_bwd(e1, p.act, p.gelu)));
+                }
+              }
+              *reinterpret_cast<uint4*>(box_d + sw) = f2_bf16x8(f);
+            }
           }
-#pragma unroll
-          for (int gg = 0; gg < 2; ++gg) {
-            const int g = it * 2 + gg;
-            const int n = nb + g * 8;
-            float f[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) f[j] = rbias;
-            if (p.bias_mode == 2) {      // the column bias rides on the scaling fma below
-              if (n + 8 <= p.N) {
-                const float4 b0 = __ldg(reinterpret_cast<const float4*>(bias_z + n));
-                const float4 b1 = __ldg(reinterpret_cast<const float4*>(bias_z + n) + 1);
-                f[0] = b0.x; f[1] = b0.y; f[2] = b0.z; f[3] = b0.w;
-                f[4] = b1.x; f[5] = b1.y; f[6] = b1.z; f[7] = b1.w;
-              } else {
-                for (int j = 0; j < 8 && n + j < p.N; ++j) f[j] = __ldg(bias_z + n + j);
-              }
-            }
-#pragma unroll
-            for (int j = 0; j < 8; ++j) f[j] = fmaf(__uint_as_float(v[gg * 8 + j]), p.alpha, f[j]);
-            const uint32_t sw = static_cast<uint32_t>((g ^ (lane & 7)) << 4) + lane * 128;
-            if constexpr (EPI == 1) {
-              if (p.act != 0) {      // ReLU / soft shrinkage (uniform over the launch)
-#pragma unroll
-                for (int j = 0; j < 8; ++j) f[j] = act_fwd(f[j], p.act, p.act_param, p.gelu);
-              }
-            }
-            if constexpr (EPI == 2) {
-              __nv_bfloat162 h[4];
-              if (p.save_deriv) {      // uniform over the launch: second output = GELU'(pre-activation)
-                float d[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) gelu_fwd_bwd(f[j], p.gelu, f[j], d[j]);
-#pragma unroll
-                for (int j = 0; j < 4; ++j) h[j] = __floats2bfloat162_rn(d[2 * j], d[2 * j + 1]);
-                *reinterpret_cast<uint4*>(box_p + sw) = *reinterpret_cast<uint4*>(h);
-              } else {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) h[j] = __floats2bfloat162_rn(f[2 * j], f[2 * j + 1]);
-                *reinterpret_cast<uint4*>(box_p + sw) = *reinterpret_cast<uint4*>(h);
-#pragma unroll
-                for (int j = 0; j < 8; ++j) f[j] = gelu_fwd(f[j], p.gelu);
-              }
-            }
-            if constexpr (EPI == 3 || EPI == 4) {
-              const uint4 ev = *reinterpret_cast<const uint4*>(esm + bx * (BM * 128) + rt * 128 + ((g ^ (rt & 7)) << 4));
-              const __nv_bfloat162* eh = reinterpret_cast<const __nv_bfloat162*>(&ev);
-              if constexpr (EPI == 3) {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                  const float2 x = __bfloat1622float2(eh[j]);
-                  f[2 * j] += x.x;
-                  f[2 * j + 1] += x.y;
-                }
-              } else if (p.act == 8) {      // uniform over the launch: the operand is the saved derivative
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                  const float2 x = __bfloat1622float2(eh[j]);
-                  f[2 * j] *= x.x;
-                  f[2 * j + 1] *= x.y;
-                }
-              } else if (p.act == 2) {      // uniform over the launch: the GELU case carries no per-element selects
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                  const float2 x = __bfloat1622float2(eh[j]);
-                  f[2 * j] *= gelu_bwd(x.x, p.gelu);
-                  f[2 * j + 1] *= gelu_bwd(x.y, p.gelu);
-                }
-              } else {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                  const float2 x = __bfloat1622float2(eh[j]);
-                  f[2 * j] *= act_bwd(x.x, p.act, p.gelu);
-                  f[2 * j + 1] *= act_bwd(x.y, p.act, p.gelu);
-                }
-              }
-            }
-            __nv_bfloat162 h[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) h[j] = __floats2bfloat162_rn(f[2 * j], f[2 * j + 1]);
-            *reinterpret_cast<uint4*>(box_d + sw) = *reinterpret_cast<uint4*>(h);
-          }
-          }
-          fence_async_smem();
+        }
+        if (!c.skip) {     // the accumulator has been read: the next tile but one may overwrite it
+          tc_fence_before();
           __syncwarp();
           if (lane == 0) {
-            const int r0 = c.mt * BM + q * 32;
-            if (r0 < p.M) {
-              if constexpr (EPI == 2) tma_store_4d(&map_p, stg_base, nb, r0, c.zlo, c.zhi);
-              tma_store_4d(&map_d, stg_base + (EPI == 2 ? 32 * 128 : (ONE_BOX ? 0 : sb * 32 * 128)), nb, r0, c.zlo, c.zhi);
-              if constexpr (EPI == 1) {
-                for (int dq = 0; dq < p.ndx; ++dq)   // the same box goes to every peer's copy (plain stores over NVLink)
-                  tma_store_4d(&maps_dx.m[dq], stg_base + sb * 32 * 128, nb, r0, c.zlo, c.zhi);
-              }
+            if constexpr (CG == 2) mbar_arrive_cluster(leader_tempty0 + 8u * buf);
+            else mbar_arrive(tempty_bar(buf));
+          }
+          ++acc_it;
+        }
+        if (nb < p.N) {
+          fence_async_smem();
+          __syncwarp();
+          const int r0 = c.mt * BM + q * 32;
+          if (lane == 0 && r0 < p.M) {
+            if constexpr (EPI == 2) tma_store_4d(&map_p, smem_base + box_off - 32 * 128, nb, r0, c.zlo, c.zhi);
+            tma_store_4d(&map_d, smem_base + box_off, nb, r0, c.zlo, c.zhi);
+            if constexpr (EPI == 1) {
+              for (int dq = 0; dq < p.ndx; ++dq)   // the same box goes to every peer's copy (plain stores over NVLink)
+                tma_store_4d(&maps_dx.m[dq], smem_base + box_off, nb, r0, c.zlo, c.zhi);
             }
             tma_store_commit();
+            if constexpr (IN_PLACE) tma_store_wait_read<0>();   // the operand buffer is free once the store has read it
           }
-          sb ^= 1;
         }
+        if constexpr (IN_PLACE) {
+          __syncwarp();
+          if (lane == 0) mbar_arrive(eempty_bar(ebuf));
+          ++epi_it;
+        }
+        continue;
       } else
 #pragma unroll 1
       for (int cc = half; cc < BN / 32; cc += 2) {
@@ -1058,11 +1081,38 @@ bool make_map(CUtensorMap* map, const GemmOperand& op, int K, int eb, int zlo_n,
 
 constexpr int SMEM_LIMIT = 232448;   // 227 KB per CTA on sm_100
 
+// CTA pairs that can be resident at once.  Every instance fills an SM with its shared memory, so one answers for all.
+int max_pairs() {
+  static const int n = [] {
+    cudaLaunchConfig_t qc;
+    memset(&qc, 0, sizeof(qc));
+    cudaLaunchAttribute qa[1];
+    qa[0].id = cudaLaunchAttributeClusterDimension;
+    qa[0].val.clusterDim.x = 2;
+    qa[0].val.clusterDim.y = 1;
+    qa[0].val.clusterDim.z = 1;
+    qc.gridDim = dim3(2 * (sm_count() / 2), 1, 1);
+    qc.blockDim = dim3(32 * (3 + epi_warps(256, 0)), 1, 1);
+    qc.dynamicSmemBytes = SMEM_LIMIT;
+    qc.attrs = qa;
+    qc.numAttrs = 1;
+    int got = 0;
+    cudaError_t e = cudaFuncSetAttribute(gemm_kernel<256, 2, 0, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&got, gemm_kernel<256, 2, 0, 2>, &qc);
+    if (e != cudaSuccess || got < 1) {
+      (void)cudaGetLastError();
+      got = sm_count() / 2;
+    }
+    return got;
+  }();
+  return n;
+}
+
 template <int BN, int EB, int EPI, int CG>
 cudaError_t launch_t(const CUtensorMap& ma, const BMaps& mb, const CUtensorMap& me, const CUtensorMap& md,
                      const CUtensorMap& mp, const DMaps& mdx, KParams& kp, cudaStream_t stream) {
-  constexpr int STAGE = A_STAGE_BYTES + (BN / CG) * 128;
-  constexpr int FIXED = stg_bytes(EPI) + 8 * (2 * MAX_STAGES + 8) + 16 + 1024;
+  constexpr int STAGE = A_STAGE_BYTES + b_stage_rows(BN, CG) * 128;
+  constexpr int FIXED = stg_bytes(BN, EPI) + 8 * (2 * MAX_STAGES + 8) + 16 + 1024;
   const int e_bytes = kp.e_tma ? 2 * BM * BN * 2 : 0;
   int stages = (SMEM_LIMIT - FIXED - e_bytes) / STAGE;
   if (stages > MAX_STAGES) stages = MAX_STAGES;
@@ -1072,33 +1122,11 @@ cudaError_t launch_t(const CUtensorMap& ma, const BMaps& mb, const CUtensorMap& 
   }
   kp.stages = stages;
   const int smem = stages * STAGE + e_bytes + FIXED;
-  const int threads = kp.e_tma ? NUM_THREADS + 32 : NUM_THREADS;
+  const int threads = 32 * (2 + epi_warps(BN, EPI) + (kp.e_tma ? 1 : 0));
   static bool configured = false;
-  static int pair_clusters = 0;     // CTA pairs that can be resident at once (CG = 2)
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(gemm_kernel<BN, EB, EPI, CG>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT);
     if (e != cudaSuccess) return e;
-    if (CG == 2) {
-      cudaLaunchConfig_t qc;
-      memset(&qc, 0, sizeof(qc));
-      cudaLaunchAttribute qa[1];
-      qa[0].id = cudaLaunchAttributeClusterDimension;
-      qa[0].val.clusterDim.x = 2;
-      qa[0].val.clusterDim.y = 1;
-      qa[0].val.clusterDim.z = 1;
-      qc.gridDim = dim3(2 * (sm_count() / 2), 1, 1);
-      qc.blockDim = dim3(NUM_THREADS + 32, 1, 1);
-      qc.dynamicSmemBytes = SMEM_LIMIT;
-      qc.attrs = qa;
-      qc.numAttrs = 1;
-      int n = 0;
-      e = cudaOccupancyMaxActiveClusters(&n, gemm_kernel<BN, EB, EPI, CG>, &qc);
-      if (e != cudaSuccess || n < 1) {
-        (void)cudaGetLastError();
-        n = sm_count() / 2;
-      }
-      pair_clusters = n;
-    }
     configured = true;
   }
   const int num_sms = sm_count();
@@ -1109,7 +1137,8 @@ cudaError_t launch_t(const CUtensorMap& ma, const BMaps& mb, const CUtensorMap& 
   }();
   kp.n_fast = forced_order >= 0 ? forced_order : (kp.m_tiles > kp.n_tiles ? 1 : 0);
   if (CG == 2) {
-    long long clusters = kp.total_tiles < pair_clusters ? kp.total_tiles : pair_clusters;
+    const int most = max_pairs();
+    long long clusters = kp.total_tiles < static_cast<uint32_t>(most) ? kp.total_tiles : most;
     if (clusters < 1) clusters = 1;
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
@@ -1126,7 +1155,7 @@ cudaError_t launch_t(const CUtensorMap& ma, const BMaps& mb, const CUtensorMap& 
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, gemm_kernel<BN, EB, EPI, CG>, ma, mb, me, md, mp, mdx, kp);
   }
-  long long grid = kp.total_tiles < num_sms ? kp.total_tiles : num_sms;
+  long long grid = kp.total_tiles < static_cast<uint32_t>(num_sms) ? kp.total_tiles : num_sms;
   if (grid < 1) grid = 1;
   gemm_kernel<BN, EB, EPI, CG><<<static_cast<unsigned>(grid), threads, smem, stream>>>(ma, mb, me, md, mp, mdx, kp);
   return cudaGetLastError();
@@ -1134,7 +1163,7 @@ cudaError_t launch_t(const CUtensorMap& ma, const BMaps& mb, const CUtensorMap& 
 
 // tensor map for the epilogue operand: plain [M rows][N contiguous] bf16 with two batch dimensions, no swizzle
 bool make_map_e(CUtensorMap* map, const void* ptr, int M, int N, long long row_stride, long long zs_lo, long long zs_hi,
-                int zlo_n, int zhi_n, int bn, int box_rows = BM) {
+                int zlo_n, int zhi_n, int box_rows = BM) {
   EncodeTiledFn enc = get_encode();
   if (!enc) return false;
   cuuint64_t dims[4] = {static_cast<cuuint64_t>(N), static_cast<cuuint64_t>(M), static_cast<cuuint64_t>(zlo_n),
@@ -1142,7 +1171,6 @@ bool make_map_e(CUtensorMap* map, const void* ptr, int M, int N, long long row_s
   cuuint64_t strides[3] = {static_cast<cuuint64_t>(row_stride) * 2,
                            static_cast<cuuint64_t>(zlo_n > 1 ? zs_lo : row_stride) * 2,
                            static_cast<cuuint64_t>(zhi_n > 1 ? zs_hi : row_stride) * 2};
-  (void)bn;
   cuuint32_t box[4] = {64, static_cast<cuuint32_t>(box_rows), 1, 1};   // 64 bf16 = one 128-byte swizzle row
   cuuint32_t estr[4] = {1, 1, 1, 1};
   if ((reinterpret_cast<uintptr_t>(ptr) & 15) || (strides[0] & 15) || (strides[1] & 15) || (strides[2] & 15)) return false;
@@ -1352,6 +1380,53 @@ cudaError_t peer_sum_launch(void* out, long long n_elems, const void* const* src
   return cudaGetLastError();
 }
 
+namespace {
+FastDiv make_div(int d) {
+  FastDiv f;
+  f.d = static_cast<uint32_t>(d);
+  f.shift = 0;
+  while ((1ull << f.shift) < f.d) ++f.shift;
+  f.mul = static_cast<uint32_t>(((((1ull << f.shift) - f.d) << 32) / f.d) + 1);
+  return f;
+}
+
+// Tile width: the fewest padded columns, a tile costing some 32 columns of its own.  Measured over 721 x 1440 tokens: 384
+// outputs take 567 us (K = 768) and 368 us (K = 384) in 192-column tiles, 664 and 469 us in 256-column tiles, a third of
+// which is padding, 640 and 392 us in 128-column tiles, which fetch the activations once more.
+int pick_bn(int N, int epi, int e_tma) {
+  if (epi == 0 && e_tma) return 128;
+  int best = 128;
+  long long cost = -1;
+  const int widths[3] = {256, 192, 128};
+  for (int i = (epi >= 3 ? 1 : 0); i < 3; ++i) {
+    const long long c = static_cast<long long>((N + widths[i] - 1) / widths[i]) * (widths[i] + 32);
+    if (cost < 0 || c < cost) {
+      cost = c;
+      best = widths[i];
+    }
+  }
+  return best;
+}
+
+// Split-k factor of an accumulating launch: whole waves of `slots` CTAs (or pairs), every split costing its tile one
+// epilogue of atomics, worth some 16 k-blocks.  (Twice as many tiles as SMs, the former rule, left a last wave that was
+// nearly empty: 704 -> 532 us per weight gradient of a 384 <-> 768 layer over 721 x 1440 tokens.)
+int pick_splits(long long base, int kblocks, int slots) {
+  int best = 1;
+  double cost = 1e300;
+  const long long most = 4ll * slots / (base > 0 ? base : 1) + 1;
+  for (int s = 1; s <= most && s <= kblocks; ++s) {
+    const double waves = static_cast<double>((base * s + slots - 1) / slots);
+    const double c = waves * ((kblocks + s - 1) / s + 16.0);
+    if (c < cost * 0.999) {
+      cost = c;
+      best = s;
+    }
+  }
+  return best;
+}
+}  // namespace
+
 cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOperand& B, const GemmEpilogue& e,
                         int* err_flag, cudaStream_t stream, const GemmPeer* peer) {
   g_err[0] = 0;
@@ -1373,9 +1448,8 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
     return cudaErrorInvalidValue;
   }
   int bn = p.bn;
-  if (bn == 0) bn = (p.N > 128) ? 256 : 128;
-  if (bn != 128 && bn != 256) {
-    snprintf(g_err, sizeof(g_err), "bn must be 128 or 256");
+  if (bn != 0 && bn != 128 && bn != 192 && bn != 256) {
+    snprintf(g_err, sizeof(g_err), "bn must be 128, 192 or 256");
     return cudaErrorInvalidValue;
   }
   if (eb == 4 && (A.mn_major || B.mn_major)) {
@@ -1397,8 +1471,6 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
   kp.zlo_n = p.zlo_n; kp.zhi_n = p.zhi_n;
   kp.splits = p.splits < 1 ? 1 : p.splits;
   const int kblocks = (p.K + bk - 1) / bk;
-  kp.k_per_split = ((kblocks + kp.splits - 1) / kp.splits) * bk;
-  if (kp.k_per_split < bk) kp.k_per_split = bk;
   kp.a_mn = A.mn_major; kp.b_mn = B.mn_major;
   kp.a_zlo = (A.zs_lo != 0 && p.zlo_n > 1); kp.a_zhi = (A.zs_hi != 0 && p.zhi_n > 1);
   kp.b_zlo = (B.zs_lo != 0 && p.zlo_n > 1); kp.b_zhi = (B.zs_hi != 0 && p.zhi_n > 1);
@@ -1419,9 +1491,6 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
   if (e.resid) vec = vec && ((reinterpret_cast<uintptr_t>(e.resid) & amask) == 0);
   if (e.preact) vec = vec && ((reinterpret_cast<uintptr_t>(e.preact) & amask) == 0);
   kp.vec_ok = vec ? 1 : 0;
-  kp.m_tiles = (p.M + BM - 1) / BM;
-  kp.n_tiles = (p.N + bn - 1) / bn;
-  kp.total_tiles = static_cast<long long>(kp.m_tiles) * kp.n_tiles * kp.splits * p.zlo_n * p.zhi_n;
   kp.err = err_flag;
   kp.nseg = 1;
   kp.ndx = 0;
@@ -1453,9 +1522,30 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
   kp.e_tma = 0;
   const bool plain = (e.rdiv <= 0 || e.rdiv >= (1 << 30)) && (e.ndiv <= 0 || e.ndiv >= (1 << 30));
   if (e.resid && !e.out_f32 && plain && kp.vec_ok && e.d_zlo >= 0 && e.d_zhi >= 0) {
-    if (make_map_e(&me, e.resid, p.M, p.N, e.rs_lo, e.d_zlo, e.d_zhi, p.zlo_n, p.zhi_n, 128)) {
-      kp.e_tma = 1;
-      bn = 128;
+    if (make_map_e(&me, e.resid, p.M, p.N, e.rs_lo, e.d_zlo, e.d_zhi, p.zlo_n, p.zhi_n)) kp.e_tma = 1;
+  }
+  // A specialised epilogue (TMA stores of bf16 tiles) when the launch fits one.
+  int epi = 0;
+  CUtensorMap md, mp;
+  DMaps mdx;
+  memset(&md, 0, sizeof(md));
+  memset(&mp, 0, sizeof(mp));
+  memset(&mdx, 0, sizeof(mdx));
+  if (eb == 2 && !e.out_f32 && kp.vec_ok && !e.accumulate && plain && e.d_zlo >= 0 && e.d_zhi >= 0 &&
+      (kp.bias_mode != 2 || ((reinterpret_cast<uintptr_t>(e.bias) & 15) == 0 && (kp.bias_zs % 4) == 0))) {
+    if (!e.resid && !e.preact && (e.act == 0 || e.act == 1 || e.act == 3 || e.act == 5)) epi = 1;
+    else if (!e.resid && e.preact && e.act == 1) epi = 2;
+    else if (e.resid && kp.e_tma && !e.preact && e.act == 0) epi = 3;
+    else if (e.resid && kp.e_tma && !e.preact && (e.act == 2 || e.act == 4 || e.act == 6 || e.act == 8)) epi = 4;
+    if (epi != 0) {
+      bool ok = make_map_e(&md, e.D, p.M, p.N, e.rs_lo, e.d_zlo, e.d_zhi, p.zlo_n, p.zhi_n, 32);
+      if (ok && epi == 2) ok = make_map_e(&mp, e.preact, p.M, p.N, e.rs_lo, e.d_zlo, e.d_zhi, p.zlo_n, p.zhi_n, 32);
+      if (ok && kp.ndx > 0) {
+        if (epi != 1) ok = false;   // replicated output goes through the plain-store epilogue or the generic one
+        for (int q = 0; ok && q < kp.ndx; ++q)
+          ok = make_map_e(&mdx.m[q], kp.Dx[q], p.M, p.N, e.rs_lo, e.d_zlo, e.d_zhi, p.zlo_n, p.zhi_n, 32);
+      }
+      if (!ok) epi = 0;
     }
   }
   // CTA pairs (256-row tiles, each CTA loads half of the B tile): single-device bf16 launches without row-triangular
@@ -1472,11 +1562,26 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
                                               peer->done_ctr == nullptr);
   const bool eligible = eb == 2 && no_peer && p.M > BM && p.rmin_a == 0 && p.rmax_a == 0;
   const int cg = (eligible && (pairs_mode == 1 || (pairs_mode == 2 && p.K >= 512))) ? 2 : 1;
+  if (bn == 0) bn = pick_bn(p.N, epi, kp.e_tma);
+  if ((eb == 4 && bn == 192) || ((epi >= 3 || kp.e_tma) && bn == 256)) bn = 128;
+  if (epi == 0 && kp.e_tma) bn = 128;
   kp.m_tiles = (p.M + BM * cg - 1) / (BM * cg);
   kp.n_tiles = (p.N + bn - 1) / bn;
-  kp.total_tiles = static_cast<long long>(kp.m_tiles) * kp.n_tiles * kp.splits * p.zlo_n * p.zhi_n;
+  const long long base_tiles = static_cast<long long>(kp.m_tiles) * kp.n_tiles * p.zlo_n * p.zhi_n;
+  if (p.splits == 0 && e.accumulate) kp.splits = pick_splits(base_tiles, kblocks, cg == 2 ? max_pairs() : sm_count());
+  kp.k_per_split = ((kblocks + kp.splits - 1) / kp.splits) * bk;
+  if (kp.k_per_split < bk) kp.k_per_split = bk;
+  if (base_tiles * kp.splits >= (1ll << 31)) {
+    snprintf(g_err, sizeof(g_err), "too many tiles");
+    return cudaErrorInvalidValue;
+  }
+  kp.total_tiles = static_cast<uint32_t>(base_tiles * kp.splits);
+  kp.dv_n = make_div(kp.n_tiles);
+  kp.dv_m = make_div(kp.m_tiles);
+  kp.dv_split = make_div(kp.splits);
+  kp.dv_zlo = make_div(p.zlo_n);
   if (!make_map(&ma, A, p.K, eb, p.zlo_n, p.zhi_n, BM)) return cudaErrorInvalidValue;
-  const int bn_box = bn / cg;     // rows of B one CTA loads per stage
+  const int bn_box = bn / cg;     // rows of a K-major B one CTA loads per stage
   BMaps mbs;
   if (kp.nseg > 1) {
     for (int q = 0; q < kp.nseg; ++q) {
@@ -1492,31 +1597,9 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
   if (!kp.e_tma) me = ma;   // unused, but must be a valid descriptor
 
   kp.plain_cols = (e.ndiv <= 0 || e.ndiv >= (1 << 30)) ? 1 : 0;
-  // pick a specialised epilogue (TMA stores of bf16 tiles) when the launch fits one
-  int epi = 0;
-  CUtensorMap md, mp;
-  memset(&md, 0, sizeof(md));
-  md = ma;
-  mp = ma;
-  DMaps mdx;
-  for (int q = 0; q < MAX_SEG - 1; ++q) mdx.m[q] = ma;   // placeholders: always valid descriptors
-  if (eb == 2 && !e.out_f32 && kp.vec_ok && !e.accumulate && plain && e.d_zlo >= 0 && e.d_zhi >= 0 &&
-      (kp.bias_mode != 2 || ((reinterpret_cast<uintptr_t>(e.bias) & 15) == 0 && (kp.bias_zs % 4) == 0))) {
-    if (!e.resid && !e.preact && (e.act == 0 || e.act == 3 || e.act == 5)) epi = 1;
-    else if (!e.resid && e.preact && e.act == 1) epi = 2;
-    else if (e.resid && kp.e_tma && !e.preact && e.act == 0) epi = 3;
-    else if (e.resid && kp.e_tma && !e.preact && (e.act == 2 || e.act == 4 || e.act == 6 || e.act == 8)) epi = 4;
-    if (epi != 0) {
-      bool ok = make_map_e(&md, e.D, p.M, p.N, e.rs_lo, e.d_zlo, e.d_zhi, p.zlo_n, p.zhi_n, bn, 32);
-      if (ok && epi == 2) ok = make_map_e(&mp, e.preact, p.M, p.N, e.rs_lo, e.d_zlo, e.d_zhi, p.zlo_n, p.zhi_n, bn, 32);
-      if (ok && kp.ndx > 0) {
-        if (epi != 1) ok = false;   // replicated output goes through the plain-store epilogue or the generic one
-        for (int q = 0; ok && q < kp.ndx; ++q)
-          ok = make_map_e(&mdx.m[q], kp.Dx[q], p.M, p.N, e.rs_lo, e.d_zlo, e.d_zhi, p.zlo_n, p.zhi_n, bn, 32);
-      }
-      if (!ok) epi = 0;
-    }
-  }
+  if (epi == 0) md = ma;       // unused maps must be valid descriptors all the same
+  if (epi != 2) mp = ma;
+  for (int q = (epi == 1 ? kp.ndx : 0); q < MAX_SEG - 1; ++q) mdx.m[q] = ma;
   if (eb == 4) {
     if (bn == 256) return launch_t<256, 4, 0, 1>(ma, mbs, me, md, mp, mdx, kp, stream);
     return launch_t<128, 4, 0, 1>(ma, mbs, me, md, mp, mdx, kp, stream);
@@ -1524,9 +1607,11 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
 #define MK_DISPATCH(EPI_)                                                                              \
   if (cg == 2) {                                                                                       \
     if (bn == 256) return launch_t<256, 2, EPI_, 2>(ma, mbs, me, md, mp, mdx, kp, stream);             \
+    if (bn == 192) return launch_t<192, 2, EPI_, 2>(ma, mbs, me, md, mp, mdx, kp, stream);             \
     return launch_t<128, 2, EPI_, 2>(ma, mbs, me, md, mp, mdx, kp, stream);                            \
   }                                                                                                    \
   if (bn == 256) return launch_t<256, 2, EPI_, 1>(ma, mbs, me, md, mp, mdx, kp, stream);               \
+  if (bn == 192) return launch_t<192, 2, EPI_, 1>(ma, mbs, me, md, mp, mdx, kp, stream);               \
   return launch_t<128, 2, EPI_, 1>(ma, mbs, me, md, mp, mdx, kp, stream);
   switch (epi) {
     case 1: { MK_DISPATCH(1) }

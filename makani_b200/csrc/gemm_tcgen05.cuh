@@ -58,10 +58,10 @@ struct GemmProblem {
   int M, N, K;
   int zlo_n, zhi_n;
   int elem_bytes;       // 2: bf16, 4: tf32
-  int splits;           // split-k factor (requires accumulate)
+  int splits;           // split-k factor (requires accumulate; 0: chosen here)
   int rmin_a, rmin_b, rmax_a, rmax_b;   // valid rows [rmin_a*z_hi+rmin_b, rmax_a*z_hi+rmax_b)
   int kmin_a, kmin_b, kmax_a, kmax_b;   // contributing k range
-  int bn;               // tile width: 128 or 256 (0 = choose)
+  int bn;               // tile width: 128, 192 or 256 (0 = choose)
 };
 
 // Optional: B operand gathered from several devices and cross-device handshakes (see gemm_tcgen05.cu).

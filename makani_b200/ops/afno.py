@@ -214,11 +214,9 @@ class _AFNOFilter(torch.autograd.Function):
              Operand(w1q, ld=2 * bs, mn_major=True, zs_lo=2 * hid * 2 * bs),
              Output(dyt, rs_lo=2 * bs, rdiv=nkx, rs_hi=nb * nkx * 2 * bs, d_zlo=nkx * 2 * bs), zlo_n=nb)
         dw1 = torch.zeros(nb, 2 * hid, 2 * bs, dtype=torch.float32, device=dev)
-        tiles = nb * ((2 * hid + 127) // 128)
-        splits = max(1, min((T + 63) // 64, (2 * _ext.sm_count() + tiles - 1) // tiles))
         gemm(2 * hid, 2 * bs, T, Operand(do1, ld=nb * 2 * hid, mn_major=True, zs_lo=2 * hid),
              Operand(y, ld=2 * C, mn_major=True, zs_lo=2 * bs),
-             Output(dw1, rs_lo=2 * bs, d_zlo=2 * hid * 2 * bs), zlo_n=nb, accumulate=True, splits=splits)
+             Output(dw1, rs_lo=2 * bs, d_zlo=2 * hid * 2 * bs), zlo_n=nb, accumulate=True, splits=0)
         db1 = do1.float().sum(dim=0) if has_b1 else None
         # adjoint of the analysis along H and along W; the skip's gradient joins in the last epilogue
         dt1 = _stage_h_blocks(dyt, plan.gh, plan, B, C, nb)                            # [H, B*ncols, 2, C]

@@ -134,16 +134,12 @@ def _conv_dgrad(dy, wq, ci, act=ACT_NONE, aux=None, x_layout=None, out=None, syn
     return dx
 
 
-def _conv_wgrad(dy, x, splits: Optional[int] = None):
+def _conv_wgrad(dy, x, splits: int = 0):
     """dW[co, ci] = sum_{b,hw} dY[b, co, hw] X[b, ci, hw] in fp32 (split-k, atomically accumulated)."""
     B, co, H, W = dy.shape
     ci = x.shape[1]
     T = H * W
     dw = torch.zeros(co, ci, dtype=torch.float32, device=dy.device)
-    if splits is None:
-        tiles = ((co + 127) // 128) * ((ci + 255) // 256) * B
-        kblocks = (T + 63) // 64
-        splits = max(1, min(kblocks, (2 * _ext.sm_count() + tiles - 1) // tiles))
     gemm(co, ci, T, _chan_rows(dy, layout_of(dy)), _chan_rows(x, layout_of(x)), Output(dw, rs_lo=ci), zlo_n=B,
          accumulate=True, splits=splits)
     return dw

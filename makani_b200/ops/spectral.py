@@ -100,7 +100,7 @@ def dft_analysis(x: torch.Tensor, mat: torch.Tensor, mat_mn: bool, mat_ld: int, 
          Operand(mat, ld=mat_ld, mn_major=mat_mn),
          Operand(x, ld=C, mn_major=True, zs_lo=W * C, zs_hi=H * W * C),
          Output(t1, rs_lo=C, d_zlo=k2 * C, d_zhi=H * k2 * C),
-         zlo_n=H, zhi_n=B, bn=128 if C <= 128 or C % 256 != 0 else 256)
+         zlo_n=H, zhi_n=B)
     return t1
 
 
@@ -112,7 +112,7 @@ def dft_synthesis(t4: torch.Tensor, mat: torch.Tensor, mat_mn: bool, mat_ld: int
          Operand(mat, ld=mat_ld, mn_major=mat_mn),
          Operand(t4, ld=C, mn_major=True, zs_lo=k2 * C, zs_hi=H * k2 * C),
          Output(y, rs_lo=C, d_zlo=W * C, d_zhi=H * W * C),
-         zlo_n=H, zhi_n=B, bn=128 if C <= 128 or C % 256 != 0 else 256)
+         zlo_n=H, zhi_n=B)
     return y
 
 

@@ -1,0 +1,68 @@
+"""Tile widths, remainders and the streaming kernels at the sizes where they can go wrong, against plain PyTorch (-m gpu)."""
+
+import pytest
+import torch
+
+from makani_b200.ops import _ext
+from makani_b200.ops.gemm import (ACT_DGELU, ACT_GELU, ACT_MULAUX, ACT_NONE, ACT_RELU, BIAS_COL, Operand, Output, gemm)
+from test_gpu_kernels import _dev, _rel, _run_both
+
+pytestmark = pytest.mark.gpu
+
+BF16 = 2.0 ** -8      # spacing of bf16 relative to the value: a rounded result is within half of it of the fp32 one
+
+
+@pytest.mark.parametrize("pair", [False, True])
+@pytest.mark.parametrize("w_mn", [False, True])
+@pytest.mark.parametrize("n", [8, 136, 192, 200, 384, 776])
+@pytest.mark.parametrize("epi", ["plain", "gelu", "relu", "gelu_pre", "gelu_deriv", "resid", "mul", "dgelu"])
+def test_gemm_192_column_tiles(pair, w_mn, n, epi):
+    """192-column tiles on single CTAs and pairs, both majors of the weight, every specialised epilogue, N from one vector
+    over one tile and its edges to several tiles, more row tiles than one wave of the smallest grid, ragged rows."""
+    dev = _dev()
+    k = 520 if pair else 72           # pairs run from K = 512 on
+    m = 128 * 9 + 40
+    torch.manual_seed(n + k)
+    x = torch.randn(2, m, k, device=dev).to(torch.bfloat16)
+    w = (torch.randn(n, k, device=dev) / k ** 0.5).to(torch.bfloat16)
+    op = Operand(w.t().contiguous(), ld=n, mn_major=True) if w_mn else Operand(w, ld=k)
+    aux = torch.randn(2, m, n, device=dev).to(torch.bfloat16) if epi in ("resid", "mul", "dgelu") else None
+    pre = torch.zeros(2, m, n, device=dev, dtype=torch.bfloat16) if epi in ("gelu_pre", "gelu_deriv") else None
+    act = {"plain": ACT_NONE, "resid": ACT_NONE, "relu": ACT_RELU, "mul": ACT_MULAUX, "dgelu": ACT_DGELU}.get(epi, ACT_GELU)
+    bias = None if epi in ("mul", "dgelu") else torch.randn(n, device=dev)
+    d = torch.zeros(2, m, n, device=dev, dtype=torch.bfloat16)
+    outs = _run_both(m, n, k, Operand(x, ld=k, zs_lo=m * k), op, Output(d, rs_lo=n, d_zlo=m * n), zlo_n=2, bias=bias,
+                     bias_mode=BIAS_COL, act=act, resid=aux, preact=pre, preact_deriv=epi == "gelu_deriv", bn=192)
+    for got, ref in outs:
+        assert _rel(got, ref) < BF16
+
+
+@pytest.mark.parametrize("tokens", [64 * 3, 64 * 400 + 8, 128 * 150 * 3])
+def test_gemm_one_box_per_tile_over_many_tiles(tokens):
+    """Outputs of one 64-column box per tile with a one-slab k loop: the store of a tile must have read its staging box
+    before the next tile, which follows at once, is written there."""
+    dev = _dev()
+    torch.manual_seed(tokens)
+    x = torch.randn(tokens, 16, device=dev).to(torch.bfloat16)
+    w = torch.randn(16, 16, device=dev).to(torch.bfloat16)
+    for _ in range(3):
+        d = torch.empty(tokens, 16, device=dev, dtype=torch.bfloat16)
+        gemm(tokens, 16, 16, Operand(x, ld=16), Operand(w, ld=16, mn_major=True), Output(d, rs_lo=16))
+        assert _rel(d, x.float() @ w.float()) < BF16
+    _ext.check_device_errors(dev)
+
+
+@pytest.mark.parametrize("bn", [0, 128, 192, 256])
+@pytest.mark.parametrize("co,ci,t", [(16, 8, 40), (384, 384, 5000), (200, 392, 64 * 9), (768, 384, 20000)])
+def test_gemm_chosen_splits(bn, co, ci, t):
+    """Weight gradients with the split-k factor left to the launcher; K from under one slab to many per split."""
+    dev = _dev()
+    torch.manual_seed(co + t)
+    dy = torch.randn(t, co, device=dev).to(torch.bfloat16)
+    x = torch.randn(t, ci, device=dev).to(torch.bfloat16)
+    dw = torch.zeros(co, ci, device=dev)
+    gemm(co, ci, t, Operand(dy, ld=co, mn_major=True), Operand(x, ld=ci, mn_major=True), Output(dw, rs_lo=ci), accumulate=True,
+         splits=0, bn=bn)
+    # fp32 sums of t exact products
+    assert _rel(dw, dy.double().t() @ x.double()) < 2.0 ** -24 * max(t, 64) ** 0.5 * 4
+    _ext.check_device_errors(dev)
