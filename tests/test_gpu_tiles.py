@@ -66,3 +66,21 @@ def test_gemm_chosen_splits(bn, co, ci, t):
     # fp32 sums of t exact products
     assert _rel(dw, dy.double().t() @ x.double()) < 2.0 ** -24 * max(t, 64) ** 0.5 * 4
     _ext.check_device_errors(dev)
+
+
+@pytest.mark.parametrize("b", [1, 2, 3])
+@pytest.mark.parametrize("i,o,x,y", [(1, 1, 1, 1), (5, 3, 4, 4), (4, 8, 16, 18), (9, 6, 7, 37), (8, 12, 40, 41)])
+def test_diagonal_contraction_edges(b, i, o, x, y):
+    """Odd and even numbers of modes (8- and 16-byte accesses), channel counts around the four per thread, odd batches."""
+    from makani_b200.ops.spectral_modes import contract_diagonal
+    dev = _dev()
+    g = torch.Generator(dev).manual_seed(i * o + x)
+    rnd = lambda *s: torch.randn(*s, dtype=torch.complex64, device=dev, generator=g)  # noqa: E731
+    a, w, dy = rnd(b, i, x, y).requires_grad_(), rnd(i, o, x, y).requires_grad_(), rnd(b, o, x, y)
+    out = contract_diagonal(a, w)
+    got = [out] + list(torch.autograd.grad(out, [a, w], dy))
+    ad, wd = a.detach().to(torch.complex128).requires_grad_(), w.detach().to(torch.complex128).requires_grad_()
+    r = torch.einsum("bixy,ioxy->boxy", ad, wd)
+    ref = [r] + list(torch.autograd.grad(r, [ad, wd], dy.to(torch.complex128)))
+    for p, q in zip(got, ref):
+        assert _rel(torch.view_as_real(p.detach()), torch.view_as_real(q.detach())) < 2.0 ** -21
