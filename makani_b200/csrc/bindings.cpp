@@ -277,6 +277,17 @@ void inorm_partial_stats(const Tensor& x, Tensor& sums) {
              "inorm_partial_stats");
 }
 
+// sums over all rows of x, whose storage is `rows` dense rows of out.numel() columns (contiguous tokens or channels-last)
+void colsum(const Tensor& x, Tensor& out) {
+  MK_CHECK(x.is_cuda() && x.scalar_type() == torch::kBFloat16 && x.is_non_overlapping_and_dense(), "colsum: dense bf16 CUDA tensor expected");
+  MK_CHECK(out.is_cuda() && out.scalar_type() == torch::kFloat32 && out.is_contiguous() && out.numel() > 0 && x.numel() % out.numel() == 0,
+           "colsum: bad output");
+  c10::cuda::CUDAGuard guard(x.device());
+  check_cuda(mk::colsum(reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()), out.data_ptr<float>(), x.numel() / out.numel(),
+                        static_cast<int>(out.numel()), cur_stream()),
+             "colsum");
+}
+
 void inorm_bwd(const Tensor& x, const Tensor& dy, c10::optional<Tensor> dx, const c10::optional<Tensor>& w,
                const c10::optional<Tensor>& b, const Tensor& stats, c10::optional<Tensor> dw, c10::optional<Tensor> db,
                c10::optional<Tensor> sums_io, int64_t C, double count, int64_t act, int64_t ext_sums) {
@@ -546,6 +557,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("clear_error_flag", &clear_error_flag);
   m.def("inorm_fwd", &inorm_fwd);
   m.def("inorm_partial_stats", &inorm_partial_stats);
+  m.def("colsum", &colsum);
   m.def("inorm_bwd", &inorm_bwd);
   m.def("inorm_cl_sums", &inorm_cl_sums, py::arg("x"), py::arg("dy"), py::arg("w"), py::arg("b"), py::arg("stats"), py::arg("sums"),
         py::arg("dw"), py::arg("db"), py::arg("B"), py::arg("C"), py::arg("act"), py::arg("mode"),

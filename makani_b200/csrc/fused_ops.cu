@@ -558,6 +558,61 @@ __global__ void __launch_bounds__(CL_THREADS) inorm_cl_apply_kernel(const __nv_b
   }
 }
 
+// ------------------------------------------------------------------------------------------ column sums
+
+// out[c] += sum_r x[r, c] for x [rows, C] bf16 (C a multiple of 8): the bias gradients.  One read of x; thread (v, r) owns
+// eight columns and every R-th row of its slab with eight 16-byte loads in flight, so the HBM latency is covered at two
+// CTAs per SM.  16200 tokens: 3072 columns 27 us, 768 columns 10 us, where a cast to fp32 and a torch sum took 185 and
+// 63 us; 2048 x 16: 4 us, where the statistics kernel of the instance norm took 37 us.
+constexpr int CS_THREADS = 256;
+__global__ void __launch_bounds__(CS_THREADS) colsum_kernel(const uint4* __restrict__ x, float* __restrict__ out, long long rows,
+                                                            int V, int vb, int slab) {
+  __shared__ __align__(16) float sh[CS_THREADS * 8];
+  const int v0 = blockIdx.x * vb;
+  const int nv = min(vb, V - v0);          // 16-byte columns of this CTA
+  const int R = CS_THREADS / vb;
+  const int v = threadIdx.x % vb, r = threadIdx.x / vb;
+  for (int i = threadIdx.x; i < nv * 8; i += CS_THREADS) sh[i] = 0.f;
+  __syncthreads();
+  if (r < R && v < nv) {
+    float a[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) a[j] = 0.f;
+    const long long t0 = static_cast<long long>(blockIdx.y) * slab;
+    const long long t1 = min(t0 + slab, rows);
+    const uint4* xv = x + v0 + v;
+    auto add = [&](const uint4& q) {
+      float f[8];
+      unpack8(q, f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) a[j] += f[j];
+    };
+    long long t = t0 + r;
+    for (; t + 7LL * R < t1; t += 8LL * R) {
+      uint4 q[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) q[u] = __ldg(xv + (t + u * R) * V);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) add(q[u]);
+    }
+    for (; t < t1; t += R) add(__ldg(xv + t * V));
+    const bool fold = vb < 32 && (vb & (vb - 1)) == 0;      // lanes with the same columns: shuffles before the atomics
+    if (fold) {
+      for (int o = 16; o >= vb; o >>= 1) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) a[j] += __shfl_xor_sync(0xffffffffu, a[j], o);
+      }
+    }
+    if (!fold || (threadIdx.x & 31) < vb) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) atomicAdd(&sh[v * 8 + j], a[j]);
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x * 4; i < nv * 8; i += CS_THREADS * 4)
+    atomicAdd(reinterpret_cast<float4*>(out + static_cast<long long>(v0) * 8 + i), *reinterpret_cast<const float4*>(sh + i));
+}
+
 // ------------------------------------------------------------------------------------------ Lp norms
 
 constexpr int LP_CHUNK = 1 << 16;   // elements of one plane handled by one CTA
@@ -1012,6 +1067,21 @@ cudaError_t inorm_cl_apply(const __nv_bfloat16* x, const __nv_bfloat16* dy, __nv
   const size_t shx = xc.npeers > 0 ? 2 * C * sizeof(float) : 0;
   if (mode == 0) inorm_cl_apply_kernel<0><<<grid, CL_THREADS, shx, s>>>(x, dy, out, w, b, sums, stats, C, T, inv, eps, act, slab, shifted, xc);
   else inorm_cl_apply_kernel<1><<<grid, CL_THREADS, shx, s>>>(x, dy, out, w, b, sums, stats, C, T, inv, eps, act, slab, 0, xc);
+  return cudaGetLastError();
+}
+
+cudaError_t colsum(const __nv_bfloat16* x, float* out, long long rows, int C, cudaStream_t s) {
+  if (rows <= 0 || C <= 0) return cudaSuccess;
+  if ((C & 7) || !aligned16(x) || !aligned16(out)) return cudaErrorInvalidValue;
+  const int V = C / 8;
+  const int parts = (V + CS_THREADS - 1) / CS_THREADS;
+  const int vb = (V + parts - 1) / parts;
+  const int R = CS_THREADS / vb;
+  // about four CTAs per SM, each with at least one full step of eight rows per thread
+  long long slab = (rows * parts + 4LL * sm_count() - 1) / (4LL * sm_count());
+  if (slab < 8LL * R) slab = 8LL * R;
+  dim3 grid(parts, static_cast<unsigned>((rows + slab - 1) / slab));
+  colsum_kernel<<<grid, CS_THREADS, 0, s>>>(reinterpret_cast<const uint4*>(x), out, rows, V, vb, static_cast<int>(slab));
   return cudaGetLastError();
 }
 

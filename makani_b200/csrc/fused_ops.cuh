@@ -58,6 +58,9 @@ cudaError_t inorm_cl_apply(const __nv_bfloat16* x, const __nv_bfloat16* dy, __nv
                            const float* sums, float* stats, int B, int C, long long T, double count, float eps, int act, int mode,
                            cudaStream_t s, const StatExchange* xch = nullptr);
 
+// out[c] += sum over rows of x[rows, C] (C % 8 == 0, 16-byte aligned; out zero-initialised by the caller)
+cudaError_t colsum(const __nv_bfloat16* x, float* out, long long rows, int C, cudaStream_t s);
+
 // ---- quadrature-weighted Lp norms on the sphere ----
 // out[plane] = (sum_hw q[h] |p-t|^P, sum_hw q[h] |t|^P), P in {1,2}.  `scratch` holds
 // planes*chunks*2 floats + planes ints (zero-initialised once; the kernel leaves the counters at zero).

@@ -9,7 +9,8 @@ from __future__ import annotations
 import torch
 
 from . import _ext
-from .gemm import ACT_GELU, ACT_MULAUX, ACT_NONE, BIAS_COL, Operand, Output, gemm, pad_to
+from .gemm import ACT_GELU, ACT_MULAUX, ACT_NONE, BIAS_COL, Operand, Output, gemm
+from .norm import row_sums
 
 
 def fast_path_ok(x: torch.Tensor) -> bool:
@@ -70,10 +71,10 @@ class _MLP2Last(torch.autograd.Function):
         dy2 = dy.reshape(-1, dy.shape[-1]).contiguous()
         dpre = _lin_dgrad(dy2, w2q, act=ACT_MULAUX, aux=dact)
         dw2 = _lin_wgrad(dy2, h)
-        db2 = dy2.float().sum(0) if ctx.flags[1] else None
+        db2 = row_sums(dy2, dy2.shape[1]) if ctx.flags[1] else None
         dx = _lin_dgrad(dpre, w1q).reshape(ctx.shp) if ctx.needs_input_grad[0] else None
         dw1 = _lin_wgrad(dpre, x2)
-        db1 = dpre.float().sum(0) if ctx.flags[0] else None
+        db1 = row_sums(dpre, dpre.shape[1]) if ctx.flags[0] else None
         return dx, dw1, db1, dw2, db2
 
 
@@ -96,7 +97,7 @@ class _LinearLast(torch.autograd.Function):
         dy2 = dy.reshape(-1, dy.shape[-1]).contiguous()
         dx = _lin_dgrad(dy2, wq).reshape(ctx.shp) if ctx.needs_input_grad[0] else None
         dw = _lin_wgrad(dy2, x2) if ctx.needs_input_grad[1] else None
-        db = dy2.float().sum(0) if ctx.has_bias else None
+        db = row_sums(dy2, dy2.shape[1]) if ctx.has_bias else None
         return dx, dw, db
 
 

@@ -136,14 +136,17 @@ def instance_norm(x: torch.Tensor, weight, bias, eps: float = 1e-6, act: str = "
     return y.to(x.dtype)
 
 
+def row_sums(x: torch.Tensor, C: int) -> torch.Tensor:
+    """fp32 [C]: sum over the rows of a dense bf16 CUDA tensor whose storage is rows of C columns (C a multiple of 8)."""
+    out = torch.zeros(C, dtype=torch.float32, device=x.device)
+    _ext.require().colsum(x, out)
+    return out
+
+
 def channel_sums(x: torch.Tensor) -> torch.Tensor:
     """sum over (batch, H, W) of a 4-D activation in fp32 (bias gradients)."""
-    if cl_supported(x):
-        ext = _ext.require()
-        B, C = x.shape[0], x.shape[1]
-        sums = torch.zeros(B, C, 2, dtype=torch.float32, device=x.device)
-        ext.inorm_cl_sums(x, None, None, None, None, sums, None, None, B, C, 0, 0)
-        return sums[..., 0].sum(0)
+    if _ext.native() and x.is_cuda and x.dtype == torch.bfloat16 and _is_cl(x) and x.shape[1] % 8 == 0:
+        return row_sums(x, x.shape[1])
     if x.is_cuda and x.dtype == torch.bfloat16 and x.is_contiguous():
         ext = _ext.require()
         B, C = x.shape[0], x.shape[1]

@@ -84,3 +84,13 @@ def test_diagonal_contraction_edges(b, i, o, x, y):
     ref = [r] + list(torch.autograd.grad(r, [ad, wd], dy.to(torch.complex128)))
     for p, q in zip(got, ref):
         assert _rel(torch.view_as_real(p.detach()), torch.view_as_real(q.detach())) < 2.0 ** -21
+
+
+@pytest.mark.parametrize("rows,c", [(1, 8), (7, 16), (2049, 24), (5000, 256), (777, 384), (300, 3072), (33, 4104), (100000, 128)])
+def test_column_sums(rows, c):
+    from makani_b200.ops.norm import row_sums
+    dev = _dev()
+    x = torch.randn(rows, c, device=dev, generator=torch.Generator(dev).manual_seed(rows)).to(torch.bfloat16)
+    got, ref = row_sums(x, c).double(), x.double().sum(0)
+    # fp32 summation: error within rows * 2^-24 of the sum of magnitudes, in practice its square root
+    assert ((got - ref).abs() <= 2.0 ** -24 * 8 * max(rows, 4) ** 0.5 * x.double().abs().sum(0) / rows ** 0.5 + 1e-6).all()
