@@ -895,6 +895,49 @@ __global__ void spectral_expand_kernel(const float2* __restrict__ w, __nv_bfloat
   }
 }
 
+// The same re-layout with 16-byte accesses on both sides, for an even number of degrees and Cin a multiple of 8: a 64-channel
+// by 32-degree tile, so that the writes are 128-byte segments (the kernel above: 64 bytes, one element per lane and
+// store) and every thread has four 16-byte loads in flight.  384 x 384 x 240: 149 -> 95 us, 6.0 TB/s over reads and writes.
+// grid: (ceil(Cin / 64), Cout, ceil(L / 32)); 256 threads
+constexpr int SX_PITCH = 64 + 8;      // bf16 per tile row (16-byte aligned rows)
+__global__ void __launch_bounds__(256) spectral_expand_vec_kernel(const float2* __restrict__ w, __nv_bfloat16* __restrict__ wx,
+                                                                  int Cin, int Cout, int L) {
+  __shared__ __align__(16) __nv_bfloat16 re[32 * SX_PITCH], im[32 * SX_PITCH];
+  const int c0 = blockIdx.x * 64, o = blockIdx.y, l0 = blockIdx.z * 32;
+  const int lp = (threadIdx.x & 15) * 2, cp = (threadIdx.x >> 4) * 2;     // two degrees, two channels (then + 32)
+  float4 v[2][2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int c = c0 + h * 32 + cp + k;
+      v[h][k] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (c < Cin && l0 + lp < L)
+        v[h][k] = __ldcs(reinterpret_cast<const float4*>(w + (static_cast<long long>(c) * Cout + o) * L + l0 + lp));
+    }
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int at = lp * SX_PITCH + h * 32 + cp;
+    *reinterpret_cast<__nv_bfloat162*>(re + at) = __floats2bfloat162_rn(v[h][0].x, v[h][1].x);
+    *reinterpret_cast<__nv_bfloat162*>(im + at) = __floats2bfloat162_rn(v[h][0].y, v[h][1].y);
+    *reinterpret_cast<__nv_bfloat162*>(re + at + SX_PITCH) = __floats2bfloat162_rn(v[h][0].z, v[h][1].z);
+    *reinterpret_cast<__nv_bfloat162*>(im + at + SX_PITCH) = __floats2bfloat162_rn(v[h][0].w, v[h][1].w);
+  }
+  __syncthreads();
+  const int cv = (threadIdx.x & 7) * 8, l = threadIdx.x >> 3;            // eight channels of one degree
+  if (l0 + l < L && c0 + cv < Cin) {
+    const uint4 r = *reinterpret_cast<const uint4*>(re + l * SX_PITCH + cv);
+    const uint4 i = *reinterpret_cast<const uint4*>(im + l * SX_PITCH + cv);
+    const uint4 n = make_uint4(i.x ^ 0x80008000u, i.y ^ 0x80008000u, i.z ^ 0x80008000u, i.w ^ 0x80008000u);
+    __nv_bfloat16* base = wx + static_cast<long long>(l0 + l) * 4 * Cout * Cin + c0 + cv;
+    const long long r0 = static_cast<long long>(o) * 2 * Cin, r1 = static_cast<long long>(Cout + o) * 2 * Cin;
+    *reinterpret_cast<uint4*>(base + r0) = r;
+    *reinterpret_cast<uint4*>(base + r0 + Cin) = n;
+    *reinterpret_cast<uint4*>(base + r1) = i;
+    *reinterpret_cast<uint4*>(base + r1 + Cin) = r;
+  }
+}
+
 // two_block == 0: dwx is the full real 2x2-block gradient [L, 2Cout, 2Cin];  two_block == 1: dwx is [2][L][Cout][Cin]
 // holding (dWr, dWi) already.  assign != 0 overwrites dw instead of accumulating into it.
 __global__ void spectral_fold_kernel(const float* __restrict__ dwx, float2* __restrict__ dw, int Cin, int Cout, int L,
@@ -933,6 +976,46 @@ __global__ void spectral_fold_kernel(const float* __restrict__ dwx, float2* __re
         *d = cur;
       }
     }
+  }
+}
+
+// dw = (dWr, dWi) with 16-byte accesses on both sides: [2][L][Cout][Cin] -> complex [Cin, Cout, L], even L, Cin a multiple
+// of 4; a 64-channel by 32-degree tile, 256-byte segments in both directions.  384 x 384 x 240: 142 -> 99 us, 5.7 TB/s.
+// grid: (ceil(Cin / 64), Cout, ceil(L / 32))
+__global__ void __launch_bounds__(256) spectral_fold_vec_kernel(const float* __restrict__ dwx, float2* __restrict__ dw, int Cin,
+                                                                int Cout, int L) {
+  __shared__ float sh[2][64][33];
+  const int c0 = blockIdx.x * 64, o = blockIdx.y, l0 = blockIdx.z * 32;
+  const int cv = (threadIdx.x & 15) * 4, lr = threadIdx.x >> 4;          // four channels of degrees lr, lr + 16
+  const long long plane = static_cast<long long>(L) * Cout * Cin;
+  float4 v[2][2];
+#pragma unroll
+  for (int p = 0; p < 2; ++p)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int l = l0 + lr + h * 16;
+      v[p][h] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (l < L && c0 + cv < Cin)
+        v[p][h] = __ldcs(reinterpret_cast<const float4*>(dwx + p * plane + (static_cast<long long>(l) * Cout + o) * Cin + c0 + cv));
+    }
+#pragma unroll
+  for (int p = 0; p < 2; ++p)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int l = lr + h * 16;
+      sh[p][cv][l] = v[p][h].x;
+      sh[p][cv + 1][l] = v[p][h].y;
+      sh[p][cv + 2][l] = v[p][h].z;
+      sh[p][cv + 3][l] = v[p][h].w;
+    }
+  __syncthreads();
+  const int lp = (threadIdx.x & 15) * 2, cr = threadIdx.x >> 4;          // two degrees of channels cr, cr + 16, ...
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int c = cr + k * 16;
+    if (c0 + c < Cin && l0 + lp < L)
+      *reinterpret_cast<float4*>(dw + (static_cast<long long>(c0 + c) * Cout + o) * L + l0 + lp) =
+          make_float4(sh[0][c][lp], sh[1][c][lp], sh[0][c][lp + 1], sh[1][c][lp + 1]);
   }
 }
 
@@ -1160,12 +1243,22 @@ cudaError_t adamw_step(const AdamEntry* table, const int* chunk_tensor, const lo
 }
 
 cudaError_t spectral_expand(const float* w, __nv_bfloat16* wx, int Cin, int Cout, int L, cudaStream_t s) {
+  if ((L & 1) == 0 && (Cin & 7) == 0 && aligned16(w) && aligned16(wx)) {
+    spectral_expand_vec_kernel<<<dim3((Cin + 63) / 64, Cout, (L + 31) / 32), 256, 0, s>>>(reinterpret_cast<const float2*>(w), wx,
+                                                                                          Cin, Cout, L);
+    return cudaGetLastError();
+  }
   dim3 grid((Cin + 31) / 32, Cout, (L + 31) / 32), block(32, 8);
   spectral_expand_kernel<<<grid, block, 0, s>>>(reinterpret_cast<const float2*>(w), wx, Cin, Cout, L);
   return cudaGetLastError();
 }
 
 cudaError_t spectral_fold(const float* dwx, float* dw, int Cin, int Cout, int L, cudaStream_t s, int two_block, int assign) {
+  if (two_block && assign && (L & 1) == 0 && (Cin & 3) == 0 && aligned16(dwx) && aligned16(dw)) {
+    spectral_fold_vec_kernel<<<dim3((Cin + 63) / 64, Cout, (L + 31) / 32), 256, 0, s>>>(dwx, reinterpret_cast<float2*>(dw), Cin,
+                                                                                        Cout, L);
+    return cudaGetLastError();
+  }
   dim3 grid((Cin + 31) / 32, Cout, (L + 31) / 32), block(32, 8);
   spectral_fold_kernel<<<grid, block, 0, s>>>(dwx, reinterpret_cast<float2*>(dw), Cin, Cout, L, two_block, assign);
   return cudaGetLastError();

@@ -94,3 +94,14 @@ def test_column_sums(rows, c):
     got, ref = row_sums(x, c).double(), x.double().sum(0)
     # fp32 summation: error within rows * 2^-24 of the sum of magnitudes, in practice its square root
     assert ((got - ref).abs() <= 2.0 ** -24 * 8 * max(rows, 4) ** 0.5 * x.double().abs().sum(0) / rows ** 0.5 + 1e-6).all()
+
+
+@pytest.mark.parametrize("ci,co,n", [(8, 3, 2), (64, 5, 32), (72, 16, 34), (136, 8, 64), (12, 4, 30), (16, 4, 33)])
+def test_spectral_weight_layouts(ci, co, n):
+    """Weight expansion and gradient folding: tile edges in channels and degrees, and the sizes that keep the scalar kernels."""
+    from makani_b200.ops.spectral import expand_weight, fold_weight_grad2
+    dev = _dev()
+    w = torch.randn(ci, co, n, dtype=torch.complex64, device=dev)
+    assert torch.equal(expand_weight(w).cpu(), expand_weight(w.cpu()))
+    dw = torch.randn(2, n, co, ci, device=dev)
+    assert torch.equal(fold_weight_grad2(dw).cpu(), fold_weight_grad2(dw.cpu()))
