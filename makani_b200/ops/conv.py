@@ -160,11 +160,11 @@ def _canon(t):
 
 class _Conv1x1(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, w, bias, resid, act, out_layout):
+    def forward(ctx, x, w, bias, resid, act, out_layout, train):
         wq = prep_weight(w)
         ci = w.shape[1]
         bias_f = bias.detach().float().contiguous() if bias is not None else None
-        y, pre = _conv_fwd(x, wq, ci, bias_f, act, resid, want_preact=(act == ACT_GELU), out_layout=out_layout)
+        y, pre = _conv_fwd(x, wq, ci, bias_f, act, resid, want_preact=(train and act == ACT_GELU), out_layout=out_layout)
         ctx.save_for_backward(x, wq, pre)
         ctx.ci = ci
         ctx.act = act
@@ -186,7 +186,7 @@ class _Conv1x1(torch.autograd.Function):
         dx = _conv_dgrad(g, wq, ctx.ci, x_layout=layout_of(x)) if ctx.needs_input_grad[0] else None
         dw = _conv_wgrad(g, x).reshape(ctx.wshape) if ctx.needs_input_grad[1] else None
         db = _chan_sum(g) if ctx.has_bias and ctx.needs_input_grad[2] else None
-        return dx, dw, db, dres, None, None
+        return dx, dw, db, dres, None, None, None
 
 
 class _MLP2(torch.autograd.Function):
@@ -194,14 +194,15 @@ class _MLP2(torch.autograd.Function):
     The hidden activation is always channels-last."""
 
     @staticmethod
-    def forward(ctx, x, w1, b1, w2, b2, resid, out_layout):
+    def forward(ctx, x, w1, b1, w2, b2, resid, out_layout, train):
         w1q, w2q = prep_weight(w1), prep_weight(w2)
         ci, ch = w1.shape[1], w1.shape[0]
         b1f = b1.detach().float().contiguous() if b1 is not None else None
         b2f = b2.detach().float().contiguous() if b2 is not None else None
         hid_layout = CL if ch % 8 == 0 else NCHW
         # the first GEMM's second output is GELU'(pre-activation): the backward epilogue then only multiplies
-        h, dact = _conv_fwd(x, w1q, ci, b1f, ACT_GELU, None, want_preact=True, out_layout=hid_layout, deriv=True)
+        # (without a backward pass to come it is not computed, nor written)
+        h, dact = _conv_fwd(x, w1q, ci, b1f, ACT_GELU, None, want_preact=train, out_layout=hid_layout, deriv=train)
         y, _ = _conv_fwd(h, w2q, ch, b2f, ACT_NONE, resid, want_preact=False, out_layout=out_layout)
         ctx.save_for_backward(x, w1q, w2q, dact, h)
         ctx.dims = (ci, ch)
@@ -221,7 +222,12 @@ class _MLP2(torch.autograd.Function):
         dx = _conv_dgrad(dpre, w1q, ci, x_layout=layout_of(x)) if ctx.needs_input_grad[0] else None
         dw1 = _conv_wgrad(dpre, x).reshape(ctx.wshapes[0])
         db1 = _chan_sum(dpre) if has_b1 else None
-        return dx, dw1, db1, dw2, db2, (dy if has_res else None), None
+        return dx, dw1, db1, dw2, db2, (dy if has_res else None), None, None
+
+
+def records_grad(*tensors) -> bool:
+    """True when autograd will record an operation on these tensors (`ctx.needs_input_grad` does not know of no_grad)."""
+    return torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in tensors)
 
 
 def _native(x, resid):
@@ -232,7 +238,8 @@ def conv1x1(x, w, bias=None, resid=None, act: str = "none", out_layout: Optional
     """1x1 convolution on a 4-D activation. CUDA bf16 -> tcgen05 GEMM; anything else -> reference torch ops."""
     if _native(x, resid):
         _ext.require()
-        return _Conv1x1.apply(x, w, bias, resid, ACT_GELU if act == "gelu" else ACT_NONE, out_layout)
+        return _Conv1x1.apply(x, w, bias, resid, ACT_GELU if act == "gelu" else ACT_NONE, out_layout,
+                              records_grad(x, w, bias, resid))
     w4 = w.reshape(w.shape[0], -1, 1, 1).to(x.dtype)
     y = torch.nn.functional.conv2d(x, w4, None if bias is None else bias.to(x.dtype))
     if act == "gelu":
@@ -246,7 +253,7 @@ def mlp2(x, w1, b1, w2, b2, resid=None, out_layout: Optional[str] = None):
     """Two-layer pointwise MLP with GELU (encoder, decoder and block MLP of the SFNO/AFNO networks)."""
     if _native(x, resid):
         _ext.require()
-        return _MLP2.apply(x, w1, b1, w2, b2, resid, out_layout)
+        return _MLP2.apply(x, w1, b1, w2, b2, resid, out_layout, records_grad(x, w1, b1, w2, b2, resid))
     f = torch.nn.functional
     h = f.gelu(f.conv2d(x, w1.reshape(w1.shape[0], -1, 1, 1).to(x.dtype), None if b1 is None else b1.to(x.dtype)),
                approximate=_ext.gelu_approximation())

@@ -9,6 +9,7 @@ from __future__ import annotations
 import torch
 
 from . import _ext
+from .conv import records_grad
 from .gemm import ACT_GELU, ACT_MULAUX, ACT_NONE, BIAS_COL, Operand, Output, gemm
 from .norm import row_sums
 
@@ -52,13 +53,14 @@ def _lin_wgrad(dy, x2):
 
 class _MLP2Last(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, w1, b1, w2, b2):
+    def forward(ctx, x, w1, b1, w2, b2, train):
         shp = x.shape
         x2 = x.reshape(-1, shp[-1])
         w1q, w2q = _wq(w1), _wq(w2)
         b1f = b1.detach().float().contiguous() if b1 is not None else None
         b2f = b2.detach().float().contiguous() if b2 is not None else None
-        h, dact = _lin_fwd(x2, w1q, b1f, ACT_GELU, True, deriv=True)     # second output: GELU'(pre-activation)
+        # second output: GELU'(pre-activation), where a backward pass will want it
+        h, dact = _lin_fwd(x2, w1q, b1f, ACT_GELU, train, deriv=train)
         y, _ = _lin_fwd(h, w2q, b2f, ACT_NONE, False)
         ctx.save_for_backward(x2, w1q, w2q, dact, h)
         ctx.flags = (b1 is not None, b2 is not None)
@@ -75,7 +77,7 @@ class _MLP2Last(torch.autograd.Function):
         dx = _lin_dgrad(dpre, w1q).reshape(ctx.shp) if ctx.needs_input_grad[0] else None
         dw1 = _lin_wgrad(dpre, x2)
         db1 = row_sums(dpre, dpre.shape[1]) if ctx.flags[0] else None
-        return dx, dw1, db1, dw2, db2
+        return dx, dw1, db1, dw2, db2, None
 
 
 class _LinearLast(torch.autograd.Function):
@@ -112,4 +114,4 @@ def linear_lastdim(x, w, b=None):
 
 def mlp2_lastdim(x, w1, b1, w2, b2):
     _ext.require()
-    return _MLP2Last.apply(x, w1, b1, w2, b2)
+    return _MLP2Last.apply(x, w1, b1, w2, b2, records_grad(x, w1, b1, w2, b2))

@@ -105,3 +105,20 @@ def test_spectral_weight_layouts(ci, co, n):
     assert torch.equal(expand_weight(w).cpu(), expand_weight(w.cpu()))
     dw = torch.randn(2, n, co, ci, device=dev)
     assert torch.equal(fold_weight_grad2(dw).cpu(), fold_weight_grad2(dw.cpu()))
+
+
+def test_mlp_without_gradients_equals_training_forward():
+    """The forward pass that writes no GELU' gives the same values, in both layouts of the tokens."""
+    from makani_b200.models.common.layers import MLP
+    from makani_b200.models.networks.afnonet import Mlp
+    dev = _dev()
+    torch.manual_seed(3)
+    m, x = MLP(16, hidden_features=40).to(dev), torch.randn(2, 16, 24, 40, device=dev).to(torch.bfloat16)
+    x = x.contiguous(memory_format=torch.channels_last)
+    t, z = Mlp(24, hidden_features=96).to(dev), torch.randn(3, 50, 24, device=dev).to(torch.bfloat16)
+    for net, inp in ((m, x), (t, z)):
+        y = net(inp)
+        assert y.requires_grad
+        with torch.no_grad():
+            assert torch.equal(net(inp), y)
+    _ext.check_device_errors(dev)
