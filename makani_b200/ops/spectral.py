@@ -25,10 +25,12 @@ from typing import Dict, Optional, Tuple
 
 import numpy as np
 import torch
+from torch.utils.weak import WeakTensorKeyDictionary
 
 from ..sht.legendre import legendre_table
 from ..sht.quadrature import precompute_latitudes
 from . import _ext
+from .conv import records_grad
 from .gemm import Operand, Output, Tri, gemm, pad_to
 
 
@@ -203,11 +205,11 @@ def fold_weight_grad2(dw2: torch.Tensor) -> torch.Tensor:
 # ------------------------------------------------------------------------------------------------ weights
 
 
-# Inference re-uses the expanded weights: they are cached per parameter while gradients are disabled and dropped when
-# the parameter is modified in place (`_version`) or by the fused optimiser, which writes through raw pointers and
-# announces every update through `note_weights_changed`.
+# Inference re-uses the expanded weights: they are kept as long as the parameter lives (a weak key, so that a new
+# parameter in recycled memory never meets them), and dropped when the parameter is modified in place (`_version`) or by
+# the fused optimiser, which writes through raw pointers and announces every update through `note_weights_changed`.
 _WEIGHT_EPOCH = 0
-_EXPANDED = {}
+_EXPANDED = WeakTensorKeyDictionary()
 
 
 def note_weights_changed() -> None:
@@ -216,17 +218,19 @@ def note_weights_changed() -> None:
     _EXPANDED.clear()
 
 
-def expand_weight(w: torch.Tensor, dtype=torch.bfloat16) -> torch.Tensor:
-    """complex [Ci, Co, L] -> real [L, 2Co, 2Ci] with rows (ri', o), columns (ri, c):  [[Wr, -Wi], [Wi, Wr]]."""
-    if not torch.is_grad_enabled() and w.is_cuda:
-        key = (w.data_ptr(), tuple(w.shape), dtype)
-        hit = _EXPANDED.get(key)
-        if hit is not None and hit[0] == (w._version, _WEIGHT_EPOCH):
-            return hit[1]
-        wx = _expand_weight(w, dtype)
-        _EXPANDED[key] = ((w._version, _WEIGHT_EPOCH), wx)
-        return wx
-    return _expand_weight(w, dtype)
+def expand_weight(w: torch.Tensor, dtype=torch.bfloat16, keep: bool = False) -> torch.Tensor:
+    """complex [Ci, Co, L] -> real [L, 2Co, 2Ci] with rows (ri', o), columns (ri, c):  [[Wr, -Wi], [Wi, Wr]].
+
+    `keep`: the caller does not record gradients, the result is kept with the parameter for its next call."""
+    if not keep or not w.is_cuda or w.is_inference():
+        return _expand_weight(w, dtype)
+    state = (w._version, _WEIGHT_EPOCH, w.data_ptr(), dtype)
+    hit = _EXPANDED.get(w)
+    if hit is not None and hit[0] == state:
+        return hit[1]
+    wx = _expand_weight(w, dtype)
+    _EXPANDED[w] = (state, wx)
+    return wx
 
 
 def _expand_weight(w: torch.Tensor, dtype=torch.bfloat16) -> torch.Tensor:
@@ -263,9 +267,9 @@ class _SpectralConv(torch.autograd.Function):
     Input and outputs are channels-last."""
 
     @staticmethod
-    def forward(ctx, x, w, plan_in: SHTPlan, plan_out: SHTPlan, want_resid: bool):
+    def forward(ctx, x, w, plan_in: SHTPlan, plan_out: SHTPlan, want_resid: bool, train: bool):
         x = _to_cl(x)
-        wx = expand_weight(w, x.dtype)
+        wx = expand_weight(w, x.dtype, keep=not train)
         t1 = dft_analysis(x, plan_in.f, False, plan_in.nlon, plan_in.k2)
         t2 = legendre_analysis(t1, plan_in.pw)
         del t1
@@ -309,7 +313,7 @@ class _SpectralConv(torch.autograd.Function):
                 del dr4, dr2
             dt1 = legendre_synthesis(dt2.contiguous(), False, plan_in.pw, plan_in.nlat)
             dx = dft_synthesis(dt1, plan_in.f, True, plan_in.nlon, plan_in.nlon)
-        return dx, dw, None, None, None
+        return dx, dw, None, None, None, None
 
 
 def spectral_conv_supported(x: torch.Tensor, w: torch.Tensor) -> bool:
@@ -319,4 +323,4 @@ def spectral_conv_supported(x: torch.Tensor, w: torch.Tensor) -> bool:
 
 def spectral_conv_dhconv(x, w, plan_in: SHTPlan, plan_out: SHTPlan, want_resid: bool):
     """Fused spherical convolution with per-degree ("dhconv") complex weights on the GEMM engine."""
-    return _SpectralConv.apply(x, w, plan_in, plan_out, want_resid)
+    return _SpectralConv.apply(x, w, plan_in, plan_out, want_resid, records_grad(x, w))

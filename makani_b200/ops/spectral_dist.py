@@ -38,6 +38,7 @@ from ..sht.legendre import legendre_table
 from ..sht.quadrature import precompute_latitudes
 from . import _ext
 from .gemm import Operand, Output, Segment, Tri, gemm, pad_to
+from .conv import records_grad
 from .spectral import _to_cl, contract_wgrad2, expand_weight, fold_weight_grad2
 
 SEG_ALIGN = 64   # elements: one 128-byte k-slab of bf16
@@ -331,10 +332,10 @@ class _DistSpectralConv(torch.autograd.Function):
     """y = iSHT_out(W . SHT_in(x)) on sharded grids, and the regridded residual when asked for."""
 
     @staticmethod
-    def forward(ctx, x, w, plan_in: DistSHTPlan, plan_out: DistSHTPlan, want_resid: bool):
+    def forward(ctx, x, w, plan_in: DistSHTPlan, plan_out: DistSHTPlan, want_resid: bool, train: bool):
         x = _to_cl(x)
         B, C = x.shape[0], x.shape[1]
-        wx = expand_weight(w, x.dtype)
+        wx = expand_weight(w, x.dtype, keep=not train)
         Co = wx.shape[1] // 2
         t2 = dist_sht_analysis(x, plan_in)
         s3, t3, ls = stage_contract(t2, wx, False, plan_in)
@@ -378,7 +379,7 @@ class _DistSpectralConv(torch.autograd.Function):
             else:
                 slot, t3v, ls = stage_contract(dt3, wx, True, plan_in)
             dx = dist_sht_synthesis(slot, t3v, ls, False, plan_in, B, C, plan_in.pw_syn, plan_in.ft_syn)
-        return dx, dw, None, None, None
+        return dx, dw, None, None, None, None
 
 
 def dist_spectral_conv_supported(x: torch.Tensor, w: torch.Tensor) -> bool:
@@ -386,4 +387,4 @@ def dist_spectral_conv_supported(x: torch.Tensor, w: torch.Tensor) -> bool:
 
 
 def dist_spectral_conv_dhconv(x, w, plan_in: DistSHTPlan, plan_out: DistSHTPlan, want_resid: bool):
-    return _DistSpectralConv.apply(x, w, plan_in, plan_out, want_resid)
+    return _DistSpectralConv.apply(x, w, plan_in, plan_out, want_resid, records_grad(x, w))

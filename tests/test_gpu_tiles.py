@@ -122,3 +122,20 @@ def test_mlp_without_gradients_equals_training_forward():
         with torch.no_grad():
             assert torch.equal(net(inp), y)
     _ext.check_device_errors(dev)
+
+
+def test_kept_weights_follow_the_parameter():
+    """Expanded weights kept for inference belong to one parameter: not to the next one in the same memory, nor to it once
+    it has changed."""
+    from makani_b200.ops.spectral import expand_weight
+    dev = _dev()
+    seen = set()
+    for k in range(4):
+        w = torch.full((8, 8, 16), complex(k, -k), dtype=torch.complex64, device=dev)
+        seen.add(w.data_ptr())
+        for _ in range(2):
+            assert torch.equal(expand_weight(w, keep=True).cpu(), expand_weight(w.cpu()))
+        w.mul_(2.0)
+        assert torch.equal(expand_weight(w, keep=True).cpu(), expand_weight(w.cpu()))
+        del w
+    assert len(seen) < 4      # the allocator did hand out the same memory again
