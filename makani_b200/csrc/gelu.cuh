@@ -120,33 +120,43 @@ __device__ __forceinline__ f32x2 f2_tanh(f32x2 u) {
   f2_unpack(u, a, b);
   return f2_pack(gelu_tanh_approx(a), gelu_tanh_approx(b));
 }
-__device__ __forceinline__ f32x2 gelu_fwd2(f32x2 x, const GeluCoef& c) {
+// The coefficients as register pairs.  The packed instructions take neither immediates nor constant-bank operands; made by
+// volatile moves once per thread, the pairs stay in registers instead of being rebuilt at every use.
+struct GeluPairs {
+  f32x2 c0, c1, c2, n0, n1, n2, half, neg1;
+};
+__device__ __forceinline__ f32x2 f2_keep(float a) {
+  f32x2 r;
+  asm volatile("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(a));
+  return r;
+}
+__device__ __forceinline__ GeluPairs gelu_pairs(const GeluCoef& c) {
+  return GeluPairs{f2_keep(c.c0), f2_keep(c.c1), f2_keep(c.c2), f2_keep(-c.c0), f2_keep(-3.f * c.c1), f2_keep(-5.f * c.c2),
+                   f2_keep(0.5f), f2_keep(-1.f)};
+}
+__device__ __forceinline__ f32x2 gelu_fwd2(f32x2 x, const GeluPairs& c) {
   const f32x2 u = f2_clamp36(f2_mul(x, x));
-  const f32x2 q = f2_fma(u, f2_fma(u, f2_pack(c.c2, c.c2), f2_pack(c.c1, c.c1)), f2_pack(c.c0, c.c0));
-  const f32x2 hx = f2_mul(x, f2_pack(0.5f, 0.5f));
+  const f32x2 q = f2_fma(u, f2_fma(u, c.c2, c.c1), c.c0);
+  const f32x2 hx = f2_mul(x, c.half);
   return f2_fma(hx, f2_tanh(f2_mul(x, q)), hx);
 }
-__device__ __forceinline__ f32x2 gelu_bwd2(f32x2 x, const GeluCoef& c) {
+__device__ __forceinline__ f32x2 gelu_bwd2(f32x2 x, const GeluPairs& c) {
   const f32x2 u = f2_clamp36(f2_mul(x, x));
-  const f32x2 q = f2_fma(u, f2_fma(u, f2_pack(c.c2, c.c2), f2_pack(c.c1, c.c1)), f2_pack(c.c0, c.c0));
-  const float n2 = -5.f * c.c2, n1 = -3.f * c.c1, n0 = -c.c0;
-  const f32x2 ndq = f2_fma(u, f2_fma(u, f2_pack(n2, n2), f2_pack(n1, n1)), f2_pack(n0, n0));
+  const f32x2 q = f2_fma(u, f2_fma(u, c.c2, c.c1), c.c0);
+  const f32x2 ndq = f2_fma(u, f2_fma(u, c.n2, c.n1), c.n0);
   const f32x2 t = f2_tanh(f2_mul(x, q));
-  const f32x2 half = f2_pack(0.5f, 0.5f);
-  const f32x2 s = f2_fma(t, t, f2_pack(-1.f, -1.f));
-  return f2_fma(f2_mul(f2_mul(x, half), s), ndq, f2_fma(t, half, half));
+  const f32x2 s = f2_fma(t, t, c.neg1);
+  return f2_fma(f2_mul(f2_mul(x, c.half), s), ndq, f2_fma(t, c.half, c.half));
 }
-__device__ __forceinline__ void gelu_fwd_bwd2(f32x2 x, const GeluCoef& c, f32x2& y, f32x2& dy) {
+__device__ __forceinline__ void gelu_fwd_bwd2(f32x2 x, const GeluPairs& c, f32x2& y, f32x2& dy) {
   const f32x2 u = f2_clamp36(f2_mul(x, x));
-  const f32x2 q = f2_fma(u, f2_fma(u, f2_pack(c.c2, c.c2), f2_pack(c.c1, c.c1)), f2_pack(c.c0, c.c0));
-  const float n2 = -5.f * c.c2, n1 = -3.f * c.c1, n0 = -c.c0;
-  const f32x2 ndq = f2_fma(u, f2_fma(u, f2_pack(n2, n2), f2_pack(n1, n1)), f2_pack(n0, n0));
+  const f32x2 q = f2_fma(u, f2_fma(u, c.c2, c.c1), c.c0);
+  const f32x2 ndq = f2_fma(u, f2_fma(u, c.n2, c.n1), c.n0);
   const f32x2 t = f2_tanh(f2_mul(x, q));
-  const f32x2 half = f2_pack(0.5f, 0.5f);
-  const f32x2 hx = f2_mul(x, half);
-  const f32x2 s = f2_fma(t, t, f2_pack(-1.f, -1.f));
+  const f32x2 hx = f2_mul(x, c.half);
+  const f32x2 s = f2_fma(t, t, c.neg1);
   y = f2_fma(hx, t, hx);
-  dy = f2_fma(f2_mul(hx, s), ndq, f2_fma(t, half, half));
+  dy = f2_fma(f2_mul(hx, s), ndq, f2_fma(t, c.half, c.half));
 }
 
 #endif  // __CUDACC__

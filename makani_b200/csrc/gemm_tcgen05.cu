@@ -196,7 +196,9 @@ __device__ __forceinline__ uint32_t mapa_u32(uint32_t addr, uint32_t rank) {
   return r;
 }
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+  // (no data passes through memory here, only the right to overwrite TMEM: a cluster-scope release would wait for the
+  // staged stores of the whole warp)
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
@@ -657,6 +659,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
     bool ok = peers_ready;
     // the "accumulator drained" barrier of a pair lives in the leader and counts the warps of both CTAs
     const uint32_t leader_tempty0 = (CG == 2) ? mapa_u32(tempty_bar(0), 0) : 0u;
+    const f32x2 alpha2 = f2_keep(p.alpha);
+    GeluPairs gelu2;
+    if constexpr (EPI == 1 || EPI == 2) gelu2 = gelu_pairs(p.gelu);
     for (uint32_t t = tile0; t < p.total_tiles; t += tile_step) {
       const TileCoord c = decode_tile<BK, CG>(p, t, crank);
       if (c.skip && p.accumulate) continue;
@@ -705,7 +710,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
             tma_store_wait_read<0>();
             __syncwarp();
           }
-          const f32x2 alpha2 = f2_pack(p.alpha, p.alpha);
           const f32x2 rbias2 = f2_pack(rbias, rbias);
           // The 64 columns of a box go through a ROLLED loop of four 16-column steps.  Unrolled, the body of one box ran
           // to tens of KB of straight-line code per epilogue flavour, the epilogue warps (each at another place
@@ -746,7 +750,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
               if constexpr (EPI == 1) {
                 if (p.act == 1) {
 #pragma unroll
-                  for (int j = 0; j < 4; ++j) f[j] = gelu_fwd2(f[j], p.gelu);
+                  for (int j = 0; j < 4; ++j) f[j] = gelu_fwd2(f[j], gelu2);
                 } else if (p.act != 0) {      // ReLU / soft shrinkage (uniform over the launch)
 #pragma unroll
                   for (int j = 0; j < 4; ++j) {
@@ -760,12 +764,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
                 f32x2 s2[4];
                 if (p.save_deriv) {      // uniform over the launch: second output = GELU'(pre-activation)
 #pragma unroll
-                  for (int j = 0; j < 4; ++j) gelu_fwd_bwd2(f[j], p.gelu, f[j], s2[j]);
+                  for (int j = 0; j < 4; ++j) gelu_fwd_bwd2(f[j], gelu2, f[j], s2[j]);
                 } else {
 #pragma unroll
                   for (int j = 0; j < 4; ++j) {
                     s2[j] = f[j];
-                    f[j] = gelu_fwd2(f[j], p.gelu);
+                    f[j] = gelu_fwd2(f[j], gelu2);
                   }
                 }
                 *reinterpret_cast<uint4*>(box_p + sw) = f2_bf16x8(s2);

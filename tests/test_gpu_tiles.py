@@ -139,3 +139,23 @@ def test_kept_weights_follow_the_parameter():
         assert torch.equal(expand_weight(w, keep=True).cpu(), expand_weight(w.cpu()))
         del w
     assert len(seen) < 4      # the allocator did hand out the same memory again
+
+
+@pytest.mark.parametrize("act", ["none", "gelu"])
+@pytest.mark.parametrize("b,c,h,w", [(1, 8, 1, 8), (2, 16, 32, 64), (1, 24, 9, 16), (1, 32, 40, 80), (1, 264, 50, 96), (1, 1024, 20, 40)])
+def test_instance_norm_channel_counts(b, c, h, w, act):
+    """Channel counts below and above a warp of 16-byte vectors (powers of two and not), fewer tokens than rows in flight."""
+    from makani_b200.ops.norm import instance_norm
+    dev = _dev()
+    g = torch.Generator(dev).manual_seed(c)
+    x = (torch.randn(b, h, w, c, device=dev, generator=g) * 1.5 + 0.7).to(torch.bfloat16).permute(0, 3, 1, 2).requires_grad_()
+    dy = torch.randn(b, h, w, c, device=dev, generator=g).to(torch.bfloat16).permute(0, 3, 1, 2)
+    wt, bs = (torch.rand(c, device=dev, generator=g) + 0.5).requires_grad_(), torch.randn(c, device=dev, generator=g).requires_grad_()
+    y = instance_norm(x, wt, bs, 1e-6, act)
+    got = [y] + list(torch.autograd.grad(y, [x, wt, bs], dy))
+    xd, wd, bd = x.detach().double().requires_grad_(), wt.detach().double().requires_grad_(), bs.detach().double().requires_grad_()
+    yr = torch.nn.functional.instance_norm(xd, None, None, wd, bd, True, 0.0, 1e-6)
+    yr = torch.nn.functional.gelu(yr) if act == "gelu" else yr
+    ref = [yr] + list(torch.autograd.grad(yr, [xd, wd, bd], dy.double()))
+    for a, r in zip(got, ref):
+        assert _rel(a, r) < BF16
