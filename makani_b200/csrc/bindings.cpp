@@ -288,6 +288,72 @@ void colsum(const Tensor& x, Tensor& out) {
              "colsum");
 }
 
+// sums of do2 [outer, groups, inner, C] over outer and inner -> out [groups, C]
+void colsum_groups(const Tensor& x, Tensor& out, int64_t outer, int64_t groups, int64_t inner) {
+  MK_CHECK(x.is_cuda() && x.scalar_type() == torch::kBFloat16 && x.is_contiguous(), "colsum_groups: contiguous bf16 CUDA tensor expected");
+  MK_CHECK(outer > 0 && groups > 0 && inner > 0 && x.numel() % (outer * groups * inner) == 0, "colsum_groups: bad extents");
+  const int64_t C = x.numel() / (outer * groups * inner);
+  MK_CHECK(out.is_cuda() && out.scalar_type() == torch::kFloat32 && out.is_contiguous() && out.numel() == groups * C, "colsum_groups: bad output");
+  c10::cuda::CUDAGuard guard(x.device());
+  check_cuda(mk::colsum(reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()), out.data_ptr<float>(), outer * inner,
+                        static_cast<int>(C), cur_stream(), static_cast<int>(groups), inner * C, static_cast<int>(inner),
+                        groups * inner * C),
+             "colsum_groups");
+}
+
+static void check_f32(const Tensor& t, int64_t n, const char* what) {
+  MK_CHECK(t.is_cuda() && t.scalar_type() == torch::kFloat32 && t.is_contiguous() && t.numel() == n, what);
+}
+
+// block weights of both AFNO layers (w [2, nb, in, out], b [2, nb, out] or none) -> wx [nb, 2 out, 2 in] bf16, bx [nb, 2 out]
+void afno_pack(const std::vector<Tensor>& w, const std::vector<c10::optional<Tensor>>& b, std::vector<Tensor> wx,
+               std::vector<Tensor> bx) {
+  MK_CHECK(w.size() == 2 && b.size() == 2 && wx.size() == 2 && bx.size() == 2 && w[0].dim() == 4 && w[1].dim() == 4,
+           "afno_pack: two layers expected");
+  const int64_t nb = w[0].size(1);
+  MK_CHECK(w[1].size(1) == nb && nb <= 32767, "afno_pack: block counts differ");
+  c10::cuda::CUDAGuard guard(w[0].device());
+  mk::AfnoLayer l[2];
+  for (int k = 0; k < 2; ++k) {
+    const int64_t ni = w[k].size(2), no = w[k].size(3);
+    check_f32(w[k], 2 * nb * ni * no, "afno_pack: weights must be contiguous fp32 [2, nb, in, out]");
+    MK_CHECK(wx[k].is_cuda() && wx[k].scalar_type() == torch::kBFloat16 && wx[k].is_contiguous() && wx[k].numel() == 4 * nb * ni * no,
+             "afno_pack: bad output");
+    const bool has = b[k].has_value() && b[k]->defined();
+    if (has) {
+      check_f32(*b[k], 2 * nb * no, "afno_pack: biases must be contiguous fp32 [2, nb, out]");
+      check_f32(bx[k], 2 * nb * no, "afno_pack: bad bias output");
+    }
+    l[k] = {w[k].data_ptr<float>(), has ? b[k]->data_ptr<float>() : nullptr, reinterpret_cast<__nv_bfloat16*>(wx[k].data_ptr()),
+            has ? bx[k].data_ptr<float>() : nullptr, static_cast<int>(ni), static_cast<int>(no)};
+  }
+  check_cuda(mk::afno_pack(l[0], l[1], static_cast<int>(nb), cur_stream()), "afno_pack");
+}
+
+// gradients of the packed weights and biases -> those of the parameters (dw [2, nb, in, out], db [2, nb, out] or none)
+void afno_fold(const std::vector<Tensor>& dwx, const std::vector<Tensor>& dbx, std::vector<Tensor> dw,
+               const std::vector<c10::optional<Tensor>>& db) {
+  MK_CHECK(dwx.size() == 2 && dbx.size() == 2 && dw.size() == 2 && db.size() == 2 && dw[0].dim() == 4 && dw[1].dim() == 4,
+           "afno_fold: two layers expected");
+  const int64_t nb = dw[0].size(1);
+  MK_CHECK(dw[1].size(1) == nb && nb <= 32767, "afno_fold: block counts differ");
+  c10::cuda::CUDAGuard guard(dw[0].device());
+  mk::AfnoGrad l[2];
+  for (int k = 0; k < 2; ++k) {
+    const int64_t ni = dw[k].size(2), no = dw[k].size(3);
+    check_f32(dw[k], 2 * nb * ni * no, "afno_fold: bad output");
+    check_f32(dwx[k], 4 * nb * ni * no, "afno_fold: bad input");
+    const bool has = db[k].has_value() && db[k]->defined();
+    if (has) {
+      check_f32(*db[k], 2 * nb * no, "afno_fold: bad bias output");
+      check_f32(dbx[k], 2 * nb * no, "afno_fold: bad bias input");
+    }
+    l[k] = {dwx[k].data_ptr<float>(), has ? dbx[k].data_ptr<float>() : nullptr, dw[k].data_ptr<float>(),
+            has ? db[k]->data_ptr<float>() : nullptr, static_cast<int>(ni), static_cast<int>(no)};
+  }
+  check_cuda(mk::afno_fold(l[0], l[1], static_cast<int>(nb), cur_stream()), "afno_fold");
+}
+
 void inorm_bwd(const Tensor& x, const Tensor& dy, c10::optional<Tensor> dx, const c10::optional<Tensor>& w,
                const c10::optional<Tensor>& b, const Tensor& stats, c10::optional<Tensor> dw, c10::optional<Tensor> db,
                c10::optional<Tensor> sums_io, int64_t C, double count, int64_t act, int64_t ext_sums) {
@@ -558,6 +624,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("inorm_fwd", &inorm_fwd);
   m.def("inorm_partial_stats", &inorm_partial_stats);
   m.def("colsum", &colsum);
+  m.def("colsum_groups", &colsum_groups);
+  m.def("afno_pack", &afno_pack);
+  m.def("afno_fold", &afno_fold);
   m.def("inorm_bwd", &inorm_bwd);
   m.def("inorm_cl_sums", &inorm_cl_sums, py::arg("x"), py::arg("dy"), py::arg("w"), py::arg("b"), py::arg("stats"), py::arg("sums"),
         py::arg("dw"), py::arg("db"), py::arg("B"), py::arg("C"), py::arg("act"), py::arg("mode"),

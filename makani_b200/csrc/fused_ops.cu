@@ -598,13 +598,15 @@ __global__ void __launch_bounds__(CL_THREADS, MODE == 0 ? 2 : 1) inorm_cl_apply_
 
 // ------------------------------------------------------------------------------------------ column sums
 
-// out[c] += sum_r x[r, c] for x [rows, C] bf16 (C a multiple of 8): the bias gradients.  One read of x; thread (v, r) owns
-// eight columns and every R-th row of its slab with eight 16-byte loads in flight, so the HBM latency is covered at two
-// CTAs per SM.  16200 tokens: 3072 columns 27 us, 768 columns 10 us, where a cast to fp32 and a torch sum took 185 and
+// out[g, c] += sum_r x_g[r, c] for bf16 rows of C columns (a multiple of 8): the bias gradients.  Row r of group g sits at
+// g * gstride + (r / inner) * ostride + (r % inner) * C elements (plain rows: inner = rows).  One read of x; thread (v, r)
+// owns eight columns and every R-th row of its slab with eight 16-byte loads in flight, so the HBM latency is covered at
+// two CTAs per SM.  16200 tokens: 3072 columns 27 us, 768 columns 10 us, where a cast to fp32 and a torch sum took 185 and
 // 63 us; 2048 x 16: 4 us, where the statistics kernel of the instance norm took 37 us.
 constexpr int CS_THREADS = 256;
 __global__ void __launch_bounds__(CS_THREADS) colsum_kernel(const uint4* __restrict__ x, float* __restrict__ out, long long rows,
-                                                            int V, int vb, int slab) {
+                                                            int V, int vb, int slab, int inner, long long ostride_v,
+                                                            long long gstride_v) {
   __shared__ __align__(16) float sh[CS_THREADS * 8];
   const int v0 = blockIdx.x * vb;
   const int nv = min(vb, V - v0);          // 16-byte columns of this CTA
@@ -618,7 +620,13 @@ __global__ void __launch_bounds__(CS_THREADS) colsum_kernel(const uint4* __restr
     for (int j = 0; j < 8; ++j) a[j] = 0.f;
     const long long t0 = static_cast<long long>(blockIdx.y) * slab;
     const long long t1 = min(t0 + slab, rows);
-    const uint4* xv = x + v0 + v;
+    const uint4* xv = x + blockIdx.z * gstride_v + v0 + v;
+    const bool plain = inner == 0;
+    auto row = [&](long long t) -> const uint4* {
+      if (plain) return xv + t * V;
+      const unsigned hi = static_cast<unsigned>(t) / static_cast<unsigned>(inner);
+      return xv + hi * ostride_v + (t - static_cast<long long>(hi) * inner) * V;
+    };
     auto add = [&](const uint4& q) {
       float f[8];
       unpack8(q, f);
@@ -629,11 +637,11 @@ __global__ void __launch_bounds__(CS_THREADS) colsum_kernel(const uint4* __restr
     for (; t + 7LL * R < t1; t += 8LL * R) {
       uint4 q[8];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) q[u] = __ldg(xv + (t + u * R) * V);
+      for (int u = 0; u < 8; ++u) q[u] = __ldg(row(t + u * R));
 #pragma unroll
       for (int u = 0; u < 8; ++u) add(q[u]);
     }
-    for (; t < t1; t += R) add(__ldg(xv + t * V));
+    for (; t < t1; t += R) add(__ldg(row(t)));
     const bool fold = vb < 32 && (vb & (vb - 1)) == 0;      // lanes with the same columns: shuffles before the atomics
     if (fold) {
       for (int o = 16; o >= vb; o >>= 1) {
@@ -648,7 +656,8 @@ __global__ void __launch_bounds__(CS_THREADS) colsum_kernel(const uint4* __restr
   }
   __syncthreads();
   for (int i = threadIdx.x * 4; i < nv * 8; i += CS_THREADS * 4)
-    atomicAdd(reinterpret_cast<float4*>(out + static_cast<long long>(v0) * 8 + i), *reinterpret_cast<const float4*>(sh + i));
+    atomicAdd(reinterpret_cast<float4*>(out + (static_cast<long long>(blockIdx.z) * V + v0) * 8 + i),
+              *reinterpret_cast<const float4*>(sh + i));
 }
 
 // ------------------------------------------------------------------------------------------ Lp norms
@@ -902,6 +911,81 @@ __global__ void __launch_bounds__(256) adamw_kernel(const AdamEntry* __restrict_
     m[i] = mj;
     v[i] = vj;
     if (sh) sh[i] = __float2bfloat16(pj);
+  }
+}
+
+// ------------------------------------------------------------------------------------------ AFNO block weights
+
+// Complex block weights [2][nb][in][out] (fp32, real and imaginary planes) -> the real form the block GEMMs read, bf16
+// [nb][2 out][2 in] with rows (ri', o), columns (ri, i): [[wr^T, -wi^T], [wi^T, wr^T]]; biases [2][nb][out] -> [nb][2 out]
+// fp32.  Both layers in one launch: the tensors are small, what counted was some twenty launches of transposes, negations
+// and concatenations per pass.  grid (ceil(max in / 32), ceil(max out / 32), 2 nb), block 32 x 8
+__global__ void __launch_bounds__(256) afno_pack_kernel(const AfnoLayer a, const AfnoLayer b, int nb) {
+  __shared__ float re[32][33], im[32][33];
+  const AfnoLayer& L = blockIdx.z < static_cast<unsigned>(nb) ? a : b;
+  const int blk = blockIdx.z % nb, i0 = blockIdx.x * 32, o0 = blockIdx.y * 32;
+  if (i0 >= L.nin || o0 >= L.nout) return;
+  const long long plane = static_cast<long long>(nb) * L.nin * L.nout;
+  const float* w = L.w + static_cast<long long>(blk) * L.nin * L.nout;
+  for (int j = threadIdx.y; j < 32; j += 8) {
+    const int i = i0 + j, o = o0 + threadIdx.x;
+    const bool in = i < L.nin && o < L.nout;
+    re[j][threadIdx.x] = in ? w[static_cast<long long>(i) * L.nout + o] : 0.f;
+    im[j][threadIdx.x] = in ? w[plane + static_cast<long long>(i) * L.nout + o] : 0.f;
+  }
+  __syncthreads();
+  __nv_bfloat16* const wx = L.wx + static_cast<long long>(blk) * 4 * L.nin * L.nout;
+  for (int j = threadIdx.y; j < 32; j += 8) {
+    const int o = o0 + j, i = i0 + threadIdx.x;
+    if (o < L.nout && i < L.nin) {
+      const float r = re[threadIdx.x][j], m = im[threadIdx.x][j];
+      __nv_bfloat16* top = wx + static_cast<long long>(o) * 2 * L.nin + i;
+      __nv_bfloat16* bot = top + static_cast<long long>(L.nout) * 2 * L.nin;
+      top[0] = __float2bfloat16(r);
+      top[L.nin] = __float2bfloat16(-m);
+      bot[0] = __float2bfloat16(m);
+      bot[L.nin] = __float2bfloat16(r);
+    }
+  }
+  if (L.b && blockIdx.x == 0 && threadIdx.y < 2) {
+    const int o = o0 + threadIdx.x;
+    if (o < L.nout)
+      L.bx[(static_cast<long long>(blk) * 2 + threadIdx.y) * L.nout + o] =
+          L.b[(static_cast<long long>(threadIdx.y) * nb + blk) * L.nout + o];
+  }
+}
+
+// The way back for the gradients: dwx fp32 [nb][2 out][2 in] -> dw [2][nb][in][out] with dwr = (d00 + d11)^T, dwi = (d10 - d01)^T,
+// and dbx [nb][2 out] -> db [2][nb][out].  Same grid.
+__global__ void __launch_bounds__(256) afno_fold_kernel(const AfnoGrad a, const AfnoGrad b, int nb) {
+  __shared__ float re[32][33], im[32][33];
+  const AfnoGrad& L = blockIdx.z < static_cast<unsigned>(nb) ? a : b;
+  const int blk = blockIdx.z % nb, i0 = blockIdx.x * 32, o0 = blockIdx.y * 32;
+  if (i0 >= L.nin || o0 >= L.nout) return;
+  const float* const wx = L.dwx + static_cast<long long>(blk) * 4 * L.nin * L.nout;
+  for (int j = threadIdx.y; j < 32; j += 8) {
+    const int o = o0 + j, i = i0 + threadIdx.x;
+    const bool in = o < L.nout && i < L.nin;
+    const float* top = wx + static_cast<long long>(o) * 2 * L.nin + i;
+    const float* bot = top + static_cast<long long>(L.nout) * 2 * L.nin;
+    re[j][threadIdx.x] = in ? top[0] + bot[L.nin] : 0.f;
+    im[j][threadIdx.x] = in ? bot[0] - top[L.nin] : 0.f;
+  }
+  __syncthreads();
+  const long long plane = static_cast<long long>(nb) * L.nin * L.nout;
+  float* w = L.dw + static_cast<long long>(blk) * L.nin * L.nout;
+  for (int j = threadIdx.y; j < 32; j += 8) {
+    const int i = i0 + j, o = o0 + threadIdx.x;
+    if (i < L.nin && o < L.nout) {
+      w[static_cast<long long>(i) * L.nout + o] = re[threadIdx.x][j];
+      w[plane + static_cast<long long>(i) * L.nout + o] = im[threadIdx.x][j];
+    }
+  }
+  if (L.db && blockIdx.x == 0 && threadIdx.y < 2) {
+    const int o = o0 + threadIdx.x;
+    if (o < L.nout)
+      L.db[(static_cast<long long>(threadIdx.y) * nb + blk) * L.nout + o] =
+          L.dbx[(static_cast<long long>(blk) * 2 + threadIdx.y) * L.nout + o];
   }
 }
 
@@ -1191,18 +1275,40 @@ cudaError_t inorm_cl_apply(const __nv_bfloat16* x, const __nv_bfloat16* dy, __nv
   return cudaGetLastError();
 }
 
-cudaError_t colsum(const __nv_bfloat16* x, float* out, long long rows, int C, cudaStream_t s) {
-  if (rows <= 0 || C <= 0) return cudaSuccess;
-  if ((C & 7) || !aligned16(x) || !aligned16(out)) return cudaErrorInvalidValue;
+cudaError_t colsum(const __nv_bfloat16* x, float* out, long long rows, int C, cudaStream_t s, int groups, long long gstride,
+                   int inner, long long ostride) {
+  if (rows <= 0 || C <= 0 || groups <= 0) return cudaSuccess;
+  if ((C & 7) || (gstride & 7) || (ostride & 7) || groups > 65535 || (inner > 0 && rows >= (1ll << 31)) || !aligned16(x) ||
+      !aligned16(out))
+    return cudaErrorInvalidValue;
   const int V = C / 8;
   const int parts = (V + CS_THREADS - 1) / CS_THREADS;
   const int vb = (V + parts - 1) / parts;
   const int R = CS_THREADS / vb;
   // about four CTAs per SM, each with at least one full step of eight rows per thread
-  long long slab = (rows * parts + 4LL * sm_count() - 1) / (4LL * sm_count());
+  long long slab = (rows * parts * groups + 4LL * sm_count() - 1) / (4LL * sm_count());
   if (slab < 8LL * R) slab = 8LL * R;
-  dim3 grid(parts, static_cast<unsigned>((rows + slab - 1) / slab));
-  colsum_kernel<<<grid, CS_THREADS, 0, s>>>(reinterpret_cast<const uint4*>(x), out, rows, V, vb, static_cast<int>(slab));
+  dim3 grid(parts, static_cast<unsigned>((rows + slab - 1) / slab), groups);
+  colsum_kernel<<<grid, CS_THREADS, 0, s>>>(reinterpret_cast<const uint4*>(x), out, rows, V, vb, static_cast<int>(slab), inner,
+                                            ostride / 8, gstride / 8);
+  return cudaGetLastError();
+}
+
+template <typename L>
+static dim3 afno_grid(const L& a, const L& b, int nb) {
+  const int in = a.nin > b.nin ? a.nin : b.nin, out = a.nout > b.nout ? a.nout : b.nout;
+  return dim3((in + 31) / 32, (out + 31) / 32, 2 * nb);
+}
+
+cudaError_t afno_pack(const AfnoLayer& a, const AfnoLayer& b, int nb, cudaStream_t s) {
+  if (nb <= 0) return cudaSuccess;
+  afno_pack_kernel<<<afno_grid(a, b, nb), dim3(32, 8), 0, s>>>(a, b, nb);
+  return cudaGetLastError();
+}
+
+cudaError_t afno_fold(const AfnoGrad& a, const AfnoGrad& b, int nb, cudaStream_t s) {
+  if (nb <= 0) return cudaSuccess;
+  afno_fold_kernel<<<afno_grid(a, b, nb), dim3(32, 8), 0, s>>>(a, b, nb);
   return cudaGetLastError();
 }
 

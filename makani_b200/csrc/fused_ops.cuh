@@ -58,8 +58,28 @@ cudaError_t inorm_cl_apply(const __nv_bfloat16* x, const __nv_bfloat16* dy, __nv
                            const float* sums, float* stats, int B, int C, long long T, double count, float eps, int act, int mode,
                            cudaStream_t s, const StatExchange* xch = nullptr);
 
-// out[c] += sum over rows of x[rows, C] (C % 8 == 0, 16-byte aligned; out zero-initialised by the caller)
-cudaError_t colsum(const __nv_bfloat16* x, float* out, long long rows, int C, cudaStream_t s);
+// out[g, c] += sum over the rows of group g of x (C % 8 == 0, 16-byte aligned; out [groups, C] zero-initialised by the caller).
+// Row r of group g: g * gstride + (r / inner) * ostride + (r % inner) * C; inner = 0: rows follow one another.
+cudaError_t colsum(const __nv_bfloat16* x, float* out, long long rows, int C, cudaStream_t s, int groups = 1,
+                   long long gstride = 0, int inner = 0, long long ostride = 0);
+
+// ---- AFNO block weights: one layer's tensors (see the kernels), two layers per launch ----
+struct AfnoLayer {
+  const float* w;          // [2][nb][nin][nout]
+  const float* b;          // [2][nb][nout] or null
+  __nv_bfloat16* wx;       // [nb][2 nout][2 nin]
+  float* bx;               // [nb][2 nout]
+  int nin, nout;
+};
+struct AfnoGrad {
+  const float* dwx;        // [nb][2 nout][2 nin]
+  const float* dbx;        // [nb][2 nout] or null
+  float* dw;               // [2][nb][nin][nout]
+  float* db;               // [2][nb][nout] or null
+  int nin, nout;
+};
+cudaError_t afno_pack(const AfnoLayer& a, const AfnoLayer& b, int nb, cudaStream_t s);
+cudaError_t afno_fold(const AfnoGrad& a, const AfnoGrad& b, int nb, cudaStream_t s);
 
 // ---- quadrature-weighted Lp norms on the sphere ----
 // out[plane] = (sum_hw q[h] |p-t|^P, sum_hw q[h] |t|^P), P in {1,2}.  `scratch` holds

@@ -81,9 +81,11 @@ class AFNO2D(nn.Module):
         xc = x.contiguous()
         if xc.is_cuda and xc.dtype == torch.float32 and torch.is_autocast_enabled():
             xc = xc.to(torch.get_autocast_gpu_dtype())     # layer norm hands fp32 on under autocast; the GEMM chain runs in bf16
-        fn = afno_ops.afno_filter if afno_ops.fast_path_ok(xc, self.num_blocks_local, hid) else afno_ops.afno_filter_reference
-        y = fn(xc, self.w1[0], self.w1[1], self.b1[0], self.b1[1], self.w2[0], self.w2[1], self.b2[0], self.b2[1],
-               kx, ncols, self.sparsity_threshold, skip=xc)
+        if afno_ops.fast_path_ok(xc, self.num_blocks_local, hid):
+            y = afno_ops.afno_filter_stacked(xc, self.w1, self.b1, self.w2, self.b2, kx, ncols, self.sparsity_threshold, skip=xc)
+        else:
+            y = afno_ops.afno_filter_reference(xc, self.w1[0], self.w1[1], self.b1[0], self.b1[1], self.w2[0], self.w2[1],
+                                               self.b2[0], self.b2[1], kx, ncols, self.sparsity_threshold, skip=xc)
         if msize > 1:
             y = gather_from_parallel_region(y, 3, self.chan_shapes, "matmul")
         return y

@@ -12,7 +12,7 @@ How: each DFT is a real GEMM against a small constant cos / sin matrix (complex 
 next to the channel index), restricted to the kept modes, so the window costs nothing and no full spectrum is ever
 materialised; the block MLP is a batched GEMM over the blocks on 2x2 real block matrices with bias + ReLU and bias +
 soft shrinkage in the epilogues; the inverse transforms are two more GEMMs and the skip is added in the last epilogue.
-Six launches forward; the backward pass is the same four transform stages run with the transposed matrices (the DFT
+Seven launches forward (one packs the weights); the backward pass is the same four transform stages run with the transposed matrices (the DFT
 matrices are orthogonal up to the Hermitian weights), two data-gradient GEMMs whose epilogues apply the ReLU / shrinkage
 masks from the saved outputs, and two weight-gradient GEMMs.  The intermediate layouts are chosen such that every
 operand of every GEMM has one uniform stride along its contraction index:
@@ -133,42 +133,72 @@ def _stage_w_synthesis(src, mat, plan: AFNOPlan, B, C, resid):
 
 
 def _stage_h_tokens(t1, plan: AFNOPlan, B, C, nb):
-    """t1 [B, ncols, H, 2, C] -> token-major spectrum Y [B*ncols*nkx, nb, 2, bs] (forward DFT along H)."""
+    """t1 [B, ncols, H, 2, C] -> token-major spectrum Y [B*ncols*nkx, nb, 2, bs] (forward DFT along H), per (b, ky, block)."""
     H, nc, nkx = plan.H, plan.ncols, plan.nkx
     bs = C // nb
     y = torch.empty(B * nc * nkx, nb, 2, bs, dtype=t1.dtype, device=t1.device)
-    gemm(2 * nkx, C, 2 * H, Operand(plan.fh, ld=plan.fh.shape[1]),
-         Operand(t1, ld=C, mn_major=True, zs_lo=H * 2 * C, zs_hi=nc * H * 2 * C),
-         Output(y, rs_lo=bs, rdiv=2, rs_hi=2 * C, ndiv=bs, ns_hi=2 * bs, d_zlo=nkx * 2 * C, d_zhi=nc * nkx * 2 * C),
-         zlo_n=nc, zhi_n=B)
+    gemm(2 * nkx, bs, 2 * H, Operand(plan.fh, ld=plan.fh.shape[1]),
+         Operand(t1, ld=C, mn_major=True, zs_lo=bs, zs_hi=H * 2 * C),
+         Output(y, rs_lo=bs, rdiv=2, rs_hi=2 * C, d_zlo=2 * bs, d_zhi=nkx * 2 * C), zlo_n=nb, zhi_n=B * nc)
     return y
+
+
+def _pack(ws, bs, dt):
+    """Weights [2, nb, in, out] (real and imaginary planes) of both layers -> real block form [nb, 2 out, 2 in] in `dt`, biases
+    [2, nb, out] -> [nb, 2 out] fp32."""
+    wx = [torch.empty(w.shape[1], 2 * w.shape[3], 2 * w.shape[2], dtype=dt, device=w.device) for w in ws]
+    bx = [None if b is None else torch.empty(b.shape[1], 2 * b.shape[2], dtype=torch.float32, device=b.device) for b in bs]
+    if ws[0].is_cuda:
+        f32 = lambda t: None if t is None else t.detach().float().contiguous()  # noqa: E731
+        none = ws[0].new_empty(0)
+        _ext.require().afno_pack([f32(w) for w in ws], [f32(b) for b in bs], wx, [none if b is None else b for b in bx])
+        return wx, bx
+    wx = [expand_complex_weight(w.detach()[0], w.detach()[1]).to(dt).contiguous() for w in ws]
+    bx = [None if b is None else b.detach().transpose(0, 1).reshape(b.shape[1], -1).float() for b in bs]
+    return wx, bx
+
+
+def _fold(dwx, dbx, shapes, bias):
+    """The adjoint of `_pack`: gradients [2, nb, in, out] and [2, nb, out] (or None) of both layers."""
+    dw = [torch.empty(s, dtype=torch.float32, device=dwx[0].device) for s in shapes]
+    db = [torch.empty(2, s[1], s[3], dtype=torch.float32, device=dwx[0].device) if h else None for s, h in zip(shapes, bias)]
+    if dwx[0].is_cuda:
+        _ext.require().afno_fold(dwx, dbx, dw, db)
+        return dw, db
+    for k, (_, nb, ni, no) in enumerate(shapes):
+        d = dwx[k].view(nb, 2, no, 2, ni)
+        dw[k][0] = (d[:, 0, :, 0] + d[:, 1, :, 1]).transpose(1, 2)
+        dw[k][1] = (d[:, 1, :, 0] - d[:, 0, :, 1]).transpose(1, 2)
+        if bias[k]:
+            db[k].copy_(dbx[k].view(nb, 2, no).transpose(0, 1))
+    return dw, db
 
 
 class _AFNOFilter(torch.autograd.Function):
     """y = irfft2(softshrink(relu(rfft2(x) W1 + b1) W2 + b2)) (+ skip) on the kept modes.
 
-    w1x [nb, 2 hid, 2 bs] and w2x [nb, 2 bs, 2 hid] are the real 2x2-block forms of the complex block weights (rows: output
-    (ri, o), columns: input (ri, i)); b1x [nb, 2 hid] / b2x [nb, 2 bs] the stacked (re, im) biases or None."""
+    w1 [2, nb, bs, hid], w2 [2, nb, hid, bs] hold real and imaginary planes of the complex block weights, b1 [2, nb, hid] and
+    b2 [2, nb, bs] those of the biases (or None); they are packed into real 2x2-block matrices here.  Every GEMM writes plain
+    rows, or rows split into (mode, re / im) pairs, so that all of them leave through TMA stores."""
 
     @staticmethod
-    def forward(ctx, x, w1x, b1x, w2x, b2x, skip, plan, lam):
+    def forward(ctx, x, w1, b1, w2, b2, skip, plan, lam):
         B, H, W, C = x.shape
-        nb = w1x.shape[0]
-        bs, hid = C // nb, w1x.shape[1] // 2
+        nb = w1.shape[1]
+        bs, hid = C // nb, w1.shape[3]
         nc, nkx = plan.ncols, plan.nkx
         T = B * nc * nkx
         dt = x.dtype
-        w1q, w2q = w1x.detach().to(dt).contiguous(), w2x.detach().to(dt).contiguous()
-        b1f = b1x.detach().float().contiguous() if b1x is not None else None
-        b2f = b2x.detach().float().contiguous() if b2x is not None else None
+        (w1q, w2q), (b1f, b2f) = _pack((w1, w2), (b1, b2), dt)
         t1 = _stage_w_analysis(x, plan.fw, plan)
         y = _stage_h_tokens(t1, plan, B, C, nb)
         o1 = torch.empty(T, nb, 2 * hid, dtype=dt, device=x.device)
         gemm(T, 2 * hid, 2 * bs, Operand(y, ld=2 * C, zs_lo=2 * bs), Operand(w1q, ld=2 * bs, zs_lo=2 * hid * 2 * bs),
              Output(o1, rs_lo=nb * 2 * hid, d_zlo=2 * hid), zlo_n=nb, bias=b1f, bias_mode=BIAS_COL, bias_zs=2 * hid, act=ACT_RELU)
         o2 = torch.empty(B * nc, nb, nkx, 2, bs, dtype=dt, device=x.device)
-        gemm(T, 2 * bs, 2 * hid, Operand(o1, ld=nb * 2 * hid, zs_lo=2 * hid), Operand(w2q, ld=2 * hid, zs_lo=2 * bs * 2 * hid),
-             Output(o2, rs_lo=2 * bs, rdiv=nkx, rs_hi=nb * nkx * 2 * bs, d_zlo=nkx * 2 * bs), zlo_n=nb, bias=b2f,
+        gemm(nkx, 2 * bs, 2 * hid, Operand(o1, ld=nb * 2 * hid, zs_lo=2 * hid, zs_hi=nkx * nb * 2 * hid),
+             Operand(w2q, ld=2 * hid, zs_lo=2 * bs * 2 * hid),
+             Output(o2, rs_lo=2 * bs, d_zlo=nkx * 2 * bs, d_zhi=nb * nkx * 2 * bs), zlo_n=nb, zhi_n=B * nc, bias=b2f,
              bias_mode=BIAS_COL, bias_zs=2 * bs, act=ACT_SHRINK, act_param=float(lam))
         t4 = _stage_h_blocks(o2, plan.gh, plan, B, C, nb)
         out = _stage_w_synthesis(t4, plan.gw, plan, B, C, skip)
@@ -176,7 +206,8 @@ class _AFNOFilter(torch.autograd.Function):
         ctx.plan, ctx.dims = plan, (B, C, nb, bs, hid)
         # skip_is_x: the skip is the input itself (the usual residual form); its gradient then rides in the epilogue of
         # the last backward GEMM instead of a separate elementwise add
-        ctx.flags = (b1x is not None, b2x is not None, skip is not None, skip is x)
+        ctx.flags = (b1 is not None, b2 is not None, skip is not None, skip is x)
+        ctx.wtypes = tuple(None if t is None else t.dtype for t in (w1, b1, w2, b2))
         return out
 
     @staticmethod
@@ -190,6 +221,12 @@ class _AFNOFilter(torch.autograd.Function):
         dy = dy.contiguous()
         dt = dy.dtype
         dev = dy.device
+        # fp32 sums of the packed weights and biases, cleared together
+        n1, n2 = 2 * hid * 2 * bs * nb, 2 * hid * nb
+        acc = torch.zeros(2 * n1 + n2 + 2 * bs * nb, dtype=torch.float32, device=dev)
+        dw1, dw2 = acc[:n1].view(nb, 2 * hid, 2 * bs), acc[n1: 2 * n1].view(nb, 2 * bs, 2 * hid)
+        db1, db2 = acc[2 * n1: 2 * n1 + n2].view(nb, 2 * hid), acc[2 * n1 + n2:].view(nb, 2 * bs)
+        native = dev.type == "cuda"
         # adjoint of the synthesis along W, then along H with the shrinkage mask (saved output != 0) in the epilogue
         dt4 = _stage_w_analysis(dy, plan.gw_t, plan)                                   # [B, ncols, H, 2, C]
         do2 = torch.empty_like(o2)
@@ -203,30 +240,38 @@ class _AFNOFilter(torch.autograd.Function):
              Operand(w2q, ld=2 * hid, mn_major=True, zs_lo=2 * bs * 2 * hid),
              Output(do1, rs_lo=nb * 2 * hid, d_zlo=2 * hid, d_zhi=nkx * nb * 2 * hid), zlo_n=nb, zhi_n=B * nc,
              act=ACT_DRELU, resid=o1)
-        dw2 = torch.zeros(nb, 2 * bs, 2 * hid, dtype=torch.float32, device=dev)
         gemm(2 * bs, 2 * hid, nkx, Operand(do2, ld=2 * bs, mn_major=True, zs_lo=nkx * 2 * bs, zs_hi=nb * nkx * 2 * bs),
              Operand(o1, ld=nb * 2 * hid, mn_major=True, zs_lo=2 * hid, zs_hi=nkx * nb * 2 * hid),
-             Output(dw2, rs_lo=2 * hid, d_zlo=2 * bs * 2 * hid), zlo_n=nb, zhi_n=B * nc, accumulate=True)
-        db2 = do2.reshape(B * nc, nb, nkx, 2 * bs).float().sum(dim=(0, 2)) if has_b2 else None
+             Output(dw2, rs_lo=2 * hid, d_zlo=2 * bs * 2 * hid), zlo_n=nb, zhi_n=B * nc, accumulate=True, splits=0)
+        if has_b2:
+            if native:
+                _ext.require().colsum_groups(do2, db2, B * nc, nb, nkx)
+            else:
+                db2.copy_(do2.reshape(B * nc, nb, nkx, 2 * bs).float().sum(dim=(0, 2)))
         # first layer
         dyt = torch.empty(B * nc, nb, nkx, 2, bs, dtype=dt, device=dev)
-        gemm(T, 2 * bs, 2 * hid, Operand(do1, ld=nb * 2 * hid, zs_lo=2 * hid),
+        gemm(nkx, 2 * bs, 2 * hid, Operand(do1, ld=nb * 2 * hid, zs_lo=2 * hid, zs_hi=nkx * nb * 2 * hid),
              Operand(w1q, ld=2 * bs, mn_major=True, zs_lo=2 * hid * 2 * bs),
-             Output(dyt, rs_lo=2 * bs, rdiv=nkx, rs_hi=nb * nkx * 2 * bs, d_zlo=nkx * 2 * bs), zlo_n=nb)
-        dw1 = torch.zeros(nb, 2 * hid, 2 * bs, dtype=torch.float32, device=dev)
+             Output(dyt, rs_lo=2 * bs, d_zlo=nkx * 2 * bs, d_zhi=nb * nkx * 2 * bs), zlo_n=nb, zhi_n=B * nc)
         gemm(2 * hid, 2 * bs, T, Operand(do1, ld=nb * 2 * hid, mn_major=True, zs_lo=2 * hid),
              Operand(y, ld=2 * C, mn_major=True, zs_lo=2 * bs),
              Output(dw1, rs_lo=2 * bs, d_zlo=2 * hid * 2 * bs), zlo_n=nb, accumulate=True, splits=0)
-        db1 = do1.float().sum(dim=0) if has_b1 else None
+        if has_b1:
+            if native:
+                _ext.require().colsum(do1, db1)
+            else:
+                db1.copy_(do1.float().sum(dim=0))
+        (gw1, gw2), (gb1, gb2) = _fold([dw1, dw2], [db1, db2], [(2, nb, bs, hid), (2, nb, hid, bs)], (has_b1, has_b2))
+        gw1, gb1, gw2, gb2 = (g if g is None else g.to(t) for g, t in zip((gw1, gb1, gw2, gb2), ctx.wtypes))
         # adjoint of the analysis along H and along W; the skip's gradient joins in the last epilogue
         dt1 = _stage_h_blocks(dyt, plan.gh, plan, B, C, nb)                            # [H, B*ncols, 2, C]
         dx = _stage_w_synthesis(dt1, plan.fw_t, plan, B, C, dy if skip_is_x else None)
-        return dx, dw1, db1, dw2, db2, (dy if (has_skip and not skip_is_x) else None), None, None
+        return dx, gw1, gb1, gw2, gb2, (dy if (has_skip and not skip_is_x) else None), None, None
 
 
 def expand_complex_weight(wr: torch.Tensor, wi: torch.Tensor) -> torch.Tensor:
     """Complex block weights [nb, in, out] (real and imaginary parts) -> real block form [nb, 2 out, 2 in] with rows
-    (ri', o), columns (ri, i): [[wr^T, -wi^T], [wi^T, wr^T]].  Plain torch, so autograd carries the gradient back."""
+    (ri', o), columns (ri, i): [[wr^T, -wi^T], [wi^T, wr^T]]."""
     wrt, wit = wr.transpose(1, 2), wi.transpose(1, 2)
     return torch.cat([torch.cat([wrt, -wit], dim=2), torch.cat([wit, wrt], dim=2)], dim=1)
 
@@ -247,12 +292,15 @@ def afno_filter(x, w1r, w1i, b1r, b1i, w2r, w2i, b2r, b2i, kx: Sequence[int], nc
     """NHWC tokens x [B, H, W, C]; block weights w1 [nb, bs, hid], w2 [nb, hid, bs] and biases b1 [nb, hid], b2 [nb, bs]
     given as real / imaginary parts (biases may be None); `kx` the kept rows and `ncols` the kept columns of the
     half-spectrum; `skip` (same shape as x) is added to the result."""
-    B, H, W, C = x.shape
-    plan = AFNOPlan.get(H, W, tuple(kx), int(ncols), x.device, x.dtype)
-    w1x, w2x = expand_complex_weight(w1r, w1i), expand_complex_weight(w2r, w2i)
-    b1x = torch.cat([b1r, b1i], dim=1) if b1r is not None else None
-    b2x = torch.cat([b2r, b2i], dim=1) if b2r is not None else None
-    return _AFNOFilter.apply(x, w1x, b1x, w2x, b2x, skip, plan, float(lam))
+    pair = lambda r, i: None if r is None else torch.stack([r, i])  # noqa: E731
+    return afno_filter_stacked(x, pair(w1r, w1i), pair(b1r, b1i), pair(w2r, w2i), pair(b2r, b2i), kx, ncols, lam, skip)
+
+
+def afno_filter_stacked(x, w1, b1, w2, b2, kx: Sequence[int], ncols: int, lam: float, skip: Optional[torch.Tensor] = None):
+    """`afno_filter` with the real and imaginary parts of each parameter in one tensor: w1 [2, nb, bs, hid], b1 [2, nb, hid],
+    w2 [2, nb, hid, bs], b2 [2, nb, bs]."""
+    plan = AFNOPlan.get(x.shape[1], x.shape[2], tuple(kx), int(ncols), x.device, x.dtype)
+    return _AFNOFilter.apply(x, w1, b1, w2, b2, skip, plan, float(lam))
 
 
 _ROW_INDEX = {}

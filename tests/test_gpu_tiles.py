@@ -159,3 +159,59 @@ def test_instance_norm_channel_counts(b, c, h, w, act):
     ref = [yr] + list(torch.autograd.grad(yr, [xd, wd, bd], dy.double()))
     for a, r in zip(got, ref):
         assert _rel(a, r) < BF16
+
+
+@pytest.mark.parametrize("rd,m", [(2, 182), (2, 6), (4, 132), (32, 96), (2, 181), (3, 180)])
+@pytest.mark.parametrize("epi", ["plain", "resid", "gelu_pre"])
+def test_gemm_split_rows(rd, m, epi):
+    """Rows addressed as (r / rd, r % rd): as a dimension of the tensor maps where rd is a power of two that divides the rows,
+    by the generic epilogue otherwise."""
+    dev = _dev()
+    k, n, hi = 72, 136, (m + rd - 1) // rd
+    torch.manual_seed(rd * m)
+    a, b = torch.randn(3, m, k, device=dev).to(torch.bfloat16), torch.randn(n, k, device=dev).to(torch.bfloat16)
+    shape = (rd, 3, hi, n)            # the low part of the row index is the slowest dimension
+    lay = dict(rs_lo=3 * hi * n, rdiv=rd, rs_hi=n, d_zlo=hi * n)
+    d = torch.zeros(shape, device=dev, dtype=torch.bfloat16)
+    aux = torch.randn(shape, device=dev).to(torch.bfloat16) if epi == "resid" else None
+    pre = torch.zeros_like(d) if epi == "gelu_pre" else None
+    outs = _run_both(m, n, k, Operand(a, ld=k, zs_lo=m * k), Operand(b, ld=k), Output(d, **lay), zlo_n=3, resid=aux, preact=pre,
+                     act=ACT_GELU if epi == "gelu_pre" else ACT_NONE)
+    for got, ref in outs:
+        assert _rel(got, ref) < BF16
+
+
+@pytest.mark.parametrize("z", [1, 2, 91, 800])
+@pytest.mark.parametrize("co,ci,k", [(16, 24, 8), (192, 192, 90), (136, 264, 200)])
+def test_gemm_batches_summed_inside_tiles(z, co, ci, k):
+    """Batches that add into one output: none, a few and many per tile, the last group shorter."""
+    dev = _dev()
+    g = torch.Generator(dev).manual_seed(z + co)
+    a = torch.randn(2, z, k, co, device=dev, generator=g).to(torch.bfloat16)
+    b = torch.randn(2, z, k, ci, device=dev, generator=g).to(torch.bfloat16)
+    d = torch.zeros(2, co, ci, device=dev)
+    gemm(co, ci, k, Operand(a, ld=co, mn_major=True, zs_lo=z * k * co, zs_hi=k * co),
+         Operand(b, ld=ci, mn_major=True, zs_lo=z * k * ci, zs_hi=k * ci), Output(d, rs_lo=ci, d_zlo=co * ci), zlo_n=2, zhi_n=z,
+         accumulate=True, splits=0)
+    _ext.check_device_errors(dev)
+    assert _rel(d, torch.einsum("lzko,lzki->loi", a.double(), b.double())) < 2.0 ** -24 * max(z * k, 64) ** 0.5 * 4
+
+
+@pytest.mark.parametrize("nb,bs,hid,bias", [(1, 8, 8, True), (3, 24, 40, True), (8, 96, 96, False), (2, 72, 32, True)])
+def test_afno_weight_packing(nb, bs, hid, bias):
+    """Packing of both layers' weights and its adjoint against the plain formulation, block sizes around the 32-wide tiles."""
+    from makani_b200.ops.afno import _fold, _pack
+    dev = _dev()
+    g = torch.Generator(dev).manual_seed(bs)
+    r = lambda *s: torch.randn(*s, device=dev, generator=g)  # noqa: E731
+    ws = (r(2, nb, bs, hid), r(2, nb, hid, bs))
+    bz = (r(2, nb, hid), r(2, nb, bs)) if bias else (None, None)
+    got, ref = _pack(ws, bz, torch.bfloat16), _pack([w.cpu() for w in ws], [None if b is None else b.cpu() for b in bz], torch.bfloat16)
+    for p, q in zip(got[0] + got[1], ref[0] + ref[1]):
+        assert (p is None and q is None) or torch.equal(p.cpu(), q)
+    dw, db = [r(nb, 2 * hid, 2 * bs), r(nb, 2 * bs, 2 * hid)], [r(nb, 2 * hid), r(nb, 2 * bs)]
+    shapes = [(2, nb, bs, hid), (2, nb, hid, bs)]
+    got = _fold(dw, db, shapes, (bias, bias))
+    ref = _fold([t.cpu() for t in dw], [t.cpu() for t in db], shapes, (bias, bias))
+    for p, q in zip(got[0] + got[1], ref[0] + ref[1]):
+        assert (p is None and q is None) or torch.equal(p.cpu(), q)
