@@ -118,16 +118,16 @@ def dft_synthesis(t4: torch.Tensor, mat: torch.Tensor, mat_mn: bool, mat_ld: int
     return y
 
 
-def legendre_analysis(t1: torch.Tensor, table: torch.Tensor) -> torch.Tensor:
-    """T2[b, l, m, n] = sum_k table[m, l, k] T1[b, k, m, n], n = (ri, c);  zero for l < m."""
+def legendre_analysis(t1: torch.Tensor, table: torch.Tensor, by_order: bool = False) -> torch.Tensor:
+    """T2[b, l, m, n] = sum_k table[m, l, k] T1[b, k, m, n], n = (ri, c);  zero for l < m.  `by_order`: as [b, m, l, n]."""
     B, H, k2, C = t1.shape
     mmax, lmax, hpt = table.shape
     n2 = 2 * C
-    t2 = torch.empty(B, lmax, mmax, n2, dtype=t1.dtype, device=t1.device)
+    t2 = torch.empty(*((B, mmax, lmax) if by_order else (B, lmax, mmax)), n2, dtype=t1.dtype, device=t1.device)
     gemm(lmax, n2, H,
          Operand(table, ld=hpt, zs_hi=lmax * hpt),
          Operand(t1, ld=k2 * C, mn_major=True, zs_hi=n2, zs_lo=H * k2 * C),
-         Output(t2, rs_lo=mmax * n2, d_zhi=n2, d_zlo=lmax * mmax * n2),
+         Output(t2, rs_lo=n2 if by_order else mmax * n2, d_zhi=lmax * n2 if by_order else n2, d_zlo=lmax * mmax * n2),
          zhi_n=mmax, zlo_n=B, tri=Tri(rmin_a=1))
     return t2
 
@@ -151,9 +151,10 @@ def legendre_synthesis(t: torch.Tensor, lm_order: bool, table: torch.Tensor, H: 
     return t4
 
 
-def contract(t2: torch.Tensor, wx: torch.Tensor, transpose_w: bool) -> torch.Tensor:
+def contract(t2: torch.Tensor, wx: torch.Tensor, transpose_w: bool, resid=None) -> torch.Tensor:
     """T3[b, m, l, q] = sum_p T2[b, l, m, p] Wx[l, q, p]   (transpose_w False; Wx [l, 2Co, 2Ci])
-       T3[b, m, l, p] = sum_q T2[b, l, m, q] Wx[l, q, p]   (transpose_w True: adjoint w.r.t. the input)."""
+       T3[b, m, l, p] = sum_q T2[b, l, m, q] Wx[l, q, p]   (transpose_w True: adjoint w.r.t. the input)
+    plus `resid`, which has the layout of the result."""
     B, lmax, mmax, kin = t2.shape
     nq, npp = wx.shape[1], wx.shape[2]
     nout = npp if transpose_w else nq
@@ -162,7 +163,7 @@ def contract(t2: torch.Tensor, wx: torch.Tensor, transpose_w: bool) -> torch.Ten
          Operand(t2, ld=kin, zs_hi=mmax * kin, zs_lo=lmax * mmax * kin),
          Operand(wx, ld=npp, mn_major=transpose_w, zs_hi=nq * npp),
          Output(t3, rs_lo=lmax * nout, d_zhi=nout, d_zlo=mmax * lmax * nout),
-         zhi_n=lmax, zlo_n=B, tri=Tri(rmax_a=1, rmax_b=1))
+         zhi_n=lmax, zlo_n=B, tri=Tri(rmax_a=1, rmax_b=1), resid=resid)
     return t3
 
 
@@ -304,14 +305,15 @@ class _SpectralConv(torch.autograd.Function):
             dw = fold_weight_grad2(contract_wgrad2(dt3, t2)).reshape(ctx.wshape)
         dx = None
         if ctx.needs_input_grad[0]:
-            dt2 = contract(dt3, wx, True)                              # [B, m, l, (ri, c)]
+            dr2 = None
             if ctx.want_resid and dr is not None:
-                dr = _to_cl(dr)
-                dr4 = dft_analysis(dr, plan_out.gt, True, plan_out.k2p, plan_out.k2)
-                dr2 = legendre_analysis(dr4, plan_out.p)               # [B, l, m, n]
-                dt2 = dt2 + dr2.transpose(1, 2)
-                del dr4, dr2
-            dt1 = legendre_synthesis(dt2.contiguous(), False, plan_in.pw, plan_in.nlat)
+                # laid out by order, as the contraction writes: its epilogue adds the residual's share
+                dr4 = dft_analysis(_to_cl(dr), plan_out.gt, True, plan_out.k2p, plan_out.k2)
+                dr2 = legendre_analysis(dr4, plan_out.p, by_order=True)
+                del dr4
+            dt2 = contract(dt3, wx, True, resid=dr2)                   # [B, m, l, (ri, c)]
+            del dr2
+            dt1 = legendre_synthesis(dt2, False, plan_in.pw, plan_in.nlat)
             dx = dft_synthesis(dt1, plan_in.f, True, plan_in.nlon, plan_in.nlon)
         return dx, dw, None, None, None, None
 
