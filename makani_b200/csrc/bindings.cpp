@@ -288,6 +288,18 @@ void colsum(const Tensor& x, Tensor& out) {
              "colsum");
 }
 
+// x fp32 [rows, cols] -> y bf16 [rows, pitch], padding columns zero
+void cast_pad(const Tensor& x, Tensor& y) {
+  MK_CHECK(x.is_cuda() && x.scalar_type() == torch::kFloat32 && x.is_contiguous() && x.dim() == 2, "cast_pad: contiguous fp32 CUDA matrix expected");
+  MK_CHECK(y.is_cuda() && y.scalar_type() == torch::kBFloat16 && y.is_contiguous() && y.dim() == 2 && y.size(0) == x.size(0) &&
+               y.size(1) >= x.size(1) && y.size(1) % 8 == 0,
+           "cast_pad: bad output");
+  c10::cuda::CUDAGuard guard(x.device());
+  check_cuda(mk::cast_pad_bf16(x.data_ptr<float>(), reinterpret_cast<__nv_bfloat16*>(y.data_ptr()), x.size(0), static_cast<int>(x.size(1)),
+                               static_cast<int>(y.size(1)), cur_stream()),
+             "cast_pad");
+}
+
 // sums of do2 [outer, groups, inner, C] over outer and inner -> out [groups, C]
 void colsum_groups(const Tensor& x, Tensor& out, int64_t outer, int64_t groups, int64_t inner) {
   MK_CHECK(x.is_cuda() && x.scalar_type() == torch::kBFloat16 && x.is_contiguous(), "colsum_groups: contiguous bf16 CUDA tensor expected");
@@ -623,6 +635,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("clear_error_flag", &clear_error_flag);
   m.def("inorm_fwd", &inorm_fwd);
   m.def("inorm_partial_stats", &inorm_partial_stats);
+  m.def("cast_pad", &cast_pad);
   m.def("colsum", &colsum);
   m.def("colsum_groups", &colsum_groups);
   m.def("afno_pack", &afno_pack);

@@ -1161,6 +1161,21 @@ __global__ void swap_ri_kernel(const uint4* __restrict__ in, uint4* __restrict__
   }
 }
 
+// fp32 [rows, cols] -> bf16 [rows, pitch], the columns from cols on zero: the weight operand of a 1x1 convolution in one launch
+// (a fill, a cast and a strided copy before); one 16-byte vector per thread
+__global__ void __launch_bounds__(256) cast_pad_kernel(const float* __restrict__ x, uint4* __restrict__ y, int cols, int pitch_v,
+                                                       long long total) {
+  const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+  if (i >= total) return;
+  const long long r = i / pitch_v;
+  const int c = static_cast<int>(i - r * pitch_v) * 8;
+  const float* p = x + r * cols + c;
+  float f[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) f[j] = c + j < cols ? p[j] : 0.f;
+  y[i] = pack8(f);
+}
+
 __global__ void cast_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ y, long long n) {
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<long long>(gridDim.x) * blockDim.x)
@@ -1425,6 +1440,15 @@ cudaError_t cast_f32_bf16(const float* x, __nv_bfloat16* y, long long n, cudaStr
   long long blocks = (n + 255) / 256;
   if (blocks > sm_count() * 16) blocks = sm_count() * 16;
   cast_kernel<<<static_cast<unsigned>(blocks), 256, 0, s>>>(x, y, n);
+  return cudaGetLastError();
+}
+
+cudaError_t cast_pad_bf16(const float* x, __nv_bfloat16* y, long long rows, int cols, int pitch, cudaStream_t s) {
+  if (rows <= 0 || cols <= 0) return cudaSuccess;
+  if ((pitch & 7) || pitch < cols || !aligned16(y)) return cudaErrorInvalidValue;
+  const long long total = rows * (pitch / 8);
+  if ((total + 255) / 256 > 0x7fffffffll) return cudaErrorInvalidValue;
+  cast_pad_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, s>>>(x, reinterpret_cast<uint4*>(y), cols, pitch / 8, total);
   return cudaGetLastError();
 }
 

@@ -120,6 +120,8 @@ cudaError_t swap_ri_bf16(const __nv_bfloat16* in, __nv_bfloat16* out, long long 
 
 // ---- small elementwise helpers ----
 cudaError_t cast_f32_bf16(const float* x, __nv_bfloat16* y, long long n, cudaStream_t s);
+// fp32 [rows, cols] -> bf16 [rows, pitch] (pitch a multiple of 8, padding columns zero)
+cudaError_t cast_pad_bf16(const float* x, __nv_bfloat16* y, long long rows, int cols, int pitch, cudaStream_t s);
 cudaError_t fill_normal_bf16(__nv_bfloat16* y, long long n, uint64_t seed, cudaStream_t s);
 
 }  // namespace mk

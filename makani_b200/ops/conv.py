@@ -64,6 +64,10 @@ def prep_weight(w: torch.Tensor, dtype=torch.bfloat16) -> torch.Tensor:
     w2 = w.reshape(w.shape[0], -1)
     co, ci = w2.shape
     cip = pad_to(ci, 8)
+    if w2.is_cuda and w2.dtype == torch.float32 and dtype == torch.bfloat16 and w2.is_contiguous() and _ext.native():
+        out = torch.empty(co, cip, dtype=dtype, device=w.device)
+        _ext.require().cast_pad(w2.detach(), out)
+        return out
     out = torch.zeros(co, cip, dtype=dtype, device=w.device)
     out[:, :ci] = w2.detach().to(dtype)
     return out

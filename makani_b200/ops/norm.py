@@ -94,9 +94,9 @@ class _InstanceNormCL(torch.autograd.Function):
         B, C, H, W = x.shape
         if not _is_cl(dy):
             dy = dy.contiguous(memory_format=torch.channels_last)
-        sums = torch.zeros(B, C, 2, dtype=torch.float32, device=x.device)
-        dw = torch.zeros(C, dtype=torch.float32, device=x.device) if ctx.affine else None
-        db = torch.zeros(C, dtype=torch.float32, device=x.device) if ctx.affine else None
+        acc = torch.zeros(2 * B + (2 if ctx.affine else 0), C, dtype=torch.float32, device=x.device)     # one clearing launch
+        sums = acc[: 2 * B].view(B, C, 2)
+        dw, db = (acc[2 * B], acc[2 * B + 1]) if ctx.affine else (None, None)
         dx = torch.empty_like(x)
         slot = ctx.slot
         if slot is not None:

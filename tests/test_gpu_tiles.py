@@ -215,3 +215,11 @@ def test_afno_weight_packing(nb, bs, hid, bias):
     ref = _fold([t.cpu() for t in dw], [t.cpu() for t in db], shapes, (bias, bias))
     for p, q in zip(got[0] + got[1], ref[0] + ref[1]):
         assert (p is None and q is None) or torch.equal(p.cpu(), q)
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 1), (16, 5), (73, 384), (384, 74), (8, 16), (300, 1001)])
+def test_convolution_weight_operand(rows, cols):
+    from makani_b200.ops.conv import prep_weight
+    dev = _dev()
+    w = torch.randn(rows, cols, 1, 1, device=dev)
+    assert torch.equal(prep_weight(w).cpu(), prep_weight(w.cpu()))
