@@ -223,3 +223,21 @@ def test_convolution_weight_operand(rows, cols):
     dev = _dev()
     w = torch.randn(rows, cols, 1, 1, device=dev)
     assert torch.equal(prep_weight(w).cpu(), prep_weight(w.cpu()))
+
+
+@pytest.mark.parametrize("acc", [False, True])
+@pytest.mark.parametrize("m,n,k", [(128, 32, 64), (200, 36, 72), (392, 384, 40), (130, 772, 520)])
+def test_gemm_fp32_output(acc, m, n, k):
+    """fp32 results stored and added through TMA: half boxes, ragged rows and columns, single CTAs and pairs, added to what
+    is there."""
+    dev = _dev()
+    g = torch.Generator(dev).manual_seed(m + n)
+    pad, pm = (n + 7) // 8 * 8, (m + 7) // 8 * 8
+    a = torch.randn(5, k, pm, device=dev, generator=g).to(torch.bfloat16)
+    b = torch.randn(5, k, pad, device=dev, generator=g).to(torch.bfloat16)
+    d = torch.full((5, m, n), 3.0 if acc else float("nan"), device=dev)
+    gemm(m, n, k, Operand(a, ld=pm, mn_major=True, zs_hi=k * pm), Operand(b, ld=pad, mn_major=True, zs_hi=k * pad),
+         Output(d, rs_lo=n, d_zhi=m * n), zhi_n=5, accumulate=acc)
+    _ext.check_device_errors(dev)
+    ref = torch.einsum("zkm,zkn->zmn", a[..., :m].double(), b[..., :n].double()) + (3.0 if acc else 0.0)
+    assert _rel(d, ref) < 2.0 ** -24 * max(k, 64) ** 0.5 * 4
