@@ -60,7 +60,7 @@ void clear_error_flag(int64_t device) {
 
 inline const char* base_ptr(const Tensor& t) { return static_cast<const char*>(t.data_ptr()); }
 
-// iparams layout: see makani_b200/ops/gemm.py (GemmSpec.pack)
+// iparams layout: see makani_b200/ops/gemm.py
 static bool parse_peer(mk::GemmPeer& g, const std::vector<int64_t>& seg, const std::vector<int64_t>& sync) {
   memset(&g, 0, sizeof(g));
   if (!seg.empty()) {
@@ -298,6 +298,65 @@ void cast_pad(const Tensor& x, Tensor& y) {
   check_cuda(mk::cast_pad_bf16(x.data_ptr<float>(), reinterpret_cast<__nv_bfloat16*>(y.data_ptr()), x.size(0), static_cast<int>(x.size(1)),
                                static_cast<int>(y.size(1)), cur_stream()),
              "cast_pad");
+}
+
+// Complex product of planar operands (GemmProblem::cplx); integer parameters in the order of `gemm_complex` in ops/gemm.py
+void gemm_complex(const Tensor& a, const Tensor& b, Tensor& d, const c10::optional<Tensor>& resid, const std::vector<int64_t>& ip) {
+  MK_CHECK(ip.size() == 27, "gemm_complex: expected 27 integer parameters, got ", ip.size());
+  MK_CHECK(a.is_cuda() && b.is_cuda() && d.is_cuda() && a.scalar_type() == torch::kBFloat16 && b.scalar_type() == torch::kBFloat16,
+           "gemm_complex: bf16 CUDA operands expected");
+  MK_CHECK(d.scalar_type() == torch::kBFloat16 || d.scalar_type() == torch::kFloat32, "gemm_complex: output must be bf16 or fp32");
+  c10::cuda::CUDAGuard guard(a.device());
+  int k = 0;
+  mk::GemmProblem p;
+  memset(&p, 0, sizeof(p));
+  p.cplx = static_cast<int>(ip[k++]);
+  MK_CHECK(p.cplx >= 1 && p.cplx <= 3, "gemm_complex: bad mode");
+  p.M = ip[k++]; p.N = ip[k++]; p.K = ip[k++];
+  p.zlo_n = ip[k++]; p.zhi_n = ip[k++];
+  p.elem_bytes = 2;
+  p.splits = 1;
+  p.rmax_a = ip[k++]; p.rmax_b = ip[k++]; p.kmax_a = ip[k++]; p.kmax_b = ip[k++];
+  MK_CHECK(p.cplx != 3 || p.zlo_n == 1, "gemm_complex: one batch of weight gradients per call");
+  mk::GemmOperand A, B;
+  const int64_t a_off = ip[k++];
+  A.rows = p.M; A.mn_major = ip[k++]; A.ld = ip[k++]; A.zs_lo = ip[k++]; A.zs_hi = ip[k++]; p.a_plane = ip[k++];
+  const int64_t b_off = ip[k++];
+  B.rows = p.N; B.mn_major = ip[k++]; B.ld = ip[k++]; B.zs_lo = 0; B.zs_hi = ip[k++]; p.b_plane = ip[k++];
+  A.ptr = base_ptr(a) + a_off * 2;
+  B.ptr = base_ptr(b) + b_off * 2;
+  const int64_t ka = p.cplx == 3 ? p.K : 2 * static_cast<int64_t>(p.K);
+  check_extent(a, a_off, {{A.mn_major ? ka : p.M, A.ld}, {A.mn_major ? p.M : ka, 1}, {p.zlo_n, A.zs_lo}, {p.zhi_n, A.zs_hi},
+                          {p.cplx == 3 ? 2 : 1, p.a_plane}}, "A");
+  check_extent(b, b_off, {{B.mn_major ? p.K : p.N, B.ld}, {B.mn_major ? p.N : p.K, 1}, {p.zhi_n, B.zs_hi}, {2, p.b_plane}}, "B");
+  mk::GemmEpilogue e;
+  memset(&e, 0, sizeof(e));
+  const int64_t d_off = ip[k++];
+  const int osz = static_cast<int>(d.element_size());
+  e.D = const_cast<char*>(base_ptr(d)) + d_off * osz;
+  e.out_f32 = d.scalar_type() == torch::kFloat32;
+  e.rs_lo = ip[k++]; e.d_half = ip[k++]; e.d_zlo = ip[k++]; e.d_zhi = ip[k++];
+  e.accumulate = ip[k++];
+  MK_CHECK(e.d_half > 0, "gemm_complex: the parts of the output must be apart");
+  check_extent(d, d_off, {{p.zhi_n, e.d_zhi}, {p.zlo_n, e.d_zlo}, {p.M, e.rs_lo}, {2, e.d_half}, {p.N, 1}}, "output");
+  e.alpha = 1.f;
+  if (resid.has_value() && resid->defined()) {
+    MK_CHECK(resid->scalar_type() == d.scalar_type() && resid->sizes() == d.sizes() && resid->strides() == d.strides() && d_off == 0,
+             "gemm_complex: residual must be laid out like the output");
+    e.resid = base_ptr(*resid);
+  }
+  Tensor ef = err_flag_for(a);
+  check_cuda(mk::gemm_launch(p, A, B, e, ef.data_ptr<int>(), cur_stream(), nullptr), "gemm_complex launch");
+}
+
+// real and imaginary planes of w (complex64 [Cin, Cout, L]) -> bf16 [L, 2, Cout, Cin]
+void spectral_planes(const Tensor& w, Tensor& wp) {
+  MK_CHECK(w.is_cuda() && w.scalar_type() == torch::kComplexFloat && w.is_contiguous() && w.dim() == 3, "spectral_planes: bad weight");
+  MK_CHECK(wp.is_cuda() && wp.scalar_type() == torch::kBFloat16 && wp.is_contiguous() && wp.numel() == 2 * w.numel(), "spectral_planes: bad output");
+  c10::cuda::CUDAGuard guard(w.device());
+  check_cuda(mk::spectral_expand(reinterpret_cast<const float*>(w.data_ptr()), reinterpret_cast<__nv_bfloat16*>(wp.data_ptr()),
+                                 static_cast<int>(w.size(0)), static_cast<int>(w.size(1)), static_cast<int>(w.size(2)), cur_stream(), 1),
+             "spectral_planes");
 }
 
 // sums of do2 [outer, groups, inner, C] over outer and inner -> out [groups, C]
@@ -636,6 +695,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("inorm_fwd", &inorm_fwd);
   m.def("inorm_partial_stats", &inorm_partial_stats);
   m.def("cast_pad", &cast_pad);
+  m.def("gemm_complex", &gemm_complex);
+  m.def("spectral_planes", &spectral_planes);
   m.def("colsum", &colsum);
   m.def("colsum_groups", &colsum_groups);
   m.def("afno_pack", &afno_pack);

@@ -992,7 +992,8 @@ __global__ void __launch_bounds__(256) afno_fold_kernel(const AfnoGrad a, const 
 // ------------------------------------------------------------------------------------------ spectral weights
 
 // grid: (Cin/32, Cout, ceil(L/32)); block 32x8
-__global__ void spectral_expand_kernel(const float2* __restrict__ w, __nv_bfloat16* __restrict__ wx, int Cin, int Cout, int L) {
+__global__ void spectral_expand_kernel(const float2* __restrict__ w, __nv_bfloat16* __restrict__ wx, int Cin, int Cout, int L,
+                                       int planar) {
   __shared__ float2 tile[32][33];
   const int c0 = blockIdx.x * 32, o = blockIdx.y, l0 = blockIdx.z * 32;
   for (int j = threadIdx.y; j < 32; j += 8) {
@@ -1006,7 +1007,13 @@ __global__ void spectral_expand_kernel(const float2* __restrict__ w, __nv_bfloat
     const int l = l0 + j, c = c0 + threadIdx.x;
     if (l < L && c < Cin) {
       const float2 v = tile[threadIdx.x][j];
-      // planar 2x2-block form: rows (ri', o), columns (ri, c):  [[Wr, -Wi], [Wi, Wr]]
+      if (planar) {
+        __nv_bfloat16* q = wx + (static_cast<long long>(l) * 2 * Cout + o) * Cin + c;
+        q[0] = __float2bfloat16(v.x);
+        q[static_cast<long long>(Cout) * Cin] = __float2bfloat16(v.y);
+        continue;
+      }
+      // 2x2-block form: rows (ri', o), columns (ri, c):  [[Wr, -Wi], [Wi, Wr]]
       __nv_bfloat16* base = wx + static_cast<long long>(l) * 4 * Cout * Cin;
       const long long r0 = static_cast<long long>(o) * 2 * Cin, r1 = static_cast<long long>(Cout + o) * 2 * Cin;
       base[r0 + c] = __float2bfloat16(v.x);
@@ -1023,7 +1030,7 @@ __global__ void spectral_expand_kernel(const float2* __restrict__ w, __nv_bfloat
 // grid: (ceil(Cin / 64), Cout, ceil(L / 32)); 256 threads
 constexpr int SX_PITCH = 64 + 8;      // bf16 per tile row (16-byte aligned rows)
 __global__ void __launch_bounds__(256) spectral_expand_vec_kernel(const float2* __restrict__ w, __nv_bfloat16* __restrict__ wx,
-                                                                  int Cin, int Cout, int L) {
+                                                                  int Cin, int Cout, int L, int planar) {
   __shared__ __align__(16) __nv_bfloat16 re[32 * SX_PITCH], im[32 * SX_PITCH];
   const int c0 = blockIdx.x * 64, o = blockIdx.y, l0 = blockIdx.z * 32;
   const int lp = (threadIdx.x & 15) * 2, cp = (threadIdx.x >> 4) * 2;     // two degrees, two channels (then + 32)
@@ -1050,6 +1057,12 @@ __global__ void __launch_bounds__(256) spectral_expand_vec_kernel(const float2* 
   if (l0 + l < L && c0 + cv < Cin) {
     const uint4 r = *reinterpret_cast<const uint4*>(re + l * SX_PITCH + cv);
     const uint4 i = *reinterpret_cast<const uint4*>(im + l * SX_PITCH + cv);
+    if (planar) {
+      __nv_bfloat16* q = wx + (static_cast<long long>(l0 + l) * 2 * Cout + o) * Cin + c0 + cv;
+      *reinterpret_cast<uint4*>(q) = r;
+      *reinterpret_cast<uint4*>(q + static_cast<long long>(Cout) * Cin) = i;
+      return;
+    }
     const uint4 n = make_uint4(i.x ^ 0x80008000u, i.y ^ 0x80008000u, i.z ^ 0x80008000u, i.w ^ 0x80008000u);
     __nv_bfloat16* base = wx + static_cast<long long>(l0 + l) * 4 * Cout * Cin + c0 + cv;
     const long long r0 = static_cast<long long>(o) * 2 * Cin, r1 = static_cast<long long>(Cout + o) * 2 * Cin;
@@ -1401,14 +1414,14 @@ cudaError_t adamw_step(const AdamEntry* table, const int* chunk_tensor, const lo
   return cudaGetLastError();
 }
 
-cudaError_t spectral_expand(const float* w, __nv_bfloat16* wx, int Cin, int Cout, int L, cudaStream_t s) {
+cudaError_t spectral_expand(const float* w, __nv_bfloat16* wx, int Cin, int Cout, int L, cudaStream_t s, int planar) {
   if ((L & 1) == 0 && (Cin & 7) == 0 && aligned16(w) && aligned16(wx)) {
     spectral_expand_vec_kernel<<<dim3((Cin + 63) / 64, Cout, (L + 31) / 32), 256, 0, s>>>(reinterpret_cast<const float2*>(w), wx,
-                                                                                          Cin, Cout, L);
+                                                                                          Cin, Cout, L, planar);
     return cudaGetLastError();
   }
   dim3 grid((Cin + 31) / 32, Cout, (L + 31) / 32), block(32, 8);
-  spectral_expand_kernel<<<grid, block, 0, s>>>(reinterpret_cast<const float2*>(w), wx, Cin, Cout, L);
+  spectral_expand_kernel<<<grid, block, 0, s>>>(reinterpret_cast<const float2*>(w), wx, Cin, Cout, L, planar);
   return cudaGetLastError();
 }
 

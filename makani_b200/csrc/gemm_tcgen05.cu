@@ -18,6 +18,15 @@
 // "stage free" and "accumulator full" signals to both CTAs.  Per tensor-core cycle every SM then takes a third less
 // data from L2 (two thirds with 128-wide tiles), which is what bounds these GEMMs.
 //
+// Complex products (p.cplx): real and imaginary planes of the operands are multiplied without ever forming the real 2x2-block
+// matrix.  The column tiles come in two halves (real, imaginary part of the result) and the k loop in two segments that
+// select the planes; the one negative product of the four uses the negation bit of the MMA's instruction descriptor.
+//   1: D(h) = sum_s A[.., s Kh + k] B(plane h ^ s),  minus at h = 0, s = 1      (product with W)
+//   2: the same, minus at h = 1, s = 0                                          (product with the conjugate of W)
+//   3: D(h) = sum_s A(plane s ^ h) B(plane s),       minus at h = 1, s = 1      (weight gradient)
+// 384 x 384 weights of 240 degrees: the operand takes 69 us to make instead of 95 (half the bytes), the products 87 - 94 us instead
+// of 105 - 114, the weight gradient one launch of 90 us instead of two of 78 and a swapped copy of 31.
+//
 // Multi-GPU use (one process per GPU, buffers mapped through CUDA IPC):
 //   * the k axis of the B operand may be cut into up to 8 segments with their own base pointers and tensor maps
 //     (the per-rank segments of a gathered buffer in this device's own memory);
@@ -108,6 +117,7 @@ struct KParams {
   int m_tiles, n_tiles;
   FastDiv dv_n, dv_m, dv_split, dv_zlo;
   uint32_t total_tiles;           // below 2^31
+  int cplx, nth, neg_half, neg_seg;   // complex product: mode, column tiles per half, the negative (half, segment)
   int zred, zhi_all;              // z_hi batches summed inside one tile (1: none), and their number
   int stages, e_tma;
   int d_zlo_on, d_zhi_on;         // fp32 output through TMA: 0 where all batches of that index add into one output
@@ -213,21 +223,23 @@ __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// Output and epilogue-operand maps are (column, r % rdiv, r / rdiv, z_lo, z_hi): a box starts at a multiple of rdiv rows.
-__device__ __forceinline__ void tma_store_tile(const CUtensorMap* map, uint32_t src, int n, int r, int zlo, int zhi) {
+// Output and epilogue-operand maps are (column, r % rdiv, r / rdiv, z_lo, z_hi): a box starts at a multiple of rdiv rows.  Complex
+// products: the second index is the half.
+__device__ __forceinline__ void tma_store_tile(const CUtensorMap* map, uint32_t src, int n, int lo, int r, int zlo, int zhi) {
   asm volatile("cp.async.bulk.tensor.5d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5, %6}], [%1];" ::"l"(map), "r"(src),
-               "r"(n), "r"(0), "r"(r), "r"(zlo), "r"(zhi)
+               "r"(n), "r"(lo), "r"(r), "r"(zlo), "r"(zhi)
                : "memory");
 }
-__device__ __forceinline__ void tma_add_tile(const CUtensorMap* map, uint32_t src, int n, int r, int zlo, int zhi) {
+__device__ __forceinline__ void tma_add_tile(const CUtensorMap* map, uint32_t src, int n, int lo, int r, int zlo, int zhi) {
   asm volatile("cp.reduce.async.bulk.tensor.5d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4, %5, %6}], [%1];" ::"l"(map),
-               "r"(src), "r"(n), "r"(0), "r"(r), "r"(zlo), "r"(zhi)
+               "r"(src), "r"(n), "r"(lo), "r"(r), "r"(zlo), "r"(zhi)
                : "memory");
 }
-__device__ __forceinline__ void tma_load_tile(uint32_t dst, const CUtensorMap* map, uint32_t bar, int n, int r, int zlo, int zhi) {
+__device__ __forceinline__ void tma_load_tile(uint32_t dst, const CUtensorMap* map, uint32_t bar, int n, int lo, int r, int zlo,
+                                              int zhi) {
   asm volatile(
       "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
-      ::"r"(dst), "l"(map), "r"(bar), "r"(n), "r"(0), "r"(r), "r"(zlo), "r"(zhi)
+      ::"r"(dst), "l"(map), "r"(bar), "r"(n), "r"(lo), "r"(r), "r"(zlo), "r"(zhi)
       : "memory");
 }
 __device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
@@ -317,6 +329,7 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t lbo_bytes
 
 struct TileCoord {
   int zhi, zlo, split, mt, nt;
+  int half;             // complex products: real (0) or imaginary (1) part; nt counts the column tiles inside the half
   int k_begin, k_end;   // element range, k_begin multiple of BK
   bool skip;
 };
@@ -342,6 +355,8 @@ __device__ __forceinline__ TileCoord decode_tile(const KParams& p, uint32_t t, i
     c.mt = take(p.dv_m);
     c.nt = take(p.dv_n);
   }
+  c.half = p.cplx != 0 && c.nt >= p.nth ? 1 : 0;
+  c.nt -= c.half * p.nth;
   c.split = take(p.dv_split);
   c.zlo = take(p.dv_zlo);
   c.zhi = static_cast<int>(t);
@@ -511,14 +526,20 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
         const TileCoord c = decode_tile<BK, CG>(p, t, crank);
         const int m0 = c.mt * BM, n0 = c.nt * BN;
         if (c.skip) continue;
-        const int azl = p.a_zlo ? c.zlo : 0, bzl = p.b_zlo ? c.zlo : 0;
-        for (int sg = 0; sg < p.nseg && ok; ++sg) {
+        int azl = p.a_zlo ? c.zlo : 0, bzl = p.b_zlo ? c.zlo : 0;
+        const int nsg = p.cplx ? 2 : p.nseg;
+        for (int sg = 0; sg < nsg && ok; ++sg) {
           int lb = c.k_begin, le = c.k_end, apos = 0;
           const CUtensorMap* mb = &map_b;
           if (p.nseg > 1) {
             seg_range<BK>(p, c, sg, lb, le);
             apos = p.seg_apos[sg];
             mb = &maps_b.m[sg];
+          } else if (p.cplx) {
+            // segment and half select the planes, which take the place of the lower batch index
+            bzl = p.cplx == 3 ? sg : (sg ^ c.half);
+            if (p.cplx == 3) azl = sg ^ c.half;
+            else apos = sg * p.K;
           }
           // (with batches summed inside the tile the k loop runs over all of them)
           const int zr_n = p.zred > 1 ? min(p.zred, p.zhi_all - c.zhi * p.zred) : 1;
@@ -600,7 +621,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
         mbar_expect_tx(efull_bar(eb), E_BYTES);
 #pragma unroll
         for (int j = 0; j < BN / 64; ++j)
-          tma_load_tile(smem_base + e_off + eb * E_BYTES + j * (BM * 128), &map_e, efull_bar(eb), c.nt * BN + j * 64,
+          tma_load_tile(smem_base + e_off + eb * E_BYTES + j * (BM * 128), &map_e, efull_bar(eb), c.nt * BN + j * 64, c.half,
                         (c.mt * BM) >> p.rd_shift, c.zlo, c.zhi);
         ++epi_it;
       }
@@ -640,9 +661,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
           }
         } else {
           nblocks = (c.k_end - c.k_begin + BK - 1) / BK;
+          if (p.cplx) nblocks *= 2;
           if (p.zred > 1) nblocks *= min(p.zred, p.zhi_all - c.zhi * p.zred);
         }
+        // the negative product of a complex one: bit 14 of the instruction descriptor negates B
+        const bool neg_half = p.cplx != 0 && c.half == p.neg_half;
         for (int kb = 0; kb < nblocks; ++kb) {
+          const uint32_t neg = neg_half && (2 * kb >= nblocks ? 1 : 0) == p.neg_seg ? 1u << 14 : 0u;
           if (!mbar_wait(full_bar(s), ph)) {
             atomicExch(p.err, 3);
             ok = false;
@@ -655,7 +680,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
           for (int kk = 0; kk < BK / UMMA_K; ++kk) {
             const uint64_t da = make_desc(sa + kk * a_kstep, a_lbo, a_sbo);
             const uint64_t db = make_desc(sb + kk * b_kstep, b_lbo, b_sbo);
-            tc_mma<EB, CG>(tmem_d, da, db, idesc, accum);
+            tc_mma<EB, CG>(tmem_d, da, db, idesc | neg, accum);
             accum = 1;
           }
           // frees the smem stage (in both CTAs of a pair) once these MMAs have read it
@@ -747,8 +772,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
           __syncwarp();
           if (lane == 0 && r0 < p.M) {
             const int zl = p.d_zlo_on ? c.zlo : 0, zh = p.d_zhi_on ? c.zhi : 0;
-            if (p.accumulate) tma_add_tile(&map_d, smem_base + box_off, nb, r0 >> p.rd_shift, zl, zh);
-            else tma_store_tile(&map_d, smem_base + box_off, nb, r0 >> p.rd_shift, zl, zh);
+            if (p.accumulate) tma_add_tile(&map_d, smem_base + box_off, nb, c.half, r0 >> p.rd_shift, zl, zh);
+            else tma_store_tile(&map_d, smem_base + box_off, nb, c.half, r0 >> p.rd_shift, zl, zh);
             tma_store_commit();
           }
         }
@@ -874,11 +899,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
           const int r0 = c.mt * BM + q * 32;
           if (lane == 0 && r0 < p.M) {
             const int rs = r0 >> p.rd_shift;
-            if constexpr (EPI == 2) tma_store_tile(&map_p, smem_base + box_off - 32 * 128, nb, rs, c.zlo, c.zhi);
-            tma_store_tile(&map_d, smem_base + box_off, nb, rs, c.zlo, c.zhi);
+            if constexpr (EPI == 2) tma_store_tile(&map_p, smem_base + box_off - 32 * 128, nb, 0, rs, c.zlo, c.zhi);
+            tma_store_tile(&map_d, smem_base + box_off, nb, c.half, rs, c.zlo, c.zhi);
             if constexpr (EPI == 1) {
               for (int dq = 0; dq < p.ndx; ++dq)   // the same box goes to every peer's copy (plain stores over NVLink)
-                tma_store_tile(&maps_dx.m[dq], smem_base + box_off, nb, rs, c.zlo, c.zhi);
+                tma_store_tile(&maps_dx.m[dq], smem_base + box_off, nb, 0, rs, c.zlo, c.zhi);
             }
             tma_store_commit();
             if constexpr (IN_PLACE) tma_store_wait_read<0>();   // the operand buffer is free once the store has read it
@@ -1238,8 +1263,9 @@ cudaError_t launch_t(const CUtensorMap& ma, const BMaps& mb, const CUtensorMap& 
 
 // Tensor map of an output or epilogue operand: [M rows][N contiguous] bf16 with two batch dimensions, 128-byte swizzle.  Rows
 // may be split, r = hi * rd + lo with rd a power of two that divides M and 32: a box is then 32 (or 128) / rd by rd rows.
+// With `halves` the second dimension is not part of the rows: two results `halves` elements apart (complex products).
 bool make_map_e(CUtensorMap* map, const void* ptr, int M, int N, int rd, long long rs_hi, long long rs_lo, long long zs_lo,
-                long long zs_hi, int zlo_n, int zhi_n, int box_rows = BM, int ob = 2) {
+                long long zs_hi, int zlo_n, int zhi_n, int box_rows = BM, int ob = 2, long long halves = 0) {
   EncodeTiledFn enc = get_encode();
   if (!enc) return false;
   const long long row_stride = rd > 1 ? rs_hi : rs_lo;
@@ -1251,6 +1277,10 @@ bool make_map_e(CUtensorMap* map, const void* ptr, int M, int N, int rd, long lo
   // one 128-byte swizzle row: 64 bf16 or 32 fp32
   cuuint32_t box[5] = {static_cast<cuuint32_t>(128 / ob), static_cast<cuuint32_t>(rd), static_cast<cuuint32_t>(box_rows / rd), 1, 1};
   cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  if (halves > 0) {
+    dims[1] = 2;
+    strides[0] = static_cast<cuuint64_t>(halves) * ob;
+  }
   if ((reinterpret_cast<uintptr_t>(ptr) & 15) || (strides[0] & 15) || (strides[1] & 15) || (strides[2] & 15) || (strides[3] & 15))
     return false;
   CUresult r = enc(map, ob == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5, const_cast<void*>(ptr), dims,
@@ -1607,7 +1637,7 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
   const bool plain = (one_stride || split_ok) && (e.ndiv <= 0 || e.ndiv >= (1 << 30));
   const int rd = one_stride ? 1 : e.rdiv;
   auto tile_map = [&](CUtensorMap* m, const void* ptr, int box_rows) {
-    return make_map_e(m, ptr, p.M, p.N, rd, e.rs_hi, e.rs_lo, e.d_zlo, e.d_zhi, p.zlo_n, p.zhi_n, box_rows);
+    return make_map_e(m, ptr, p.M, p.N, rd, e.rs_hi, e.rs_lo, e.d_zlo, e.d_zhi, p.zlo_n, p.zhi_n, box_rows, 2, e.d_half);
   };
   kp.rd_shift = 0;
   while (plain && (1 << kp.rd_shift) < rd) ++kp.rd_shift;
@@ -1643,7 +1673,8 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
       e.d_zlo >= 0 && e.d_zhi >= 0 && (e.accumulate || ((e.d_zlo > 0 || p.zlo_n == 1) && (e.d_zhi > 0 || p.zhi_n == 1)))) {
     kp.d_zlo_on = e.d_zlo > 0;
     kp.d_zhi_on = e.d_zhi > 0;
-    if (make_map_e(&md, e.D, p.M, p.N, rd, e.rs_hi, e.rs_lo, e.d_zlo, e.d_zhi, kp.d_zlo_on ? p.zlo_n : 1, kp.d_zhi_on ? p.zhi_n : 1, 32, 4))
+    if (make_map_e(&md, e.D, p.M, p.N, rd, e.rs_hi, e.rs_lo, e.d_zlo, e.d_zhi, kp.d_zlo_on ? p.zlo_n : 1, kp.d_zhi_on ? p.zhi_n : 1, 32, 4,
+                   e.d_half))
       epi = 5;
   }
   // CTA pairs (256-row tiles, each CTA loads half of the B tile): single-device bf16 launches without row-triangular
@@ -1658,13 +1689,24 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
   }();
   const bool no_peer = (peer == nullptr) || (peer->nseg <= 1 && peer->ndx == 0 && peer->nwait == 0 && peer->nsig == 0 &&
                                               peer->done_ctr == nullptr);
-  const bool eligible = eb == 2 && no_peer && p.M > BM && p.rmin_a == 0 && p.rmax_a == 0;
+  const bool eligible = eb == 2 && no_peer && p.M > BM && p.rmin_a == 0 && p.rmax_a == 0 && (p.cplx == 0 || p.cplx == 3);
   const int cg = (eligible && (pairs_mode == 1 || (pairs_mode == 2 && p.K >= 512))) ? 2 : 1;
   if (bn == 0) bn = pick_bn(p.N, epi, kp.e_tma);
   if ((eb == 4 && bn == 192) || ((epi == 3 || epi == 4 || kp.e_tma) && bn == 256)) bn = 128;
   if (epi == 0 && kp.e_tma) bn = 128;
   kp.m_tiles = (p.M + BM * cg - 1) / (BM * cg);
   kp.n_tiles = (p.N + bn - 1) / bn;
+  kp.cplx = p.cplx;
+  kp.nth = kp.n_tiles;
+  kp.neg_half = p.cplx == 1 ? 0 : 1;
+  kp.neg_seg = p.cplx == 2 ? 0 : 1;
+  if (p.cplx) {
+    if (eb != 2 || (epi != 1 && epi != 3 && epi != 5) || kp.splits != 1 || p.splits == 0 || kp.nseg != 1 || rd != 1) {
+      snprintf(g_err, sizeof(g_err), "complex product: bf16 operands, plain rows, aligned output with or without residual");
+      return cudaErrorInvalidValue;
+    }
+    kp.n_tiles *= 2;
+  }
   // Batches that add into one output (d_zhi = 0) are summed inside the tiles as far as the SMs stay busy: 728 products of
   // 192 x 192 with 90 summands each spent their time in 107 MB of fp32 atomics (44 us, now 29).
   const int slots = cg == 2 ? max_pairs() : sm_count();
@@ -1691,7 +1733,11 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
   kp.dv_m = make_div(kp.m_tiles);
   kp.dv_split = make_div(kp.splits);
   kp.dv_zlo = make_div(p.zlo_n);
-  if (!make_map(&ma, A, p.K, eb, p.zlo_n, p.zhi_n, BM)) return cudaErrorInvalidValue;
+  // planes take the place of the lower batch index
+  GemmOperand Am = A, Bm = B;
+  if (p.cplx) Bm.zs_lo = p.b_plane;
+  if (p.cplx == 3) Am.zs_lo = p.a_plane;
+  if (!make_map(&ma, Am, p.cplx && p.cplx != 3 ? 2 * p.K : p.K, eb, p.cplx == 3 ? 2 : p.zlo_n, p.zhi_n, BM)) return cudaErrorInvalidValue;
   const int bn_box = bn / cg;     // rows of a K-major B one CTA loads per stage
   BMaps mbs;
   if (kp.nseg > 1) {
@@ -1702,7 +1748,7 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
     }
     for (int q = kp.nseg; q < MAX_SEG; ++q) mbs.m[q] = mbs.m[0];
   } else {
-    if (!make_map(&mb, B, p.K, eb, p.zlo_n, p.zhi_n, bn_box)) return cudaErrorInvalidValue;
+    if (!make_map(&mb, Bm, p.K, eb, p.cplx ? 2 : p.zlo_n, p.zhi_n, bn_box)) return cudaErrorInvalidValue;
     for (int q = 0; q < MAX_SEG; ++q) mbs.m[q] = mb;
   }
   if (!kp.e_tma) me = ma;   // unused, but must be a valid descriptor

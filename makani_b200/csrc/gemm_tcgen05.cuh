@@ -52,6 +52,7 @@ struct GemmEpilogue {
                         // addressing and dtype as D
   // optional second output: the pre-activation value (alpha*acc + bias) in the same layout / dtype
   void* preact;
+  long long d_half = 0; // complex products: elements between the real and the imaginary part of the output (and of `resid`)
 };
 
 struct GemmProblem {
@@ -61,6 +62,10 @@ struct GemmProblem {
   int splits;           // split-k factor (requires accumulate; 0: chosen here)
   int rmin_a, rmin_b, rmax_a, rmax_b;   // valid rows [rmin_a*z_hi+rmin_b, rmax_a*z_hi+rmax_b)
   int kmin_a, kmin_b, kmax_a, kmax_b;   // contributing k range
+  // Complex products of planar operands (0: none; modes in gemm_tcgen05.cu): N and K are those of one part; `b_plane` (and for
+  // mode 3 `a_plane`) elements between the real and imaginary planes; for modes 1 and 2 the parts of A follow one another in k
+  int cplx = 0;
+  long long a_plane = 0, b_plane = 0;
   int bn;               // tile width: 128, 192 or 256 (0 = choose)
 };
 

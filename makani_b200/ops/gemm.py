@@ -223,6 +223,23 @@ def gemm(M: int, N: int, K: int, A: Operand, B: Operand, D: Output, *, zlo_n: in
     ext.gemm(A.tensor, B.tensor, D.tensor, bias, resid, preact, ip, float(alpha))
 
 
+def gemm_complex(mode: int, M: int, N: int, K: int, A: Operand, B: Operand, D: Output, d_half: int, *, zlo_n: int = 1, zhi_n: int = 1,
+                 a_plane: int = 0, b_plane: int = 0, resid=None, accumulate: bool = False, rmax=(0, _BIG), kmax=(0, _BIG)) -> None:
+    """Product of complex operands given as real and imaginary planes (CUDA bf16; N and K count one part):
+
+        mode 1   D(h)[r, n] = sum_s sum_k A[r, s K + k] B(h ^ s)[n, k],   minus for h = 0, s = 1:  A times W
+        mode 2   the same, minus for h = 1, s = 0:                                                A times conj(W)
+        mode 3   D(h)[r, n] = sum_s sum_k A(s ^ h)[r, k] B(s)[n, k],      minus for h = 1, s = 1:  sum over k of A conj(B)
+
+    `b_plane` / `a_plane`: elements between the planes of an operand; `d_half`: between the parts of D.  `rmax`, `kmax`: (slope,
+    offset) of the valid rows / contributing k in the batch index z_hi, as in `Tri`.  `resid` is laid out like D and added."""
+    ip = [mode, M, N, K, zlo_n, zhi_n, rmax[0], rmax[1], kmax[0], kmax[1],
+          A.offset, int(A.mn_major), A.ld, A.zs_lo, A.zs_hi, a_plane,
+          B.offset, int(B.mn_major), B.ld, B.zs_hi, b_plane,
+          D.offset, D.rs_lo, d_half, D.d_zlo, D.d_zhi, int(accumulate)]
+    _ext.require().gemm_complex(A.tensor, B.tensor, D.tensor, resid, ip)
+
+
 def _f32_bits(x: float) -> int:
     import struct
     return struct.unpack("<I", struct.pack("<f", float(x)))[0]

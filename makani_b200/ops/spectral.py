@@ -9,7 +9,7 @@ truncation pass ever touches HBM:
     x  [B, H, W, C]                  real grid data, channels-last (bf16)
     S1 longitude DFT      -> T1 [B, H, (m,ri), C]       A = DFT matrix [(m,ri), W], batched over latitude rows
     S2 Legendre analysis  -> T2 [B, l, m, (ri, C)]      A = P_l^m(theta_k) w_k, batched over m, rows l < m skipped
-    S3 complex contraction-> T3 [B, m, l, (ri, Co)]     B = W_l as a real 2x2-block matrix, batched over l, rows m > l skipped
+    S3 complex contraction-> T3 [B, m, l, (ri, Co)]     B = real and imaginary planes of W_l, batched over l, rows m > l skipped
     S4 Legendre synthesis -> T4 [B, H', (m,ri), Co]     k-loop restricted to l >= m
     S5 inverse DFT        -> y  [B, H', W', Co]
 
@@ -31,7 +31,7 @@ from ..sht.legendre import legendre_table
 from ..sht.quadrature import precompute_latitudes
 from . import _ext
 from .conv import records_grad
-from .gemm import Operand, Output, Tri, gemm, pad_to
+from .gemm import Operand, Output, Tri, gemm, gemm_complex, pad_to
 
 
 class SHTPlan:
@@ -154,8 +154,19 @@ def legendre_synthesis(t: torch.Tensor, lm_order: bool, table: torch.Tensor, H: 
 def contract(t2: torch.Tensor, wx: torch.Tensor, transpose_w: bool, resid=None) -> torch.Tensor:
     """T3[b, m, l, q] = sum_p T2[b, l, m, p] Wx[l, q, p]   (transpose_w False; Wx [l, 2Co, 2Ci])
        T3[b, m, l, p] = sum_q T2[b, l, m, q] Wx[l, q, p]   (transpose_w True: adjoint w.r.t. the input)
-    plus `resid`, which has the layout of the result."""
+    plus `resid`, which has the layout of the result.  Wx is the real block form or the planes of `weight_planes`."""
     B, lmax, mmax, kin = t2.shape
+    if wx.dim() == 4:
+        # planes [l, 2, Co, Ci]: half the bytes of the real block matrix, in memory and through L2
+        co, ci = wx.shape[2], wx.shape[3]
+        n, k = (ci, co) if transpose_w else (co, ci)
+        t3 = torch.empty(B, mmax, lmax, 2 * n, dtype=t2.dtype, device=t2.device)
+        gemm_complex(2 if transpose_w else 1, mmax, n, k,
+                     Operand(t2, ld=kin, zs_hi=mmax * kin, zs_lo=lmax * mmax * kin),
+                     Operand(wx, ld=ci, mn_major=transpose_w, zs_hi=2 * co * ci),
+                     Output(t3, rs_lo=lmax * 2 * n, d_zhi=2 * n, d_zlo=mmax * lmax * 2 * n), n, zhi_n=lmax, zlo_n=B,
+                     b_plane=co * ci, resid=resid, rmax=(1, 1))
+        return t3
     nq, npp = wx.shape[1], wx.shape[2]
     nout = npp if transpose_w else nq
     t3 = torch.empty(B, mmax, lmax, nout, dtype=t2.dtype, device=t2.device)
@@ -172,10 +183,20 @@ def contract_wgrad2(dt: torch.Tensor, t2: torch.Tensor, l0: int = 0, m0: int = 0
 
         dWr[l, o, c] = sum_{b, m <= l} dTr T2r + dTi T2i        dWi[l, o, c] = sum_{b, m <= l} dTi T2r - dTr T2i
 
-    Both are GEMMs over k = (m, ri) (the two parts sit side by side in memory); the second one reads a copy of dT
-    with its parts swapped and one sign flipped.  `l0`, `m0`: global offsets of the local (l, m) block."""
+    On CUDA one complex product over the planes of both operands.  Otherwise both are GEMMs over k = (m, ri) (the two parts sit
+    side by side in memory); the second one reads a copy of dT with its parts swapped and one sign flipped.  `l0`, `m0`:
+    global offsets of the local (l, m) block."""
     B, L, M, nq = dt.shape
     co, ci = nq // 2, t2.shape[3] // 2
+    if dt.is_cuda and dt.dtype == torch.bfloat16 and co % 8 == 0 and ci % 8 == 0 and dt.is_contiguous() and t2.is_contiguous() and _ext.native():
+        out = (torch.empty if B == 1 else torch.zeros)(2, L, co, ci, dtype=torch.float32, device=dt.device)
+        for b in range(B):
+            gemm_complex(3, co, ci, M,
+                         Operand(dt, ld=nq, mn_major=True, zs_hi=M * nq, offset=b * L * M * nq),
+                         Operand(t2, ld=2 * ci, mn_major=True, zs_hi=M * 2 * ci, offset=b * L * M * 2 * ci),
+                         Output(out, rs_lo=ci, d_zhi=co * ci), L * co * ci, zhi_n=L, a_plane=co, b_plane=ci, accumulate=(B > 1),
+                         kmax=(1, 1 + l0 - m0))
+        return out
     if dt.is_cuda and dt.dtype == torch.bfloat16 and co % 8 == 0 and dt.is_contiguous() and _ext.native():
         dts = torch.empty_like(dt)
         _ext.require().swap_ri(dt, dts, co)
@@ -223,13 +244,29 @@ def expand_weight(w: torch.Tensor, dtype=torch.bfloat16, keep: bool = False) -> 
     """complex [Ci, Co, L] -> real [L, 2Co, 2Ci] with rows (ri', o), columns (ri, c):  [[Wr, -Wi], [Wi, Wr]].
 
     `keep`: the caller does not record gradients, the result is kept with the parameter for its next call."""
+    return _kept(w, dtype, _expand_weight, keep)
+
+
+def weight_planes(w: torch.Tensor, dtype=torch.bfloat16, keep: bool = False) -> torch.Tensor:
+    """complex [Ci, Co, L] on CUDA -> real and imaginary planes [L, 2, Co, Ci] in bf16; elsewhere the block form of `expand_weight`."""
+    return _kept(w, dtype, _planes if w.is_cuda and dtype == torch.bfloat16 else _expand_weight, keep)
+
+
+def _planes(w: torch.Tensor, dtype) -> torch.Tensor:
+    ci, co, L = w.shape
+    wp = torch.empty(L, 2, co, ci, dtype=dtype, device=w.device)
+    _ext.require().spectral_planes(w.detach().contiguous(), wp)
+    return wp
+
+
+def _kept(w: torch.Tensor, dtype, make, keep: bool) -> torch.Tensor:
     if not keep or not w.is_cuda or w.is_inference():
-        return _expand_weight(w, dtype)
-    state = (w._version, _WEIGHT_EPOCH, w.data_ptr(), dtype)
+        return make(w, dtype)
+    state = (w._version, _WEIGHT_EPOCH, w.data_ptr(), dtype, make)
     hit = _EXPANDED.get(w)
     if hit is not None and hit[0] == state:
         return hit[1]
-    wx = _expand_weight(w, dtype)
+    wx = make(w, dtype)
     _EXPANDED[w] = (state, wx)
     return wx
 
@@ -270,7 +307,7 @@ class _SpectralConv(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, plan_in: SHTPlan, plan_out: SHTPlan, want_resid: bool, train: bool):
         x = _to_cl(x)
-        wx = expand_weight(w, x.dtype, keep=not train)
+        wx = weight_planes(w, x.dtype, keep=not train)
         t1 = dft_analysis(x, plan_in.f, False, plan_in.nlon, plan_in.k2)
         t2 = legendre_analysis(t1, plan_in.pw)
         del t1

@@ -241,3 +241,29 @@ def test_gemm_fp32_output(acc, m, n, k):
     _ext.check_device_errors(dev)
     ref = torch.einsum("zkm,zkn->zmn", a[..., :m].double(), b[..., :n].double()) + (3.0 if acc else 0.0)
     assert _rel(d, ref) < 2.0 ** -24 * max(k, 64) ** 0.5 * 4
+
+
+@pytest.mark.parametrize("b,l,m,co,ci", [(1, 5, 6, 8, 8), (2, 33, 34, 24, 40), (1, 70, 66, 72, 200), (1, 140, 141, 384, 136)])
+def test_planar_spectral_products(b, l, m, co, ci):
+    """Product with the planar weights, its adjoint (with a residual) and the weight gradient against complex einsum: parts that
+    are no whole slabs or tiles, one to three row tiles, orders above the degree skipped."""
+    from makani_b200.ops.spectral import contract, contract_wgrad2, weight_planes
+    dev = _dev()
+    g = torch.Generator(dev).manual_seed(l * ci)
+    keep = (torch.arange(m, device=dev)[None] <= torch.arange(l, device=dev)[:, None]).view(1, l, m, 1)
+    t2 = (torch.randn(b, l, m, 2 * ci, device=dev, generator=g) * keep).to(torch.bfloat16)
+    dt = (torch.randn(b, l, m, 2 * co, device=dev, generator=g) * keep).to(torch.bfloat16)
+    w = torch.randn(ci, co, l, dtype=torch.complex64, device=dev, generator=g)
+    wp = weight_planes(w)
+    wd = torch.complex(wp[:, 0].double(), wp[:, 1].double())                   # [l, co, ci], as rounded
+    cplx = lambda t: torch.complex(t[..., : t.shape[-1] // 2].double(), t[..., t.shape[-1] // 2:].double())  # noqa: E731
+    parts = lambda z: torch.cat([z.real, z.imag], dim=-1)  # noqa: E731
+    y = contract(t2, wp, False)
+    assert _rel(y, parts(torch.einsum("blmc,loc->bmlo", cplx(t2), wd))) < BF16
+    res = torch.randn(b, m, l, 2 * ci, device=dev, generator=g).to(torch.bfloat16)
+    dx = contract(dt, wp, True, resid=res)
+    assert _rel(dx, parts(torch.einsum("blmo,loc->bmlc", cplx(dt), wd.conj())) + res.double()) < BF16
+    dw = contract_wgrad2(dt, t2)
+    ref = torch.einsum("blmo,blmc->loc", cplx(dt), cplx(t2).conj())
+    assert _rel(dw, torch.stack([ref.real, ref.imag])) < 2.0 ** -24 * max(b * m, 64) ** 0.5 * 4
+    _ext.check_device_errors(dev)
