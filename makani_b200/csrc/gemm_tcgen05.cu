@@ -202,6 +202,21 @@ __device__ __forceinline__ void tma_load_4d_pair(uint32_t dst, const CUtensorMap
       : "memory");
 }
 
+// One lane of a converged warp, always the same one.  The compiler knows that a single thread runs behind it and issues the
+// TMA / MMA / commit instructions, which take uniform registers, as they are; behind `lane == 0` it guards each of them
+// against differing operands.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred P1;\n\t"
+      "elect.sync _|P1, 0xffffffff;\n\t"
+      "selp.b32 %0, 1, 0, P1;\n\t"
+      "}\n"
+      : "=r"(ok));
+  return ok != 0;
+}
+
 // address of the same shared-memory offset in CTA `rank` of the cluster
 __device__ __forceinline__ uint32_t mapa_u32(uint32_t addr, uint32_t rank) {
   uint32_t r;
@@ -264,36 +279,26 @@ __device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
                : "memory");
 }
 
+// One MMA; the operand descriptors come as halves (see desc_hi, desc_lo)
 template <int EB, int CG>
-__device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accum) {
-  if constexpr (EB == 2 && CG == 2) {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
-        "}\n" ::"r"(tmem_d),
-        "l"(da), "l"(db), "r"(idesc), "r"(accum)
-        : "memory");
-  } else if constexpr (EB == 2) {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
-        "}\n" ::"r"(tmem_d),
-        "l"(da), "l"(db), "r"(idesc), "r"(accum)
-        : "memory");
-  } else {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t"
-        "}\n" ::"r"(tmem_d),
-        "l"(da), "l"(db), "r"(idesc), "r"(accum)
-        : "memory");
-  }
+__device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
+                                       uint32_t accum) {
+#define MK_MMA(FORM)                                                 \
+  asm volatile(                                                      \
+      "{\n\t"                                                        \
+      ".reg .pred p;\n\t"                                            \
+      ".reg .b64 da, db;\n\t"                                        \
+      "mov.b64 da, {%1, %2};\n\t"                                    \
+      "mov.b64 db, {%3, %4};\n\t"                                    \
+      "setp.ne.b32 p, %6, 0;\n\t"                                    \
+      "tcgen05.mma." FORM " [%0], da, db, %5, p;\n\t"                \
+      "}\n" ::"r"(tmem_d),                                           \
+      "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accum) \
+      : "memory")
+  if constexpr (EB == 2 && CG == 2) MK_MMA("cta_group::2.kind::f16");
+  else if constexpr (EB == 2) MK_MMA("cta_group::1.kind::f16");
+  else MK_MMA("cta_group::1.kind::tf32");
+#undef MK_MMA
 }
 
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
@@ -316,16 +321,14 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// Shared-memory matrix descriptor, 128-byte swizzle, sm_100 version field = 1.
-__device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((saddr & 0x3FFFF) >> 4);
-  d |= static_cast<uint64_t>((lbo_bytes >> 4) & 0x3FFF) << 16;
-  d |= static_cast<uint64_t>((sbo_bytes >> 4) & 0x3FFF) << 32;
-  d |= static_cast<uint64_t>(1) << 46;   // descriptor version
-  d |= static_cast<uint64_t>(2) << 61;   // SWIZZLE_128B
-  return d;
+// Shared-memory matrix descriptor, 128-byte swizzle, sm_100 version field = 1, as two halves: only the low one changes from
+// one MMA to the next, by the distance in bytes / 16.  The issuing thread builds them itself, one dependent instruction after
+// the other, while the tensor cores wait: building eight 64-bit descriptors for every k slab took longer than the slab's MMAs
+// (768 -> 384 outputs over 721 x 1440 tokens: 662 -> 581 us; 16200 x 768 -> 3072: 104 -> 84 us, with the elected lanes above).
+__device__ __forceinline__ uint32_t desc_lo(uint32_t saddr, uint32_t lbo_bytes) {
+  return ((saddr & 0x3FFFF) >> 4) | ((lbo_bytes >> 4) << 16);
 }
+__device__ __forceinline__ uint32_t desc_hi(uint32_t sbo_bytes) { return (sbo_bytes >> 4) | (1u << 14) | (2u << 29); }
 
 struct TileCoord {
   int zhi, zlo, split, mt, nt;
@@ -514,19 +517,74 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       int s = 0;
       uint32_t ph = 0;
       bool ok = peers_ready;
       if (p.sync.nwait > 0) asm volatile("fence.proxy.async;" ::: "memory");   // flags acquired in the prologue order the TMA loads below
-      // pair: every load of both CTAs is counted on the leader's "full" barrier
+      // pair: every load of both CTAs is counted on the leader's "full" barrier.  The leader announces the bytes of both; the
+      // partner's loads may land first (the barrier's byte count goes negative for a moment, its phase cannot complete
+      // before the leader's arrival)
       const uint32_t leader_full0 = (CG == 2) ? mapa_u32(full_bar(0), 0) : 0u;
       const uint32_t load_bytes = A_STAGE_BYTES + (p.b_mn ? B_STAGE_BYTES : BNL * 128);
+      const bool a_mn = p.a_mn != 0, b_mn = p.b_mn != 0;
+      // the next stage: waits until it is free and loads the k slabs of A at ka, rows m0, and of B at kb, rows nb
+      auto stage = [&](const CUtensorMap* mb, int ka, int m0, int azl, int azh, int kb, int nb, int bzl, int bzh) {
+        if (!mbar_wait(empty_bar(s), ph ^ 1u)) {
+          atomicExch(p.err, 1);
+          return false;
+        }
+        const uint32_t sa = smem_base + s * STAGE_BYTES;
+        const uint32_t sb = sa + A_STAGE_BYTES;
+        if constexpr (CG == 2) {
+          if (crank == 0) mbar_expect_tx(full_bar(s), 2 * load_bytes);
+          const uint32_t bar = leader_full0 + 8u * s;
+          if (!a_mn) {
+            tma_load_4d_pair(sa, &map_a, bar, ka, m0, azl, azh);
+          } else {
+#pragma unroll
+            for (int j = 0; j < BM / MN_BOX; ++j) tma_load_4d_pair(sa + j * (BK * 128), &map_a, bar, m0 + j * MN_BOX, ka, azl, azh);
+          }
+          if (!b_mn) {
+            tma_load_4d_pair(sb, mb, bar, kb, nb, bzl, bzh);
+          } else {
+#pragma unroll
+            for (int j = 0; j < B_STAGE_BYTES / (BK * 128); ++j)
+              tma_load_4d_pair(sb + j * (BK * 128), mb, bar, nb + j * MN_BOX, kb, bzl, bzh);
+          }
+        } else {
+          const uint32_t bar = full_bar(s);
+          mbar_expect_tx(bar, load_bytes);
+          if (!a_mn) {
+            tma_load_4d(sa, &map_a, bar, ka, m0, azl, azh);
+          } else {
+#pragma unroll
+            for (int j = 0; j < BM / MN_BOX; ++j) tma_load_4d(sa + j * (BK * 128), &map_a, bar, m0 + j * MN_BOX, ka, azl, azh);
+          }
+          if (!b_mn) {
+            tma_load_4d(sb, mb, bar, kb, nb, bzl, bzh);
+          } else {
+#pragma unroll
+            for (int j = 0; j < BN / MN_BOX; ++j) tma_load_4d(sb + j * (BK * 128), mb, bar, nb + j * MN_BOX, kb, bzl, bzh);
+          }
+        }
+        if (++s == STAGES) {
+          s = 0;
+          ph ^= 1u;
+        }
+        return true;
+      };
+      const bool simple = p.nseg <= 1 && p.cplx == 0 && p.zred <= 1;
       for (uint32_t t = tile0; t < p.total_tiles && ok; t += tile_step) {
         const TileCoord c = decode_tile<BK, CG>(p, t, crank);
-        const int m0 = c.mt * BM, n0 = c.nt * BN;
         if (c.skip) continue;
+        const int m0 = c.mt * BM, nb = c.nt * BN + (CG == 2 ? crank * BNL : 0);
         int azl = p.a_zlo ? c.zlo : 0, bzl = p.b_zlo ? c.zlo : 0;
+        if (simple) {
+          const int azh = p.a_zhi ? c.zhi : 0, bzh = p.b_zhi ? c.zhi : 0;
+          for (int k = c.k_begin; k < c.k_end && ok; k += BK) ok = stage(&map_b, k, m0, azl, azh, k, nb, bzl, bzh);
+          continue;
+        }
         const int nsg = p.cplx ? 2 : p.nseg;
         for (int sg = 0; sg < nsg && ok; ++sg) {
           int lb = c.k_begin, le = c.k_end, apos = 0;
@@ -544,59 +602,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
           // (with batches summed inside the tile the k loop runs over all of them)
           const int zr_n = p.zred > 1 ? min(p.zred, p.zhi_all - c.zhi * p.zred) : 1;
           for (int zr = 0; zr < zr_n && ok; ++zr) {
-          const int zh = p.zred > 1 ? c.zhi * p.zred + zr : c.zhi;
-          const int azh = p.a_zhi ? zh : 0, bzh = p.b_zhi ? zh : 0;
-          for (int k = lb; k < le; k += BK) {
-            if (!mbar_wait(empty_bar(s), ph ^ 1u)) {
-              atomicExch(p.err, 1);
-              ok = false;
-              break;
-            }
-            const uint32_t sa = smem_base + s * STAGE_BYTES;
-            const uint32_t sb = sa + A_STAGE_BYTES;
-            const int ka = apos + k;
-            if constexpr (CG == 2) {
-              // the leader announces the bytes of both CTAs; the partner's loads may land first (the barrier's byte
-              // count goes negative for a moment, its phase cannot complete before the leader's arrival)
-              if (crank == 0) mbar_expect_tx(full_bar(s), 2 * load_bytes);
-              const uint32_t lbar = leader_full0 + 8u * s;
-              const int nb0 = n0 + crank * BNL;
-              if (!p.a_mn) {
-                tma_load_4d_pair(sa, &map_a, lbar, ka, m0, azl, azh);
-              } else {
-#pragma unroll
-                for (int j = 0; j < BM / MN_BOX; ++j)
-                  tma_load_4d_pair(sa + j * (BK * 128), &map_a, lbar, m0 + j * MN_BOX, ka, azl, azh);
-              }
-              if (!p.b_mn) {
-                tma_load_4d_pair(sb, mb, lbar, k, nb0, bzl, bzh);
-              } else {
-#pragma unroll
-                for (int j = 0; j < B_STAGE_BYTES / (BK * 128); ++j)
-                  tma_load_4d_pair(sb + j * (BK * 128), mb, lbar, nb0 + j * MN_BOX, k, bzl, bzh);
-              }
-            } else {
-              mbar_expect_tx(full_bar(s), load_bytes);
-              if (!p.a_mn) {
-                tma_load_4d(sa, &map_a, full_bar(s), ka, m0, azl, azh);
-              } else {
-#pragma unroll
-                for (int j = 0; j < BM / MN_BOX; ++j)
-                  tma_load_4d(sa + j * (BK * 128), &map_a, full_bar(s), m0 + j * MN_BOX, ka, azl, azh);
-              }
-              if (!p.b_mn) {
-                tma_load_4d(sb, mb, full_bar(s), k, n0, bzl, bzh);
-              } else {
-#pragma unroll
-                for (int j = 0; j < BN / MN_BOX; ++j)
-                  tma_load_4d(sb + j * (BK * 128), mb, full_bar(s), n0 + j * MN_BOX, k, bzl, bzh);
-              }
-            }
-            if (++s == STAGES) {
-              s = 0;
-              ph ^= 1u;
-            }
-          }
+            const int zh = p.zred > 1 ? c.zhi * p.zred + zr : c.zhi;
+            const int azh = p.a_zhi ? zh : 0, bzh = p.b_zhi ? zh : 0;
+            for (int k = lb; k < le && ok; k += BK) ok = stage(mb, apos + k, m0, azl, azh, k, nb, bzl, bzh);
           }
         }
       }
@@ -607,7 +615,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
     // epilogue of tile t has released its buffer.  Issued from the operand producer's loop, that wait held back the
     // A and B loads of the tiles in between; issued from another lane of the producer warp, its polling held up that
     // warp's TMA issue.
-    if (lane == 0 && p.e_tma && peers_ready) {
+    if (elect_one() && p.e_tma && peers_ready) {
       if (p.sync.nwait > 0) asm volatile("fence.proxy.async;" ::: "memory");
       uint32_t epi_it = 0;
       for (uint32_t t = tile0; t < p.total_tiles; t += tile_step) {
@@ -628,7 +636,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && crank == 0) {
+    if (elect_one() && crank == 0) {
       // instruction descriptor: fp32 accumulate, operand format, majors, N, M (256 rows for a CTA pair)
       const uint32_t fmt = (EB == 2) ? 1u : 2u;   // BF16 : TF32
       const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | (static_cast<uint32_t>(p.a_mn) << 15) |
@@ -636,8 +644,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
                              (static_cast<uint32_t>((BM * CG) >> 4) << 24);
       const uint32_t a_lbo = p.a_mn ? BK * 128 : 16, a_sbo = 1024;
       const uint32_t b_lbo = p.b_mn ? BK * 128 : 16, b_sbo = 1024;
-      const uint32_t a_kstep = p.a_mn ? UMMA_K * 128 : 32;
-      const uint32_t b_kstep = p.b_mn ? UMMA_K * 128 : 32;
+      const uint32_t a_kstep = (p.a_mn ? UMMA_K * 128 : 32) >> 4;
+      const uint32_t b_kstep = (p.b_mn ? UMMA_K * 128 : 32) >> 4;
+      const uint32_t a_hi = desc_hi(a_sbo), b_hi = desc_hi(b_sbo);
+      const uint32_t a_lo0 = desc_lo(smem_base, a_lbo), b_lo0 = desc_lo(smem_base + A_STAGE_BYTES, b_lbo);
       int s = 0;
       uint32_t ph = 0, acc_it = 0;
       bool ok = peers_ready;
@@ -664,23 +674,21 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
           if (p.cplx) nblocks *= 2;
           if (p.zred > 1) nblocks *= min(p.zred, p.zhi_all - c.zhi * p.zred);
         }
-        // the negative product of a complex one: bit 14 of the instruction descriptor negates B
-        const bool neg_half = p.cplx != 0 && c.half == p.neg_half;
+        // the negative product of a complex one: bit 14 of the instruction descriptor negates B in one half of the k loop
+        const uint32_t neg = p.cplx != 0 && c.half == p.neg_half ? 1u << 14 : 0u;
+        const int kneg = p.neg_seg ? nblocks >> 1 : 0, kpos = p.neg_seg ? nblocks : nblocks >> 1;
         for (int kb = 0; kb < nblocks; ++kb) {
-          const uint32_t neg = neg_half && (2 * kb >= nblocks ? 1 : 0) == p.neg_seg ? 1u << 14 : 0u;
           if (!mbar_wait(full_bar(s), ph)) {
             atomicExch(p.err, 3);
             ok = false;
             break;
           }
           tc_fence_after();
-          const uint32_t sa = smem_base + s * STAGE_BYTES;
-          const uint32_t sb = sa + A_STAGE_BYTES;
+          const uint32_t off = static_cast<uint32_t>(s) * (STAGE_BYTES >> 4);
+          const uint32_t id = idesc | (kb >= kneg && kb < kpos ? neg : 0u);
 #pragma unroll
           for (int kk = 0; kk < BK / UMMA_K; ++kk) {
-            const uint64_t da = make_desc(sa + kk * a_kstep, a_lbo, a_sbo);
-            const uint64_t db = make_desc(sb + kk * b_kstep, b_lbo, b_sbo);
-            tc_mma<EB, CG>(tmem_d, da, db, idesc | neg, accum);
+            tc_mma<EB, CG>(tmem_d, a_lo0 + off + kk * a_kstep, a_hi, b_lo0 + off + kk * b_kstep, b_hi, id, accum);
             accum = 1;
           }
           // frees the smem stage (in both CTAs of a pair) once these MMAs have read it
@@ -770,7 +778,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
           }
           fence_async_smem();
           __syncwarp();
-          if (lane == 0 && r0 < p.M) {
+          if (elect_one() && r0 < p.M) {
             const int zl = p.d_zlo_on ? c.zlo : 0, zh = p.d_zhi_on ? c.zhi : 0;
             if (p.accumulate) tma_add_tile(&map_d, smem_base + box_off, nb, c.half, r0 >> p.rd_shift, zl, zh);
             else tma_store_tile(&map_d, smem_base + box_off, nb, c.half, r0 >> p.rd_shift, zl, zh);
@@ -780,7 +788,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
         if (!c.skip) {
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) {
+          if (elect_one()) {
             if constexpr (CG == 2) mbar_arrive_cluster(leader_tempty0 + 8u * buf);
             else mbar_arrive(tempty_bar(buf));
           }
@@ -887,7 +895,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
         if (!c.skip) {     // the accumulator has been read: the next tile but one may overwrite it
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) {
+          if (elect_one()) {
             if constexpr (CG == 2) mbar_arrive_cluster(leader_tempty0 + 8u * buf);
             else mbar_arrive(tempty_bar(buf));
           }
@@ -897,7 +905,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
           fence_async_smem();
           __syncwarp();
           const int r0 = c.mt * BM + q * 32;
-          if (lane == 0 && r0 < p.M) {
+          if (elect_one() && r0 < p.M) {
             const int rs = r0 >> p.rd_shift;
             if constexpr (EPI == 2) tma_store_tile(&map_p, smem_base + box_off - 32 * 128, nb, 0, rs, c.zlo, c.zhi);
             tma_store_tile(&map_d, smem_base + box_off, nb, c.half, rs, c.zlo, c.zhi);
@@ -911,7 +919,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
         }
         if constexpr (IN_PLACE) {
           __syncwarp();
-          if (lane == 0) mbar_arrive(eempty_bar(ebuf));
+          if (elect_one()) mbar_arrive(eempty_bar(ebuf));
           ++epi_it;
         }
         continue;
@@ -1075,7 +1083,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
 
   // ------------------------------------------------------------------ teardown
   if constexpr (EPI != 0) {
-    if (warp >= 2 && warp < E_WARP && lane == 0) {
+    if (warp >= 2 && warp < E_WARP) {      // (bulk groups belong to the lane that committed them)
       tma_store_wait_all();
       asm volatile("fence.proxy.async;" ::: "memory");   // order the bulk stores before the generic-proxy signalling below
     }
