@@ -1686,11 +1686,11 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
       epi = 5;
   }
   // CTA pairs (256-row tiles, each CTA loads half of the B tile): single-device bf16 launches without row-triangular
-  // structure and with at least two row blocks.  MAKANI_B200_CTA_PAIRS=0 keeps every launch on single CTAs.
-  // Measured at 721x1440 (1 GPU, CUDA events): pairs win where the k loop is long (K = 768 convolutions, weight
-  // gradients, the longitude DFT: 3-11 %) and lose where it is short (K = 384: the epilogue, not the operand fill, is
-  // the bound there, and a pair has half as many independent tiles in flight), so the default is K >= 512.
-  // MAKANI_B200_CTA_PAIRS=0 / 1 forces none / all eligible launches.
+  // structure and with at least two row blocks.  Measured pairs / single CTAs, us: 384 -> 768 with GELU and its derivative over
+  // 721 x 1440 tokens 870 / 1043, its gradient 784 / 860, 768 -> 384 575 / 608, 73 -> 384 gradient 275 / 284, Legendre synthesis
+  // (K = 240) 29 / 31, longitude DFT 344 / 377, token MLP 16200 x 768 -> 3072 84 / 112.  Short k loops over few rows are faster
+  // on single CTAs (K = 192, 8190 rows: 17.0 / 15.7), and so are outputs whose rows pairs would pad (384 of 512 rows of a
+  // weight gradient: 327 / 290; per-degree gradients 89 / 78).  MAKANI_B200_CTA_PAIRS=0 / 1 forces none / all eligible launches.
   static const int pairs_mode = [] {
     const char* e = getenv("MAKANI_B200_CTA_PAIRS");
     return (e && e[0] == '0') ? 0 : ((e && e[0] == '1') ? 1 : 2);
@@ -1698,7 +1698,9 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
   const bool no_peer = (peer == nullptr) || (peer->nseg <= 1 && peer->ndx == 0 && peer->nwait == 0 && peer->nsig == 0 &&
                                               peer->done_ctr == nullptr);
   const bool eligible = eb == 2 && no_peer && p.M > BM && p.rmin_a == 0 && p.rmax_a == 0 && (p.cplx == 0 || p.cplx == 3);
-  const int cg = (eligible && (pairs_mode == 1 || (pairs_mode == 2 && p.K >= 512))) ? 2 : 1;
+  const int pad1 = (p.M + BM - 1) / BM * BM, pad2 = (p.M + 2 * BM - 1) / (2 * BM) * (2 * BM);
+  const bool pays = (p.K >= 200 || p.M >= 65536) && pad2 * 8 <= pad1 * 9;
+  const int cg = (eligible && (pairs_mode == 1 || (pairs_mode == 2 && pays))) ? 2 : 1;
   if (bn == 0) bn = pick_bn(p.N, epi, kp.e_tma);
   if ((eb == 4 && bn == 192) || ((epi == 3 || epi == 4 || kp.e_tma) && bn == 256)) bn = 128;
   if (epi == 0 && kp.e_tma) bn = 128;
