@@ -197,12 +197,8 @@ def contract_wgrad2(dt: torch.Tensor, t2: torch.Tensor, l0: int = 0, m0: int = 0
                          Output(out, rs_lo=ci, d_zhi=co * ci), L * co * ci, zhi_n=L, a_plane=co, b_plane=ci, accumulate=(B > 1),
                          kmax=(1, 1 + l0 - m0))
         return out
-    if dt.is_cuda and dt.dtype == torch.bfloat16 and co % 8 == 0 and dt.is_contiguous() and _ext.native():
-        dts = torch.empty_like(dt)
-        _ext.require().swap_ri(dt, dts, co)
-    else:
-        d5 = dt.view(B, L, M, 2, co)
-        dts = torch.cat([d5[..., 1:2, :], -d5[..., 0:1, :]], dim=-2).contiguous()
+    d5 = dt.view(B, L, M, 2, co)
+    dts = torch.cat([d5[..., 1:2, :], -d5[..., 0:1, :]], dim=-2).contiguous()
     out = (torch.empty if B == 1 else torch.zeros)(2, L, co, ci, dtype=torch.float32, device=dt.device)
     tri = Tri(kmax_a=2, kmax_b=2 * (1 + l0 - m0))
     for part, a in enumerate((dt, dts)):
@@ -237,7 +233,8 @@ _EXPANDED = WeakTensorKeyDictionary()
 def note_weights_changed() -> None:
     global _WEIGHT_EPOCH
     _WEIGHT_EPOCH += 1
-    _EXPANDED.clear()
+    if len(_EXPANDED):
+        _EXPANDED.clear()
 
 
 def expand_weight(w: torch.Tensor, dtype=torch.bfloat16, keep: bool = False) -> torch.Tensor:
