@@ -1641,7 +1641,9 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
   // Rows split by a power of two (the (mode, re / im) rows of the DFT stages) are one more dimension of the tensor map: the AFNO
   // stages at 90 x 180 tokens take 14 - 21 us each, 22 - 44 us through the generic epilogue.
   const bool one_stride = e.rdiv <= 0 || e.rdiv >= (1 << 30);
-  const bool split_ok = !one_stride && e.rdiv <= 32 && (e.rdiv & (e.rdiv - 1)) == 0 && p.M % e.rdiv == 0 && e.rs_hi > 0 && e.rs_lo > 0;
+  // (rdiv = 1 puts every row at rs_hi: the map's row stride would be rs_lo)
+  const bool split_ok = !one_stride && e.rdiv > 1 && e.rdiv <= 32 && (e.rdiv & (e.rdiv - 1)) == 0 && p.M % e.rdiv == 0 && e.rs_hi > 0 &&
+                        e.rs_lo > 0;
   const bool plain = (one_stride || split_ok) && (e.ndiv <= 0 || e.ndiv >= (1 << 30));
   const int rd = one_stride ? 1 : e.rdiv;
   auto tile_map = [&](CUtensorMap* m, const void* ptr, int box_rows) {

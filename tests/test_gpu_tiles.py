@@ -181,6 +181,22 @@ def test_gemm_split_rows(rd, m, epi):
         assert _rel(got, ref) < BF16
 
 
+@pytest.mark.parametrize("m", [1, 40, 300])
+@pytest.mark.parametrize("epi", ["plain", "resid", "fp32"])
+def test_gemm_split_rows_of_one(m, epi):
+    """rdiv = 1: row r lies at r * rs_hi, and rs_lo, a shorter or a longer distance, is never used."""
+    dev = _dev()
+    k, n = 72, 136
+    torch.manual_seed(m)
+    a, b = torch.randn(m, k, device=dev).to(torch.bfloat16), torch.randn(n, k, device=dev).to(torch.bfloat16)
+    for lo in (8, 4 * n):
+        d = torch.zeros(m, 2 * n, device=dev, dtype=torch.float32 if epi == "fp32" else torch.bfloat16)
+        aux = torch.randn(m, 2 * n, device=dev).to(torch.bfloat16) if epi == "resid" else None
+        outs = _run_both(m, n, k, Operand(a, ld=k), Operand(b, ld=k), Output(d, rs_lo=lo, rdiv=1, rs_hi=2 * n), resid=aux)
+        for got, ref in outs:
+            assert _rel(got, ref) < BF16
+
+
 @pytest.mark.parametrize("z", [1, 2, 91, 800])
 @pytest.mark.parametrize("co,ci,k", [(16, 24, 8), (192, 192, 90), (136, 264, 200)])
 def test_gemm_batches_summed_inside_tiles(z, co, ci, k):
