@@ -1717,6 +1717,11 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
       snprintf(g_err, sizeof(g_err), "complex product: bf16 operands, plain rows, aligned output with or without residual");
       return cudaErrorInvalidValue;
     }
+    // the second part of a K-major A starts at k = K, a coordinate of the contiguous dimension: a whole number of 16-byte vectors
+    if (p.cplx != 3 && !A.mn_major && (p.K % (16 / eb)) != 0) {
+      snprintf(g_err, sizeof(g_err), "complex product: the parts of A must be multiples of %d elements", 16 / eb);
+      return cudaErrorInvalidValue;
+    }
     kp.n_tiles *= 2;
   }
   // Batches that add into one output (d_zhi = 0) are summed inside the tiles as far as the SMs stay busy: 728 products of

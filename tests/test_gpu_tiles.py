@@ -283,3 +283,14 @@ def test_planar_spectral_products(b, l, m, co, ci):
     ref = torch.einsum("blmo,blmc->loc", cplx(dt), cplx(t2).conj())
     assert _rel(dw, torch.stack([ref.real, ref.imag])) < 2.0 ** -24 * max(b * m, 64) ** 0.5 * 4
     _ext.check_device_errors(dev)
+
+
+@pytest.mark.parametrize("co", [4, 12, 20])
+def test_planar_product_refuses_parts_off_a_vector(co):
+    """The adjoint reads the imaginary part of its operand at element co: refused by the host where that is no 16-byte boundary."""
+    from makani_b200.ops.spectral import contract
+    dev = _dev()
+    dt = torch.zeros(1, 6, 7, 2 * co, device=dev, dtype=torch.bfloat16)
+    wp = torch.zeros(6, 2, co, 16, device=dev, dtype=torch.bfloat16)
+    with pytest.raises(RuntimeError, match="multiples of 8"):
+        contract(dt, wp, True)
