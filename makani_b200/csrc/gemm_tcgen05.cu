@@ -1728,17 +1728,19 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
   // 192 x 192 with 90 summands each spent their time in 107 MB of fp32 atomics (44 us, now 29).
   const int slots = cg == 2 ? max_pairs() : sm_count();
   const bool no_tri = p.rmin_a == 0 && p.rmax_a == 0 && p.kmin_a == 0 && p.kmax_a == 0;
+  // (a bias or an activation is applied once per partial sum, and a segmented k axis is walked by one CTA: one split there)
+  const bool choose = p.splits == 0 && e.accumulate && kp.bias_mode == 0 && e.act == 0 && kp.nseg == 1;
   kp.zred = 1;
   kp.zhi_all = p.zhi_n;
   long long base_tiles = static_cast<long long>(kp.m_tiles) * kp.n_tiles * p.zlo_n;
-  if (p.splits == 0 && e.accumulate && e.d_zhi == 0 && p.zhi_n > 1 && no_tri && kp.nseg == 1) {
+  if (choose && e.d_zhi == 0 && p.zhi_n > 1 && no_tri) {
     const int groups = pick_splits(base_tiles, p.zhi_n * (kblocks > 0 ? kblocks : 1), slots);
     kp.zred = (p.zhi_n + groups - 1) / groups;
     if (kp.zred < 1) kp.zred = 1;
   }
   kp.zhi_n = (p.zhi_n + kp.zred - 1) / kp.zred;
   base_tiles *= kp.zhi_n;
-  if (p.splits == 0 && e.accumulate && kp.zred == 1) kp.splits = pick_splits(base_tiles, kblocks, slots);
+  if (choose && kp.zred == 1) kp.splits = pick_splits(base_tiles, kblocks, slots);
   kp.k_per_split = ((kblocks + kp.splits - 1) / kp.splits) * bk;
   if (kp.k_per_split < bk) kp.k_per_split = bk;
   if (base_tiles * kp.splits >= (1ll << 31)) {

@@ -4,7 +4,7 @@ import pytest
 import torch
 
 from makani_b200.ops import _ext
-from makani_b200.ops.gemm import (ACT_DGELU, ACT_GELU, ACT_MULAUX, ACT_NONE, ACT_RELU, BIAS_COL, Operand, Output, gemm)
+from makani_b200.ops.gemm import (ACT_DGELU, ACT_GELU, ACT_MULAUX, ACT_NONE, ACT_RELU, BIAS_COL, BIAS_ROW, Operand, Output, gemm)
 from test_gpu_kernels import _dev, _rel, _run_both
 
 pytestmark = pytest.mark.gpu
@@ -294,3 +294,24 @@ def test_planar_product_refuses_parts_off_a_vector(co):
     wp = torch.zeros(6, 2, co, 16, device=dev, dtype=torch.bfloat16)
     with pytest.raises(RuntimeError, match="multiples of 8"):
         contract(dt, wp, True)
+
+
+@pytest.mark.parametrize("z", [1, 7])
+@pytest.mark.parametrize("opt", ["bias_row", "bias_col", "relu"])
+def test_chosen_splits_leave_the_epilogue_alone(z, opt):
+    """splits = 0 with a bias or an activation: applied to each whole product, never to the partial sums of one."""
+    dev = _dev()
+    m, n, k = 136, 72, 64 * 40
+    g = torch.Generator(dev).manual_seed(z)
+    a = torch.randn(z, k, m, device=dev, generator=g).to(torch.bfloat16)
+    b = torch.randn(z, k, n, device=dev, generator=g).to(torch.bfloat16)
+    bias = None if opt == "relu" else torch.randn(m if opt == "bias_row" else n, device=dev, generator=g) * 100
+    d = torch.zeros(m, n, device=dev)
+    gemm(m, n, k, Operand(a, ld=m, mn_major=True, zs_hi=k * m), Operand(b, ld=n, mn_major=True, zs_hi=k * n), Output(d, rs_lo=n), zhi_n=z,
+         accumulate=True, splits=0, bias=bias, bias_mode=BIAS_ROW if opt == "bias_row" else BIAS_COL,
+         act=ACT_RELU if opt == "relu" else ACT_NONE)
+    _ext.check_device_errors(dev)
+    ref = torch.einsum("zkm,zkn->zmn", a.double(), b.double())
+    ref = torch.relu(ref) if opt == "relu" else ref + (bias[:, None] if opt == "bias_row" else bias[None, :]).double()
+    # fp32 sums of k exact products, truncated by the tensor core at every 16 of them
+    assert _rel(d, ref.sum(0)) < 2.0 ** -24 * (k / 16)
