@@ -1527,13 +1527,17 @@ int pick_bn(int N, int epi, int e_tma) {
 }
 
 // Split-k factor of an accumulating launch: whole waves of `slots` CTAs (or pairs), every split costing its tile one
-// epilogue of atomics, worth some 16 k-blocks.  (Twice as many tiles as SMs, the former rule, left a last wave that was
-// nearly empty: 704 -> 532 us per weight gradient of a 384 <-> 768 layer over 721 x 1440 tokens.)
-int pick_splits(long long base, int kblocks, int slots) {
-  int best = 1;
+// epilogue of atomics, worth some 16 k-blocks, and no fewer partial sums than `least`.
+//
+// `least` is twice the SMs over the 128 x 256 tiles.  The tensor core truncates its running sum at every step, so that an
+// accumulation over k products is off by about k / 16 * 2^-23.  By time alone a 384 x 768 gradient over 721 x 1440 tokens ran in 16
+// chains with an error of 7.5e-5 against 64 bits (one-signed operands: 3.9e-4); 48 chains, again whole waves, give 2.5e-5 (1.1e-4)
+// in 580 us, 16 took 573.  Twice the tiles without whole waves: 33 chains, 3.6e-5, 757 us.
+int pick_splits(long long base, int kblocks, int slots, int least) {
+  int best = least < kblocks ? least : (kblocks > 0 ? kblocks : 1);
   double cost = 1e300;
-  const long long most = 4ll * slots / (base > 0 ? base : 1) + 1;
-  for (int s = 1; s <= most && s <= kblocks; ++s) {
+  const long long most = least + 4ll * slots / (base > 0 ? base : 1);
+  for (int s = best; s <= most && s <= kblocks; ++s) {
     const double waves = static_cast<double>((base * s + slots - 1) / slots);
     const double c = waves * ((kblocks + s - 1) / s + 16.0);
     if (c < cost * 0.999) {
@@ -1734,13 +1738,16 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
   kp.zhi_all = p.zhi_n;
   long long base_tiles = static_cast<long long>(kp.m_tiles) * kp.n_tiles * p.zlo_n;
   if (choose && e.d_zhi == 0 && p.zhi_n > 1 && no_tri) {
-    const int groups = pick_splits(base_tiles, p.zhi_n * (kblocks > 0 ? kblocks : 1), slots);
+    const int groups = pick_splits(base_tiles, p.zhi_n * (kblocks > 0 ? kblocks : 1), slots, 1);
     kp.zred = (p.zhi_n + groups - 1) / groups;
     if (kp.zred < 1) kp.zred = 1;
   }
   kp.zhi_n = (p.zhi_n + kp.zred - 1) / kp.zred;
   base_tiles *= kp.zhi_n;
-  if (choose && kp.zred == 1) kp.splits = pick_splits(base_tiles, kblocks, slots);
+  if (choose && kp.zred == 1) {
+    const long long wide = static_cast<long long>((p.M + BM - 1) / BM) * ((p.N + 255) / 256) * p.zlo_n * p.zhi_n;
+    kp.splits = pick_splits(base_tiles, kblocks, slots, static_cast<int>((2 * sm_count() + wide - 1) / wide));
+  }
   kp.k_per_split = ((kblocks + kp.splits - 1) / kp.splits) * bk;
   if (kp.k_per_split < bk) kp.k_per_split = bk;
   if (base_tiles * kp.splits >= (1ll << 31)) {

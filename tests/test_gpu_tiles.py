@@ -315,3 +315,31 @@ def test_chosen_splits_leave_the_epilogue_alone(z, opt):
     ref = torch.relu(ref) if opt == "relu" else ref + (bias[:, None] if opt == "bias_row" else bias[None, :]).double()
     # fp32 sums of k exact products, truncated by the tensor core at every 16 of them
     assert _rel(d, ref.sum(0)) < 2.0 ** -24 * (k / 16)
+
+
+@pytest.mark.parametrize("sign", ["zero_mean", "one_signed"])
+@pytest.mark.parametrize("co,ci,t", [(16, 16, 4096), (64, 64, 115200), (384, 768, 200000), (384, 384, 1038240), (768, 3072, 16200)])
+def test_chosen_splits_keep_the_sums_short(sign, co, ci, t):
+    """The tensor core truncates its running sum at every 16 products: the chosen factor gives chains no longer, and sums no less
+    exact, than twice as many 128 x 256 tiles as SMs would."""
+    dev = _dev()
+    g = torch.Generator(dev).manual_seed(co)
+    rnd = lambda *s: torch.randn(*s, device=dev, generator=g)  # noqa: E731
+    dy, x = (rnd(t, co), rnd(t, ci)) if sign == "zero_mean" else (rnd(t, co).abs(), rnd(t, ci).abs())
+    dy, x = dy.to(torch.bfloat16), x.to(torch.bfloat16)
+    ref = torch.zeros(co, ci, dtype=torch.float64, device=dev)
+    for p, q in zip(dy.split(131072), x.split(131072)):
+        ref += p.double().t() @ q.double()
+    tiles = ((co + 127) // 128) * ((ci + 255) // 256)
+    sms = torch.cuda.get_device_properties(dev).multi_processor_count
+    err = {}
+    for splits in (0, min((t + 63) // 64, (2 * sms + tiles - 1) // tiles)):
+        dw = torch.zeros(co, ci, device=dev)
+        gemm(co, ci, t, Operand(dy, ld=co, mn_major=True), Operand(x, ld=ci, mn_major=True), Output(dw, rs_lo=ci), accumulate=True,
+             splits=splits)
+        err[splits] = _rel(dw, ref)
+    _ext.check_device_errors(dev)
+    chosen, least = err.pop(0), next(iter(err))
+    # (the order of the fp32 additions between the chains differs from run to run: 2^-24 each, at random)
+    assert chosen <= err[least] * 1.02 + 2.0 ** -24
+    assert chosen <= t / least / 16 * 2.0 ** -23 + 2.0 ** -23
