@@ -118,7 +118,6 @@ struct KParams {
   FastDiv dv_n, dv_m, dv_split, dv_zlo;
   uint32_t total_tiles;           // below 2^31
   int cplx, nth, neg_half, neg_seg;   // complex product: mode, column tiles per half, the negative (half, segment)
-  int zred, zhi_all;              // z_hi batches summed inside one tile (1: none), and their number
   int stages, e_tma;
   int d_zlo_on, d_zhi_on;         // fp32 output through TMA: 0 where all batches of that index add into one output
   int rd_shift;                   // log2 of rdiv where the output leaves through TMA (0: rows have one stride)
@@ -574,14 +573,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
         }
         return true;
       };
-      const bool simple = p.nseg <= 1 && p.cplx == 0 && p.zred <= 1;
+      const bool simple = p.nseg <= 1 && p.cplx == 0;
       for (uint32_t t = tile0; t < p.total_tiles && ok; t += tile_step) {
         const TileCoord c = decode_tile<BK, CG>(p, t, crank);
         if (c.skip) continue;
         const int m0 = c.mt * BM, nb = c.nt * BN + (CG == 2 ? crank * BNL : 0);
         int azl = p.a_zlo ? c.zlo : 0, bzl = p.b_zlo ? c.zlo : 0;
+        const int azh = p.a_zhi ? c.zhi : 0, bzh = p.b_zhi ? c.zhi : 0;
         if (simple) {
-          const int azh = p.a_zhi ? c.zhi : 0, bzh = p.b_zhi ? c.zhi : 0;
           for (int k = c.k_begin; k < c.k_end && ok; k += BK) ok = stage(&map_b, k, m0, azl, azh, k, nb, bzl, bzh);
           continue;
         }
@@ -599,13 +598,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
             if (p.cplx == 3) azl = sg ^ c.half;
             else apos = sg * p.K;
           }
-          // (with batches summed inside the tile the k loop runs over all of them)
-          const int zr_n = p.zred > 1 ? min(p.zred, p.zhi_all - c.zhi * p.zred) : 1;
-          for (int zr = 0; zr < zr_n && ok; ++zr) {
-            const int zh = p.zred > 1 ? c.zhi * p.zred + zr : c.zhi;
-            const int azh = p.a_zhi ? zh : 0, bzh = p.b_zhi ? zh : 0;
-            for (int k = lb; k < le && ok; k += BK) ok = stage(mb, apos + k, m0, azl, azh, k, nb, bzl, bzh);
-          }
+          for (int k = lb; k < le && ok; k += BK) ok = stage(mb, apos + k, m0, azl, azh, k, nb, bzl, bzh);
         }
       }
     }
@@ -672,7 +665,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
         } else {
           nblocks = (c.k_end - c.k_begin + BK - 1) / BK;
           if (p.cplx) nblocks *= 2;
-          if (p.zred > 1) nblocks *= min(p.zred, p.zhi_all - c.zhi * p.zred);
         }
         // the negative product of a complex one: bit 14 of the instruction descriptor negates B in one half of the k loop
         const uint32_t neg = p.cplx != 0 && c.half == p.neg_half ? 1u << 14 : 0u;
@@ -1728,23 +1720,11 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
     }
     kp.n_tiles *= 2;
   }
-  // Batches that add into one output (d_zhi = 0) are summed inside the tiles as far as the SMs stay busy: 728 products of
-  // 192 x 192 with 90 summands each spent their time in 107 MB of fp32 atomics (44 us, now 29).
   const int slots = cg == 2 ? max_pairs() : sm_count();
-  const bool no_tri = p.rmin_a == 0 && p.rmax_a == 0 && p.kmin_a == 0 && p.kmax_a == 0;
   // (a bias or an activation is applied once per partial sum, and a segmented k axis is walked by one CTA: one split there)
   const bool choose = p.splits == 0 && e.accumulate && kp.bias_mode == 0 && e.act == 0 && kp.nseg == 1;
-  kp.zred = 1;
-  kp.zhi_all = p.zhi_n;
-  long long base_tiles = static_cast<long long>(kp.m_tiles) * kp.n_tiles * p.zlo_n;
-  if (choose && e.d_zhi == 0 && p.zhi_n > 1 && no_tri) {
-    const int groups = pick_splits(base_tiles, p.zhi_n * (kblocks > 0 ? kblocks : 1), slots, 1);
-    kp.zred = (p.zhi_n + groups - 1) / groups;
-    if (kp.zred < 1) kp.zred = 1;
-  }
-  kp.zhi_n = (p.zhi_n + kp.zred - 1) / kp.zred;
-  base_tiles *= kp.zhi_n;
-  if (choose && kp.zred == 1) {
+  const long long base_tiles = static_cast<long long>(kp.m_tiles) * kp.n_tiles * p.zlo_n * p.zhi_n;
+  if (choose) {
     const long long wide = static_cast<long long>((p.M + BM - 1) / BM) * ((p.N + 255) / 256) * p.zlo_n * p.zhi_n;
     kp.splits = pick_splits(base_tiles, kblocks, slots, static_cast<int>((2 * sm_count() + wide - 1) / wide));
   }

@@ -200,7 +200,7 @@ def test_gemm_split_rows_of_one(m, epi):
 @pytest.mark.parametrize("z", [1, 2, 91, 800])
 @pytest.mark.parametrize("co,ci,k", [(16, 24, 8), (192, 192, 90), (136, 264, 200)])
 def test_gemm_batches_summed_inside_tiles(z, co, ci, k):
-    """Batches that add into one output: none, a few and many per tile, the last group shorter."""
+    """Batches that add into one output: one, a few and many."""
     dev = _dev()
     g = torch.Generator(dev).manual_seed(z + co)
     a = torch.randn(2, z, k, co, device=dev, generator=g).to(torch.bfloat16)
@@ -343,3 +343,20 @@ def test_chosen_splits_keep_the_sums_short(sign, co, ci, t):
     # (the order of the fp32 additions between the chains differs from run to run: 2^-24 each, at random)
     assert chosen <= err[least] * 1.02 + 2.0 ** -24
     assert chosen <= t / least / 16 * 2.0 ** -23 + 2.0 ** -23
+
+
+@pytest.mark.parametrize("sign", ["zero_mean", "one_signed"])
+def test_batches_into_one_output_keep_their_own_sums(sign):
+    """A batch is summed by itself and added in fp32: the tensor core's truncation does not grow with the number of batches."""
+    dev = _dev()
+    z, k, n = 91, 90, 192
+    g = torch.Generator(dev).manual_seed(5)
+    a, b = (torch.randn(z, k, n, device=dev, generator=g) for _ in range(2))
+    a, b = (a.abs(), b.abs()) if sign == "one_signed" else (a, b)
+    a, b = a.to(torch.bfloat16), b.to(torch.bfloat16)
+    d = torch.zeros(n, n, device=dev)
+    gemm(n, n, k, Operand(a, ld=n, mn_major=True, zs_hi=k * n), Operand(b, ld=n, mn_major=True, zs_hi=k * n), Output(d, rs_lo=n), zhi_n=z,
+         accumulate=True, splits=0)
+    _ext.check_device_errors(dev)
+    # k / 16 truncations per batch, then z roundings of 2^-24 at random
+    assert _rel(d, torch.einsum("zko,zki->oi", a.double(), b.double())) < (k / 16) * 2.0 ** -24 + 2.0 ** -24 * z ** 0.5 / 4
