@@ -1684,11 +1684,17 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
       epi = 5;
   }
   // CTA pairs (256-row tiles, each CTA loads half of the B tile): single-device bf16 launches without row-triangular
-  // structure and with at least two row blocks.  Measured pairs / single CTAs, us: 384 -> 768 with GELU and its derivative over
-  // 721 x 1440 tokens 870 / 1043, its gradient 784 / 860, 768 -> 384 575 / 608, 73 -> 384 gradient 275 / 284, Legendre synthesis
-  // (K = 240) 29 / 31, longitude DFT 344 / 377, token MLP 16200 x 768 -> 3072 84 / 112.  Short k loops over few rows are faster
-  // on single CTAs (K = 192, 8190 rows: 17.0 / 15.7), and so are outputs whose rows pairs would pad (384 of 512 rows of a
-  // weight gradient: 327 / 290; per-degree gradients 89 / 78).  MAKANI_B200_CTA_PAIRS=0 / 1 forces none / all eligible launches.
+  // structure and with at least two row blocks.  MAKANI_B200_CTA_PAIRS=0 / 1 forces none / all eligible launches.  Measured, time on
+  // single CTAs over time on pairs (plain store, product with an operand, GELU with two outputs):
+  //   K = 768, 115200 rows: 1.07 - 1.30.  From K = 512 on the long k loop pays for the pair's longer start.
+  //   K = 256 - 448: 1024 - 8192 rows 0.89 - 0.96 (768 outputs at 8192 rows 0.91 - 1.09); 16200 rows, 384 outputs 0.92 - 0.99, 768
+  //   outputs 0.98 - 1.13; 115200 rows, 384 and 768 outputs 1.03 - 1.23.  A pair has half as many tiles in flight: it pays from
+  //   two waves of tiles on.
+  //   K = 200, 232, 504 (rows of no whole 64 bytes: loads touch one more sector, and a pair loads half of B): 1024 - 8192 rows
+  //   0.95 - 1.06 (504, 768 outputs: 1.11 - 1.23), 16200 rows 1.01 - 1.16, 32768 rows 1.03 - 1.19.
+  //   K < 200, 65536 rows and more: 16, 80, 136, 184: 1.02 - 1.50; 64, 96, 128, 160, 192: 0.92 - 1.15, but for 384 outputs times an
+  //   operand over 518400 rows at 160 and 192 (0.81 - 0.88).
+  // Outputs whose rows pairs would pad stay on single CTAs (384 of 512 rows of a weight gradient: 327 us on pairs, 290 us).
   static const int pairs_mode = [] {
     const char* e = getenv("MAKANI_B200_CTA_PAIRS");
     return (e && e[0] == '0') ? 0 : ((e && e[0] == '1') ? 1 : 2);
@@ -1697,7 +1703,9 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
                                               peer->done_ctr == nullptr);
   const bool eligible = eb == 2 && no_peer && p.M > BM && p.rmin_a == 0 && p.rmax_a == 0 && (p.cplx == 0 || p.cplx == 3);
   const int pad1 = (p.M + BM - 1) / BM * BM, pad2 = (p.M + 2 * BM - 1) / (2 * BM) * (2 * BM);
-  const bool pays = (p.K >= 200 || p.M >= 65536) && pad2 * 8 <= pad1 * 9;
+  const long long z_all = static_cast<long long>(p.zlo_n) * p.zhi_n;
+  const bool waves = pad1 / BM * ((p.N + 255) / 256) * z_all >= 2 * sm_count();
+  const bool pays = (p.K >= 512 || p.M >= 65536 || (p.K >= 200 && (waves || p.K % 32 != 0))) && pad2 * 8 <= pad1 * 9;
   const int cg = (eligible && (pairs_mode == 1 || (pairs_mode == 2 && pays))) ? 2 : 1;
   if (bn == 0) bn = pick_bn(p.N, epi, kp.e_tma);
   if ((eb == 4 && bn == 192) || ((epi == 3 || epi == 4 || kp.e_tma) && bn == 256)) bn = 128;
