@@ -133,14 +133,42 @@ def _stage_w_synthesis(src, mat, plan: AFNOPlan, B, C, resid):
 
 
 def _stage_h_tokens(t1, plan: AFNOPlan, B, C, nb):
-    """t1 [B, ncols, H, 2, C] -> token-major spectrum Y [B*ncols*nkx, nb, 2, bs] (forward DFT along H), per (b, ky, block)."""
+    """t1 [B, ncols, H, 2, C] -> token-major spectrum Y [B*ncols*nkx, nb, 2, bs] (forward DFT along H).
+
+    One GEMM per (b, ky, block) leaves through TMA stores, but fills only bs of a tile's 128 columns; one per (b, ky) over all
+    channels fills its tiles and splits the columns in the generic epilogue.  90 x 91 modes, us per block / all: 8 blocks of 96
+    29 / 33, of 64 26 / 27, of 32 21 / 18 (batch 2: 40 / 26), 16 of 48 39 / 33, 48 of 16 127 / 33; up to some three waves of
+    tiles the first one is ahead with narrow blocks too (40 x 41 modes, 8 blocks of 32: 8.4 / 10.6)."""
     H, nc, nkx = plan.H, plan.ncols, plan.nkx
     bs = C // nb
     y = torch.empty(B * nc * nkx, nb, 2, bs, dtype=t1.dtype, device=t1.device)
-    gemm(2 * nkx, bs, 2 * H, Operand(plan.fh, ld=plan.fh.shape[1]),
-         Operand(t1, ld=C, mn_major=True, zs_lo=bs, zs_hi=H * 2 * C),
-         Output(y, rs_lo=bs, rdiv=2, rs_hi=2 * C, d_zlo=2 * bs, d_zhi=nkx * 2 * C), zlo_n=nb, zhi_n=B * nc)
+    if bs >= 64 or nb * B * nc * ((2 * nkx + 127) // 128) <= 3 * _ext.sm_count():
+        gemm(2 * nkx, bs, 2 * H, Operand(plan.fh, ld=plan.fh.shape[1]),
+             Operand(t1, ld=C, mn_major=True, zs_lo=bs, zs_hi=H * 2 * C),
+             Output(y, rs_lo=bs, rdiv=2, rs_hi=2 * C, d_zlo=2 * bs, d_zhi=nkx * 2 * C), zlo_n=nb, zhi_n=B * nc)
+    else:
+        gemm(2 * nkx, C, 2 * H, Operand(plan.fh, ld=plan.fh.shape[1]),
+             Operand(t1, ld=C, mn_major=True, zs_lo=H * 2 * C, zs_hi=nc * H * 2 * C),
+             Output(y, rs_lo=bs, rdiv=2, rs_hi=2 * C, ndiv=bs, ns_hi=2 * bs, d_zlo=nkx * 2 * C, d_zhi=nc * nkx * 2 * C),
+             zlo_n=nc, zhi_n=B)
     return y
+
+
+def _tokens_to_blocks(src, w: Operand, out, plan: AFNOPlan, B, nb, n, k, **epilogue):
+    """src [B*ncols*nkx, nb, k] times the weights of each block -> out [B*ncols, nb, nkx, n].
+
+    One GEMM per (b, ky, block) writes plain rows through TMA stores, but its nkx rows may leave most of a 128-row tile empty; one
+    per block over all rows fills its tiles and splits the rows in the generic epilogue.  Second layer and its input gradient
+    together, us per column / all rows: 90 x 91 modes, 8 blocks of 96 43 / 92, of 64 43 / 63, of 32 43 / 38, 16 of 48 79 / 105;
+    45 x 46 modes, 8 of 96 29 / 29; 40 x 41 modes, 8 of 96 29 / 29, of 32 29 / 15, batch 2, of 64 43 / 35; 22 x 23, 8 of 96 23 / 28."""
+    nc, nkx = plan.ncols, plan.nkx
+    rows, cols = -(-nkx // 128) * 128, max(128, -(-n // 64) * 64)
+    if n > 128 or nkx * n >= 0.45 * rows * cols:
+        gemm(nkx, n, k, Operand(src, ld=nb * k, zs_lo=k, zs_hi=nkx * nb * k), w,
+             Output(out, rs_lo=n, d_zlo=nkx * n, d_zhi=nb * nkx * n), zlo_n=nb, zhi_n=B * nc, **epilogue)
+    else:
+        gemm(B * nc * nkx, n, k, Operand(src, ld=nb * k, zs_lo=k), w,
+             Output(out, rs_lo=n, rdiv=nkx, rs_hi=nb * nkx * n, d_zlo=nkx * n), zlo_n=nb, **epilogue)
 
 
 def _pack(ws, bs, dt):
@@ -178,8 +206,8 @@ class _AFNOFilter(torch.autograd.Function):
     """y = irfft2(softshrink(relu(rfft2(x) W1 + b1) W2 + b2)) (+ skip) on the kept modes.
 
     w1 [2, nb, bs, hid], w2 [2, nb, hid, bs] hold real and imaginary planes of the complex block weights, b1 [2, nb, hid] and
-    b2 [2, nb, bs] those of the biases (or None); they are packed into real 2x2-block matrices here.  Every GEMM writes plain
-    rows, or rows split into (mode, re / im) pairs, so that all of them leave through TMA stores."""
+    b2 [2, nb, bs] those of the biases (or None); they are packed into real 2x2-block matrices here.  The GEMMs write plain rows,
+    or rows split into (mode, re / im) pairs, and so leave through TMA stores, but where narrow blocks would leave their tiles empty."""
 
     @staticmethod
     def forward(ctx, x, w1, b1, w2, b2, skip, plan, lam):
@@ -196,10 +224,8 @@ class _AFNOFilter(torch.autograd.Function):
         gemm(T, 2 * hid, 2 * bs, Operand(y, ld=2 * C, zs_lo=2 * bs), Operand(w1q, ld=2 * bs, zs_lo=2 * hid * 2 * bs),
              Output(o1, rs_lo=nb * 2 * hid, d_zlo=2 * hid), zlo_n=nb, bias=b1f, bias_mode=BIAS_COL, bias_zs=2 * hid, act=ACT_RELU)
         o2 = torch.empty(B * nc, nb, nkx, 2, bs, dtype=dt, device=x.device)
-        gemm(nkx, 2 * bs, 2 * hid, Operand(o1, ld=nb * 2 * hid, zs_lo=2 * hid, zs_hi=nkx * nb * 2 * hid),
-             Operand(w2q, ld=2 * hid, zs_lo=2 * bs * 2 * hid),
-             Output(o2, rs_lo=2 * bs, d_zlo=nkx * 2 * bs, d_zhi=nb * nkx * 2 * bs), zlo_n=nb, zhi_n=B * nc, bias=b2f,
-             bias_mode=BIAS_COL, bias_zs=2 * bs, act=ACT_SHRINK, act_param=float(lam))
+        _tokens_to_blocks(o1, Operand(w2q, ld=2 * hid, zs_lo=2 * bs * 2 * hid), o2, plan, B, nb, 2 * bs, 2 * hid, bias=b2f,
+                          bias_mode=BIAS_COL, bias_zs=2 * bs, act=ACT_SHRINK, act_param=float(lam))
         t4 = _stage_h_blocks(o2, plan.gh, plan, B, C, nb)
         out = _stage_w_synthesis(t4, plan.gw, plan, B, C, skip)
         ctx.save_for_backward(y, o1, o2, w1q, w2q)
@@ -250,9 +276,7 @@ class _AFNOFilter(torch.autograd.Function):
                 db2.copy_(do2.reshape(B * nc, nb, nkx, 2 * bs).float().sum(dim=(0, 2)))
         # first layer
         dyt = torch.empty(B * nc, nb, nkx, 2, bs, dtype=dt, device=dev)
-        gemm(nkx, 2 * bs, 2 * hid, Operand(do1, ld=nb * 2 * hid, zs_lo=2 * hid, zs_hi=nkx * nb * 2 * hid),
-             Operand(w1q, ld=2 * bs, mn_major=True, zs_lo=2 * hid * 2 * bs),
-             Output(dyt, rs_lo=2 * bs, d_zlo=nkx * 2 * bs, d_zhi=nb * nkx * 2 * bs), zlo_n=nb, zhi_n=B * nc)
+        _tokens_to_blocks(do1, Operand(w1q, ld=2 * bs, mn_major=True, zs_lo=2 * hid * 2 * bs), dyt, plan, B, nb, 2 * bs, 2 * hid)
         gemm(2 * hid, 2 * bs, T, Operand(do1, ld=nb * 2 * hid, mn_major=True, zs_lo=2 * hid),
              Operand(y, ld=2 * C, mn_major=True, zs_lo=2 * bs),
              Output(dw1, rs_lo=2 * bs, d_zlo=2 * hid * 2 * bs), zlo_n=nb, accumulate=True, splits=0)

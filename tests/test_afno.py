@@ -45,6 +45,13 @@ def test_afno_chain_matches_fft_formulation(cfg):
         assert _rel(a, b) < 1e-5
 
 
+@pytest.mark.parametrize("cfg", [(1, 8, 14, 512, 64, 1, 1.0, 2), (2, 9, 14, 144, 2, 1, 0.7, 2), (1, 70, 12, 64, 1, 1, 1.0, 2),
+                                 (1, 5, 6, 16, 2, 1, 0.4, 2)])
+def test_afno_chain_narrow_and_wide_blocks(cfg):
+    """Both forms of the stages between tokens and blocks: many narrow blocks, wide ones, a full row tile, a single kept row."""
+    test_afno_chain_matches_fft_formulation(cfg)
+
+
 def test_afno_windows():
     assert afno.mode_window_v1(90, 180, 1.0) == (tuple(range(90)), 46)
     rows, cols = afno.mode_window_v1(90, 180, 0.5)
