@@ -167,3 +167,17 @@ def test_lamb_matches_a_direct_restatement():
             a = torch.view_as_real(p.detach()) if p.is_complex() else p.detach()
             b = torch.view_as_real(r) if r.is_complex() else r
             assert torch.allclose(a, b, rtol=1e-5, atol=1e-6)
+
+
+def test_sync_params_announces_changed_weights(tmp_path):
+    """Parameters are written through `.data`, which no version counter shows: what is derived from them must be dropped."""
+    import torch.distributed as dist
+    from makani_b200.ops import spectral
+    from makani_b200.parallel.helpers import sync_params
+    dist.init_process_group("gloo", init_method=f"file://{tmp_path}/store", rank=0, world_size=1)
+    try:
+        before = spectral._WEIGHT_EPOCH
+        sync_params(torch.nn.Linear(2, 2))
+        assert spectral._WEIGHT_EPOCH > before
+    finally:
+        dist.destroy_process_group()
