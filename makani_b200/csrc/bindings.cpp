@@ -58,6 +58,22 @@ void clear_error_flag(int64_t device) {
   if (it != m.end()) it->second.zero_();
 }
 
+// (current stream, what it is capturing) of a device: 0 nothing, -1 unknown, else the number of the capture, unique in the process
+std::pair<int64_t, int64_t> stream_state(int64_t device) {
+  c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
+  cudaStream_t s = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream();
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  int64_t cap = 0;
+  if (cudaStreamGetCaptureInfo(s, &st, &id) != cudaSuccess) {
+    (void)cudaGetLastError();
+    cap = -1;
+  } else if (st != cudaStreamCaptureStatusNone) {
+    cap = st == cudaStreamCaptureStatusActive ? static_cast<int64_t>(id) : -1;
+  }
+  return {reinterpret_cast<int64_t>(s), cap};
+}
+
 inline const char* base_ptr(const Tensor& t) { return static_cast<const char*>(t.data_ptr()); }
 
 // iparams layout: see makani_b200/ops/gemm.py
@@ -692,6 +708,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("set_gelu_tanh", [](int64_t on) { mk::set_gelu_tanh(static_cast<int>(on)); });
   m.def("read_error_flag", &read_error_flag);
   m.def("clear_error_flag", &clear_error_flag);
+  m.def("stream_state", &stream_state);
   m.def("inorm_fwd", &inorm_fwd);
   m.def("inorm_partial_stats", &inorm_partial_stats);
   m.def("cast_pad", &cast_pad);

@@ -225,7 +225,9 @@ def fold_weight_grad2(dw2: torch.Tensor) -> torch.Tensor:
 
 # Inference re-uses the expanded weights: they are kept as long as the parameter lives (a weak key, so that a new
 # parameter in recycled memory never meets them), and dropped when the parameter is modified in place (`_version`) or by
-# the fused optimiser, which writes through raw pointers and announces every update through `note_weights_changed`.
+# a writer that `_version` does not see and that says so through `note_weights_changed` (the fused optimiser, which writes
+# through raw pointers, and every write to `.data`).  They serve the stream that made them only, and never a capture: a
+# captured pass expands the weights itself, so that its replays read the values of the day from memory of their own.
 _WEIGHT_EPOCH = 0
 _EXPANDED = WeakTensorKeyDictionary()
 
@@ -259,7 +261,10 @@ def _planes(w: torch.Tensor, dtype) -> torch.Tensor:
 def _kept(w: torch.Tensor, dtype, make, keep: bool) -> torch.Tensor:
     if not keep or not w.is_cuda or w.is_inference():
         return make(w, dtype)
-    state = (w._version, _WEIGHT_EPOCH, w.data_ptr(), dtype, make)
+    stream, capture = _ext.require().stream_state(w.device.index)
+    if capture:
+        return make(w, dtype)
+    state = (w._version, _WEIGHT_EPOCH, w.data_ptr(), dtype, make, stream)
     hit = _EXPANDED.get(w)
     if hit is not None and hit[0] == state:
         return hit[1]

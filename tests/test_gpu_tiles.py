@@ -360,3 +360,71 @@ def test_batches_into_one_output_keep_their_own_sums(sign):
     _ext.check_device_errors(dev)
     # k / 16 truncations per batch, then z roundings of 2^-24 at random
     assert _rel(d, torch.einsum("zko,zki->oi", a.double(), b.double())) < (k / 16) * 2.0 ** -24 + 2.0 ** -24 * z ** 0.5 / 4
+
+
+def _spectral_layer(dev, seed=3):
+    from makani_b200.models.common.spectral_convolution import SpectralConv
+    from makani_b200.sht import InverseRealSHT, RealSHT
+    torch.manual_seed(seed)
+    fwd = RealSHT(17, 32, lmax=16, mmax=17, grid="equiangular").to(dev)
+    inv = InverseRealSHT(17, 32, lmax=16, mmax=17, grid="equiangular").to(dev)
+    m = SpectralConv(fwd, inv, 16, 16, operator_type="dhconv").to(dev)
+    x = torch.randn(1, 17, 32, 16, device=dev).to(torch.bfloat16).permute(0, 3, 1, 2)
+    return m, x
+
+
+def _count_expansions(monkeypatch):
+    from makani_b200.ops import spectral
+    made, real = [], spectral._planes
+    monkeypatch.setattr(spectral, "_planes", lambda w, dtype: made.append(1) or real(w, dtype))
+    return made
+
+
+def test_captured_pass_expands_its_own_weights(monkeypatch):
+    """A pass captured after eager ones, then weights that change and an eager pass that drops the kept expansion: the replay
+    reads the new weights, from memory of its own; and what a capture made serves no eager pass."""
+    dev = _dev()
+    m, x = _spectral_layer(dev)
+    made = _count_expansions(monkeypatch)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.no_grad(), torch.cuda.stream(side):
+        m(x)
+        m(x)
+        assert len(made) == 1                                  # kept between eager passes of one stream
+        side.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=side):
+            y = m(x)[0]
+        assert len(made) == 2
+        for k in range(3):
+            m.weight.copy_(torch.randn_like(m.weight))
+            want = m(x)[0].clone()
+            junk = [torch.randn_like(m.weight) for _ in range(4)]       # the dropped expansion's memory is handed out again
+            g.replay()
+            assert torch.equal(y, want), k
+            del junk
+        assert len(made) == 5
+        m.weight.data.mul_(2.0)
+        from makani_b200.ops.spectral import note_weights_changed
+        note_weights_changed()
+        want = m(x)[0]
+        g.replay()
+        assert torch.equal(y, want)
+    torch.cuda.synchronize()
+    _ext.check_device_errors(dev)
+
+
+def test_kept_weights_serve_one_stream(monkeypatch):
+    """An expansion may still be in flight on the stream that makes it: another stream makes its own."""
+    dev = _dev()
+    m, x = _spectral_layer(dev)
+    made = _count_expansions(monkeypatch)
+    with torch.no_grad():
+        a = m(x)[0]
+        torch.cuda.synchronize()
+        side = torch.cuda.Stream()
+        with torch.cuda.stream(side):
+            b = m(x)[0]
+        torch.cuda.synchronize()
+    assert len(made) == 2 and torch.equal(a, b)
