@@ -335,7 +335,7 @@ class _DistSpectralConv(torch.autograd.Function):
     def forward(ctx, x, w, plan_in: DistSHTPlan, plan_out: DistSHTPlan, want_resid: bool, train: bool):
         x = _to_cl(x)
         B, C = x.shape[0], x.shape[1]
-        wx = expand_weight(w, x.dtype, keep=not train)
+        wx = expand_weight(w, x.dtype, keep=not train, share=train)
         Co = wx.shape[1] // 2
         t2 = dist_sht_analysis(x, plan_in)
         s3, t3, ls = stage_contract(t2, wx, False, plan_in)

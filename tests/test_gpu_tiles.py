@@ -428,3 +428,87 @@ def test_kept_weights_serve_one_stream(monkeypatch):
             b = m(x)[0]
         torch.cuda.synchronize()
     assert len(made) == 2 and torch.equal(a, b)
+
+
+def test_recorded_passes_share_one_expansion(monkeypatch):
+    """The steps of a roll-out share one expansion, which goes with the last of their graphs; weights changed in place, announced or
+    not once the graphs are gone, or a new parameter in the same memory, are expanded anew."""
+    from makani_b200.ops import spectral
+    dev = _dev()
+    m, x = _spectral_layer(dev)
+    made = _count_expansions(monkeypatch)
+
+    def rollout(steps, inp=x):
+        y = inp
+        for _ in range(steps):
+            y = m(y)[0]
+        return y
+
+    y = rollout(3)
+    assert len(made) == 1
+    g = torch.autograd.grad(y.float().square().mean(), m.weight)[0]
+    assert len(spectral._RECORDED) == 1 and next(iter(spectral._RECORDED.values()))[1]() is None      # nothing outlives the graph
+    monkeypatch.setattr(spectral, "_RECORDED", type(spectral._RECORDED)())
+    real = spectral._kept
+    with monkeypatch.context() as mp:
+        mp.setattr(spectral, "_kept", lambda w, dtype, make, keep, share: real(w, dtype, make, False, False))
+        y2 = rollout(3)
+        g2 = torch.autograd.grad(y2.float().square().mean(), m.weight)[0]
+    assert torch.equal(y, y2) and torch.equal(g, g2)
+    del y, y2
+    a = rollout(1)
+    with torch.no_grad():
+        m.weight.mul_(1.5)                  # while a graph lives: the version shows it
+    b = rollout(1)
+    assert not torch.equal(a, b)
+    del a, b
+    m.weight.data.mul_(0.5)                 # unannounced: with no graph alive nothing is kept that this could make stale
+    got = rollout(1)
+    spectral.note_weights_changed()
+    with torch.no_grad():
+        assert torch.equal(got, m(x)[0])
+    del got
+    seen = set()
+    for k in range(4):                      # new parameters, one after the other in the same memory
+        m.weight = torch.nn.Parameter(torch.full_like(m.weight.detach(), complex(k, -k)))
+        seen.add(m.weight.data_ptr())
+        got = rollout(1)
+        with torch.no_grad():
+            spectral.note_weights_changed()
+            assert torch.equal(got, m(x)[0]), k
+        del got
+    _ext.check_device_errors(dev)
+
+
+def test_captured_training_shares_inside_the_capture(monkeypatch):
+    """Two forward passes, their backward pass and an update in one graph: one expansion per replay, of that replay's weights."""
+    dev = _dev()
+    m, x = _spectral_layer(dev)
+    made = _count_expansions(monkeypatch)
+
+    def step():
+        y = m(m(x)[0])[0]
+        g = torch.autograd.grad(y.float().square().mean(), m.weight)[0]
+        with torch.no_grad():
+            m.weight.add_(g, alpha=-10.0)
+        return y
+
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    start = m.weight.detach().clone()
+    with torch.cuda.stream(side):
+        want = [step().detach().clone() for _ in range(4)]
+        assert len(made) == 4
+        with torch.no_grad():
+            m.weight.copy_(start)
+        side.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            y = step()
+        assert len(made) == 5
+        for k in range(4):
+            graph.replay()
+            assert _rel(y, want[k]) < 1e-6, k
+        assert _rel(want[3], want[0]) > 1e-3
+    torch.cuda.synchronize()
+    _ext.check_device_errors(dev)
