@@ -137,7 +137,9 @@ def instance_norm(x: torch.Tensor, weight, bias, eps: float = 1e-6, act: str = "
 
 
 def row_sums(x: torch.Tensor, C: int) -> torch.Tensor:
-    """fp32 [C]: sum over the rows of a dense bf16 CUDA tensor whose storage is rows of C columns (C a multiple of 8)."""
+    """fp32 [C]: sum over the rows of a contiguous bf16 CUDA tensor [..., C]."""
+    if C % 8 or x.data_ptr() % 16:          # the kernel reads whole 16-byte vectors
+        return x.reshape(-1, C).float().sum(0)
     out = torch.zeros(C, dtype=torch.float32, device=x.device)
     _ext.require().colsum(x, out)
     return out
@@ -146,7 +148,7 @@ def row_sums(x: torch.Tensor, C: int) -> torch.Tensor:
 def channel_sums(x: torch.Tensor) -> torch.Tensor:
     """sum over (batch, H, W) of a 4-D activation in fp32 (bias gradients)."""
     if _ext.native() and x.is_cuda and x.dtype == torch.bfloat16 and _is_cl(x) and x.shape[1] % 8 == 0:
-        return row_sums(x, x.shape[1])
+        return row_sums(x.permute(0, 2, 3, 1), x.shape[1])
     if x.is_cuda and x.dtype == torch.bfloat16 and x.is_contiguous():
         ext = _ext.require()
         B, C = x.shape[0], x.shape[1]

@@ -512,3 +512,16 @@ def test_captured_training_shares_inside_the_capture(monkeypatch):
         assert _rel(want[3], want[0]) > 1e-3
     torch.cuda.synchronize()
     _ext.check_device_errors(dev)
+
+
+@pytest.mark.parametrize("shift", [1, 4, 8])
+def test_linear_bias_alone_trains(shift):
+    """A linear layer with a frozen weight on inputs without gradient: its bias trains also where the gradient handed in is no
+    multiple of 16 bytes into its storage."""
+    from makani_b200.ops.linear import linear_lastdim
+    dev = _dev()
+    x = torch.randn(3, 50, 24, device=dev).to(torch.bfloat16)
+    w, b = torch.randn(16, 24, device=dev), torch.zeros(16, device=dev, requires_grad=True)
+    dy = torch.randn(3 * 50 * 16 + shift, device=dev).to(torch.bfloat16)[shift:].view(3, 50, 16)
+    g, = torch.autograd.grad(linear_lastdim(x, w, b), b, dy)
+    assert _rel(g, dy.double().sum((0, 1))) < 2.0 ** -22
