@@ -293,14 +293,21 @@ void inorm_partial_stats(const Tensor& x, Tensor& sums) {
              "inorm_partial_stats");
 }
 
+static Tensor colsum_buffer(const Tensor& x, int64_t rows, int64_t C, int64_t groups) {
+  return torch::empty({static_cast<int64_t>(mk::colsum_scratch(rows, static_cast<int>(C), static_cast<int>(groups)))},
+                      x.options().dtype(torch::kFloat32));
+}
+
 // sums over all rows of x, whose storage is `rows` dense rows of out.numel() columns (contiguous tokens or channels-last)
 void colsum(const Tensor& x, Tensor& out) {
   MK_CHECK(x.is_cuda() && x.scalar_type() == torch::kBFloat16 && x.is_non_overlapping_and_dense(), "colsum: dense bf16 CUDA tensor expected");
   MK_CHECK(out.is_cuda() && out.scalar_type() == torch::kFloat32 && out.is_contiguous() && out.numel() > 0 && x.numel() % out.numel() == 0,
            "colsum: bad output");
   c10::cuda::CUDAGuard guard(x.device());
-  check_cuda(mk::colsum(reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()), out.data_ptr<float>(), x.numel() / out.numel(),
-                        static_cast<int>(out.numel()), cur_stream()),
+  const int64_t C = out.numel(), rows = x.numel() / C;
+  Tensor part = colsum_buffer(x, rows, C, 1);
+  check_cuda(mk::colsum(reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()), out.data_ptr<float>(),
+                        part.numel() ? part.data_ptr<float>() : nullptr, rows, static_cast<int>(C), cur_stream()),
              "colsum");
 }
 
@@ -382,9 +389,10 @@ void colsum_groups(const Tensor& x, Tensor& out, int64_t outer, int64_t groups, 
   const int64_t C = x.numel() / (outer * groups * inner);
   MK_CHECK(out.is_cuda() && out.scalar_type() == torch::kFloat32 && out.is_contiguous() && out.numel() == groups * C, "colsum_groups: bad output");
   c10::cuda::CUDAGuard guard(x.device());
-  check_cuda(mk::colsum(reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()), out.data_ptr<float>(), outer * inner,
-                        static_cast<int>(C), cur_stream(), static_cast<int>(groups), inner * C, static_cast<int>(inner),
-                        groups * inner * C),
+  Tensor part = colsum_buffer(x, outer * inner, C, groups);
+  check_cuda(mk::colsum(reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()), out.data_ptr<float>(),
+                        part.numel() ? part.data_ptr<float>() : nullptr, outer * inner, static_cast<int>(C), cur_stream(),
+                        static_cast<int>(groups), inner * C, static_cast<int>(inner), groups * inner * C),
              "colsum_groups");
 }
 

@@ -598,13 +598,15 @@ __global__ void __launch_bounds__(CL_THREADS, MODE == 0 ? 2 : 1) inorm_cl_apply_
 
 // ------------------------------------------------------------------------------------------ column sums
 
-// out[g, c] += sum_r x_g[r, c] for bf16 rows of C columns (a multiple of 8): the bias gradients.  Row r of group g sits at
-// g * gstride + (r / inner) * ostride + (r % inner) * C elements (plain rows: inner = rows).  One read of x; thread (v, r)
+// out[g, c] = sum_r x_g[r, c] for bf16 rows of C columns (a multiple of 8): the bias gradients.  Row r of group g sits at
+// g * gstride + (r / inner) * ostride + (r % inner) * C elements (plain rows: inner = 0).  One read of x; thread (v, r)
 // owns eight columns and every R-th row of its slab with eight 16-byte loads in flight, so the HBM latency is covered at
-// two CTAs per SM.  16200 tokens: 3072 columns 27 us, 768 columns 10 us, where a cast to fp32 and a torch sum took 185 and
-// 63 us; 2048 x 16: 4 us, where the statistics kernel of the instance norm took 37 us.
+// two CTAs per SM.  Every sum is taken in one fixed order, inside a CTA and over the slabs, so a call repeats itself bit for bit:
+// the CTAs leave their sums in `part` ([groups][slabs][C]) and a second launch adds the slabs (one slab: straight to out).
+// 16200 tokens: 3072 columns 20 us, 768 columns 9.5 us; 1038240 tokens of 384 columns 122 us (6.6 TB/s); 2048 x 16: 3.6 us.  Atomics
+// into a cleared buffer took 18, 11.7, 119 and 4.0 us, each time with other bits, 3.6e-7 off 64 bits where this is 1e-7 off.
 constexpr int CS_THREADS = 256;
-__global__ void __launch_bounds__(CS_THREADS) colsum_kernel(const uint4* __restrict__ x, float* __restrict__ out, long long rows,
+__global__ void __launch_bounds__(CS_THREADS) colsum_kernel(const uint4* __restrict__ x, float* __restrict__ part, long long rows,
                                                             int V, int vb, int slab, int inner, long long ostride_v,
                                                             long long gstride_v) {
   __shared__ __align__(16) float sh[CS_THREADS * 8];
@@ -612,8 +614,7 @@ __global__ void __launch_bounds__(CS_THREADS) colsum_kernel(const uint4* __restr
   const int nv = min(vb, V - v0);          // 16-byte columns of this CTA
   const int R = CS_THREADS / vb;
   const int v = threadIdx.x % vb, r = threadIdx.x / vb;
-  for (int i = threadIdx.x; i < nv * 8; i += CS_THREADS) sh[i] = 0.f;
-  __syncthreads();
+  const bool fold = vb < 32 && (vb & (vb - 1)) == 0;      // lanes with the same columns: shuffles, then one lane per warp
   if (r < R && v < nv) {
     float a[8];
 #pragma unroll
@@ -642,7 +643,6 @@ __global__ void __launch_bounds__(CS_THREADS) colsum_kernel(const uint4* __restr
       for (int u = 0; u < 8; ++u) add(q[u]);
     }
     for (; t < t1; t += R) add(__ldg(row(t)));
-    const bool fold = vb < 32 && (vb & (vb - 1)) == 0;      // lanes with the same columns: shuffles before the atomics
     if (fold) {
       for (int o = 16; o >= vb; o >>= 1) {
 #pragma unroll
@@ -650,14 +650,40 @@ __global__ void __launch_bounds__(CS_THREADS) colsum_kernel(const uint4* __restr
       }
     }
     if (!fold || (threadIdx.x & 31) < vb) {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) atomicAdd(&sh[v * 8 + j], a[j]);
+      // row `r` of sums, or the warp's: vb * 8 floats each
+      float4* const q = reinterpret_cast<float4*>(sh + ((fold ? threadIdx.x >> 5 : r) * vb + v) * 8);
+      q[0] = make_float4(a[0], a[1], a[2], a[3]);
+      q[1] = make_float4(a[4], a[5], a[6], a[7]);
     }
   }
   __syncthreads();
-  for (int i = threadIdx.x * 4; i < nv * 8; i += CS_THREADS * 4)
-    atomicAdd(reinterpret_cast<float4*>(out + (static_cast<long long>(blockIdx.z) * V + v0) * 8 + i),
-              *reinterpret_cast<const float4*>(sh + i));
+  const int n = fold ? CS_THREADS / 32 : R;
+  float* const dst = part + ((static_cast<long long>(blockIdx.z) * gridDim.y + blockIdx.y) * V + v0) * 8;
+  for (int i = threadIdx.x; i < nv * 8; i += CS_THREADS) {
+    float t = 0.f;
+    for (int k = 0; k < n; ++k) t += sh[k * vb * 8 + i];
+    dst[i] = t;
+  }
+}
+
+// out[g, c] = sum over the slabs (592 of them at most); 32 columns by 32 slabs at a time per CTA.  grid (ceil(C / 32), groups)
+__global__ void __launch_bounds__(1024) colsum_slabs_kernel(const float* __restrict__ part, float* __restrict__ out, int slabs, int C) {
+  __shared__ float sh[32][33];
+  const int c = blockIdx.x * 32 + threadIdx.x;
+  float a = 0.f;
+  if (c < C) {
+    const float* p = part + static_cast<long long>(blockIdx.y) * slabs * C + c;
+#pragma unroll 8
+    for (int k = threadIdx.y; k < slabs; k += 32) a += p[static_cast<long long>(k) * C];
+  }
+  sh[threadIdx.y][threadIdx.x] = a;
+  __syncthreads();
+  // warp w adds up column w
+  a = sh[threadIdx.x][threadIdx.y];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+  const int cw = blockIdx.x * 32 + threadIdx.y;
+  if (threadIdx.x == 0 && cw < C) out[static_cast<long long>(blockIdx.y) * C + cw] = a;
 }
 
 // ------------------------------------------------------------------------------------------ Lp norms
@@ -1303,22 +1329,44 @@ cudaError_t inorm_cl_apply(const __nv_bfloat16* x, const __nv_bfloat16* dy, __nv
   return cudaGetLastError();
 }
 
-cudaError_t colsum(const __nv_bfloat16* x, float* out, long long rows, int C, cudaStream_t s, int groups, long long gstride,
-                   int inner, long long ostride) {
-  if (rows <= 0 || C <= 0 || groups <= 0) return cudaSuccess;
-  if ((C & 7) || (gstride & 7) || (ostride & 7) || groups > 65535 || (inner > 0 && rows >= (1ll << 31)) || !aligned16(x) ||
-      !aligned16(out))
-    return cudaErrorInvalidValue;
-  const int V = C / 8;
-  const int parts = (V + CS_THREADS - 1) / CS_THREADS;
-  const int vb = (V + parts - 1) / parts;
-  const int R = CS_THREADS / vb;
+namespace {
+struct ColsumPlan {
+  int V, parts, vb;         // 16-byte columns, CTAs along them, columns of one CTA
+  long long slab, slabs;    // rows of one CTA, CTAs along the rows
+};
+ColsumPlan colsum_plan(long long rows, int C, int groups) {
+  ColsumPlan p;
+  p.V = C / 8;
+  p.parts = (p.V + CS_THREADS - 1) / CS_THREADS;
+  p.vb = (p.V + p.parts - 1) / p.parts;
+  const int R = CS_THREADS / p.vb;
   // about four CTAs per SM, each with at least one full step of eight rows per thread
-  long long slab = (rows * parts * groups + 4LL * sm_count() - 1) / (4LL * sm_count());
-  if (slab < 8LL * R) slab = 8LL * R;
-  dim3 grid(parts, static_cast<unsigned>((rows + slab - 1) / slab), groups);
-  colsum_kernel<<<grid, CS_THREADS, 0, s>>>(reinterpret_cast<const uint4*>(x), out, rows, V, vb, static_cast<int>(slab), inner,
-                                            ostride / 8, gstride / 8);
+  p.slab = (rows * p.parts * groups + 4LL * sm_count() - 1) / (4LL * sm_count());
+  if (p.slab < 8LL * R) p.slab = 8LL * R;
+  p.slabs = (rows + p.slab - 1) / p.slab;
+  return p;
+}
+}  // namespace
+
+long long colsum_scratch(long long rows, int C, int groups) {
+  if (rows <= 0 || C <= 0 || (C & 7) || groups <= 0) return 0;
+  const ColsumPlan p = colsum_plan(rows, C, groups);
+  return p.slabs > 1 ? p.slabs * groups * C : 0;
+}
+
+cudaError_t colsum(const __nv_bfloat16* x, float* out, float* scratch, long long rows, int C, cudaStream_t s, int groups,
+                   long long gstride, int inner, long long ostride) {
+  if (C <= 0 || groups <= 0) return cudaSuccess;
+  if (rows <= 0) return cudaMemsetAsync(out, 0, sizeof(float) * static_cast<size_t>(C) * groups, s);
+  if ((C & 7) || (gstride & 7) || (ostride & 7) || groups > 65535 || (inner > 0 && rows >= (1ll << 31)) || !aligned16(x) ||
+      !aligned16(out) || (scratch == nullptr && colsum_scratch(rows, C, groups) > 0))
+    return cudaErrorInvalidValue;
+  const ColsumPlan p = colsum_plan(rows, C, groups);
+  float* const part = p.slabs > 1 ? scratch : out;
+  colsum_kernel<<<dim3(p.parts, static_cast<unsigned>(p.slabs), groups), CS_THREADS, 0, s>>>(
+      reinterpret_cast<const uint4*>(x), part, rows, p.V, p.vb, static_cast<int>(p.slab), inner, ostride / 8, gstride / 8);
+  if (p.slabs > 1)
+    colsum_slabs_kernel<<<dim3((C + 31) / 32, groups), dim3(32, 32), 0, s>>>(part, out, static_cast<int>(p.slabs), C);
   return cudaGetLastError();
 }
 

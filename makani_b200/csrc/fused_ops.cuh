@@ -58,9 +58,11 @@ cudaError_t inorm_cl_apply(const __nv_bfloat16* x, const __nv_bfloat16* dy, __nv
                            const float* sums, float* stats, int B, int C, long long T, double count, float eps, int act, int mode,
                            cudaStream_t s, const StatExchange* xch = nullptr);
 
-// out[g, c] += sum over the rows of group g of x (C % 8 == 0, 16-byte aligned; out [groups, C] zero-initialised by the caller).
-// Row r of group g: g * gstride + (r / inner) * ostride + (r % inner) * C; inner = 0: rows follow one another.
-cudaError_t colsum(const __nv_bfloat16* x, float* out, long long rows, int C, cudaStream_t s, int groups = 1,
+// out[g, c] = sum over the rows of group g of x (C % 8 == 0, 16-byte aligned), in one fixed order; `scratch` holds
+// colsum_scratch() floats.  Row r of group g: g * gstride + (r / inner) * ostride + (r % inner) * C; inner = 0: rows follow
+// one another.
+long long colsum_scratch(long long rows, int C, int groups = 1);
+cudaError_t colsum(const __nv_bfloat16* x, float* out, float* scratch, long long rows, int C, cudaStream_t s, int groups = 1,
                    long long gstride = 0, int inner = 0, long long ostride = 0);
 
 // ---- AFNO block weights: one layer's tensors (see the kernels), two layers per launch ----

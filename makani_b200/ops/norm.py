@@ -140,7 +140,7 @@ def row_sums(x: torch.Tensor, C: int) -> torch.Tensor:
     """fp32 [C]: sum over the rows of a contiguous bf16 CUDA tensor [..., C]."""
     if C % 8 or x.data_ptr() % 16:          # the kernel reads whole 16-byte vectors
         return x.reshape(-1, C).float().sum(0)
-    out = torch.zeros(C, dtype=torch.float32, device=x.device)
+    out = torch.empty(C, dtype=torch.float32, device=x.device)
     _ext.require().colsum(x, out)
     return out
 

@@ -525,3 +525,34 @@ def test_linear_bias_alone_trains(shift):
     dy = torch.randn(3 * 50 * 16 + shift, device=dev).to(torch.bfloat16)[shift:].view(3, 50, 16)
     g, = torch.autograd.grad(linear_lastdim(x, w, b), b, dy)
     assert _rel(g, dy.double().sum((0, 1))) < 2.0 ** -22
+
+
+@pytest.mark.parametrize("rows,c", [(1, 8), (2049, 24), (5000, 256), (16200, 768), (33, 4104), (1000003, 16), (115200, 384)])
+def test_column_sums_repeat_themselves(rows, c):
+    """One fixed order of the additions: the same bits on every call, whatever else keeps the SMs busy."""
+    from makani_b200.ops.norm import row_sums
+    dev = _dev()
+    x = (torch.randn(rows, c, device=dev, generator=torch.Generator(dev).manual_seed(c)) * 1e3).to(torch.bfloat16)
+    first = row_sums(x, c)
+    side, busy = torch.cuda.Stream(), torch.randn(4096, 4096, device=dev)
+    for k in range(8):
+        with torch.cuda.stream(side):
+            busy = torch.sin(busy)
+        assert torch.equal(row_sums(x, c), first), k
+    torch.cuda.synchronize()
+
+
+def test_afno_bias_gradients_repeat_themselves():
+    from makani_b200.models.networks.afnonet import AFNO2D
+    dev = _dev()
+    torch.manual_seed(2)
+    m = AFNO2D(128, num_blocks=4).to(dev)
+    x, dy = (torch.randn(2, 24, 48, 128, device=dev).to(torch.bfloat16) for _ in range(2))
+    grads = [torch.autograd.grad(m(x), [m.b1, m.b2], dy) for _ in range(6)]
+    for g in grads[1:]:
+        assert torch.equal(g[0], grads[0][0]) and torch.equal(g[1], grads[0][1])
+
+
+def test_column_sums_of_no_rows():
+    from makani_b200.ops.norm import row_sums
+    assert torch.equal(row_sums(torch.empty(0, 16, device=_dev(), dtype=torch.bfloat16), 16).cpu(), torch.zeros(16))
