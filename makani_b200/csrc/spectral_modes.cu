@@ -30,8 +30,7 @@ __device__ __forceinline__ void cfmac(float2& acc, float2 a, float2 b) {   // ac
 }
 
 constexpr int TS = 128;   // threads per CTA along the mode index
-constexpr int TO = 4;     // channels per thread on the summed-over-nothing side (a mode's activations are loaded once for four)
-constexpr int TU = 4;     // steps of the channel sum whose loads are in flight together
+constexpr int TU = 8;     // steps of the channel sum whose loads are in flight together
 
 // NV neighbouring modes of one thread: one 16-byte access (NV = 2) where rows keep that alignment, else 8 bytes.
 template <int NV>
@@ -77,71 +76,64 @@ __device__ __forceinline__ void st_modes(float2* p, const Modes<NV>& m, bool str
 // The sum over one channel index of the weights, forward (over i) or input gradient (over o):
 //   CONJ 0: out[b, o, s] = sum_i a[b, i, s] w[i, o, s]        P = O outputs, Q = I summed
 //   CONJ 1: out[b, i, s] = sum_o a[b, o, s] conj(w[i, o, s])  P = I outputs, Q = O summed
-// with w at (q * wq + p * wp) rows of S modes.  Bound by reading w once (8 bytes per complex product): the loads of TU
-// steps times TO outputs are in flight together (256 bytes per thread with NV = 2), and a pair of samples (NB = 2) shares
-// one pass over w.  64 channels, 180 x 180 modes (1.06 GB of weights): 240 -> 185 us forward, 165 -> 174 us backward.  grid (ceil(S / (TS NV)), ceil(P / TO), ceil(B / NB))
+// with w at (q * wq + p * wp) rows of S modes.  Bound by reading w once (8 bytes per complex product): one output per thread with
+// the loads of TU steps in flight, and a pair of samples (NB = 2) shares one pass over w.  Four outputs per thread, which
+// load the activations once for four, leave too few CTAs where there are few channels or modes, and their loads go to four
+// distant rows.  us, one output / four / one thread per output and sample without loads in flight, input gradient (forward):
+//   64 channels, 180 x 180 modes  173 / 185 / 177 (174 / 187 / 242)      two samples  199 / 225 / 342 (200 / 223 / 420)
+//   16 x 64, 90 x 90               27 /  61 /  45  (21 /  25 /  26)      24, 24 x 24   12 /  26 /  21  (12 /  27 /  31)
+// grid (ceil(S / (TS NV)), P, ceil(B / NB))
 template <int NV, int NB, int CONJ>
 __global__ void __launch_bounds__(TS) diag_sum_kernel(const float2* __restrict__ a, const float2* __restrict__ w,
                                                       float2* __restrict__ out, int B, int P, int Q, long long wp, long long wq,
                                                       long long S) {
   const long long s = (static_cast<long long>(blockIdx.x) * TS + threadIdx.x) * NV;
-  const int p0 = blockIdx.y * TO, b0 = blockIdx.z * NB;
+  const int p = blockIdx.y, b0 = blockIdx.z * NB;
   if (s >= S) return;
-  const int np = min(TO, P - p0), nb = min(NB, B - b0);
-  Modes<NV> acc[NB][TO];
+  const int nb = min(NB, B - b0);
+  Modes<NV> acc[NB];
 #pragma unroll
   for (int b = 0; b < NB; ++b)
 #pragma unroll
-    for (int j = 0; j < TO; ++j)
-#pragma unroll
-      for (int h = 0; h < NV; ++h) acc[b][j].v[h] = make_float2(0.f, 0.f);
+    for (int h = 0; h < NV; ++h) acc[b].v[h] = make_float2(0.f, 0.f);
   const float2* const ap = a + static_cast<long long>(b0) * Q * S + s;
-  const float2* const wr = w + p0 * wp * S + s;
-  auto step = [&](const Modes<NV> (&av)[NB], const Modes<NV> (&wv)[TO]) {
+  const float2* const wr = w + p * wp * S + s;
+  auto step = [&](const Modes<NV> (&av)[NB], const Modes<NV>& wv) {
 #pragma unroll
     for (int b = 0; b < NB; ++b)
 #pragma unroll
-      for (int j = 0; j < TO; ++j)
-#pragma unroll
-        for (int h = 0; h < NV; ++h) {
-          if (CONJ) cfmac(acc[b][j].v[h], av[b].v[h], wv[j].v[h]);
-          else cfma(acc[b][j].v[h], av[b].v[h], wv[j].v[h]);
-        }
-  };
-  int q = 0;
-  if (np == TO && nb == NB) {
-    for (; q + TU <= Q; q += TU) {
-      Modes<NV> av[TU][NB], wv[TU][TO];
-#pragma unroll
-      for (int u = 0; u < TU; ++u) {
-#pragma unroll
-        for (int j = 0; j < TO; ++j) wv[u][j] = ld_modes_once<NV>(wr + ((q + u) * wq + j * wp) * S);
-#pragma unroll
-        for (int b = 0; b < NB; ++b) av[u][b] = ld_modes<NV>(ap + (static_cast<long long>(b) * Q + q + u) * S);
+      for (int h = 0; h < NV; ++h) {
+        if (CONJ) cfmac(acc[b].v[h], av[b].v[h], wv.v[h]);
+        else cfma(acc[b].v[h], av[b].v[h], wv.v[h]);
       }
-#pragma unroll
-      for (int u = 0; u < TU; ++u) step(av[u], wv[u]);
-    }
-  }
-  for (; q < Q; ++q) {
-    Modes<NV> av[NB], wv[TO];
-#pragma unroll
-    for (int j = 0; j < TO; ++j) wv[j] = ld_modes_once<NV>(wr + (q * wq + (j < np ? j : 0) * wp) * S);
+  };
+  auto load = [&](int q, Modes<NV> (&av)[NB], Modes<NV>& wv) {
+    wv = ld_modes_once<NV>(wr + q * wq * S);
 #pragma unroll
     for (int b = 0; b < NB; ++b) av[b] = ld_modes<NV>(ap + (static_cast<long long>(b < nb ? b : 0) * Q + q) * S);
+  };
+  int q = 0;
+  for (; q + TU <= Q; q += TU) {
+    Modes<NV> av[TU][NB], wv[TU];
+#pragma unroll
+    for (int u = 0; u < TU; ++u) load(q + u, av[u], wv[u]);
+#pragma unroll
+    for (int u = 0; u < TU; ++u) step(av[u], wv[u]);
+  }
+  for (; q < Q; ++q) {
+    Modes<NV> av[NB], wv;
+    load(q, av, wv);
     step(av, wv);
   }
 #pragma unroll
   for (int b = 0; b < NB; ++b)
-#pragma unroll
-    for (int j = 0; j < TO; ++j)
-      if (b < nb && j < np) st_modes<NV>(out + (static_cast<long long>(b0 + b) * P + p0 + j) * S + s, acc[b][j], false);
+    if (b < nb) st_modes<NV>(out + (static_cast<long long>(b0 + b) * P + p) * S + s, acc[b], false);
 }
 
 // dw[i, o, s] = sum_b conj(a[b, i, s]) dy[b, o, s]: bound by writing dw; a thread makes TI x TO weights from TI + TO loads (one
 // weight from two loads before, with 8-byte stores: 538 -> 165 us for the 1.06 GB above, 6.4 TB/s).
 // grid (ceil(S / (TS NV)), ceil(O / TO), ceil(I / TI))
-constexpr int TI = 4;
+constexpr int TI = 4, TO = 4;
 template <int NV>
 __global__ void __launch_bounds__(TS) diag_wgrad_kernel(const float2* __restrict__ a, const float2* __restrict__ dy,
                                                         float2* __restrict__ dw, int B, int I, int O, long long S) {
@@ -222,7 +214,7 @@ cudaError_t diag_sum(const float* a, const float* w, float* out, int B, int P, i
   float2* op = reinterpret_cast<float2*>(out);
   const int nb = B > 1 ? 2 : 1;
   const bool pairs = pairs_ok(a, w, out, S);
-  const dim3 grid(cdiv(S, pairs ? 2 * TS : TS), cdiv(P, TO), cdiv(B, nb));
+  const dim3 grid(cdiv(S, pairs ? 2 * TS : TS), P, cdiv(B, nb));
   if (pairs && nb == 2) diag_sum_kernel<2, 2, CONJ><<<grid, TS, 0, st>>>(ap, wr, op, B, P, Q, wp, wq, S);
   else if (pairs) diag_sum_kernel<2, 1, CONJ><<<grid, TS, 0, st>>>(ap, wr, op, B, P, Q, wp, wq, S);
   else if (nb == 2) diag_sum_kernel<1, 2, CONJ><<<grid, TS, 0, st>>>(ap, wr, op, B, P, Q, wp, wq, S);

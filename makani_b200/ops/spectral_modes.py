@@ -6,7 +6,7 @@
 
 With a batch of one or two samples per GPU these are matrix-vector products per mode: there is no tile for the tensor
 cores, the cost is reading the weights once.  The kernels (`csrc/spectral_modes.cu`) run their threads along the mode
-index, read every weight element once per sample with streaming loads, and serve forward, input gradient (conjugated
+index, read every weight element once per pair of samples with streaming loads, and serve forward, input gradient (conjugated
 weights) and weight gradient.  Anything that is not contiguous complex64 on CUDA goes through `torch.einsum`.
 """
 
