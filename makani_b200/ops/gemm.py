@@ -176,6 +176,42 @@ def _emulate(M, N, K, A: Operand, B: Operand, D: Output, zlo_n, zhi_n, alpha, bi
         fd.index_put_((idx,), vals)
 
 
+def _emulate_complex(mode, M, N, K, A: Operand, B: Operand, D: Output, d_half, zlo_n, zhi_n, a_plane, b_plane, resid, accumulate,
+                     rmax, kmax):
+    fa, fb, fd = _flat(A.tensor), _flat(B.tensor), _flat(D.tensor)
+    cdt = torch.float64 if fa.dtype == torch.float64 else torch.float32
+
+    def view(op: Operand, flat, at, rows, zs_lo):
+        rs, ks = (1, op.ld) if op.mn_major else (op.ld, 1)
+        return flat[op.offset + at:].as_strided((zhi_n, zlo_n, rows, K), (op.zs_hi, zs_lo, rs, ks)).to(cdt)
+
+    dev = fa.device
+    zh = torch.arange(zhi_n, device=dev).view(-1, 1, 1, 1)
+    zl = torch.arange(zlo_n, device=dev).view(1, -1, 1, 1)
+    r = torch.arange(M, device=dev).view(1, 1, -1, 1)
+    n = torch.arange(N, device=dev).view(1, 1, 1, -1)
+    kmask = (torch.arange(K, device=dev).view(1, 1, 1, -1) < kmax[0] * zh + kmax[1]).to(cdt)
+    rmask = (r < rmax[0] * zh + rmax[1]).to(cdt)
+    minus = {1: (0, 1), 2: (1, 0), 3: (1, 1)}[mode]       # (part of the result, segment of the k loop)
+    for h in range(2):
+        acc = torch.zeros(zhi_n, zlo_n, M, N, dtype=cdt, device=dev)
+        for sg in range(2):
+            if mode == 3:
+                a, b = view(A, fa, (sg ^ h) * a_plane, M, A.zs_lo), view(B, fb, sg * b_plane, N, 0)
+            else:
+                a, b = view(A, fa, sg * K * (A.ld if A.mn_major else 1), M, A.zs_lo), view(B, fb, (h ^ sg) * b_plane, N, 0)
+            part = torch.matmul(a * kmask, b.transpose(-1, -2)) * rmask
+            acc = acc - part if (h, sg) == minus else acc + part
+        idx = (D.offset + h * d_half + zh * D.d_zhi + zl * D.d_zlo + r * D.rs_lo + n).expand(zhi_n, zlo_n, M, N).reshape(-1)
+        vals = acc.reshape(-1)
+        if resid is not None:
+            vals = vals + _flat(resid)[idx].to(cdt)
+        if accumulate:
+            fd.index_add_(0, idx, vals.to(fd.dtype))
+        else:
+            fd.index_put_((idx,), vals.to(fd.dtype))
+
+
 def gemm(M: int, N: int, K: int, A: Operand, B: Operand, D: Output, *, zlo_n: int = 1, zhi_n: int = 1, alpha: float = 1.0,
          bias: Optional[torch.Tensor] = None, bias_mode: int = BIAS_NONE, act: int = ACT_NONE,
          resid: Optional[torch.Tensor] = None, resid_offset: int = 0, preact: Optional[torch.Tensor] = None,
@@ -225,7 +261,7 @@ def gemm(M: int, N: int, K: int, A: Operand, B: Operand, D: Output, *, zlo_n: in
 
 def gemm_complex(mode: int, M: int, N: int, K: int, A: Operand, B: Operand, D: Output, d_half: int, *, zlo_n: int = 1, zhi_n: int = 1,
                  a_plane: int = 0, b_plane: int = 0, resid=None, accumulate: bool = False, rmax=(0, _BIG), kmax=(0, _BIG)) -> None:
-    """Product of complex operands given as real and imaginary planes (CUDA bf16; N and K count one part):
+    """Product of complex operands given as real and imaginary planes (bf16 on CUDA; N and K count one part):
 
         mode 1   D(h)[r, n] = sum_s sum_k A[r, s K + k] B(h ^ s)[n, k],   minus for h = 0, s = 1:  A times W
         mode 2   the same, minus for h = 1, s = 0:                                                A times conj(W)
@@ -233,6 +269,9 @@ def gemm_complex(mode: int, M: int, N: int, K: int, A: Operand, B: Operand, D: O
 
     `b_plane` / `a_plane`: elements between the planes of an operand; `d_half`: between the parts of D.  `rmax`, `kmax`: (slope,
     offset) of the valid rows / contributing k in the batch index z_hi, as in `Tri`.  `resid` is laid out like D and added."""
+    if not A.tensor.is_cuda:
+        _emulate_complex(mode, M, N, K, A, B, D, d_half, zlo_n, zhi_n, a_plane, b_plane, resid, accumulate, rmax, kmax)
+        return
     ip = [mode, M, N, K, zlo_n, zhi_n, rmax[0], rmax[1], kmax[0], kmax[1],
           A.offset, int(A.mn_major), A.ld, A.zs_lo, A.zs_hi, a_plane,
           B.offset, int(B.mn_major), B.ld, B.zs_hi, b_plane,

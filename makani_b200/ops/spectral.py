@@ -183,30 +183,17 @@ def contract_wgrad2(dt: torch.Tensor, t2: torch.Tensor, l0: int = 0, m0: int = 0
 
         dWr[l, o, c] = sum_{b, m <= l} dTr T2r + dTi T2i        dWi[l, o, c] = sum_{b, m <= l} dTi T2r - dTr T2i
 
-    On CUDA one complex product over the planes of both operands.  Otherwise both are GEMMs over k = (m, ri) (the two parts sit
-    side by side in memory); the second one reads a copy of dT with its parts swapped and one sign flipped.  `l0`, `m0`:
-    global offsets of the local (l, m) block."""
+    One complex product over the planes of both operands per sample.  `l0`, `m0`: global offsets of the local (l, m) block."""
     B, L, M, nq = dt.shape
     co, ci = nq // 2, t2.shape[3] // 2
-    if dt.is_cuda and dt.dtype == torch.bfloat16 and co % 8 == 0 and ci % 8 == 0 and dt.is_contiguous() and t2.is_contiguous() and _ext.native():
-        out = (torch.empty if B == 1 else torch.zeros)(2, L, co, ci, dtype=torch.float32, device=dt.device)
-        for b in range(B):
-            gemm_complex(3, co, ci, M,
-                         Operand(dt, ld=nq, mn_major=True, zs_hi=M * nq, offset=b * L * M * nq),
-                         Operand(t2, ld=2 * ci, mn_major=True, zs_hi=M * 2 * ci, offset=b * L * M * 2 * ci),
-                         Output(out, rs_lo=ci, d_zhi=co * ci), L * co * ci, zhi_n=L, a_plane=co, b_plane=ci, accumulate=(B > 1),
-                         kmax=(1, 1 + l0 - m0))
-        return out
-    d5 = dt.view(B, L, M, 2, co)
-    dts = torch.cat([d5[..., 1:2, :], -d5[..., 0:1, :]], dim=-2).contiguous()
+    dt, t2 = dt.contiguous(), t2.contiguous()
     out = (torch.empty if B == 1 else torch.zeros)(2, L, co, ci, dtype=torch.float32, device=dt.device)
-    tri = Tri(kmax_a=2, kmax_b=2 * (1 + l0 - m0))
-    for part, a in enumerate((dt, dts)):
-        gemm(co, ci, 2 * M,
-             Operand(a, ld=co, mn_major=True, zs_hi=M * nq, zs_lo=L * M * nq),
-             Operand(t2, ld=ci, mn_major=True, zs_hi=M * 2 * ci, zs_lo=L * M * 2 * ci),
-             Output(out, rs_lo=ci, offset=part * L * co * ci, d_zhi=co * ci),
-             zhi_n=L, zlo_n=B, accumulate=(B > 1), tri=tri)
+    for b in range(B):
+        gemm_complex(3, co, ci, M,
+                     Operand(dt, ld=nq, mn_major=True, zs_hi=M * nq, offset=b * L * M * nq),
+                     Operand(t2, ld=2 * ci, mn_major=True, zs_hi=M * 2 * ci, offset=b * L * M * 2 * ci),
+                     Output(out, rs_lo=ci, d_zhi=co * ci), L * co * ci, zhi_n=L, a_plane=co, b_plane=ci, accumulate=(B > 1),
+                     kmax=(1, 1 + l0 - m0))
     return out
 
 
@@ -256,11 +243,13 @@ def expand_weight(w: torch.Tensor, dtype=torch.bfloat16, keep: bool = False, sha
 
 
 def weight_planes(w: torch.Tensor, dtype=torch.bfloat16, keep: bool = False, share: bool = False) -> torch.Tensor:
-    """complex [Ci, Co, L] on CUDA -> real and imaginary planes [L, 2, Co, Ci] in bf16; elsewhere the block form of `expand_weight`."""
-    return _kept(w, dtype, _planes if w.is_cuda and dtype == torch.bfloat16 else _expand_weight, keep, share)
+    """complex [Ci, Co, L] -> its real and imaginary planes [L, 2, Co, Ci]."""
+    return _kept(w, dtype, _planes, keep, share)
 
 
 def _planes(w: torch.Tensor, dtype) -> torch.Tensor:
+    if not w.is_cuda or dtype != torch.bfloat16:
+        return torch.stack([w.real, w.imag]).permute(3, 0, 2, 1).to(dtype).contiguous()
     ci, co, L = w.shape
     wp = torch.empty(L, 2, co, ci, dtype=dtype, device=w.device)
     _ext.require().spectral_planes(w.detach().contiguous(), wp)

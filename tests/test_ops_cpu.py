@@ -181,3 +181,30 @@ def test_sync_params_announces_changed_weights(tmp_path):
         assert spectral._WEIGHT_EPOCH > before
     finally:
         dist.destroy_process_group()
+
+
+@pytest.mark.parametrize("b,l,m,co,ci", [(1, 5, 6, 8, 16), (2, 9, 7, 6, 4)])
+def test_planar_spectral_products_emulated(b, l, m, co, ci):
+    """The product with planar weights, its adjoint with a residual and the weight gradient, emulated with the kernel's addressing,
+    against complex einsum and against the real block form."""
+    from makani_b200.ops.spectral import contract, contract_wgrad2, weight_planes
+    torch.manual_seed(l)
+    keep = (torch.arange(m)[None] <= torch.arange(l)[:, None]).view(1, l, m, 1)
+    t2, dt = torch.randn(b, l, m, 2 * ci) * keep, torch.randn(b, l, m, 2 * co) * keep
+    w = torch.randn(ci, co, l, dtype=torch.complex64)
+    wp = weight_planes(w, torch.float32)
+    assert wp.shape == (l, 2, co, ci)
+    cplx = lambda t: torch.complex(*t.chunk(2, dim=-1))  # noqa: E731
+    parts = lambda z: torch.cat([z.real, z.imag], dim=-1)  # noqa: E731
+    y = contract(t2, wp, False)
+    torch.testing.assert_close(y, parts(torch.einsum("blmc,col->bmlo", cplx(t2), w)), atol=1e-5, rtol=1e-5)
+    torch.testing.assert_close(y, contract(t2, expand_weight(w, torch.float32), False), atol=1e-5, rtol=1e-5)
+    res = torch.randn(b, m, l, 2 * ci)
+    dx = contract(dt, wp, True, resid=res)
+    torch.testing.assert_close(dx, parts(torch.einsum("blmo,col->bmlc", cplx(dt), w.conj())) + res, atol=1e-5, rtol=1e-5)
+    # a block of a larger problem: its first order and degree are m0 and l0
+    for l0, m0 in ((0, 0), (2, 3)):
+        keep = (torch.arange(m)[None] + m0 <= torch.arange(l)[:, None] + l0).view(1, l, m, 1)
+        got = contract_wgrad2(dt * keep, t2 * keep, l0, m0)
+        ref = torch.einsum("blmo,blmc->loc", cplx(dt * keep), cplx(t2 * keep).conj())
+        torch.testing.assert_close(got, torch.stack([ref.real, ref.imag]), atol=1e-5, rtol=1e-5)
