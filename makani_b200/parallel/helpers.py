@@ -85,5 +85,5 @@ def sync_params(model: torch.nn.Module, mode: str = "broadcast") -> None:
                     t.div_(comm.get_size(g))
                 else:
                     raise ValueError(f"unknown sync mode {mode}")
-    from ..ops.spectral import note_weights_changed
+    from makani_b200.ops.spectral import note_weights_changed
     note_weights_changed()      # written through `.data`: no parameter's version shows it
