@@ -1774,13 +1774,16 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
     if (bn == 256) return launch_t<256, 4, 0, 1>(ma, mbs, me, md, mp, mdx, kp, stream);
     return launch_t<128, 4, 0, 1>(ma, mbs, me, md, mp, mdx, kp, stream);
   }
+  // (epilogues with an operand in shared memory: at most 192 columns, see above)
 #define MK_DISPATCH(EPI_)                                                                              \
+  if constexpr (EPI_ != 3 && EPI_ != 4) {                                                              \
+    if (bn == 256 && cg == 2) return launch_t<256, 2, EPI_, 2>(ma, mbs, me, md, mp, mdx, kp, stream);  \
+    if (bn == 256) return launch_t<256, 2, EPI_, 1>(ma, mbs, me, md, mp, mdx, kp, stream);             \
+  }                                                                                                    \
   if (cg == 2) {                                                                                       \
-    if (bn == 256) return launch_t<256, 2, EPI_, 2>(ma, mbs, me, md, mp, mdx, kp, stream);             \
     if (bn == 192) return launch_t<192, 2, EPI_, 2>(ma, mbs, me, md, mp, mdx, kp, stream);             \
     return launch_t<128, 2, EPI_, 2>(ma, mbs, me, md, mp, mdx, kp, stream);                            \
   }                                                                                                    \
-  if (bn == 256) return launch_t<256, 2, EPI_, 1>(ma, mbs, me, md, mp, mdx, kp, stream);               \
   if (bn == 192) return launch_t<192, 2, EPI_, 1>(ma, mbs, me, md, mp, mdx, kp, stream);               \
   return launch_t<128, 2, EPI_, 1>(ma, mbs, me, md, mp, mdx, kp, stream);
   switch (epi) {
