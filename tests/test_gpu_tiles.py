@@ -18,9 +18,9 @@ BF16 = 2.0 ** -8      # spacing of bf16 relative to the value: a rounded result 
 @pytest.mark.parametrize("epi", ["plain", "gelu", "relu", "gelu_pre", "gelu_deriv", "resid", "mul", "dgelu"])
 def test_gemm_192_column_tiles(pair, w_mn, n, epi):
     """192-column tiles on single CTAs and pairs, both majors of the weight, every specialised epilogue, N from one vector
-    over one tile and its edges to several tiles, more row tiles than one wave of the smallest grid, ragged rows."""
+    over one tile and its edges to several tiles, ragged rows (many tiles per CTA: test_gemm_many_tiles_per_cta)."""
     dev = _dev()
-    k = 520 if pair else 72           # pairs run from K = 512 on
+    k = 520 if pair else 72           # pairs run from K = 512 on, and with fewer where the tiles are many
     m = 128 * 9 + 40
     torch.manual_seed(n + k)
     x = torch.randn(2, m, k, device=dev).to(torch.bfloat16)
@@ -556,3 +556,58 @@ def test_afno_bias_gradients_repeat_themselves():
 def test_column_sums_of_no_rows():
     from makani_b200.ops.norm import row_sums
     assert torch.equal(row_sums(torch.empty(0, 16, device=_dev(), dtype=torch.bfloat16), 16).cpu(), torch.zeros(16))
+
+
+@pytest.mark.parametrize("k", [40, 136, 264, 384])
+@pytest.mark.parametrize("n", [384, 72, 520])
+@pytest.mark.parametrize("epi", ["plain", "gelu", "resid", "mul", "dgelu", "gelu_pre", "gelu_deriv", "fp32"])
+def test_gemm_many_tiles_per_cta(k, n, epi):
+    """At least four tiles per CTA and per pair: every operand buffer, staging box and accumulator is used again and again.  Short
+    k loops run on single CTAs, 264 and 384 on pairs; one 64-column box per warp, ragged columns, ragged rows."""
+    dev = _dev()
+    z, m = 4, 128 * 150 + 40
+    g = torch.Generator(dev).manual_seed(k + n)
+    rnd = lambda *s: torch.randn(*s, device=dev, generator=g)  # noqa: E731
+    x, w = rnd(z, m, k).to(torch.bfloat16), (rnd(n, k) / k ** 0.5).to(torch.bfloat16)
+    aux = rnd(z, m, n).to(torch.bfloat16) if epi in ("resid", "mul", "dgelu") else None
+    bias = rnd(n) if epi in ("plain", "gelu", "resid", "gelu_pre", "gelu_deriv") else None
+    act = {"resid": ACT_NONE, "plain": ACT_NONE, "fp32": ACT_NONE, "mul": ACT_MULAUX, "dgelu": ACT_DGELU}.get(epi, ACT_GELU)
+    acc = x.double() @ w.double().t() + (bias.double() if bias is not None else 0.0)
+    leaf = (aux if epi == "dgelu" else acc).double().requires_grad_()
+    slope, = torch.autograd.grad(torch.nn.functional.gelu(leaf).sum(), leaf)
+    second = acc if epi == "gelu_pre" else slope
+    ref = {"plain": lambda: acc, "fp32": lambda: acc, "resid": lambda: acc + aux.double(), "mul": lambda: acc * aux.double(),
+           "dgelu": lambda: acc * slope}.get(epi, lambda: torch.nn.functional.gelu(acc))()
+    for _ in range(3):
+        d = torch.full((z, m, n), float("nan"), device=dev, dtype=torch.float32 if epi == "fp32" else torch.bfloat16)
+        pre = torch.full_like(d, float("nan")) if epi in ("gelu_pre", "gelu_deriv") else None
+        gemm(m, n, k, Operand(x, ld=k, zs_lo=m * k), Operand(w, ld=k), Output(d, rs_lo=n, d_zlo=m * n), zlo_n=z, bias=bias,
+             bias_mode=BIAS_COL, act=act, resid=aux, preact=pre, preact_deriv=epi == "gelu_deriv")
+        # on the GPU and in full: one element of one tile counts.  bf16 rounding is half of BF16 of a value; the fp32 sum behind it and
+        # the kernel's GELU (a polynomial and tanh.approx, 2^-10) add less than as much
+        for got, want in ((d, ref), (pre, second)):
+            if got is not None:
+                scale = want.square().mean().sqrt()
+                tol = 2.0 ** -18 if epi == "fp32" else BF16
+                assert ((got.double() - want).abs() <= tol * (want.abs() + scale)).all()
+    _ext.check_device_errors(dev)
+
+
+@pytest.mark.parametrize("b,l,m,co,ci", [(1, 240, 241, 256, 256), (2, 210, 211, 200, 136), (1, 202, 203, 256, 184), (1, 208, 209, 248, 384)])
+def test_planar_weight_gradient_on_pairs(b, l, m, co, ci):
+    """More than one row tile with little padding and 200 orders or more: the planar weight gradient runs on CTA pairs, with the
+    negated segment, degree-limited k ranges and, for 136 to 192 and 384 columns, a pair's half of one and a half boxes."""
+    from makani_b200.ops.spectral import contract_wgrad2
+    dev = _dev()
+    g = torch.Generator(dev).manual_seed(l)
+    keep = (torch.arange(m, device=dev)[None] <= torch.arange(l, device=dev)[:, None]).view(1, l, m, 1)
+    t2 = (torch.randn(b, l, m, 2 * ci, device=dev, generator=g) * keep).to(torch.bfloat16)
+    dt = (torch.randn(b, l, m, 2 * co, device=dev, generator=g) * keep).to(torch.bfloat16)
+    cplx = lambda t: torch.complex(t[..., : t.shape[-1] // 2].double(), t[..., t.shape[-1] // 2:].double())  # noqa: E731
+    ref = torch.einsum("blmo,blmc->loc", cplx(dt), cplx(t2).conj())
+    ref = torch.stack([ref.real, ref.imag])
+    for _ in range(2):
+        got = contract_wgrad2(dt, t2)
+        assert _rel(got, ref) < 2.0 ** -24 * (b * m) ** 0.5 * 4
+        assert (got.double() - ref).abs().max() < 2.0 ** -16 * ref.abs().max()
+    _ext.check_device_errors(dev)
