@@ -1500,16 +1500,20 @@ FastDiv make_div(int d) {
   return f;
 }
 
-// Tile width: the fewest padded columns, a tile costing some 32 columns of its own.  Measured over 721 x 1440 tokens: 384
-// outputs take 567 us (K = 768) and 368 us (K = 384) in 192-column tiles, 664 and 469 us in 256-column tiles, a third of
-// which is padding, 640 and 392 us in 128-column tiles, which fetch the activations once more.
+// Tile width: the fewest padded columns, a tile costing some 32 columns of its own, 64 in the plain store, which waits for the
+// activations (every tile of a row fetches them once more) rather than for its epilogue.  Measured, us in 256 / 192 / 128 columns:
+//   plain, 115200 rows, K = 384: 384 outputs 44 / 43 / -; 520: 59 / 58 / -; 640: 63 / 68 / 69; 776: 82 / 85 / 93;
+//   K = 96: 384: 32 / 28 / -; 640: 42 / 50 / 49;  16200 rows, K = 768: 384: 16 / 14 / -; 640: 20 / 22 / 23
+//   GELU with two outputs, 115200 rows, K = 96: 384: 59 / 48 / -; 640: 78 / - / 84; 776: 145 / 108 / -
+//   fp32 gradients of 320 rows over 115200 tokens: 384: 47 / 38 / 39; 640: 63 / 60 / 59; 776: 89 / 86 / 88
+//   times an operand (no 256): K = 96, 384: - / 39 / 41; 576: - / 54 / 61;  K = 384, 384: - / 54 / 50; 576: - / 70 / 74
 int pick_bn(int N, int epi, int e_tma) {
   if (epi == 0 && e_tma) return 128;
   int best = 128;
   long long cost = -1;
-  const int widths[3] = {256, 192, 128};
+  const int widths[3] = {256, 192, 128}, own = epi == 1 ? 64 : 32;
   for (int i = (epi == 3 || epi == 4 ? 1 : 0); i < 3; ++i) {
-    const long long c = static_cast<long long>((N + widths[i] - 1) / widths[i]) * (widths[i] + 32);
+    const long long c = static_cast<long long>((N + widths[i] - 1) / widths[i]) * (widths[i] + own);
     if (cost < 0 || c < cost) {
       cost = c;
       best = widths[i];
