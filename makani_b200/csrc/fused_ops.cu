@@ -320,8 +320,8 @@ __device__ __forceinline__ void cl_rows(const uint4* xv, const uint4* gv, int V,
   }
 }
 
-// Two CTAs per SM for the forward kernels; the backward ones hold their constants and eight loads in up to 128 registers of
-// one CTA.
+// Two CTAs per SM for the forward kernels; the backward ones hold their constants and eight loads in the 128 registers that one
+// CTA leaves (four registers of the sums kernel do not fit and are spilled).
 template <int MODE>
 __global__ void __launch_bounds__(CL_THREADS, MODE == 0 ? 2 : 1) inorm_cl_sums_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
                                                                    const float* __restrict__ w, const float* __restrict__ b,

@@ -57,10 +57,10 @@ def available() -> bool:
     return _MOD is not None
 
 
-# number of kernels of this extension launched by the current process (each binding call launches exactly one)
+# number of kernel-launching calls into this extension by the current process (the column sums launch a second kernel)
 LAUNCHES = 0
 _NON_KERNEL = {"read_error_flag", "clear_error_flag", "lp_scratch_floats", "adam_entry_bytes", "peer_alloc", "peer_open",
-               "peer_close", "peer_free", "tensor_from_ptr", "set_gelu_tanh"}
+               "peer_close", "peer_free", "tensor_from_ptr", "set_gelu_tanh", "stream_state"}
 
 
 class _Counting:

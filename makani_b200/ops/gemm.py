@@ -225,7 +225,8 @@ def gemm(M: int, N: int, K: int, A: Operand, B: Operand, D: Output, *, zlo_n: in
     `makani_b200.parallel.peer.sync_descriptor` (CUDA only).  `dests` lists device addresses of additional copies of
     the output buffer (peers' memory) that receive the same bf16 stores as `D.tensor`.
 
-    `splits` cuts the k axis of an accumulating launch into that many partial sums (0: chosen for whole waves of CTAs).
+    `splits` cuts the k axis of an accumulating launch into that many partial sums (0: chosen for whole waves of CTAs and short
+    sums; one where a bias or an activation is applied).
 
     `preact` receives the value before the activation; with `preact_deriv` (act = ACT_GELU only) it receives GELU' of
     that value instead, which the backward pass multiplies in with `act=ACT_MULAUX, resid=<that tensor>`."""

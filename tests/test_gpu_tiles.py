@@ -430,6 +430,13 @@ def test_kept_weights_serve_one_stream(monkeypatch):
     assert len(made) == 2 and torch.equal(a, b)
 
 
+def test_launch_count_counts_launches():
+    dev = _dev()
+    n = _ext.launch_count()
+    _ext.require().stream_state(dev.index)
+    assert _ext.launch_count() == n
+
+
 def test_recorded_passes_share_one_expansion(monkeypatch):
     """The steps of a roll-out share one expansion, which goes with the last of their graphs; weights changed in place, announced or
     not once the graphs are gone, or a new parameter in the same memory, are expanded anew."""
