@@ -329,6 +329,18 @@ __device__ __forceinline__ uint32_t desc_lo(uint32_t saddr, uint32_t lbo_bytes) 
 }
 __device__ __forceinline__ uint32_t desc_hi(uint32_t sbo_bytes) { return (sbo_bytes >> 4) | (1u << 14) | (2u << 29); }
 
+__device__ __forceinline__ uint4 pack_bf16x8(const float (&x)[8]) {
+  f32x2 f[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) f[j] = f2_pack(x[2 * j], x[2 * j + 1]);
+  return f2_bf16x8(f);
+}
+
+template <int V>
+struct IntC {
+  static constexpr int value = V;
+};
+
 struct TileCoord {
   int zhi, zlo, split, mt, nt;
   int half;             // complex products: real (0) or imaginary (1) part; nt counts the column tiles inside the half
@@ -796,8 +808,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
         // the box this warp's output is written to: staging (1, 2) or the operand's own box (3, 4)
         const uint32_t box_off = IN_PLACE ? e_off + ebuf * E_BYTES + bx * (BM * 128) + q * (32 * 128)
                                           : stg_off + (warp - 2) * stg_warp_bytes(EPI) + (EPI == 2 ? 32 * 128 : 0);
-        uint8_t* const box_d = smem + box_off + lane * 128;
-        uint8_t* const box_p = box_d - 32 * 128;      // second output (2)
         if (nb < p.N) {     // uniform across the warp
           const uint32_t taddr = tmem_base + buf * BN + bx * 64 + (static_cast<uint32_t>(q * 32) << 16);
           // the previous store of this warp must have read its box (the operand box was released after that already)
@@ -810,43 +820,39 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
           // to tens of KB of straight-line code per epilogue flavour, the epilogue warps (each at another place
           // in it) missed the instruction caches on most fetches, and "no instruction" was their top stall reason.
           // Arithmetic is on pairs of columns (fma / mul on f32x2): same roundings, half the instructions.
+          // What is uniform over the launch (column bias, activation) selects one of several copies of the loop, not a branch
+          // inside it: every branch that rejoins with the accumulators in registers copied them (12.6 instructions per
+          // output element of a plain store, half of them moves).  384 -> 768 with GELU, 721 x 1440 tokens: 831 -> 626 us without the
+          // second output, 961 -> 928 us with it; 384 -> 768 over 240 x 480 tokens without: 103 -> 84 us.
+          uint8_t* const sw_d = smem + box_off + lane * 128;
+          const uint32_t l7 = static_cast<uint32_t>(lane & 7) << 4;
+          auto columns = [&](auto bias_c, auto act_c) {
+            constexpr bool COL_BIAS = decltype(bias_c)::value != 0;
+            constexpr int ACT = decltype(act_c)::value;
 #pragma unroll 1
-          for (int it = 0; it < 4; ++it) {
-            uint32_t v[16];
-            if (!c.skip) {
+            for (int it = 0; it < 4; ++it) {
+              uint32_t v[16];
               tmem_ld16(taddr + it * 16, v);
-            } else {
 #pragma unroll
-              for (int j = 0; j < 16; ++j) v[j] = 0u;
-            }
-#pragma unroll
-            for (int gg = 0; gg < 2; ++gg) {
-              const int g = it * 2 + gg;
-              const int n = nb + g * 8;
-              f32x2 f[4];
-#pragma unroll
-              for (int j = 0; j < 4; ++j) f[j] = rbias2;
-              if (p.bias_mode == 2) {      // the column bias rides on the scaling fma below
-                if (n + 8 <= p.N) {
+              for (int gg = 0; gg < 2; ++gg) {
+                const uint32_t sw = static_cast<uint32_t>((it * 2 + gg) << 4) ^ l7;
+                f32x2 f[4];
+                if constexpr (COL_BIAS) {      // rides on the scaling fma (columns past N are clipped by the store)
+                  const int n = min(nb + it * 16 + gg * 8, p.N - 8);
                   const ulonglong2 b0 = __ldg(reinterpret_cast<const ulonglong2*>(bias_z + n));
                   const ulonglong2 b1 = __ldg(reinterpret_cast<const ulonglong2*>(bias_z + n) + 1);
                   f[0] = b0.x; f[1] = b0.y; f[2] = b1.x; f[3] = b1.y;
                 } else {
 #pragma unroll
-                  for (int j = 0; j < 4; ++j)
-                    f[j] = f2_pack(n + 2 * j < p.N ? __ldg(bias_z + n + 2 * j) : 0.f,
-                                   n + 2 * j + 1 < p.N ? __ldg(bias_z + n + 2 * j + 1) : 0.f);
+                  for (int j = 0; j < 4; ++j) f[j] = rbias2;
                 }
-              }
 #pragma unroll
-              for (int j = 0; j < 4; ++j)
-                f[j] = f2_fma(f2_pack(__uint_as_float(v[gg * 8 + 2 * j]), __uint_as_float(v[gg * 8 + 2 * j + 1])), alpha2, f[j]);
-              const uint32_t sw = static_cast<uint32_t>((g ^ (lane & 7)) << 4);
-              if constexpr (EPI == 1) {
-                if (p.act == 1) {
+                for (int j = 0; j < 4; ++j)
+                  f[j] = f2_fma(f2_pack(__uint_as_float(v[gg * 8 + 2 * j]), __uint_as_float(v[gg * 8 + 2 * j + 1])), alpha2, f[j]);
+                if constexpr (EPI == 1 && ACT == 1) {
 #pragma unroll
                   for (int j = 0; j < 4; ++j) f[j] = gelu_fwd2(f[j], gelu2);
-                } else if (p.act != 0) {      // ReLU / soft shrinkage (uniform over the launch)
+                } else if constexpr (EPI == 1 && ACT != 0) {      // ReLU / soft shrinkage
 #pragma unroll
                   for (int j = 0; j < 4; ++j) {
                     float x, y;
@@ -854,34 +860,86 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
                     f[j] = f2_pack(act_fwd(x, p.act, p.act_param, p.gelu), act_fwd(y, p.act, p.act_param, p.gelu));
                   }
                 }
-              }
-              if constexpr (EPI == 2) {
-                f32x2 s2[4];
-                if (p.save_deriv) {      // uniform over the launch: second output = GELU'(pre-activation)
-#pragma unroll
-                  for (int j = 0; j < 4; ++j) gelu_fwd_bwd2(f[j], gelu2, f[j], s2[j]);
-                } else {
+                if constexpr (EPI == 2) {      // second output: GELU' of the pre-activation, or the pre-activation itself
+                  f32x2 s2[4];
 #pragma unroll
                   for (int j = 0; j < 4; ++j) {
-                    s2[j] = f[j];
-                    f[j] = gelu_fwd2(f[j], gelu2);
+                    if constexpr (ACT == 1) {
+                      gelu_fwd_bwd2(f[j], gelu2, f[j], s2[j]);
+                    } else {
+                      s2[j] = f[j];
+                      f[j] = gelu_fwd2(f[j], gelu2);
+                    }
+                  }
+                  *reinterpret_cast<uint4*>(sw_d - 32 * 128 + sw) = f2_bf16x8(s2);
+                }
+                if constexpr (IN_PLACE) {
+                  f32x2 e[4];
+                  f2_unpack8(*reinterpret_cast<const uint4*>(sw_d + sw), e);
+#pragma unroll
+                  for (int j = 0; j < 4; ++j) {
+                    if constexpr (EPI == 3) f[j] = f2_add(f[j], e[j]);
+                    else if constexpr (ACT == 8) f[j] = f2_mul(f[j], e[j]);      // the operand is the saved derivative
+                    else {
+                      float e0, e1;
+                      f2_unpack(e[j], e0, e1);
+                      f[j] = f2_mul(f[j], f2_pack(act_bwd(e0, p.act, p.gelu), act_bwd(e1, p.act, p.gelu)));
+                    }
                   }
                 }
-                *reinterpret_cast<uint4*>(box_p + sw) = f2_bf16x8(s2);
+                *reinterpret_cast<uint4*>(sw_d + sw) = f2_bf16x8(f);
+              }
+            }
+          };
+          auto with_act = [&](auto bias_c) {
+            if constexpr (EPI == 1) {
+              if (p.act == 0) columns(bias_c, IntC<0>{});
+              else if (p.act == 1) columns(bias_c, IntC<1>{});
+              else columns(bias_c, IntC<3>{});
+            } else if constexpr (EPI == 2) {
+              if (p.save_deriv) columns(bias_c, IntC<1>{});
+              else columns(bias_c, IntC<0>{});
+            } else if constexpr (EPI == 3) {
+              columns(bias_c, IntC<0>{});
+            } else {
+              if (p.act == 8) columns(bias_c, IntC<8>{});
+              else columns(bias_c, IntC<0>{});
+            }
+          };
+          if (c.skip) {
+            // no product reaches this tile (triangular structure): the epilogue of zeros
+#pragma unroll 1
+            for (int g = 0; g < 8; ++g) {
+              const uint32_t sw = static_cast<uint32_t>(g << 4) ^ l7;
+              float x[8];
+#pragma unroll
+              for (int j = 0; j < 8; ++j)
+                x[j] = p.bias_mode == 2 ? __ldg(bias_z + min(nb + g * 8, p.N - 8) + j) : rbias;
+              if constexpr (EPI == 2) {
+                float d[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) d[j] = p.save_deriv ? gelu_bwd(x[j], p.gelu) : x[j];
+                *reinterpret_cast<uint4*>(sw_d - 32 * 128 + sw) = pack_bf16x8(d);
+              }
+              if constexpr (EPI == 1 || EPI == 2) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) x[j] = act_fwd(x[j], p.act, p.act_param, p.gelu);
               }
               if constexpr (IN_PLACE) {
-                const uint4 ev = *reinterpret_cast<const uint4*>(box_d + sw);
+                const uint4 ev = *reinterpret_cast<const uint4*>(sw_d + sw);
                 const uint32_t ew[4] = {ev.x, ev.y, ev.z, ev.w};
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                  const float e0 = __uint_as_float(ew[j] << 16), e1 = __uint_as_float(ew[j] & 0xffff0000u);
-                  if constexpr (EPI == 3) f[j] = f2_add(f[j], f2_pack(e0, e1));
-                  else if (p.act == 8) f[j] = f2_mul(f[j], f2_pack(e0, e1));      // uniform: the operand is the saved derivative
-                  else f[j] = f2_mul(f[j], f2_pack(act_bwd(e0, p.act, p.gelu), act_bwd(e1, p.act, p.gelu)));
+                for (int j = 0; j < 8; ++j) {
+                  const float e = __uint_as_float(j & 1 ? ew[j / 2] & 0xffff0000u : ew[j / 2] << 16);
+                  x[j] = EPI == 3 ? x[j] + e : x[j] * act_bwd(e, p.act, p.gelu);
                 }
               }
-              *reinterpret_cast<uint4*>(box_d + sw) = f2_bf16x8(f);
+              *reinterpret_cast<uint4*>(sw_d + sw) = pack_bf16x8(x);
             }
+          } else if (p.bias_mode == 2) {
+            with_act(IntC<1>{});
+          } else {
+            with_act(IntC<0>{});
           }
         }
         if (!c.skip) {     // the accumulator has been read: the next tile but one may overwrite it
@@ -1662,7 +1720,7 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
   memset(&mp, 0, sizeof(mp));
   memset(&mdx, 0, sizeof(mdx));
   if (eb == 2 && !e.out_f32 && kp.vec_ok && !e.accumulate && plain && e.d_zlo >= 0 && e.d_zhi >= 0 &&
-      (kp.bias_mode != 2 || ((reinterpret_cast<uintptr_t>(e.bias) & 15) == 0 && (kp.bias_zs % 4) == 0))) {
+      (kp.bias_mode != 2 || (p.N % 8 == 0 && (reinterpret_cast<uintptr_t>(e.bias) & 15) == 0 && (kp.bias_zs % 4) == 0))) {
     if (!e.resid && !e.preact && (e.act == 0 || e.act == 1 || e.act == 3 || e.act == 5)) epi = 1;
     else if (!e.resid && e.preact && e.act == 1) epi = 2;
     else if (e.resid && kp.e_tma && !e.preact && e.act == 0) epi = 3;
