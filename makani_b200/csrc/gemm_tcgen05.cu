@@ -2,11 +2,11 @@
 // accumulators in tensor memory -> tcgen05.ld epilogue with fused bias / GELU / residual / scatter.
 //
 // Roles per CTA (one CTA per SM; EW epilogue warps: one per 64-column box and lane quarter of the tile, see epi_warps):
-//   warp 0         : TMA producer (one elected lane)
+//   warps 0, EW+2  : TMA producers (one elected lane each), which fill every second stage of the ring
 //   warp 1         : TMEM allocator + MMA issuer (one elected lane)
 //   warps 2..EW+1  : epilogue; warp w reads TMEM lanes [32*(w%4), 32*(w%4)+32) and the 64-column box (w-2)/4 (generic
 //                    epilogue: alternating 32-column chunks)
-//   warp EW+2      : only in launches whose epilogue operand (residual, saved pre-activation) is prefetched by TMA: its
+//   warp EW+3      : only in launches whose epilogue operand (residual, saved pre-activation) is prefetched by TMA: its
 //                    producer, so that waiting for a free operand buffer never delays A and B
 // Two accumulator buffers in TMEM let the epilogue of tile i overlap the main loop of tile i+1.
 // Every mbarrier wait is bounded; on expiry the kernel records a code in *err and drains.
@@ -58,7 +58,7 @@ __host__ __device__ constexpr int epi_warps(int bn, int epi) { return epi == 0 ?
 // Register bound, given as a thread count: the warps of one scheduler's register bank (5, 4 or 3 of them) leave room for one
 // 64-register warp of the gradient all-reduce, which overlaps with these GEMMs in data-parallel training.
 __host__ __device__ constexpr int bound_threads(int bn, int epi) {
-  return epi == 0 || bn == 128 ? 352 : (bn == 192 ? 576 : 736);
+  return epi == 0 || bn == 128 ? 384 : (bn == 192 ? 576 : 736);
 }
 constexpr int MAX_STAGES = 6;
 constexpr int MAX_SEG = 8;
@@ -433,7 +433,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
   constexpr int BNL = BN / CG;            // rows of the B tile this CTA contributes (a pair splits the tile)
   constexpr int B_STAGE_BYTES = b_stage_rows(BN, CG) * 128;
   constexpr int EW = epi_warps(BN, EPI);
-  constexpr int E_WARP = 2 + EW;
+  constexpr int PRODUCER_2 = 2 + EW;      // second TMA producer
+  constexpr int E_WARP = 3 + EW;
   constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
   constexpr int MN_BOX = 128 / EB;        // extent of an MN-major box along the contiguous dimension
   constexpr uint32_t TMEM_COLS = BN == 128 ? 256 : 512;   // two accumulators, rounded up to a power of two
@@ -526,11 +527,16 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
   const uint32_t tmem_base = *tmem_slot;
   const bool peers_ready = tmem_slot[1] != 0u;
 
-  if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer
+  if (warp == 0 || warp == PRODUCER_2) {
+    // ------------------------------------------------------------------ TMA producers
+    // Two warps take the k slabs of this CTA in turn.  One slab costs a producer its wait, its byte count and two to six TMA
+    // instructions one after the other, some 450 - 700 cycles; a slab's MMAs take 256 - 512, and with a single producer it was
+    // this thread that most launches waited for, with the loads in flight far from filling the ring.  Back to back, under the power
+    // cap: 768 -> 384 over 721 x 1440 tokens 699 -> 649 us, its gradient 707 -> 650, 384 -> 768 with GELU and GELU' 928 -> 882.
     if (elect_one()) {
-      int s = 0;
-      uint32_t ph = 0;
+      const uint32_t me = warp == 0 ? 0u : 1u;
+      int s = static_cast<int>(me);
+      uint32_t ph = 0, slab = 0;      // slab: slabs of the CTA so far; this producer fills those of its parity
       bool ok = peers_ready;
       if (p.sync.nwait > 0) asm volatile("fence.proxy.async;" ::: "memory");   // flags acquired in the prologue order the TMA loads below
       // pair: every load of both CTAs is counted on the leader's "full" barrier.  The leader announces the bytes of both; the
@@ -539,7 +545,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
       const uint32_t leader_full0 = (CG == 2) ? mapa_u32(full_bar(0), 0) : 0u;
       const uint32_t load_bytes = A_STAGE_BYTES + (p.b_mn ? B_STAGE_BYTES : BNL * 128);
       const bool a_mn = p.a_mn != 0, b_mn = p.b_mn != 0;
-      // the next stage: waits until it is free and loads the k slabs of A at ka, rows m0, and of B at kb, rows nb
+      // this producer's next stage: waits until it is free and loads the k slabs of A at ka, rows m0, and of B at kb, rows nb
       auto stage = [&](const CUtensorMap* mb, int ka, int m0, int azl, int azh, int kb, int nb, int bzl, int bzh) {
         if (!mbar_wait(empty_bar(s), ph ^ 1u)) {
           atomicExch(p.err, 1);
@@ -579,8 +585,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
             for (int j = 0; j < BN / MN_BOX; ++j) tma_load_4d(sb + j * (BK * 128), mb, bar, nb + j * MN_BOX, kb, bzl, bzh);
           }
         }
-        if (++s == STAGES) {
-          s = 0;
+        s += 2;
+        if (s >= STAGES) {
+          s -= STAGES;
           ph ^= 1u;
         }
         return true;
@@ -592,25 +599,25 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
         const int m0 = c.mt * BM, nb = c.nt * BN + (CG == 2 ? crank * BNL : 0);
         int azl = p.a_zlo ? c.zlo : 0, bzl = p.b_zlo ? c.zlo : 0;
         const int azh = p.a_zhi ? c.zhi : 0, bzh = p.b_zhi ? c.zhi : 0;
-        if (simple) {
-          for (int k = c.k_begin; k < c.k_end && ok; k += BK) ok = stage(&map_b, k, m0, azl, azh, k, nb, bzl, bzh);
-          continue;
-        }
-        const int nsg = p.cplx ? 2 : p.nseg;
+        const int nsg = simple ? 1 : (p.cplx ? 2 : p.nseg);
         for (int sg = 0; sg < nsg && ok; ++sg) {
           int lb = c.k_begin, le = c.k_end, apos = 0;
           const CUtensorMap* mb = &map_b;
-          if (p.nseg > 1) {
-            seg_range<BK>(p, c, sg, lb, le);
-            apos = p.seg_apos[sg];
-            mb = &maps_b.m[sg];
-          } else if (p.cplx) {
-            // segment and half select the planes, which take the place of the lower batch index
-            bzl = p.cplx == 3 ? sg : (sg ^ c.half);
-            if (p.cplx == 3) azl = sg ^ c.half;
-            else apos = sg * p.K;
+          if (!simple) {
+            if (p.nseg > 1) {
+              seg_range<BK>(p, c, sg, lb, le);
+              apos = p.seg_apos[sg];
+              mb = &maps_b.m[sg];
+            } else {
+              // segment and half select the planes, which take the place of the lower batch index
+              bzl = p.cplx == 3 ? sg : (sg ^ c.half);
+              if (p.cplx == 3) azl = sg ^ c.half;
+              else apos = sg * p.K;
+            }
           }
-          for (int k = lb; k < le && ok; k += BK) ok = stage(mb, apos + k, m0, azl, azh, k, nb, bzl, bzh);
+          for (int k = lb + static_cast<int>((slab ^ me) & 1u) * BK; k < le && ok; k += 2 * BK)
+            ok = stage(mb, apos + k, m0, azl, azh, k, nb, bzl, bzh);
+          if (le > lb) slab += static_cast<uint32_t>(le - lb + BK - 1) / BK;
         }
       }
     }
@@ -1133,7 +1140,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
 
   // ------------------------------------------------------------------ teardown
   if constexpr (EPI != 0) {
-    if (warp >= 2 && warp < E_WARP) {      // (bulk groups belong to the lane that committed them)
+    if (warp >= 2 && warp < PRODUCER_2) {      // (bulk groups belong to the lane that committed them)
       tma_store_wait_all();
       asm volatile("fence.proxy.async;" ::: "memory");   // order the bulk stores before the generic-proxy signalling below
     }
@@ -1250,7 +1257,7 @@ int max_pairs() {
     qa[0].val.clusterDim.y = 1;
     qa[0].val.clusterDim.z = 1;
     qc.gridDim = dim3(2 * (sm_count() / 2), 1, 1);
-    qc.blockDim = dim3(32 * (3 + epi_warps(256, 0)), 1, 1);
+    qc.blockDim = dim3(32 * (4 + epi_warps(256, 0)), 1, 1);
     qc.dynamicSmemBytes = SMEM_LIMIT;
     qc.attrs = qa;
     qc.numAttrs = 1;
@@ -1280,7 +1287,7 @@ cudaError_t launch_t(const CUtensorMap& ma, const BMaps& mb, const CUtensorMap& 
   }
   kp.stages = stages;
   const int smem = stages * STAGE + e_bytes + FIXED;
-  const int threads = 32 * (2 + epi_warps(BN, EPI) + (kp.e_tma ? 1 : 0));
+  const int threads = 32 * (3 + epi_warps(BN, EPI) + (kp.e_tma ? 1 : 0));
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(gemm_kernel<BN, EB, EPI, CG>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT);
