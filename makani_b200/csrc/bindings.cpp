@@ -131,12 +131,41 @@ static void check_extent(const Tensor& t, int64_t off, std::initializer_list<std
 
 void gemm_impl(const Tensor& a, const Tensor& b, Tensor& d, const c10::optional<Tensor>& bias,
                const c10::optional<Tensor>& resid, const c10::optional<Tensor>& preact, const std::vector<int64_t>& ip,
-               double alpha, const mk::GemmPeer* peer);
+               double alpha, const mk::GemmPeer* peer, mk::GemmRowSums* rows = nullptr);
 
 void gemm(const Tensor& a, const Tensor& b, Tensor& d, const c10::optional<Tensor>& bias,
           const c10::optional<Tensor>& resid, const c10::optional<Tensor>& preact, const std::vector<int64_t>& ip,
           double alpha) {
   gemm_impl(a, b, d, bias, resid, preact, ip, alpha, nullptr);
+}
+
+// Weight gradient with the sums of the rows of A beside it; false: the launch had no place for them, `sums` is untouched
+bool gemm_row_sums(const Tensor& a, const Tensor& b, Tensor& d, Tensor& sums, const std::vector<int64_t>& ip, double alpha) {
+  MK_CHECK(ip.size() == 40, "gemm: expected 40 integer parameters, got ", ip.size());
+  const int64_t groups = ip[27] != 0 ? ip[3] : 1;      // z_lo batches with outputs of their own
+  MK_CHECK(sums.is_cuda() && sums.scalar_type() == torch::kFloat32 && sums.is_contiguous() && sums.numel() == groups * ip[0] &&
+               sums.get_device() == a.get_device(),
+           "gemm: row sums must be contiguous fp32 CUDA of the rows of A");
+  Tensor part;      // freed to the allocator on return: later work of this stream only
+  struct Ctx {
+    Tensor* part;
+    const Tensor* like;
+  } ctx{&part, &sums};
+  mk::GemmRowSums rows;
+  rows.out = sums.data_ptr<float>();
+  rows.ctx = &ctx;
+  rows.scratch = [](void* c, long long floats) -> float* {
+    Ctx& x = *static_cast<Ctx*>(c);
+    try {
+      *x.part = torch::empty({floats}, x.like->options());
+    } catch (const std::exception&) {
+      return nullptr;
+    }
+    return x.part->data_ptr<float>();
+  };
+  rows.done = 0;
+  gemm_impl(a, b, d, c10::nullopt, c10::nullopt, c10::nullopt, ip, alpha, nullptr, &rows);
+  return rows.done != 0;
 }
 
 // GEMM whose B operand is gathered from peer devices along k and/or that takes part in cross-device handshakes
@@ -189,7 +218,7 @@ void peer_publish(const Tensor& src, int64_t rows, int64_t row_bytes, int64_t sr
 
 void gemm_impl(const Tensor& a, const Tensor& b, Tensor& d, const c10::optional<Tensor>& bias,
                const c10::optional<Tensor>& resid, const c10::optional<Tensor>& preact, const std::vector<int64_t>& ip,
-               double alpha, const mk::GemmPeer* peer) {
+               double alpha, const mk::GemmPeer* peer, mk::GemmRowSums* rows) {
   MK_CHECK(ip.size() == 40, "gemm: expected 40 integer parameters, got ", ip.size());
   MK_CHECK(a.is_cuda() && b.is_cuda() && d.is_cuda(), "gemm: tensors must be CUDA");
   MK_CHECK(a.scalar_type() == b.scalar_type(), "gemm: A and B dtypes differ");
@@ -264,7 +293,7 @@ void gemm_impl(const Tensor& a, const Tensor& b, Tensor& d, const c10::optional<
     e.preact = const_cast<char*>(base_ptr(*preact)) + preact_off * osz;
   }
   Tensor ef = err_flag_for(a);
-  check_cuda(mk::gemm_launch(p, A, B, e, ef.data_ptr<int>(), cur_stream(), peer), "gemm launch");
+  check_cuda(mk::gemm_launch(p, A, B, e, ef.data_ptr<int>(), cur_stream(), peer, rows), "gemm launch");
 }
 
 void inorm_fwd(const Tensor& x, Tensor& y, const c10::optional<Tensor>& w, const c10::optional<Tensor>& b, Tensor& stats,
@@ -709,6 +738,7 @@ void peer_allreduce(const std::vector<int64_t>& data_ptrs, const std::vector<int
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  m.def("gemm_row_sums", &gemm_row_sums);
   m.def("gemm", &gemm, "tcgen05 GEMM with fused epilogue");
   m.def("gemm_peer", &gemm_peer, "tcgen05 GEMM reading its B operand from peer devices");
   m.def("peer_sum", &peer_sum, "sum of the local segments of a peer buffer with the consumer handshake");

@@ -666,7 +666,7 @@ __global__ void __launch_bounds__(CS_THREADS) colsum_kernel(const uint4* __restr
   }
 }
 
-// out[g, c] = sum over the slabs (592 of them at most); 32 columns by 32 slabs at a time per CTA.  grid (ceil(C / 32), groups)
+// out[g, c] = sum over the slabs (some hundreds of them); 32 columns by 32 slabs at a time per CTA.  grid (ceil(C / 32), groups)
 __global__ void __launch_bounds__(1024) colsum_slabs_kernel(const float* __restrict__ part, float* __restrict__ out, int slabs, int C) {
   __shared__ float sh[32][33];
   const int c = blockIdx.x * 32 + threadIdx.x;
@@ -1365,8 +1365,12 @@ cudaError_t colsum(const __nv_bfloat16* x, float* out, float* scratch, long long
   float* const part = p.slabs > 1 ? scratch : out;
   colsum_kernel<<<dim3(p.parts, static_cast<unsigned>(p.slabs), groups), CS_THREADS, 0, s>>>(
       reinterpret_cast<const uint4*>(x), part, rows, p.V, p.vb, static_cast<int>(p.slab), inner, ostride / 8, gstride / 8);
-  if (p.slabs > 1)
-    colsum_slabs_kernel<<<dim3((C + 31) / 32, groups), dim3(32, 32), 0, s>>>(part, out, static_cast<int>(p.slabs), C);
+  if (p.slabs > 1) return colsum_add_slabs(part, out, static_cast<int>(p.slabs), C, groups, s);
+  return cudaGetLastError();
+}
+
+cudaError_t colsum_add_slabs(const float* part, float* out, int slabs, int C, int groups, cudaStream_t s) {
+  colsum_slabs_kernel<<<dim3((C + 31) / 32, groups), dim3(32, 32), 0, s>>>(part, out, slabs, C);
   return cudaGetLastError();
 }
 

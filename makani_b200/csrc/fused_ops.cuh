@@ -64,6 +64,8 @@ cudaError_t inorm_cl_apply(const __nv_bfloat16* x, const __nv_bfloat16* dy, __nv
 long long colsum_scratch(long long rows, int C, int groups = 1);
 cudaError_t colsum(const __nv_bfloat16* x, float* out, float* scratch, long long rows, int C, cudaStream_t s, int groups = 1,
                    long long gstride = 0, int inner = 0, long long ostride = 0);
+// out[g, c] = sum of part[g, 0 .. slabs, c], in a fixed order
+cudaError_t colsum_add_slabs(const float* part, float* out, int slabs, int C, int groups, cudaStream_t s);
 
 // ---- AFNO block weights: one layer's tensors (see the kernels), two layers per launch ----
 struct AfnoLayer {

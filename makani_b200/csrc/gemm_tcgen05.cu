@@ -8,6 +8,8 @@
 //                    epilogue: alternating 32-column chunks)
 //   warp EW+3      : only in launches whose epilogue operand (residual, saved pre-activation) is prefetched by TMA: its
 //                    producer, so that waiting for a free operand buffer never delays A and B
+//   warps EW+3..   : only in launches that also sum the rows of A (bias gradients): eight warps that add up every stage before it is
+//                    freed
 // Two accumulator buffers in TMEM let the epilogue of tile i overlap the main loop of tile i+1.
 // Every mbarrier wait is bounded; on expiry the kernel records a code in *err and drains.
 //
@@ -58,9 +60,11 @@ __host__ __device__ constexpr int epi_warps(int bn, int epi) { return epi == 0 ?
 // Register bound, given as a thread count: the warps of one scheduler's register bank (5, 4 or 3 of them) leave room for one
 // 64-register warp of the gradient all-reduce, which overlaps with these GEMMs in data-parallel training.
 __host__ __device__ constexpr int bound_threads(int bn, int epi) {
+  if (epi == 5) return 32 * (epi_warps(bn, 5) + 12);      // with the row sums: 19, 23 or 27 warps of at most 64 registers
   return epi == 0 || bn == 128 ? 384 : (bn == 192 ? 576 : 736);
 }
 constexpr int MAX_STAGES = 6;
+constexpr int SUM_WARPS = 8;
 constexpr int MAX_SEG = 8;
 
 // Handshake of a kernel that consumes buffers its peers have filled and/or fills a buffer that its peers consume.
@@ -121,6 +125,9 @@ struct KParams {
   int stages, e_tma;
   int d_zlo_on, d_zhi_on;         // fp32 output through TMA: 0 where all batches of that index add into one output
   int rd_shift;                   // log2 of rdiv where the output leaves through TMA (0: rows have one stride)
+  float* rowsum;                  // partial sums of the rows of A over k, [group][slab][row] (null: none)
+  int producers;                  // TMA producer warps at work
+  int rs_groups, rs_slabs;        // groups: z_lo batches with outputs of their own; slabs of one group
   int n_fast;                     // tile order: 1 = n-tile index fastest, 0 = m-tile index fastest
   int* err;
   // ---- B operand gathered from several devices: segment s of the k axis was written by rank s into the local buffer
@@ -149,6 +156,10 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
 
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive_n(uint32_t bar, uint32_t count) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
 
 // Bounded wait: polls the barrier and gives up after WAIT_LIMIT_NS of wall time. Returns false on expiry.
@@ -435,6 +446,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
   constexpr int EW = epi_warps(BN, EPI);
   constexpr int PRODUCER_2 = 2 + EW;      // second TMA producer
   constexpr int E_WARP = 3 + EW;
+  constexpr int SUM_WARP = 3 + EW;        // (no instance has both)
   constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
   constexpr int MN_BOX = 128 / EB;        // extent of an MN-major box along the contiguous dimension
   constexpr uint32_t TMEM_COLS = BN == 128 ? 256 : 512;   // two accumulators, rounded up to a power of two
@@ -459,7 +471,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
   auto tempty_bar = [&](int b) { return bar_base + 8u * (2 * MAX_STAGES + 2 + b); };
   auto efull_bar = [&](int b) { return bar_base + 8u * (2 * MAX_STAGES + 4 + b); };
   auto eempty_bar = [&](int b) { return bar_base + 8u * (2 * MAX_STAGES + 6 + b); };
-  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bar_ptr + 8 * (2 * MAX_STAGES + 8));
+  auto sum_bar = [&](int st) { return bar_base + 8u * (2 * MAX_STAGES + 8 + st); };
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bar_ptr + 8 * (3 * MAX_STAGES + 8));
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -471,7 +484,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(full_bar(s), 1);
-      mbar_init(empty_bar(s), 1);
+      mbar_init(empty_bar(s), EPI == 5 && p.rowsum != nullptr ? 1 + SUM_WARPS : 1);
+      if constexpr (EPI == 5) mbar_init(sum_bar(s), 1);
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(tfull_bar(b), 1);
@@ -533,7 +547,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
     // instructions one after the other, some 450 - 700 cycles; a slab's MMAs take 256 - 512, and with a single producer it was
     // this thread that most launches waited for, with the loads in flight far from filling the ring.  Back to back, under the power
     // cap: 768 -> 384 over 721 x 1440 tokens 699 -> 649 us, its gradient 707 -> 650, 384 -> 768 with GELU and GELU' 928 -> 882.
-    if (elect_one()) {
+    //
+    // With an odd number of stages both fill every stage, in turn.  Neither mistakes one lap for another: stages are freed in the
+    // order of their MMAs, so that having met the release of slab g - 2 - STAGES a producer that waits for slab g - STAGES knows
+    // slab g - 2 STAGES free.  Where the row sums' warps hold stages too there is no such order, and one producer fills them all
+    // (p.producers).
+    if (elect_one() && (warp == 0 || p.producers == 2)) {
+      const int step = p.producers;
       const uint32_t me = warp == 0 ? 0u : 1u;
       int s = static_cast<int>(me);
       uint32_t ph = 0, slab = 0;      // slab: slabs of the CTA so far; this producer fills those of its parity
@@ -546,10 +566,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
       const uint32_t load_bytes = A_STAGE_BYTES + (p.b_mn ? B_STAGE_BYTES : BNL * 128);
       const bool a_mn = p.a_mn != 0, b_mn = p.b_mn != 0;
       // this producer's next stage: waits until it is free and loads the k slabs of A at ka, rows m0, and of B at kb, rows nb
-      auto stage = [&](const CUtensorMap* mb, int ka, int m0, int azl, int azh, int kb, int nb, int bzl, int bzh) {
+      auto stage = [&](const CUtensorMap* mb, int ka, int m0, int azl, int azh, int kb, int nb, int bzl, int bzh, bool pass) {
         if (!mbar_wait(empty_bar(s), ph ^ 1u)) {
           atomicExch(p.err, 1);
           return false;
+        }
+        if constexpr (EPI == 5) {
+          if (pass) mbar_arrive_n(empty_bar(s), SUM_WARPS);
         }
         const uint32_t sa = smem_base + s * STAGE_BYTES;
         const uint32_t sb = sa + A_STAGE_BYTES;
@@ -585,7 +608,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
             for (int j = 0; j < BN / MN_BOX; ++j) tma_load_4d(sb + j * (BK * 128), mb, bar, nb + j * MN_BOX, kb, bzl, bzh);
           }
         }
-        s += 2;
+        s += step;
         if (s >= STAGES) {
           s -= STAGES;
           ph ^= 1u;
@@ -615,9 +638,94 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
               else apos = sg * p.K;
             }
           }
-          for (int k = lb + static_cast<int>((slab ^ me) & 1u) * BK; k < le && ok; k += 2 * BK)
-            ok = stage(mb, apos + k, m0, azl, azh, k, nb, bzl, bzh);
+          const int k0 = lb + static_cast<int>((slab ^ me) & (step - 1)) * BK;
+          if constexpr (EPI == 5) {
+            if (p.rowsum) {
+              int turn = k0 > lb ? 1 : 0;      // slab modulo the column tiles
+              for (int k = k0; k < le && ok; k += step * BK) {
+                while (turn >= p.n_tiles) turn -= p.n_tiles;
+                // another tile's turn: the row sums' warps pass this slab by (the stage is this producer's until it is loaded,
+                // so the arrival counts for its next release)
+                ok = stage(mb, apos + k, m0, azl, azh, k, nb, bzl, bzh, turn != c.nt);
+                turn += step;
+              }
+              slab += static_cast<uint32_t>(le - lb + BK - 1) / BK;
+              continue;
+            }
+          }
+          for (int k = k0; k < le && ok; k += step * BK) ok = stage(mb, apos + k, m0, azl, azh, k, nb, bzl, bzh, false);
           if (le > lb) slab += static_cast<uint32_t>(le - lb + BK - 1) / BK;
+        }
+      }
+    }
+  } else if (EPI == 5 && warp >= SUM_WARP) {
+    // ------------------------------------------------------------------ sums of the rows of A (bias gradients)
+    // The gradient of a bias is the sum over the tokens of the matrix that the weight gradient has in shared memory anyway:
+    // read from there, it costs no pass over memory (0.8 or 1.6 GB and two launches at 721 x 1440 tokens).  A is MN-major: a stage
+    // holds 64 tokens as rows of 64 channels, twice.  Warp w adds up 16 tokens of one half, a lane 8 channels of every fourth
+    // token, in fp32; the column tiles of one row block, which load the same slabs, take the slabs in turn, and for the others
+    // the producer frees the stage in the name of these warps.  Every warp writes a partial sum per tile, and a second launch adds
+    // them in a fixed order: as exact as the pass of their own that they replace (errors against 64 bits 3.5e-8 one-signed, 1e-7
+    // zero-mean, 721 x 1440 tokens, both).  Gradient and sums, a pass of their own / from here, us, 721 x 1440 tokens: 384 x 768
+    // 746 / 642, 768 x 384 766 / 736, 384 x 384 451 / 353; 240 x 480: 104 / 91, 111 / 98, 69 / 55; 2048 tokens: 32 / 24.
+    if constexpr (EPI == 5) {
+      const int w = warp - SUM_WARP, bx = w >> 2;
+      const uint32_t cgroup = lane & 7;
+      const int k0 = (w & 3) * 16 + (lane >> 3);
+      const uint8_t* const col = smem + bx * (BK * 128) + k0 * 128;
+      const uint32_t at0 = (cgroup ^ (k0 & 7)) << 4, at1 = (cgroup ^ ((k0 + 4) & 7)) << 4;
+      // The thread that issues the MMAs passes every slab in order and announces those of this tile's turn; waiting for the loads'
+      // own barrier, these warps could meet the parity of another lap, since they skip slabs.  In a pair that barrier lives in the
+      // leader; there the announcement is a commit, which reaches both CTAs when the slab's MMAs are done (told by one thread to
+      // another, at cluster scope, 768 x 384 over 721 x 1440 tokens took 950 us).
+      uint32_t seen = 0;               // parity of each stage's announcements
+      uint32_t first = 0;              // stage of the tile's first slab
+      bool ok = peers_ready;
+      for (uint32_t t = tile0; t < p.total_tiles; t += tile_step) {
+        const TileCoord c = decode_tile<BK, CG>(p, t, crank);
+        f32x2 acc[4] = {0ull, 0ull, 0ull, 0ull};
+        const int nblocks = c.skip ? 0 : (c.k_end - c.k_begin + BK - 1) / BK;
+        uint32_t s = (first + c.nt) % STAGES;
+        for (int kb = c.nt; kb < nblocks && ok; kb += p.n_tiles) {
+          const uint32_t want = (seen >> s) & 1u;
+          ok = __all_sync(0xffffffffu, mbar_wait(sum_bar(s), want));
+          if (!ok) {
+            if (lane == 0) atomicExch(p.err, 7);
+            break;
+          }
+          seen ^= 1u << s;
+          const uint8_t* const st = col + s * STAGE_BYTES;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            f32x2 v[4];
+            f2_unpack8(*reinterpret_cast<const uint4*>(st + i * (4 * 128) + (i & 1 ? at1 : at0)), v);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[j] = f2_add(acc[j], v[j]);
+          }
+          __syncwarp();
+          if (elect_one()) mbar_arrive(empty_bar(s));
+          s = (s + p.n_tiles) % STAGES;
+        }
+        first = (first + nblocks) % STAGES;
+        // lanes l, l + 8, l + 16, l + 24 hold the same channels
+        const int group = p.rs_groups > 1 ? c.zlo : 0;
+        const int z = p.rs_groups > 1 ? c.zhi : c.zhi * p.zlo_n + c.zlo;
+        const long long slab = ((static_cast<long long>(z) * p.splits + c.split) * p.n_tiles + c.nt) * 4 + (w & 3);
+        const int r0 = c.mt * BM + bx * 64 + static_cast<int>(cgroup) * 8;
+        float* const out = p.rowsum + (static_cast<long long>(group) * p.rs_slabs + slab) * p.M + r0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          float a, b;
+          f2_unpack(acc[j], a, b);
+#pragma unroll
+          for (int o = 8; o < 32; o <<= 1) {
+            a += __shfl_xor_sync(0xffffffffu, a, o);
+            b += __shfl_xor_sync(0xffffffffu, b, o);
+          }
+          if (lane < 8) {
+            if (r0 + 2 * j < p.M) out[2 * j] = a;
+            if (r0 + 2 * j + 1 < p.M) out[2 * j + 1] = b;
+          }
         }
       }
     }
@@ -687,6 +795,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
         }
         // the negative product of a complex one: bit 14 of the instruction descriptor negates B in one half of the k loop
         const uint32_t neg = p.cplx != 0 && c.half == p.neg_half ? 1u << 14 : 0u;
+        int turn = 0;
         const int kneg = p.neg_seg ? nblocks >> 1 : 0, kpos = p.neg_seg ? nblocks : nblocks >> 1;
         for (int kb = 0; kb < nblocks; ++kb) {
           if (!mbar_wait(full_bar(s), ph)) {
@@ -705,6 +814,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
           // frees the smem stage (in both CTAs of a pair) once these MMAs have read it
           if constexpr (CG == 2) tc_commit_pair(empty_bar(s));
           else tc_commit(empty_bar(s));
+          if constexpr (EPI == 5) {
+            if (p.rowsum) {      // announces the slabs that this tile sums up
+              if (turn == c.nt) {
+                if constexpr (CG == 2) tc_commit_pair(sum_bar(s));
+                else mbar_arrive(sum_bar(s));
+              }
+              if (++turn == p.n_tiles) turn = 0;
+            }
+          }
           if (++s == STAGES) {
             s = 0;
             ph ^= 1u;
@@ -1277,7 +1395,7 @@ template <int BN, int EB, int EPI, int CG>
 cudaError_t launch_t(const CUtensorMap& ma, const BMaps& mb, const CUtensorMap& me, const CUtensorMap& md,
                      const CUtensorMap& mp, const DMaps& mdx, KParams& kp, cudaStream_t stream) {
   constexpr int STAGE = A_STAGE_BYTES + b_stage_rows(BN, CG) * 128;
-  constexpr int FIXED = stg_bytes(BN, EPI) + 8 * (2 * MAX_STAGES + 8) + 16 + 1024;
+  constexpr int FIXED = stg_bytes(BN, EPI) + 8 * (3 * MAX_STAGES + 8) + 16 + 1024;
   const int e_bytes = kp.e_tma ? 2 * BM * BN * 2 : 0;
   int stages = (SMEM_LIMIT - FIXED - e_bytes) / STAGE;
   if (stages > MAX_STAGES) stages = MAX_STAGES;
@@ -1285,9 +1403,15 @@ cudaError_t launch_t(const CUtensorMap& ma, const BMaps& mb, const CUtensorMap& 
     snprintf(g_err, sizeof(g_err), "not enough shared memory for the requested tile configuration");
     return cudaErrorInvalidValue;
   }
+  // (see the producers: with row sums, an even number of stages for two of them)
+  kp.producers = 2;
+  if (kp.rowsum && stages % 2 != 0) {
+    if (stages > 3) --stages;
+    else kp.producers = 1;
+  }
   kp.stages = stages;
   const int smem = stages * STAGE + e_bytes + FIXED;
-  const int threads = 32 * (3 + epi_warps(BN, EPI) + (kp.e_tma ? 1 : 0));
+  const int threads = 32 * (3 + epi_warps(BN, EPI) + (kp.rowsum ? SUM_WARPS : (kp.e_tma ? 1 : 0)));
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(gemm_kernel<BN, EB, EPI, CG>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT);
@@ -1611,8 +1735,9 @@ int pick_splits(long long base, int kblocks, int slots, int least) {
 }  // namespace
 
 cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOperand& B, const GemmEpilogue& e,
-                        int* err_flag, cudaStream_t stream, const GemmPeer* peer) {
+                        int* err_flag, cudaStream_t stream, const GemmPeer* peer, GemmRowSums* rows) {
   g_err[0] = 0;
+  if (rows) rows->done = 0;
   if (p.M <= 0 || p.N <= 0 || p.zlo_n <= 0 || p.zhi_n <= 0) return cudaSuccess;
   // cuTensorMapEncodeTiled is a driver call: make sure this host thread has the primary context bound (threads
   // that only inherited the device index, e.g. autograd workers, do not until their first runtime call)
@@ -1812,6 +1937,18 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
     return cudaErrorInvalidValue;
   }
   kp.total_tiles = static_cast<uint32_t>(base_tiles * kp.splits);
+  // sums of the rows of A: only where the launch has A's tokens in shared memory as rows, all of them and each once
+  if (rows && epi == 5 && A.mn_major && p.cplx == 0 && kp.nseg == 1 && p.rmin_a == 0 && p.rmin_b <= 0 && p.rmax_a == 0 && p.rmax_b >= p.M &&
+      p.kmin_a == 0 && p.kmin_b <= 0 && p.kmax_a == 0 && p.kmax_b >= p.K && (p.zlo_n == 1 || A.zs_lo != 0) && (p.zhi_n == 1 || A.zs_hi != 0) &&
+      (p.zhi_n == 1 || e.d_zhi == 0)) {
+    kp.rs_groups = p.zlo_n > 1 && e.d_zlo != 0 ? p.zlo_n : 1;
+    const long long slabs = z_all / kp.rs_groups * kp.splits * kp.n_tiles * 4;
+    if (slabs < (1 << 20) && kp.rs_groups < 65536) {
+      kp.rs_slabs = static_cast<int>(slabs);
+      kp.rowsum = rows->scratch(rows->ctx, slabs * kp.rs_groups * p.M);
+      if (!kp.rowsum) return cudaErrorMemoryAllocation;
+    }
+  }
   kp.dv_n = make_div(kp.n_tiles);
   kp.dv_m = make_div(kp.m_tiles);
   kp.dv_split = make_div(kp.splits);
@@ -1855,14 +1992,20 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
   }                                                                                                    \
   if (bn == 192) return launch_t<192, 2, EPI_, 1>(ma, mbs, me, md, mp, mdx, kp, stream);               \
   return launch_t<128, 2, EPI_, 1>(ma, mbs, me, md, mp, mdx, kp, stream);
-  switch (epi) {
-    case 1: { MK_DISPATCH(1) }
-    case 2: { MK_DISPATCH(2) }
-    case 3: { MK_DISPATCH(3) }
-    case 4: { MK_DISPATCH(4) }
-    case 5: { MK_DISPATCH(5) }
-    default: { MK_DISPATCH(0) }
-  }
+  auto run = [&]() -> cudaError_t {
+    switch (epi) {
+      case 1: { MK_DISPATCH(1) }
+      case 2: { MK_DISPATCH(2) }
+      case 3: { MK_DISPATCH(3) }
+      case 4: { MK_DISPATCH(4) }
+      case 5: { MK_DISPATCH(5) }
+      default: { MK_DISPATCH(0) }
+    }
+  };
+  const cudaError_t launched = run();
+  if (launched != cudaSuccess || !kp.rowsum) return launched;
+  rows->done = 1;
+  return colsum_add_slabs(kp.rowsum, rows->out, kp.rs_slabs, p.M, kp.rs_groups, stream);
 #undef MK_DISPATCH
 }
 

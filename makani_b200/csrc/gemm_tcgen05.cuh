@@ -85,6 +85,15 @@ struct GemmPeer {
   void* Dx[7];                     // base pointers matching GemmEpilogue::D (offset already applied)
 };
 
+// Optional: the sums over k of the rows of A (the gradient of a bias, beside the weight gradient), fp32 [M], or [z_lo][M] where the
+// z_lo batches have outputs of their own.  Taken where A is MN-major bf16 and the output is fp32 with plain rows; `done` says so.
+struct GemmRowSums {
+  float* out;
+  float* (*scratch)(void* ctx, long long floats);      // device memory until the work of this launch is done; null on failure
+  void* ctx;
+  int done;
+};
+
 // Copy of a strided 2-D block into the same place of `ndst` destination buffers (this device's and its peers'),
 // with the producer side of the handshake in `g` (wait list 0, signal list 0) executed by the same kernel.
 cudaError_t peer_publish_launch(const void* src, long long rows, long long row_bytes, long long src_stride_bytes,
@@ -99,7 +108,8 @@ cudaError_t peer_sum_launch(void* out, long long n_elems, const void* const* src
 // Returns cudaSuccess or an error; never throws.  `err_flag` is a device int that the kernel sets to a
 // non-zero code when a bounded barrier wait runs out (the launch still terminates).
 cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOperand& B,
-                        const GemmEpilogue& e, int* err_flag, cudaStream_t stream, const GemmPeer* peer = nullptr);
+                        const GemmEpilogue& e, int* err_flag, cudaStream_t stream, const GemmPeer* peer = nullptr,
+                        GemmRowSums* rows = nullptr);
 
 const char* gemm_last_error();
 

@@ -252,7 +252,6 @@ class _AFNOFilter(torch.autograd.Function):
         acc = torch.zeros(2 * n1 + n2 + 2 * bs * nb, dtype=torch.float32, device=dev)
         dw1, dw2 = acc[:n1].view(nb, 2 * hid, 2 * bs), acc[n1: 2 * n1].view(nb, 2 * bs, 2 * hid)
         db1, db2 = acc[2 * n1: 2 * n1 + n2].view(nb, 2 * hid), acc[2 * n1 + n2:].view(nb, 2 * bs)
-        native = dev.type == "cuda"
         # adjoint of the synthesis along W, then along H with the shrinkage mask (saved output != 0) in the epilogue
         dt4 = _stage_w_analysis(dy, plan.gw_t, plan)                                   # [B, ncols, H, 2, C]
         do2 = torch.empty_like(o2)
@@ -266,25 +265,21 @@ class _AFNOFilter(torch.autograd.Function):
              Operand(w2q, ld=2 * hid, mn_major=True, zs_lo=2 * bs * 2 * hid),
              Output(do1, rs_lo=nb * 2 * hid, d_zlo=2 * hid, d_zhi=nkx * nb * 2 * hid), zlo_n=nb, zhi_n=B * nc,
              act=ACT_DRELU, resid=o1)
-        gemm(2 * bs, 2 * hid, nkx, Operand(do2, ld=2 * bs, mn_major=True, zs_lo=nkx * 2 * bs, zs_hi=nb * nkx * 2 * bs),
-             Operand(o1, ld=nb * 2 * hid, mn_major=True, zs_lo=2 * hid, zs_hi=nkx * nb * 2 * hid),
-             Output(dw2, rs_lo=2 * hid, d_zlo=2 * bs * 2 * hid), zlo_n=nb, zhi_n=B * nc, accumulate=True, splits=0)
-        if has_b2:
-            if native:
-                _ext.require().colsum_groups(do2, db2, B * nc, nb, nkx)
-            else:
-                db2.copy_(do2.reshape(B * nc, nb, nkx, 2 * bs).float().sum(dim=(0, 2)))
+        done = gemm(2 * bs, 2 * hid, nkx, Operand(do2, ld=2 * bs, mn_major=True, zs_lo=nkx * 2 * bs, zs_hi=nb * nkx * 2 * bs),
+                    Operand(o1, ld=nb * 2 * hid, mn_major=True, zs_lo=2 * hid, zs_hi=nkx * nb * 2 * hid),
+                    Output(dw2, rs_lo=2 * hid, d_zlo=2 * bs * 2 * hid), zlo_n=nb, zhi_n=B * nc, accumulate=True, splits=0,
+                    row_sums=db2 if has_b2 else None) or not has_b2
+        if not done:
+            _ext.require().colsum_groups(do2, db2, B * nc, nb, nkx)
         # first layer
         dyt = torch.empty(B * nc, nb, nkx, 2, bs, dtype=dt, device=dev)
         _tokens_to_blocks(do1, Operand(w1q, ld=2 * bs, mn_major=True, zs_lo=2 * hid * 2 * bs), dyt, plan, B, nb, 2 * bs, 2 * hid)
-        gemm(2 * hid, 2 * bs, T, Operand(do1, ld=nb * 2 * hid, mn_major=True, zs_lo=2 * hid),
-             Operand(y, ld=2 * C, mn_major=True, zs_lo=2 * bs),
-             Output(dw1, rs_lo=2 * bs, d_zlo=2 * hid * 2 * bs), zlo_n=nb, accumulate=True, splits=0)
-        if has_b1:
-            if native:
-                _ext.require().colsum(do1, db1)
-            else:
-                db1.copy_(do1.float().sum(dim=0))
+        done = gemm(2 * hid, 2 * bs, T, Operand(do1, ld=nb * 2 * hid, mn_major=True, zs_lo=2 * hid),
+                    Operand(y, ld=2 * C, mn_major=True, zs_lo=2 * bs),
+                    Output(dw1, rs_lo=2 * bs, d_zlo=2 * hid * 2 * bs), zlo_n=nb, accumulate=True, splits=0,
+                    row_sums=db1 if has_b1 else None) or not has_b1
+        if not done:
+            _ext.require().colsum(do1, db1)
         (gw1, gw2), (gb1, gb2) = _fold([dw1, dw2], [db1, db2], [(2, nb, bs, hid), (2, nb, hid, bs)], (has_b1, has_b2))
         gw1, gb1, gw2, gb2 = (g if g is None else g.to(t) for g, t in zip((gw1, gb1, gw2, gb2), ctx.wtypes))
         # adjoint of the analysis along H and along W; the skip's gradient joins in the last epilogue

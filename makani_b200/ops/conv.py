@@ -138,15 +138,19 @@ def _conv_dgrad(dy, wq, ci, act=ACT_NONE, aux=None, x_layout=None, out=None, syn
     return dx
 
 
-def _conv_wgrad(dy, x, splits: int = 0):
-    """dW[co, ci] = sum_{b,hw} dY[b, co, hw] X[b, ci, hw] in fp32 (split-k, atomically accumulated)."""
+def _conv_wgrad(dy, x, splits: int = 0, bias: bool = False):
+    """dW[co, ci] = sum_{b,hw} dY[b, co, hw] X[b, ci, hw] in fp32 (split-k, atomically accumulated); with `bias` also
+    db[co] = sum_{b,hw} dY[b, co, hw], from the same launch where it reads dY as tokens."""
     B, co, H, W = dy.shape
     ci = x.shape[1]
     T = H * W
     dw = torch.zeros(co, ci, dtype=torch.float32, device=dy.device)
-    gemm(co, ci, T, _chan_rows(dy, layout_of(dy)), _chan_rows(x, layout_of(x)), Output(dw, rs_lo=ci), zlo_n=B,
-         accumulate=True, splits=splits)
-    return dw
+    db = torch.empty(co, dtype=torch.float32, device=dy.device) if bias else None
+    done = gemm(co, ci, T, _chan_rows(dy, layout_of(dy)), _chan_rows(x, layout_of(x)), Output(dw, rs_lo=ci), zlo_n=B,
+                accumulate=True, splits=splits, row_sums=db)
+    if not bias:
+        return dw
+    return dw, db if done else _chan_sum(dy)
 
 
 def _chan_sum(dy):
@@ -188,8 +192,13 @@ class _Conv1x1(torch.autograd.Function):
         else:
             g = dy
         dx = _conv_dgrad(g, wq, ctx.ci, x_layout=layout_of(x)) if ctx.needs_input_grad[0] else None
-        dw = _conv_wgrad(g, x).reshape(ctx.wshape) if ctx.needs_input_grad[1] else None
-        db = _chan_sum(g) if ctx.has_bias and ctx.needs_input_grad[2] else None
+        dw = db = None
+        want_db = ctx.has_bias and ctx.needs_input_grad[2]
+        if ctx.needs_input_grad[1]:
+            dw, db = _conv_wgrad(g, x, bias=True) if want_db else (_conv_wgrad(g, x), None)
+            dw = dw.reshape(ctx.wshape)
+        elif want_db:
+            db = _chan_sum(g)
         return dx, dw, db, dres, None, None, None
 
 
@@ -221,12 +230,10 @@ class _MLP2(torch.autograd.Function):
         has_b1, has_b2, has_res = ctx.flags
         dy = _canon(dy)
         dpre = _conv_dgrad(dy, w2q, ch, act=ACT_MULAUX, aux=dact, x_layout=layout_of(dact))
-        dw2 = _conv_wgrad(dy, h).reshape(ctx.wshapes[1])
-        db2 = _chan_sum(dy) if has_b2 else None
+        dw2, db2 = _conv_wgrad(dy, h, bias=True) if has_b2 else (_conv_wgrad(dy, h), None)
         dx = _conv_dgrad(dpre, w1q, ci, x_layout=layout_of(x)) if ctx.needs_input_grad[0] else None
-        dw1 = _conv_wgrad(dpre, x).reshape(ctx.wshapes[0])
-        db1 = _chan_sum(dpre) if has_b1 else None
-        return dx, dw1, db1, dw2, db2, (dy if has_res else None), None, None
+        dw1, db1 = _conv_wgrad(dpre, x, bias=True) if has_b1 else (_conv_wgrad(dpre, x), None)
+        return dx, dw1.reshape(ctx.wshapes[0]), db1, dw2.reshape(ctx.wshapes[1]), db2, (dy if has_res else None), None, None
 
 
 def records_grad(*tensors) -> bool:

@@ -217,7 +217,7 @@ def gemm(M: int, N: int, K: int, A: Operand, B: Operand, D: Output, *, zlo_n: in
          resid: Optional[torch.Tensor] = None, resid_offset: int = 0, preact: Optional[torch.Tensor] = None,
          preact_offset: int = 0, accumulate: bool = False, splits: int = 1, tri: Optional[Tri] = None, bn: int = 0,
          segments=None, sync=None, dests=None, act_param: float = 0.0, bias_zs: int = 0,
-         preact_deriv: bool = False) -> None:
+         preact_deriv: bool = False, row_sums: Optional[torch.Tensor] = None) -> bool:
     """Run the batched GEMM described above, writing into `D.tensor` in place.
 
     `segments` (list of `Segment`) spreads the k axis of B over several devices: `K` is then the padded k extent
@@ -229,7 +229,11 @@ def gemm(M: int, N: int, K: int, A: Operand, B: Operand, D: Output, *, zlo_n: in
     sums; one where a bias or an activation is applied).
 
     `preact` receives the value before the activation; with `preact_deriv` (act = ACT_GELU only) it receives GELU' of
-    that value instead, which the backward pass multiplies in with `act=ACT_MULAUX, resid=<that tensor>`."""
+    that value instead, which the backward pass multiplies in with `act=ACT_MULAUX, resid=<that tensor>`.
+
+    `row_sums` (fp32 [M], or [zlo_n, M] where the z_lo batches have outputs of their own) receives the sums over k and the batches
+    of the rows of A: the gradient of a bias beside that of the weights.  Returns whether it did (an MN-major A and an fp32 output
+    with plain rows); where not, the tensor is untouched."""
     tri = tri or Tri()
     assert not preact_deriv or (act == ACT_GELU and preact is not None)
     if bias is None:
@@ -237,7 +241,11 @@ def gemm(M: int, N: int, K: int, A: Operand, B: Operand, D: Output, *, zlo_n: in
     if not A.tensor.is_cuda:
         _emulate(M, N, K, A, B, D, zlo_n, zhi_n, alpha, bias, bias_mode, act, resid, resid_offset, preact, preact_offset,
                  accumulate, tri, segments, act_param, bias_zs, preact_deriv)
-        return
+        if row_sums is not None:
+            rs, ks = (1, A.ld) if A.mn_major else (A.ld, 1)
+            a = _flat(A.tensor)[A.offset:].as_strided((zhi_n, zlo_n, M, K), (A.zs_hi, A.zs_lo, rs, ks)).float()
+            row_sums.copy_((a.sum(dim=(0, 3)) if D.d_zlo else a.sum(dim=(0, 1, 3))).reshape(row_sums.shape))
+        return row_sums is not None
     ext = _ext.require()
     ip = [M, N, K, zlo_n, zhi_n, splits, bn,
           tri.rmin_a, tri.rmin_b, tri.rmax_a, tri.rmax_b, tri.kmin_a, tri.kmin_b, tri.kmax_a, tri.kmax_b,
@@ -256,8 +264,12 @@ def gemm(M: int, N: int, K: int, A: Operand, B: Operand, D: Output, *, zlo_n: in
             raise ValueError("a single-segment operand is an ordinary operand: pass it as B")
         ext.gemm_peer(A.tensor, B.tensor, D.tensor, bias, resid, preact, ip, float(alpha), seg, list(sync or []),
                       [int(d) for d in (dests or [])])
-        return
+        return False
+    if row_sums is not None:
+        assert bias is None and resid is None and preact is None
+        return ext.gemm_row_sums(A.tensor, B.tensor, D.tensor, row_sums, ip, float(alpha))
     ext.gemm(A.tensor, B.tensor, D.tensor, bias, resid, preact, ip, float(alpha))
+    return False
 
 
 def gemm_complex(mode: int, M: int, N: int, K: int, A: Operand, B: Operand, D: Output, d_half: int, *, zlo_n: int = 1, zhi_n: int = 1,

@@ -41,14 +41,17 @@ def _lin_dgrad(dy, wq, act=ACT_NONE, aux=None):
     return dx
 
 
-def _lin_wgrad(dy, x2):
+def _lin_wgrad(dy, x2, bias=False):
     T, O = dy.shape
     C = x2.shape[1]
     dw = torch.zeros(O, C, dtype=torch.float32, device=dy.device)
     # dW[o, c] = sum_t dY[t, o] X[t, c]: both operands row-contiguous in their own index, K = t
-    gemm(O, C, T, Operand(dy, ld=O, mn_major=True), Operand(x2, ld=C, mn_major=True), Output(dw, rs_lo=C),
-         accumulate=True, splits=0)
-    return dw
+    db = torch.empty(O, dtype=torch.float32, device=dy.device) if bias else None
+    done = gemm(O, C, T, Operand(dy, ld=O, mn_major=True), Operand(x2, ld=C, mn_major=True), Output(dw, rs_lo=C),
+                accumulate=True, splits=0, row_sums=db)
+    if not bias:
+        return dw
+    return dw, db if done else row_sums(dy, O)
 
 
 class _MLP2Last(torch.autograd.Function):
@@ -72,11 +75,9 @@ class _MLP2Last(torch.autograd.Function):
         x2, w1q, w2q, dact, h = ctx.saved_tensors
         dy2 = dy.reshape(-1, dy.shape[-1]).contiguous()
         dpre = _lin_dgrad(dy2, w2q, act=ACT_MULAUX, aux=dact)
-        dw2 = _lin_wgrad(dy2, h)
-        db2 = row_sums(dy2, dy2.shape[1]) if ctx.flags[1] else None
+        dw2, db2 = _lin_wgrad(dy2, h, bias=True) if ctx.flags[1] else (_lin_wgrad(dy2, h), None)
         dx = _lin_dgrad(dpre, w1q).reshape(ctx.shp) if ctx.needs_input_grad[0] else None
-        dw1 = _lin_wgrad(dpre, x2)
-        db1 = row_sums(dpre, dpre.shape[1]) if ctx.flags[0] else None
+        dw1, db1 = _lin_wgrad(dpre, x2, bias=True) if ctx.flags[0] else (_lin_wgrad(dpre, x2), None)
         return dx, dw1, db1, dw2, db2, None
 
 
@@ -98,8 +99,11 @@ class _LinearLast(torch.autograd.Function):
         x2, wq = ctx.saved_tensors
         dy2 = dy.reshape(-1, dy.shape[-1]).contiguous()
         dx = _lin_dgrad(dy2, wq).reshape(ctx.shp) if ctx.needs_input_grad[0] else None
-        dw = _lin_wgrad(dy2, x2) if ctx.needs_input_grad[1] else None
-        db = row_sums(dy2, dy2.shape[1]) if ctx.has_bias else None
+        dw = db = None
+        if ctx.needs_input_grad[1]:
+            dw, db = _lin_wgrad(dy2, x2, bias=True) if ctx.has_bias else (_lin_wgrad(dy2, x2), None)
+        elif ctx.has_bias:
+            db = row_sums(dy2, dy2.shape[1])
         return dx, dw, db
 
 

@@ -618,3 +618,40 @@ def test_planar_weight_gradient_on_pairs(b, l, m, co, ci):
         assert _rel(got, ref) < 2.0 ** -24 * (b * m) ** 0.5 * 4
         assert (got.double() - ref).abs().max() < 2.0 ** -16 * ref.abs().max()
     _ext.check_device_errors(dev)
+
+
+@pytest.mark.parametrize("m,n,k,zlo,zhi,groups", [
+    (8, 8, 1, 1, 1, False),             # one token, the smallest operands
+    (72, 40, 63, 2, 1, False),          # part of one slab, batches that add up
+    (136, 384, 1000, 1, 1, False),      # two row blocks, two column tiles that take the slabs in turn
+    (384, 768, 30001, 1, 1, False),     # three row blocks on single CTAs, many splits, a ragged last slab
+    (768, 384, 65537, 1, 1, False),     # CTA pairs
+    (520, 256, 4097, 3, 1, False),      # pairs with a padded row block, batches
+    (192, 192, 91, 8, 45, True),        # one vector per group, summed over the other batch index
+])
+def test_row_sums_beside_the_weight_gradient(m, n, k, zlo, zhi, groups):
+    from makani_b200.ops.gemm import Operand, Output, gemm
+    g = torch.Generator(device="cuda").manual_seed(m + k)
+    # one-signed, so that nothing cancels
+    a = (torch.rand(zhi, zlo, k, m, device="cuda", generator=g) + 0.5).bfloat16()
+    b = torch.randn(zhi, zlo, k, n, device="cuda", generator=g).bfloat16()
+    outs = zlo if groups else 1
+
+    def run(sums):
+        d = torch.zeros(outs, m, n, device="cuda")
+        done = gemm(m, n, k, Operand(a, ld=m, mn_major=True, zs_lo=k * m, zs_hi=zlo * k * m),
+                    Operand(b, ld=n, mn_major=True, zs_lo=k * n, zs_hi=zlo * k * n),
+                    Output(d, rs_lo=n, d_zlo=m * n if groups else 0), zlo_n=zlo, zhi_n=zhi, accumulate=True, splits=0, row_sums=sums)
+        return d, done
+
+    sums, again = (torch.full((outs, m), float("nan"), device="cuda") for _ in range(2))
+    d, done = run(sums)
+    _, _ = run(again)
+    plain, _ = run(None)
+    assert done and torch.equal(sums, again)
+    # a lane adds up to four tokens of every 64 one after the other, then some 64 partial sums: each step rounds to 2^-24
+    ref = a.double().sum(dim=(0, 2) if groups else (0, 1, 2)).reshape(outs, m)
+    steps = 4 * -(-k // 64) + 64
+    assert ((sums.double() - ref).abs() <= steps * 2.0 ** -24 * ref).all()
+    # the gradient itself: the same chains, added up in another order
+    assert (d - plain).norm() <= 1e-6 * plain.norm() + 1e-12
