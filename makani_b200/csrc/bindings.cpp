@@ -401,6 +401,42 @@ void gemm_complex(const Tensor& a, const Tensor& b, Tensor& d, const c10::option
   check_cuda(mk::gemm_launch(p, A, B, e, ef.data_ptr<int>(), cur_stream(), nullptr), "gemm_complex launch");
 }
 
+// Folded Fourier transform (GemmProblem::cplx 4 and 5): table [rows, 2 parts of a_part columns], B planes and output over z
+void gemm_fold(const Tensor& a, const Tensor& b, Tensor& d, const std::vector<int64_t>& ip) {
+  MK_CHECK(ip.size() == 17, "gemm_fold: expected 17 integer parameters, got ", ip.size());
+  MK_CHECK(a.is_cuda() && b.is_cuda() && d.is_cuda() && a.scalar_type() == torch::kBFloat16 && b.scalar_type() == torch::kBFloat16 &&
+               d.scalar_type() == torch::kBFloat16,
+           "gemm_fold: bf16 CUDA operands expected");
+  c10::cuda::CUDAGuard guard(a.device());
+  int k = 0;
+  mk::GemmProblem p;
+  memset(&p, 0, sizeof(p));
+  p.cplx = static_cast<int>(ip[k++]);
+  MK_CHECK(p.cplx == 4 || p.cplx == 5, "gemm_fold: bad mode");
+  p.rows = ip[k++]; p.M = ip[k++]; p.N = ip[k++]; p.K = ip[k++]; p.mirror = ip[k++];
+  p.zlo_n = 1; p.zhi_n = ip[k++];
+  p.elem_bytes = 2;
+  p.splits = 1;
+  p.rmax_b = p.kmax_b = 1 << 30;
+  mk::GemmOperand A, B;
+  A.rows = p.rows; A.mn_major = 0; A.ld = ip[k++]; A.zs_lo = 0; A.zs_hi = 0; p.a_plane = ip[k++];
+  const int64_t b_off = ip[k++];
+  B.rows = p.N; B.mn_major = ip[k++]; B.ld = ip[k++]; B.zs_lo = 0; B.zs_hi = ip[k++]; p.b_plane = ip[k++];
+  A.ptr = base_ptr(a);
+  B.ptr = base_ptr(b) + b_off * 2;
+  check_extent(a, 0, {{p.rows, A.ld}, {2, p.a_plane}, {p.K, 1}}, "A");
+  check_extent(b, b_off, {{B.mn_major ? p.K : p.N, B.ld}, {B.mn_major ? p.N : p.K, 1}, {p.zhi_n, B.zs_hi}, {2, p.b_plane}}, "B");
+  mk::GemmEpilogue e;
+  memset(&e, 0, sizeof(e));
+  const int64_t d_off = ip[k++];
+  e.D = const_cast<char*>(base_ptr(d)) + d_off * 2;
+  e.rs_lo = ip[k++]; e.d_zhi = ip[k++];
+  check_extent(d, d_off, {{p.zhi_n, e.d_zhi}, {p.rows, e.rs_lo}, {p.N, 1}}, "output");
+  e.alpha = 1.f;
+  Tensor ef = err_flag_for(a);
+  check_cuda(mk::gemm_launch(p, A, B, e, ef.data_ptr<int>(), cur_stream(), nullptr), "gemm_fold launch");
+}
+
 // real and imaginary planes of w (complex64 [Cin, Cout, L]) -> bf16 [L, 2, Cout, Cin]
 void spectral_planes(const Tensor& w, Tensor& wp) {
   MK_CHECK(w.is_cuda() && w.scalar_type() == torch::kComplexFloat && w.is_contiguous() && w.dim() == 3, "spectral_planes: bad weight");
@@ -751,6 +787,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("inorm_partial_stats", &inorm_partial_stats);
   m.def("cast_pad", &cast_pad);
   m.def("gemm_complex", &gemm_complex);
+  m.def("gemm_fold", &gemm_fold);
   m.def("spectral_planes", &spectral_planes);
   m.def("colsum", &colsum);
   m.def("colsum_groups", &colsum_groups);

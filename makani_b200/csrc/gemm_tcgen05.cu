@@ -20,12 +20,19 @@
 // "stage free" and "accumulator full" signals to both CTAs.  Per tensor-core cycle every SM then takes a third less
 // data from L2 (two thirds with 128-wide tiles), which is what bounds these GEMMs.
 //
-// Complex products (p.cplx): real and imaginary planes of the operands are multiplied without ever forming the real 2x2-block
+// Complex products (p.cplx = 1, 2, 3): real and imaginary planes of the operands are multiplied without ever forming the real 2x2-block
 // matrix.  The column tiles come in two halves (real, imaginary part of the result) and the k loop in two segments that
 // select the planes; the one negative product of the four uses the negation bit of the MMA's instruction descriptor.
 //   1: D(h) = sum_s A[.., s Kh + k] B(plane h ^ s),  minus at h = 0, s = 1      (product with W)
 //   2: the same, minus at h = 1, s = 0                                          (product with the conjugate of W)
 //   3: D(h) = sum_s A(plane s ^ h) B(plane s),       minus at h = 1, s = 1      (weight gradient)
+// Folded transforms (p.cplx = 4, 5): a Fourier matrix has rows r and R - r that differ in nothing but the sign of one half of their
+// columns, so one product of half the rows serves both.  The two halves are two segments of the k loop with accumulators of their
+// own, and the epilogue stores their sum at row r and their difference at row R - r, both from fp32:
+//   4: rows are longitudes (synthesis): the halves are the cosine and the sine terms, i.e. the real and imaginary planes of B
+//   5: rows are (order, re / im) pairs of all orders up to half the points (analysis): the halves are the even and the odd
+//      points; the pairs keep their order, and the imaginary difference changes its sign
+//
 // 384 x 384 weights of 240 degrees: the operand takes 69 us to make instead of 95 (half the bytes), the products 87 - 94 us instead
 // of 105 - 114, the weight gradient one launch of 90 us instead of two of 78 and a swapped copy of 31.
 //
@@ -121,6 +128,8 @@ struct KParams {
   int m_tiles, n_tiles;
   FastDiv dv_n, dv_m, dv_split, dv_zlo;
   uint32_t total_tiles;           // below 2^31
+  int a_part;                     // k coordinate of the second part of a K-major A (complex and folded products)
+  int mirror, m_half, fold_rows;  // folded products: rows r and mirror - r; rows past m_half are the mirrors' business
   int cplx, nth, neg_half, neg_seg;   // complex product: mode, column tiles per half, the negative (half, segment)
   int stages, e_tma;
   int d_zlo_on, d_zhi_on;         // fp32 output through TMA: 0 where all batches of that index add into one output
@@ -408,13 +417,14 @@ __device__ __forceinline__ TileCoord decode_tile(const KParams& p, uint32_t t, i
 // Specialised epilogues leave through TMA stores of 32-row x 128-byte boxes, one per epilogue warp and output.  Without an
 // epilogue operand (1, 2) the boxes are staged in a buffer of their own; with one (3, 4) the warp overwrites the operand's
 // box in place, element by element, and the store reads from there: no staging, so 192-column tiles fit.
-__host__ __device__ constexpr int stg_warp_bytes(int epi) { return epi == 2 ? 2 * 32 * 128 : (epi == 1 || epi == 5 ? 32 * 128 : 0); }
+__host__ __device__ constexpr int stg_warp_bytes(int epi) { return epi == 2 || epi == 6 ? 2 * 32 * 128 : (epi == 1 || epi == 5 ? 32 * 128 : 0); }
 __host__ __device__ constexpr int stg_bytes(int bn, int epi) { return epi_warps(bn, epi) * stg_warp_bytes(epi); }
 
 // EPI selects a compile-time specialised epilogue (bf16 output but for 5):
 //   0 generic (all options decided at run time)      1 plain store
 //   2 GELU + saved pre-activation                     3 + residual (TMA-prefetched)      4 * GELU'(aux) (TMA-prefetched)
 //   5 fp32 output, stored or added (split-k, summed batches): weight gradients
+//   6 sum and difference of two accumulators, stored at row r and its mirror row (folded transforms)
 // rows of B per stage: whole MN-major boxes of 64 (a pair's half of a 192-wide tile is one and a half of them)
 __host__ __device__ constexpr int b_stage_rows(int bn, int cg) { return (bn / cg + 63) / 64 * 64; }
 
@@ -449,7 +459,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
   constexpr int SUM_WARP = 3 + EW;        // (no instance has both)
   constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
   constexpr int MN_BOX = 128 / EB;        // extent of an MN-major box along the contiguous dimension
-  constexpr uint32_t TMEM_COLS = BN == 128 ? 256 : 512;   // two accumulators, rounded up to a power of two
+  constexpr int ACC_COLS = EPI == 6 ? 2 * BN : BN;        // columns of one accumulator buffer
+  constexpr uint32_t TMEM_COLS = ACC_COLS == 128 ? 256 : 512;   // two of them, rounded up to a power of two
   constexpr uint32_t E_BYTES = BM * BN * 2;    // bf16 epilogue-operand tile
   const int STAGES = p.stages;
 
@@ -635,7 +646,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
               // segment and half select the planes, which take the place of the lower batch index
               bzl = p.cplx == 3 ? sg : (sg ^ c.half);
               if (p.cplx == 3) azl = sg ^ c.half;
-              else apos = sg * p.K;
+              else apos = sg * p.a_part;
             }
           }
           const int k0 = lb + static_cast<int>((slab ^ me) & (step - 1)) * BK;
@@ -780,7 +791,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
           break;
         }
         tc_fence_after();
-        const uint32_t tmem_d = tmem_base + buf * BN;
+        const uint32_t tmem_d = tmem_base + buf * ACC_COLS;
         uint32_t accum = 0;
         int nblocks = 0;
         if (p.nseg > 1) {
@@ -797,6 +808,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
         const uint32_t neg = p.cplx != 0 && c.half == p.neg_half ? 1u << 14 : 0u;
         int turn = 0;
         const int kneg = p.neg_seg ? nblocks >> 1 : 0, kpos = p.neg_seg ? nblocks : nblocks >> 1;
+        const int khalf = nblocks >> 1;
         for (int kb = 0; kb < nblocks; ++kb) {
           if (!mbar_wait(full_bar(s), ph)) {
             atomicExch(p.err, 3);
@@ -806,9 +818,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
           tc_fence_after();
           const uint32_t off = static_cast<uint32_t>(s) * (STAGE_BYTES >> 4);
           const uint32_t id = idesc | (kb >= kneg && kb < kpos ? neg : 0u);
+          uint32_t acc_d = tmem_d;
+          if constexpr (EPI == 6) {      // the second half of the columns has an accumulator of its own
+            if (kb >= khalf) acc_d = tmem_d + BN;
+            if (kb == khalf) accum = 0;
+          }
 #pragma unroll
           for (int kk = 0; kk < BK / UMMA_K; ++kk) {
-            tc_mma<EB, CG>(tmem_d, a_lo0 + off + kk * a_kstep, a_hi, b_lo0 + off + kk * b_kstep, b_hi, id, accum);
+            tc_mma<EB, CG>(acc_d, a_lo0 + off + kk * a_kstep, a_hi, b_lo0 + off + kk * b_kstep, b_hi, id, accum);
             accum = 1;
           }
           // frees the smem stage (in both CTAs of a pair) once these MMAs have read it
@@ -894,7 +911,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
           for (int it = 0; it < 2; ++it) {
             uint32_t v[16];
             if (!c.skip) {
-              tmem_ld16(tmem_base + buf * BN + bx * 64 + h * 32 + it * 16 + (static_cast<uint32_t>(q * 32) << 16), v);
+              tmem_ld16(tmem_base + buf * ACC_COLS + bx * 64 + h * 32 + it * 16 + (static_cast<uint32_t>(q * 32) << 16), v);
             } else {
 #pragma unroll
               for (int j = 0; j < 16; ++j) v[j] = 0u;
@@ -924,6 +941,64 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
           ++acc_it;
         }
         continue;
+      } else if constexpr (EPI == 6) {
+        // ---------------- sum and difference: two boxes of 32 rows, the second in the order of the mirror rows
+        const int nb = n0 + half * 64;
+        const uint32_t box_off = stg_off + (warp - 2) * stg_warp_bytes(6);
+        const int r0 = c.mt * BM + q * 32;
+        const bool any = nb < p.N && r0 <= p.m_half;      // uniform across the warp
+        const bool pairs = p.cplx == 5;
+        if (any) {
+          const uint32_t taddr = tmem_base + buf * ACC_COLS + half * 64 + (static_cast<uint32_t>(q * 32) << 16);
+          tma_store_wait_read<0>();
+          __syncwarp();
+          const int ml = pairs ? 30 - lane + 2 * (lane & 1) : 31 - lane;
+          uint8_t* const sum_row = smem + box_off + lane * 128;
+          uint8_t* const dif_row = smem + box_off + 32 * 128 + ml * 128;
+          const uint32_t l7 = static_cast<uint32_t>(lane & 7) << 4, m7 = static_cast<uint32_t>(ml & 7) << 4;
+          const f32x2 minus = f2_keep(-1.f);
+          const f32x2 sign = f2_keep(pairs && (lane & 1) ? -1.f : 1.f);
+#pragma unroll 1
+          for (int it = 0; it < 4; ++it) {
+            uint32_t u[16], v[16];
+            tmem_ld16(taddr + it * 16, u);
+            tmem_ld16(taddr + BN + it * 16, v);
+#pragma unroll
+            for (int gg = 0; gg < 2; ++gg) {
+              const uint32_t g = static_cast<uint32_t>((it * 2 + gg) << 4);
+              f32x2 a[4], d[4];
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const f32x2 x = f2_pack(__uint_as_float(u[gg * 8 + 2 * j]), __uint_as_float(u[gg * 8 + 2 * j + 1]));
+                const f32x2 y = f2_pack(__uint_as_float(v[gg * 8 + 2 * j]), __uint_as_float(v[gg * 8 + 2 * j + 1]));
+                a[j] = f2_add(x, y);
+                d[j] = f2_mul(f2_fma(y, minus, x), sign);
+              }
+              *reinterpret_cast<uint4*>(sum_row + (g ^ l7)) = f2_bf16x8(a);
+              *reinterpret_cast<uint4*>(dif_row + (g ^ m7)) = f2_bf16x8(d);
+            }
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (elect_one()) {
+          if constexpr (CG == 2) mbar_arrive_cluster(leader_tempty0 + 8u * buf);
+          else mbar_arrive(tempty_bar(buf));
+        }
+        ++acc_it;
+        if (any) {
+          fence_async_smem();
+          __syncwarp();
+          // Row 0 has its mirror past the end where that is no row (clipped).  Past m_half the sums are the mirrors of earlier rows'
+          // differences, bit for bit (the tables are symmetric to the bit), so the last box may store both.
+          if (elect_one()) {
+            tma_store_tile(&map_d, smem_base + box_off, nb, 0, r0, c.zlo, c.zhi);
+            const int m0 = p.mirror - r0 - (pairs ? 30 : 31);
+            if (m0 < p.fold_rows) tma_store_tile(&map_d, smem_base + box_off + 32 * 128, nb, 0, m0, c.zlo, c.zhi);
+            tma_store_commit();
+          }
+        }
+        continue;
       } else if constexpr (EPI != 0) {
         // ---------------- specialised bf16 epilogues: registers -> swizzled smem box -> TMA store (full lines, clipped
         // at the matrix edge by the tensor map)
@@ -934,7 +1009,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
         const uint32_t box_off = IN_PLACE ? e_off + ebuf * E_BYTES + bx * (BM * 128) + q * (32 * 128)
                                           : stg_off + (warp - 2) * stg_warp_bytes(EPI) + (EPI == 2 ? 32 * 128 : 0);
         if (nb < p.N) {     // uniform across the warp
-          const uint32_t taddr = tmem_base + buf * BN + bx * 64 + (static_cast<uint32_t>(q * 32) << 16);
+          const uint32_t taddr = tmem_base + buf * ACC_COLS + bx * 64 + (static_cast<uint32_t>(q * 32) << 16);
           // the previous store of this warp must have read its box (the operand box was released after that already)
           if constexpr (!IN_PLACE) {
             tma_store_wait_read<0>();
@@ -1103,7 +1178,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
       for (int cc = half; cc < BN / 32; cc += 2) {
         const int nc = n0 + cc * 32;
         if (nc >= p.N) break;       // uniform across the warp
-        const uint32_t taddr = tmem_base + buf * BN + cc * 32 + (static_cast<uint32_t>(q * 32) << 16);
+        const uint32_t taddr = tmem_base + buf * ACC_COLS + cc * 32 + (static_cast<uint32_t>(q * 32) << 16);
         // rolled: one copy of the (large, many-layout) body serves the four 8-column groups, which keeps the
         // epilogue within the instruction cache
 #pragma unroll 1
@@ -1836,8 +1911,9 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
                         e.rs_lo > 0;
   const bool plain = (one_stride || split_ok) && (e.ndiv <= 0 || e.ndiv >= (1 << 30));
   const int rd = one_stride ? 1 : e.rdiv;
+  const bool folded = p.cplx == 4 || p.cplx == 5;
   auto tile_map = [&](CUtensorMap* m, const void* ptr, int box_rows) {
-    return make_map_e(m, ptr, p.M, p.N, rd, e.rs_hi, e.rs_lo, e.d_zlo, e.d_zhi, p.zlo_n, p.zhi_n, box_rows, 2, e.d_half);
+    return make_map_e(m, ptr, folded ? p.rows : p.M, p.N, rd, e.rs_hi, e.rs_lo, e.d_zlo, e.d_zhi, p.zlo_n, p.zhi_n, box_rows, 2, e.d_half);
   };
   kp.rd_shift = 0;
   while (plain && (1 << kp.rd_shift) < rd) ++kp.rd_shift;
@@ -1853,7 +1929,8 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
   memset(&mdx, 0, sizeof(mdx));
   if (eb == 2 && !e.out_f32 && kp.vec_ok && !e.accumulate && plain && e.d_zlo >= 0 && e.d_zhi >= 0 &&
       (kp.bias_mode != 2 || (p.N % 8 == 0 && (reinterpret_cast<uintptr_t>(e.bias) & 15) == 0 && (kp.bias_zs % 4) == 0))) {
-    if (!e.resid && !e.preact && (e.act == 0 || e.act == 1 || e.act == 3 || e.act == 5)) epi = 1;
+    if (folded) epi = !e.resid && !e.preact && e.act == 0 && !e.bias && e.alpha == 1.f && kp.ndx == 0 ? 6 : 0;
+    else if (!e.resid && !e.preact && (e.act == 0 || e.act == 1 || e.act == 3 || e.act == 5)) epi = 1;
     else if (!e.resid && e.preact && e.act == 1) epi = 2;
     else if (e.resid && kp.e_tma && !e.preact && e.act == 0) epi = 3;
     else if (e.resid && kp.e_tma && !e.preact && (e.act == 2 || e.act == 4 || e.act == 6 || e.act == 8)) epi = 4;
@@ -1895,7 +1972,7 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
   }();
   const bool no_peer = (peer == nullptr) || (peer->nseg <= 1 && peer->ndx == 0 && peer->nwait == 0 && peer->nsig == 0 &&
                                               peer->done_ctr == nullptr);
-  const bool eligible = eb == 2 && no_peer && p.M > BM && p.rmin_a == 0 && p.rmax_a == 0 && (p.cplx == 0 || p.cplx == 3);
+  const bool eligible = eb == 2 && no_peer && p.M > BM && p.rmin_a == 0 && p.rmax_a == 0 && (p.cplx == 0 || p.cplx >= 3);
   const int pad1 = (p.M + BM - 1) / BM * BM, pad2 = (p.M + 2 * BM - 1) / (2 * BM) * (2 * BM);
   const long long z_all = static_cast<long long>(p.zlo_n) * p.zhi_n;
   const bool waves = pad1 / BM * ((p.N + 255) / 256) * z_all >= 2 * sm_count();
@@ -1903,14 +1980,26 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
   const int cg = (eligible && (pairs_mode == 1 || (pairs_mode == 2 && pays))) ? 2 : 1;
   if (bn == 0) bn = pick_bn(p.N, epi, kp.e_tma);
   if ((eb == 4 && bn == 192) || ((epi == 3 || epi == 4 || kp.e_tma) && bn == 256)) bn = 128;
-  if (epi == 0 && kp.e_tma) bn = 128;
+  if ((epi == 0 && kp.e_tma) || epi == 6) bn = 128;
   kp.m_tiles = (p.M + BM * cg - 1) / (BM * cg);
   kp.n_tiles = (p.N + bn - 1) / bn;
   kp.cplx = p.cplx;
   kp.nth = kp.n_tiles;
   kp.neg_half = p.cplx == 1 ? 0 : 1;
   kp.neg_seg = p.cplx == 2 ? 0 : 1;
-  if (p.cplx) {
+  kp.a_part = p.K;
+  if (folded) {
+    // (from 64 rows on the mirror rows' boxes start at or after row 0, and the last box of sums ends inside the table)
+    if (epi != 6 || kp.splits != 1 || p.splits == 0 || kp.nseg != 1 || rd != 1 || A.mn_major || p.mirror < 64 || (p.a_plane % 8) != 0 ||
+        p.M > p.mirror / 2 + 2 || p.rows < p.mirror / 2 + 32 || p.zlo_n != 1) {
+      snprintf(g_err, sizeof(g_err), "folded product: bf16, K-major tables, plain aligned rows, at least 64 of them");
+      return cudaErrorInvalidValue;
+    }
+    kp.a_part = static_cast<int>(p.a_plane);
+    kp.mirror = p.mirror;
+    kp.m_half = p.mirror / 2;
+    kp.fold_rows = p.rows;
+  } else if (p.cplx) {
     if (eb != 2 || (epi != 1 && epi != 3 && epi != 5) || kp.splits != 1 || p.splits == 0 || kp.nseg != 1 || rd != 1) {
       snprintf(g_err, sizeof(g_err), "complex product: bf16 operands, plain rows, aligned output with or without residual");
       return cudaErrorInvalidValue;
@@ -1957,7 +2046,8 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
   GemmOperand Am = A, Bm = B;
   if (p.cplx) Bm.zs_lo = p.b_plane;
   if (p.cplx == 3) Am.zs_lo = p.a_plane;
-  if (!make_map(&ma, Am, p.cplx && p.cplx != 3 ? 2 * p.K : p.K, eb, p.cplx == 3 ? 2 : p.zlo_n, p.zhi_n, BM)) return cudaErrorInvalidValue;
+  const int ka = folded ? kp.a_part + p.K : (p.cplx && p.cplx != 3 ? 2 * p.K : p.K);
+  if (!make_map(&ma, Am, ka, eb, p.cplx == 3 ? 2 : p.zlo_n, p.zhi_n, BM)) return cudaErrorInvalidValue;
   const int bn_box = bn / cg;     // rows of a K-major B one CTA loads per stage
   BMaps mbs;
   if (kp.nseg > 1) {
@@ -1976,6 +2066,8 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
   if (epi == 0) md = ma;       // unused maps must be valid descriptors all the same
   if (epi != 2) mp = ma;
   for (int q = (epi == 1 ? kp.ndx : 0); q < MAX_SEG - 1; ++q) mdx.m[q] = ma;
+  if (epi == 6)
+    return cg == 2 ? launch_t<128, 2, 6, 2>(ma, mbs, me, md, mp, mdx, kp, stream) : launch_t<128, 2, 6, 1>(ma, mbs, me, md, mp, mdx, kp, stream);
   if (eb == 4) {
     if (bn == 256) return launch_t<256, 4, 0, 1>(ma, mbs, me, md, mp, mdx, kp, stream);
     return launch_t<128, 4, 0, 1>(ma, mbs, me, md, mp, mdx, kp, stream);

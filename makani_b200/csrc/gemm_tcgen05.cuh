@@ -65,7 +65,10 @@ struct GemmProblem {
   // Complex products of planar operands (0: none; modes in gemm_tcgen05.cu): N and K are those of one part; `b_plane` (and for
   // mode 3 `a_plane`) elements between the real and imaginary planes; for modes 1 and 2 the parts of A follow one another in k
   int cplx = 0;
+  // Folded transforms (modes 4, 5): M rows are computed, `rows` stored (row r and row mirror - r); A has `rows` rows, its second part
+  // starts at k = a_plane
   long long a_plane = 0, b_plane = 0;
+  int rows = 0, mirror = 0;
   int bn;               // tile width: 128, 192 or 256 (0 = choose)
 };
 

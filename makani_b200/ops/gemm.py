@@ -292,6 +292,35 @@ def gemm_complex(mode: int, M: int, N: int, K: int, A: Operand, B: Operand, D: O
     _ext.require().gemm_complex(A.tensor, B.tensor, D.tensor, resid, ip)
 
 
+def gemm_fold(rows: int, M: int, N: int, K: int, mirror: int, pairs: bool, table: torch.Tensor, part: int, B: Operand, b_plane: int,
+              D: Output, *, zhi_n: int = 1) -> None:
+    """Product with a table whose rows r and mirror - r differ only in the sign of one half of their columns (bf16 on CUDA):
+
+        P(s)[r, n] = sum_k table[r, s part + k] B(s)[n, k],   s = 0, 1, r < M
+        D[r] = P(0)[r] + P(1)[r],   D[mirror - r] = P(0)[r] - P(1)[r],   both where they are one of the `rows` rows of D
+
+    With `pairs` the rows are (order, re / im) pairs: row 2 m + ri has its mirror at mirror - 2 m + ri, and the imaginary one its
+    sign changed.  `M` rows cover one half and its middle.  `b_plane`: elements between the two planes of B; z_hi batches B and D."""
+    if not B.tensor.is_cuda:
+        fb, fd = _flat(B.tensor), _flat(D.tensor)
+        cdt = torch.float64 if fb.dtype == torch.float64 else torch.float32
+        rs, ks = (1, B.ld) if B.mn_major else (B.ld, 1)
+        acc = [torch.matmul(table[:M, s * part: s * part + K].to(cdt),
+                            fb[B.offset + s * b_plane:].as_strided((zhi_n, K, N), (B.zs_hi, ks, rs)).to(cdt)) for s in range(2)]
+        r = torch.arange(M)
+        sign = torch.where((r % 2 == 1) & pairs, -1.0, 1.0).to(cdt).view(1, -1, 1)
+        z = torch.arange(zhi_n).view(-1, 1, 1)
+        n = torch.arange(N).view(1, 1, -1)
+        for row, val in ((r, acc[0] + acc[1]), (mirror - r + (2 * (r % 2) if pairs else 0), (acc[0] - acc[1]) * sign)):
+            keep = (row >= 0) & (row < rows)
+            idx = D.offset + z * D.d_zhi + row[keep].view(1, -1, 1) * D.rs_lo + n
+            fd.index_put_((idx.reshape(-1),), val[:, keep].to(fd.dtype).reshape(-1))
+        return
+    ip = [5 if pairs else 4, rows, M, N, K, mirror, zhi_n, table.shape[1], part,
+          B.offset, int(B.mn_major), B.ld, B.zs_hi, b_plane, D.offset, D.rs_lo, D.d_zhi]
+    _ext.require().gemm_fold(table, B.tensor, D.tensor, ip)
+
+
 def _f32_bits(x: float) -> int:
     import struct
     return struct.unpack("<I", struct.pack("<f", float(x)))[0]

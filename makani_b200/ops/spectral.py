@@ -8,10 +8,11 @@ truncation pass ever touches HBM:
 
     x  [B, H, W, C]                  real grid data, channels-last (bf16)
     S1 longitude DFT      -> T1 [B, H, (m,ri), C]       A = DFT matrix [(m,ri), W], batched over latitude rows
+                                                        (folded: orders m and W / 2 - m share their products)
     S2 Legendre analysis  -> T2 [B, l, m, (ri, C)]      A = P_l^m(theta_k) w_k, batched over m, rows l < m skipped
     S3 complex contraction-> T3 [B, m, l, (ri, Co)]     B = real and imaginary planes of W_l, batched over l, rows m > l skipped
     S4 Legendre synthesis -> T4 [B, H', (m,ri), Co]     k-loop restricted to l >= m
-    S5 inverse DFT        -> y  [B, H', W', Co]
+    S5 inverse DFT        -> y  [B, H', W', Co]         (folded: longitudes i and W' - i share their products)
 
 (ri = real/imaginary part; the Legendre tables are padded along latitude to 16-byte TMA strides.)
 The adjoints used by the backward pass are the same five launches with the constant operands read in the
@@ -31,7 +32,7 @@ from ..sht.legendre import legendre_table
 from ..sht.quadrature import precompute_latitudes
 from . import _ext
 from .conv import records_grad
-from .gemm import Operand, Output, Tri, gemm, gemm_complex, pad_to
+from .gemm import Operand, Output, Tri, gemm, gemm_complex, gemm_fold, pad_to
 
 
 class SHTPlan:
@@ -42,9 +43,10 @@ class SHTPlan:
     def __init__(self, nlat: int, nlon: int, lmax: int, mmax: int, grid: str, device, dtype=torch.bfloat16):
         self.nlat, self.nlon, self.lmax, self.mmax, self.grid = nlat, nlon, lmax, mmax, grid
         self.device, self.dtype = torch.device(device), dtype
-        self.hp = pad_to(nlat, 8)          # padded latitude extent of T1/T4 rows and of the tables
+# rows of the tables start on 128-byte boundaries: a 128-byte row of a TMA box is then one line, not two
+        self.hp = pad_to(nlat, 64)         # padded latitude extent of the Legendre tables
         self.k2 = 2 * mmax                 # DFT K extent (m, ri)
-        self.k2p = pad_to(self.k2, 8)
+        self.k2p = pad_to(self.k2, 64)
         theta, wq = precompute_latitudes(nlat, grid)
         self.theta, self.wq = theta, wq
         p = legendre_table(mmax, lmax, theta)                     # [m, l, k] float64
@@ -71,6 +73,53 @@ class SHTPlan:
         g[:, 0:self.k2:2] = (cm * np.cos(ang)).T
         g[:, 1:self.k2:2] = (-cm * np.sin(ang)).T
         self.gt = torch.from_numpy(g.astype(np.float32)).to(self.device, dtype).contiguous()     # [W, (m,ri) padded]
+
+        # The same matrices with their columns in two halves, for `gemm_fold`: (synthesis, forward) -> table.  The synthesis (rows are
+        # longitudes) folds from the 64 rows on that `gemm_fold` asks for.  The analysis (rows (m, ri)) only saves work where most
+        # orders up to half the points are kept, order m sharing its products with order W / 2 - m.  us, whole / folded:
+        #   synthesis, 384 channels: 721 x 1440, 241 orders 430 / 336; 240 x 480, 241 60 / 49; 360 x 720, 361 157 / 132;
+        #   180 x 360, 181 33 / 28;  200 channels: 181 x 360, 120 18.8 / 18.5;  64 channels, 2 x 64 x 128, 65 12.0 / 9.9
+        #   analysis: 240 x 480, 241 58 / 47; 360 x 720, 361 155 / 131, 241 of them 111 / 121; 181 x 360, 120 20.5 / 18.5 (adjoint
+        #   16.4 / 18.5); 100 x 200, 81 11.8 / 10.0
+        self.folds_synthesis = nlon >= 64
+        self.folds_analysis = nlon >= 64 and nlon % 2 == 0 and 8 * mmax > 3 * nlon and 2 * mmax >= nlon // 2 + 32
+        self._folded = {(syn, fwd): self._fold_table(syn, fwd) for fwd in (True, False) for syn in (True, False)
+                        if (self.folds_synthesis if syn else self.folds_analysis)}
+
+    def _fold_table(self, synthesis: bool, forward: bool) -> torch.Tensor:
+        """The inverse transform's matrix (`synthesis`; rows are longitudes, halves the cosine and sine terms) or the forward one's
+        (rows (m, ri), halves the even and odd points), from the coefficients of the forward transform (`forward`) or of the
+        inverse one.  Symmetric to the bit: a row and its mirror hold the same numbers, and those that cancel are zero.  The halves
+        start on 128-byte boundaries, so that a TMA row is one line (721 x 1440: 364 -> 336 us)."""
+        W, mmax = self.nlon, self.mmax
+        ang = 2.0 * np.pi * ((np.arange(mmax)[:, None] * np.arange(W)[None, :]) % W) / W
+        scale = np.full((mmax, 1), 2.0 * np.pi / W if forward else 2.0)
+        if not forward:
+            scale[0] = 1.0
+            if W % 2 == 0 and mmax > W // 2:
+                scale[W // 2] = 1.0
+        c, s = scale * np.cos(ang), -scale * np.sin(ang)              # [m, i]
+        h = W // 2
+        if synthesis:
+            i = np.arange(h + 1, W)
+            c[:, i], s[:, i] = c[:, W - i], -s[:, W - i]
+            s[:, 0] = 0.0
+            if W % 2 == 0:
+                s[:, h] = 0.0
+            t = np.zeros((W, 2, pad_to(mmax, 64)), dtype=np.float32)
+            t[:, 0, :mmax], t[:, 1, :mmax] = c.T, s.T
+        else:
+            if h % 2 == 0 and h // 2 < mmax:
+                c[h // 2, 1::2] = 0.0
+                s[h // 2, 0::2] = 0.0
+            m = np.arange(h // 2 + 1, mmax)
+            sign = np.where(np.arange(W) % 2 == 0, 1.0, -1.0)[None, :]
+            c[m], s[m] = sign * c[h - m], -sign * s[h - m]
+            t = np.zeros((mmax, 2, 2, pad_to(h, 64)), dtype=np.float32)                  # [m, ri, half, point]
+            for ri, x in enumerate((c, s)):
+                t[:, ri, 0, :h], t[:, ri, 1, :h] = x[:, 0::2], x[:, 1::2]
+        t = t.reshape(-1, 2 * t.shape[-1])
+        return torch.from_numpy(t).to(self.device, self.dtype).contiguous()
 
     @classmethod
     def get(cls, nlat, nlon, lmax, mmax, grid, device, dtype=torch.bfloat16) -> "SHTPlan":
@@ -115,6 +164,31 @@ def dft_synthesis(t4: torch.Tensor, mat: torch.Tensor, mat_mn: bool, mat_ld: int
          Operand(t4, ld=C, mn_major=True, zs_lo=k2 * C, zs_hi=H * k2 * C),
          Output(y, rs_lo=C, d_zlo=W * C, d_zhi=H * W * C),
          zlo_n=H, zhi_n=B)
+    return y
+
+
+def analyse(x: torch.Tensor, plan: SHTPlan, forward: bool = True) -> torch.Tensor:
+    """Longitude DFT of x (`forward`), or the adjoint of the inverse one: [B, H, (m, ri), C]."""
+    if not plan.folds_analysis:
+        return dft_analysis(x, plan.f, False, plan.nlon, plan.k2) if forward else dft_analysis(x, plan.gt, True, plan.k2p, plan.k2)
+    B, C, H, W = x.shape
+    k2, table = plan.k2, plan._folded[False, forward]
+    t1 = torch.empty(B, H, k2, C, dtype=x.dtype, device=x.device)
+    gemm_fold(k2, 2 * (W // 4 + 1), C, W // 2, W, True, table, table.shape[1] // 2,
+              Operand(x, ld=2 * C, mn_major=True, zs_hi=W * C), C, Output(t1, rs_lo=C, d_zhi=k2 * C), zhi_n=B * H)
+    return t1
+
+
+def synthesise(t4: torch.Tensor, plan: SHTPlan, forward: bool = False) -> torch.Tensor:
+    """Inverse longitude DFT of t4 [B, H, (m, ri), C], or the adjoint of the forward one (`forward`); channels-last."""
+    W = plan.nlon
+    if not plan.folds_synthesis:
+        return dft_synthesis(t4, plan.f, True, W, W) if forward else dft_synthesis(t4, plan.gt, False, plan.k2p, W)
+    B, H, k2, C = t4.shape
+    table = plan._folded[True, forward]
+    y = torch.empty(B, C, H, W, dtype=t4.dtype, device=t4.device, memory_format=torch.channels_last)
+    gemm_fold(W, W // 2 + 1, C, plan.mmax, W, False, table, table.shape[1] // 2,
+              Operand(t4, ld=2 * C, mn_major=True, zs_hi=k2 * C), C, Output(y, rs_lo=C, d_zhi=W * C), zhi_n=B * H)
     return y
 
 
@@ -311,18 +385,18 @@ class _SpectralConv(torch.autograd.Function):
     def forward(ctx, x, w, plan_in: SHTPlan, plan_out: SHTPlan, want_resid: bool, train: bool):
         x = _to_cl(x)
         wx = weight_planes(w, x.dtype, keep=not train, share=train)
-        t1 = dft_analysis(x, plan_in.f, False, plan_in.nlon, plan_in.k2)
+        t1 = analyse(x, plan_in)
         t2 = legendre_analysis(t1, plan_in.pw)
         del t1
         t3 = contract(t2, wx, False)
         t4 = legendre_synthesis(t3, False, plan_out.p, plan_out.nlat)
         del t3
-        y = dft_synthesis(t4, plan_out.gt, False, plan_out.k2p, plan_out.nlon)
+        y = synthesise(t4, plan_out)
         del t4
         r = None
         if want_resid:
             t4r = legendre_synthesis(t2, True, plan_out.p, plan_out.nlat)
-            r = dft_synthesis(t4r, plan_out.gt, False, plan_out.k2p, plan_out.nlon)
+            r = synthesise(t4r, plan_out)
         ctx.save_for_backward(t2, wx)
         ctx.plans = (plan_in, plan_out)
         ctx.want_resid = want_resid
@@ -337,7 +411,7 @@ class _SpectralConv(torch.autograd.Function):
         plan_in, plan_out = ctx.plans
         dy = _to_cl(dy)
         # adjoint of the inverse DFT / synthesis on the output grid
-        dt4 = dft_analysis(dy, plan_out.gt, True, plan_out.k2p, plan_out.k2)
+        dt4 = analyse(dy, plan_out, forward=False)
         dt3 = legendre_analysis(dt4, plan_out.p)                       # [B, l, m, (ri, o)]
         del dt4
         dw = None
@@ -348,13 +422,13 @@ class _SpectralConv(torch.autograd.Function):
             dr2 = None
             if ctx.want_resid and dr is not None:
                 # laid out by order, as the contraction writes: its epilogue adds the residual's share
-                dr4 = dft_analysis(_to_cl(dr), plan_out.gt, True, plan_out.k2p, plan_out.k2)
+                dr4 = analyse(_to_cl(dr), plan_out, forward=False)
                 dr2 = legendre_analysis(dr4, plan_out.p, by_order=True)
                 del dr4
             dt2 = contract(dt3, wx, True, resid=dr2)                   # [B, m, l, (ri, c)]
             del dr2
             dt1 = legendre_synthesis(dt2, False, plan_in.pw, plan_in.nlat)
-            dx = dft_synthesis(dt1, plan_in.f, True, plan_in.nlon, plan_in.nlon)
+            dx = synthesise(dt1, plan_in, forward=True)
         return dx, dw, None, None, None, None
 
 

@@ -655,3 +655,32 @@ def test_row_sums_beside_the_weight_gradient(m, n, k, zlo, zhi, groups):
     assert ((sums.double() - ref).abs() <= steps * 2.0 ** -24 * ref).all()
     # the gradient itself: the same chains, added up in another order
     assert (d - plain).norm() <= 1e-6 * plain.norm() + 1e-12
+
+
+@pytest.mark.parametrize("b,h,w,mmax,c", [
+    (1, 2, 64, 33, 8),          # half a tile of rows, one vector of channels, the mirror boxes at row 1
+    (2, 3, 72, 36, 136),        # the Nyquist order left out, a ragged second column tile
+    (1, 5, 90, 46, 64),         # an odd number of pairs of points
+    (1, 4, 65, 20, 16),         # an odd number of longitudes
+    (1, 3, 248, 125, 200),      # rows past the middle in the last box
+    (1, 80, 480, 241, 384),     # pairs of CTAs, several tiles per pair
+    (1, 7, 1440, 241, 72),      # few of the orders: the analysis stays whole
+])
+def test_folded_transforms(b, h, w, mmax, c):
+    from makani_b200.ops.spectral import SHTPlan, analyse, synthesise
+    dev = _dev()
+    plan = SHTPlan(h, w, h, mmax, "legendre-gauss", dev)
+    g = torch.Generator(dev).manual_seed(w)
+    t4 = torch.randn(b, h, 2 * mmax, c, device=dev, generator=g).to(torch.bfloat16)
+    td, f, gt = t4.double(), plan.f.double(), plan.gt[:, :plan.k2].double()
+    pairs = [(synthesise(t4, plan).permute(0, 2, 3, 1), gt @ td), (synthesise(t4, plan, forward=True).permute(0, 2, 3, 1), f.t() @ td)]
+    assert torch.equal(synthesise(t4, plan), synthesise(t4, plan))      # rows written twice are written with the same bits
+    if w % 8 == 0:
+        x = torch.randn(b, h, w, c, device=dev, generator=g).to(torch.bfloat16).permute(0, 3, 1, 2)
+        xd = x.permute(0, 2, 3, 1).double()
+        pairs += [(analyse(x, plan), f @ xd), (analyse(x, plan, forward=False), gt.t() @ xd)]
+        assert torch.equal(analyse(x, plan), analyse(x, plan))
+    # bf16 outputs; the whole matrices round the same angles to bf16, a few entries to the other neighbour
+    for got, ref in pairs:
+        assert got.shape == ref.shape and _rel(got, ref) < BF16
+    _ext.check_device_errors(dev)

@@ -208,3 +208,34 @@ def test_planar_spectral_products_emulated(b, l, m, co, ci):
         got = contract_wgrad2(dt * keep, t2 * keep, l0, m0)
         ref = torch.einsum("blmo,blmc->loc", cplx(dt * keep), cplx(t2 * keep).conj())
         torch.testing.assert_close(got, torch.stack([ref.real, ref.imag]), atol=1e-5, rtol=1e-5)
+
+
+@pytest.mark.parametrize("h,w,mmax,analysis", [(3, 64, 33, True), (3, 64, 32, True), (2, 65, 33, False), (2, 72, 37, True), (2, 80, 41, True),
+                                               (2, 90, 46, True), (2, 100, 40, False), (2, 100, 41, True), (2, 96, 49, True),
+                                               (3, 128, 20, False), (2, 62, 32, False)])
+def test_folded_transforms_equal_the_whole_ones(h, w, mmax, analysis):
+    """Every plan the rule folds (odd and even halves, all orders or some, the Nyquist order kept or not) against the whole
+    matrices; few points, an odd number of them or few orders stay whole."""
+    from makani_b200.ops.spectral import SHTPlan, analyse, dft_analysis, dft_synthesis, synthesise
+    plan = SHTPlan(h, w, h, mmax, "legendre-gauss", "cpu", torch.float64)
+    assert plan.folds_synthesis == (w >= 64) and plan.folds_analysis == analysis
+    g = torch.Generator().manual_seed(w)
+    x = torch.randn(2, h, w, 8, generator=g, dtype=torch.float64).permute(0, 3, 1, 2)
+    t4 = torch.randn(2, h, 2 * mmax, 8, generator=g, dtype=torch.float64)
+    pairs = [(analyse(x, plan), dft_analysis(x, plan.f, False, w, plan.k2)),
+             (analyse(x, plan, forward=False), dft_analysis(x, plan.gt, True, plan.k2p, plan.k2)),
+             (synthesise(t4, plan), dft_synthesis(t4, plan.gt, False, plan.k2p, w)),
+             (synthesise(t4, plan, forward=True), dft_synthesis(t4, plan.f, True, w, w))]
+    for got, ref in pairs:      # the tables are fp32 numbers of the same angles
+        assert got.shape == ref.shape and (got - ref).abs().max() <= 1e-6 * ref.abs().max()
+    # rows that mirror each other hold the same numbers
+    for (syn, _), table in plan._folded.items():
+        a, b = table.reshape(table.shape[0], 2, -1).unbind(1)
+        if syn:
+            assert torch.equal(a[1:], a[1:].flip(0)) and torch.equal(b[1:], -b[1:].flip(0))
+        else:
+            r = torch.arange(2 * mmax)
+            mirror = w - r + 2 * (r % 2)
+            ok = mirror < 2 * mmax
+            sign = (1.0 - 2.0 * (r[ok] % 2))[:, None]
+            assert torch.equal(a[mirror[ok]], sign * a[ok]) and torch.equal(b[mirror[ok]], -sign * b[ok])
