@@ -1,14 +1,10 @@
 // Python bindings (pybind11 / torch tensors) for the sm_100a kernels. Every entry validates device, dtype
 // and contiguity, launches on the current CUDA stream and raises on a launch error.
-#include <torch/extension.h>
-#include <ATen/cuda/CUDAContext.h>
-#include <c10/cuda/CUDAGuard.h>
-
 #include <algorithm>
-#include <cstdint>
 #include <cstring>
 #include <map>
-#include <vector>
+
+#include "host.h"
 
 #include "fused_ops.cuh"
 #include "gelu.cuh"
@@ -20,7 +16,8 @@ namespace {
 
 using torch::Tensor;
 
-#define MK_CHECK(cond, ...) TORCH_CHECK(cond, "makani_b200: ", __VA_ARGS__)
+void gemm_complex(const Tensor& a, const Tensor& b, Tensor& d, const c10::optional<Tensor>& resid, const std::vector<int64_t>& ip);
+void gemm_fold(const Tensor& a, const Tensor& b, Tensor& d, const std::vector<int64_t>& ip);
 
 inline void check_cuda(cudaError_t e, const char* what) {
   TORCH_CHECK(e == cudaSuccess, "makani_b200: ", what, " failed: ", cudaGetErrorString(e), " ", mk::gemm_last_error());
@@ -76,7 +73,6 @@ std::pair<int64_t, int64_t> stream_state(int64_t device) {
 
 inline const char* base_ptr(const Tensor& t) { return static_cast<const char*>(t.data_ptr()); }
 
-// iparams layout: see makani_b200/ops/gemm.py
 static bool parse_peer(mk::GemmPeer& g, const std::vector<int64_t>& seg, const std::vector<int64_t>& sync) {
   memset(&g, 0, sizeof(g));
   if (!seg.empty()) {
@@ -129,50 +125,64 @@ static void check_extent(const Tensor& t, int64_t off, std::initializer_list<std
            "..", hi + before, " of ", total, ")");
 }
 
-void gemm_impl(const Tensor& a, const Tensor& b, Tensor& d, const c10::optional<Tensor>& bias,
-               const c10::optional<Tensor>& resid, const c10::optional<Tensor>& preact, const std::vector<int64_t>& ip,
-               double alpha, const mk::GemmPeer* peer, mk::GemmRowSums* rows = nullptr);
+inline const Tensor* defined(const c10::optional<Tensor>& t) { return t.has_value() && t->defined() ? &*t : nullptr; }
+
+// iparams layout: see makani_b200/ops/gemm.py
+mkh::Gemm parse_gemm(const Tensor& a, const Tensor& b, Tensor& d, const c10::optional<Tensor>& bias, const c10::optional<Tensor>& resid,
+                     c10::optional<Tensor>& preact, const std::vector<int64_t>& ip, double alpha) {
+  MK_CHECK(ip.size() == 40, "gemm: expected 40 integer parameters, got ", ip.size());
+  mkh::Gemm g;
+  int k = 0;
+  g.M = ip[k++]; g.N = ip[k++]; g.K = ip[k++];
+  g.zlo_n = ip[k++]; g.zhi_n = ip[k++]; g.splits = ip[k++]; g.bn = ip[k++];
+  for (int64_t* t : {&g.tri.rmin_a, &g.tri.rmin_b, &g.tri.rmax_a, &g.tri.rmax_b, &g.tri.kmin_a, &g.tri.kmin_b, &g.tri.kmax_a, &g.tri.kmax_b})
+    *t = ip[k++];
+  for (auto* o : {&g.A, &g.B}) {
+    o->offset = ip[k++]; o->mn_major = ip[k++] != 0; o->ld = ip[k++]; o->zs_lo = ip[k++]; o->zs_hi = ip[k++];
+  }
+  g.A.t = &a;
+  g.B.t = &b;
+  g.D.t = &d;
+  g.D.offset = ip[k++];
+  g.accumulate = ip[k++] != 0;
+  g.D.d_zlo = ip[k++]; g.D.d_zhi = ip[k++]; g.D.rdiv = ip[k++]; g.D.rs_hi = ip[k++]; g.D.rs_lo = ip[k++]; g.D.ndiv = ip[k++];
+  g.D.ns_hi = ip[k++];
+  g.alpha = alpha;
+  g.bias = defined(bias);
+  g.bias_mode = static_cast<int>(ip[k++]);
+  const int64_t actw = ip[k++];     // low byte: activation code; bit 8: the second output holds the derivative
+  g.act = static_cast<int>(actw & 0xff);
+  g.preact_deriv = ((actw >> 8) & 1) != 0;
+  g.resid = defined(resid);
+  g.resid_offset = ip[k++];
+  g.preact = preact.has_value() && preact->defined() ? &*preact : nullptr;
+  g.preact_offset = ip[k++];
+  const uint32_t bits = static_cast<uint32_t>(ip[k++]);      // bit pattern of the activation parameter (fp32)
+  memcpy(&g.act_param, &bits, sizeof(g.act_param));
+  g.bias_zs = ip[k++];
+  return g;
+}
 
 void gemm(const Tensor& a, const Tensor& b, Tensor& d, const c10::optional<Tensor>& bias,
-          const c10::optional<Tensor>& resid, const c10::optional<Tensor>& preact, const std::vector<int64_t>& ip,
+          const c10::optional<Tensor>& resid, c10::optional<Tensor> preact, const std::vector<int64_t>& ip,
           double alpha) {
-  gemm_impl(a, b, d, bias, resid, preact, ip, alpha, nullptr);
+  mkh::run(parse_gemm(a, b, d, bias, resid, preact, ip, alpha));
 }
 
 // Weight gradient with the sums of the rows of A beside it; false: the launch had no place for them, `sums` is untouched
 bool gemm_row_sums(const Tensor& a, const Tensor& b, Tensor& d, Tensor& sums, const std::vector<int64_t>& ip, double alpha) {
-  MK_CHECK(ip.size() == 40, "gemm: expected 40 integer parameters, got ", ip.size());
-  const int64_t groups = ip[27] != 0 ? ip[3] : 1;      // z_lo batches with outputs of their own
-  MK_CHECK(sums.is_cuda() && sums.scalar_type() == torch::kFloat32 && sums.is_contiguous() && sums.numel() == groups * ip[0] &&
-               sums.get_device() == a.get_device(),
-           "gemm: row sums must be contiguous fp32 CUDA of the rows of A");
-  Tensor part;      // freed to the allocator on return: later work of this stream only
-  struct Ctx {
-    Tensor* part;
-    const Tensor* like;
-  } ctx{&part, &sums};
-  mk::GemmRowSums rows;
-  rows.out = sums.data_ptr<float>();
-  rows.ctx = &ctx;
-  rows.scratch = [](void* c, long long floats) -> float* {
-    Ctx& x = *static_cast<Ctx*>(c);
-    try {
-      *x.part = torch::empty({floats}, x.like->options());
-    } catch (const std::exception&) {
-      return nullptr;
-    }
-    return x.part->data_ptr<float>();
-  };
-  rows.done = 0;
-  gemm_impl(a, b, d, c10::nullopt, c10::nullopt, c10::nullopt, ip, alpha, nullptr, &rows);
-  return rows.done != 0;
+  c10::optional<Tensor> none;
+  mkh::Gemm g = parse_gemm(a, b, d, none, none, none, ip, alpha);
+  g.row_sums = &sums;
+  return mkh::run(g);
 }
 
 // GEMM whose B operand is gathered from peer devices along k and/or that takes part in cross-device handshakes
 void gemm_peer(const Tensor& a, const Tensor& b, Tensor& d, const c10::optional<Tensor>& bias,
-               const c10::optional<Tensor>& resid, const c10::optional<Tensor>& preact, const std::vector<int64_t>& ip,
+               const c10::optional<Tensor>& resid, c10::optional<Tensor> preact, const std::vector<int64_t>& ip,
                double alpha, const std::vector<int64_t>& seg, const std::vector<int64_t>& sync,
                const std::vector<int64_t>& dests) {
+  MK_CHECK(ip.size() == 40, "gemm: expected 40 integer parameters, got ", ip.size());
   mk::GemmPeer g;
   parse_peer(g, seg, sync);
   MK_CHECK(dests.size() <= 7, "gemm_peer: at most 7 additional destinations");
@@ -180,7 +190,7 @@ void gemm_peer(const Tensor& a, const Tensor& b, Tensor& d, const c10::optional<
   const int64_t d_off = ip[25];
   const int64_t osz = d.element_size();
   for (size_t q = 0; q < dests.size(); ++q) g.Dx[q] = reinterpret_cast<char*>(dests[q]) + d_off * osz;
-  gemm_impl(a, b, d, bias, resid, preact, ip, alpha, &g);
+  mkh::run(parse_gemm(a, b, d, bias, resid, preact, ip, alpha), &g);
 }
 
 // out (bf16, contiguous in memory) = sum of the segments at `srcs` (+ bias over the innermost `C` channels)
@@ -216,85 +226,122 @@ void peer_publish(const Tensor& src, int64_t rows, int64_t row_bytes, int64_t sr
              "peer_publish");
 }
 
-void gemm_impl(const Tensor& a, const Tensor& b, Tensor& d, const c10::optional<Tensor>& bias,
-               const c10::optional<Tensor>& resid, const c10::optional<Tensor>& preact, const std::vector<int64_t>& ip,
-               double alpha, const mk::GemmPeer* peer, mk::GemmRowSums* rows) {
-  MK_CHECK(ip.size() == 40, "gemm: expected 40 integer parameters, got ", ip.size());
+}  // namespace
+
+namespace mkh {
+
+int64_t& launches() {
+  static thread_local int64_t n = 0;
+  return n;
+}
+
+void check(cudaError_t e, const char* what) { check_cuda(e, what); }
+
+bool run(const Gemm& g, const mk::GemmPeer* peer) {
+  const Tensor &a = *g.A.t, &b = *g.B.t, &d = *g.D.t;
   MK_CHECK(a.is_cuda() && b.is_cuda() && d.is_cuda(), "gemm: tensors must be CUDA");
   MK_CHECK(a.scalar_type() == b.scalar_type(), "gemm: A and B dtypes differ");
   const int eb = static_cast<int>(a.element_size());
   MK_CHECK((a.scalar_type() == torch::kBFloat16) || (a.scalar_type() == torch::kFloat32), "gemm: operands must be bf16 or fp32");
   MK_CHECK((d.scalar_type() == torch::kBFloat16) || (d.scalar_type() == torch::kFloat32), "gemm: output must be bf16 or fp32");
   c10::cuda::CUDAGuard guard(a.device());
-  int k = 0;
   mk::GemmProblem p;
-  p.M = ip[k++]; p.N = ip[k++]; p.K = ip[k++];
-  p.zlo_n = ip[k++]; p.zhi_n = ip[k++];
+  p.M = g.M; p.N = g.N; p.K = g.K;
+  p.zlo_n = g.zlo_n; p.zhi_n = g.zhi_n;
   p.elem_bytes = eb;
-  p.splits = ip[k++]; p.bn = ip[k++];
-  p.rmin_a = ip[k++]; p.rmin_b = ip[k++]; p.rmax_a = ip[k++]; p.rmax_b = ip[k++];
-  p.kmin_a = ip[k++]; p.kmin_b = ip[k++]; p.kmax_a = ip[k++]; p.kmax_b = ip[k++];
+  p.splits = g.splits; p.bn = g.bn;
+  p.rmin_a = g.tri.rmin_a; p.rmin_b = g.tri.rmin_b; p.rmax_a = g.tri.rmax_a; p.rmax_b = g.tri.rmax_b;
+  p.kmin_a = g.tri.kmin_a; p.kmin_b = g.tri.kmin_b; p.kmax_a = g.tri.kmax_a; p.kmax_b = g.tri.kmax_b;
   mk::GemmOperand A, B;
-  const int64_t a_off = ip[k++];
-  A.rows = p.M; A.mn_major = ip[k++]; A.ld = ip[k++]; A.zs_lo = ip[k++]; A.zs_hi = ip[k++];
-  const int64_t b_off = ip[k++];
-  B.rows = p.N; B.mn_major = ip[k++]; B.ld = ip[k++]; B.zs_lo = ip[k++]; B.zs_hi = ip[k++];
-  A.ptr = base_ptr(a) + a_off * eb;
-  B.ptr = base_ptr(b) + b_off * eb;
+  A.rows = p.M; A.mn_major = g.A.mn_major; A.ld = g.A.ld; A.zs_lo = g.A.zs_lo; A.zs_hi = g.A.zs_hi;
+  B.rows = p.N; B.mn_major = g.B.mn_major; B.ld = g.B.ld; B.zs_lo = g.B.zs_lo; B.zs_hi = g.B.zs_hi;
+  A.ptr = base_ptr(a) + g.A.offset * eb;
+  B.ptr = base_ptr(b) + g.B.offset * eb;
   // operand extents: the TMA descriptors clip rows and K to the problem, so the corner elements bound every load
-  check_extent(a, a_off, {{A.mn_major ? p.K : p.M, A.ld}, {A.mn_major ? p.M : p.K, 1}, {p.zlo_n, A.zs_lo}, {p.zhi_n, A.zs_hi}}, "A");
+  check_extent(a, g.A.offset, {{A.mn_major ? p.K : p.M, A.ld}, {A.mn_major ? p.M : p.K, 1}, {p.zlo_n, A.zs_lo}, {p.zhi_n, A.zs_hi}}, "A");
   if (peer == nullptr || peer->nseg == 0)   // with segments B is gathered from the segment pointers instead
-    check_extent(b, b_off, {{B.mn_major ? p.K : p.N, B.ld}, {B.mn_major ? p.N : p.K, 1}, {p.zlo_n, B.zs_lo}, {p.zhi_n, B.zs_hi}}, "B");
+    check_extent(b, g.B.offset, {{B.mn_major ? p.K : p.N, B.ld}, {B.mn_major ? p.N : p.K, 1}, {p.zlo_n, B.zs_lo}, {p.zhi_n, B.zs_hi}}, "B");
   mk::GemmEpilogue e;
-  const int64_t d_off = ip[k++];
   const int osz = static_cast<int>(d.element_size());
-  e.D = const_cast<char*>(base_ptr(d)) + d_off * osz;
+  e.D = const_cast<char*>(base_ptr(d)) + g.D.offset * osz;
   e.out_f32 = d.scalar_type() == torch::kFloat32;
-  e.accumulate = ip[k++];
-  e.d_zlo = ip[k++]; e.d_zhi = ip[k++];
-  e.rdiv = ip[k++]; e.rs_hi = ip[k++]; e.rs_lo = ip[k++];
-  e.ndiv = ip[k++]; e.ns_hi = ip[k++];
+  e.accumulate = g.accumulate;
+  e.d_zlo = g.D.d_zlo; e.d_zhi = g.D.d_zhi;
+  e.rdiv = g.D.rdiv; e.rs_hi = g.D.rs_hi; e.rs_lo = g.D.rs_lo;
+  e.ndiv = g.D.ndiv; e.ns_hi = g.D.ns_hi;
   {
     const int64_t rdiv = e.rdiv > 0 ? e.rdiv : (1 << 30), ndiv = e.ndiv > 0 ? e.ndiv : (1 << 30);   // <= 0: no split
-    check_extent(d, d_off, {{p.zhi_n, e.d_zhi}, {p.zlo_n, e.d_zlo}, {(p.M + rdiv - 1) / rdiv, e.rs_hi},
-                            {std::min<int64_t>(p.M, rdiv), e.rs_lo}, {(p.N + ndiv - 1) / ndiv, e.ns_hi},
-                            {std::min<int64_t>(p.N, ndiv), 1}}, "output");
+    check_extent(d, g.D.offset, {{p.zhi_n, e.d_zhi}, {p.zlo_n, e.d_zlo}, {(p.M + rdiv - 1) / rdiv, e.rs_hi},
+                                 {std::min<int64_t>(p.M, rdiv), e.rs_lo}, {(p.N + ndiv - 1) / ndiv, e.ns_hi},
+                                 {std::min<int64_t>(p.N, ndiv), 1}}, "output");
   }
-  e.alpha = static_cast<float>(alpha);
-  e.bias_mode = ip[k++];
-  {
-    const int64_t actw = ip[k++];     // low byte: activation code; bit 8: the second output holds the derivative
-    e.act = static_cast<int>(actw & 0xff);
-    e.save_deriv = static_cast<int>((actw >> 8) & 1);
-  }
-  const int64_t resid_off = ip[k++];
-  const int64_t preact_off = ip[k++];
-  {
-    // bit pattern of the activation parameter (fp32), then one reserved slot
-    const uint32_t bits = static_cast<uint32_t>(ip[k++]);
-    float f;
-    memcpy(&f, &bits, sizeof(f));
-    e.act_param = f;
-    e.bias_zs = ip[k++];
-  }
+  e.alpha = static_cast<float>(g.alpha);
+  e.bias_mode = g.bias_mode;
+  e.act = g.act;
+  e.save_deriv = g.preact_deriv ? 1 : 0;
+  e.act_param = g.act_param;
+  e.bias_zs = g.bias_zs;
   e.bias = nullptr;
-  if (bias.has_value() && bias->defined()) {
-    MK_CHECK(bias->is_cuda() && bias->scalar_type() == torch::kFloat32 && bias->is_contiguous(), "gemm: bias must be contiguous fp32 CUDA");
-    e.bias = bias->data_ptr<float>();
+  if (g.bias && g.bias->defined()) {
+    MK_CHECK(g.bias->is_cuda() && g.bias->scalar_type() == torch::kFloat32 && g.bias->is_contiguous(), "gemm: bias must be contiguous fp32 CUDA");
+    e.bias = g.bias->data_ptr<float>();
   }
   e.resid = nullptr;
-  if (resid.has_value() && resid->defined()) {
-    MK_CHECK(resid->scalar_type() == d.scalar_type(), "gemm: residual dtype must match output");
-    e.resid = base_ptr(*resid) + resid_off * osz;
+  if (g.resid && g.resid->defined()) {
+    MK_CHECK(g.resid->scalar_type() == d.scalar_type(), "gemm: residual dtype must match output");
+    e.resid = base_ptr(*g.resid) + g.resid_offset * osz;
   }
   e.preact = nullptr;
-  if (preact.has_value() && preact->defined()) {
-    MK_CHECK(preact->scalar_type() == d.scalar_type(), "gemm: preact dtype must match output");
-    e.preact = const_cast<char*>(base_ptr(*preact)) + preact_off * osz;
+  if (g.preact && g.preact->defined()) {
+    MK_CHECK(g.preact->scalar_type() == d.scalar_type(), "gemm: preact dtype must match output");
+    e.preact = const_cast<char*>(base_ptr(*g.preact)) + g.preact_offset * osz;
+  }
+  Tensor part;      // freed to the allocator on return: later work of this stream only
+  struct Ctx {
+    Tensor* part;
+    const Tensor* like;
+  } ctx{&part, g.row_sums};
+  mk::GemmRowSums rows;
+  if (g.row_sums) {
+    const Tensor& sums = *g.row_sums;
+    const int64_t groups = g.D.d_zlo != 0 ? g.zlo_n : 1;      // z_lo batches with outputs of their own
+    MK_CHECK(sums.is_cuda() && sums.scalar_type() == torch::kFloat32 && sums.is_contiguous() && sums.numel() == groups * g.M &&
+                 sums.get_device() == a.get_device(),
+             "gemm: row sums must be contiguous fp32 CUDA of the rows of A");
+    rows.out = sums.data_ptr<float>();
+    rows.ctx = &ctx;
+    rows.scratch = [](void* c, long long floats) -> float* {
+      Ctx& x = *static_cast<Ctx*>(c);
+      try {
+        *x.part = torch::empty({floats}, x.like->options());
+      } catch (const std::exception&) {
+        return nullptr;
+      }
+      return x.part->data_ptr<float>();
+    };
+    rows.done = 0;
   }
   Tensor ef = err_flag_for(a);
-  check_cuda(mk::gemm_launch(p, A, B, e, ef.data_ptr<int>(), cur_stream(), peer, rows), "gemm launch");
+  ++launches();
+  check_cuda(mk::gemm_launch(p, A, B, e, ef.data_ptr<int>(), stream(), peer, g.row_sums ? &rows : nullptr), "gemm launch");
+  return g.row_sums && rows.done != 0;
 }
+
+void complex_product(const Tensor& a, const Tensor& b, Tensor& d, const Tensor* resid, const std::vector<int64_t>& ip) {
+  ++launches();
+  c10::optional<Tensor> r;
+  if (resid && resid->defined()) r = *resid;
+  gemm_complex(a, b, d, r, ip);
+}
+
+void folded_product(const Tensor& a, const Tensor& b, Tensor& d, const std::vector<int64_t>& ip) {
+  ++launches();
+  gemm_fold(a, b, d, ip);
+}
+
+}  // namespace mkh
+
+namespace {
 
 void inorm_fwd(const Tensor& x, Tensor& y, const c10::optional<Tensor>& w, const c10::optional<Tensor>& b, Tensor& stats,
                int64_t C, double eps, int64_t act, int64_t ext_stats) {
@@ -774,6 +821,8 @@ void peer_allreduce(const std::vector<int64_t>& data_ptrs, const std::vector<int
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  m.def("launches", []() { return mkh::launches(); }, "kernel launches of this thread's layer passes");
+  mkh::bind_layers(m);
   m.def("gemm_row_sums", &gemm_row_sums);
   m.def("gemm", &gemm, "tcgen05 GEMM with fused epilogue");
   m.def("gemm_peer", &gemm_peer, "tcgen05 GEMM reading its B operand from peer devices");

@@ -20,7 +20,7 @@ BUILD = os.path.join(HERE, "build")
 TARGET = os.path.join(HERE, "_C.so")
 
 CU_SOURCES = ["gemm_tcgen05.cu", "fused_ops.cu", "peer.cu", "spectral_modes.cu", "no_alloc.cu"]
-CPP_SOURCES = ["bindings.cpp"]
+CPP_SOURCES = ["bindings.cpp", "layers.cpp"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",

@@ -60,7 +60,12 @@ def available() -> bool:
 # number of kernel-launching calls into this extension by the current process (the column sums launch a second kernel)
 LAUNCHES = 0
 _NON_KERNEL = {"read_error_flag", "clear_error_flag", "lp_scratch_floats", "adam_entry_bytes", "peer_alloc", "peer_open",
-               "peer_close", "peer_free", "tensor_from_ptr", "set_gelu_tanh", "stream_state"}
+               "peer_close", "peer_free", "tensor_from_ptr", "set_gelu_tanh", "stream_state", "launches"}
+
+
+# passes over whole layers, which count their launches themselves
+_LAYERS = {"conv_forward", "conv_backward", "mlp_forward", "mlp_backward", "norm_forward", "norm_backward", "spectral_forward",
+           "spectral_backward", "afno_forward", "afno_backward"}
 
 
 class _Counting:
@@ -76,6 +81,13 @@ class _Counting:
             raw = getattr(self._mod, name)
             if name in _NON_KERNEL:
                 fn = raw
+            elif name in _LAYERS:
+                def fn(*args, __raw=raw, __count=self._mod.launches, **kwargs):
+                    global LAUNCHES
+                    before = __count()
+                    out = __raw(*args, **kwargs)
+                    LAUNCHES += __count() - before
+                    return out
             else:
                 def fn(*args, __raw=raw, **kwargs):
                     global LAUNCHES

@@ -71,6 +71,7 @@ class AFNOPlan:
         self.fw, self.fw_t = prep(fw), prep(fw.t())           # [2 ncols, W],  [W, 2 ncols]
         self.gw, self.gw_t = prep(gw), prep(gw.t())           # [W, 2 ncols],  [2 ncols, W]
         self.fh, self.gh = prep(fh), prep(fh.t())             # [2 nkx, 2 H],  [2 H, 2 nkx]  (inverse = transpose)
+        self.tables = [self.fw, self.fw_t, self.gw, self.gw_t, self.fh, self.gh]      # as the native passes take them
 
     @staticmethod
     def get(H, W, kx, ncols, device, dtype) -> "AFNOPlan":
@@ -217,6 +218,15 @@ class _AFNOFilter(torch.autograd.Function):
         nc, nkx = plan.ncols, plan.nkx
         T = B * nc * nkx
         dt = x.dtype
+        ctx.plan, ctx.dims = plan, (B, C, nb, bs, hid)
+        # skip_is_x: the skip is the input itself (the usual residual form); its gradient then rides in the epilogue of
+        # the last backward GEMM instead of a separate elementwise add
+        ctx.flags = (b1 is not None, b2 is not None, skip is not None, skip is x)
+        ctx.wtypes = tuple(None if t is None else t.dtype for t in (w1, b1, w2, b2))
+        if x.is_cuda:
+            out, *saved = _ext.require().afno_forward(x, w1, b1, w2, b2, skip, plan.tables, [H, W, nkx, nc, nb], float(lam))
+            ctx.save_for_backward(*saved)
+            return out
         (w1q, w2q), (b1f, b2f) = _pack((w1, w2), (b1, b2), dt)
         t1 = _stage_w_analysis(x, plan.fw, plan)
         y = _stage_h_tokens(t1, plan, B, C, nb)
@@ -229,11 +239,6 @@ class _AFNOFilter(torch.autograd.Function):
         t4 = _stage_h_blocks(o2, plan.gh, plan, B, C, nb)
         out = _stage_w_synthesis(t4, plan.gw, plan, B, C, skip)
         ctx.save_for_backward(y, o1, o2, w1q, w2q)
-        ctx.plan, ctx.dims = plan, (B, C, nb, bs, hid)
-        # skip_is_x: the skip is the input itself (the usual residual form); its gradient then rides in the epilogue of
-        # the last backward GEMM instead of a separate elementwise add
-        ctx.flags = (b1 is not None, b2 is not None, skip is not None, skip is x)
-        ctx.wtypes = tuple(None if t is None else t.dtype for t in (w1, b1, w2, b2))
         return out
 
     @staticmethod
@@ -245,6 +250,10 @@ class _AFNOFilter(torch.autograd.Function):
         H, nc, nkx = plan.H, plan.ncols, plan.nkx
         T = B * nc * nkx
         dy = dy.contiguous()
+        if dy.is_cuda:
+            dx, *grads = _ext.require().afno_backward(dy, y, o1, o2, w1q, w2q, plan.tables, [H, plan.W, nkx, nc, nb], has_b1, has_b2, skip_is_x)
+            gw1, gb1, gw2, gb2 = (g if g is None else g.to(t) for g, t in zip(grads, ctx.wtypes))
+            return dx, gw1, gb1, gw2, gb2, (dy if (has_skip and not skip_is_x) else None), None, None
         dt = dy.dtype
         dev = dy.device
         # fp32 sums of the packed weights and biases, cleared together

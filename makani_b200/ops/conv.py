@@ -159,6 +159,9 @@ def _chan_sum(dy):
     return channel_sums(dy)
 
 
+_LAYOUT_CODE = {None: -1, NCHW: 0, CL: 1}      # as the native passes (csrc/layers.cpp) take it
+
+
 def _canon(t):
     """Gradients arrive in whatever layout autograd produced; bring them to a supported dense layout."""
     if layout_of(t) is None:
@@ -169,10 +172,8 @@ def _canon(t):
 class _Conv1x1(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, bias, resid, act, out_layout, train):
-        wq = prep_weight(w)
         ci = w.shape[1]
-        bias_f = bias.detach().float().contiguous() if bias is not None else None
-        y, pre = _conv_fwd(x, wq, ci, bias_f, act, resid, want_preact=(train and act == ACT_GELU), out_layout=out_layout)
+        y, wq, pre = _ext.require().conv_forward(x, w, bias, resid, act, _LAYOUT_CODE[out_layout], train and act == ACT_GELU)
         ctx.save_for_backward(x, wq, pre)
         ctx.ci = ci
         ctx.act = act
@@ -191,15 +192,9 @@ class _Conv1x1(torch.autograd.Function):
             g = dgelu_mul(dy, pre)
         else:
             g = dy
-        dx = _conv_dgrad(g, wq, ctx.ci, x_layout=layout_of(x)) if ctx.needs_input_grad[0] else None
-        dw = db = None
-        want_db = ctx.has_bias and ctx.needs_input_grad[2]
-        if ctx.needs_input_grad[1]:
-            dw, db = _conv_wgrad(g, x, bias=True) if want_db else (_conv_wgrad(g, x), None)
-            dw = dw.reshape(ctx.wshape)
-        elif want_db:
-            db = _chan_sum(g)
-        return dx, dw, db, dres, None, None, None
+        dx, dw, db = _ext.require().conv_backward(g, x, wq, ctx.ci, ctx.needs_input_grad[0], ctx.needs_input_grad[1],
+                                                  ctx.has_bias and ctx.needs_input_grad[2])
+        return dx, (None if dw is None else dw.reshape(ctx.wshape)), db, dres, None, None, None
 
 
 class _MLP2(torch.autograd.Function):
@@ -208,17 +203,11 @@ class _MLP2(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, w1, b1, w2, b2, resid, out_layout, train):
-        w1q, w2q = prep_weight(w1), prep_weight(w2)
-        ci, ch = w1.shape[1], w1.shape[0]
-        b1f = b1.detach().float().contiguous() if b1 is not None else None
-        b2f = b2.detach().float().contiguous() if b2 is not None else None
-        hid_layout = CL if ch % 8 == 0 else NCHW
         # the first GEMM's second output is GELU'(pre-activation): the backward epilogue then only multiplies
         # (without a backward pass to come it is not computed, nor written)
-        h, dact = _conv_fwd(x, w1q, ci, b1f, ACT_GELU, None, want_preact=train, out_layout=hid_layout, deriv=train)
-        y, _ = _conv_fwd(h, w2q, ch, b2f, ACT_NONE, resid, want_preact=False, out_layout=out_layout)
+        y, w1q, w2q, dact, h = _ext.require().mlp_forward(x, w1, b1, w2, b2, resid, _LAYOUT_CODE[out_layout], train)
         ctx.save_for_backward(x, w1q, w2q, dact, h)
-        ctx.dims = (ci, ch)
+        ctx.ci = w1.shape[1]
         ctx.flags = (b1 is not None, b2 is not None, resid is not None)
         ctx.wshapes = (w1.shape, w2.shape)
         return y
@@ -226,13 +215,9 @@ class _MLP2(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x, w1q, w2q, dact, h = ctx.saved_tensors
-        ci, ch = ctx.dims
         has_b1, has_b2, has_res = ctx.flags
         dy = _canon(dy)
-        dpre = _conv_dgrad(dy, w2q, ch, act=ACT_MULAUX, aux=dact, x_layout=layout_of(dact))
-        dw2, db2 = _conv_wgrad(dy, h, bias=True) if has_b2 else (_conv_wgrad(dy, h), None)
-        dx = _conv_dgrad(dpre, w1q, ci, x_layout=layout_of(x)) if ctx.needs_input_grad[0] else None
-        dw1, db1 = _conv_wgrad(dpre, x, bias=True) if has_b1 else (_conv_wgrad(dpre, x), None)
+        dx, dw1, db1, dw2, db2 = _ext.require().mlp_backward(dy, x, w1q, w2q, dact, h, ctx.ci, ctx.needs_input_grad[0], has_b1, has_b2)
         return dx, dw1.reshape(ctx.wshapes[0]), db1, dw2.reshape(ctx.wshapes[1]), db2, (dy if has_res else None), None, None
 
 

@@ -62,12 +62,18 @@ class _InstanceNormCL(torch.autograd.Function):
     def forward(ctx, x, weight, bias, eps, act, count, reduce_fn, slot=None):
         ext = _ext.require()
         B, C, H, W = x.shape
+        ctx.act, ctx.cnt, ctx.reduce_fn, ctx.slot = int(act), float(count if count else H * W), reduce_fn, slot
+        ctx.affine = weight is not None
+        if slot is None and reduce_fn is None:
+            y, stats, wf, bf = ext.norm_forward(x, weight, bias, float(eps), ctx.act, ctx.cnt)
+            ctx.save_for_backward(x, wf, bf, stats)
+            return y
         y = torch.empty_like(x)     # preserves channels_last
         sums = torch.zeros(B, C, 2, dtype=torch.float32, device=x.device)
         stats = torch.empty(B, C, 2, dtype=torch.float32, device=x.device)
         wf = weight.detach().float().contiguous() if weight is not None else None
         bf = bias.detach().float().contiguous() if bias is not None else None
-        cnt = float(count if count else H * W)
+        cnt = ctx.cnt
         if slot is not None:
             from ..parallel.peer import sync_descriptor
             slot.set_layout(B * C * 8)
@@ -76,15 +82,11 @@ class _InstanceNormCL(torch.autograd.Function):
             ext.inorm_cl_apply(x, None, y, wf, bf, sums, stats, B, C, cnt, float(eps), int(act), 0,
                                sync_descriptor(consume=slot), slot.sources())
         else:
-            # statistics local to this device are accumulated around the first token (mode bit 1): no cancellation in
-            # E[x^2] - E[x]^2 for fields with |mean| >> std; sums merged across ranks stay unshifted
-            m0 = 2 if reduce_fn is None else 0
-            ext.inorm_cl_sums(x, None, None, None, None, sums, None, None, B, C, 0, m0)
-            if reduce_fn is not None:
-                sums = reduce_fn(sums)
-            ext.inorm_cl_apply(x, None, y, wf, bf, sums, stats, B, C, cnt, float(eps), int(act), m0)
+            # (sums merged across ranks are not shifted to the first token, as those of one device are)
+            ext.inorm_cl_sums(x, None, None, None, None, sums, None, None, B, C, 0, 0)
+            sums = reduce_fn(sums)
+            ext.inorm_cl_apply(x, None, y, wf, bf, sums, stats, B, C, cnt, float(eps), int(act), 0)
         ctx.save_for_backward(x, wf, bf, stats)
-        ctx.act, ctx.cnt, ctx.reduce_fn, ctx.affine, ctx.slot = int(act), cnt, reduce_fn, weight is not None, slot
         return y
 
     @staticmethod
@@ -94,6 +96,9 @@ class _InstanceNormCL(torch.autograd.Function):
         B, C, H, W = x.shape
         if not _is_cl(dy):
             dy = dy.contiguous(memory_format=torch.channels_last)
+        if ctx.slot is None and ctx.reduce_fn is None:
+            dx, dw, db = ext.norm_backward(x, dy, wf, bf, stats, ctx.affine, ctx.act, ctx.cnt)
+            return dx, dw, db, None, None, None, None, None
         acc = torch.zeros(2 * B + (2 if ctx.affine else 0), C, dtype=torch.float32, device=x.device)     # one clearing launch
         sums = acc[: 2 * B].view(B, C, 2)
         dw, db = (acc[2 * B], acc[2 * B + 1]) if ctx.affine else (None, None)
@@ -108,8 +113,7 @@ class _InstanceNormCL(torch.autograd.Function):
                                sync_descriptor(consume=slot), slot.sources())
         else:
             ext.inorm_cl_sums(x, dy, wf, bf, stats, sums, dw, db, B, C, ctx.act, 1)
-            if ctx.reduce_fn is not None:
-                sums = ctx.reduce_fn(sums)
+            sums = ctx.reduce_fn(sums)
             ext.inorm_cl_apply(x, dy, dx, wf, bf, sums, stats, B, C, ctx.cnt, 0.0, ctx.act, 1)
         return dx, dw, db, None, None, None, None, None
 

@@ -86,6 +86,11 @@ class SHTPlan:
         self._folded = {(syn, fwd): self._fold_table(syn, fwd) for fwd in (True, False) for syn in (True, False)
                         if (self.folds_synthesis if syn else self.folds_analysis)}
 
+        # what the native passes take: matrices (empty where one is not folded) and extents
+        none = torch.empty(0, device=self.device, dtype=dtype)
+        self.native = ([self.f, self.gt, self.pw, self.p] + [self._folded.get((syn, fwd), none) for syn in (True, False) for fwd in (True, False)],
+                       [nlat, nlon, lmax, mmax])
+
     def _fold_table(self, synthesis: bool, forward: bool) -> torch.Tensor:
         """The inverse transform's matrix (`synthesis`; rows are longitudes, halves the cosine and sine terms) or the forward one's
         (rows (m, ri), halves the even and odd points), from the coefficients of the forward transform (`forward`) or of the
@@ -385,6 +390,13 @@ class _SpectralConv(torch.autograd.Function):
     def forward(ctx, x, w, plan_in: SHTPlan, plan_out: SHTPlan, want_resid: bool, train: bool):
         x = _to_cl(x)
         wx = weight_planes(w, x.dtype, keep=not train, share=train)
+        ctx.plans = (plan_in, plan_out)
+        ctx.want_resid = want_resid
+        ctx.wshape = w.shape
+        if x.is_cuda:
+            y, r, t2 = _ext.require().spectral_forward(x, wx, *plan_in.native, *plan_out.native, want_resid)
+            ctx.save_for_backward(t2, wx)
+            return (y, r) if want_resid else y
         t1 = analyse(x, plan_in)
         t2 = legendre_analysis(t1, plan_in.pw)
         del t1
@@ -398,9 +410,6 @@ class _SpectralConv(torch.autograd.Function):
             t4r = legendre_synthesis(t2, True, plan_out.p, plan_out.nlat)
             r = synthesise(t4r, plan_out)
         ctx.save_for_backward(t2, wx)
-        ctx.plans = (plan_in, plan_out)
-        ctx.want_resid = want_resid
-        ctx.wshape = w.shape
         if want_resid:
             return y, r
         return y
@@ -410,6 +419,11 @@ class _SpectralConv(torch.autograd.Function):
         t2, wx = ctx.saved_tensors
         plan_in, plan_out = ctx.plans
         dy = _to_cl(dy)
+        if dy.is_cuda:
+            dr = _to_cl(dr) if ctx.want_resid and dr is not None else None
+            dx, dw = _ext.require().spectral_backward(dy, dr, t2, wx, *plan_in.native, *plan_out.native, ctx.needs_input_grad[0],
+                                                      ctx.needs_input_grad[1])
+            return dx, (None if dw is None else dw.reshape(ctx.wshape)), None, None, None, None
         # adjoint of the inverse DFT / synthesis on the output grid
         dt4 = analyse(dy, plan_out, forward=False)
         dt3 = legendre_analysis(dt4, plan_out.p)                       # [B, l, m, (ri, o)]
