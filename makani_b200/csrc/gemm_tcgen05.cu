@@ -1989,10 +1989,12 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
   kp.neg_seg = p.cplx == 2 ? 0 : 1;
   kp.a_part = p.K;
   if (folded) {
-    // (from 64 rows on the mirror rows' boxes start at or after row 0, and the last box of sums ends inside the table)
+    // (from 64 rows on the mirror rows' boxes start at or after row 0, and the last box of sums ends inside the table; the computed
+    // rows and their mirrors make up all rows, or some would stay unwritten)
     if (epi != 6 || kp.splits != 1 || p.splits == 0 || kp.nseg != 1 || rd != 1 || A.mn_major || p.mirror < 64 || (p.a_plane % 8) != 0 ||
-        p.M > p.mirror / 2 + 2 || p.rows < p.mirror / 2 + 32 || p.zlo_n != 1) {
-      snprintf(g_err, sizeof(g_err), "folded product: bf16, K-major tables, plain aligned rows, at least 64 of them");
+        p.M != (p.cplx == 5 ? 2 * (p.mirror / 4 + 1) : p.mirror / 2 + 1) || p.rows < p.mirror / 2 + 32 ||
+        p.rows > p.mirror + (p.cplx == 5 ? 2 : 0) || p.zlo_n != 1) {
+      snprintf(g_err, sizeof(g_err), "folded product: bf16, K-major tables, plain aligned rows, at least 64 of them, each computed or a mirror");
       return cudaErrorInvalidValue;
     }
     kp.a_part = static_cast<int>(p.a_plane);

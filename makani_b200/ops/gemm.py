@@ -300,7 +300,10 @@ def gemm_fold(rows: int, M: int, N: int, K: int, mirror: int, pairs: bool, table
         D[r] = P(0)[r] + P(1)[r],   D[mirror - r] = P(0)[r] - P(1)[r],   both where they are one of the `rows` rows of D
 
     With `pairs` the rows are (order, re / im) pairs: row 2 m + ri has its mirror at mirror - 2 m + ri, and the imaginary one its
-    sign changed.  `M` rows cover one half and its middle.  `b_plane`: elements between the two planes of B; z_hi batches B and D."""
+    sign changed.  `M` rows cover one half and its middle, all that are not mirrors of others, and `rows` end with the mirrors of
+    the first ones, so that every row of D is written.  `b_plane`: elements between the two planes of B; z_hi batches B and D."""
+    if M != (2 * (mirror // 4 + 1) if pairs else mirror // 2 + 1) or not M <= rows <= mirror + (2 if pairs else 0):
+        raise ValueError(f"gemm_fold: {M} computed rows and their mirrors at {mirror} do not make up {rows} rows")
     if not B.tensor.is_cuda:
         fb, fd = _flat(B.tensor), _flat(D.tensor)
         cdt = torch.float64 if fb.dtype == torch.float64 else torch.float32

@@ -81,8 +81,10 @@ class SHTPlan:
         #   180 x 360, 181 33 / 28;  200 channels: 181 x 360, 120 18.8 / 18.5;  64 channels, 2 x 64 x 128, 65 12.0 / 9.9
         #   analysis: 240 x 480, 241 58 / 47; 360 x 720, 361 155 / 131, 241 of them 111 / 121; 181 x 360, 120 20.5 / 18.5 (adjoint
         #   16.4 / 18.5); 100 x 200, 81 11.8 / 10.0
+        # Orders past half the points, which alias, have no mirror and stay whole.
         self.folds_synthesis = nlon >= 64
-        self.folds_analysis = nlon >= 64 and nlon % 2 == 0 and 8 * mmax > 3 * nlon and 2 * mmax >= nlon // 2 + 32
+        self.folds_analysis = (nlon >= 64 and nlon % 2 == 0 and 8 * mmax > 3 * nlon and
+                               nlon // 2 + 32 <= 2 * mmax <= nlon + 2)
         self._folded = {(syn, fwd): self._fold_table(syn, fwd) for fwd in (True, False) for syn in (True, False)
                         if (self.folds_synthesis if syn else self.folds_analysis)}
 

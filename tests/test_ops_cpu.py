@@ -239,3 +239,19 @@ def test_folded_transforms_equal_the_whole_ones(h, w, mmax, analysis):
             ok = mirror < 2 * mmax
             sign = (1.0 - 2.0 * (r[ok] % 2))[:, None]
             assert torch.equal(a[mirror[ok]], sign * a[ok]) and torch.equal(b[mirror[ok]], -sign * b[ok])
+
+
+@pytest.mark.parametrize("w,mmax", [(64, 34), (90, 60), (96, 97)])
+def test_orders_past_half_the_points_are_transformed_whole(w, mmax):
+    """Orders past w / 2 have no mirror among the rows that a folded analysis writes."""
+    from makani_b200.ops.gemm import Operand, Output, gemm_fold
+    from makani_b200.ops.spectral import SHTPlan, analyse, dft_analysis
+    plan = SHTPlan(4, w, 4, mmax, "legendre-gauss", "cpu", torch.float64)
+    x = torch.randn(1, 4, w, 8, dtype=torch.float64).permute(0, 3, 1, 2)
+    assert torch.equal(analyse(x, plan), dft_analysis(x, plan.f, False, w, plan.k2))
+    assert torch.equal(analyse(x, plan, forward=False), dft_analysis(x, plan.gt, True, plan.k2p, plan.k2))
+    # and a product that would leave rows of its output unwritten is refused
+    table, d = torch.zeros(2 * mmax, w, dtype=torch.float64), torch.zeros(4, 2 * mmax, 8, dtype=torch.float64)
+    with pytest.raises(ValueError):
+        gemm_fold(2 * mmax, 2 * (w // 4 + 1), 8, w // 2, w, True, table, w // 2, Operand(x, ld=16, mn_major=True, zs_hi=w * 8), 8,
+                  Output(d, rs_lo=8, d_zhi=2 * mmax * 8), zhi_n=4)
