@@ -469,6 +469,7 @@ void gemm_fold(const Tensor& a, const Tensor& b, Tensor& d, const std::vector<in
   A.rows = p.rows; A.mn_major = 0; A.ld = ip[k++]; A.zs_lo = 0; A.zs_hi = 0; p.a_plane = ip[k++];
   const int64_t b_off = ip[k++];
   B.rows = p.N; B.mn_major = ip[k++]; B.ld = ip[k++]; B.zs_lo = 0; B.zs_hi = ip[k++]; p.b_plane = ip[k++];
+  MK_CHECK(p.K <= p.a_plane, "gemm_fold: more columns than a half of the table has");
   A.ptr = base_ptr(a);
   B.ptr = base_ptr(b) + b_off * 2;
   check_extent(a, 0, {{p.rows, A.ld}, {2, p.a_plane}, {p.K, 1}}, "A");

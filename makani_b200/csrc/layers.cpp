@@ -291,13 +291,12 @@ std::tuple<Tensor, OptTensor, OptTensor> norm_backward(const Tensor& x, const Te
 // extents [nlat, nlon, lmax, mmax]
 struct Plan {
   const std::vector<Tensor>& t;
-  int64_t nlat, nlon, mmax, k2;
+  int64_t nlat, nlon, k2;
   Plan(const std::vector<Tensor>& tables, const std::vector<int64_t>& n) : t(tables) {
     MK_CHECK(tables.size() == 8 && n.size() == 4, "spectral plan: eight tables and four extents expected");
     nlat = n[0];
     nlon = n[1];
-    mmax = n[3];
-    k2 = 2 * mmax;
+    k2 = 2 * n[3];
   }
 };
 
@@ -326,7 +325,7 @@ Tensor synthesise(const Tensor& t4, const Plan& p, bool forward) {
   Tensor y = at::empty({B, C, H, W}, t4.options(), at::MemoryFormat::ChannelsLast);
   const Tensor& fold = p.t[forward ? 4 : 5];
   if (fold.numel()) {
-    mkh::folded_product(fold, t4, y, {4, W, W / 2 + 1, C, p.mmax, W, B * H, fold.size(1), fold.size(1) / 2, 0, 1, 2 * C, k2 * C, C, 0, C, W * C});
+    mkh::folded_product(fold, t4, y, {4, W, W / 2 + 1, C, k2 / 2, W, B * H, fold.size(1), fold.size(1) / 2, 0, 1, 2 * C, k2 * C, C, 0, C, W * C});
     return y;
   }
   const Tensor& m = p.t[forward ? 0 : 1];

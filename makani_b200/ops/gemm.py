@@ -304,6 +304,8 @@ def gemm_fold(rows: int, M: int, N: int, K: int, mirror: int, pairs: bool, table
     the first ones, so that every row of D is written.  `b_plane`: elements between the two planes of B; z_hi batches B and D."""
     if M != (2 * (mirror // 4 + 1) if pairs else mirror // 2 + 1) or not M <= rows <= mirror + (2 if pairs else 0):
         raise ValueError(f"gemm_fold: {M} computed rows and their mirrors at {mirror} do not make up {rows} rows")
+    if K > part:
+        raise ValueError(f"gemm_fold: {K} columns, a half of the table has {part}")
     if not B.tensor.is_cuda:
         fb, fd = _flat(B.tensor), _flat(D.tensor)
         cdt = torch.float64 if fb.dtype == torch.float64 else torch.float32

@@ -187,14 +187,15 @@ def analyse(x: torch.Tensor, plan: SHTPlan, forward: bool = True) -> torch.Tenso
 
 
 def synthesise(t4: torch.Tensor, plan: SHTPlan, forward: bool = False) -> torch.Tensor:
-    """Inverse longitude DFT of t4 [B, H, (m, ri), C], or the adjoint of the forward one (`forward`); channels-last."""
+    """Inverse longitude DFT of t4 [B, H, (m, ri), C], or the adjoint of the forward one (`forward`); channels-last.  t4 may hold
+    fewer orders than the plan: those of a forward transform that keeps fewer than the inverse one."""
     W = plan.nlon
     if not plan.folds_synthesis:
         return dft_synthesis(t4, plan.f, True, W, W) if forward else dft_synthesis(t4, plan.gt, False, plan.k2p, W)
     B, H, k2, C = t4.shape
     table = plan._folded[True, forward]
     y = torch.empty(B, C, H, W, dtype=t4.dtype, device=t4.device, memory_format=torch.channels_last)
-    gemm_fold(W, W // 2 + 1, C, plan.mmax, W, False, table, table.shape[1] // 2,
+    gemm_fold(W, W // 2 + 1, C, k2 // 2, W, False, table, table.shape[1] // 2,
               Operand(t4, ld=2 * C, mn_major=True, zs_hi=k2 * C), C, Output(y, rs_lo=C, d_zhi=W * C), zhi_n=B * H)
     return y
 

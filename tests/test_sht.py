@@ -88,3 +88,20 @@ def test_gemm_chain_matches_reference_forward_and_backward(B, C, Co):
     gx2, gw2 = torch.autograd.grad([yref, rref], [x, w], [gy, gr])
     assert (gx - gx2).abs().max().item() < 1e-5
     assert (gw - gw2).abs().max().item() < 1e-4
+
+
+@pytest.mark.parametrize("nlon,lmax,m_in,m_out", [(128, 33, 24, 33), (128, 33, 20, 65), (48, 16, 12, 17)])
+def test_fewer_orders_forward_than_inverse(nlon, lmax, m_in, m_out):
+    """A forward transform that keeps fewer orders than the inverse one: the orders it does not keep are zero."""
+    dt, nlat, C, Co = torch.float64, nlon // 2, 8, 16
+    pin = SHTPlan(nlat, nlon, lmax, m_in, "equiangular", "cpu", dt)
+    pout = SHTPlan(nlat, nlon, lmax, m_out, "legendre-gauss", "cpu", dt)
+    torch.manual_seed(3)
+    x = torch.randn(2, C, nlat, nlon, dtype=dt)
+    w = torch.randn(C, Co, lmax, dtype=torch.complex128)
+    y, r = spectral_conv_dhconv(x, w, pin, pout, True)
+    c = torch.zeros(2, C, lmax, m_out, dtype=torch.complex128)
+    c[..., :m_in] = RealSHT(nlat, nlon, lmax, m_in, "equiangular").double()(x)
+    isht = InverseRealSHT(nlat, nlon, lmax, m_out, "legendre-gauss").double()
+    for got, ref in ((y, isht(torch.einsum("bixy,iox->boxy", c, w))), (r, isht(c))):
+        assert (got - ref).abs().max() < 1e-6 * ref.abs().max()      # the tables are fp32 numbers
