@@ -71,6 +71,12 @@ std::pair<int64_t, int64_t> stream_state(int64_t device) {
   return {reinterpret_cast<int64_t>(s), cap};
 }
 
+inline float* f32_ptr(const c10::optional<Tensor>& t) {
+  if (!t.has_value() || !t->defined()) return nullptr;
+  MK_CHECK(t->is_cuda(), "statistics and parameters must be CUDA tensors");
+  return t->data_ptr<float>();
+}
+
 inline const char* base_ptr(const Tensor& t) { return static_cast<const char*>(t.data_ptr()); }
 
 static bool parse_peer(mk::GemmPeer& g, const std::vector<int64_t>& seg, const std::vector<int64_t>& sync) {
@@ -288,12 +294,12 @@ bool run(const Gemm& g, const mk::GemmPeer* peer) {
   }
   e.resid = nullptr;
   if (g.resid && g.resid->defined()) {
-    MK_CHECK(g.resid->scalar_type() == d.scalar_type(), "gemm: residual dtype must match output");
+    MK_CHECK(g.resid->is_cuda() && g.resid->scalar_type() == d.scalar_type(), "gemm: the residual must be a CUDA tensor of the output's type");
     e.resid = base_ptr(*g.resid) + g.resid_offset * osz;
   }
   e.preact = nullptr;
   if (g.preact && g.preact->defined()) {
-    MK_CHECK(g.preact->scalar_type() == d.scalar_type(), "gemm: preact dtype must match output");
+    MK_CHECK(g.preact->is_cuda() && g.preact->scalar_type() == d.scalar_type(), "gemm: preact must be a CUDA tensor of the output's type");
     e.preact = const_cast<char*>(base_ptr(*g.preact)) + g.preact_offset * osz;
   }
   Tensor part;      // freed to the allocator on return: later work of this stream only
@@ -351,8 +357,7 @@ void inorm_fwd(const Tensor& x, Tensor& y, const c10::optional<Tensor>& w, const
   c10::cuda::CUDAGuard guard(x.device());
   const int64_t planes = stats.numel() / 2;
   const int64_t hw = x.numel() / planes;
-  const float* wp = (w.has_value() && w->defined()) ? w->data_ptr<float>() : nullptr;
-  const float* bp = (b.has_value() && b->defined()) ? b->data_ptr<float>() : nullptr;
+  const float *wp = f32_ptr(w), *bp = f32_ptr(b);
   check_cuda(mk::inorm_fwd(reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()), reinterpret_cast<__nv_bfloat16*>(y.data_ptr()), wp, bp,
                            stats.data_ptr<float>(), static_cast<int>(planes), static_cast<int>(C), hw, static_cast<float>(eps),
                            static_cast<int>(act), static_cast<int>(ext_stats), cur_stream()),
@@ -570,12 +575,9 @@ void inorm_bwd(const Tensor& x, const Tensor& dy, c10::optional<Tensor> dx, cons
   c10::cuda::CUDAGuard guard(x.device());
   const int64_t planes = stats.numel() / 2;
   const int64_t hw = x.numel() / planes;
-  auto fp = [](const c10::optional<Tensor>& t) -> float* {
-    return (t.has_value() && t->defined()) ? t->data_ptr<float>() : nullptr;
-  };
   __nv_bfloat16* dxp = (dx.has_value() && dx->defined()) ? reinterpret_cast<__nv_bfloat16*>(dx->data_ptr()) : nullptr;
   check_cuda(mk::inorm_bwd(reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()), reinterpret_cast<const __nv_bfloat16*>(dy.data_ptr()),
-                           dxp, fp(w), fp(b), stats.data_ptr<float>(), fp(dw), fp(db), fp(sums_io), static_cast<int>(planes),
+                           dxp, f32_ptr(w), f32_ptr(b), stats.data_ptr<float>(), f32_ptr(dw), f32_ptr(db), f32_ptr(sums_io), static_cast<int>(planes),
                            static_cast<int>(C), hw, count, static_cast<int>(act), static_cast<int>(ext_sums), cur_stream()),
              "inorm_bwd");
 }
@@ -618,12 +620,11 @@ void inorm_cl_sums(const Tensor& x, const c10::optional<Tensor>& dy, const c10::
   MK_CHECK(sums.scalar_type() == torch::kFloat32 && sums.is_contiguous() && sums.numel() == B * C * 2, "inorm_cl_sums: bad sums");
   c10::cuda::CUDAGuard guard(x.device());
   const int64_t T = x.numel() / (B * C);
-  auto fp = [](const c10::optional<Tensor>& t) -> float* { return (t.has_value() && t->defined()) ? t->data_ptr<float>() : nullptr; };
   const __nv_bfloat16* dyp = (dy.has_value() && dy->defined()) ? reinterpret_cast<const __nv_bfloat16*>(dy->data_ptr()) : nullptr;
   mk::StatExchange xc;
   const bool ex = make_exchange(xc, sync, dsts, true, x);
-  check_cuda(mk::inorm_cl_sums(reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()), dyp, fp(w), fp(b), fp(stats), sums.data_ptr<float>(),
-                               fp(dw), fp(db), static_cast<int>(B), static_cast<int>(C), T, static_cast<int>(act), static_cast<int>(mode),
+  check_cuda(mk::inorm_cl_sums(reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()), dyp, f32_ptr(w), f32_ptr(b), f32_ptr(stats), sums.data_ptr<float>(),
+                               f32_ptr(dw), f32_ptr(db), static_cast<int>(B), static_cast<int>(C), T, static_cast<int>(act), static_cast<int>(mode),
                                cur_stream(), ex ? &xc : nullptr),
              "inorm_cl_sums");
 }
@@ -634,12 +635,11 @@ void inorm_cl_apply(const Tensor& x, const c10::optional<Tensor>& dy, Tensor& ou
   MK_CHECK(x.is_cuda() && x.scalar_type() == torch::kBFloat16 && out.scalar_type() == torch::kBFloat16, "inorm_cl_apply: bf16 CUDA expected");
   c10::cuda::CUDAGuard guard(x.device());
   const int64_t T = x.numel() / (B * C);
-  auto fp = [](const c10::optional<Tensor>& t) -> float* { return (t.has_value() && t->defined()) ? t->data_ptr<float>() : nullptr; };
   const __nv_bfloat16* dyp = (dy.has_value() && dy->defined()) ? reinterpret_cast<const __nv_bfloat16*>(dy->data_ptr()) : nullptr;
   mk::StatExchange xc;
   const bool ex = make_exchange(xc, sync, srcs, false, x);
   check_cuda(mk::inorm_cl_apply(reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()), dyp, reinterpret_cast<__nv_bfloat16*>(out.data_ptr()),
-                                fp(w), fp(b), sums.data_ptr<float>(), fp(stats), static_cast<int>(B), static_cast<int>(C), T, count,
+                                f32_ptr(w), f32_ptr(b), sums.data_ptr<float>(), f32_ptr(stats), static_cast<int>(B), static_cast<int>(C), T, count,
                                 static_cast<float>(eps), static_cast<int>(act), static_cast<int>(mode), cur_stream(), ex ? &xc : nullptr),
              "inorm_cl_apply");
 }

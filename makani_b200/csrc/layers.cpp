@@ -27,7 +27,12 @@ Tensor zeros_f32(at::IntArrayRef shape, const Tensor& like) { return at::zeros(s
 Tensor empty_f32(at::IntArrayRef shape, const Tensor& like) { return at::empty(shape, like.options().dtype(at::kFloat)); }
 Tensor value(const OptTensor& t) { return t.has_value() ? *t : Tensor(); }
 OptTensor maybe(const Tensor& t) { return t.defined() ? OptTensor(t) : OptTensor(); }
-Tensor as_f32(const OptTensor& t) { return t.has_value() && t->defined() ? t->detach().to(at::kFloat).contiguous() : Tensor(); }
+// (a parameter on the host or another GPU is refused: its address would reach a kernel, or its copy be paid for on every call)
+Tensor as_f32(const OptTensor& t, const Tensor& like) {
+  if (!t.has_value() || !t->defined()) return Tensor();
+  MK_CHECK(t->device() == like.device(), "layers: tensors must be on one CUDA device");
+  return t->detach().to(at::kFloat).contiguous();
+}
 
 // ------------------------------------------------------------------------------------------ pointwise convolutions and linear layers
 
@@ -80,9 +85,10 @@ mkh::Operand channel_rows(const Act& x) {
 
 // fp32 [Co, Ci(, 1, 1)] -> bf16 [Co, pad8(Ci)]
 Tensor prep_weight(const Tensor& w, const Tensor& like) {
+  MK_CHECK(w.device() == like.device(), "layers: tensors must be on one CUDA device");
   const Tensor w2 = w.detach().reshape({w.size(0), -1});
   const int64_t co = w2.size(0), ci = w2.size(1), pitch = (ci + 7) / 8 * 8;
-  if (w2.is_cuda() && w2.scalar_type() == at::kFloat && w2.is_contiguous()) {
+  if (w2.scalar_type() == at::kFloat && w2.is_contiguous()) {
     Tensor out = at::empty({co, pitch}, like.options());
     ++mkh::launches();
     mkh::check(mk::cast_pad_bf16(w2.data_ptr<float>(), bf_mut(out), co, static_cast<int>(ci), static_cast<int>(pitch), mkh::stream()), "cast_pad");
@@ -197,7 +203,7 @@ bool out_cl(int64_t layout, const Tensor& resid, int64_t co) {
 std::tuple<Tensor, Tensor, OptTensor> conv_forward(const Tensor& x, const Tensor& w, const OptTensor& bias, const OptTensor& resid, int64_t act,
                                                    int64_t layout, bool want_pre) {
   c10::cuda::CUDAGuard guard(x.device());
-  const Tensor wq = prep_weight(w, x), b = as_f32(bias), r = value(resid);
+  const Tensor wq = prep_weight(w, x), b = as_f32(bias, x), r = value(resid);
   Tensor pre;
   const Act y = forward(act_of(x), wq, w.size(1), b, static_cast<int>(act), r, want_pre ? &pre : nullptr, false, out_cl(layout, r, w.size(0)));
   return {y.t, wq, maybe(pre)};
@@ -218,7 +224,7 @@ std::tuple<OptTensor, OptTensor, OptTensor> conv_backward(const Tensor& dy, cons
 std::tuple<Tensor, Tensor, Tensor, OptTensor, OptTensor> mlp_forward(const Tensor& x, const Tensor& w1, const OptTensor& b1, const Tensor& w2,
                                                                      const OptTensor& b2, const OptTensor& resid, int64_t layout, bool train) {
   c10::cuda::CUDAGuard guard(x.device());
-  const Tensor w1q = prep_weight(w1, x), w2q = prep_weight(w2, x), b1f = as_f32(b1), b2f = as_f32(b2), r = value(resid);
+  const Tensor w1q = prep_weight(w1, x), w2q = prep_weight(w2, x), b1f = as_f32(b1, x), b2f = as_f32(b2, x), r = value(resid);
   const int64_t ch = w1.size(0);
   Tensor dact;
   const Act h = forward(act_of(x), w1q, w1.size(1), b1f, mkh::ACT_GELU, Tensor(), train ? &dact : nullptr, train, default_cl(ch));
@@ -248,7 +254,7 @@ std::tuple<Tensor, Tensor, OptTensor, OptTensor> norm_forward(const Tensor& x, c
   c10::cuda::CUDAGuard guard(x.device());
   const int64_t B = x.size(0), C = x.size(1), T = x.size(2) * x.size(3);
   Tensor y = at::empty_like(x), sums = zeros_f32({B, C, 2}, x), stats = empty_f32({B, C, 2}, x);
-  const Tensor w = as_f32(weight), b = as_f32(bias);
+  const Tensor w = as_f32(weight, x), b = as_f32(bias, x);
   MK_CHECK((!w.defined() || w.numel() == C) && (!b.defined() || b.numel() == C), "norm_forward: one weight and bias per channel expected");
   mkh::launches() += 2;
   // statistics local to this device are accumulated around the first token (mode bit 1): no cancellation in E[x^2] - E[x]^2 for
@@ -540,7 +546,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor> afno_forward(const Te
   const int64_t nb = p.nb, bs = p.bs, hid = w1.size(3);
   MK_CHECK(nb <= 32767, "afno_forward: at most 32767 blocks");
   const Tensor w[2] = {w1.detach().to(at::kFloat).contiguous(), w2.detach().to(at::kFloat).contiguous()};
-  const Tensor b[2] = {as_f32(b1), as_f32(b2)};
+  const Tensor b[2] = {as_f32(b1, x), as_f32(b2, x)};
   Tensor wq[2], bq[2];
   mk::AfnoLayer l[2];
   for (int k = 0; k < 2; ++k) {

@@ -684,3 +684,33 @@ def test_folded_transforms(b, h, w, mmax, c):
     for got, ref in pairs:
         assert got.shape == ref.shape and _rel(got, ref) < BF16
     _ext.check_device_errors(dev)
+
+
+@pytest.mark.parametrize("what", ["conv_weight", "conv_bias", "conv_residual", "mlp_weight", "linear_weight", "linear_bias", "token_mlp_weight",
+                                  "norm_weight_cl", "norm_bias_cl", "norm_weight_nchw", "afno_weight", "afno_bias"])
+def test_host_tensors_beside_cuda_activations_are_refused(what):
+    from makani_b200.ops.afno import afno_filter_stacked
+    from makani_b200.ops.conv import conv1x1, mlp2
+    from makani_b200.ops.linear import linear_lastdim, mlp2_lastdim
+    from makani_b200.ops.norm import instance_norm
+    dev = _dev()
+    x = torch.randn(1, 16, 8, 16, device=dev).bfloat16().contiguous(memory_format=torch.channels_last)
+    tok = torch.randn(32, 16, device=dev).bfloat16()
+    on = lambda *shape, host=False: torch.randn(*shape, device="cpu" if host else dev)  # noqa: E731
+    planes = torch.randn(1, 8, 8, 16, device=dev).bfloat16()
+    calls = {
+        "conv_weight": lambda: conv1x1(x, on(16, 16, 1, 1, host=True)),
+        "conv_bias": lambda: conv1x1(x, on(16, 16, 1, 1), on(16, host=True)),
+        "conv_residual": lambda: conv1x1(x, on(16, 16, 1, 1), None, x.cpu()),
+        "mlp_weight": lambda: mlp2(x, on(32, 16, 1, 1), on(32), on(16, 32, 1, 1, host=True), on(16)),
+        "linear_weight": lambda: linear_lastdim(tok, on(16, 16, host=True)),
+        "linear_bias": lambda: linear_lastdim(tok, on(16, 16), on(16, host=True)),
+        "token_mlp_weight": lambda: mlp2_lastdim(tok, on(32, 16, host=True), on(32), on(16, 32), on(16)),
+        "norm_weight_cl": lambda: instance_norm(x, on(16, host=True), on(16)),
+        "norm_bias_cl": lambda: instance_norm(x, on(16), on(16, host=True)),
+        "norm_weight_nchw": lambda: instance_norm(x.contiguous(), on(16, host=True), on(16)),
+        "afno_weight": lambda: afno_filter_stacked(planes, on(2, 2, 8, 8, host=True), None, on(2, 2, 8, 8), None, (0, 1, 7), 3, 0.0),
+        "afno_bias": lambda: afno_filter_stacked(planes, on(2, 2, 8, 8), on(2, 2, 8, host=True), on(2, 2, 8, 8), None, (0, 1, 7), 3, 0.0),
+    }
+    with pytest.raises(RuntimeError):
+        calls[what]()
