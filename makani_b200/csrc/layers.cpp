@@ -83,10 +83,11 @@ mkh::Operand channel_rows(const Act& x) {
   return x.cl ? mkh::Operand{&x.t, x.C, true, 0, x.T * x.C, 0} : mkh::Operand{&x.t, x.T, false, 0, x.C * x.T, 0};
 }
 
-// fp32 [Co, Ci(, 1, 1)] -> bf16 [Co, pad8(Ci)]
+// fp32 [Co, Ci(, 1, 1)] -> bf16 [Co, pad8(Ci)]; bf16 weights of a linear layer as they are
 Tensor prep_weight(const Tensor& w, const Tensor& like) {
   MK_CHECK(w.device() == like.device(), "layers: tensors must be on one CUDA device");
   const Tensor w2 = w.detach().reshape({w.size(0), -1});
+  if (like.dim() == 2 && w.dim() == 2 && w2.scalar_type() == like.scalar_type() && w2.size(1) % 8 == 0) return w2.contiguous();
   const int64_t co = w2.size(0), ci = w2.size(1), pitch = (ci + 7) / 8 * 8;
   if (w2.scalar_type() == at::kFloat && w2.is_contiguous()) {
     Tensor out = at::empty({co, pitch}, like.options());

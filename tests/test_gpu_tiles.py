@@ -714,3 +714,12 @@ def test_host_tensors_beside_cuda_activations_are_refused(what):
     }
     with pytest.raises(RuntimeError):
         calls[what]()
+
+
+def test_bf16_weights_of_linear_layers_are_not_copied():
+    dev = _dev()
+    x, w = torch.randn(64, 24, device=dev).bfloat16(), torch.randn(16, 24, device=dev).bfloat16()
+    y, wq, _ = _ext.require().conv_forward(x, w, None, None, 0, -1, False)
+    assert wq.data_ptr() == w.data_ptr() and _rel(y, x.double() @ w.double().t()) < BF16
+    wt = torch.randn(24, 16, device=dev).bfloat16().t()      # strided: a copy, as ever
+    assert _rel(_ext.require().conv_forward(x, wt, None, None, 0, -1, False)[0], x.double() @ wt.double().t()) < BF16
