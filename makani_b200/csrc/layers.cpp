@@ -409,7 +409,11 @@ std::tuple<Tensor, OptTensor, Tensor> spectral_forward(const Tensor& x, const Te
   const Plan pi(in, in_n), po(out, out_n);
   MK_CHECK(wx.dim() == 4 && wx.size(3) == x.size(1) && wx.size(0) == in[2].size(1), "spectral_forward: the weights do not match the field");
   const Tensor t2 = legendre_analysis(analyse(x, pi, true), in[2], false);
-  const Tensor y = synthesise(legendre_synthesis(contract(t2, wx, false, Tensor()), false, out[3], po.nlat), po, false);
+  Tensor t3 = contract(t2, wx, false, Tensor());
+  Tensor t4 = legendre_synthesis(t3, false, out[3], po.nlat);
+  t3.reset();
+  const Tensor y = synthesise(t4, po, false);
+  t4.reset();
   Tensor r;
   if (want_resid) r = synthesise(legendre_synthesis(t2, true, out[3], po.nlat), po, false);
   return {y, maybe(r), t2};

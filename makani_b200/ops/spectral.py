@@ -385,6 +385,45 @@ def fold_weight_grad(dwx: torch.Tensor) -> torch.Tensor:
 # ------------------------------------------------------------------------------------------------ autograd
 
 
+def forward_stages(x, wx, plan_in: SHTPlan, plan_out: SHTPlan, want_resid: bool):
+    """(y, r or None, T2), launch by launch: the pass on the CPU, and what `spectral_forward` of csrc/layers.cpp does on the GPU."""
+    t1 = analyse(x, plan_in)
+    t2 = legendre_analysis(t1, plan_in.pw)
+    del t1
+    t3 = contract(t2, wx, False)
+    t4 = legendre_synthesis(t3, False, plan_out.p, plan_out.nlat)
+    del t3
+    y = synthesise(t4, plan_out)
+    del t4
+    r = None
+    if want_resid:
+        t4r = legendre_synthesis(t2, True, plan_out.p, plan_out.nlat)
+        r = synthesise(t4r, plan_out)
+    return y, r, t2
+
+
+def backward_stages(dy, dr, t2, wx, plan_in: SHTPlan, plan_out: SHTPlan, need_x: bool, need_w: bool):
+    """(dx, dw) as `spectral_backward` of csrc/layers.cpp has them on the GPU; dr: the gradient of the residual, or None."""
+    # adjoint of the inverse DFT / synthesis on the output grid
+    dt4 = analyse(dy, plan_out, forward=False)
+    dt3 = legendre_analysis(dt4, plan_out.p)                       # [B, l, m, (ri, o)]
+    del dt4
+    dw = fold_weight_grad2(contract_wgrad2(dt3, t2)) if need_w else None
+    dx = None
+    if need_x:
+        dr2 = None
+        if dr is not None:
+            # laid out by order, as the contraction writes: its epilogue adds the residual's share
+            dr4 = analyse(dr, plan_out, forward=False)
+            dr2 = legendre_analysis(dr4, plan_out.p, by_order=True)
+            del dr4
+        dt2 = contract(dt3, wx, True, resid=dr2)                   # [B, m, l, (ri, c)]
+        del dr2
+        dt1 = legendre_synthesis(dt2, False, plan_in.pw, plan_in.nlat)
+        dx = synthesise(dt1, plan_in, forward=True)
+    return dx, dw
+
+
 class _SpectralConv(torch.autograd.Function):
     """y = iSHT_out(W . SHT_in(x)) and, when `want_resid`, r = iSHT_out(SHT_in(x)) (regridded residual).
     Input and outputs are channels-last."""
@@ -398,55 +437,23 @@ class _SpectralConv(torch.autograd.Function):
         ctx.wshape = w.shape
         if x.is_cuda:
             y, r, t2 = _ext.require().spectral_forward(x, wx, *plan_in.native, *plan_out.native, want_resid)
-            ctx.save_for_backward(t2, wx)
-            return (y, r) if want_resid else y
-        t1 = analyse(x, plan_in)
-        t2 = legendre_analysis(t1, plan_in.pw)
-        del t1
-        t3 = contract(t2, wx, False)
-        t4 = legendre_synthesis(t3, False, plan_out.p, plan_out.nlat)
-        del t3
-        y = synthesise(t4, plan_out)
-        del t4
-        r = None
-        if want_resid:
-            t4r = legendre_synthesis(t2, True, plan_out.p, plan_out.nlat)
-            r = synthesise(t4r, plan_out)
+        else:
+            y, r, t2 = forward_stages(x, wx, plan_in, plan_out, want_resid)
         ctx.save_for_backward(t2, wx)
-        if want_resid:
-            return y, r
-        return y
+        return (y, r) if want_resid else y
 
     @staticmethod
     def backward(ctx, dy, dr=None):
         t2, wx = ctx.saved_tensors
         plan_in, plan_out = ctx.plans
         dy = _to_cl(dy)
+        dr = _to_cl(dr) if ctx.want_resid and dr is not None else None
         if dy.is_cuda:
-            dr = _to_cl(dr) if ctx.want_resid and dr is not None else None
             dx, dw = _ext.require().spectral_backward(dy, dr, t2, wx, *plan_in.native, *plan_out.native, ctx.needs_input_grad[0],
                                                       ctx.needs_input_grad[1])
-            return dx, (None if dw is None else dw.reshape(ctx.wshape)), None, None, None, None
-        # adjoint of the inverse DFT / synthesis on the output grid
-        dt4 = analyse(dy, plan_out, forward=False)
-        dt3 = legendre_analysis(dt4, plan_out.p)                       # [B, l, m, (ri, o)]
-        del dt4
-        dw = None
-        if ctx.needs_input_grad[1]:
-            dw = fold_weight_grad2(contract_wgrad2(dt3, t2)).reshape(ctx.wshape)
-        dx = None
-        if ctx.needs_input_grad[0]:
-            dr2 = None
-            if ctx.want_resid and dr is not None:
-                # laid out by order, as the contraction writes: its epilogue adds the residual's share
-                dr4 = analyse(_to_cl(dr), plan_out, forward=False)
-                dr2 = legendre_analysis(dr4, plan_out.p, by_order=True)
-                del dr4
-            dt2 = contract(dt3, wx, True, resid=dr2)                   # [B, m, l, (ri, c)]
-            del dr2
-            dt1 = legendre_synthesis(dt2, False, plan_in.pw, plan_in.nlat)
-            dx = synthesise(dt1, plan_in, forward=True)
-        return dx, dw, None, None, None, None
+        else:
+            dx, dw = backward_stages(dy, dr, t2, wx, plan_in, plan_out, ctx.needs_input_grad[0], ctx.needs_input_grad[1])
+        return dx, (None if dw is None else dw.reshape(ctx.wshape)), None, None, None, None
 
 
 def spectral_conv_supported(x: torch.Tensor, w: torch.Tensor) -> bool:
