@@ -50,9 +50,8 @@ class SHTPlan:
         theta, wq = precompute_latitudes(nlat, grid)
         self.theta, self.wq = theta, wq
         p = legendre_table(mmax, lmax, theta)                     # [m, l, k] float64
-        pw = p * wq[None, None, :]
         tab = np.zeros((2, mmax, lmax, self.hp), dtype=np.float32)
-        tab[0, :, :, :nlat] = pw
+        np.multiply(p, wq, out=tab[0, :, :, :nlat], casting="same_kind")
         tab[1, :, :, :nlat] = p
         self.pw = torch.from_numpy(tab[0]).to(self.device, dtype).contiguous()   # analysis table (weighted)
         self.p = torch.from_numpy(tab[1]).to(self.device, dtype).contiguous()    # synthesis table
@@ -60,21 +59,22 @@ class SHTPlan:
         phi = 2.0 * np.pi * np.arange(nlon) / nlon
         m = np.arange(mmax)[:, None]
         ang = m * phi[None, :]
-        f = np.zeros((self.k2, nlon), dtype=np.float64)
-        f[0::2] = np.cos(ang) * (2.0 * np.pi / nlon)
-        f[1::2] = -np.sin(ang) * (2.0 * np.pi / nlon)
-        self.f = torch.from_numpy(f.astype(np.float32)).to(self.device, dtype).contiguous()      # [(m,ri), W]
+        cos, sin = np.cos(ang), np.sin(ang)
+        f = np.empty((self.k2, nlon), dtype=np.float32)
+        f[0::2] = cos * (2.0 * np.pi / nlon)
+        f[1::2] = -sin * (2.0 * np.pi / nlon)
+        self.f = torch.from_numpy(f).to(self.device, dtype).contiguous()      # [(m,ri), W]
         # inverse DFT: x_i = sum_m c_m (Xr cos - Xi sin); c_0 = 1, c_m = 2, Nyquist (if kept) = 1
         cm = np.full((mmax, 1), 2.0)
         cm[0] = 1.0
         if nlon % 2 == 0 and mmax > nlon // 2:
             cm[nlon // 2] = 1.0
-        g = np.zeros((nlon, self.k2p), dtype=np.float64)
-        g[:, 0:self.k2:2] = (cm * np.cos(ang)).T
-        g[:, 1:self.k2:2] = (-cm * np.sin(ang)).T
-        self.gt = torch.from_numpy(g.astype(np.float32)).to(self.device, dtype).contiguous()     # [W, (m,ri) padded]
+        g = np.zeros((nlon, self.k2p), dtype=np.float32)
+        g[:, 0:self.k2:2] = (cm * cos).T
+        g[:, 1:self.k2:2] = (-cm * sin).T
+        self.gt = torch.from_numpy(g).to(self.device, dtype).contiguous()     # [W, (m,ri) padded]
 
-        # The same matrices with their columns in two halves, for `gemm_fold`: (synthesis, forward) -> table.  The synthesis (rows are
+        # The same matrices with their columns in two halves, for `gemm_fold`.  The synthesis (rows are
         # longitudes) folds from the 64 rows on that `gemm_fold` asks for.  The analysis (rows (m, ri)) only saves work where most
         # orders up to half the points are kept, order m sharing its products with order W / 2 - m.  us, whole / folded:
         #   synthesis, 384 channels: 721 x 1440, 241 orders 430 / 336; 240 x 480, 241 60 / 49; 360 x 720, 361 157 / 132;
@@ -85,48 +85,50 @@ class SHTPlan:
         self.folds_synthesis = nlon >= 64
         self.folds_analysis = (nlon >= 64 and nlon % 2 == 0 and 8 * mmax > 3 * nlon and
                                nlon // 2 + 32 <= 2 * mmax <= nlon + 2)
-        self._folded = {(syn, fwd): self._fold_table(syn, fwd) for fwd in (True, False) for syn in (True, False)
-                        if (self.folds_synthesis if syn else self.folds_analysis)}
+        self._folded = self._fold_tables()
 
         # what the native passes take: matrices (empty where one is not folded) and extents
         none = torch.empty(0, device=self.device, dtype=dtype)
         self.native = ([self.f, self.gt, self.pw, self.p] + [self._folded.get((syn, fwd), none) for syn in (True, False) for fwd in (True, False)],
                        [nlat, nlon, lmax, mmax])
 
-    def _fold_table(self, synthesis: bool, forward: bool) -> torch.Tensor:
-        """The inverse transform's matrix (`synthesis`; rows are longitudes, halves the cosine and sine terms) or the forward one's
-        (rows (m, ri), halves the even and odd points), from the coefficients of the forward transform (`forward`) or of the
-        inverse one.  Symmetric to the bit: a row and its mirror hold the same numbers, and those that cancel are zero.  The halves
-        start on 128-byte boundaries, so that a TMA row is one line (721 x 1440: 364 -> 336 us)."""
+    def _fold_tables(self) -> Dict[Tuple[bool, bool], torch.Tensor]:
+        """(synthesis, forward) -> the inverse transform's matrix (`synthesis`; rows are longitudes, halves the cosine and sine terms)
+        or the forward one's (rows (m, ri), halves the even and odd points), from the coefficients of the forward transform
+        (`forward`) or of the inverse one.  Symmetric to the bit: a row and its mirror hold the same numbers, and those that cancel
+        are zero.  The halves start on 128-byte boundaries, so that a TMA row is one line (721 x 1440: 364 -> 336 us)."""
         W, mmax = self.nlon, self.mmax
-        ang = 2.0 * np.pi * ((np.arange(mmax)[:, None] * np.arange(W)[None, :]) % W) / W
-        scale = np.full((mmax, 1), 2.0 * np.pi / W if forward else 2.0)
-        if not forward:
-            scale[0] = 1.0
-            if W % 2 == 0 and mmax > W // 2:
-                scale[W // 2] = 1.0
-        c, s = scale * np.cos(ang), -scale * np.sin(ang)              # [m, i]
-        h = W // 2
-        if synthesis:
-            i = np.arange(h + 1, W)
-            c[:, i], s[:, i] = c[:, W - i], -s[:, W - i]
-            s[:, 0] = 0.0
-            if W % 2 == 0:
-                s[:, h] = 0.0
-            t = np.zeros((W, 2, pad_to(mmax, 64)), dtype=np.float32)
-            t[:, 0, :mmax], t[:, 1, :mmax] = c.T, s.T
-        else:
-            if h % 2 == 0 and h // 2 < mmax:
-                c[h // 2, 1::2] = 0.0
-                s[h // 2, 0::2] = 0.0
-            m = np.arange(h // 2 + 1, mmax)
-            sign = np.where(np.arange(W) % 2 == 0, 1.0, -1.0)[None, :]
-            c[m], s[m] = sign * c[h - m], -sign * s[h - m]
-            t = np.zeros((mmax, 2, 2, pad_to(h, 64)), dtype=np.float32)                  # [m, ri, half, point]
-            for ri, x in enumerate((c, s)):
-                t[:, ri, 0, :h], t[:, ri, 1, :h] = x[:, 0::2], x[:, 1::2]
-        t = t.reshape(-1, 2 * t.shape[-1])
-        return torch.from_numpy(t).to(self.device, self.dtype).contiguous()
+        if not (self.folds_synthesis or self.folds_analysis):
+            return {}
+        h, angle = W // 2, 2.0 * np.pi * np.arange(W) / W
+        at = np.arange(mmax)[:, None] * np.arange(W)[None, :] % W
+        cos, sin = np.cos(angle)[at], np.sin(angle)[at]              # [m, i]
+        tables = {}
+        for forward in (True, False):
+            scale = np.full((mmax, 1), 2.0 * np.pi / W if forward else 2.0)
+            if not forward:
+                scale[0] = 1.0
+                if W % 2 == 0 and mmax > W // 2:
+                    scale[W // 2] = 1.0
+            c, s = scale * cos, -scale * sin
+            if self.folds_synthesis:
+                t = np.zeros((W, 2, pad_to(mmax, 64)), dtype=np.float32)
+                t[:, 0, :mmax], t[:, 1, :mmax] = c.T, s.T
+                t[h + 1:, 0], t[h + 1:, 1] = t[W - h - 1:0:-1, 0], -t[W - h - 1:0:-1, 1]
+                t[0, 1] = 0.0
+                if W % 2 == 0:
+                    t[h, 1] = 0.0
+                tables[True, forward] = t
+            if self.folds_analysis:
+                t = np.zeros((mmax, 2, 2, pad_to(h, 64)), dtype=np.float32)                  # [m, ri, half, point]
+                for ri, x in enumerate((c, s)):
+                    t[:, ri, 0, :h], t[:, ri, 1, :h] = x[:, 0::2], x[:, 1::2]
+                if h % 2 == 0 and h // 2 < mmax:
+                    t[h // 2, 0, 1] = t[h // 2, 1, 0] = 0.0
+                m = np.arange(h // 2 + 1, mmax)
+                t[m] = t[h - m] * np.array([[1.0, -1.0], [-1.0, 1.0]], dtype=np.float32)[:, :, None]
+                tables[False, forward] = t.reshape(2 * mmax, 2, -1)
+        return {k: torch.from_numpy(t.reshape(t.shape[0], -1)).to(self.device, self.dtype).contiguous() for k, t in tables.items()}
 
     @classmethod
     def get(cls, nlat, nlon, lmax, mmax, grid, device, dtype=torch.bfloat16) -> "SHTPlan":
