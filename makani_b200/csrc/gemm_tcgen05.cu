@@ -129,7 +129,7 @@ struct KParams {
   FastDiv dv_n, dv_m, dv_split, dv_zlo;
   uint32_t total_tiles;           // below 2^31
   int a_part;                     // k coordinate of the second part of a K-major A (complex and folded products)
-  int mirror, m_half, fold_rows;  // folded products: rows r and mirror - r; rows past m_half are the mirrors' business
+  int mirror, fold_rows;          // folded products: rows r < M and mirror - r, which are the rows M to fold_rows
   int cplx, nth, neg_half, neg_seg;   // complex product: mode, column tiles per half, the negative (half, segment)
   int stages, e_tma;
   int d_zlo_on, d_zhi_on;         // fp32 output through TMA: 0 where all batches of that index add into one output
@@ -946,7 +946,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
         const int nb = n0 + half * 64;
         const uint32_t box_off = stg_off + (warp - 2) * stg_warp_bytes(6);
         const int r0 = c.mt * BM + q * 32;
-        const bool any = nb < p.N && r0 <= p.m_half;      // uniform across the warp
+        const bool any = nb < p.N && r0 < p.M;      // uniform across the warp
         const bool pairs = p.cplx == 5;
         if (any) {
           const uint32_t taddr = tmem_base + buf * ACC_COLS + half * 64 + (static_cast<uint32_t>(q * 32) << 16);
@@ -989,13 +989,23 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
         if (any) {
           fence_async_smem();
           __syncwarp();
-          // Row 0 has its mirror past the end where that is no row (clipped).  Past m_half the sums are the mirrors of earlier rows'
-          // differences, bit for bit (the tables are symmetric to the bit), so the last box may store both.
+          // Every row leaves once: sums up to row M (clipped by their tensor map), differences from there on.  Row 0 has its mirror
+          // past the end where that is no row (clipped).  The last box of differences may begin before row M, which no tensor map
+          // clips: one box of the W / 64 takes the ordinary path.
+          const int m0 = p.mirror - r0 - (pairs ? 30 : 31);
           if (elect_one()) {
             tma_store_tile(&map_d, smem_base + box_off, nb, 0, r0, c.zlo, c.zhi);
-            const int m0 = p.mirror - r0 - (pairs ? 30 : 31);
-            if (m0 < p.fold_rows) tma_store_tile(&map_d, smem_base + box_off + 32 * 128, nb, 0, m0, c.zlo, c.zhi);
+            if (m0 >= p.M && m0 < p.fold_rows) tma_store_tile(&map_p, smem_base + box_off + 32 * 128, nb, 0, m0, c.zlo, c.zhi);
             tma_store_commit();
+          }
+          if (m0 < p.M) {
+            __nv_bfloat16* const out = static_cast<__nv_bfloat16*>(p.D) + c.zhi * p.d_zhi;
+            for (int i = lane; i < 32 * 8; i += 32) {
+              const int j = i >> 3, row = m0 + j, col = nb + (i & 7) * 8;
+              if (row < p.M || row >= p.fold_rows || col >= p.N) continue;
+              *reinterpret_cast<uint4*>(out + row * p.rs_lo + col) =
+                  *reinterpret_cast<const uint4*>(smem + box_off + (32 + j) * 128 + (((i ^ j) & 7) << 4));
+            }
           }
         }
         continue;
@@ -1912,13 +1922,13 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
   const bool plain = (one_stride || split_ok) && (e.ndiv <= 0 || e.ndiv >= (1 << 30));
   const int rd = one_stride ? 1 : e.rdiv;
   const bool folded = p.cplx == 4 || p.cplx == 5;
-  auto tile_map = [&](CUtensorMap* m, const void* ptr, int box_rows) {
-    return make_map_e(m, ptr, folded ? p.rows : p.M, p.N, rd, e.rs_hi, e.rs_lo, e.d_zlo, e.d_zhi, p.zlo_n, p.zhi_n, box_rows, 2, e.d_half);
+  auto tile_map = [&](CUtensorMap* m, const void* ptr, int box_rows, int rows_of) {
+    return make_map_e(m, ptr, rows_of, p.N, rd, e.rs_hi, e.rs_lo, e.d_zlo, e.d_zhi, p.zlo_n, p.zhi_n, box_rows, 2, e.d_half);
   };
   kp.rd_shift = 0;
   while (plain && (1 << kp.rd_shift) < rd) ++kp.rd_shift;
   if (e.resid && !e.out_f32 && plain && kp.vec_ok && e.d_zlo >= 0 && e.d_zhi >= 0) {
-    if (tile_map(&me, e.resid, BM)) kp.e_tma = 1;
+    if (tile_map(&me, e.resid, BM, p.M)) kp.e_tma = 1;
   }
   // A specialised epilogue (TMA stores of bf16 tiles) when the launch fits one.
   int epi = 0;
@@ -1935,12 +1945,13 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
     else if (e.resid && kp.e_tma && !e.preact && e.act == 0) epi = 3;
     else if (e.resid && kp.e_tma && !e.preact && (e.act == 2 || e.act == 4 || e.act == 6 || e.act == 8)) epi = 4;
     if (epi != 0) {
-      bool ok = tile_map(&md, e.D, 32);
-      if (ok && epi == 2) ok = tile_map(&mp, e.preact, 32);
+      bool ok = tile_map(&md, e.D, 32, p.M);
+      if (ok && epi == 2) ok = tile_map(&mp, e.preact, 32, p.M);
+      if (ok && epi == 6) ok = tile_map(&mp, e.D, 32, p.rows);      // the mirror rows
       if (ok && kp.ndx > 0) {
         if (epi != 1) ok = false;   // replicated output goes through the plain-store epilogue or the generic one
         for (int q = 0; ok && q < kp.ndx; ++q)
-          ok = tile_map(&mdx.m[q], kp.Dx[q], 32);
+          ok = tile_map(&mdx.m[q], kp.Dx[q], 32, p.M);
       }
       if (!ok) epi = 0;
     }
@@ -1992,6 +2003,7 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
     // (from 64 rows on the mirror rows' boxes start at or after row 0, and the last box of sums ends inside the table; the computed
     // rows and their mirrors make up all rows, or some would stay unwritten)
     if (epi != 6 || kp.splits != 1 || p.splits == 0 || kp.nseg != 1 || rd != 1 || A.mn_major || p.mirror < 64 || (p.a_plane % 8) != 0 ||
+        (p.N % 8) != 0 ||
         p.M != (p.cplx == 5 ? 2 * (p.mirror / 4 + 1) : p.mirror / 2 + 1) || p.rows < p.mirror / 2 + 32 ||
         p.rows > p.mirror + (p.cplx == 5 ? 2 : 0) || p.zlo_n != 1) {
       snprintf(g_err, sizeof(g_err), "folded product: bf16, K-major tables, plain aligned rows, at least 64 of them, each computed or a mirror");
@@ -1999,7 +2011,6 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
     }
     kp.a_part = static_cast<int>(p.a_plane);
     kp.mirror = p.mirror;
-    kp.m_half = p.mirror / 2;
     kp.fold_rows = p.rows;
   } else if (p.cplx) {
     if (eb != 2 || (epi != 1 && epi != 3 && epi != 5) || kp.splits != 1 || p.splits == 0 || kp.nseg != 1 || rd != 1) {
@@ -2066,7 +2077,7 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
   if (!kp.e_tma) me = ma;   // unused, but must be a valid descriptor
 
   if (epi == 0) md = ma;       // unused maps must be valid descriptors all the same
-  if (epi != 2) mp = ma;
+  if (epi != 2 && epi != 6) mp = ma;
   for (int q = (epi == 1 ? kp.ndx : 0); q < MAX_SEG - 1; ++q) mdx.m[q] = ma;
   if (epi == 6)
     return cg == 2 ? launch_t<128, 2, 6, 2>(ma, mbs, me, md, mp, mdx, kp, stream) : launch_t<128, 2, 6, 1>(ma, mbs, me, md, mp, mdx, kp, stream);

@@ -297,7 +297,7 @@ def gemm_fold(rows: int, M: int, N: int, K: int, mirror: int, pairs: bool, table
     """Product with a table whose rows r and mirror - r differ only in the sign of one half of their columns (bf16 on CUDA):
 
         P(s)[r, n] = sum_k table[r, s part + k] B(s)[n, k],   s = 0, 1, r < M
-        D[r] = P(0)[r] + P(1)[r],   D[mirror - r] = P(0)[r] - P(1)[r],   both where they are one of the `rows` rows of D
+        D[r] = P(0)[r] + P(1)[r],   D[mirror - r] = P(0)[r] - P(1)[r]   where that is one of the rows from M up to `rows`
 
     With `pairs` the rows are (order, re / im) pairs: row 2 m + ri has its mirror at mirror - 2 m + ri, and the imaginary one its
     sign changed.  `M` rows cover one half and its middle, all that are not mirrors of others, and `rows` end with the mirrors of
@@ -316,8 +316,8 @@ def gemm_fold(rows: int, M: int, N: int, K: int, mirror: int, pairs: bool, table
         sign = torch.where((r % 2 == 1) & pairs, -1.0, 1.0).to(cdt).view(1, -1, 1)
         z = torch.arange(zhi_n).view(-1, 1, 1)
         n = torch.arange(N).view(1, 1, -1)
-        for row, val in ((r, acc[0] + acc[1]), (mirror - r + (2 * (r % 2) if pairs else 0), (acc[0] - acc[1]) * sign)):
-            keep = (row >= 0) & (row < rows)
+        for first, row, val in ((0, r, acc[0] + acc[1]), (M, mirror - r + (2 * (r % 2) if pairs else 0), (acc[0] - acc[1]) * sign)):
+            keep = (row >= first) & (row < rows)
             idx = D.offset + z * D.d_zhi + row[keep].view(1, -1, 1) * D.rs_lo + n
             fd.index_put_((idx.reshape(-1),), val[:, keep].to(fd.dtype).reshape(-1))
         return

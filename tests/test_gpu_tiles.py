@@ -723,3 +723,37 @@ def test_bf16_weights_of_linear_layers_are_not_copied():
     assert wq.data_ptr() == w.data_ptr() and _rel(y, x.double() @ w.double().t()) < BF16
     wt = torch.randn(24, 16, device=dev).bfloat16().t()      # strided: a copy, as ever
     assert _rel(_ext.require().conv_forward(x, wt, None, None, 0, -1, False)[0], x.double() @ wt.double().t()) < BF16
+
+
+@pytest.mark.parametrize("rows,mirror,pairs,n,k,z", [
+    (64, 64, False, 8, 16, 3),           # the last box of sums holds one row
+    (65, 65, False, 72, 40, 2),          # no row is its own mirror
+    (90, 90, False, 136, 46, 2),
+    (126, 126, False, 264, 8, 1),        # the computed rows end with a box
+    (480, 480, False, 384, 241, 5),      # CTA pairs
+    (66, 64, True, 16, 32, 2),           # all orders
+    (64, 64, True, 8, 32, 1),            # all but the last
+    (92, 90, True, 72, 45, 3),           # an odd number of points in each half
+    (450, 480, True, 136, 240, 2),
+])
+def test_folded_products_write_every_row_once(rows, mirror, pairs, n, k, z):
+    """Rows past the middle are differences of the rows before it, whatever the table holds there: each row is written once."""
+    from makani_b200.ops.gemm import gemm_fold, pad_to
+    dev = _dev()
+    g = torch.Generator().manual_seed(rows + n)
+    m, part = (2 * (mirror // 4 + 1) if pairs else mirror // 2 + 1), pad_to(k, 64)
+    table = torch.randint(-1, 2, (rows, 2 * part), generator=g).float()
+    table[m:] = 97.0
+    b = torch.randint(-1, 2, (z, k, 2, n), generator=g).float()
+    b[:, :, :, ::3] = 0.0      # columns of zeros
+    out = []
+    for d in ("cpu", dev, dev, dev):
+        dt = torch.float32 if d == "cpu" else torch.bfloat16
+        y = torch.full((z, rows, n), float("nan"), device=d, dtype=dt)
+        gemm_fold(rows, m, n, k, mirror, pairs, table.to(d, dt), part, Operand(b.to(d, dt), ld=2 * n, mn_major=True, zs_hi=k * 2 * n), n,
+                  Output(y, rs_lo=n, d_zhi=rows * n), zhi_n=z)
+        out.append(y)
+    # whole numbers: the products and sums are exact, the results rounded once
+    assert torch.equal(out[1].cpu(), out[0].to(torch.bfloat16))
+    assert all(torch.equal(y.view(torch.int16), out[1].view(torch.int16)) for y in out[2:])
+    _ext.check_device_errors(dev)
