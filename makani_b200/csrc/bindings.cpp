@@ -500,20 +500,6 @@ void spectral_planes(const Tensor& w, Tensor& wp) {
              "spectral_planes");
 }
 
-// sums of do2 [outer, groups, inner, C] over outer and inner -> out [groups, C]
-void colsum_groups(const Tensor& x, Tensor& out, int64_t outer, int64_t groups, int64_t inner) {
-  MK_CHECK(x.is_cuda() && x.scalar_type() == torch::kBFloat16 && x.is_contiguous(), "colsum_groups: contiguous bf16 CUDA tensor expected");
-  MK_CHECK(outer > 0 && groups > 0 && inner > 0 && x.numel() % (outer * groups * inner) == 0, "colsum_groups: bad extents");
-  const int64_t C = x.numel() / (outer * groups * inner);
-  MK_CHECK(out.is_cuda() && out.scalar_type() == torch::kFloat32 && out.is_contiguous() && out.numel() == groups * C, "colsum_groups: bad output");
-  c10::cuda::CUDAGuard guard(x.device());
-  Tensor part = colsum_buffer(x, outer * inner, C, groups);
-  check_cuda(mk::colsum(reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()), out.data_ptr<float>(),
-                        part.numel() ? part.data_ptr<float>() : nullptr, outer * inner, static_cast<int>(C), cur_stream(),
-                        static_cast<int>(groups), inner * C, static_cast<int>(inner), groups * inner * C),
-             "colsum_groups");
-}
-
 static void check_f32(const Tensor& t, int64_t n, const char* what) {
   MK_CHECK(t.is_cuda() && t.scalar_type() == torch::kFloat32 && t.is_contiguous() && t.numel() == n, what);
 }
@@ -840,7 +826,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_fold", &gemm_fold);
   m.def("spectral_planes", &spectral_planes);
   m.def("colsum", &colsum);
-  m.def("colsum_groups", &colsum_groups);
   m.def("afno_pack", &afno_pack);
   m.def("afno_fold", &afno_fold);
   m.def("inorm_bwd", &inorm_bwd);

@@ -2,9 +2,11 @@
 //
 // One launch from Python took 15 - 20 us of host time (operand objects, 40 converted integers, the binding), and the small networks
 // and filters, whose kernels take 5 - 20 us each, waited for it (a training pass of a 32 x 64 network of 16 channels 2589 -> 1786 us,
-// the AFNO filter of 90 x 180 tokens 461 -> 281).  The passes are those of ops/conv.py, ops/linear.py, ops/norm.py,
-// ops/spectral.py and ops/afno.py, which say what each launch computes, run them on the CPU (emulated) and hold the variants for
-// several GPUs; rules that pick among launches are in both and have to agree.
+// the AFNO filter of 90 x 180 tokens 461 -> 281).  Python says launch by launch what each pass does: `forward_stages` and
+// `backward_stages` of ops/spectral.py and ops/afno.py, which also run the passes on the CPU (emulated), and `_conv_fwd`, `_conv_dgrad`
+// and `_conv_wgrad` of ops/conv.py, of which convolutions, linear layers (tokens are a channels-last image) and MLPs are made.
+// The instance norm is two launches in either direction, as for several GPUs in ops/norm.py.  Strides, and rules that pick among
+// launches, are in both: tests/test_gpu_native_passes.py compares the two on the same tensors, bit by bit.
 #include "host.h"
 
 #include <pybind11/stl.h>

@@ -73,6 +73,9 @@ class AFNOPlan:
         self.fh, self.gh = prep(fh), prep(fh.t())             # [2 nkx, 2 H],  [2 H, 2 nkx]  (inverse = transpose)
         self.tables = [self.fw, self.fw_t, self.gw, self.gw_t, self.fh, self.gh]      # as the native passes take them
 
+    def extents(self, nb: int):
+        return [self.H, self.W, self.nkx, self.ncols, nb]
+
     @staticmethod
     def get(H, W, kx, ncols, device, dtype) -> "AFNOPlan":
         key = (H, W, tuple(kx), ncols, str(device), dtype)
@@ -203,6 +206,70 @@ def _fold(dwx, dbx, shapes, bias):
     return dw, db
 
 
+def forward_stages(x, w1, b1, w2, b2, skip, plan: AFNOPlan, lam: float):
+    """(result, then what the backward pass reads: y, o1, o2 and the packed weights), launch by launch: the pass on the CPU, and what
+    `afno_forward` of csrc/layers.cpp does on the GPU."""
+    B, C, nb, hid = x.shape[0], x.shape[3], w1.shape[1], w1.shape[3]
+    bs, nc, nkx = C // nb, plan.ncols, plan.nkx
+    T = B * nc * nkx
+    (w1q, w2q), (b1f, b2f) = _pack((w1, w2), (b1, b2), x.dtype)
+    t1 = _stage_w_analysis(x, plan.fw, plan)
+    y = _stage_h_tokens(t1, plan, B, C, nb)
+    o1 = torch.empty(T, nb, 2 * hid, dtype=x.dtype, device=x.device)
+    gemm(T, 2 * hid, 2 * bs, Operand(y, ld=2 * C, zs_lo=2 * bs), Operand(w1q, ld=2 * bs, zs_lo=2 * hid * 2 * bs),
+         Output(o1, rs_lo=nb * 2 * hid, d_zlo=2 * hid), zlo_n=nb, bias=b1f, bias_mode=BIAS_COL, bias_zs=2 * hid, act=ACT_RELU)
+    o2 = torch.empty(B * nc, nb, nkx, 2, bs, dtype=x.dtype, device=x.device)
+    _tokens_to_blocks(o1, Operand(w2q, ld=2 * hid, zs_lo=2 * bs * 2 * hid), o2, plan, B, nb, 2 * bs, 2 * hid, bias=b2f,
+                      bias_mode=BIAS_COL, bias_zs=2 * bs, act=ACT_SHRINK, act_param=lam)
+    t4 = _stage_h_blocks(o2, plan.gh, plan, B, C, nb)
+    return _stage_w_synthesis(t4, plan.gw, plan, B, C, skip), y, o1, o2, w1q, w2q
+
+
+def backward_stages(dy, y, o1, o2, w1q, w2q, plan: AFNOPlan, has_b1: bool, has_b2: bool, add_dy: bool):
+    """(dx, gradients of w1, b1, w2, b2 in fp32) as `afno_backward` of csrc/layers.cpp has them on the GPU; `add_dy`: the skip was the
+    input, its gradient joins dx."""
+    B, H, _, C = dy.shape
+    nb, hid = o1.shape[1], o1.shape[2] // 2
+    bs, nc, nkx = C // nb, plan.ncols, plan.nkx
+    T = B * nc * nkx
+    dt, dev = dy.dtype, dy.device
+    # fp32 sums of the packed weights and biases, cleared together
+    n1, n2 = 2 * hid * 2 * bs * nb, 2 * hid * nb
+    acc = torch.zeros(2 * n1 + n2 + 2 * bs * nb, dtype=torch.float32, device=dev)
+    dw1, dw2 = acc[:n1].view(nb, 2 * hid, 2 * bs), acc[n1: 2 * n1].view(nb, 2 * bs, 2 * hid)
+    db1, db2 = acc[2 * n1: 2 * n1 + n2].view(nb, 2 * hid), acc[2 * n1 + n2:].view(nb, 2 * bs)
+    # adjoint of the synthesis along W, then along H with the shrinkage mask (saved output != 0) in the epilogue
+    dt4 = _stage_w_analysis(dy, plan.gw_t, plan)                                   # [B, ncols, H, 2, C]
+    do2 = torch.empty_like(o2)
+    gemm(2 * nkx, bs, 2 * H, Operand(plan.fh, ld=plan.fh.shape[1]),
+         Operand(dt4, ld=C, mn_major=True, zs_lo=bs, zs_hi=H * 2 * C),
+         Output(do2, rs_lo=bs, d_zlo=nkx * 2 * bs, d_zhi=nb * nkx * 2 * bs), zlo_n=nb, zhi_n=B * nc,
+         act=ACT_DSHRINK, resid=o2)
+    # second layer: data gradient with the ReLU mask (saved output > 0), weight gradient summed over the (b, ky) batches
+    do1 = torch.empty_like(o1)
+    gemm(nkx, 2 * hid, 2 * bs, Operand(do2, ld=2 * bs, zs_lo=nkx * 2 * bs, zs_hi=nb * nkx * 2 * bs),
+         Operand(w2q, ld=2 * hid, mn_major=True, zs_lo=2 * bs * 2 * hid),
+         Output(do1, rs_lo=nb * 2 * hid, d_zlo=2 * hid, d_zhi=nkx * nb * 2 * hid), zlo_n=nb, zhi_n=B * nc,
+         act=ACT_DRELU, resid=o1)
+    summed = gemm(2 * bs, 2 * hid, nkx, Operand(do2, ld=2 * bs, mn_major=True, zs_lo=nkx * 2 * bs, zs_hi=nb * nkx * 2 * bs),
+                  Operand(o1, ld=nb * 2 * hid, mn_major=True, zs_lo=2 * hid, zs_hi=nkx * nb * 2 * hid),
+                  Output(dw2, rs_lo=2 * hid, d_zlo=2 * bs * 2 * hid), zlo_n=nb, zhi_n=B * nc, accumulate=True, splits=0,
+                  row_sums=db2 if has_b2 else None)
+    assert summed or not has_b2
+    # first layer
+    dyt = torch.empty(B * nc, nb, nkx, 2, bs, dtype=dt, device=dev)
+    _tokens_to_blocks(do1, Operand(w1q, ld=2 * bs, mn_major=True, zs_lo=2 * hid * 2 * bs), dyt, plan, B, nb, 2 * bs, 2 * hid)
+    summed = gemm(2 * hid, 2 * bs, T, Operand(do1, ld=nb * 2 * hid, mn_major=True, zs_lo=2 * hid),
+                  Operand(y, ld=2 * C, mn_major=True, zs_lo=2 * bs),
+                  Output(dw1, rs_lo=2 * bs, d_zlo=2 * hid * 2 * bs), zlo_n=nb, accumulate=True, splits=0,
+                  row_sums=db1 if has_b1 else None)
+    assert summed or not has_b1
+    (gw1, gw2), (gb1, gb2) = _fold([dw1, dw2], [db1, db2], [(2, nb, bs, hid), (2, nb, hid, bs)], (has_b1, has_b2))
+    # adjoint of the analysis along H and along W; the skip's gradient joins in the last epilogue
+    dt1 = _stage_h_blocks(dyt, plan.gh, plan, B, C, nb)                            # [H, B*ncols, 2, C]
+    return _stage_w_synthesis(dt1, plan.fw_t, plan, B, C, dy if add_dy else None), gw1, gb1, gw2, gb2
+
+
 class _AFNOFilter(torch.autograd.Function):
     """y = irfft2(softshrink(relu(rfft2(x) W1 + b1) W2 + b2)) (+ skip) on the kept modes.
 
@@ -212,88 +279,27 @@ class _AFNOFilter(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, w1, b1, w2, b2, skip, plan, lam):
-        B, H, W, C = x.shape
-        nb = w1.shape[1]
-        bs, hid = C // nb, w1.shape[3]
-        nc, nkx = plan.ncols, plan.nkx
-        T = B * nc * nkx
-        dt = x.dtype
-        ctx.plan, ctx.dims = plan, (B, C, nb, bs, hid)
+        ctx.plan, ctx.nb = plan, w1.shape[1]
         # skip_is_x: the skip is the input itself (the usual residual form); its gradient then rides in the epilogue of
         # the last backward GEMM instead of a separate elementwise add
         ctx.flags = (b1 is not None, b2 is not None, skip is not None, skip is x)
         ctx.wtypes = tuple(None if t is None else t.dtype for t in (w1, b1, w2, b2))
         if x.is_cuda:
-            out, *saved = _ext.require().afno_forward(x, w1, b1, w2, b2, skip, plan.tables, [H, W, nkx, nc, nb], float(lam))
-            ctx.save_for_backward(*saved)
-            return out
-        (w1q, w2q), (b1f, b2f) = _pack((w1, w2), (b1, b2), dt)
-        t1 = _stage_w_analysis(x, plan.fw, plan)
-        y = _stage_h_tokens(t1, plan, B, C, nb)
-        o1 = torch.empty(T, nb, 2 * hid, dtype=dt, device=x.device)
-        gemm(T, 2 * hid, 2 * bs, Operand(y, ld=2 * C, zs_lo=2 * bs), Operand(w1q, ld=2 * bs, zs_lo=2 * hid * 2 * bs),
-             Output(o1, rs_lo=nb * 2 * hid, d_zlo=2 * hid), zlo_n=nb, bias=b1f, bias_mode=BIAS_COL, bias_zs=2 * hid, act=ACT_RELU)
-        o2 = torch.empty(B * nc, nb, nkx, 2, bs, dtype=dt, device=x.device)
-        _tokens_to_blocks(o1, Operand(w2q, ld=2 * hid, zs_lo=2 * bs * 2 * hid), o2, plan, B, nb, 2 * bs, 2 * hid, bias=b2f,
-                          bias_mode=BIAS_COL, bias_zs=2 * bs, act=ACT_SHRINK, act_param=float(lam))
-        t4 = _stage_h_blocks(o2, plan.gh, plan, B, C, nb)
-        out = _stage_w_synthesis(t4, plan.gw, plan, B, C, skip)
-        ctx.save_for_backward(y, o1, o2, w1q, w2q)
+            out, *saved = _ext.require().afno_forward(x, w1, b1, w2, b2, skip, plan.tables, plan.extents(w1.shape[1]), float(lam))
+        else:
+            out, *saved = forward_stages(x, w1, b1, w2, b2, skip, plan, float(lam))
+        ctx.save_for_backward(*saved)
         return out
 
     @staticmethod
     def backward(ctx, dy):
-        y, o1, o2, w1q, w2q = ctx.saved_tensors
-        plan = ctx.plan
-        B, C, nb, bs, hid = ctx.dims
         has_b1, has_b2, has_skip, skip_is_x = ctx.flags
-        H, nc, nkx = plan.H, plan.ncols, plan.nkx
-        T = B * nc * nkx
-        dy = dy.contiguous()
+        plan, dy = ctx.plan, dy.contiguous()
         if dy.is_cuda:
-            dx, *grads = _ext.require().afno_backward(dy, y, o1, o2, w1q, w2q, plan.tables, [H, plan.W, nkx, nc, nb], has_b1, has_b2, skip_is_x)
-            gw1, gb1, gw2, gb2 = (g if g is None else g.to(t) for g, t in zip(grads, ctx.wtypes))
-            return dx, gw1, gb1, gw2, gb2, (dy if (has_skip and not skip_is_x) else None), None, None
-        dt = dy.dtype
-        dev = dy.device
-        # fp32 sums of the packed weights and biases, cleared together
-        n1, n2 = 2 * hid * 2 * bs * nb, 2 * hid * nb
-        acc = torch.zeros(2 * n1 + n2 + 2 * bs * nb, dtype=torch.float32, device=dev)
-        dw1, dw2 = acc[:n1].view(nb, 2 * hid, 2 * bs), acc[n1: 2 * n1].view(nb, 2 * bs, 2 * hid)
-        db1, db2 = acc[2 * n1: 2 * n1 + n2].view(nb, 2 * hid), acc[2 * n1 + n2:].view(nb, 2 * bs)
-        # adjoint of the synthesis along W, then along H with the shrinkage mask (saved output != 0) in the epilogue
-        dt4 = _stage_w_analysis(dy, plan.gw_t, plan)                                   # [B, ncols, H, 2, C]
-        do2 = torch.empty_like(o2)
-        gemm(2 * nkx, bs, 2 * H, Operand(plan.fh, ld=plan.fh.shape[1]),
-             Operand(dt4, ld=C, mn_major=True, zs_lo=bs, zs_hi=H * 2 * C),
-             Output(do2, rs_lo=bs, d_zlo=nkx * 2 * bs, d_zhi=nb * nkx * 2 * bs), zlo_n=nb, zhi_n=B * nc,
-             act=ACT_DSHRINK, resid=o2)
-        # second layer: data gradient with the ReLU mask (saved output > 0), weight gradient summed over the (b, ky) batches
-        do1 = torch.empty_like(o1)
-        gemm(nkx, 2 * hid, 2 * bs, Operand(do2, ld=2 * bs, zs_lo=nkx * 2 * bs, zs_hi=nb * nkx * 2 * bs),
-             Operand(w2q, ld=2 * hid, mn_major=True, zs_lo=2 * bs * 2 * hid),
-             Output(do1, rs_lo=nb * 2 * hid, d_zlo=2 * hid, d_zhi=nkx * nb * 2 * hid), zlo_n=nb, zhi_n=B * nc,
-             act=ACT_DRELU, resid=o1)
-        done = gemm(2 * bs, 2 * hid, nkx, Operand(do2, ld=2 * bs, mn_major=True, zs_lo=nkx * 2 * bs, zs_hi=nb * nkx * 2 * bs),
-                    Operand(o1, ld=nb * 2 * hid, mn_major=True, zs_lo=2 * hid, zs_hi=nkx * nb * 2 * hid),
-                    Output(dw2, rs_lo=2 * hid, d_zlo=2 * bs * 2 * hid), zlo_n=nb, zhi_n=B * nc, accumulate=True, splits=0,
-                    row_sums=db2 if has_b2 else None) or not has_b2
-        if not done:
-            _ext.require().colsum_groups(do2, db2, B * nc, nb, nkx)
-        # first layer
-        dyt = torch.empty(B * nc, nb, nkx, 2, bs, dtype=dt, device=dev)
-        _tokens_to_blocks(do1, Operand(w1q, ld=2 * bs, mn_major=True, zs_lo=2 * hid * 2 * bs), dyt, plan, B, nb, 2 * bs, 2 * hid)
-        done = gemm(2 * hid, 2 * bs, T, Operand(do1, ld=nb * 2 * hid, mn_major=True, zs_lo=2 * hid),
-                    Operand(y, ld=2 * C, mn_major=True, zs_lo=2 * bs),
-                    Output(dw1, rs_lo=2 * bs, d_zlo=2 * hid * 2 * bs), zlo_n=nb, accumulate=True, splits=0,
-                    row_sums=db1 if has_b1 else None) or not has_b1
-        if not done:
-            _ext.require().colsum(do1, db1)
-        (gw1, gw2), (gb1, gb2) = _fold([dw1, dw2], [db1, db2], [(2, nb, bs, hid), (2, nb, hid, bs)], (has_b1, has_b2))
-        gw1, gb1, gw2, gb2 = (g if g is None else g.to(t) for g, t in zip((gw1, gb1, gw2, gb2), ctx.wtypes))
-        # adjoint of the analysis along H and along W; the skip's gradient joins in the last epilogue
-        dt1 = _stage_h_blocks(dyt, plan.gh, plan, B, C, nb)                            # [H, B*ncols, 2, C]
-        dx = _stage_w_synthesis(dt1, plan.fw_t, plan, B, C, dy if skip_is_x else None)
+            dx, *grads = _ext.require().afno_backward(dy, *ctx.saved_tensors, plan.tables, plan.extents(ctx.nb), has_b1, has_b2, skip_is_x)
+        else:
+            dx, *grads = backward_stages(dy, *ctx.saved_tensors, plan, has_b1, has_b2, skip_is_x)
+        gw1, gb1, gw2, gb2 = (g if g is None else g.to(t) for g, t in zip(grads, ctx.wtypes))
         return dx, gw1, gb1, gw2, gb2, (dy if (has_skip and not skip_is_x) else None), None, None
 
 
