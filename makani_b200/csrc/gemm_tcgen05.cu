@@ -129,6 +129,7 @@ struct KParams {
   FastDiv dv_n, dv_m, dv_split, dv_zlo;
   uint32_t total_tiles;           // below 2^31
   int a_part;                     // k coordinate of the second part of a K-major A (complex and folded products)
+  int n_full;                     // columns in whole 16-byte vectors of the output
   int mirror, fold_rows;          // folded products: rows r < M and mirror - r, which are the rows M to fold_rows
   int cplx, nth, neg_half, neg_seg;   // complex product: mode, column tiles per half, the negative (half, segment)
   int stages, e_tma;
@@ -425,6 +426,9 @@ __host__ __device__ constexpr int stg_bytes(int bn, int epi) { return epi_warps(
 //   2 GELU + saved pre-activation                     3 + residual (TMA-prefetched)      4 * GELU'(aux) (TMA-prefetched)
 //   5 fp32 output, stored or added (split-k, summed batches): weight gradients
 //   6 sum and difference of two accumulators, stored at row r and its mirror row (folded transforms)
+// RAGGED (1 to 4): widths that are no multiple of 8.  A TMA store writes whole 16-byte vectors, also over the edge of its tensor map, and
+// what lies behind the last column in a wider matrix is not this launch's: the columns of a last, partial vector leave one by one.
+// Instances of their own (128 columns, single CTAs), as the others have no registers to spare.
 // rows of B per stage: whole MN-major boxes of 64 (a pair's half of a 192-wide tile is one and a half of them)
 __host__ __device__ constexpr int b_stage_rows(int bn, int cg) { return (bn / cg + 63) / 64 * 64; }
 
@@ -443,7 +447,7 @@ __device__ __forceinline__ unsigned int ld_acquire_sys_u32(const unsigned int* p
   return v;
 }
 
-template <int BN, int EB, int EPI, int CG>
+template <int BN, int EB, int EPI, int CG, bool RAGGED>
 __global__ void __launch_bounds__(bound_threads(BN, EPI), 1)
 gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ BMaps maps_b,
             const __grid_constant__ CUtensorMap map_e, const __grid_constant__ CUtensorMap map_d,
@@ -1165,7 +1169,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
           fence_async_smem();
           __syncwarp();
           const int r0 = c.mt * BM + q * 32;
-          if (elect_one() && r0 < p.M) {
+          if (elect_one() && r0 < p.M && (!RAGGED || nb < p.n_full)) {
             const int rs = r0 >> p.rd_shift;
             if constexpr (EPI == 2) tma_store_tile(&map_p, smem_base + box_off - 32 * 128, nb, 0, rs, c.zlo, c.zhi);
             tma_store_tile(&map_d, smem_base + box_off, nb, c.half, rs, c.zlo, c.zhi);
@@ -1175,6 +1179,22 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
             }
             tma_store_commit();
             if constexpr (IN_PLACE) tma_store_wait_read<0>();   // the operand buffer is free once the store has read it
+          }
+          if constexpr (RAGGED) {
+            if (nb + 64 > p.n_full && row_ok) {
+              const long long at = row_off + p.n_full;
+              const uint8_t* const box = smem + box_off + lane * 128 + (((p.n_full - nb) << 1) ^ ((lane & 7) << 4));
+              auto tail = [&](const uint8_t* from, void* to) {
+                const uint4 v = *reinterpret_cast<const uint4*>(from);
+                const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+                uint16_t* const o = static_cast<uint16_t*>(to) + at;
+#pragma unroll
+                for (int j = 0; j < 7; ++j)
+                  if (p.n_full + j < p.N) o[j] = static_cast<uint16_t>(w[j / 2] >> (16 * (j & 1)));
+              };
+              tail(box, p.D);
+              if constexpr (EPI == 2) tail(box - 32 * 128, p.preact);
+            }
           }
         }
         if constexpr (IN_PLACE) {
@@ -1465,8 +1485,8 @@ int max_pairs() {
     qc.attrs = qa;
     qc.numAttrs = 1;
     int got = 0;
-    cudaError_t e = cudaFuncSetAttribute(gemm_kernel<256, 2, 0, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&got, gemm_kernel<256, 2, 0, 2>, &qc);
+    cudaError_t e = cudaFuncSetAttribute(gemm_kernel<256, 2, 0, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&got, gemm_kernel<256, 2, 0, 2, false>, &qc);
     if (e != cudaSuccess || got < 1) {
       (void)cudaGetLastError();
       got = sm_count() / 2;
@@ -1476,7 +1496,7 @@ int max_pairs() {
   return n;
 }
 
-template <int BN, int EB, int EPI, int CG>
+template <int BN, int EB, int EPI, int CG, bool RAGGED = false>
 cudaError_t launch_t(const CUtensorMap& ma, const BMaps& mb, const CUtensorMap& me, const CUtensorMap& md,
                      const CUtensorMap& mp, const DMaps& mdx, KParams& kp, cudaStream_t stream) {
   constexpr int STAGE = A_STAGE_BYTES + b_stage_rows(BN, CG) * 128;
@@ -1499,7 +1519,7 @@ cudaError_t launch_t(const CUtensorMap& ma, const BMaps& mb, const CUtensorMap& 
   const int threads = 32 * (3 + epi_warps(BN, EPI) + (kp.rowsum ? SUM_WARPS : (kp.e_tma ? 1 : 0)));
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_kernel<BN, EB, EPI, CG>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT);
+    cudaError_t e = cudaFuncSetAttribute(gemm_kernel<BN, EB, EPI, CG, RAGGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT);
     if (e != cudaSuccess) return e;
     configured = true;
   }
@@ -1527,11 +1547,11 @@ cudaError_t launch_t(const CUtensorMap& ma, const BMaps& mb, const CUtensorMap& 
     cfg.stream = stream;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, gemm_kernel<BN, EB, EPI, CG>, ma, mb, me, md, mp, mdx, kp);
+    return cudaLaunchKernelEx(&cfg, gemm_kernel<BN, EB, EPI, CG, RAGGED>, ma, mb, me, md, mp, mdx, kp);
   }
   long long grid = kp.total_tiles < static_cast<uint32_t>(num_sms) ? kp.total_tiles : num_sms;
   if (grid < 1) grid = 1;
-  gemm_kernel<BN, EB, EPI, CG><<<static_cast<unsigned>(grid), threads, smem, stream>>>(ma, mb, me, md, mp, mdx, kp);
+  gemm_kernel<BN, EB, EPI, CG, RAGGED><<<static_cast<unsigned>(grid), threads, smem, stream>>>(ma, mb, me, md, mp, mdx, kp);
   return cudaGetLastError();
 }
 
@@ -1922,13 +1942,13 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
   const bool plain = (one_stride || split_ok) && (e.ndiv <= 0 || e.ndiv >= (1 << 30));
   const int rd = one_stride ? 1 : e.rdiv;
   const bool folded = p.cplx == 4 || p.cplx == 5;
-  auto tile_map = [&](CUtensorMap* m, const void* ptr, int box_rows, int rows_of) {
-    return make_map_e(m, ptr, rows_of, p.N, rd, e.rs_hi, e.rs_lo, e.d_zlo, e.d_zhi, p.zlo_n, p.zhi_n, box_rows, 2, e.d_half);
+  auto tile_map = [&](CUtensorMap* m, const void* ptr, int box_rows, int rows_of, int cols_of) {
+    return make_map_e(m, ptr, rows_of, cols_of, rd, e.rs_hi, e.rs_lo, e.d_zlo, e.d_zhi, p.zlo_n, p.zhi_n, box_rows, 2, e.d_half);
   };
   kp.rd_shift = 0;
   while (plain && (1 << kp.rd_shift) < rd) ++kp.rd_shift;
   if (e.resid && !e.out_f32 && plain && kp.vec_ok && e.d_zlo >= 0 && e.d_zhi >= 0) {
-    if (tile_map(&me, e.resid, BM, p.M)) kp.e_tma = 1;
+    if (tile_map(&me, e.resid, BM, p.M, p.N)) kp.e_tma = 1;
   }
   // A specialised epilogue (TMA stores of bf16 tiles) when the launch fits one.
   int epi = 0;
@@ -1937,7 +1957,9 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
   memset(&md, 0, sizeof(md));
   memset(&mp, 0, sizeof(mp));
   memset(&mdx, 0, sizeof(mdx));
-  if (eb == 2 && !e.out_f32 && kp.vec_ok && !e.accumulate && plain && e.d_zlo >= 0 && e.d_zhi >= 0 &&
+  kp.n_full = p.N / 8 * 8;
+  const bool columns_ok = kp.n_full == p.N || p.cplx != 0 || (kp.n_full > 0 && kp.ndx == 0);
+  if (eb == 2 && !e.out_f32 && kp.vec_ok && !e.accumulate && plain && e.d_zlo >= 0 && e.d_zhi >= 0 && columns_ok &&
       (kp.bias_mode != 2 || (p.N % 8 == 0 && (reinterpret_cast<uintptr_t>(e.bias) & 15) == 0 && (kp.bias_zs % 4) == 0))) {
     if (folded) epi = !e.resid && !e.preact && e.act == 0 && !e.bias && e.alpha == 1.f && kp.ndx == 0 ? 6 : 0;
     else if (!e.resid && !e.preact && (e.act == 0 || e.act == 1 || e.act == 3 || e.act == 5)) epi = 1;
@@ -1945,19 +1967,22 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
     else if (e.resid && kp.e_tma && !e.preact && e.act == 0) epi = 3;
     else if (e.resid && kp.e_tma && !e.preact && (e.act == 2 || e.act == 4 || e.act == 6 || e.act == 8)) epi = 4;
     if (epi != 0) {
-      bool ok = tile_map(&md, e.D, 32, p.M);
-      if (ok && epi == 2) ok = tile_map(&mp, e.preact, 32, p.M);
-      if (ok && epi == 6) ok = tile_map(&mp, e.D, 32, p.rows);      // the mirror rows
+      const int cols = p.cplx ? p.N : kp.n_full;
+      bool ok = tile_map(&md, e.D, 32, p.M, cols);
+      if (ok && epi == 2) ok = tile_map(&mp, e.preact, 32, p.M, cols);
+      if (ok && epi == 6) ok = tile_map(&mp, e.D, 32, p.rows, cols);      // the mirror rows
       if (ok && kp.ndx > 0) {
         if (epi != 1) ok = false;   // replicated output goes through the plain-store epilogue or the generic one
         for (int q = 0; ok && q < kp.ndx; ++q)
-          ok = tile_map(&mdx.m[q], kp.Dx[q], 32, p.M);
+          ok = tile_map(&mdx.m[q], kp.Dx[q], 32, p.M, cols);
       }
       if (!ok) epi = 0;
     }
   }
   // fp32 results with nothing but a scale: a dimension whose batches all add into one output is left out of the map
+  // (a partial last vector may be added to, what lies behind it by zero, but not stored)
   if (eb == 2 && e.out_f32 && kp.vec_ok && plain && !e.resid && !e.preact && e.act == 0 && kp.bias_mode == 0 && kp.ndx == 0 &&
+      (e.accumulate || p.N % 4 == 0) &&
       e.d_zlo >= 0 && e.d_zhi >= 0 && (e.accumulate || ((e.d_zlo > 0 || p.zlo_n == 1) && (e.d_zhi > 0 || p.zhi_n == 1)))) {
     kp.d_zlo_on = e.d_zlo > 0;
     kp.d_zhi_on = e.d_zhi > 0;
@@ -1983,7 +2008,8 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
   }();
   const bool no_peer = (peer == nullptr) || (peer->nseg <= 1 && peer->ndx == 0 && peer->nwait == 0 && peer->nsig == 0 &&
                                               peer->done_ctr == nullptr);
-  const bool eligible = eb == 2 && no_peer && p.M > BM && p.rmin_a == 0 && p.rmax_a == 0 && (p.cplx == 0 || p.cplx >= 3);
+  const bool ragged = epi >= 1 && epi <= 4 && kp.n_full != p.N && p.cplx == 0;
+  const bool eligible = eb == 2 && no_peer && !ragged && p.M > BM && p.rmin_a == 0 && p.rmax_a == 0 && (p.cplx == 0 || p.cplx >= 3);
   const int pad1 = (p.M + BM - 1) / BM * BM, pad2 = (p.M + 2 * BM - 1) / (2 * BM) * (2 * BM);
   const long long z_all = static_cast<long long>(p.zlo_n) * p.zhi_n;
   const bool waves = pad1 / BM * ((p.N + 255) / 256) * z_all >= 2 * sm_count();
@@ -1991,7 +2017,7 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
   const int cg = (eligible && (pairs_mode == 1 || (pairs_mode == 2 && pays))) ? 2 : 1;
   if (bn == 0) bn = pick_bn(p.N, epi, kp.e_tma);
   if ((eb == 4 && bn == 192) || ((epi == 3 || epi == 4 || kp.e_tma) && bn == 256)) bn = 128;
-  if ((epi == 0 && kp.e_tma) || epi == 6) bn = 128;
+  if ((epi == 0 && kp.e_tma) || epi == 6 || ragged) bn = 128;
   kp.m_tiles = (p.M + BM * cg - 1) / (BM * cg);
   kp.n_tiles = (p.N + bn - 1) / bn;
   kp.cplx = p.cplx;
@@ -2087,6 +2113,9 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
   }
   // (epilogues with an operand in shared memory: at most 192 columns, see above)
 #define MK_DISPATCH(EPI_)                                                                              \
+  if constexpr (EPI_ >= 1 && EPI_ <= 4) {                                                              \
+    if (ragged) return launch_t<128, 2, EPI_, 1, true>(ma, mbs, me, md, mp, mdx, kp, stream);          \
+  }                                                                                                    \
   if constexpr (EPI_ != 3 && EPI_ != 4) {                                                              \
     if (bn == 256 && cg == 2) return launch_t<256, 2, EPI_, 2>(ma, mbs, me, md, mp, mdx, kp, stream);  \
     if (bn == 256) return launch_t<256, 2, EPI_, 1>(ma, mbs, me, md, mp, mdx, kp, stream);             \

@@ -757,3 +757,28 @@ def test_folded_products_write_every_row_once(rows, mirror, pairs, n, k, z):
     assert torch.equal(out[1].cpu(), out[0].to(torch.bfloat16))
     assert all(torch.equal(y.view(torch.int16), out[1].view(torch.int16)) for y in out[2:])
     _ext.check_device_errors(dev)
+
+
+@pytest.mark.parametrize("n", [4, 60, 73, 131, 256 + 1, 764])
+@pytest.mark.parametrize("kind", ["plain", "relu", "row_bias", "preact", "resid", "mulaux", "fp32", "split_rows"])
+def test_ragged_widths_leave_the_columns_behind_them_alone(n, kind):
+    """A product into the first n columns of a wider matrix, whole vectors and the columns of a partial one."""
+    dev = _dev()
+    g = torch.Generator(dev).manual_seed(n)
+    t, k, z = 300, 72, 2
+    ld = -(-n // 8) * 8 + 8
+    dt = torch.float32 if kind == "fp32" else torch.bfloat16
+    x, w = (torch.randn(*s, device=dev, generator=g).bfloat16() for s in ((z, t, k), (n, k)))
+    y, pre = (torch.full((z, t, ld), 7.0, device=dev, dtype=dt) for _ in range(2))
+    r, bias = torch.randn(z, t, ld, device=dev, generator=g).bfloat16(), torch.randn(t, device=dev, generator=g)
+    kw = {"relu": dict(act=ACT_RELU), "row_bias": dict(bias=bias, bias_mode=BIAS_ROW), "preact": dict(act=ACT_GELU, preact=pre),
+          "resid": dict(resid=r), "mulaux": dict(act=ACT_MULAUX, resid=r)}.get(kind, {})
+    out = Output(y, rs_lo=t // 2 * ld, rs_hi=ld, rdiv=2, d_zlo=t * ld) if kind == "split_rows" else Output(y, rs_lo=ld, d_zlo=t * ld)
+    gemm(t, n, k, Operand(x, ld=k, zs_lo=t * k), Operand(w, ld=k), out, zlo_n=z, **kw)
+    a = x.double() @ w.double().t()
+    ref = {"relu": a.clamp(min=0), "row_bias": a + bias[:, None], "preact": torch.nn.functional.gelu(a, approximate=_ext.gelu_approximation()),
+           "resid": a + r[..., :n], "mulaux": a * r[..., :n], "split_rows": torch.cat([a[:, 0::2], a[:, 1::2]], 1)}.get(kind, a)
+    assert _rel(y[..., :n], ref) < BF16 and (y[..., n:] == 7.0).all()
+    if kind == "preact":
+        assert _rel(pre[..., :n], a) < BF16 and (pre[..., n:] == 7.0).all()
+    _ext.check_device_errors(dev)
