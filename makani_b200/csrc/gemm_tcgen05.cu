@@ -428,7 +428,8 @@ __host__ __device__ constexpr int stg_bytes(int bn, int epi) { return epi_warps(
 //   6 sum and difference of two accumulators, stored at row r and its mirror row (folded transforms)
 // RAGGED (1 to 4): widths that are no multiple of 8.  A TMA store writes whole 16-byte vectors, also over the edge of its tensor map, and
 // what lies behind the last column in a wider matrix is not this launch's: the columns of a last, partial vector leave one by one.
-// Instances of their own (128 columns, single CTAs), as the others have no registers to spare.
+// Instances of their own (128 columns, single CTAs), as the others have no registers to spare.  384 -> 764 over 115200 tokens with a
+// column bias, us: 107 (GELU 128), through the generic epilogue 242 (418); 768 columns 72 (88).
 // rows of B per stage: whole MN-major boxes of 64 (a pair's half of a 192-wide tile is one and a half of them)
 __host__ __device__ constexpr int b_stage_rows(int bn, int cg) { return (bn / cg + 63) / 64 * 64; }
 
@@ -1041,7 +1042,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
           uint8_t* const sw_d = smem + box_off + lane * 128;
           const uint32_t l7 = static_cast<uint32_t>(lane & 7) << 4;
           auto columns = [&](auto bias_c, auto act_c) {
-            constexpr bool COL_BIAS = decltype(bias_c)::value != 0;
+            constexpr int COL_BIAS = decltype(bias_c)::value;
             constexpr int ACT = decltype(act_c)::value;
 #pragma unroll 1
             for (int it = 0; it < 4; ++it) {
@@ -1051,11 +1052,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
               for (int gg = 0; gg < 2; ++gg) {
                 const uint32_t sw = static_cast<uint32_t>((it * 2 + gg) << 4) ^ l7;
                 f32x2 f[4];
-                if constexpr (COL_BIAS) {      // rides on the scaling fma (columns past N are clipped by the store)
+                if constexpr (COL_BIAS == 1) {      // rides on the scaling fma (columns past N are clipped by the store)
                   const int n = min(nb + it * 16 + gg * 8, p.N - 8);
                   const ulonglong2 b0 = __ldg(reinterpret_cast<const ulonglong2*>(bias_z + n));
                   const ulonglong2 b1 = __ldg(reinterpret_cast<const ulonglong2*>(bias_z + n) + 1);
                   f[0] = b0.x; f[1] = b0.y; f[2] = b1.x; f[3] = b1.y;
+                } else if constexpr (COL_BIAS == 2) {      // (RAGGED)
+                  const int n = nb + it * 16 + gg * 8;
+#pragma unroll
+                  for (int j = 0; j < 4; ++j) f[j] = f2_pack(__ldg(bias_z + min(n + 2 * j, p.N - 1)), __ldg(bias_z + min(n + 2 * j + 1, p.N - 1)));
                 } else {
 #pragma unroll
                   for (int j = 0; j < 4; ++j) f[j] = rbias2;
@@ -1128,7 +1133,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
               float x[8];
 #pragma unroll
               for (int j = 0; j < 8; ++j)
-                x[j] = p.bias_mode == 2 ? __ldg(bias_z + min(nb + g * 8, p.N - 8) + j) : rbias;
+                x[j] = p.bias_mode != 2 ? rbias : __ldg(bias_z + (RAGGED ? min(nb + g * 8 + j, p.N - 1) : min(nb + g * 8, p.N - 8) + j));
               if constexpr (EPI == 2) {
                 float d[8];
 #pragma unroll
@@ -1151,7 +1156,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
               *reinterpret_cast<uint4*>(sw_d + sw) = pack_bf16x8(x);
             }
           } else if (p.bias_mode == 2) {
-            with_act(IntC<1>{});
+            with_act(IntC<RAGGED ? 2 : 1>{});
           } else {
             with_act(IntC<0>{});
           }
@@ -1960,7 +1965,7 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
   kp.n_full = p.N / 8 * 8;
   const bool columns_ok = kp.n_full == p.N || p.cplx != 0 || (kp.n_full > 0 && kp.ndx == 0);
   if (eb == 2 && !e.out_f32 && kp.vec_ok && !e.accumulate && plain && e.d_zlo >= 0 && e.d_zhi >= 0 && columns_ok &&
-      (kp.bias_mode != 2 || (p.N % 8 == 0 && (reinterpret_cast<uintptr_t>(e.bias) & 15) == 0 && (kp.bias_zs % 4) == 0))) {
+      (kp.bias_mode != 2 || ((reinterpret_cast<uintptr_t>(e.bias) & 15) == 0 && (kp.bias_zs % 4) == 0))) {
     if (folded) epi = !e.resid && !e.preact && e.act == 0 && !e.bias && e.alpha == 1.f && kp.ndx == 0 ? 6 : 0;
     else if (!e.resid && !e.preact && (e.act == 0 || e.act == 1 || e.act == 3 || e.act == 5)) epi = 1;
     else if (!e.resid && e.preact && e.act == 1) epi = 2;
