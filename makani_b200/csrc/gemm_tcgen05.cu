@@ -53,6 +53,8 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <algorithm>
+
 namespace mk {
 
 namespace {
@@ -1501,6 +1503,39 @@ int max_pairs() {
   return n;
 }
 
+// Grid of a folded product.  CTA c walks the tiles c, c + grid, ...: where the tiles of one batch and the grid have a factor in common, a
+// CTA meets the same few of them in every batch, and if those are the ones with few rows or columns it runs ahead of its
+// neighbours.  It idles at the end, and on the way the halves of the 128-byte lines that two tiles share are written so far apart in
+// time that they leave L2 one by one.  A grid without a common factor mixes them.  Synthesis of 1440 points, 64 orders, 136 channels
+// 150 -> 88, 200 channels 187 -> 108; of 256 points, 129 orders, 384 channels 35 -> 30 us.
+long long mixed_grid(long long grid, const KParams& kp, int bm, int bn) {
+  const int tiles = kp.m_tiles * kp.n_tiles;
+  if (tiles <= 1 || tiles > 256 || kp.total_tiles <= static_cast<uint32_t>(grid)) return grid;
+  auto gcd = [](long long a, long long b) {
+    while (b) {
+      const long long t = a % b;
+      a = b;
+      b = t;
+    }
+    return a;
+  };
+  const int classes = static_cast<int>(gcd(grid, tiles));
+  long long least = 0, most = 0;
+  for (int c = 0; c < classes; ++c) {
+    long long area = 0;
+    for (int i = c; i < tiles; i += classes) {
+      const int mt = kp.n_fast ? i / kp.n_tiles : i % kp.m_tiles, nt = kp.n_fast ? i % kp.n_tiles : i / kp.m_tiles;
+      area += static_cast<long long>(std::min(bm, kp.M - mt * bm)) * std::min(bn, kp.N - nt * bn);
+    }
+    least = c == 0 ? area : std::min(least, area);
+    most = std::max(most, area);
+  }
+  if (most * 4 <= least * 5) return grid;
+  for (long long g = grid - 1; g > grid - 8 && g > 0; --g)
+    if (gcd(g, tiles) == 1) return g;
+  return grid;
+}
+
 template <int BN, int EB, int EPI, int CG, bool RAGGED = false>
 cudaError_t launch_t(const CUtensorMap& ma, const BMaps& mb, const CUtensorMap& me, const CUtensorMap& md,
                      const CUtensorMap& mp, const DMaps& mdx, KParams& kp, cudaStream_t stream) {
@@ -1539,6 +1574,7 @@ cudaError_t launch_t(const CUtensorMap& ma, const BMaps& mb, const CUtensorMap& 
     const int most = max_pairs();
     long long clusters = kp.total_tiles < static_cast<uint32_t>(most) ? kp.total_tiles : most;
     if (clusters < 1) clusters = 1;
+    if constexpr (EPI == 6) clusters = mixed_grid(clusters, kp, 2 * BM, BN);
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cudaLaunchAttribute attr[1];
@@ -1556,6 +1592,7 @@ cudaError_t launch_t(const CUtensorMap& ma, const BMaps& mb, const CUtensorMap& 
   }
   long long grid = kp.total_tiles < static_cast<uint32_t>(num_sms) ? kp.total_tiles : num_sms;
   if (grid < 1) grid = 1;
+  if constexpr (EPI == 6) grid = mixed_grid(grid, kp, BM, BN);
   gemm_kernel<BN, EB, EPI, CG, RAGGED><<<static_cast<unsigned>(grid), threads, smem, stream>>>(ma, mb, me, md, mp, mdx, kp);
   return cudaGetLastError();
 }

@@ -828,3 +828,24 @@ def test_column_bias_over_ragged_widths_leaves_through_tma():
         return min(out)
 
     assert best(764) < 2.0 * best(768)
+
+
+def test_folded_products_with_a_narrow_last_tile_keep_their_ctas_together():
+    """136 of 256 columns: CTAs that met only the tiles of 8 columns ran ahead, and shared lines left L2 half by half (150 us, 256
+    channels 106)."""
+    from makani_b200.ops.spectral import SHTPlan, folded_synthesis
+    dev = _dev()
+    plan = SHTPlan(8, 1440, 8, 64, "legendre-gauss", dev)
+
+    def best(c):
+        t4, out = torch.randn(1, 721, 128, c, device=dev).bfloat16(), []
+        for _ in range(8):
+            t0, t1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            t0.record()
+            folded_synthesis(t4, plan)
+            t1.record()
+            torch.cuda.synchronize()
+            out.append(t0.elapsed_time(t1))
+        return min(out)
+
+    assert best(136) < 1.15 * best(256)
