@@ -1881,6 +1881,8 @@ int pick_splits(long long base, int kblocks, int slots, int least) {
 }
 }  // namespace
 
+int gemm_plain_columns(int n) { return pick_bn(n, 1, 0); }
+
 cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOperand& B, const GemmEpilogue& e,
                         int* err_flag, cudaStream_t stream, const GemmPeer* peer, GemmRowSums* rows) {
   g_err[0] = 0;

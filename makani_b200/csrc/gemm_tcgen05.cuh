@@ -116,4 +116,7 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
 
 const char* gemm_last_error();
 
+// columns of a tile that gemm_launch chooses for a plain bf16 store of n
+int gemm_plain_columns(int n);
+
 }  // namespace mk

@@ -309,12 +309,19 @@ struct Plan {
   }
 };
 
+// (the rule of `folding_pays` in ops/spectral.py, which says why)
+bool folding_pays(int64_t rows, int64_t folded_rows, int64_t k, int64_t folded_k, int64_t C) {
+  auto up = [](int64_t a, int64_t b) { return (a + b - 1) / b; };
+  auto tiles = [&](int64_t r, int64_t w) { return up(r, 128) * up(C, w) * w; };
+  return tiles(folded_rows, 128) * (2 * up(folded_k, 64) + 1) < tiles(rows, mk::gemm_plain_columns(static_cast<int>(C))) * (up(k, 64) + 1);
+}
+
 Tensor analyse(const Tensor& x, const Plan& p, bool forward) {
   const int64_t B = x.size(0), C = x.size(1), H = x.size(2), W = x.size(3), k2 = p.k2;
   MK_CHECK(H == p.nlat && W == p.nlon, "spectral plan: the grid does not match the field");
   Tensor t1 = at::empty({B, H, k2, C}, x.options());
   const Tensor& fold = p.t[forward ? 6 : 7];
-  if (fold.numel()) {
+  if (fold.numel() && (folding_pays(k2, 2 * (W / 4 + 1), W, W / 2, C) || (forward && W % 8 != 0))) {
     mkh::folded_product(fold, x, t1, {5, k2, 2 * (W / 4 + 1), C, W / 2, W, B * H, fold.size(1), fold.size(1) / 2, 0, 1, 2 * C, W * C, C, 0, C, k2 * C});
     return t1;
   }
@@ -333,7 +340,7 @@ Tensor synthesise(const Tensor& t4, const Plan& p, bool forward) {
   const int64_t B = t4.size(0), H = t4.size(1), k2 = t4.size(2), C = t4.size(3), W = p.nlon;
   Tensor y = at::empty({B, C, H, W}, t4.options(), at::MemoryFormat::ChannelsLast);
   const Tensor& fold = p.t[forward ? 4 : 5];
-  if (fold.numel()) {
+  if (fold.numel() && (folding_pays(W, W / 2 + 1, k2, k2 / 2, C) || (forward && W % 8 != 0))) {
     mkh::folded_product(fold, t4, y, {4, W, W / 2 + 1, C, k2 / 2, W, B * H, fold.size(1), fold.size(1) / 2, 0, 1, 2 * C, k2 * C, C, 0, C, W * C});
     return y;
   }

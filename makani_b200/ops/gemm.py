@@ -326,6 +326,11 @@ def gemm_fold(rows: int, M: int, N: int, K: int, mirror: int, pairs: bool, table
     _ext.require().gemm_fold(table, B.tensor, D.tensor, ip)
 
 
+def plain_columns(n: int) -> int:
+    """Columns of a tile that the engine chooses for a plain store of `n` (`gemm_plain_columns` of csrc/gemm_tcgen05.cu)."""
+    return min((256, 192, 128), key=lambda w: -(-n // w) * (w + 64))
+
+
 def _f32_bits(x: float) -> int:
     import struct
     return struct.unpack("<I", struct.pack("<f", float(x)))[0]

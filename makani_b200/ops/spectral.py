@@ -8,13 +8,13 @@ truncation pass ever touches HBM:
 
     x  [B, H, W, C]                  real grid data, channels-last (bf16)
     S1 longitude DFT      -> T1 [B, H, (m,ri), C]       A = DFT matrix [(m,ri), W], batched over latitude rows
-                                                        (folded: orders m and W / 2 - m share their products)
+                                                        (or folded: orders m and W / 2 - m share their products)
     S2 Legendre analysis  -> T2 [B, l, m, (ri, C)]      A = P_l^m(theta_k) w_k, batched over m, rows l < m skipped
     S3 complex contraction-> T3 [B, m, l, (ri, Co)]     B = real and imaginary planes of W_l, batched over l, rows m > l skipped
     S4 Legendre synthesis -> T4 [B, H', (m,ri), Co]     k-loop restricted to l >= m
-    S5 inverse DFT        -> y  [B, H', W', Co]         (folded: longitudes i and W' - i share their products)
+    S5 inverse DFT        -> y  [B, H', W', Co]         (or folded: longitudes i and W' - i share their products)
 
-(ri = real/imaginary part; the Legendre tables are padded along latitude to 16-byte TMA strides.)
+(ri = real/imaginary part; the rows of all tables start on 128-byte boundaries.)
 The adjoints used by the backward pass are the same five launches with the constant operands read in the
 other major (no transposed copies of the tables are stored).
 """
@@ -32,7 +32,7 @@ from ..sht.legendre import legendre_table
 from ..sht.quadrature import precompute_latitudes
 from . import _ext
 from .conv import records_grad
-from .gemm import Operand, Output, Tri, gemm, gemm_complex, gemm_fold, pad_to
+from .gemm import Operand, Output, Tri, gemm, gemm_complex, gemm_fold, pad_to, plain_columns
 
 
 class SHTPlan:
@@ -43,7 +43,7 @@ class SHTPlan:
     def __init__(self, nlat: int, nlon: int, lmax: int, mmax: int, grid: str, device, dtype=torch.bfloat16):
         self.nlat, self.nlon, self.lmax, self.mmax, self.grid = nlat, nlon, lmax, mmax, grid
         self.device, self.dtype = torch.device(device), dtype
-# rows of the tables start on 128-byte boundaries: a 128-byte row of a TMA box is then one line, not two
+        # rows of the tables start on 128-byte boundaries: a 128-byte row of a TMA box is then one line, not two
         self.hp = pad_to(nlat, 64)         # padded latitude extent of the Legendre tables
         self.k2 = 2 * mmax                 # DFT K extent (m, ri)
         self.k2p = pad_to(self.k2, 64)
@@ -74,14 +74,10 @@ class SHTPlan:
         g[:, 1:self.k2:2] = (-cm * sin).T
         self.gt = torch.from_numpy(g).to(self.device, dtype).contiguous()     # [W, (m,ri) padded]
 
-        # The same matrices with their columns in two halves, for `gemm_fold`.  The synthesis (rows are
-        # longitudes) folds from the 64 rows on that `gemm_fold` asks for.  The analysis (rows (m, ri)) only saves work where most
-        # orders up to half the points are kept, order m sharing its products with order W / 2 - m.  us, whole / folded:
-        #   synthesis, 384 channels: 721 x 1440, 241 orders 430 / 336; 240 x 480, 241 60 / 49; 360 x 720, 361 157 / 132;
-        #   180 x 360, 181 33 / 28;  200 channels: 181 x 360, 120 18.8 / 18.5;  64 channels, 2 x 64 x 128, 65 12.0 / 9.9
-        #   analysis: 240 x 480, 241 58 / 47; 360 x 720, 361 155 / 131, 241 of them 111 / 121; 181 x 360, 120 20.5 / 18.5 (adjoint
-        #   16.4 / 18.5); 100 x 200, 81 11.8 / 10.0
-        # Orders past half the points, which alias, have no mirror and stay whole.
+        # The same matrices with their columns in two halves, for `gemm_fold`.  The synthesis (rows are longitudes) may fold from the 64
+        # rows on that `gemm_fold` asks for.  The analysis (rows (m, ri)) only saves work where most orders up to half the points are
+        # kept, order m sharing its products with order W / 2 - m; orders past half the points, which alias, have no mirror and
+        # stay whole.  `folding_pays` decides for a number of channels.
         self.folds_synthesis = nlon >= 64
         self.folds_analysis = (nlon >= 64 and nlon % 2 == 0 and 8 * mmax > 3 * nlon and
                                nlon // 2 + 32 <= 2 * mmax <= nlon + 2)
@@ -176,10 +172,19 @@ def dft_synthesis(t4: torch.Tensor, mat: torch.Tensor, mat_mn: bool, mat_ld: int
     return y
 
 
-def analyse(x: torch.Tensor, plan: SHTPlan, forward: bool = True) -> torch.Tensor:
-    """Longitude DFT of x (`forward`), or the adjoint of the inverse one: [B, H, (m, ri), C]."""
-    if not plan.folds_analysis:
-        return dft_analysis(x, plan.f, False, plan.nlon, plan.k2) if forward else dft_analysis(x, plan.gt, True, plan.k2p, plan.k2)
+def folding_pays(rows: int, folded_rows: int, k: int, folded_k: int, C: int) -> bool:
+    """Whether a folded product of two halves of `folded_k` columns beats the whole one: fewer columns of 128-row tiles, each counted
+    with its slabs of 64 products and one more for its epilogue.  The folded product halves rows or products, but rounds them up
+    to whole tiles and slabs once more (129 of 256 rows are two tiles, as all 256 are; 32 orders are one slab, and two halves of them
+    two) and has tiles of 128 columns only.  Some 1700 transforms of 64 to 1440 points, 8 to 361 orders and 16 to 768 channels: always
+    folding takes 3.9 % more than the better of the two, never 9.9 %, this rule 0.6 %.  Synthesis, us, whole / folded: 1440 points, 64
+    orders, 136 channels 102 / 88, 264 channels 281 / 144; 256 points, 129 orders, 384 channels 24 / 30; 128 points, 32 orders,
+    768 channels 27 % slower folded.  The native passes (csrc/layers.cpp) have the same rule."""
+    tiles = lambda r, w: -(-r // 128) * -(-C // w) * w      # noqa: E731
+    return tiles(folded_rows, 128) * (2 * -(-folded_k // 64) + 1) < tiles(rows, plain_columns(C)) * (-(-k // 64) + 1)
+
+
+def folded_analysis(x: torch.Tensor, plan: SHTPlan, forward: bool = True) -> torch.Tensor:
     B, C, H, W = x.shape
     k2, table = plan.k2, plan._folded[False, forward]
     t1 = torch.empty(B, H, k2, C, dtype=x.dtype, device=x.device)
@@ -188,18 +193,31 @@ def analyse(x: torch.Tensor, plan: SHTPlan, forward: bool = True) -> torch.Tenso
     return t1
 
 
-def synthesise(t4: torch.Tensor, plan: SHTPlan, forward: bool = False) -> torch.Tensor:
-    """Inverse longitude DFT of t4 [B, H, (m, ri), C], or the adjoint of the forward one (`forward`); channels-last.  t4 may hold
-    fewer orders than the plan: those of a forward transform that keeps fewer than the inverse one."""
-    W = plan.nlon
-    if not plan.folds_synthesis:
-        return dft_synthesis(t4, plan.f, True, W, W) if forward else dft_synthesis(t4, plan.gt, False, plan.k2p, W)
+def folded_synthesis(t4: torch.Tensor, plan: SHTPlan, forward: bool = False) -> torch.Tensor:
     B, H, k2, C = t4.shape
-    table = plan._folded[True, forward]
+    W, table = plan.nlon, plan._folded[True, forward]
     y = torch.empty(B, C, H, W, dtype=t4.dtype, device=t4.device, memory_format=torch.channels_last)
     gemm_fold(W, W // 2 + 1, C, k2 // 2, W, False, table, table.shape[1] // 2,
               Operand(t4, ld=2 * C, mn_major=True, zs_hi=k2 * C), C, Output(y, rs_lo=C, d_zhi=W * C), zhi_n=B * H)
     return y
+
+
+def analyse(x: torch.Tensor, plan: SHTPlan, forward: bool = True) -> torch.Tensor:
+    """Longitude DFT of x (`forward`), or the adjoint of the inverse one: [B, H, (m, ri), C].  (The whole matrix of the forward transform
+    has rows of W columns: only the folded ones are aligned for any W.)"""
+    W = plan.nlon
+    if plan.folds_analysis and (folding_pays(plan.k2, 2 * (W // 4 + 1), W, W // 2, x.shape[1]) or (forward and W % 8)):
+        return folded_analysis(x, plan, forward)
+    return dft_analysis(x, plan.f, False, W, plan.k2) if forward else dft_analysis(x, plan.gt, True, plan.k2p, plan.k2)
+
+
+def synthesise(t4: torch.Tensor, plan: SHTPlan, forward: bool = False) -> torch.Tensor:
+    """Inverse longitude DFT of t4 [B, H, (m, ri), C], or the adjoint of the forward one (`forward`); channels-last.  t4 may hold
+    fewer orders than the plan: those of a forward transform that keeps fewer than the inverse one."""
+    W, k2 = plan.nlon, t4.shape[2]
+    if plan.folds_synthesis and (folding_pays(W, W // 2 + 1, k2, k2 // 2, t4.shape[3]) or (forward and W % 8)):
+        return folded_synthesis(t4, plan, forward)
+    return dft_synthesis(t4, plan.f, True, W, W) if forward else dft_synthesis(t4, plan.gt, False, plan.k2p, W)
 
 
 def legendre_analysis(t1: torch.Tensor, table: torch.Tensor, by_order: bool = False) -> torch.Tensor:

@@ -32,12 +32,13 @@ def _peak(fn):
 
 
 @pytest.mark.parametrize("b,c,co,h,w,ho,wo,lmax,m_in,m_out,resid", [
-    (2, 16, 24, 33, 64, 16, 32, 16, 17, 17, True),       # folded to whole, regridded residual
+    (2, 16, 24, 33, 64, 16, 32, 16, 17, 17, True),       # regridded residual
     (1, 40, 8, 48, 96, 45, 90, 40, 46, 46, True),        # 90 longitudes out: an odd half; ragged channels
     (2, 8, 16, 32, 64, 33, 65, 32, 33, 33, False),       # an odd number of longitudes out
-    (1, 136, 72, 40, 80, 40, 80, 40, 41, 41, False),     # two column tiles, both transforms folded both ways
+    (1, 136, 72, 40, 80, 40, 80, 40, 41, 41, False),     # two column tiles
     (2, 16, 16, 24, 48, 24, 48, 24, 25, 25, False),      # nothing folded
     (1, 16, 32, 48, 96, 48, 96, 40, 12, 12, True),       # few orders: the analysis stays whole
+    (1, 64, 72, 96, 192, 96, 192, 96, 97, 97, True),     # both transforms folded in both directions
 ])
 def test_spectral_passes(b, c, co, h, w, ho, wo, lmax, m_in, m_out, resid):
     from makani_b200.ops.spectral import SHTPlan, backward_stages, forward_stages, weight_planes

@@ -273,3 +273,38 @@ def test_a_plan_computes_its_angles_once(monkeypatch):
     plan = SHTPlan(h, w, h, m, "legendre-gauss", "cpu")
     assert len(plan._folded) == 4
     assert all(n <= 1.5 * m * w for n in seen.values())
+
+
+@pytest.mark.parametrize("h,w,mmax", [(3, 64, 33), (3, 64, 32), (2, 65, 33), (2, 72, 37), (2, 80, 41), (2, 90, 46), (2, 100, 41), (2, 96, 49),
+                                      (2, 128, 20)])
+def test_folded_forms_equal_the_whole_ones(h, w, mmax):
+    """The folded forms themselves, also where the rule prefers the whole ones."""
+    from makani_b200.ops.spectral import SHTPlan, dft_analysis, dft_synthesis, folded_analysis, folded_synthesis
+    plan = SHTPlan(h, w, h, mmax, "legendre-gauss", "cpu", torch.float64)
+    g = torch.Generator().manual_seed(w)
+    t4 = torch.randn(2, h, 2 * mmax, 8, generator=g, dtype=torch.float64)
+    x = torch.randn(2, h, w, 8, generator=g, dtype=torch.float64).permute(0, 3, 1, 2)
+    pairs = [(folded_synthesis(t4, plan), dft_synthesis(t4, plan.gt, False, plan.k2p, w)),
+             (folded_synthesis(t4, plan, forward=True), dft_synthesis(t4, plan.f, True, w, w))]
+    if plan.folds_analysis:
+        pairs += [(folded_analysis(x, plan), dft_analysis(x, plan.f, False, w, plan.k2)),
+                  (folded_analysis(x, plan, forward=False), dft_analysis(x, plan.gt, True, plan.k2p, plan.k2))]
+    for got, ref in pairs:      # the tables are fp32 numbers of the same angles
+        assert got.shape == ref.shape and (got - ref).abs().max() <= 1e-6 * ref.abs().max()
+
+
+def test_folding_where_it_pays():
+    """Both sides of the rule, at the grids of the recipes and where the folded form was measured to be slower."""
+    from makani_b200.ops.gemm import plain_columns
+    from makani_b200.ops.spectral import folding_pays
+    synthesis = lambda w, m, c: folding_pays(w, w // 2 + 1, 2 * m, m, c)  # noqa: E731
+    analysis = lambda w, m, c: folding_pays(2 * m, 2 * (w // 4 + 1), w, w // 2, c)  # noqa: E731
+    assert [plain_columns(c) for c in (8, 128, 136, 200, 256, 264, 384, 640, 776)] == [128, 128, 192, 256, 256, 192, 192, 256, 256]
+    for args in ((1440, 241, 384), (480, 241, 384), (720, 361, 384), (1440, 64, 136), (1440, 361, 72)):
+        assert synthesis(*args)
+    for args in ((256, 129, 384), (128, 32, 768), (64, 33, 384), (360, 8, 384), (256, 32, 320)):
+        assert not synthesis(*args)
+    for args in ((480, 241, 384), (720, 361, 384), (360, 181, 200)):
+        assert analysis(*args)
+    for args in ((64, 33, 384), (96, 40, 768), (256, 97, 384)):
+        assert not analysis(*args)
