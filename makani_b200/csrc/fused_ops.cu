@@ -666,7 +666,7 @@ __global__ void __launch_bounds__(CS_THREADS) colsum_kernel(const uint4* __restr
   }
 }
 
-// out[g, c] = sum over the slabs (some hundreds of them); 32 columns by 32 slabs at a time per CTA.  grid (ceil(C / 32), groups)
+// out[g, c] = sum over the slabs (some hundreds of them, 4096 at most); 32 columns by 32 slabs at a time per CTA.  grid (ceil(C / 32), groups)
 __global__ void __launch_bounds__(1024) colsum_slabs_kernel(const float* __restrict__ part, float* __restrict__ out, int slabs, int C) {
   __shared__ float sh[32][33];
   const int c = blockIdx.x * 32 + threadIdx.x;

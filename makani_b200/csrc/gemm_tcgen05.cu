@@ -2109,16 +2109,18 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
     return cudaErrorInvalidValue;
   }
   kp.total_tiles = static_cast<uint32_t>(base_tiles * kp.splits);
-  // sums of the rows of A: only where the launch has A's tokens in shared memory as rows, all of them and each once
+  // Sums of the rows of A: only where the launch has A's tokens in shared memory as rows, all of them and each once, and where adding up
+  // the partial sums stays short.  Every batch, split and column tile leaves four of them per row; gradient and sums beside it over
+  // gradient and a pass of its own, by partial sums: 258 0.75, 512 0.70, 2048 0.73, 3072 0.90, 4096 1.03, 11648 1.06, 12288 0.96 - 1.09,
+  // 32768 1.65, 262144 2.1 - 2.5 (67 MB of them for 64 rows).
   if (rows && epi == 5 && A.mn_major && p.cplx == 0 && kp.nseg == 1 && p.rmin_a == 0 && p.rmin_b <= 0 && p.rmax_a == 0 && p.rmax_b >= p.M &&
       p.kmin_a == 0 && p.kmin_b <= 0 && p.kmax_a == 0 && p.kmax_b >= p.K && (p.zlo_n == 1 || A.zs_lo != 0) && (p.zhi_n == 1 || A.zs_hi != 0) &&
       (p.zhi_n == 1 || e.d_zhi == 0)) {
     kp.rs_groups = p.zlo_n > 1 && e.d_zlo != 0 ? p.zlo_n : 1;
     const long long slabs = z_all / kp.rs_groups * kp.splits * kp.n_tiles * 4;
-    if (slabs < (1 << 20) && kp.rs_groups < 65536) {
+    if (slabs <= 4096 && kp.rs_groups < 65536) {
       kp.rs_slabs = static_cast<int>(slabs);
-      kp.rowsum = rows->scratch(rows->ctx, slabs * kp.rs_groups * p.M);
-      if (!kp.rowsum) return cudaErrorMemoryAllocation;
+      kp.rowsum = rows->scratch(rows->ctx, slabs * kp.rs_groups * p.M);      // (null: no memory for them, the caller's pass needs less)
     }
   }
   kp.dv_n = make_div(kp.n_tiles);

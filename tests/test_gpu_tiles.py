@@ -849,3 +849,18 @@ def test_folded_products_with_a_narrow_last_tile_keep_their_ctas_together():
         return min(out)
 
     assert best(136) < 1.15 * best(256)
+
+
+@pytest.mark.parametrize("b,taken", [(1024, True), (1025, False)])
+def test_row_sums_of_very_many_batches_are_a_pass_of_their_own(b, taken):
+    """Four partial sums per row and batch: past 4096 adding them up takes longer than reading the matrix once more."""
+    from makani_b200.ops.conv import _conv_wgrad
+    dev = _dev()
+    g = torch.Generator(dev).manual_seed(b)
+    dy, x = (torch.randint(-1, 2, (b, 8, 8, 64), device=dev, generator=g).bfloat16().permute(0, 3, 1, 2) for _ in range(2))
+    d, sums = torch.zeros(64, 64, device=dev), torch.empty(64, device=dev)
+    assert gemm(64, 64, 64, Operand(dy, ld=64, mn_major=True, zs_lo=64 * 64), Operand(x, ld=64, mn_major=True, zs_lo=64 * 64), Output(d, rs_lo=64),
+                zlo_n=b, accumulate=True, splits=0, row_sums=sums) == taken
+    dw, db = _conv_wgrad(dy, x, bias=True)
+    assert torch.equal(db, dy.float().sum((0, 2, 3)))
+    assert torch.equal(dw, torch.einsum("bohw,bihw->oi", dy.float(), x.float()))
