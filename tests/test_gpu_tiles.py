@@ -864,3 +864,25 @@ def test_row_sums_of_very_many_batches_are_a_pass_of_their_own(b, taken):
     dw, db = _conv_wgrad(dy, x, bias=True)
     assert torch.equal(db, dy.float().sum((0, 2, 3)))
     assert torch.equal(dw, torch.einsum("bohw,bihw->oi", dy.float(), x.float()))
+
+
+@pytest.mark.parametrize("m,n,k,zlo", [
+    (1120, 384, 4097, 1),       # CTA pairs, the second of the last pair without rows
+    (1096, 40, 513, 2),         # the same, ragged, batches that add up
+    (768, 384, 65537, 1),       # one token in the last slab
+    (384, 768, 30001, 1),       # single CTAs, many splits
+    (520, 256, 4097, 3),
+])
+def test_row_sums_count_every_token_once(m, n, k, zlo):
+    """Whole numbers whose sums fp32 holds: exact in any order.  The last token of a batch weighs more than any other."""
+    dev = _dev()
+    g = torch.Generator(dev).manual_seed(k)
+    a = torch.randint(0, 4, (zlo, k, m), device=dev, generator=g).bfloat16()
+    a[:, -1] = torch.randint(100, 256, (zlo, m), device=dev, generator=g).bfloat16()
+    b = torch.randint(-1, 2, (zlo, k, n), device=dev, generator=g).bfloat16()
+    d, sums = torch.zeros(m, n, device=dev), torch.full((m,), float("nan"), device=dev)
+    assert gemm(m, n, k, Operand(a, ld=m, mn_major=True, zs_lo=k * m), Operand(b, ld=n, mn_major=True, zs_lo=k * n), Output(d, rs_lo=n),
+                zlo_n=zlo, accumulate=True, splits=0, row_sums=sums)
+    assert torch.equal(sums.double(), a.double().sum((0, 1)))
+    assert torch.equal(d.double(), (a.double().transpose(1, 2) @ b.double()).sum(0))
+    _ext.check_device_errors(dev)
