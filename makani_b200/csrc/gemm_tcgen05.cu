@@ -8,8 +8,8 @@
 //                    epilogue: alternating 32-column chunks)
 //   warp EW+3      : only in launches whose epilogue operand (residual, saved pre-activation) is prefetched by TMA: its
 //                    producer, so that waiting for a free operand buffer never delays A and B
-//   warps EW+3..   : only in launches that also sum the rows of A (bias gradients): eight warps that add up every stage before it is
-//                    freed
+//   warps EW+3..   : only in launches that also sum the rows of A (bias gradients): eight warps that add up the stages of their tile's
+//                    turn before these are freed; the producer releases the others in their name
 // Two accumulator buffers in TMEM let the epilogue of tile i overlap the main loop of tile i+1.
 // Every mbarrier wait is bounded; on expiry the kernel records a code in *err and drains.
 //
@@ -18,7 +18,7 @@
 // completion is counted on the leader CTA's barrier); the leader issues tcgen05.mma.cta_group::2, which reads both
 // CTAs' shared memory and writes 128 accumulator rows into each CTA's TMEM; tcgen05.commit multicasts the
 // "stage free" and "accumulator full" signals to both CTAs.  Per tensor-core cycle every SM then takes a third less
-// data from L2 (two thirds with 128-wide tiles), which is what bounds these GEMMs.
+// data from L2 (two thirds with 128-wide tiles).
 //
 // Complex products (p.cplx = 1, 2, 3): real and imaginary planes of the operands are multiplied without ever forming the real 2x2-block
 // matrix.  The column tiles come in two halves (real, imaginary part of the result) and the k loop in two segments that
@@ -26,15 +26,15 @@
 //   1: D(h) = sum_s A[.., s Kh + k] B(plane h ^ s),  minus at h = 0, s = 1      (product with W)
 //   2: the same, minus at h = 1, s = 0                                          (product with the conjugate of W)
 //   3: D(h) = sum_s A(plane s ^ h) B(plane s),       minus at h = 1, s = 1      (weight gradient)
+// 384 x 384 weights of 240 degrees: the operand takes 69 us to make instead of 95 (half the bytes), the products 87 - 94 us instead
+// of 105 - 114, the weight gradient one launch of 90 us instead of two of 78 and a swapped copy of 31.
+//
 // Folded transforms (p.cplx = 4, 5): a Fourier matrix has rows r and R - r that differ in nothing but the sign of one half of their
 // columns, so one product of half the rows serves both.  The two halves are two segments of the k loop with accumulators of their
 // own, and the epilogue stores their sum at row r and their difference at row R - r, both from fp32:
 //   4: rows are longitudes (synthesis): the halves are the cosine and the sine terms, i.e. the real and imaginary planes of B
 //   5: rows are (order, re / im) pairs of all orders up to half the points (analysis): the halves are the even and the odd
 //      points; the pairs keep their order, and the imaginary difference changes its sign
-//
-// 384 x 384 weights of 240 degrees: the operand takes 69 us to make instead of 95 (half the bytes), the products 87 - 94 us instead
-// of 105 - 114, the weight gradient one launch of 90 us instead of two of 78 and a swapped copy of 31.
 //
 // Multi-GPU use (one process per GPU, buffers mapped through CUDA IPC):
 //   * the k axis of the B operand may be cut into up to 8 segments with their own base pointers and tensor maps

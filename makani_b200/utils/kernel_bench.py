@@ -87,14 +87,26 @@ def cases(H, W, dev, B=1, layout="cl"):
 
     out["conv_wgrad"] = wgrad
 
-    def dft_fwd():
-        from ..ops.spectral import SHTPlan, dft_analysis
-        plan = SHTPlan.get(H, W, H // 3, W // 6 + 1, "equiangular", dev)
-        x = torch.randn(1, C, H, W, device=dev).to(bf).contiguous(memory_format=torch.channels_last)
-        nbytes = C * hw * 2 + plan.k2 * C * H * 2
-        return (lambda: dft_analysis(x, plan.f, False, plan.nlon, plan.k2)), nbytes, 2.0 * plan.k2 * W * C * H
+    def wgrad_bias():
+        dy = lay(torch.randn(1, C, H, W, device=dev).to(bf))
+        x = lay(torch.randn(1, C2, H, W, device=dev).to(bf))
+        return (lambda: _conv_wgrad(dy, x, bias=True)), (C + C2) * hw * 2, 2.0 * C * C2 * hw
 
-    out["dft_analysis"] = dft_fwd
+    out["conv_wgrad_bias"] = wgrad_bias                          # and the bias gradient from the same shared memory
+
+    # longitude transforms as the spherical convolutions run them, whole or folded; operations are those of the whole matrices
+    def dft(h, w, grid, mmax, forward):
+        from ..ops.spectral import SHTPlan, analyse, synthesise
+        plan = SHTPlan.get(h, w, H // 3, mmax, grid, dev)
+        x = torch.randn(1, C, h, w, device=dev).to(bf).contiguous(memory_format=torch.channels_last)
+        t = torch.randn(1, h, plan.k2, C, device=dev).to(bf)
+        fn = (lambda: analyse(x, plan)) if forward else (lambda: synthesise(t, plan))
+        return fn, (x.numel() + t.numel()) * 2, 2.0 * plan.k2 * w * C * h
+
+    out["dft_analysis"] = lambda: dft(H, W, "equiangular", W // 6 + 1, True)
+    out["dft_synthesis"] = lambda: dft(H, W, "equiangular", W // 6 + 1, False)
+    out["dft_analysis_internal"] = lambda: dft(H // 3, W // 3, "legendre-gauss", W // 6 + 1, True)
+    out["dft_synthesis_internal"] = lambda: dft(H // 3, W // 3, "legendre-gauss", W // 6 + 1, False)
 
     def inorm():
         from ..ops.norm import instance_norm
@@ -202,7 +214,7 @@ def main():
                    roofline_seconds=roof, fraction_of_roofline=roof / t, peaks=src)
         results.append(res)
         if not args.json:
-            print(f"{name:18s} {t * 1e3:8.3f} ms  {res['gbytes_per_s']:8.1f} GB/s  {res['tflops']:7.1f} TFLOP/s  "
+            print(f"{name:24s} {t * 1e3:8.3f} ms  {res['gbytes_per_s']:8.1f} GB/s  {res['tflops']:7.1f} TFLOP/s  "
                   f"{100 * res['fraction_of_roofline']:5.1f}% of {src} roofline")
         del fn
         torch.cuda.empty_cache()
