@@ -1296,7 +1296,7 @@ cudaError_t inorm_cl_sums(const __nv_bfloat16* x, const __nv_bfloat16* dy, const
   // mode: bit 0 = backward pass, bit 1 = forward statistics shifted by the first token (local statistics only)
   const int shifted = ((mode >> 1) & 1) && (!xch || xch->npeers == 0);
   mode &= 1;
-  if (!cl_ok(C)) return cudaErrorInvalidValue;
+  if (!cl_ok(C) || !aligned16(x) || !aligned16(dy)) return cudaErrorInvalidValue;      // (16-byte loads)
   StatExchange xc;
   memset(&xc, 0, sizeof(xc));
   if (xch) xc = *xch;
@@ -1316,7 +1316,7 @@ cudaError_t inorm_cl_apply(const __nv_bfloat16* x, const __nv_bfloat16* dy, __nv
   // mode: bit 0 = backward pass, bit 1 = forward statistics shifted by the first token (local statistics only)
   const int shifted = ((mode >> 1) & 1) && (!xch || xch->npeers == 0);
   mode &= 1;
-  if (!cl_ok(C)) return cudaErrorInvalidValue;
+  if (!cl_ok(C) || !aligned16(x) || !aligned16(dy) || !aligned16(out)) return cudaErrorInvalidValue;
   StatExchange xc;
   memset(&xc, 0, sizeof(xc));
   if (xch) xc = *xch;

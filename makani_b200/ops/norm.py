@@ -120,7 +120,7 @@ class _InstanceNormCL(torch.autograd.Function):
 
 def cl_supported(x) -> bool:
     return (_ext.native() and x.is_cuda and x.dtype == torch.bfloat16 and _is_cl(x) and x.shape[1] % 8 == 0
-            and x.shape[1] <= 1024)
+            and x.shape[1] <= 1024 and x.data_ptr() % 16 == 0)
 
 
 def instance_norm(x: torch.Tensor, weight, bias, eps: float = 1e-6, act: str = "none", count=None, reduce_fn=None,

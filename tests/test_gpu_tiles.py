@@ -912,3 +912,17 @@ def test_activations_in_the_epilogue_cost_about_as_much_as_none():
         assert best(act=act, resid=r) < 1.25 * saved
     assert best(act=ACT_DGELU, resid=r) < 1.6 * saved
     assert best(act=ACT_SHRINK, act_param=0.1) < 1.6 * best()
+
+
+def test_norm_of_a_field_off_a_16_byte_boundary():
+    """The channels-last kernels load whole 16-byte vectors; elsewhere the field is copied first, and the kernels themselves refuse it."""
+    from makani_b200.ops.norm import instance_norm
+    dev = _dev()
+    b, c, h, w = 2, 16, 6, 8
+    x = torch.randn(b * h * w * c + 1, device=dev).bfloat16()[1:].view(b, h, w, c).permute(0, 3, 1, 2)
+    assert x.data_ptr() % 16 and x.is_contiguous(memory_format=torch.channels_last)
+    wt, bi = torch.randn(c, device=dev), torch.randn(c, device=dev)
+    ref = torch.nn.functional.instance_norm(x.double(), None, None, wt.double(), bi.double(), eps=1e-6)
+    assert _rel(instance_norm(x, wt, bi, 1e-6), ref) < BF16
+    with pytest.raises(RuntimeError, match="invalid argument"):
+        _ext.require().norm_forward(x, wt, bi, 1e-6, 0, float(h * w))
