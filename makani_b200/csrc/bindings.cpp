@@ -243,6 +243,8 @@ int64_t& launches() {
 
 void check(cudaError_t e, const char* what) { check_cuda(e, what); }
 
+int* error_word(const Tensor& like) { return err_flag_for(like).data_ptr<int>(); }
+
 bool run(const Gemm& g, const mk::GemmPeer* peer) {
   const Tensor &a = *g.A.t, &b = *g.B.t, &d = *g.D.t;
   MK_CHECK(a.is_cuda() && b.is_cuda() && d.is_cuda(), "gemm: tensors must be CUDA");
@@ -611,7 +613,7 @@ void inorm_cl_sums(const Tensor& x, const c10::optional<Tensor>& dy, const c10::
   const bool ex = make_exchange(xc, sync, dsts, true, x);
   check_cuda(mk::inorm_cl_sums(reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()), dyp, f32_ptr(w), f32_ptr(b), f32_ptr(stats), sums.data_ptr<float>(),
                                f32_ptr(dw), f32_ptr(db), static_cast<int>(B), static_cast<int>(C), T, static_cast<int>(act), static_cast<int>(mode),
-                               cur_stream(), ex ? &xc : nullptr),
+                               err_flag_for(x).data_ptr<int>(), cur_stream(), ex ? &xc : nullptr),
              "inorm_cl_sums");
 }
 
@@ -626,7 +628,8 @@ void inorm_cl_apply(const Tensor& x, const c10::optional<Tensor>& dy, Tensor& ou
   const bool ex = make_exchange(xc, sync, srcs, false, x);
   check_cuda(mk::inorm_cl_apply(reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()), dyp, reinterpret_cast<__nv_bfloat16*>(out.data_ptr()),
                                 f32_ptr(w), f32_ptr(b), sums.data_ptr<float>(), f32_ptr(stats), static_cast<int>(B), static_cast<int>(C), T, count,
-                                static_cast<float>(eps), static_cast<int>(act), static_cast<int>(mode), cur_stream(), ex ? &xc : nullptr),
+                                static_cast<float>(eps), static_cast<int>(act), static_cast<int>(mode), err_flag_for(x).data_ptr<int>(), cur_stream(),
+                                ex ? &xc : nullptr),
              "inorm_cl_apply");
 }
 

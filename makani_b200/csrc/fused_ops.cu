@@ -4,6 +4,8 @@
 #include "fused_ops.cuh"
 #include "gelu.cuh"
 #include <cstring>
+#include <type_traits>
+
 
 #include <math.h>
 
@@ -256,10 +258,27 @@ __global__ void __launch_bounds__(NT) inorm_bwd_kernel(const __nv_bfloat16* __re
 }
 
 // ------------------------------------------------------------------------------------------ instance norm, channels-last
-// x: [B, T, C] with C contiguous (C % 8 == 0, C <= 1024).  Thread (v, r) = (tid % V, tid / V), V = C / 8, owns 8
-// channels and walks the tokens r, r + R, ... of its slab, so per-channel constants stay in registers.
+// x: [B, T, C] with C contiguous (C % 8 == 0, C <= 1024).  Thread (v, r) = (tid % V, tid / V), V = C / CH, owns CH
+// channels of every row it meets, so per-channel constants stay in registers.
 
-constexpr int CL_THREADS = 512;
+// The four kernels: channels of a thread, most threads that work on rows (whole rows of them are used, one more warp loads), rows per thread in
+// a stage of the ring and stages.  One CTA per SM.  721 x 1440 x 384, us, by (rows, stages): forward sums (1, 8) 147, (2, 5) 139; forward output
+// (1, 8) 274, (2, 5) 285, (2, 3) 260; gradient with GELU (1, 8) 428, (2, 4) 387, (4, 2) 370, by four channels and 992 threads (4, 3) 389.
+// The backward sums wait for the fp32 pipe and the issue slots, not for rows: without a test per row 330 instead of 352, and by four channels of
+// a thread as by eight, but 51 us instead of 61 at 240 x 480.
+struct ClForwardSums { static constexpr int CH = 8, THREADS = 992, LAPS = 2, DEPTH = 5, TENSORS = 1; };
+struct ClForwardApply { static constexpr int CH = 8, THREADS = 992, LAPS = 2, DEPTH = 3, TENSORS = 1; };
+struct ClBackwardSums { static constexpr int CH = 4, THREADS = 992, LAPS = 4, DEPTH = 3, TENSORS = 2; };
+struct ClBackwardApply { static constexpr int CH = 8, THREADS = 608, LAPS = 4, DEPTH = 2, TENSORS = 2; };
+template <int MODE>
+using ClSums = std::conditional_t<MODE == 0, ClForwardSums, ClBackwardSums>;
+template <int MODE>
+using ClApply = std::conditional_t<MODE == 0, ClForwardApply, ClBackwardApply>;
+template <int CH>
+using ClWord = std::conditional_t<CH == 8, uint4, uint2>;      // the channels of a thread
+template <typename P>
+__host__ __device__ constexpr int cl_ring_bytes(int threads) { return P::DEPTH * P::LAPS * P::TENSORS * 2 * P::CH * threads; }
+constexpr int CL_BARRIERS = 128;      // bytes in front of the ring
 
 // mode 0: sums of (x, x^2).  mode 1: sums of (g, g * xhat) with g = dy * act'(xhat * w + b) for the backward pass.
 __device__ __forceinline__ unsigned int xch_ld_acquire(const unsigned int* ptr) {
@@ -300,54 +319,144 @@ __device__ void xch_signal(const StatExchange& xc) {
     if (xc.sig[peer]) atomicAdd_system(xc.sig[peer], 1u);
 }
 
-// Walks the rows t, t + R, ... below t1 of one 16-byte column (two tensors in the backward pass, MODE 1), ROWS of them in
-// flight per thread, and hands each to `use(t, x, dy)`.
-template <int MODE, int ROWS, typename Use>
-__device__ __forceinline__ void cl_rows(const uint4* xv, const uint4* gv, int V, long long t, long long t1, int R, Use&& use) {
-  for (; t + (ROWS - 1LL) * R < t1; t += static_cast<long long>(ROWS) * R) {
-    uint4 x[ROWS], g[ROWS];
-#pragma unroll
-    for (int u = 0; u < ROWS; ++u) {
-      x[u] = xv[(t + u * R) * V];
-      if (MODE == 1) g[u] = gv[(t + u * R) * V];
+// The rows of one image travel through a ring in shared memory: the last warp of the CTA fetches stages of whole, consecutive rows (of one
+// tensor, or of two in the backward pass) by bulk copies, the others work on them: thread (v, r) on column v of the rows r, r + R, ... of a
+// stage, handed to `use(t, x, dy)` (V columns of ClWord, the channels of a thread).  The copies never wait for the arithmetic (GELU' of
+// every element) and no registers hold rows on their way.  With the rows in registers, loaded four at a time, load and arithmetic took turns;
+// copied by every thread for itself (cp.async), 721 x 1440 tokens took 5 % longer than that, and with the stages of a CTA following one
+// another (here they are dealt out over the CTAs: all read one window of some MB that moves through the tensor) 8 %.
+__device__ __forceinline__ bool cl_wait(uint32_t bar, uint32_t parity, int* err) {
+  unsigned long long t0 = 0;
+  for (uint32_t it = 0;; ++it) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred P1;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, P1;\n\t"
+        "}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (ok) return true;
+    if ((it & 63u) == 63u) {
+      const unsigned long long now = xch_ns();
+      if (t0 == 0) t0 = now;
+      else if (now - t0 > 2000000000ull) {
+        if (err) atomicExch(err, 58);
+        return false;
+      }
     }
-#pragma unroll
-    for (int u = 0; u < ROWS; ++u) use(t + u * R, x[u], MODE == 1 ? g[u] : x[u]);
-  }
-  for (; t < t1; t += R) {
-    const uint4 x = xv[t * V];
-    use(t, x, MODE == 1 ? gv[t * V] : x);
   }
 }
+__device__ __forceinline__ void cl_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
+}
+template <typename P>
+__device__ __forceinline__ void cl_init(uint4* smem) {      // (by all threads, once; a barrier of the CTA before cl_rows)
+  if (threadIdx.x == 0) {
+    const uint32_t bars = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
+    for (int i = 0; i < P::DEPTH; ++i) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bars + 16 * i), "r"(1u));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bars + 16 * i + 8), "r"(blockDim.x / 32 - 1));
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+}
+template <typename P, bool BACK, typename Use>
+__device__ __forceinline__ void cl_rows(uint4* smem, const __nv_bfloat16* x, const __nv_bfloat16* dy, int V, int r, int R, long long T, int* err,
+                                        Use&& use) {
+  using Word = ClWord<P::CH>;
+  static_assert(P::DEPTH * 16 <= CL_BARRIERS && P::DEPTH * P::LAPS * P::TENSORS >= 4, "the partial sums take the ring's place");
+  const uint32_t bars = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
+  const Word* const ring = reinterpret_cast<const Word*>(smem + CL_BARRIERS / 16);
+  const int rows = P::LAPS * R, half = rows * V;      // rows and words of one tensor in a stage
+  const long long hop = static_cast<long long>(gridDim.x) * rows;
+  const long long stages = (T + rows - 1) / rows;
+  const int count = blockIdx.x < stages ? static_cast<int>((stages - 1 - blockIdx.x) / gridDim.x) + 1 : 0;
+  long long t = static_cast<long long>(blockIdx.x + (BACK ? (count - 1LL) * gridDim.x : 0)) * rows;
+  int s = 0;
+  uint32_t ph = 0;
+  auto next = [&]() {
+    t += BACK ? -hop : hop;
+    if (++s == P::DEPTH) {
+      s = 0;
+      ph ^= 1u;
+    }
+  };
+  if (threadIdx.x / 32 == blockDim.x / 32 - 1) {
+    if ((threadIdx.x & 31) == 0) {
+      const uint32_t dst = bars + CL_BARRIERS, row = V * sizeof(Word);
+      for (int k = 0; k < count; ++k, next()) {
+        if (!cl_wait(bars + 16 * s + 8, ph ^ 1u, err)) break;
+        const uint32_t bytes = static_cast<uint32_t>(min(static_cast<long long>(rows), T - t)) * row;
+        const uint32_t at = dst + s * P::TENSORS * rows * row;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bars + 16 * s), "r"(P::TENSORS * bytes) : "memory");
+        cl_copy(at, reinterpret_cast<const char*>(x) + t * row, bytes, bars + 16 * s);
+        if (P::TENSORS == 2) cl_copy(at + rows * row, reinterpret_cast<const char*>(dy) + t * row, bytes, bars + 16 * s);
+      }
+    }
+    return;
+  }
+  for (int k = 0; k < count; ++k, next()) {
+    if (!cl_wait(bars + 16 * s, ph, err)) break;
+    const Word* at = ring + s * P::TENSORS * half + threadIdx.x;
+    if (r < R) {
+      if (t + rows <= T) {
+#pragma unroll
+        for (int u = 0; u < P::LAPS; ++u) use(t + u * R + r, at[u * R * V], at[u * R * V + (P::TENSORS == 1 ? 0 : half)]);
+      } else {
+#pragma unroll 1
+        for (int i = r; i < T - t; i += R, at += R * V) use(t + i, at[0], at[P::TENSORS == 1 ? 0 : half]);
+      }
+    }
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bars + 16 * s + 8) : "memory");
+  }
+}
+// bf16 channels of a thread as pairs of fp32
+__device__ __forceinline__ void cl_unpack(const uint4& w, f32x2 (&f)[4]) { f2_unpack8(w, f); }
+__device__ __forceinline__ void cl_unpack(const uint2& w, f32x2 (&f)[2]) {
+  f[0] = f2_pack(__uint_as_float(w.x << 16), __uint_as_float(w.x & 0xffff0000u));
+  f[1] = f2_pack(__uint_as_float(w.y << 16), __uint_as_float(w.y & 0xffff0000u));
+}
 
-// Two CTAs per SM for the forward kernels; the backward ones hold their constants and eight loads in the 128 registers that one
-// CTA leaves (four registers of the sums kernel do not fit and are spilled).
 template <int MODE>
-__global__ void __launch_bounds__(CL_THREADS, MODE == 0 ? 2 : 1) inorm_cl_sums_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
+__global__ void __launch_bounds__(ClSums<MODE>::THREADS + 32, 1) inorm_cl_sums_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
                                                                    const float* __restrict__ w, const float* __restrict__ b,
                                                                    const float* __restrict__ stats, float* __restrict__ sums,
                                                                    float* __restrict__ dw, float* __restrict__ db, int C, long long T,
-                                                                   int act, int slab, int shifted, const StatExchange xc) {
-  extern __shared__ float sh_acc[];   // [C][2]
-  const GeluPairs gc = gelu_pairs(coef_of(act));
-  const int V = C >> 3;
-  const int R = CL_THREADS / V;
+                                                                   int act, int shifted, const StatExchange xc) {
+  extern __shared__ __align__(16) uint4 cl_ring[];
+  GeluBwdPairs gc;
+  if constexpr (MODE == 1) gc = gelu_bwd_pairs(coef_of(act));
+  using P = ClSums<MODE>;
+  using Word = ClWord<P::CH>;
+  constexpr int PAIRS = P::CH / 2;
+  const int V = C / P::CH;
+  const int R = (static_cast<int>(blockDim.x) - 32) / V;
   const int v = threadIdx.x % V, r = threadIdx.x / V;
   const int bidx = blockIdx.y;
-  for (int i = threadIdx.x; i < 2 * C; i += CL_THREADS) sh_acc[i] = 0.f;
+  cl_init<P>(cl_ring);
   __syncthreads();
-  if (r < R) {
-    // Pairs of channels in packed fp32 arithmetic: with scalar instructions the backward pass (GELU' twice per element over
-    // both kernels) was bound by instruction issue, not by HBM.  721 x 1440 x 384 with GELU: sums 418 -> 347 us, gradient
-    // 471 -> 418 us (2.4 GB, 5.7 TB/s); forward sums 148 -> 135 us, output 268 -> 264 us (6.0 TB/s).
+  // partial sums of the rows of threads, in the ring's place: those of row r from C r on, sums before products
+  f32x2* const part = reinterpret_cast<f32x2*>(cl_ring);
+  f32x2 a0[PAIRS], a1[PAIRS];
+  {
+    // Pairs of channels in packed fp32 arithmetic: a packed instruction takes two cycles of a scheduler's fp32 pipe, three where it reads three
+    // different register pairs, but one issue slot (GELU' with the polynomials by single instructions, whose coefficients need no
+    // registers: sums 330 us instead of 305).  721 x 1440 x 384 with GELU, rows in registers -> through the ring: forward 413 -> 393 us,
+    // backward 775 -> 657 (without GELU 413 -> 392, 650 -> 617); 240 x 480: 83 -> 64, 140 -> 101; 97 x 192: 48 -> 34, 67 -> 42.
+    // Both passes one after the other without a pause, under the power cap: 1222 -> 1107.
     // Backward: pre = x ka + kb with ka = w rstd, kb = b - mean ka is the value the forward pass activated, and
     // sum g xhat = rstd sum g (x - mean).
-    f32x2 a0[4], a1[4], nmean[4], ka[4], kb[4];
+    f32x2 nmean[PAIRS], ka[PAIRS], kb[PAIRS];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < PAIRS; ++j) {
       a0[j] = a1[j] = f2_pack(0.f, 0.f);
       if (MODE == 1) {
-        const int c = v * 8 + 2 * j;
+        const int c = v * P::CH + 2 * j;
         const float4 st = *reinterpret_cast<const float4*>(stats + (static_cast<long long>(bidx) * C + c) * 2);
         const float a = (w ? w[c] : 1.f) * st.y, d = (w ? w[c + 1] : 1.f) * st.w;
         nmean[j] = f2_pack(-st.x, -st.z);
@@ -355,37 +464,34 @@ __global__ void __launch_bounds__(CL_THREADS, MODE == 0 ? 2 : 1) inorm_cl_sums_k
         kb[j] = f2_pack((b ? b[c] : 0.f) - st.x * a, (b ? b[c + 1] : 0.f) - st.z * d);
       }
     }
-    const long long t0 = static_cast<long long>(blockIdx.x) * slab;
-    long long t1 = t0 + slab;
-    if (t1 > T) t1 = T;
-    const uint4* xv = reinterpret_cast<const uint4*>(x + static_cast<long long>(bidx) * T * C) + v;
-    const uint4* gv = MODE == 1 ? reinterpret_cast<const uint4*>(dy + static_cast<long long>(bidx) * T * C) + v : nullptr;
+    const __nv_bfloat16* const xb = x + static_cast<long long>(bidx) * T * C;
+    const __nv_bfloat16* const gb = MODE == 1 ? dy + static_cast<long long>(bidx) * T * C : nullptr;
     // Shifted sums: sum (x - s) and sum (x - s)^2 with s = the sample's first token, so that the one-pass variance
     // E[(x-s)^2] - E[x-s]^2 does not cancel when |mean| >> std.  (Only when the statistics are local to this device:
     // sums that are merged across ranks need one common shift and stay unshifted.)
-    f32x2 nsft[4];
+    f32x2 nsft[PAIRS];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) nsft[j] = f2_pack(0.f, 0.f);
+    for (int j = 0; j < PAIRS; ++j) nsft[j] = f2_pack(0.f, 0.f);
     if (MODE == 0 && shifted) {
-      f2_unpack8(xv[0], nsft);
+      cl_unpack(reinterpret_cast<const Word*>(xb)[v], nsft);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) nsft[j] = f2_mul(nsft[j], f2_pack(-1.f, -1.f));
+      for (int j = 0; j < PAIRS; ++j) nsft[j] = f2_mul(nsft[j], f2_pack(-1.f, -1.f));
     }
-    auto accum = [&](const uint4& xr, const uint4& gr) {
-      f32x2 f[4];
-      f2_unpack8(xr, f);
-      if (MODE == 0) {
+    auto accum = [&](const Word& xr, const Word& gr) {
+      f32x2 f[PAIRS];
+      cl_unpack(xr, f);
+      if constexpr (MODE == 0) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < PAIRS; ++j) {
           const f32x2 d = f2_add(f[j], nsft[j]);
           a0[j] = f2_add(a0[j], d);
           a1[j] = f2_fma(d, d, a1[j]);
         }
       } else {
-        f32x2 g[4];
-        f2_unpack8(gr, g);
+        f32x2 g[PAIRS];
+        cl_unpack(gr, g);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < PAIRS; ++j) {
           f32x2 gg = g[j];
           if (act) gg = f2_mul(gg, gelu_bwd2(f2_fma(f[j], ka[j], kb[j]), gc));
           a0[j] = f2_add(a0[j], gg);
@@ -393,55 +499,68 @@ __global__ void __launch_bounds__(CL_THREADS, MODE == 0 ? 2 : 1) inorm_cl_sums_k
         }
       }
     };
-    cl_rows<MODE, 4>(xv, gv, V, t0 + r, t1, R, [&](long long, const uint4& xr, const uint4& gr) { accum(xr, gr); });
+    cl_rows<P, false>(cl_ring, xb, gb, V, r, R, T, xc.err, [&](long long, const Word& xr, const Word& gr) { accum(xr, gr); });
     if (MODE == 1) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int c = v * 8 + 2 * j;
+      for (int j = 0; j < PAIRS; ++j) {
+        const int c = v * P::CH + 2 * j;
         const float4 st = *reinterpret_cast<const float4*>(stats + (static_cast<long long>(bidx) * C + c) * 2);
         a1[j] = f2_mul(a1[j], f2_pack(st.y, st.w));
       }
     }
-    // Few channels: the lanes of a warp that own the same ones (V a power of two below 32) are summed by shuffles first.
-    // At 16 channels 256 threads added to the same 32 words: 37 us for a 2048-token image.
-    const bool fold = V < 32 && (V & (V - 1)) == 0;
-    if (fold) {
-      for (int o = 16; o >= V; o >>= 1) {
+  }
+  // Added up without atomics: those on fp32 in shared memory are loops of compare and swap, and with R threads on each word the end of a CTA
+  // took some 14 us.
+  __syncthreads();
+  const int words = C / 2;      // pairs of channels
+  if (r < R) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          a0[j] = f2_add(a0[j], __shfl_xor_sync(0xffffffffu, a0[j], o));
-          a1[j] = f2_add(a1[j], __shfl_xor_sync(0xffffffffu, a1[j], o));
-        }
-      }
-    }
-    if (!fold || (threadIdx.x & 31) < V) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        float s0, s1, q0, q1;
-        f2_unpack(a0[j], s0, s1);
-        f2_unpack(a1[j], q0, q1);
-        float* const acc = &sh_acc[(v * 8 + 2 * j) * 2];
-        atomicAdd(acc, s0);
-        atomicAdd(acc + 1, q0);
-        atomicAdd(acc + 2, s1);
-        atomicAdd(acc + 3, q1);
-      }
+    for (int j = 0; j < PAIRS; ++j) {
+      part[r * C + j * V + v] = a0[j];
+      part[r * C + words + j * V + v] = a1[j];
     }
   }
   __syncthreads();
-  // one 16-byte vector atomic per two channels (C is a multiple of 8, the buffer is 16-byte aligned)
-  for (int i = threadIdx.x * 4; i < 2 * C; i += CL_THREADS * 4) {
-    const float4 val = *reinterpret_cast<const float4*>(sh_acc + i);
-    atomicAdd(reinterpret_cast<float4*>(sums + static_cast<long long>(bidx) * 2 * C + i), val);
+  // in two steps where many rows of threads meet: S parts of the rows, then these
+  const int S = min(min(R, 32), static_cast<int>(blockDim.x) / words);
+  if (S > 1) {
+    const int g = threadIdx.x / words, at = threadIdx.x - g * words;
+    f32x2 s = f2_pack(0.f, 0.f), q = s;
+    if (g < S) {
+      for (int k = g; k < R; k += S) {
+        s = f2_add(s, part[k * C + at]);
+        q = f2_add(q, part[k * C + words + at]);
+      }
+    }
+    __syncthreads();
+    if (g < S) {
+      part[g * C + at] = s;
+      part[g * C + words + at] = q;
+    }
+    __syncthreads();
+  }
+  const int left = S > 1 ? S : R;
+  for (int i = threadIdx.x; i < words; i += blockDim.x) {
+    const int j = i / V, vv = i - j * V;
+    f32x2 s = f2_pack(0.f, 0.f), q = s;
+    for (int k = 0; k < left; ++k) {
+      s = f2_add(s, part[k * C + i]);
+      q = f2_add(q, part[k * C + words + i]);
+    }
+    float s0, s1, q0, q1;
+    f2_unpack(s, s0, s1);
+    f2_unpack(q, q0, q1);
+    const int c = vv * P::CH + 2 * j;
+    // one 16-byte vector atomic per two channels (C is a multiple of 8, the buffer is 16-byte aligned)
+    atomicAdd(reinterpret_cast<float4*>(sums + (static_cast<long long>(bidx) * C + c) * 2), make_float4(s0, q0, s1, q1));
     if (MODE == 1) {
-      const int c = i >> 1;
       if (db) {
-        atomicAdd(db + c, val.x);
-        atomicAdd(db + c + 1, val.z);
+        atomicAdd(db + c, s0);
+        atomicAdd(db + c + 1, s1);
       }
       if (dw) {
-        atomicAdd(dw + c, val.y);
-        atomicAdd(dw + c + 1, val.w);
+        atomicAdd(dw + c, q0);
+        atomicAdd(dw + c + 1, q1);
       }
     }
   }
@@ -460,7 +579,7 @@ __global__ void __launch_bounds__(CL_THREADS, MODE == 0 ? 2 : 1) inorm_cl_sums_k
     if (last_s == 1) {
       __threadfence();
       const int n = static_cast<int>(gridDim.y) * 2 * C;
-      for (int i = threadIdx.x; i < n; i += CL_THREADS) {
+      for (int i = threadIdx.x; i < n; i += blockDim.x) {
         const float val = __ldcg(sums + i);
         for (int q = 0; q < xc.ndst; ++q) xc.dst[q][i] = val;
       }
@@ -476,16 +595,20 @@ __global__ void __launch_bounds__(CL_THREADS, MODE == 0 ? 2 : 1) inorm_cl_sums_k
 // mode 0: y = act(xhat * w + b), statistics derived from `sums` (and stored to `stats`).
 // mode 1: dx = rstd * w * (g - s1/T - xhat * s2/T) with (s1, s2) in `sums`, (mean, rstd) in `stats`.
 template <int MODE>
-__global__ void __launch_bounds__(CL_THREADS, MODE == 0 ? 2 : 1) inorm_cl_apply_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
+__global__ void __launch_bounds__(ClApply<MODE>::THREADS + 32, 1) inorm_cl_apply_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
                                                                     __nv_bfloat16* __restrict__ out, const float* __restrict__ w,
                                                                     const float* __restrict__ b, const float* __restrict__ sums,
                                                                     float* __restrict__ stats, int C, long long T, float inv_count,
-                                                                    float eps, int act, int slab, int shifted, const StatExchange xc) {
+                                                                    float eps, int act, int shifted, const StatExchange xc) {
+  using P = ClApply<MODE>;
   const int V = C >> 3;
-  const int R = CL_THREADS / V;
+  const int R = (static_cast<int>(blockDim.x) - 32) / V;
   const int v = threadIdx.x % V, r = threadIdx.x / V;
   const int bidx = blockIdx.y;
-  extern __shared__ float sh_sum[];   // [C][2] merged sums of this sample (exchange mode only)
+  extern __shared__ __align__(16) uint4 cl_ring[];
+  // [C][2] merged sums of this sample (exchange mode only), behind the ring
+  float* const sh_sum = reinterpret_cast<float*>(cl_ring + CL_BARRIERS / 16 + P::DEPTH * P::LAPS * P::TENSORS * R * V);
+  cl_init<P>(cl_ring);
   if (xc.npeers > 0) {
     // every peer's sums must have arrived in the local buffer
     __shared__ int ok_s;
@@ -494,18 +617,17 @@ __global__ void __launch_bounds__(CL_THREADS, MODE == 0 ? 2 : 1) inorm_cl_apply_
     if (!ok_s) return;
     // merge the segments once per CTA (coalesced, L1 bypassed: the buffer is rewritten by peers between launches);
     // fixed order, so every rank computes bit-identical statistics
-    for (int i = threadIdx.x; i < 2 * C; i += CL_THREADS) {
+    for (int i = threadIdx.x; i < 2 * C; i += blockDim.x) {
       float acc = 0.f;
       for (int q = 0; q < xc.nsrc; ++q) acc += __ldcg(xc.src + q * xc.src_stride + static_cast<long long>(bidx) * 2 * C + i);
       sh_sum[i] = acc;
     }
     __syncthreads();
   }
-  if (r >= R) {
-    if (xc.npeers > 0) __syncthreads();   // matches the barrier before the completion count below
-    return;
-  }
-  const GeluPairs gc = gelu_pairs(coef_of(act));
+  __syncthreads();
+  std::conditional_t<MODE == 0, GeluPairs, GeluBwdPairs> gc;
+  if constexpr (MODE == 0) gc = gelu_pairs(coef_of(act));
+  else gc = gelu_bwd_pairs(coef_of(act));
   // per-channel constants, two channels each.  Forward: y = act(x ka + kb).  Backward: dx = ka (g + k1 + (x - mean) k2)
   f32x2 ka[4], kb[4], nmean[4], k1[4], k2[4];
   float sft[8];                                      // shift of the statistics pass (the sample's first token) or 0
@@ -556,17 +678,12 @@ __global__ void __launch_bounds__(CL_THREADS, MODE == 0 ? 2 : 1) inorm_cl_apply_
       k2[j] = f2_pack(v2[0], v2[1]);
     }
   }
-  const long long t0 = static_cast<long long>(blockIdx.x) * slab;
-  long long t1 = t0 + slab;
-  if (t1 > T) t1 = T;
   const long long base = static_cast<long long>(bidx) * T * C;
-  const uint4* xv = reinterpret_cast<const uint4*>(x + base) + v;
-  const uint4* gv = MODE == 1 ? reinterpret_cast<const uint4*>(dy + base) + v : nullptr;
   uint4* ov = reinterpret_cast<uint4*>(out + base) + v;
   auto transform = [&](const uint4& xr, const uint4& gr) -> uint4 {
     f32x2 f[4];
     f2_unpack8(xr, f);
-    if (MODE == 0) {
+    if constexpr (MODE == 0) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         f[j] = f2_fma(f[j], ka[j], kb[j]);
@@ -584,8 +701,8 @@ __global__ void __launch_bounds__(CL_THREADS, MODE == 0 ? 2 : 1) inorm_cl_apply_
     }
     return f2_bf16x8(f);
   };
-  cl_rows<MODE, MODE == 0 ? 3 : 4>(xv, gv, V, t0 + r, t1, R,
-                                   [&](long long t, const uint4& xr, const uint4& gr) { ov[t * V] = transform(xr, gr); });
+  // From the end: the last rows that the sums' pass has read are still in L2
+  cl_rows<P, true>(cl_ring, x + base, MODE == 1 ? dy + base : nullptr, V, r, R, T, xc.err, [&](long long t, const uint4& xr, const uint4& gr) { ov[t * V] = transform(xr, gr); });
   if (xc.npeers > 0) {
     // the last CTA tells the peers that this rank is done with their sums
     __syncthreads();
@@ -1279,18 +1396,28 @@ cudaError_t inorm_bwd(const __nv_bfloat16* x, const __nv_bfloat16* dy, __nv_bflo
   return cudaGetLastError();
 }
 
-static inline bool cl_ok(int C) { return C % 8 == 0 && C >= 8 && C <= 1024 && (CL_THREADS / (C / 8)) >= 1; }
-// tokens per CTA: enough CTAs to fill the machine a few times over, but at least a few passes of the row loop each
-static inline int cl_slab(int C, long long T, int B, int ctas_per_sm = 4) {
-  const int R = CL_THREADS / (C / 8);
-  long long target = (static_cast<long long>(ctas_per_sm) * sm_count() + B - 1) / B;
-  long long slab = (T + target - 1) / target;
-  if (slab < 4LL * R) slab = 4LL * R;
-  return static_cast<int>(slab);
+static inline bool cl_ok(int C) { return C % 8 == 0 && C >= 8 && C <= 1024; }
+namespace {
+// One CTA per SM, all of them at once, and no more than there are stages.  Small fields spread over the SMs by smaller CTAs.
+constexpr int CL_FEWEST = 128;      // threads (2048 x 16, both passes: 28 us, from CTAs of full size 40, with rows in registers 34)
+template <typename P, typename Kernel, typename... Args>
+cudaError_t cl_launch(Kernel* kernel, int C, long long T, int B, size_t fixed, cudaStream_t stream, Args... args) {
+  static const cudaError_t allowed = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                          CL_BARRIERS + cl_ring_bytes<P>(P::THREADS) + 2 * 1024 * static_cast<int>(sizeof(float)));
+  if (allowed != cudaSuccess) return allowed;
+  const int V = C / P::CH;
+  const long long most = std::max(1, sm_count() / B);
+  const long long share = (T + P::LAPS * most - 1) / (P::LAPS * most);      // rows of threads that would give every CTA one stage
+  const int R = static_cast<int>(std::min<long long>(P::THREADS / V, std::max<long long>(share, (CL_FEWEST + V - 1) / V)));
+  const long long need = (T + P::LAPS * R - 1) / (P::LAPS * R);
+  const dim3 grid(static_cast<unsigned>(std::min(most, need)), B);
+  kernel<<<grid, (V * R + 31) / 32 * 32 + 32, CL_BARRIERS + cl_ring_bytes<P>(V * R) + fixed, stream>>>(args...);
+  return cudaGetLastError();
 }
+}  // namespace
 
 cudaError_t inorm_cl_sums(const __nv_bfloat16* x, const __nv_bfloat16* dy, const float* w, const float* b, const float* stats,
-                          float* sums, float* dw, float* db, int B, int C, long long T, int act, int mode, cudaStream_t s,
+                          float* sums, float* dw, float* db, int B, int C, long long T, int act, int mode, int* err, cudaStream_t s,
                           const StatExchange* xch) {
   if (act) act = gelu_tanh() ? 2 : 1;
   // mode: bit 0 = backward pass, bit 1 = forward statistics shifted by the first token (local statistics only)
@@ -1299,18 +1426,15 @@ cudaError_t inorm_cl_sums(const __nv_bfloat16* x, const __nv_bfloat16* dy, const
   if (!cl_ok(C) || !aligned16(x) || !aligned16(dy)) return cudaErrorInvalidValue;      // (16-byte loads)
   StatExchange xc;
   memset(&xc, 0, sizeof(xc));
+  xc.err = err;
   if (xch) xc = *xch;
-  // every CTA ends with 2C atomics on the same [B, C, 2] words: fewer, longer CTAs than the streaming pass
-  const int slab = cl_slab(C, T, B, 2);
-  dim3 grid(static_cast<unsigned>((T + slab - 1) / slab), B);
-  const size_t sh = 2 * C * sizeof(float);
-  if (mode == 0) inorm_cl_sums_kernel<0><<<grid, CL_THREADS, sh, s>>>(x, dy, w, b, stats, sums, dw, db, C, T, act, slab, shifted, xc);
-  else inorm_cl_sums_kernel<1><<<grid, CL_THREADS, sh, s>>>(x, dy, w, b, stats, sums, dw, db, C, T, act, slab, 0, xc);
-  return cudaGetLastError();
+  if (mode == 0)
+    return cl_launch<ClSums<0>>(inorm_cl_sums_kernel<0>, C, T, B, 0, s, x, dy, w, b, stats, sums, dw, db, C, T, act, shifted, xc);
+  return cl_launch<ClSums<1>>(inorm_cl_sums_kernel<1>, C, T, B, 0, s, x, dy, w, b, stats, sums, dw, db, C, T, act, 0, xc);
 }
 
 cudaError_t inorm_cl_apply(const __nv_bfloat16* x, const __nv_bfloat16* dy, __nv_bfloat16* out, const float* w, const float* b,
-                           const float* sums, float* stats, int B, int C, long long T, double count, float eps, int act, int mode,
+                           const float* sums, float* stats, int B, int C, long long T, double count, float eps, int act, int mode, int* err,
                            cudaStream_t s, const StatExchange* xch) {
   if (act) act = gelu_tanh() ? 2 : 1;
   // mode: bit 0 = backward pass, bit 1 = forward statistics shifted by the first token (local statistics only)
@@ -1319,14 +1443,13 @@ cudaError_t inorm_cl_apply(const __nv_bfloat16* x, const __nv_bfloat16* dy, __nv
   if (!cl_ok(C) || !aligned16(x) || !aligned16(dy) || !aligned16(out)) return cudaErrorInvalidValue;
   StatExchange xc;
   memset(&xc, 0, sizeof(xc));
+  xc.err = err;
   if (xch) xc = *xch;
-  const int slab = cl_slab(C, T, B);
-  dim3 grid(static_cast<unsigned>((T + slab - 1) / slab), B);
   const float inv = static_cast<float>(1.0 / count);
   const size_t shx = xc.npeers > 0 ? 2 * C * sizeof(float) : 0;
-  if (mode == 0) inorm_cl_apply_kernel<0><<<grid, CL_THREADS, shx, s>>>(x, dy, out, w, b, sums, stats, C, T, inv, eps, act, slab, shifted, xc);
-  else inorm_cl_apply_kernel<1><<<grid, CL_THREADS, shx, s>>>(x, dy, out, w, b, sums, stats, C, T, inv, eps, act, slab, 0, xc);
-  return cudaGetLastError();
+  if (mode == 0)
+    return cl_launch<ClApply<0>>(inorm_cl_apply_kernel<0>, C, T, B, shx, s, x, dy, out, w, b, sums, stats, C, T, inv, eps, act, shifted, xc);
+  return cl_launch<ClApply<1>>(inorm_cl_apply_kernel<1>, C, T, B, shx, s, x, dy, out, w, b, sums, stats, C, T, inv, eps, act, 0, xc);
 }
 
 namespace {

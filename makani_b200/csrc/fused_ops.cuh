@@ -47,16 +47,16 @@ struct StatExchange {
 };
 
 // ---- instance norm on channels-last data x[B, T, C] (C contiguous, C % 8 == 0, C <= 1024) ----
-// sums: [B, C, 2] fp32, zero-initialised by the caller, accumulated atomically.
+// sums: [B, C, 2] fp32, zero-initialised by the caller, accumulated atomically.  `err`: the device error word, for bounded waits.
 //   mode 0: (sum x, sum x^2);   mode 1: (sum g, sum g*xhat), also accumulated over B into dw / db.
 cudaError_t inorm_cl_sums(const __nv_bfloat16* x, const __nv_bfloat16* dy, const float* w, const float* b, const float* stats,
-                          float* sums, float* dw, float* db, int B, int C, long long T, int act, int mode, cudaStream_t s,
+                          float* sums, float* dw, float* db, int B, int C, long long T, int act, int mode, int* err, cudaStream_t s,
                           const StatExchange* xch = nullptr);
 // mode 0: out = act(xhat * w + b) with statistics from `sums` over `count` elements (stats [B, C, 2] written);
 // mode 1: out = dx from the merged backward sums.
 cudaError_t inorm_cl_apply(const __nv_bfloat16* x, const __nv_bfloat16* dy, __nv_bfloat16* out, const float* w, const float* b,
                            const float* sums, float* stats, int B, int C, long long T, double count, float eps, int act, int mode,
-                           cudaStream_t s, const StatExchange* xch = nullptr);
+                           int* err, cudaStream_t s, const StatExchange* xch = nullptr);
 
 // out[g, c] = sum over the rows of group g of x (C % 8 == 0, 16-byte aligned), in one fixed order; `scratch` holds
 // colsum_scratch() floats.  Row r of group g: g * gstride + (r / inner) * ostride + (r % inner) * C; inner = 0: rows follow

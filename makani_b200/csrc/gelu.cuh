@@ -140,13 +140,22 @@ __device__ __forceinline__ f32x2 gelu_fwd2(f32x2 x, const GeluPairs& c) {
   const f32x2 hx = f2_mul(x, c.half);
   return f2_fma(hx, f2_tanh(f2_mul(x, q)), hx);
 }
-__device__ __forceinline__ f32x2 gelu_bwd2(f32x2 x, const GeluPairs& c) {
+// The derivative by itself, a + a (1 - t) x dq with a = (1 + t) / 2, one instruction less than beside the function: through
+// -t = tanh(-x q), as the packed instructions have no negation
+struct GeluBwdPairs {
+  f32x2 m0, m1, m2, d0, d1, d2, half, nhalf;
+};
+__device__ __forceinline__ GeluBwdPairs gelu_bwd_pairs(const GeluCoef& c) {
+  return GeluBwdPairs{f2_keep(-c.c0), f2_keep(-c.c1), f2_keep(-c.c2), f2_keep(c.c0), f2_keep(3.f * c.c1), f2_keep(5.f * c.c2), f2_keep(0.5f),
+                      f2_keep(-0.5f)};
+}
+__device__ __forceinline__ f32x2 gelu_bwd2(f32x2 x, const GeluBwdPairs& c) {
   const f32x2 u = f2_clamp36(f2_mul(x, x));
-  const f32x2 q = f2_fma(u, f2_fma(u, c.c2, c.c1), c.c0);
-  const f32x2 ndq = f2_fma(u, f2_fma(u, c.n2, c.n1), c.n0);
-  const f32x2 t = f2_tanh(f2_mul(x, q));
-  const f32x2 s = f2_fma(t, t, c.neg1);
-  return f2_fma(f2_mul(f2_mul(x, c.half), s), ndq, f2_fma(t, c.half, c.half));
+  const f32x2 mq = f2_fma(u, f2_fma(u, c.m2, c.m1), c.m0);
+  const f32x2 dq = f2_fma(u, f2_fma(u, c.d2, c.d1), c.d0);
+  const f32x2 mt = f2_tanh(f2_mul(x, mq));
+  const f32x2 a = f2_fma(mt, c.nhalf, c.half);
+  return f2_fma(f2_mul(f2_fma(mt, a, a), x), dq, a);
 }
 __device__ __forceinline__ void gelu_fwd_bwd2(f32x2 x, const GeluPairs& c, f32x2& y, f32x2& dy) {
   const f32x2 u = f2_clamp36(f2_mul(x, x));

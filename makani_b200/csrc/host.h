@@ -60,6 +60,8 @@ void complex_product(const Tensor& a, const Tensor& b, Tensor& d, const Tensor* 
 void folded_product(const Tensor& a, const Tensor& b, Tensor& d, const std::vector<int64_t>& ip);
 
 void check(cudaError_t e, const char* what);
+// the device error word that kernels with bounded waits report to
+int* error_word(const Tensor& like);
 inline cudaStream_t stream() { return at::cuda::getCurrentCUDAStream().stream(); }
 
 // kernel launches of this thread's layer passes

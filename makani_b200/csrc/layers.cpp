@@ -263,10 +263,11 @@ std::tuple<Tensor, Tensor, OptTensor, OptTensor> norm_forward(const Tensor& x, c
   // statistics local to this device are accumulated around the first token (mode bit 1): no cancellation in E[x^2] - E[x]^2 for
   // fields with |mean| >> std
   mkh::check(mk::inorm_cl_sums(bf(x), nullptr, nullptr, nullptr, nullptr, sums.data_ptr<float>(), nullptr, nullptr, static_cast<int>(B),
-                               static_cast<int>(C), T, 0, 2, mkh::stream()),
+                               static_cast<int>(C), T, 0, 2, mkh::error_word(x), mkh::stream()),
              "inorm_cl_sums");
   mkh::check(mk::inorm_cl_apply(bf(x), nullptr, bf_mut(y), f32_or_null(w), f32_or_null(b), sums.data_ptr<float>(), stats.data_ptr<float>(),
-                                static_cast<int>(B), static_cast<int>(C), T, count, static_cast<float>(eps), static_cast<int>(act), 2, mkh::stream()),
+                                static_cast<int>(B), static_cast<int>(C), T, count, static_cast<float>(eps), static_cast<int>(act), 2, mkh::error_word(x),
+                                mkh::stream()),
              "inorm_cl_apply");
   return {y, stats, maybe(w), maybe(b)};
 }
@@ -286,10 +287,11 @@ std::tuple<Tensor, OptTensor, OptTensor> norm_backward(const Tensor& x, const Te
   }
   mkh::launches() += 2;
   mkh::check(mk::inorm_cl_sums(bf(x), bf(dy), f32_or_null(w), f32_or_null(b), stats.data_ptr<float>(), acc.data_ptr<float>(), f32_mut(dw), f32_mut(db),
-                               static_cast<int>(B), static_cast<int>(C), T, static_cast<int>(act), 1, mkh::stream()),
+                               static_cast<int>(B), static_cast<int>(C), T, static_cast<int>(act), 1, mkh::error_word(x), mkh::stream()),
              "inorm_cl_sums");
   mkh::check(mk::inorm_cl_apply(bf(x), bf(dy), bf_mut(dx), f32_or_null(w), f32_or_null(b), acc.data_ptr<float>(), stats.data_ptr<float>(),
-                                static_cast<int>(B), static_cast<int>(C), T, count, 0.f, static_cast<int>(act), 1, mkh::stream()),
+                                static_cast<int>(B), static_cast<int>(C), T, count, 0.f, static_cast<int>(act), 1, mkh::error_word(x),
+                                mkh::stream()),
              "inorm_cl_apply");
   return {dx, maybe(dw), maybe(db)};
 }

@@ -162,6 +162,43 @@ def test_instance_norm_channel_counts(b, c, h, w, act):
         assert _rel(a, r) < BF16
 
 
+@pytest.mark.parametrize("b,c,h,w", [
+    (1, 384, 1, 1), (1, 8, 1, 3),            # fewer rows than threads
+    (1, 384, 7, 7), (1, 384, 1, 50), (1, 384, 3, 17),      # a stage of 50 (forward) or 40 and 24 rows (backward): one less, full, one more
+    (1, 384, 130, 151),                      # several stages per CTA, the last one ragged
+    (3, 8, 61, 67), (1, 16, 300, 301),       # many rows per thread column: sums in two steps
+    (2, 1000, 19, 23), (1, 1024, 40, 41),    # fewest rows per stage
+    (149, 16, 5, 9),                         # more images than SMs
+])
+def test_instance_norm_rows_of_the_ring(b, c, h, w):
+    """Both passes, with a mean as large as the spread, against float64: statistics to fp32, fields to one rounding to bf16."""
+    from makani_b200.ops import _ext
+    dev = _dev()
+    g = torch.Generator(dev).manual_seed(c + h)
+    x, dy = ((torch.randn(b, h, w, c, device=dev, generator=g) + 1.0).bfloat16().permute(0, 3, 1, 2) for _ in range(2))
+    wt, bi = (torch.randn(c, device=dev, generator=g) for _ in range(2))
+    ext, eps, n = _ext.require(), 1e-2, float(h * w)
+    for act in (0, 1):
+        y, stats, wf, bf = ext.norm_forward(x, wt, bi, eps, act, n)
+        dx, dw, db = ext.norm_backward(x, dy, wf, bf, stats, True, act, n)
+        xd, wd, bd = x.double().requires_grad_(), wt.double().requires_grad_(), bi.double().requires_grad_()
+        mean = xd.mean((2, 3), keepdim=True)
+        rstd = 1.0 / torch.sqrt((xd - mean).square().mean((2, 3), keepdim=True) + eps)
+        yd = (xd - mean) * rstd * wd[:, None, None] + bd[:, None, None]
+        yd = torch.nn.functional.gelu(yd) if act else yd
+        want = torch.autograd.grad(yd, [xd, wd, bd], dy.double())
+        assert (stats[..., 0].double() - mean[..., 0, 0]).abs().max() < 1e-5
+        assert (stats[..., 1].double() / rstd[..., 0, 0] - 1.0).abs().max() < 1e-5
+        # half a unit of 2^-8 per value; GELU is 5.5e-5 off, its derivative 2e-4 times (1 + |x|), at outputs of order 1
+        assert (y.double() - yd).norm() < (2.0 ** -8 + (1e-4 if act else 0.0)) * yd.norm() + 1e-6
+        scale = (dy.double().norm() * (rstd * wd[:, None, None]).abs().max())      # dx is a difference of terms of this size
+        assert (dx.double() - want[0]).norm() < 2.0 ** -8 * want[0].norm() + (2e-3 if act else 1e-5) * scale
+        for got, ref, size in ((dw, want[1], (dy.double() * (xd - mean) * rstd)), (db, want[2], dy.double())):
+            bound = size.abs().sum((0, 2, 3)).norm()
+            assert (got.double() - ref).norm() <= (2e-3 if act else 1e-5) * bound
+    _ext.check_device_errors(dev)
+
+
 @pytest.mark.parametrize("rd,m", [(2, 182), (2, 6), (4, 132), (32, 96), (2, 181), (3, 180)])
 @pytest.mark.parametrize("epi", ["plain", "resid", "gelu_pre"])
 def test_gemm_split_rows(rd, m, epi):
