@@ -3,6 +3,7 @@
 // over HBM (vectorised 16-byte accesses) and keeps reductions in fp32.
 #include "fused_ops.cuh"
 #include "gelu.cuh"
+#include "launch.cuh"
 #include <cstring>
 #include <type_traits>
 
@@ -439,6 +440,7 @@ __global__ void __launch_bounds__(ClSums<MODE>::THREADS + 32, 1) inorm_cl_sums_k
   const int v = threadIdx.x % V, r = threadIdx.x / V;
   const int bidx = blockIdx.y;
   cl_init<P>(cl_ring);
+  chain_begin(x, dy, w, b, stats);
   __syncthreads();
   // partial sums of the rows of threads, in the ring's place: those of row r from C r on, sums before products
   f32x2* const part = reinterpret_cast<f32x2*>(cl_ring);
@@ -609,6 +611,7 @@ __global__ void __launch_bounds__(ClApply<MODE>::THREADS + 32, 1) inorm_cl_apply
   // [C][2] merged sums of this sample (exchange mode only), behind the ring
   float* const sh_sum = reinterpret_cast<float*>(cl_ring + CL_BARRIERS / 16 + P::DEPTH * P::LAPS * P::TENSORS * R * V);
   cl_init<P>(cl_ring);
+  chain_begin(x, dy, w, b, sums, stats);
   if (xc.npeers > 0) {
     // every peer's sums must have arrived in the local buffer
     __shared__ int ok_s;
@@ -727,6 +730,7 @@ __global__ void __launch_bounds__(CS_THREADS) colsum_kernel(const uint4* __restr
                                                             int V, int vb, int slab, int inner, long long ostride_v,
                                                             long long gstride_v) {
   __shared__ __align__(16) float sh[CS_THREADS * 8];
+  chain_begin(x);
   const int v0 = blockIdx.x * vb;
   const int nv = min(vb, V - v0);          // 16-byte columns of this CTA
   const int R = CS_THREADS / vb;
@@ -786,6 +790,7 @@ __global__ void __launch_bounds__(CS_THREADS) colsum_kernel(const uint4* __restr
 // out[g, c] = sum over the slabs (some hundreds of them, 4096 at most); 32 columns by 32 slabs at a time per CTA.  grid (ceil(C / 32), groups)
 __global__ void __launch_bounds__(1024) colsum_slabs_kernel(const float* __restrict__ part, float* __restrict__ out, int slabs, int C) {
   __shared__ float sh[32][33];
+  chain_begin(part);
   const int c = blockIdx.x * 32 + threadIdx.x;
   float a = 0.f;
   if (c < C) {
@@ -1065,7 +1070,8 @@ __global__ void __launch_bounds__(256) adamw_kernel(const AdamEntry* __restrict_
 // and concatenations per pass.  grid (ceil(max in / 32), ceil(max out / 32), 2 nb), block 32 x 8
 __global__ void __launch_bounds__(256) afno_pack_kernel(const AfnoLayer a, const AfnoLayer b, int nb) {
   __shared__ float re[32][33], im[32][33];
-  const AfnoLayer& L = blockIdx.z < static_cast<unsigned>(nb) ? a : b;
+  AfnoLayer L = blockIdx.z < static_cast<unsigned>(nb) ? a : b;
+  chain_begin(L.w, L.b);
   const int blk = blockIdx.z % nb, i0 = blockIdx.x * 32, o0 = blockIdx.y * 32;
   if (i0 >= L.nin || o0 >= L.nout) return;
   const long long plane = static_cast<long long>(nb) * L.nin * L.nout;
@@ -1102,7 +1108,8 @@ __global__ void __launch_bounds__(256) afno_pack_kernel(const AfnoLayer a, const
 // and dbx [nb][2 out] -> db [2][nb][out].  Same grid.
 __global__ void __launch_bounds__(256) afno_fold_kernel(const AfnoGrad a, const AfnoGrad b, int nb) {
   __shared__ float re[32][33], im[32][33];
-  const AfnoGrad& L = blockIdx.z < static_cast<unsigned>(nb) ? a : b;
+  AfnoGrad L = blockIdx.z < static_cast<unsigned>(nb) ? a : b;
+  chain_begin(L.dwx, L.dbx);
   const int blk = blockIdx.z % nb, i0 = blockIdx.x * 32, o0 = blockIdx.y * 32;
   if (i0 >= L.nin || o0 >= L.nout) return;
   const float* const wx = L.dwx + static_cast<long long>(blk) * 4 * L.nin * L.nout;
@@ -1321,6 +1328,7 @@ __global__ void swap_ri_kernel(const uint4* __restrict__ in, uint4* __restrict__
 // (a fill, a cast and a strided copy before); one 16-byte vector per thread
 __global__ void __launch_bounds__(256) cast_pad_kernel(const float* __restrict__ x, uint4* __restrict__ y, int cols, int pitch_v,
                                                        long long total) {
+  chain_begin(x);
   const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
   if (i >= total) return;
   const long long r = i / pitch_v;
@@ -1401,7 +1409,7 @@ namespace {
 // One CTA per SM, all of them at once, and no more than there are stages.  Small fields spread over the SMs by smaller CTAs.
 constexpr int CL_FEWEST = 128;      // threads (2048 x 16, both passes: 28 us, from CTAs of full size 40, with rows in registers 34)
 template <typename P, typename Kernel, typename... Args>
-cudaError_t cl_launch(Kernel* kernel, int C, long long T, int B, size_t fixed, cudaStream_t stream, Args... args) {
+cudaError_t cl_launch(Kernel* kernel, int C, long long T, int B, size_t fixed, bool peers, cudaStream_t stream, Args... args) {
   static const cudaError_t allowed = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                           CL_BARRIERS + cl_ring_bytes<P>(P::THREADS) + 2 * 1024 * static_cast<int>(sizeof(float)));
   if (allowed != cudaSuccess) return allowed;
@@ -1411,8 +1419,7 @@ cudaError_t cl_launch(Kernel* kernel, int C, long long T, int B, size_t fixed, c
   const int R = static_cast<int>(std::min<long long>(P::THREADS / V, std::max<long long>(share, (CL_FEWEST + V - 1) / V)));
   const long long need = (T + P::LAPS * R - 1) / (P::LAPS * R);
   const dim3 grid(static_cast<unsigned>(std::min(most, need)), B);
-  kernel<<<grid, (V * R + 31) / 32 * 32 + 32, CL_BARRIERS + cl_ring_bytes<P>(V * R) + fixed, stream>>>(args...);
-  return cudaGetLastError();
+  return launch_chained(kernel, grid, dim3((V * R + 31) / 32 * 32 + 32), CL_BARRIERS + cl_ring_bytes<P>(V * R) + fixed, stream, 1, !peers, args...);
 }
 }  // namespace
 
@@ -1429,8 +1436,8 @@ cudaError_t inorm_cl_sums(const __nv_bfloat16* x, const __nv_bfloat16* dy, const
   xc.err = err;
   if (xch) xc = *xch;
   if (mode == 0)
-    return cl_launch<ClSums<0>>(inorm_cl_sums_kernel<0>, C, T, B, 0, s, x, dy, w, b, stats, sums, dw, db, C, T, act, shifted, xc);
-  return cl_launch<ClSums<1>>(inorm_cl_sums_kernel<1>, C, T, B, 0, s, x, dy, w, b, stats, sums, dw, db, C, T, act, 0, xc);
+    return cl_launch<ClSums<0>>(inorm_cl_sums_kernel<0>, C, T, B, 0, xc.npeers > 0, s, x, dy, w, b, stats, sums, dw, db, C, T, act, shifted, xc);
+  return cl_launch<ClSums<1>>(inorm_cl_sums_kernel<1>, C, T, B, 0, xc.npeers > 0, s, x, dy, w, b, stats, sums, dw, db, C, T, act, 0, xc);
 }
 
 cudaError_t inorm_cl_apply(const __nv_bfloat16* x, const __nv_bfloat16* dy, __nv_bfloat16* out, const float* w, const float* b,
@@ -1448,8 +1455,8 @@ cudaError_t inorm_cl_apply(const __nv_bfloat16* x, const __nv_bfloat16* dy, __nv
   const float inv = static_cast<float>(1.0 / count);
   const size_t shx = xc.npeers > 0 ? 2 * C * sizeof(float) : 0;
   if (mode == 0)
-    return cl_launch<ClApply<0>>(inorm_cl_apply_kernel<0>, C, T, B, shx, s, x, dy, out, w, b, sums, stats, C, T, inv, eps, act, shifted, xc);
-  return cl_launch<ClApply<1>>(inorm_cl_apply_kernel<1>, C, T, B, shx, s, x, dy, out, w, b, sums, stats, C, T, inv, eps, act, 0, xc);
+    return cl_launch<ClApply<0>>(inorm_cl_apply_kernel<0>, C, T, B, shx, xc.npeers > 0, s, x, dy, out, w, b, sums, stats, C, T, inv, eps, act, shifted, xc);
+  return cl_launch<ClApply<1>>(inorm_cl_apply_kernel<1>, C, T, B, shx, xc.npeers > 0, s, x, dy, out, w, b, sums, stats, C, T, inv, eps, act, 0, xc);
 }
 
 namespace {
@@ -1486,15 +1493,15 @@ cudaError_t colsum(const __nv_bfloat16* x, float* out, float* scratch, long long
     return cudaErrorInvalidValue;
   const ColsumPlan p = colsum_plan(rows, C, groups);
   float* const part = p.slabs > 1 ? scratch : out;
-  colsum_kernel<<<dim3(p.parts, static_cast<unsigned>(p.slabs), groups), CS_THREADS, 0, s>>>(
-      reinterpret_cast<const uint4*>(x), part, rows, p.V, p.vb, static_cast<int>(p.slab), inner, ostride / 8, gstride / 8);
-  if (p.slabs > 1) return colsum_add_slabs(part, out, static_cast<int>(p.slabs), C, groups, s);
-  return cudaGetLastError();
+  const cudaError_t e = launch_chained(colsum_kernel, dim3(p.parts, static_cast<unsigned>(p.slabs), groups), dim3(CS_THREADS), 0, s, 1, true,
+                                       reinterpret_cast<const uint4*>(x), part, rows, p.V, p.vb, static_cast<int>(p.slab), inner, ostride / 8,
+                                       gstride / 8);
+  if (e == cudaSuccess && p.slabs > 1) return colsum_add_slabs(part, out, static_cast<int>(p.slabs), C, groups, s);
+  return e;
 }
 
 cudaError_t colsum_add_slabs(const float* part, float* out, int slabs, int C, int groups, cudaStream_t s) {
-  colsum_slabs_kernel<<<dim3((C + 31) / 32, groups), dim3(32, 32), 0, s>>>(part, out, slabs, C);
-  return cudaGetLastError();
+  return launch_chained(colsum_slabs_kernel, dim3((C + 31) / 32, groups), dim3(32, 32), 0, s, 1, true, part, out, slabs, C);
 }
 
 template <typename L>
@@ -1505,14 +1512,12 @@ static dim3 afno_grid(const L& a, const L& b, int nb) {
 
 cudaError_t afno_pack(const AfnoLayer& a, const AfnoLayer& b, int nb, cudaStream_t s) {
   if (nb <= 0) return cudaSuccess;
-  afno_pack_kernel<<<afno_grid(a, b, nb), dim3(32, 8), 0, s>>>(a, b, nb);
-  return cudaGetLastError();
+  return launch_chained(afno_pack_kernel, afno_grid(a, b, nb), dim3(32, 8), 0, s, 1, true, a, b, nb);
 }
 
 cudaError_t afno_fold(const AfnoGrad& a, const AfnoGrad& b, int nb, cudaStream_t s) {
   if (nb <= 0) return cudaSuccess;
-  afno_fold_kernel<<<afno_grid(a, b, nb), dim3(32, 8), 0, s>>>(a, b, nb);
-  return cudaGetLastError();
+  return launch_chained(afno_fold_kernel, afno_grid(a, b, nb), dim3(32, 8), 0, s, 1, true, a, b, nb);
 }
 
 // The 16-byte path of the loss kernels needs every row to hold a whole number of vectors, 16-byte aligned planes and
@@ -1636,8 +1641,8 @@ cudaError_t cast_pad_bf16(const float* x, __nv_bfloat16* y, long long rows, int 
   if ((pitch & 7) || pitch < cols || !aligned16(y)) return cudaErrorInvalidValue;
   const long long total = rows * (pitch / 8);
   if ((total + 255) / 256 > 0x7fffffffll) return cudaErrorInvalidValue;
-  cast_pad_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, s>>>(x, reinterpret_cast<uint4*>(y), cols, pitch / 8, total);
-  return cudaGetLastError();
+  return launch_chained(cast_pad_kernel, dim3(static_cast<unsigned>((total + 255) / 256)), dim3(256), 0, s, 1, true, x, reinterpret_cast<uint4*>(y), cols,
+                        pitch / 8, total);
 }
 
 cudaError_t fill_normal_bf16(__nv_bfloat16* y, long long n, uint64_t seed, cudaStream_t s) {

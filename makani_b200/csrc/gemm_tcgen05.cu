@@ -46,6 +46,7 @@
 #include "gemm_tcgen05.cuh"
 #include "gelu.cuh"
 #include "fused_ops.cuh"
+#include "launch.cuh"
 
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -513,6 +514,25 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 1) {
+    if constexpr (CG == 2) {
+      // the same warp of both CTAs allocates, with the same destination offset
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                       smem_u32(const_cast<uint32_t*>(tmem_slot))),
+                   "r"(TMEM_COLS)
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                       smem_u32(const_cast<uint32_t*>(tmem_slot))),
+                   "r"(TMEM_COLS)
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+  }
+  chain_begin();
+  if (threadIdx.x == 0) {
     // segments written by the peers (and the peers' copies this kernel overwrites) must be ready: bounded wait on local flags.
     // The whole CTA waits (not only the producer) so that no epilogue store of an all-zero tile can run early.
     bool ok = true;
@@ -535,22 +555,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
       }
     }
     tmem_slot[1] = ok ? 1u : 0u;
-  }
-  if (warp == 1) {
-    if constexpr (CG == 2) {
-      // the same warp of both CTAs allocates, with the same destination offset
-      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                       smem_u32(const_cast<uint32_t*>(tmem_slot))),
-                   "r"(TMEM_COLS)
-                   : "memory");
-      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-    } else {
-      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                       smem_u32(const_cast<uint32_t*>(tmem_slot))),
-                   "r"(TMEM_COLS)
-                   : "memory");
-      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
   }
   tc_fence_before();
   __syncthreads();
@@ -1580,26 +1584,15 @@ cudaError_t launch_t(const CUtensorMap& ma, const BMaps& mb, const CUtensorMap& 
     long long clusters = kp.total_tiles < static_cast<uint32_t>(most) ? kp.total_tiles : most;
     if (clusters < 1) clusters = 1;
     if constexpr (EPI == 6) clusters = mixed_grid(clusters, kp, 2 * BM, BN);
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof(cfg));
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(static_cast<unsigned>(2 * clusters), 1, 1);
-    cfg.blockDim = dim3(threads, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, gemm_kernel<BN, EB, EPI, CG, RAGGED>, ma, mb, me, md, mp, mdx, kp);
+    return launch_chained(gemm_kernel<BN, EB, EPI, CG, RAGGED>, dim3(static_cast<unsigned>(2 * clusters)), dim3(threads), smem, stream, 2, true, ma, mb,
+                          me, md, mp, mdx, kp);
   }
   long long grid = kp.total_tiles < static_cast<uint32_t>(num_sms) ? kp.total_tiles : num_sms;
   if (grid < 1) grid = 1;
   if constexpr (EPI == 6) grid = mixed_grid(grid, kp, BM, BN);
-  gemm_kernel<BN, EB, EPI, CG, RAGGED><<<static_cast<unsigned>(grid), threads, smem, stream>>>(ma, mb, me, md, mp, mdx, kp);
-  return cudaGetLastError();
+  const bool alone = kp.nseg <= 1 && kp.ndx == 0 && kp.sync.nwait == 0 && kp.sync.nsig == 0 && kp.sync.done_ctr == nullptr;
+  return launch_chained(gemm_kernel<BN, EB, EPI, CG, RAGGED>, dim3(static_cast<unsigned>(grid)), dim3(threads), smem, stream, 1, alone, ma, mb, me, md,
+                        mp, mdx, kp);
 }
 
 // Tensor map of an output or epilogue operand: [M rows][N contiguous] bf16 with two batch dimensions, 128-byte swizzle.  Rows

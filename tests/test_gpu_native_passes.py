@@ -234,3 +234,42 @@ def test_afno_passes(b, h, w, c, nb, f, frac, bias, skip):
     for a, e in zip(back[1:], want[1:]):
         _close_sums(a, e)
     _ext.check_device_errors(dev)
+
+
+def test_launches_that_begin_early_see_their_operands():
+    """Dependent launches of a microsecond each, all of which begin while the one before them ends: the bits of the same launches with the
+    device idle in between, eager and from a graph, also where the allocator hands memory on from one to the next."""
+    dev = _dev()
+    g = torch.Generator(dev).manual_seed(11)
+    ext = _ext.require()
+    x = _cl(g, 1, 64, 24, 32)
+    ws = [torch.randn(c, k, 1, 1, device=dev, generator=g) * k ** -0.5 for c, k in ((136, 64), (24, 136), (64, 24))]
+    b = [torch.randn(w.shape[0], device=dev, generator=g) for w in ws]
+
+    def chain(pause):
+        y, sums = x, []
+        for _ in range(4):
+            for w, bi in zip(ws, b):
+                y, wq, _ = ext.conv_forward(y, w, bi, None, 0, -1, False)
+                pause()
+                sums.append(ext.conv_backward(y, y, wq, w.shape[0], False, False, True)[2])      # column sums: two launches
+                pause()
+        return y, sums
+
+    want, want_sums = chain(torch.cuda.synchronize)
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        chain(lambda: None)
+        graph = torch.cuda.CUDAGraph()
+    stream.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        captured = chain(lambda: None)
+    for k in range(20):
+        if k % 2:
+            graph.replay()
+            y, sums = captured
+        else:
+            y, sums = chain(lambda: None)
+        torch.cuda.synchronize()
+        assert torch.equal(y, want) and all(torch.equal(a, e) for a, e in zip(sums, want_sums))
+    _ext.check_device_errors(dev)
