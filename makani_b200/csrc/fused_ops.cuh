@@ -120,6 +120,11 @@ cudaError_t spectral_expand(const float* w, __nv_bfloat16* wx, int Cin, int Cout
 cudaError_t spectral_fold(const float* dwx, float* dw, int Cin, int Cout, int L, cudaStream_t s, int two_block = 0,
                           int assign = 0);
 
+// dw (complex64 [ci, co, L], 32-byte aligned) = the gradient of the spectral weights from dt [L, M, (re, im) co] and t2 [L, M, (re, im) ci], zero
+// above m = l (spectral_wgrad.cu; co and ci multiples of 8, L of 4)
+cudaError_t spectral_wgrad(const __nv_bfloat16* dt, const __nv_bfloat16* t2, float* dw, int co, int ci, int L, int M, int* err_flag, cudaStream_t s);
+bool spectral_wgrad_pays(int co, int ci, int L, int samples);
+
 // rows of (re[C], im[C]) -> (im[C], -re[C]) (bf16, C % 8 == 0): the operand of the imaginary-part weight gradient
 cudaError_t swap_ri_bf16(const __nv_bfloat16* in, __nv_bfloat16* out, long long rows, int C, cudaStream_t s);
 

@@ -397,13 +397,26 @@ Tensor contract(const Tensor& t2, const Tensor& wx, bool adjoint, const Tensor& 
   return t3;
 }
 
+// dw[c, o, l] from dt [B, l, m, (ri, o)] and t2 [B, l, m, (ri, c)]: each sample a sum of its own
 Tensor spectral_weight_gradient(const Tensor& dt, const Tensor& t2) {
-  const int64_t B = dt.size(0), L = dt.size(1), M = dt.size(2), nq = dt.size(3), co = nq / 2, ci = t2.size(3) / 2;
+  MK_CHECK(dt.is_cuda() && t2.is_cuda() && dt.device() == t2.device() && dt.scalar_type() == at::kBFloat16 && t2.scalar_type() == at::kBFloat16 &&
+               dt.dim() == 4 && t2.dim() == 4 && dt.is_contiguous() && t2.is_contiguous() && dt.sizes().slice(0, 3) == t2.sizes().slice(0, 3) &&
+               dt.size(3) % 16 == 0 && t2.size(3) % 16 == 0,
+           "spectral weight gradient: contiguous bf16 CUDA coefficients of a multiple of 8 channels expected");
+  c10::cuda::CUDAGuard guard(dt.device());
+  const int64_t B = dt.size(0), L = dt.size(1), M = dt.size(2), co = dt.size(3) / 2, ci = t2.size(3) / 2;
   Tensor dw = at::empty({ci, co, L}, dt.options().dtype(at::kComplexFloat));
+  if (mk::spectral_wgrad_pays(static_cast<int>(co), static_cast<int>(ci), static_cast<int>(L), static_cast<int>(B))) {
+    ++mkh::launches();
+    mkh::check(mk::spectral_wgrad(bf(dt), bf(t2), reinterpret_cast<float*>(dw.data_ptr()), static_cast<int>(co), static_cast<int>(ci), static_cast<int>(L),
+                                  static_cast<int>(M), mkh::error_word(dt), mkh::stream()),
+               "spectral_wgrad");
+    return dw;
+  }
   Tensor planes = B > 1 ? zeros_f32({2, L, co, ci}, dt) : empty_f32({2, L, co, ci}, dt);
   for (int64_t b = 0; b < B; ++b)
     mkh::complex_product(dt, t2, planes, nullptr,
-                         {3, co, ci, M, 1, L, 0, mkh::BIG, 1, 1, b * L * M * nq, 1, nq, 0, M * nq, co,
+                         {3, co, ci, M, 1, L, 0, mkh::BIG, 1, 1, b * L * M * 2 * co, 1, 2 * co, 0, M * 2 * co, co,
                           b * L * M * 2 * ci, 1, 2 * ci, M * 2 * ci, ci, 0, ci, L * co * ci, 0, co * ci, B > 1 ? 1 : 0});
   ++mkh::launches();
   mkh::check(mk::spectral_fold(planes.data_ptr<float>(), reinterpret_cast<float*>(dw.data_ptr()), static_cast<int>(ci), static_cast<int>(co),
@@ -701,6 +714,7 @@ void bind_layers(pybind11::module_& m) {
   m.def("norm_backward", &norm_backward);
   m.def("spectral_forward", &spectral_forward);
   m.def("spectral_backward", &spectral_backward);
+  m.def("spectral_weight_gradient", &spectral_weight_gradient);
   m.def("afno_forward", &afno_forward);
   m.def("afno_backward", &afno_backward);
 }

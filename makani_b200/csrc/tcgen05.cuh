@@ -1,0 +1,240 @@
+// Device primitives of the kernels that run on the tensor cores (tcgen05 + TMEM + TMA) and the host side of their tensor maps.
+#pragma once
+#include <cuda.h>
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "gemm_tcgen05.cuh"
+
+namespace mk {
+
+// ---- host (gemm_tcgen05.cu)
+// tensor map of an operand: boxes of 128 bytes of the contiguous dimension by 64 (MN-major) or `box_rows_kmajor` rows
+bool make_map(CUtensorMap* map, const GemmOperand& op, int K, int eb, int zlo_n, int zhi_n, int box_rows_kmajor);
+// Tensor map of an output or epilogue operand: [M rows][N contiguous] with two batch dimensions, 128-byte swizzle.  Rows
+// may be split, r = hi * rd + lo with rd a power of two that divides M and 32: a box is then 32 (or 128) / rd by rd rows.
+// With `halves` the second dimension is not part of the rows: two results `halves` elements apart (complex products).
+bool make_map_e(CUtensorMap* map, const void* ptr, int M, int N, int rd, long long rs_hi, long long rs_lo, long long zs_lo,
+                long long zs_hi, int zlo_n, int zhi_n, int box_rows = 128, int ob = 2, long long halves = 0);
+// CTA pairs that can be resident at once.  Every kernel of them fills an SM with its shared memory, so one answers for all.
+int max_pairs();
+// cuTensorMapEncodeTiled is a driver call: binds the primary context to this host thread (not while `stream` is capturing)
+void bind_context(cudaStream_t stream);
+
+constexpr int SMEM_LIMIT = 232448;   // 227 KB per CTA on sm_100
+
+#ifdef __CUDACC__
+constexpr uint64_t WAIT_LIMIT_NS = 2000000000ull;   // 2 s per barrier wait
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) {
+  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
+}
+
+__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive_n(uint32_t bar, uint32_t count) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+
+// Bounded wait: polls the barrier and gives up after WAIT_LIMIT_NS of wall time. Returns false on expiry.
+__device__ __forceinline__ uint64_t global_ns() {
+  uint64_t t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
+}
+
+// The suspend-time hint lets the hardware park a waiting thread until the phase completes (it wakes at once when it
+// does) instead of returning to the polling loop every few dozen cycles: the three single-thread roles of a CTA spend
+// most of their time waiting, and their polling instructions competed with the epilogue warps for issue slots.
+constexpr uint32_t MBAR_SUSPEND_HINT_NS = 4000;
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
+  uint64_t t0 = 0;
+  for (uint32_t it = 0;; ++it) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred P1;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2, %3;\n\t"
+        "selp.b32 %0, 1, 0, P1;\n\t"
+        "}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity), "r"(MBAR_SUSPEND_HINT_NS)
+        : "memory");
+    if (ok) return true;
+    if ((it & 63u) == 63u) {
+      const uint64_t now = global_ns();
+      if (t0 == 0) t0 = now;
+      else if (now - t0 > WAIT_LIMIT_NS) return false;
+    }
+  }
+}
+
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2,
+                                            int c3) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+      ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+      : "memory");
+}
+
+// CTA-pair form: the destination is this CTA's shared memory, the barrier that counts the bytes lives in the leader CTA
+__device__ __forceinline__ void tma_load_4d_pair(uint32_t dst, const CUtensorMap* map, uint32_t leader_bar, int c0, int c1,
+                                                 int c2, int c3) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+      ::"r"(dst), "l"(map), "r"(leader_bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+      : "memory");
+}
+
+// One lane of a converged warp, always the same one.  The compiler knows that a single thread runs behind it and issues the
+// TMA / MMA / commit instructions, which take uniform registers, as they are; behind `lane == 0` it guards each of them
+// against differing operands.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred P1;\n\t"
+      "elect.sync _|P1, 0xffffffff;\n\t"
+      "selp.b32 %0, 1, 0, P1;\n\t"
+      "}\n"
+      : "=r"(ok));
+  return ok != 0;
+}
+
+// address of the same shared-memory offset in CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t mapa_u32(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
+  // (no data passes through memory here, only the right to overwrite TMEM: a cluster-scope release would wait for the
+  // staged stores of the whole warp)
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+__device__ __forceinline__ uint32_t cluster_ctarank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// Output and epilogue-operand maps are (column, r % rdiv, r / rdiv, z_lo, z_hi): a box starts at a multiple of rdiv rows.  Complex
+// products: the second index is the half.
+__device__ __forceinline__ void tma_store_tile(const CUtensorMap* map, uint32_t src, int n, int lo, int r, int zlo, int zhi) {
+  asm volatile("cp.async.bulk.tensor.5d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5, %6}], [%1];" ::"l"(map), "r"(src),
+               "r"(n), "r"(lo), "r"(r), "r"(zlo), "r"(zhi)
+               : "memory");
+}
+__device__ __forceinline__ void tma_add_tile(const CUtensorMap* map, uint32_t src, int n, int lo, int r, int zlo, int zhi) {
+  asm volatile("cp.reduce.async.bulk.tensor.5d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4, %5, %6}], [%1];" ::"l"(map),
+               "r"(src), "r"(n), "r"(lo), "r"(r), "r"(zlo), "r"(zhi)
+               : "memory");
+}
+__device__ __forceinline__ void tma_load_tile(uint32_t dst, const CUtensorMap* map, uint32_t bar, int n, int lo, int r, int zlo,
+                                              int zhi) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
+      ::"r"(dst), "l"(map), "r"(bar), "r"(n), "r"(lo), "r"(r), "r"(zlo), "r"(zhi)
+      : "memory");
+}
+__device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void tma_store_wait_read() {
+  asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+
+__device__ __forceinline__ void tc_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+// pair form: arrives on the barrier at this offset in both CTAs of the pair
+__device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
+  const unsigned short mask = 3;
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+               "h"(mask)
+               : "memory");
+}
+
+// One MMA; the operand descriptors come as halves (see desc_hi, desc_lo)
+template <int EB, int CG>
+__device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
+                                       uint32_t accum) {
+#define MK_MMA(FORM)                                                 \
+  asm volatile(                                                      \
+      "{\n\t"                                                        \
+      ".reg .pred p;\n\t"                                            \
+      ".reg .b64 da, db;\n\t"                                        \
+      "mov.b64 da, {%1, %2};\n\t"                                    \
+      "mov.b64 db, {%3, %4};\n\t"                                    \
+      "setp.ne.b32 p, %6, 0;\n\t"                                    \
+      "tcgen05.mma." FORM " [%0], da, db, %5, p;\n\t"                \
+      "}\n" ::"r"(tmem_d),                                           \
+      "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accum) \
+      : "memory")
+  if constexpr (EB == 2 && CG == 2) MK_MMA("cta_group::2.kind::f16");
+  else if constexpr (EB == 2) MK_MMA("cta_group::1.kind::f16");
+  else MK_MMA("cta_group::1.kind::tf32");
+#undef MK_MMA
+}
+
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+      : "r"(taddr)
+      : "memory");
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// In two steps: the request, and the wait for all requests, after which `v` holds the values (the wait names them, so that nothing that uses them
+// moves in front of it)
+__device__ __forceinline__ void tmem_req4(uint32_t taddr, uint32_t (&v)[4]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+               : "r"(taddr)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_wait4(uint32_t (&v)[4]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3])::"memory");
+}
+
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(taddr)
+      : "memory");
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// Shared-memory matrix descriptor, 128-byte swizzle, sm_100 version field = 1, as two halves: only the low one changes from
+// one MMA to the next, by the distance in bytes / 16.  The issuing thread builds them itself, one dependent instruction after
+// the other, while the tensor cores wait: building eight 64-bit descriptors for every k slab took longer than the slab's MMAs
+// (768 -> 384 outputs over 721 x 1440 tokens: 662 -> 581 us; 16200 x 768 -> 3072: 104 -> 84 us, with the elected lanes above).
+__device__ __forceinline__ uint32_t desc_lo(uint32_t saddr, uint32_t lbo_bytes) {
+  return ((saddr & 0x3FFFF) >> 4) | ((lbo_bytes >> 4) << 16);
+}
+__device__ __forceinline__ uint32_t desc_hi(uint32_t sbo_bytes) { return (sbo_bytes >> 4) | (1u << 14) | (2u << 29); }
+#endif  // __CUDACC__
+
+}  // namespace mk

@@ -167,6 +167,11 @@ ERROR_CODES = {
     44: "segment-sum kernel: a peer's segment did not arrive",
     56: "instance-norm statistics: peers still read the previous sums",
     57: "instance-norm apply: a peer's sums did not arrive",
+    58: "instance norm: rows never arrived, or their stage was never freed",
+    70: "spectral weight gradient: shared-memory stage never freed",
+    71: "spectral weight gradient: accumulators never drained",
+    72: "spectral weight gradient: operands never arrived",
+    73: "spectral weight gradient: accumulators never completed",
 }
 
 

@@ -309,6 +309,13 @@ def fold_weight_grad2(dw2: torch.Tensor) -> torch.Tensor:
     return torch.complex(dw2[0], dw2[1]).permute(2, 1, 0).contiguous()
 
 
+def weight_gradient(dt: torch.Tensor, t2: torch.Tensor) -> torch.Tensor:
+    """Both at once for a whole transform: on the GPU one launch per sample that writes complex64 [Ci, Co, L] (csrc/spectral_wgrad.cu)."""
+    if dt.is_cuda and _ext.native():
+        return _ext.require().spectral_weight_gradient(dt, t2)
+    return fold_weight_grad2(contract_wgrad2(dt, t2))
+
+
 # ------------------------------------------------------------------------------------------------ weights
 
 
@@ -428,7 +435,7 @@ def backward_stages(dy, dr, t2, wx, plan_in: SHTPlan, plan_out: SHTPlan, need_x:
     dt4 = analyse(dy, plan_out, forward=False)
     dt3 = legendre_analysis(dt4, plan_out.p)                       # [B, l, m, (ri, o)]
     del dt4
-    dw = fold_weight_grad2(contract_wgrad2(dt3, t2)) if need_w else None
+    dw = weight_gradient(dt3, t2) if need_w else None
     dx = None
     if need_x:
         dr2 = None

@@ -963,3 +963,30 @@ def test_norm_of_a_field_off_a_16_byte_boundary():
     assert _rel(instance_norm(x, wt, bi, 1e-6), ref) < BF16
     with pytest.raises(RuntimeError, match="invalid argument"):
         _ext.require().norm_forward(x, wt, bi, 1e-6, 0, float(h * w))
+
+
+@pytest.mark.parametrize("b,l,m,co,ci", [
+    (1, 296, 5, 8, 8),            # as few channels as there are, orders in part of one slab
+    (1, 80, 81, 136, 72),         # second tiles of 8 outputs and 8 inputs
+    (1, 28, 64, 200, 328),        # a slab that is full, more orders than degrees
+    (1, 20, 21, 384, 384),        # whole tiles
+    (1, 132, 66, 128, 200),       # two slabs, the second of two orders
+    (1, 196, 197, 256, 64),       # four slabs
+    (2, 80, 81, 136, 72), (1, 82, 83, 136, 72), (1, 8, 9, 16, 16),      # two samples, degrees off four, few tiles: planes and their re-layout
+])
+def test_spectral_weight_gradient_in_its_own_layout(b, l, m, co, ci):
+    """Against complex float64 and against the planes with their re-layout; every element written (memory full of NaN before)."""
+    from makani_b200.ops.spectral import contract_wgrad2, fold_weight_grad2, weight_gradient
+    dev = _dev()
+    g = torch.Generator(dev).manual_seed(l + co)
+    keep = (torch.arange(m, device=dev)[None] <= torch.arange(l, device=dev)[:, None]).view(1, l, m, 1)
+    t2, dt = ((torch.randn(b, l, m, 2 * c, device=dev, generator=g) * keep).to(torch.bfloat16) for c in (ci, co))
+    cplx = lambda t: torch.complex(t[..., : t.shape[-1] // 2].double(), t[..., t.shape[-1] // 2:].double())  # noqa: E731
+    ref = torch.einsum("blmo,blmc->col", cplx(dt), cplx(t2).conj())
+    full = torch.full((ci, co, l), float("nan"), dtype=torch.complex64, device=dev)
+    del full      # the next tensor of this size takes its place
+    got = weight_gradient(dt, t2)
+    bound = 2.0 ** -24 * max(b * m, 64) ** 0.5 * 4      # fp32 sums of up to b m products, truncated every 16
+    assert got.shape == ref.shape and _rel(torch.view_as_real(got), torch.view_as_real(ref)) < bound
+    assert _rel(torch.view_as_real(got), torch.view_as_real(fold_weight_grad2(contract_wgrad2(dt, t2)))) < bound
+    _ext.check_device_errors(dev)
