@@ -1326,13 +1326,16 @@ void bind_context(cudaStream_t stream) {
 }
 
 namespace {
-// Grid of a folded product.  CTA c walks the tiles c, c + grid, ...: where the tiles of one batch and the grid have a factor in common, a
-// CTA meets the same few of them in every batch, and if those are the ones with few rows or columns it runs ahead of its
-// neighbours.  It idles at the end, and on the way the halves of the 128-byte lines that two tiles share are written so far apart in
-// time that they leave L2 one by one.  A grid without a common factor mixes them.  Synthesis of 1440 points, 64 orders, 136 channels
-// 150 -> 88, 200 channels 187 -> 108; of 256 points, 129 orders, 384 channels 35 -> 30 us.
+// Grid of a product with tiles of few rows or columns.  CTA c walks the tiles c, c + grid, ...: where the tiles of one batch and the grid have
+// a factor in common, a CTA meets the same few of them in every batch, and if those are the narrow ones it runs ahead of its
+// neighbours.  It idles at the end, and on the way what two tiles share (the halves of 128-byte lines of a folded product's output, the rows of
+// activations of a plain one) is met so far apart in time that it leaves L2 in between.  A grid without a common factor mixes
+// them.  Synthesis of 1440 points, 64 orders, 136 channels 150 -> 88, 200 channels 187 -> 108; of 256 points, 129 orders, 384 channels
+// 35 -> 30 us.  Where a batch has many row tiles, all alike, the column tiles of one row take the place of a batch, and no wave may be added.
 long long mixed_grid(long long grid, const KParams& kp, int bm, int bn) {
-  const int tiles = kp.m_tiles * kp.n_tiles;
+  const bool columns = static_cast<long long>(kp.m_tiles) * kp.n_tiles > 256;
+  if (columns && !kp.n_fast) return grid;
+  const int tiles = columns ? kp.n_tiles : kp.m_tiles * kp.n_tiles;
   if (tiles <= 1 || tiles > 256 || kp.total_tiles <= static_cast<uint32_t>(grid)) return grid;
   auto gcd = [](long long a, long long b) {
     while (b) {
@@ -1347,15 +1350,16 @@ long long mixed_grid(long long grid, const KParams& kp, int bm, int bn) {
   for (int c = 0; c < classes; ++c) {
     long long area = 0;
     for (int i = c; i < tiles; i += classes) {
-      const int mt = kp.n_fast ? i / kp.n_tiles : i % kp.m_tiles, nt = kp.n_fast ? i % kp.n_tiles : i / kp.m_tiles;
+      const int mt = columns ? 0 : (kp.n_fast ? i / kp.n_tiles : i % kp.m_tiles), nt = kp.n_fast ? i % kp.n_tiles : i / kp.m_tiles;
       area += static_cast<long long>(std::min(bm, kp.M - mt * bm)) * std::min(bn, kp.N - nt * bn);
     }
     least = c == 0 ? area : std::min(least, area);
     most = std::max(most, area);
   }
   if (most * 4 <= least * 5) return grid;
+  const long long total = kp.total_tiles;
   for (long long g = grid - 1; g > grid - 8 && g > 0; --g)
-    if (gcd(g, tiles) == 1) return g;
+    if (gcd(g, tiles) == 1) return columns && (total + g - 1) / g > (total + grid - 1) / grid + total / (16 * grid) ? grid : g;
   return grid;
 }
 
@@ -1397,13 +1401,13 @@ cudaError_t launch_t(const CUtensorMap& ma, const BMaps& mb, const CUtensorMap& 
     const int most = max_pairs();
     long long clusters = kp.total_tiles < static_cast<uint32_t>(most) ? kp.total_tiles : most;
     if (clusters < 1) clusters = 1;
-    if constexpr (EPI == 6) clusters = mixed_grid(clusters, kp, 2 * BM, BN);
+    if constexpr (EPI != 0 && EPI != 5) clusters = mixed_grid(clusters, kp, 2 * BM, BN);
     return launch_chained(gemm_kernel<BN, EB, EPI, CG, RAGGED>, dim3(static_cast<unsigned>(2 * clusters)), dim3(threads), smem, stream, 2, true, ma, mb,
                           me, md, mp, mdx, kp);
   }
   long long grid = kp.total_tiles < static_cast<uint32_t>(num_sms) ? kp.total_tiles : num_sms;
   if (grid < 1) grid = 1;
-  if constexpr (EPI == 6) grid = mixed_grid(grid, kp, BM, BN);
+  if constexpr (EPI != 0 && EPI != 5) grid = mixed_grid(grid, kp, BM, BN);
   const bool alone = kp.nseg <= 1 && kp.ndx == 0 && kp.sync.nwait == 0 && kp.sync.nsig == 0 && kp.sync.done_ctr == nullptr;
   return launch_chained(gemm_kernel<BN, EB, EPI, CG, RAGGED>, dim3(static_cast<unsigned>(grid)), dim3(threads), smem, stream, 1, alone, ma, mb, me, md,
                         mp, mdx, kp);

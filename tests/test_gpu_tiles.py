@@ -990,3 +990,27 @@ def test_spectral_weight_gradient_in_its_own_layout(b, l, m, co, ci):
     assert got.shape == ref.shape and _rel(torch.view_as_real(got), torch.view_as_real(ref)) < bound
     assert _rel(torch.view_as_real(got), torch.view_as_real(fold_weight_grad2(contract_wgrad2(dt, t2)))) < bound
     _ext.check_device_errors(dev)
+
+
+@pytest.mark.parametrize("n,epi", [(264, "plain"), (264, "resid"), (264, "mul"), (200, "gelu_deriv"), (776, "plain"), (328, "gelu_deriv")])
+def test_narrow_last_column_tile_over_many_rows(n, epi):
+    """Many rows and an even number of column tiles, the last one narrow: the grid has no factor in common with them, every tile is still met."""
+    dev = _dev()
+    g = torch.Generator(dev).manual_seed(n)
+    m, k = 256 * 148 + 40, 72
+    x, w = torch.randn(m, k, device=dev, generator=g).to(torch.bfloat16), (torch.randn(n, k, device=dev, generator=g) * k ** -0.5).to(torch.bfloat16)
+    aux = torch.randn(m, n, device=dev, generator=g).to(torch.bfloat16) if epi in ("resid", "mul") else None
+    pre = torch.full((m, n), float("nan"), device=dev, dtype=torch.bfloat16) if epi == "gelu_deriv" else None
+    d = torch.full((m, n), float("nan"), device=dev, dtype=torch.bfloat16)
+    gemm(m, n, k, Operand(x, ld=k), Operand(w, ld=k), Output(d, rs_lo=n), resid=aux, preact=pre, preact_deriv=pre is not None,
+         act={"mul": ACT_MULAUX, "gelu_deriv": ACT_GELU}.get(epi, ACT_NONE))
+    z = (x.double() @ w.double().t())
+    if epi == "gelu_deriv":
+        z.requires_grad_()
+        y = torch.nn.functional.gelu(z)
+        (dy,) = torch.autograd.grad(y.sum(), z)
+        assert _rel(pre, dy) < BF16
+    else:
+        y = z if aux is None else (z + aux.double() if epi == "resid" else z * aux.double())
+    assert _rel(d, y.detach()) < BF16
+    _ext.check_device_errors(dev)
