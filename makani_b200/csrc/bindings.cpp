@@ -304,7 +304,8 @@ bool run(const Gemm& g, const mk::GemmPeer* peer) {
     MK_CHECK(g.preact->is_cuda() && g.preact->scalar_type() == d.scalar_type(), "gemm: preact must be a CUDA tensor of the output's type");
     e.preact = const_cast<char*>(base_ptr(*g.preact)) + g.preact_offset * osz;
   }
-  Tensor part;      // freed to the allocator on return: later work of this stream only
+  Tensor own;      // freed to the allocator on return: later work of this stream only
+  Tensor& part = g.sums_later ? g.sums_later->part : own;
   struct Ctx {
     Tensor* part;
     const Tensor* like;
@@ -328,10 +329,12 @@ bool run(const Gemm& g, const mk::GemmPeer* peer) {
       return x.part->data_ptr<float>();
     };
     rows.done = 0;
+    rows.later = g.sums_later != nullptr;
   }
   Tensor ef = err_flag_for(a);
   ++launches();
   check_cuda(mk::gemm_launch(p, A, B, e, ef.data_ptr<int>(), stream(), peer, g.row_sums ? &rows : nullptr), "gemm launch");
+  if (g.row_sums && rows.done && g.sums_later) g.sums_later->slabs = rows.slabs;
   return g.row_sums && rows.done != 0;
 }
 
@@ -401,8 +404,8 @@ void cast_pad(const Tensor& x, Tensor& y) {
                y.size(1) >= x.size(1) && y.size(1) % 8 == 0,
            "cast_pad: bad output");
   c10::cuda::CUDAGuard guard(x.device());
-  check_cuda(mk::cast_pad_bf16(x.data_ptr<float>(), reinterpret_cast<__nv_bfloat16*>(y.data_ptr()), x.size(0), static_cast<int>(x.size(1)),
-                               static_cast<int>(y.size(1)), cur_stream()),
+  check_cuda(mk::cast_pad_bf16({x.data_ptr<float>(), reinterpret_cast<__nv_bfloat16*>(y.data_ptr()), x.size(0), static_cast<int>(x.size(1)),
+                               static_cast<int>(y.size(1))}, cur_stream()),
              "cast_pad");
 }
 

@@ -3,6 +3,7 @@
 // over HBM (vectorised 16-byte accesses) and keeps reductions in fp32.
 #include "fused_ops.cuh"
 #include "gelu.cuh"
+#include "gemm_tcgen05.cuh"
 #include "launch.cuh"
 #include <cstring>
 #include <type_traits>
@@ -788,9 +789,14 @@ __global__ void __launch_bounds__(CS_THREADS) colsum_kernel(const uint4* __restr
 }
 
 // out[g, c] = sum over the slabs (some hundreds of them, 4096 at most); 32 columns by 32 slabs at a time per CTA.  grid (ceil(C / 32), groups)
-__global__ void __launch_bounds__(1024) colsum_slabs_kernel(const float* __restrict__ part, float* __restrict__ out, int slabs, int C) {
+__global__ void __launch_bounds__(1024) colsum_slabs_kernel(const RowSlabs first, const RowSlabs second) {
   __shared__ float sh[32][33];
-  chain_begin(part);
+  RowSlabs j = blockIdx.z == 0 ? first : second;
+  chain_begin(j.part);
+  const float* const part = j.part;
+  float* const out = j.out;
+  const int slabs = j.slabs, C = j.C;
+  if (blockIdx.x * 32 >= C || static_cast<int>(blockIdx.y) >= j.groups) return;
   const int c = blockIdx.x * 32 + threadIdx.x;
   float a = 0.f;
   if (c < C) {
@@ -1324,20 +1330,34 @@ __global__ void swap_ri_kernel(const uint4* __restrict__ in, uint4* __restrict__
   }
 }
 
-// fp32 [rows, cols] -> bf16 [rows, pitch], the columns from cols on zero: the weight operand of a 1x1 convolution in one launch
-// (a fill, a cast and a strided copy before); one 16-byte vector per thread
-__global__ void __launch_bounds__(256) cast_pad_kernel(const float* __restrict__ x, uint4* __restrict__ y, int cols, int pitch_v,
-                                                       long long total) {
-  chain_begin(x);
-  const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-  if (i >= total) return;
+// fp32 [rows, cols] -> bf16 [rows, pitch], the columns from cols on zero: the weight operands of one or two pointwise layers in one launch
+// (a fill, a cast and a strided copy each before); one 16-byte vector per thread
+__global__ void __launch_bounds__(256) cast_pad_kernel(CastPad a, CastPad b) {
+  chain_begin(a.x, b.x);
+  long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+  const long long na = a.rows * (a.pitch / 8);
+  const bool second = i >= na;
+  if (second) i -= na;
+  const CastPad& m = second ? b : a;
+  const int pitch_v = m.pitch / 8;
+  if (i >= m.rows * pitch_v) return;
   const long long r = i / pitch_v;
   const int c = static_cast<int>(i - r * pitch_v) * 8;
-  const float* p = x + r * cols + c;
+  const float* p = m.x + r * m.cols + c;
   float f[8];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) f[j] = c + j < cols ? p[j] : 0.f;
-  y[i] = pack8(f);
+  for (int j = 0; j < 8; ++j) f[j] = c + j < m.cols ? p[j] : 0.f;
+  reinterpret_cast<uint4*>(m.y)[i] = pack8(f);
+}
+
+__global__ void __launch_bounds__(256) clear_kernel(float* a, long long na, float* b, long long nb) {
+  chain_begin();
+  const long long va = na / 4, vb = nb / 4, step = static_cast<long long>(gridDim.x) * blockDim.x;
+  const long long first = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+  for (long long i = first; i < va + vb; i += step)
+    reinterpret_cast<float4*>(i < va ? a : b)[i < va ? i : i - va] = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (first < na - va * 4) a[va * 4 + first] = 0.f;
+  if (first < nb - vb * 4) b[vb * 4 + first] = 0.f;
 }
 
 __global__ void cast_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ y, long long n) {
@@ -1496,13 +1516,14 @@ cudaError_t colsum(const __nv_bfloat16* x, float* out, float* scratch, long long
   const cudaError_t e = launch_chained(colsum_kernel, dim3(p.parts, static_cast<unsigned>(p.slabs), groups), dim3(CS_THREADS), 0, s, 1, true,
                                        reinterpret_cast<const uint4*>(x), part, rows, p.V, p.vb, static_cast<int>(p.slab), inner, ostride / 8,
                                        gstride / 8);
-  if (e == cudaSuccess && p.slabs > 1) return colsum_add_slabs(part, out, static_cast<int>(p.slabs), C, groups, s);
+  if (e == cudaSuccess && p.slabs > 1) return colsum_add_slabs(RowSlabs{part, out, static_cast<int>(p.slabs), C, groups}, s);
   return e;
 }
 
-cudaError_t colsum_add_slabs(const float* part, float* out, int slabs, int C, int groups, cudaStream_t s) {
-  return launch_chained(colsum_slabs_kernel, dim3((C + 31) / 32, groups), dim3(32, 32), 0, s, 1, true, part, out, slabs, C);
+cudaError_t colsum_add_slabs(const RowSlabs& a, const RowSlabs& b, cudaStream_t s) {
+  return launch_chained(colsum_slabs_kernel, dim3((std::max(a.C, b.C) + 31) / 32, std::max(a.groups, b.groups), b.C > 0 ? 2 : 1), dim3(32, 32), 0, s, 1, true, a, b);
 }
+cudaError_t colsum_add_slabs(const RowSlabs& a, cudaStream_t s) { return colsum_add_slabs(a, RowSlabs(), s); }
 
 template <typename L>
 static dim3 afno_grid(const L& a, const L& b, int nb) {
@@ -1636,13 +1657,28 @@ cudaError_t cast_f32_bf16(const float* x, __nv_bfloat16* y, long long n, cudaStr
   return cudaGetLastError();
 }
 
-cudaError_t cast_pad_bf16(const float* x, __nv_bfloat16* y, long long rows, int cols, int pitch, cudaStream_t s) {
-  if (rows <= 0 || cols <= 0) return cudaSuccess;
-  if ((pitch & 7) || pitch < cols || !aligned16(y)) return cudaErrorInvalidValue;
-  const long long total = rows * (pitch / 8);
+cudaError_t cast_pad_bf16(const CastPad& a, const CastPad& b, cudaStream_t s) {
+  long long total = 0;
+  for (const CastPad* m : {&a, &b}) {
+    if (m->rows <= 0 || m->cols <= 0) continue;
+    if ((m->pitch & 7) || m->pitch < m->cols || !aligned16(m->y)) return cudaErrorInvalidValue;
+    total += m->rows * (m->pitch / 8);
+  }
+  if (total == 0) return cudaSuccess;
   if ((total + 255) / 256 > 0x7fffffffll) return cudaErrorInvalidValue;
-  return launch_chained(cast_pad_kernel, dim3(static_cast<unsigned>((total + 255) / 256)), dim3(256), 0, s, 1, true, x, reinterpret_cast<uint4*>(y), cols,
-                        pitch / 8, total);
+  const CastPad none = {nullptr, nullptr, 0, 0, 8};
+  return launch_chained(cast_pad_kernel, dim3(static_cast<unsigned>((total + 255) / 256)), dim3(256), 0, s, 1, true, a.rows > 0 && a.cols > 0 ? a : none,
+                        b.rows > 0 && b.cols > 0 ? b : none);
+}
+cudaError_t cast_pad_bf16(const CastPad& a, cudaStream_t s) { return cast_pad_bf16(a, CastPad{nullptr, nullptr, 0, 0, 8}, s); }
+
+cudaError_t clear_f32(float* a, long long na, float* b, long long nb, cudaStream_t s) {
+  if (!a) na = 0;
+  if (!b) nb = 0;
+  if (na + nb <= 0) return cudaSuccess;
+  if (!aligned16(a) || !aligned16(b)) return cudaErrorInvalidValue;
+  const long long blocks = std::min<long long>((na / 4 + nb / 4 + 255) / 256 + 1, 4LL * sm_count());
+  return launch_chained(clear_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, s, 1, true, a, na, b, nb);
 }
 
 cudaError_t fill_normal_bf16(__nv_bfloat16* y, long long n, uint64_t seed, cudaStream_t s) {

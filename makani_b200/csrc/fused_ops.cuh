@@ -64,8 +64,10 @@ cudaError_t inorm_cl_apply(const __nv_bfloat16* x, const __nv_bfloat16* dy, __nv
 long long colsum_scratch(long long rows, int C, int groups = 1);
 cudaError_t colsum(const __nv_bfloat16* x, float* out, float* scratch, long long rows, int C, cudaStream_t s, int groups = 1,
                    long long gstride = 0, int inner = 0, long long ostride = 0);
-// out[g, c] = sum of part[g, 0 .. slabs, c], in a fixed order
-cudaError_t colsum_add_slabs(const float* part, float* out, int slabs, int C, int groups, cudaStream_t s);
+// out[g, c] = sum of part[g, 0 .. slabs, c], in a fixed order, for one or two sets of them
+struct RowSlabs;
+cudaError_t colsum_add_slabs(const RowSlabs& a, cudaStream_t s);
+cudaError_t colsum_add_slabs(const RowSlabs& a, const RowSlabs& b, cudaStream_t s);
 
 // ---- AFNO block weights: one layer's tensors (see the kernels), two layers per launch ----
 struct AfnoLayer {
@@ -131,7 +133,16 @@ cudaError_t swap_ri_bf16(const __nv_bfloat16* in, __nv_bfloat16* out, long long 
 // ---- small elementwise helpers ----
 cudaError_t cast_f32_bf16(const float* x, __nv_bfloat16* y, long long n, cudaStream_t s);
 // fp32 [rows, cols] -> bf16 [rows, pitch] (pitch a multiple of 8, padding columns zero)
-cudaError_t cast_pad_bf16(const float* x, __nv_bfloat16* y, long long rows, int cols, int pitch, cudaStream_t s);
+struct CastPad {
+  const float* x;
+  __nv_bfloat16* y;
+  long long rows;
+  int cols, pitch;
+};
+cudaError_t cast_pad_bf16(const CastPad& a, cudaStream_t s);
+cudaError_t cast_pad_bf16(const CastPad& a, const CastPad& b, cudaStream_t s);
+// zeros in one or two buffers (16-byte aligned; null: none)
+cudaError_t clear_f32(float* a, long long na, float* b, long long nb, cudaStream_t s);
 cudaError_t fill_normal_bf16(__nv_bfloat16* y, long long n, uint64_t seed, cudaStream_t s);
 
 }  // namespace mk

@@ -1363,6 +1363,12 @@ long long mixed_grid(long long grid, const KParams& kp, int bm, int bn) {
   return grid;
 }
 
+// Most tiles of a CTA (or pair) in a launch that begins while the one before it ends.  Its CTAs take the SMs in the order in which these become
+// free, and where CTAs that share operands land on different halves of the chip these are fetched twice: long launches lose more than
+// the gap they save.  384 -> 384 channels over 721 x 1440 tokens (110 tiles) 342 us in the ordinary way, 354 chained; the decoder's
+// training pass 1930 / 1960.
+constexpr long long CHAINED_WAVES = 32;
+
 template <int BN, int EB, int EPI, int CG, bool RAGGED = false>
 cudaError_t launch_t(const CUtensorMap& ma, const BMaps& mb, const CUtensorMap& me, const CUtensorMap& md,
                      const CUtensorMap& mp, const DMaps& mdx, KParams& kp, cudaStream_t stream) {
@@ -1402,13 +1408,14 @@ cudaError_t launch_t(const CUtensorMap& ma, const BMaps& mb, const CUtensorMap& 
     long long clusters = kp.total_tiles < static_cast<uint32_t>(most) ? kp.total_tiles : most;
     if (clusters < 1) clusters = 1;
     if constexpr (EPI != 0 && EPI != 5) clusters = mixed_grid(clusters, kp, 2 * BM, BN);
-    return launch_chained(gemm_kernel<BN, EB, EPI, CG, RAGGED>, dim3(static_cast<unsigned>(2 * clusters)), dim3(threads), smem, stream, 2, true, ma, mb,
+    return launch_chained(gemm_kernel<BN, EB, EPI, CG, RAGGED>, dim3(static_cast<unsigned>(2 * clusters)), dim3(threads), smem, stream, 2,
+                          kp.total_tiles <= CHAINED_WAVES * clusters, ma, mb,
                           me, md, mp, mdx, kp);
   }
   long long grid = kp.total_tiles < static_cast<uint32_t>(num_sms) ? kp.total_tiles : num_sms;
   if (grid < 1) grid = 1;
   if constexpr (EPI != 0 && EPI != 5) grid = mixed_grid(grid, kp, BM, BN);
-  const bool alone = kp.nseg <= 1 && kp.ndx == 0 && kp.sync.nwait == 0 && kp.sync.nsig == 0 && kp.sync.done_ctr == nullptr;
+  const bool alone = kp.total_tiles <= CHAINED_WAVES * grid && kp.nseg <= 1 && kp.ndx == 0 && kp.sync.nwait == 0 && kp.sync.nsig == 0 && kp.sync.done_ctr == nullptr;
   return launch_chained(gemm_kernel<BN, EB, EPI, CG, RAGGED>, dim3(static_cast<unsigned>(grid)), dim3(threads), smem, stream, 1, alone, ma, mb, me, md,
                         mp, mdx, kp);
 }
@@ -1988,7 +1995,8 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
   const cudaError_t launched = run();
   if (launched != cudaSuccess || !kp.rowsum) return launched;
   rows->done = 1;
-  return colsum_add_slabs(kp.rowsum, rows->out, kp.rs_slabs, p.M, kp.rs_groups, stream);
+  rows->slabs = {kp.rowsum, rows->out, kp.rs_slabs, p.M, kp.rs_groups};
+  return rows->later ? cudaSuccess : colsum_add_slabs(rows->slabs, stream);
 #undef MK_DISPATCH
 }
 

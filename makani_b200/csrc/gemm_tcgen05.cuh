@@ -88,6 +88,13 @@ struct GemmPeer {
   void* Dx[7];                     // base pointers matching GemmEpilogue::D (offset already applied)
 };
 
+// Partial sums [groups][slabs][C] that are to be added up over the slabs
+struct RowSlabs {
+  const float* part = nullptr;
+  float* out = nullptr;
+  int slabs = 0, C = 0, groups = 0;
+};
+
 // Optional: the sums over k of the rows of A (the gradient of a bias, beside the weight gradient), fp32 [M], or [z_lo][M] where the
 // z_lo batches have outputs of their own.  Taken where A is MN-major bf16 and the output is fp32 with plain rows; `done` says so.
 struct GemmRowSums {
@@ -95,6 +102,8 @@ struct GemmRowSums {
   float* (*scratch)(void* ctx, long long floats);      // device memory until the work of this launch is done; null on failure
   void* ctx;
   int done;
+  bool later = false;      // the caller adds `slabs` up (colsum_add_slabs), with those of another launch
+  RowSlabs slabs;
 };
 
 // Copy of a strided 2-D block into the same place of `ndst` destination buffers (this device's and its peers'),

@@ -33,6 +33,11 @@ struct Tri {
 };
 enum { ACT_NONE = 0, ACT_GELU = 1, ACT_RELU = 3, ACT_DRELU = 4, ACT_SHRINK = 5, ACT_DSHRINK = 6, ACT_MULAUX = 8 };
 enum { BIAS_NONE = 0, BIAS_ROW = 1, BIAS_COL = 2 };
+// Partial row sums of a launch, held until they are added up
+struct SumsLater {
+  Tensor part;
+  mk::RowSlabs slabs;
+};
 struct Gemm {
   int64_t M = 0, N = 0, K = 0;
   Operand A, B;
@@ -51,6 +56,7 @@ struct Gemm {
   int64_t preact_offset = 0;
   bool preact_deriv = false, accumulate = false;
   Tensor* row_sums = nullptr;        // see mk::GemmRowSums
+  SumsLater* sums_later = nullptr;   // the partial sums are added up with another launch's
 };
 
 // Validates, launches on the current stream and raises; whether the row sums were taken.

@@ -25,8 +25,17 @@ const __nv_bfloat16* bf(const Tensor& t) { return reinterpret_cast<const __nv_bf
 __nv_bfloat16* bf_mut(const Tensor& t) { return reinterpret_cast<__nv_bfloat16*>(t.data_ptr()); }
 const float* f32_or_null(const Tensor& t) { return t.defined() ? t.data_ptr<float>() : nullptr; }
 float* f32_mut(const Tensor& t) { return t.defined() ? t.data_ptr<float>() : nullptr; }
-Tensor zeros_f32(at::IntArrayRef shape, const Tensor& like) { return at::zeros(shape, like.options().dtype(at::kFloat)); }
 Tensor empty_f32(at::IntArrayRef shape, const Tensor& like) { return at::empty(shape, like.options().dtype(at::kFloat)); }
+// zeros in one or two tensors, one launch
+void clear(Tensor& a, Tensor* b = nullptr) {
+  ++mkh::launches();
+  mkh::check(mk::clear_f32(a.data_ptr<float>(), a.numel(), b ? b->data_ptr<float>() : nullptr, b ? b->numel() : 0, mkh::stream()), "clear");
+}
+Tensor zeros_f32(at::IntArrayRef shape, const Tensor& like) {
+  Tensor t = empty_f32(shape, like);
+  clear(t);
+  return t;
+}
 Tensor value(const OptTensor& t) { return t.has_value() ? *t : Tensor(); }
 OptTensor maybe(const Tensor& t) { return t.defined() ? OptTensor(t) : OptTensor(); }
 // (a parameter on the host or another GPU is refused: its address would reach a kernel, or its copy be paid for on every call)
@@ -85,20 +94,35 @@ mkh::Operand channel_rows(const Act& x) {
   return x.cl ? mkh::Operand{&x.t, x.C, true, 0, x.T * x.C, 0} : mkh::Operand{&x.t, x.T, false, 0, x.C * x.T, 0};
 }
 
-// fp32 [Co, Ci(, 1, 1)] -> bf16 [Co, pad8(Ci)]; bf16 weights of a linear layer as they are
-Tensor prep_weight(const Tensor& w, const Tensor& like) {
-  MK_CHECK(w.device() == like.device(), "layers: tensors must be on one CUDA device");
-  const Tensor w2 = w.detach().reshape({w.size(0), -1});
-  if (like.dim() == 2 && w.dim() == 2 && w2.scalar_type() == like.scalar_type() && w2.size(1) % 8 == 0) return w2.contiguous();
-  const int64_t co = w2.size(0), ci = w2.size(1), pitch = (ci + 7) / 8 * 8;
-  if (w2.scalar_type() == at::kFloat && w2.is_contiguous()) {
-    Tensor out = at::empty({co, pitch}, like.options());
-    ++mkh::launches();
-    mkh::check(mk::cast_pad_bf16(w2.data_ptr<float>(), bf_mut(out), co, static_cast<int>(ci), static_cast<int>(pitch), mkh::stream()), "cast_pad");
-    return out;
+// fp32 [Co, Ci(, 1, 1)] -> bf16 [Co, pad8(Ci)], of one or two layers in one launch; bf16 weights of a linear layer as they are
+void prep_weights(std::initializer_list<const Tensor*> ws, const Tensor& like, Tensor* out) {
+  Tensor held[2];
+  mk::CastPad jobs[2] = {};
+  int n = 0;
+  for (const Tensor* w : ws) {
+    MK_CHECK(w->device() == like.device(), "layers: tensors must be on one CUDA device");
+    const Tensor w2 = w->detach().reshape({w->size(0), -1});
+    const int64_t co = w2.size(0), ci = w2.size(1), pitch = (ci + 7) / 8 * 8;
+    if (like.dim() == 2 && w->dim() == 2 && w2.scalar_type() == like.scalar_type() && ci % 8 == 0) {
+      *out++ = w2.contiguous();
+    } else if (w2.scalar_type() == at::kFloat && w2.is_contiguous()) {
+      *out = at::empty({co, pitch}, like.options());
+      jobs[n] = {w2.data_ptr<float>(), bf_mut(*out), co, static_cast<int>(ci), static_cast<int>(pitch)};
+      held[n++] = w2;
+      ++out;
+    } else {
+      *out = at::zeros({co, pitch}, like.options());
+      out->narrow(1, 0, ci).copy_(w2);
+      ++out;
+    }
   }
-  Tensor out = at::zeros({co, pitch}, like.options());
-  out.narrow(1, 0, ci).copy_(w2);
+  if (n == 0) return;
+  ++mkh::launches();
+  mkh::check(n == 2 ? mk::cast_pad_bf16(jobs[0], jobs[1], mkh::stream()) : mk::cast_pad_bf16(jobs[0], mkh::stream()), "cast_pad");
+}
+Tensor prep_weight(const Tensor& w, const Tensor& like) {
+  Tensor out;
+  prep_weights({&w}, like, &out);
   return out;
 }
 
@@ -172,9 +196,9 @@ Tensor channel_sums(const Act& x) {
   return x.t.dim() == 2 ? x.t.to(at::kFloat).sum(0) : x.t.to(at::kFloat).sum(at::IntArrayRef{0, 2, 3});
 }
 
-// dw[co, ci] = sum over batch and tokens of dy x, and the sums of dy beside it
-Tensor weight_gradient(const Act& dy, const Act& x, Tensor* db) {
-  Tensor dw = zeros_f32({dy.C, x.C}, dy.t);
+// dw[co, ci] (cleared before) += sum over batch and tokens of dy x, and the sums of dy beside it: complete, or (`later`) once their slabs are
+// added up
+void weight_gradient(const Act& dy, const Act& x, Tensor& dw, Tensor* db, mkh::SumsLater* later = nullptr) {
   Gemm g;
   g.M = dy.C;
   g.N = x.C;
@@ -190,10 +214,10 @@ Tensor weight_gradient(const Act& dy, const Act& x, Tensor* db) {
   if (db) {
     sums = empty_f32({dy.C}, dy.t);
     g.row_sums = &sums;
+    g.sums_later = later;
   }
   const bool done = mkh::run(g);
   if (db) *db = done ? sums : channel_sums(dy);
-  return dw;
 }
 
 bool default_cl(int64_t co) { return co % 8 == 0; }
@@ -218,8 +242,12 @@ std::tuple<OptTensor, OptTensor, OptTensor> conv_backward(const Tensor& dy, cons
   const Act g = act_of(dy), xa = act_of(x);
   Tensor dx, dw, db;
   if (need_x) dx = data_gradient(g, wq, ci, mkh::ACT_NONE, Tensor(), xa.cl).t;
-  if (need_w) dw = weight_gradient(g, xa, need_b ? &db : nullptr);
-  else if (need_b) db = channel_sums(g);
+  if (need_w) {
+    dw = zeros_f32({g.C, xa.C}, x);
+    weight_gradient(g, xa, dw, need_b ? &db : nullptr);
+  } else if (need_b) {
+    db = channel_sums(g);
+  }
   return {maybe(dx), maybe(dw), maybe(db)};
 }
 
@@ -227,7 +255,9 @@ std::tuple<OptTensor, OptTensor, OptTensor> conv_backward(const Tensor& dy, cons
 std::tuple<Tensor, Tensor, Tensor, OptTensor, OptTensor> mlp_forward(const Tensor& x, const Tensor& w1, const OptTensor& b1, const Tensor& w2,
                                                                      const OptTensor& b2, const OptTensor& resid, int64_t layout, bool train) {
   c10::cuda::CUDAGuard guard(x.device());
-  const Tensor w1q = prep_weight(w1, x), w2q = prep_weight(w2, x), b1f = as_f32(b1, x), b2f = as_f32(b2, x), r = value(resid);
+  Tensor wq[2];
+  prep_weights({&w1, &w2}, x, wq);
+  const Tensor &w1q = wq[0], &w2q = wq[1], b1f = as_f32(b1, x), b2f = as_f32(b2, x), r = value(resid);
   const int64_t ch = w1.size(0);
   Tensor dact;
   const Act h = forward(act_of(x), w1q, w1.size(1), b1f, mkh::ACT_GELU, Tensor(), train ? &dact : nullptr, train, default_cl(ch));
@@ -240,11 +270,18 @@ std::tuple<OptTensor, Tensor, OptTensor, Tensor, OptTensor> mlp_backward(const T
                                                                          bool has_b2) {
   c10::cuda::CUDAGuard guard(x.device());
   const Act g = act_of(dy), xa = act_of(x), ha = act_of(h);
+  Tensor db1, db2, dx, dw1 = empty_f32({ha.C, xa.C}, x), dw2 = empty_f32({g.C, ha.C}, x);
+  // (one launch each that clears both gradients, casts both weights, adds up both sums: at 16200 tokens every small launch costs some 4 us)
+  clear(dw1, &dw2);
   const Act dpre = data_gradient(g, w2q, ha.C, mkh::ACT_MULAUX, dact, ha.cl);
-  Tensor db1, db2, dx;
-  const Tensor dw2 = weight_gradient(g, ha, has_b2 ? &db2 : nullptr);
+  mkh::SumsLater s1, s2;
+  weight_gradient(g, ha, dw2, has_b2 ? &db2 : nullptr, &s2);
   if (need_x) dx = data_gradient(dpre, w1q, ci, mkh::ACT_NONE, Tensor(), xa.cl).t;
-  const Tensor dw1 = weight_gradient(dpre, xa, has_b1 ? &db1 : nullptr);
+  weight_gradient(dpre, xa, dw1, has_b1 ? &db1 : nullptr, &s1);
+  if (s1.slabs.C > 0 || s2.slabs.C > 0)
+    mkh::check(s1.slabs.C > 0 && s2.slabs.C > 0 ? mk::colsum_add_slabs(s1.slabs, s2.slabs, mkh::stream())
+                                                : mk::colsum_add_slabs(s1.slabs.C > 0 ? s1.slabs : s2.slabs, mkh::stream()),
+               "colsum_add_slabs");
   return {maybe(dx), dw1, maybe(db1), dw2, maybe(db2)};
 }
 

@@ -273,3 +273,27 @@ def test_launches_that_begin_early_see_their_operands():
         torch.cuda.synchronize()
         assert torch.equal(y, want) and all(torch.equal(a, e) for a, e in zip(sums, want_sums))
     _ext.check_device_errors(dev)
+
+
+@pytest.mark.parametrize("co,ch", [(1, 8), (3, 8), (4, 24), (9, 40), (73, 384)])
+def test_mlp_gradients_are_added_to_zero(co, ch):
+    """Both weight gradients of an MLP start from zero, whatever the memory held, and both bias gradients are complete: numbers of values off
+    and at whole vectors, sums from the slabs of the gradients and by passes of their own (fields out)."""
+    dev = _dev()
+    g = torch.Generator(dev).manual_seed(ch)
+    ext, ci = _ext.require(), 8
+    for out, layout in ((0, "nchw"), (1, "cl")) if co % 8 == 0 else ((0, "nchw"),):
+        x = _cl(g, 2, ci, 8, 16)
+        w1, w2 = torch.randn(ch, ci, 1, 1, device=dev, generator=g), torch.randn(co, ch, 1, 1, device=dev, generator=g)
+        b1, b2 = torch.randn(ch, device=dev, generator=g), torch.randn(co, device=dev, generator=g)
+        y, w1q, w2q, dact, h = ext.mlp_forward(x, w1, b1, w2, b2, None, out, True)
+        dy = _as(_cl(g, 2, co, 8, 16), layout)
+        held = [torch.full((k,), float("nan"), device=dev) for k in (ch * ci, co * ch, co, ch, 4096)]
+        del held      # the gradients take their places
+        _, dw1, db1, dw2, db2 = ext.mlp_backward(dy, x, w1q, w2q, dact, h, ci, True, True, True)
+        rows = lambda t: t.double().permute(1, 0, 2, 3).flatten(1)  # noqa: E731
+        dpre = (torch.einsum("oc,bohw->bchw", w2q[:, :ch].double(), dy.double()) * dact.double()).bfloat16()
+        for got, ref, tol in ((dw2, rows(dy) @ rows(h).t(), 1e-6), (db2, dy.double().sum((0, 2, 3)), 1e-6),
+                              (dw1, rows(dpre) @ rows(x).t(), 1e-2), (db1, dpre.double().sum((0, 2, 3)), 1e-2)):      # (dpre: other roundings)
+            assert (got.double() - ref).norm() <= tol * ref.norm()
+    _ext.check_device_errors(dev)
