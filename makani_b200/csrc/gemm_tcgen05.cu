@@ -1844,8 +1844,10 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
                    e.d_half))
       epi = 5;
   }
-  // CTA pairs (256-row tiles, each CTA loads half of the B tile): single-device bf16 launches without row-triangular
-  // structure and with at least two row blocks.  MAKANI_B200_CTA_PAIRS=0 / 1 forces none / all eligible launches.  Measured, time on
+  // CTA pairs (256-row tiles, each CTA loads half of the B tile): single-device bf16 launches with at least two row blocks and no
+  // row-triangular structure, unless one pair covers all rows: the half that single CTAs would skip for half of the batches costs
+  // less than their loads (Legendre analysis of 240 degrees, 241 orders, 384 channels, 240 latitudes 53 -> 46 us, 721 latitudes 102 -> 88; 256
+  // channels and 180 degrees the same).  MAKANI_B200_CTA_PAIRS=0 / 1 forces none / all eligible launches.  Measured, time on
   // single CTAs over time on pairs (plain store, product with an operand, GELU with two outputs):
   //   K = 768, 115200 rows: 1.07 - 1.30.  From K = 512 on the long k loop pays for the pair's longer start.
   //   K = 256 - 448: 1024 - 8192 rows 0.89 - 0.96 (768 outputs at 8192 rows 0.91 - 1.09); 16200 rows, 384 outputs 0.92 - 0.99, 768
@@ -1863,7 +1865,8 @@ cudaError_t gemm_launch(const GemmProblem& p, const GemmOperand& A, const GemmOp
   const bool no_peer = (peer == nullptr) || (peer->nseg <= 1 && peer->ndx == 0 && peer->nwait == 0 && peer->nsig == 0 &&
                                               peer->done_ctr == nullptr);
   const bool ragged = epi >= 1 && epi <= 4 && kp.n_full != p.N && p.cplx == 0;
-  const bool eligible = eb == 2 && no_peer && !ragged && p.M > BM && p.rmin_a == 0 && p.rmax_a == 0 && (p.cplx == 0 || p.cplx >= 3);
+  const bool triangle = (p.rmin_a != 0 || p.rmax_a != 0) && (p.cplx != 0 || p.M > 2 * BM);
+  const bool eligible = eb == 2 && no_peer && !ragged && p.M > BM && !triangle && (p.cplx == 0 || p.cplx >= 3);
   const int pad1 = (p.M + BM - 1) / BM * BM, pad2 = (p.M + 2 * BM - 1) / (2 * BM) * (2 * BM);
   const long long z_all = static_cast<long long>(p.zlo_n) * p.zhi_n;
   const bool waves = pad1 / BM * ((p.N + 255) / 256) * z_all >= 2 * sm_count();

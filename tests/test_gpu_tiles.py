@@ -5,7 +5,7 @@ import torch
 
 from makani_b200.ops import _ext
 from makani_b200.ops.gemm import (ACT_DGELU, ACT_DRELU, ACT_DSHRINK, ACT_GELU, ACT_MULAUX, ACT_NONE, ACT_RELU, ACT_SHRINK, BIAS_COL,
-                                  BIAS_ROW, Operand, Output, gemm)
+                                  BIAS_ROW, Operand, Output, Tri, gemm)
 from test_gpu_kernels import _dev, _rel, _run_both
 
 pytestmark = pytest.mark.gpu
@@ -1013,4 +1013,23 @@ def test_narrow_last_column_tile_over_many_rows(n, epi):
     else:
         y = z if aux is None else (z + aux.double() if epi == "resid" else z * aux.double())
     assert _rel(d, y.detach()) < BF16
+    _ext.check_device_errors(dev)
+
+
+@pytest.mark.parametrize("l,m,h,n", [(129, 130, 216, 48), (240, 241, 240, 136), (256, 9, 520, 200), (257, 20, 208, 72)])
+def test_triangular_rows_on_one_pair(l, m, h, n):
+    """Row-triangular products whose rows one CTA pair covers (and one more row than that): zeros below the first valid row, also for
+    batches that have none in the first half of the pair, and nothing left unwritten."""
+    dev = _dev()
+    g = torch.Generator(dev).manual_seed(l)
+    hp = (h + 7) // 8 * 8
+    keep = (torch.arange(l, device=dev)[None] >= torch.arange(m, device=dev)[:, None])[..., None]
+    table = torch.randn(m, l, hp, device=dev, generator=g).mul(keep).to(torch.bfloat16)
+    table[..., h:] = 0
+    x = torch.randn(m, h, n, device=dev, generator=g).to(torch.bfloat16)
+    d = torch.full((m, l, n), float("nan"), device=dev, dtype=torch.bfloat16)
+    gemm(l, n, h, Operand(table, ld=hp, zs_hi=l * hp), Operand(x, ld=n, mn_major=True, zs_hi=h * n), Output(d, rs_lo=n, d_zhi=l * n), zhi_n=m,
+         tri=Tri(rmin_a=1))
+    ref = torch.einsum("mlh,mhn->mln", table[..., :h].double(), x.double())
+    assert _rel(d, ref) < BF16 and bool((d[~keep.expand_as(d)] == 0).all())
     _ext.check_device_errors(dev)
