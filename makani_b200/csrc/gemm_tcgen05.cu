@@ -1363,11 +1363,12 @@ long long mixed_grid(long long grid, const KParams& kp, int bm, int bn) {
   return grid;
 }
 
-// Most tiles of a CTA (or pair) in a launch that begins while the one before it ends.  Its CTAs take the SMs in the order in which these become
-// free, and where CTAs that share operands land on different halves of the chip these are fetched twice: long launches lose more than
-// the gap they save.  384 -> 384 channels over 721 x 1440 tokens (110 tiles) 342 us in the ordinary way, 354 chained; the decoder's
-// training pass 1930 / 1960.
-constexpr long long CHAINED_WAVES = 32;
+// Most k slabs of a CTA (or pair) in a launch that begins while the one before it ends.  Its CTAs take the SMs in the order in which these
+// become free, and where CTAs that share operands land on different halves of the chip these are fetched twice: long launches lose more
+// than the gap they save.  384 -> 384 channels over 721 x 1440 tokens (660 slabs) 342 us in the ordinary way, 354 chained; the decoder's training
+// pass, with the gradients of its weights (330 slabs and more) chained 1984, without 1969.  The products of 115200 tokens or 16200 x 768
+// -> 3072 have 110 to 150: 596 -> 582 and 518 -> 503 chained.
+constexpr long long CHAINED_SLABS = 256;
 
 template <int BN, int EB, int EPI, int CG, bool RAGGED = false>
 cudaError_t launch_t(const CUtensorMap& ma, const BMaps& mb, const CUtensorMap& me, const CUtensorMap& md,
@@ -1397,6 +1398,7 @@ cudaError_t launch_t(const CUtensorMap& ma, const BMaps& mb, const CUtensorMap& 
     configured = true;
   }
   const int num_sms = sm_count();
+  const long long slabs = static_cast<long long>(kp.k_per_split) * (kp.cplx ? 2 : 1) * EB / 128;
   // tile order (MAKANI_B200_TILE_ORDER=m|n forces one order for A/B timing)
   static const int forced_order = [] {
     const char* e = getenv("MAKANI_B200_TILE_ORDER");
@@ -1409,13 +1411,13 @@ cudaError_t launch_t(const CUtensorMap& ma, const BMaps& mb, const CUtensorMap& 
     if (clusters < 1) clusters = 1;
     if constexpr (EPI != 0 && EPI != 5) clusters = mixed_grid(clusters, kp, 2 * BM, BN);
     return launch_chained(gemm_kernel<BN, EB, EPI, CG, RAGGED>, dim3(static_cast<unsigned>(2 * clusters)), dim3(threads), smem, stream, 2,
-                          kp.total_tiles <= CHAINED_WAVES * clusters, ma, mb,
+                          kp.total_tiles * slabs <= CHAINED_SLABS * clusters, ma, mb,
                           me, md, mp, mdx, kp);
   }
   long long grid = kp.total_tiles < static_cast<uint32_t>(num_sms) ? kp.total_tiles : num_sms;
   if (grid < 1) grid = 1;
   if constexpr (EPI != 0 && EPI != 5) grid = mixed_grid(grid, kp, BM, BN);
-  const bool alone = kp.total_tiles <= CHAINED_WAVES * grid && kp.nseg <= 1 && kp.ndx == 0 && kp.sync.nwait == 0 && kp.sync.nsig == 0 && kp.sync.done_ctr == nullptr;
+  const bool alone = kp.total_tiles * slabs <= CHAINED_SLABS * grid && kp.nseg <= 1 && kp.ndx == 0 && kp.sync.nwait == 0 && kp.sync.nsig == 0 && kp.sync.done_ctr == nullptr;
   return launch_chained(gemm_kernel<BN, EB, EPI, CG, RAGGED>, dim3(static_cast<unsigned>(grid)), dim3(threads), smem, stream, 1, alone, ma, mb, me, md,
                         mp, mdx, kp);
 }
