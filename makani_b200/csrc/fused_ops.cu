@@ -441,7 +441,7 @@ __global__ void __launch_bounds__(ClSums<MODE>::THREADS + 32, 1) inorm_cl_sums_k
   const int v = threadIdx.x % V, r = threadIdx.x / V;
   const int bidx = blockIdx.y;
   cl_init<P>(cl_ring);
-  chain_begin(x, dy, w, b, stats);
+  chain_begin(xc.npeers == 0, x, dy, w, b, stats);
   __syncthreads();
   // partial sums of the rows of threads, in the ring's place: those of row r from C r on, sums before products
   f32x2* const part = reinterpret_cast<f32x2*>(cl_ring);
@@ -612,7 +612,7 @@ __global__ void __launch_bounds__(ClApply<MODE>::THREADS + 32, 1) inorm_cl_apply
   // [C][2] merged sums of this sample (exchange mode only), behind the ring
   float* const sh_sum = reinterpret_cast<float*>(cl_ring + CL_BARRIERS / 16 + P::DEPTH * P::LAPS * P::TENSORS * R * V);
   cl_init<P>(cl_ring);
-  chain_begin(x, dy, w, b, sums, stats);
+  chain_begin(xc.npeers == 0, x, dy, w, b, sums, stats);
   if (xc.npeers > 0) {
     // every peer's sums must have arrived in the local buffer
     __shared__ int ok_s;
@@ -731,7 +731,7 @@ __global__ void __launch_bounds__(CS_THREADS) colsum_kernel(const uint4* __restr
                                                             int V, int vb, int slab, int inner, long long ostride_v,
                                                             long long gstride_v) {
   __shared__ __align__(16) float sh[CS_THREADS * 8];
-  chain_begin(x);
+  chain_begin(true, x);
   const int v0 = blockIdx.x * vb;
   const int nv = min(vb, V - v0);          // 16-byte columns of this CTA
   const int R = CS_THREADS / vb;
@@ -792,7 +792,7 @@ __global__ void __launch_bounds__(CS_THREADS) colsum_kernel(const uint4* __restr
 __global__ void __launch_bounds__(1024) colsum_slabs_kernel(const RowSlabs first, const RowSlabs second) {
   __shared__ float sh[32][33];
   RowSlabs j = blockIdx.z == 0 ? first : second;
-  chain_begin(j.part);
+  chain_begin(true, j.part);
   const float* const part = j.part;
   float* const out = j.out;
   const int slabs = j.slabs, C = j.C;
@@ -1077,7 +1077,7 @@ __global__ void __launch_bounds__(256) adamw_kernel(const AdamEntry* __restrict_
 __global__ void __launch_bounds__(256) afno_pack_kernel(const AfnoLayer a, const AfnoLayer b, int nb) {
   __shared__ float re[32][33], im[32][33];
   AfnoLayer L = blockIdx.z < static_cast<unsigned>(nb) ? a : b;
-  chain_begin(L.w, L.b);
+  chain_begin(true, L.w, L.b);
   const int blk = blockIdx.z % nb, i0 = blockIdx.x * 32, o0 = blockIdx.y * 32;
   if (i0 >= L.nin || o0 >= L.nout) return;
   const long long plane = static_cast<long long>(nb) * L.nin * L.nout;
@@ -1115,7 +1115,7 @@ __global__ void __launch_bounds__(256) afno_pack_kernel(const AfnoLayer a, const
 __global__ void __launch_bounds__(256) afno_fold_kernel(const AfnoGrad a, const AfnoGrad b, int nb) {
   __shared__ float re[32][33], im[32][33];
   AfnoGrad L = blockIdx.z < static_cast<unsigned>(nb) ? a : b;
-  chain_begin(L.dwx, L.dbx);
+  chain_begin(true, L.dwx, L.dbx);
   const int blk = blockIdx.z % nb, i0 = blockIdx.x * 32, o0 = blockIdx.y * 32;
   if (i0 >= L.nin || o0 >= L.nout) return;
   const float* const wx = L.dwx + static_cast<long long>(blk) * 4 * L.nin * L.nout;
@@ -1333,7 +1333,7 @@ __global__ void swap_ri_kernel(const uint4* __restrict__ in, uint4* __restrict__
 // fp32 [rows, cols] -> bf16 [rows, pitch], the columns from cols on zero: the weight operands of one or two pointwise layers in one launch
 // (a fill, a cast and a strided copy each before); one 16-byte vector per thread
 __global__ void __launch_bounds__(256) cast_pad_kernel(CastPad a, CastPad b) {
-  chain_begin(a.x, b.x);
+  chain_begin(true, a.x, b.x);
   long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
   const long long na = a.rows * (a.pitch / 8);
   const bool second = i >= na;
@@ -1351,7 +1351,7 @@ __global__ void __launch_bounds__(256) cast_pad_kernel(CastPad a, CastPad b) {
 }
 
 __global__ void __launch_bounds__(256) clear_kernel(float* a, long long na, float* b, long long nb) {
-  chain_begin();
+  chain_begin(true);
   const long long va = na / 4, vb = nb / 4, step = static_cast<long long>(gridDim.x) * blockDim.x;
   const long long first = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
   for (long long i = first; i < va + vb; i += step)

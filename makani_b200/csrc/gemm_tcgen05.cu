@@ -333,7 +333,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ B
       asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
   }
-  chain_begin();
+  chain_begin(p.sync.nwait == 0);
   if (threadIdx.x == 0) {
     // segments written by the peers (and the peers' copies this kernel overwrites) must be ready: bounded wait on local flags.
     // The whole CTA waits (not only the producer) so that no epilogue store of an all-zero tile can run early.

@@ -4,7 +4,8 @@
 // set up what is theirs (barriers, tensor memory) and wait in `chain_begin` until that kernel is complete and its writes are visible.
 // `chain_begin` also lets the next kernel of the chain begin in the same way.  Every kernel launched like this calls it, in all its threads,
 // before its first access to global memory; a complete kernel has then seen all kernels before it complete.  Kernels that wait for other
-// devices are launched in the ordinary way.
+// devices are launched in the ordinary way, and the next one begins when they are complete: blocks that wait behind a wait would hold
+// shared memory that kernels of other streams may need.
 //
 // What it saves is the time between two launches (some 2 us) and the set-up: the AFNO filter of 90 x 180 tokens, 17 products of 10 - 20 us,
 // 256 -> 236 us a training pass, the token MLP (16200 x 768 -> 3072) 525 -> 511, the MLP of 240 x 480 tokens 600 -> 590.  For grids of one wave: a block that begins later pays for the
@@ -18,11 +19,11 @@
 namespace mk {
 
 #ifdef __CUDACC__
-// `p`: pointers whose loads the compiler may take for constant during the kernel (const __restrict__) and could move in front of the wait; they
+// `next` false: the next kernel does not begin before this one is complete.  `p`: pointers whose loads the compiler may take for constant during the kernel (const __restrict__) and could move in front of the wait; they
 // come out of it as new values.
 template <typename... P>
-__device__ __forceinline__ void chain_begin(P&... p) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+__device__ __forceinline__ void chain_begin(bool next, P&... p) {
+  if (next) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   auto renew = [](auto& q) { asm volatile("" : "+l"(q)::"memory"); };
   (renew(p), ...);

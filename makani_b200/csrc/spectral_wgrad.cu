@@ -68,7 +68,7 @@ spectral_wgrad_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  chain_begin();
+  chain_begin(true);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
