@@ -8,8 +8,9 @@
 // shared memory that kernels of other streams may need.
 //
 // What it saves is the time between two launches (some 2 us) and the set-up: the AFNO filter of 90 x 180 tokens, 17 products of 10 - 20 us,
-// 256 -> 236 us a training pass, the token MLP (16200 x 768 -> 3072) 525 -> 511, the MLP of 240 x 480 tokens 600 -> 590.  For grids of one wave: a block that begins later pays for the
-// wait without need (the re-layout of the spectral weights, 18432 blocks, 70 -> 90 and 99 -> 134 us; launched in the ordinary way).
+// 256 -> 236 us a training pass, the token MLP (16200 x 768 -> 3072) 525 -> 511, the MLP of 240 x 480 tokens 600 -> 590.  For grids of one
+// wave: a block that begins later pays for the wait without need (the re-layout of the spectral weights, 18432 blocks, 70 -> 90 and
+// 99 -> 134 us; launched in the ordinary way).
 #pragma once
 #include <cuda_runtime.h>
 #include <string.h>
