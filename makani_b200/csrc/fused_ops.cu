@@ -5,6 +5,7 @@
 #include "gelu.cuh"
 #include "gemm_tcgen05.cuh"
 #include "launch.cuh"
+#include "norm_ring.h"
 #include <cstring>
 #include <type_traits>
 
@@ -263,24 +264,12 @@ __global__ void __launch_bounds__(NT) inorm_bwd_kernel(const __nv_bfloat16* __re
 // x: [B, T, C] with C contiguous (C % 8 == 0, C <= 1024).  Thread (v, r) = (tid % V, tid / V), V = C / CH, owns CH
 // channels of every row it meets, so per-channel constants stay in registers.
 
-// The four kernels: channels of a thread, most threads that work on rows (whole rows of them are used, one more warp loads), rows per thread in
-// a stage of the ring and stages.  One CTA per SM.  721 x 1440 x 384, us, by (rows, stages): forward sums (1, 8) 147, (2, 5) 139; forward output
-// (1, 8) 274, (2, 5) 285, (2, 3) 260; gradient with GELU (1, 8) 428, (2, 4) 387, (4, 2) 370, by four channels and 992 threads (4, 3) 389.
-// The backward sums wait for the fp32 pipe and the issue slots, not for rows: without a test per row 330 instead of 352, and by four channels of
-// a thread as by eight, but 51 us instead of 61 at 240 x 480.
-struct ClForwardSums { static constexpr int CH = 8, THREADS = 992, LAPS = 2, DEPTH = 5, TENSORS = 1; };
-struct ClForwardApply { static constexpr int CH = 8, THREADS = 992, LAPS = 2, DEPTH = 3, TENSORS = 1; };
-struct ClBackwardSums { static constexpr int CH = 4, THREADS = 992, LAPS = 4, DEPTH = 3, TENSORS = 2; };
-struct ClBackwardApply { static constexpr int CH = 8, THREADS = 608, LAPS = 4, DEPTH = 2, TENSORS = 2; };
 template <int MODE>
 using ClSums = std::conditional_t<MODE == 0, ClForwardSums, ClBackwardSums>;
 template <int MODE>
 using ClApply = std::conditional_t<MODE == 0, ClForwardApply, ClBackwardApply>;
 template <int CH>
 using ClWord = std::conditional_t<CH == 8, uint4, uint2>;      // the channels of a thread
-template <typename P>
-__host__ __device__ constexpr int cl_ring_bytes(int threads) { return P::DEPTH * P::LAPS * P::TENSORS * 2 * P::CH * threads; }
-constexpr int CL_BARRIERS = 128;      // bytes in front of the ring
 
 // mode 0: sums of (x, x^2).  mode 1: sums of (g, g * xhat) with g = dy * act'(xhat * w + b) for the backward pass.
 __device__ __forceinline__ unsigned int xch_ld_acquire(const unsigned int* ptr) {
@@ -367,12 +356,12 @@ __device__ __forceinline__ void cl_init(uint4* smem) {      // (by all threads, 
   }
 }
 template <typename P, bool BACK, typename Use>
-__device__ __forceinline__ void cl_rows(uint4* smem, const __nv_bfloat16* x, const __nv_bfloat16* dy, int V, int r, int R, long long T, int* err,
-                                        Use&& use) {
+__device__ __forceinline__ void cl_rows(uint4* smem, int offset, const __nv_bfloat16* x, const __nv_bfloat16* dy, int V, int r, int R, long long T,
+                                        int* err, Use&& use) {
   using Word = ClWord<P::CH>;
-  static_assert(P::DEPTH * 16 <= CL_BARRIERS && P::DEPTH * P::LAPS * P::TENSORS >= 4, "the partial sums take the ring's place");
+  static_assert(P::DEPTH * 16 <= CL_BARRIERS, "two barriers a stage");
   const uint32_t bars = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
-  const Word* const ring = reinterpret_cast<const Word*>(smem + CL_BARRIERS / 16);
+  const Word* const ring = reinterpret_cast<const Word*>(smem + offset / 16);
   const int rows = P::LAPS * R, half = rows * V;      // rows and words of one tensor in a stage
   const long long hop = static_cast<long long>(gridDim.x) * rows;
   const long long stages = (T + rows - 1) / rows;
@@ -389,7 +378,7 @@ __device__ __forceinline__ void cl_rows(uint4* smem, const __nv_bfloat16* x, con
   };
   if (threadIdx.x / 32 == blockDim.x / 32 - 1) {
     if ((threadIdx.x & 31) == 0) {
-      const uint32_t dst = bars + CL_BARRIERS, row = V * sizeof(Word);
+      const uint32_t dst = bars + offset, row = V * sizeof(Word);
       for (int k = 0; k < count; ++k, next()) {
         if (!cl_wait(bars + 16 * s + 8, ph ^ 1u, err)) break;
         const uint32_t bytes = static_cast<uint32_t>(min(static_cast<long long>(rows), T - t)) * row;
@@ -429,22 +418,23 @@ __global__ void __launch_bounds__(ClSums<MODE>::THREADS + 32, 1) inorm_cl_sums_k
                                                                    const float* __restrict__ w, const float* __restrict__ b,
                                                                    const float* __restrict__ stats, float* __restrict__ sums,
                                                                    float* __restrict__ dw, float* __restrict__ db, int C, long long T,
-                                                                   int act, int shifted, const StatExchange xc) {
+                                                                   int R, int act, int shifted, const StatExchange xc) {
   extern __shared__ __align__(16) uint4 cl_ring[];
   GeluBwdPairs gc;
   if constexpr (MODE == 1) gc = gelu_bwd_pairs(coef_of(act));
   using P = ClSums<MODE>;
   using Word = ClWord<P::CH>;
   constexpr int PAIRS = P::CH / 2;
+  static_assert(cl_sums_fit<P>(), "the partial sums take the ring's place");
   const int V = C / P::CH;
-  const int R = (static_cast<int>(blockDim.x) - 32) / V;
   const int v = threadIdx.x % V, r = threadIdx.x / V;
   const int bidx = blockIdx.y;
   cl_init<P>(cl_ring);
   chain_begin(xc.npeers == 0, x, dy, w, b, stats);
   __syncthreads();
+  constexpr int RING = cl_ring_offset(0, false);
   // partial sums of the rows of threads, in the ring's place: those of row r from C r on, sums before products
-  f32x2* const part = reinterpret_cast<f32x2*>(cl_ring);
+  f32x2* const part = reinterpret_cast<f32x2*>(cl_ring + RING / 16);
   f32x2 a0[PAIRS], a1[PAIRS];
   {
     // Pairs of channels in packed fp32 arithmetic: a packed instruction takes two cycles of a scheduler's fp32 pipe, three where it reads three
@@ -502,7 +492,7 @@ __global__ void __launch_bounds__(ClSums<MODE>::THREADS + 32, 1) inorm_cl_sums_k
         }
       }
     };
-    cl_rows<P, false>(cl_ring, xb, gb, V, r, R, T, xc.err, [&](long long, const Word& xr, const Word& gr) { accum(xr, gr); });
+    cl_rows<P, false>(cl_ring, RING, xb, gb, V, r, R, T, xc.err, [&](long long, const Word& xr, const Word& gr) { accum(xr, gr); });
     if (MODE == 1) {
 #pragma unroll
       for (int j = 0; j < PAIRS; ++j) {
@@ -601,16 +591,16 @@ template <int MODE>
 __global__ void __launch_bounds__(ClApply<MODE>::THREADS + 32, 1) inorm_cl_apply_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
                                                                     __nv_bfloat16* __restrict__ out, const float* __restrict__ w,
                                                                     const float* __restrict__ b, const float* __restrict__ sums,
-                                                                    float* __restrict__ stats, int C, long long T, float inv_count,
+                                                                    float* __restrict__ stats, int C, long long T, int R, float inv_count,
                                                                     float eps, int act, int shifted, const StatExchange xc) {
   using P = ClApply<MODE>;
   const int V = C >> 3;
-  const int R = (static_cast<int>(blockDim.x) - 32) / V;
   const int v = threadIdx.x % V, r = threadIdx.x / V;
   const int bidx = blockIdx.y;
   extern __shared__ __align__(16) uint4 cl_ring[];
-  // [C][2] merged sums of this sample (exchange mode only), behind the ring
-  float* const sh_sum = reinterpret_cast<float*>(cl_ring + CL_BARRIERS / 16 + P::DEPTH * P::LAPS * P::TENSORS * R * V);
+  // [C][2] merged sums of this sample (exchange mode only), in front of the ring
+  float* const sh_sum = reinterpret_cast<float*>(cl_ring + CL_BARRIERS / 16);
+  const int ring = cl_ring_offset(C, xc.npeers > 0);
   cl_init<P>(cl_ring);
   chain_begin(xc.npeers == 0, x, dy, w, b, sums, stats);
   if (xc.npeers > 0) {
@@ -706,7 +696,8 @@ __global__ void __launch_bounds__(ClApply<MODE>::THREADS + 32, 1) inorm_cl_apply
     return f2_bf16x8(f);
   };
   // From the end: the last rows that the sums' pass has read are still in L2
-  cl_rows<P, true>(cl_ring, x + base, MODE == 1 ? dy + base : nullptr, V, r, R, T, xc.err, [&](long long t, const uint4& xr, const uint4& gr) { ov[t * V] = transform(xr, gr); });
+  cl_rows<P, true>(cl_ring, ring, x + base, MODE == 1 ? dy + base : nullptr, V, r, R, T, xc.err,
+                   [&](long long t, const uint4& xr, const uint4& gr) { ov[t * V] = transform(xr, gr); });
   if (xc.npeers > 0) {
     // the last CTA tells the peers that this rank is done with their sums
     __syncthreads();
@@ -1424,22 +1415,13 @@ cudaError_t inorm_bwd(const __nv_bfloat16* x, const __nv_bfloat16* dy, __nv_bflo
   return cudaGetLastError();
 }
 
-static inline bool cl_ok(int C) { return C % 8 == 0 && C >= 8 && C <= 1024; }
+static inline bool cl_ok(int C) { return C % 8 == 0 && C >= 8 && C <= CL_CHANNELS; }
 namespace {
-// One CTA per SM, all of them at once, and no more than there are stages.  Small fields spread over the SMs by smaller CTAs.
-constexpr int CL_FEWEST = 128;      // threads (2048 x 16, both passes: 28 us, from CTAs of full size 40, with rows in registers 34)
-template <typename P, typename Kernel, typename... Args>
-cudaError_t cl_launch(Kernel* kernel, int C, long long T, int B, size_t fixed, bool peers, cudaStream_t stream, Args... args) {
-  static const cudaError_t allowed = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                          CL_BARRIERS + cl_ring_bytes<P>(P::THREADS) + 2 * 1024 * static_cast<int>(sizeof(float)));
-  if (allowed != cudaSuccess) return allowed;
-  const int V = C / P::CH;
-  const long long most = std::max(1, sm_count() / B);
-  const long long share = (T + P::LAPS * most - 1) / (P::LAPS * most);      // rows of threads that would give every CTA one stage
-  const int R = static_cast<int>(std::min<long long>(P::THREADS / V, std::max<long long>(share, (CL_FEWEST + V - 1) / V)));
-  const long long need = (T + P::LAPS * R - 1) / (P::LAPS * R);
-  const dim3 grid(static_cast<unsigned>(std::min(most, need)), B);
-  return launch_chained(kernel, grid, dim3((V * R + 31) / 32 * 32 + 32), CL_BARRIERS + cl_ring_bytes<P>(V * R) + fixed, stream, 1, !peers, args...);
+template <typename P, typename Kernel>
+cudaError_t cl_allow(Kernel* kernel) {
+  static const cudaError_t allowed =
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, cl_ring_offset(CL_CHANNELS, true) + cl_ring_bytes<P>(P::THREADS));
+  return allowed;
 }
 }  // namespace
 
@@ -1455,9 +1437,15 @@ cudaError_t inorm_cl_sums(const __nv_bfloat16* x, const __nv_bfloat16* dy, const
   memset(&xc, 0, sizeof(xc));
   xc.err = err;
   if (xch) xc = *xch;
-  if (mode == 0)
-    return cl_launch<ClSums<0>>(inorm_cl_sums_kernel<0>, C, T, B, 0, xc.npeers > 0, s, x, dy, w, b, stats, sums, dw, db, C, T, act, shifted, xc);
-  return cl_launch<ClSums<1>>(inorm_cl_sums_kernel<1>, C, T, B, 0, xc.npeers > 0, s, x, dy, w, b, stats, sums, dw, db, C, T, act, 0, xc);
+  auto launch = [&](auto* kernel, auto params) {
+    using P = decltype(params);
+    const cudaError_t allowed = cl_allow<P>(kernel);
+    if (allowed != cudaSuccess) return allowed;
+    const ClGeometry g = cl_geometry<P>(C, T, B, sm_count(), false);
+    return launch_chained(kernel, dim3(g.ctas, B), dim3(g.threads), g.bytes, s, 1, xc.npeers == 0, x, dy, w, b, stats, sums, dw, db, C, T, g.rows, act,
+                          shifted, xc);
+  };
+  return mode == 0 ? launch(inorm_cl_sums_kernel<0>, ClSums<0>()) : launch(inorm_cl_sums_kernel<1>, ClSums<1>());
 }
 
 cudaError_t inorm_cl_apply(const __nv_bfloat16* x, const __nv_bfloat16* dy, __nv_bfloat16* out, const float* w, const float* b,
@@ -1473,10 +1461,15 @@ cudaError_t inorm_cl_apply(const __nv_bfloat16* x, const __nv_bfloat16* dy, __nv
   xc.err = err;
   if (xch) xc = *xch;
   const float inv = static_cast<float>(1.0 / count);
-  const size_t shx = xc.npeers > 0 ? 2 * C * sizeof(float) : 0;
-  if (mode == 0)
-    return cl_launch<ClApply<0>>(inorm_cl_apply_kernel<0>, C, T, B, shx, xc.npeers > 0, s, x, dy, out, w, b, sums, stats, C, T, inv, eps, act, shifted, xc);
-  return cl_launch<ClApply<1>>(inorm_cl_apply_kernel<1>, C, T, B, shx, xc.npeers > 0, s, x, dy, out, w, b, sums, stats, C, T, inv, eps, act, 0, xc);
+  auto launch = [&](auto* kernel, auto params) {
+    using P = decltype(params);
+    const cudaError_t allowed = cl_allow<P>(kernel);
+    if (allowed != cudaSuccess) return allowed;
+    const ClGeometry g = cl_geometry<P>(C, T, B, sm_count(), xc.npeers > 0);
+    return launch_chained(kernel, dim3(g.ctas, B), dim3(g.threads), g.bytes, s, 1, xc.npeers == 0, x, dy, out, w, b, sums, stats, C, T, g.rows, inv, eps,
+                          act, shifted, xc);
+  };
+  return mode == 0 ? launch(inorm_cl_apply_kernel<0>, ClApply<0>()) : launch(inorm_cl_apply_kernel<1>, ClApply<1>());
 }
 
 namespace {

@@ -1,0 +1,53 @@
+// Launch geometry of the channels-last instance norm (fused_ops.cu): plain host code, one place for what the launcher asks for and the kernels
+// address, so that it can be checked for all sizes without a GPU.
+#pragma once
+#include <algorithm>
+
+#ifdef __CUDACC__
+#define MK_HOST_DEVICE __host__ __device__
+#else
+#define MK_HOST_DEVICE
+#endif
+
+namespace mk {
+
+// The four kernels: channels of a thread, most threads that work on rows (whole rows of them are used, one more warp loads), rows per thread in
+// a stage of the ring and stages.  One CTA per SM.  721 x 1440 x 384, us, by (rows, stages): forward sums (1, 8) 147, (2, 5) 139; forward output
+// (1, 8) 274, (2, 5) 285, (2, 3) 260; gradient with GELU (1, 8) 428, (2, 4) 387, (4, 2) 370, by four channels and 992 threads (4, 3) 389.
+// The backward sums wait for the fp32 pipe and the issue slots, not for rows: without a test per row 330 instead of 352, and by four channels of
+// a thread as by eight, but 51 us instead of 61 at 240 x 480.
+struct ClForwardSums { static constexpr int CH = 8, THREADS = 992, LAPS = 2, DEPTH = 5, TENSORS = 1; };
+struct ClForwardApply { static constexpr int CH = 8, THREADS = 992, LAPS = 2, DEPTH = 3, TENSORS = 1; };
+struct ClBackwardSums { static constexpr int CH = 4, THREADS = 992, LAPS = 4, DEPTH = 3, TENSORS = 2; };
+struct ClBackwardApply { static constexpr int CH = 8, THREADS = 608, LAPS = 4, DEPTH = 2, TENSORS = 2; };
+
+constexpr int CL_CHANNELS = 1024;     // most channels
+constexpr int CL_BARRIERS = 128;      // bytes in front of all else
+constexpr int CL_FEWEST = 128;        // threads (2048 x 16, both passes: 28 us, from CTAs of full size 40, with rows in registers 34)
+
+// Shared memory: barriers, the merged sums of one image ([C][2] fp32, where the statistics cross devices), the ring.  The ring comes last: what
+// stands in front of it does not depend on the rows of threads.
+MK_HOST_DEVICE constexpr int cl_ring_offset(int C, bool merged) { return CL_BARRIERS + (merged ? 8 * C : 0); }
+template <typename P>
+MK_HOST_DEVICE constexpr int cl_ring_bytes(int threads) { return P::DEPTH * P::LAPS * P::TENSORS * 2 * P::CH * threads; }
+// the partial sums of all rows of threads (16 bytes for two channels) take the ring's place
+template <typename P>
+MK_HOST_DEVICE constexpr bool cl_sums_fit() { return P::DEPTH * P::LAPS * P::TENSORS * 2 >= 8; }
+
+// Rows of threads (R: the kernels are told, they cannot derive it from a block of whole warps), threads of a CTA, CTAs per image, bytes of
+// shared memory
+struct ClGeometry {
+  int rows, threads, ctas, bytes;
+};
+// One CTA per SM, all of them at once, and no more than there are stages.  Small fields spread over the SMs by smaller CTAs.
+template <typename P>
+ClGeometry cl_geometry(int C, long long T, int B, int sms, bool merged) {
+  const int V = C / P::CH;
+  const long long most = std::max(1, sms / B);
+  const long long share = (T + P::LAPS * most - 1) / (P::LAPS * most);      // rows of threads that would give every CTA one stage
+  const int R = static_cast<int>(std::min<long long>(P::THREADS / V, std::max<long long>(share, (CL_FEWEST + V - 1) / V)));
+  const long long need = (T + P::LAPS * R - 1) / (P::LAPS * R);
+  return {R, (V * R + 31) / 32 * 32 + 32, static_cast<int>(std::min(most, need)), cl_ring_offset(C, merged) + cl_ring_bytes<P>(V * R)};
+}
+
+}  // namespace mk

@@ -313,7 +313,7 @@ def case_fused_repeat():
     _ext.check_device_errors(dev)
 
 
-def case_peer_instance_norm():
+def case_peer_instance_norm(B=2, C=64, H=45, W=64):
     """Spatially sharded instance norm whose statistics cross the ranks inside the kernels (peer memory) == serial op;
     forward (with fused GELU), input and affine gradients; used twice so that the handshake counters carry over."""
     from makani_b200.ops import _ext, norm as norm_ops
@@ -321,7 +321,6 @@ def case_peer_instance_norm():
     assert os.environ.get("MK_DEVICE") == "cuda"
     dev = torch.device("cuda", comm.get_local_rank())
     torch.manual_seed(11)
-    B, C, H, W = 2, 64, 45, 64
     x = (torch.randn(B, C, H, W) * 2.0 + 0.5).to(dev, torch.bfloat16).contiguous(memory_format=torch.channels_last)
     g = torch.randn(B, C, H, W).to(dev, torch.bfloat16).contiguous(memory_format=torch.channels_last)
     mod = DistributedInstanceNorm2d(C, eps=1e-6, affine=True).to(dev)
@@ -349,6 +348,13 @@ def case_peer_instance_norm():
         dist.all_reduce(dw, group=comm.get_group("spatial"))
         dist.all_reduce(db, group=comm.get_group("spatial"))
         assert _rel(dw, wr.grad) < 3e-2 and _rel(db, br.grad) < 3e-2, (_rel(dw, wr.grad), _rel(db, br.grad))
+
+
+def case_peer_instance_norm_widths():
+    """The same where the rows of threads of a CTA fill no whole warps."""
+    for shape in ((1, 24, 20, 16), (1, 64, 180, 360), (2, 72, 96, 140), (1, 96, 60, 60), (1, 128, 44, 164), (1, 192, 50, 72)):
+        case_peer_instance_norm(*shape)
+
 
 def case_peer_allreduce():
     """In-kernel peer-memory all-reduce == NCCL all-reduce: fp32 and bf16, sizes that are not multiples of the vector

@@ -1033,3 +1033,84 @@ def test_triangular_rows_on_one_pair(l, m, h, n):
     ref = torch.einsum("mlh,mhn->mln", table[..., :h].double(), x.double())
     assert _rel(d, ref) < BF16 and bool((d[~keep.expand_as(d)] == 0).all())
     _ext.check_device_errors(dev)
+
+
+@pytest.mark.parametrize("b,c,t", [(1, 24, 100), (1, 48, 100), (2, 72, 3360), (1, 64, 32400), (1, 96, 1800), (1, 128, 3601), (3, 192, 700), (1, 16, 18000),
+                                   (1, 1024, 333), (2, 384, 6720)])
+def test_instance_norm_with_statistics_of_two_devices(b, c, t):
+    """The exchange form of the four kernels on one of two halves of a field, at rows of threads that fill no whole warps (and some that do): the other
+    half's sums are in place and all flags set before the launches, so that nothing waits.  Against float64 of the whole field."""
+    dev = _dev()
+    g = torch.Generator(dev).manual_seed(c + t)
+    ext, eps, n = _ext.require(), 1e-2, float(2 * t)
+    x, dy = ((torch.randn(2, b, t, c, device=dev, generator=g) + 0.5).bfloat16() for _ in range(2))
+    wt, bi = (torch.randn(c, device=dev, generator=g) for _ in range(2))
+    # flags[8] that are waited for | counters of the waits | launches done | signals[8]
+    ctrl = torch.zeros(32, dtype=torch.int32, device=dev)
+    ctrl[:8] = 1000
+    at = ctrl.data_ptr()
+    bumped, done, signals = at + 32, at + 36, at + 64
+    sync = [1, 1, done, at, bumped, 0, bumped, 2, 0, 0, 0, 0, 0, 2, signals, signals + 4] + [0] * 6 + [0] * 9
+    segments, copy = torch.zeros(2, b, c, 2, device=dev), torch.zeros(b, c, 2, device=dev)
+    xd, wd, bd = x.double().requires_grad_(), wt.double().requires_grad_(), bi.double().requires_grad_()
+    mean = xd.mean((0, 2), keepdim=True)
+    rstd = 1.0 / torch.sqrt((xd - mean).square().mean((0, 2), keepdim=True) + eps)
+    for act in (0, 1):
+        yd = (xd - mean) * rstd * wd + bd
+        yd = torch.nn.functional.gelu(yd) if act else yd
+        (want,) = torch.autograd.grad(yd, xd, dy.double(), retain_graph=True)
+        stats = torch.empty(b, c, 2, device=dev)
+
+        def other(a0, a1):
+            """The second device's sums"""
+            segments[1] = torch.stack([a0[1], a1[1]], -1).float()
+
+        def both(run):
+            segments[0] = copy[:] = float("nan")
+            sums = torch.zeros(b, c, 2, device=dev)
+            run(sums)
+            assert torch.equal(sums, segments[0]) and torch.equal(sums, copy)
+
+        dsts, srcs = [segments[0].data_ptr(), copy.data_ptr()], [segments[0].data_ptr(), segments[1].data_ptr()]
+        other(x.double().sum(2), x.double().square().sum(2))
+        both(lambda sums: ext.inorm_cl_sums(x[0], None, None, None, None, sums, None, None, b, c, 0, 0, sync, dsts))
+        y, dx = torch.full_like(x[0], float("nan")), torch.full_like(x[0], float("nan"))
+        ext.inorm_cl_apply(x[0], None, y, wt, bi, segments[0], stats, b, c, n, eps, act, 0, sync, srcs)
+        assert (stats[..., 0].double() - mean[0, :, 0]).abs().max() < 1e-5
+        assert (stats[..., 1].double() / rstd[0, :, 0] - 1.0).abs().max() < 1e-5
+        # half a unit of 2^-8 per value; GELU is 5.5e-5 off, its derivative 2e-4 times (1 + |x|), at outputs of order 1
+        assert (y.double() - yd[0]).norm() < (2.0 ** -8 + (1e-4 if act else 0.0)) * yd[0].norm() + 1e-6
+        pre = ((xd - mean) * rstd * wd + bd).detach().requires_grad_()
+        (slope,) = torch.autograd.grad(torch.nn.functional.gelu(pre).sum() if act else pre.sum(), pre)
+        gd = (dy.double() * slope)
+        other(gd.sum(2), (gd * (xd - mean) * rstd).sum(2).detach())
+        dw, db = torch.zeros(c, device=dev), torch.zeros(c, device=dev)
+        both(lambda sums: ext.inorm_cl_sums(x[0], dy[0], wt, bi, stats, sums, dw, db, b, c, act, 1, sync, dsts))
+        ext.inorm_cl_apply(x[0], dy[0], dx, wt, bi, segments[0], stats, b, c, n, 0.0, act, 1, sync, srcs)
+        scale = dy.double().norm() * (rstd * wd).abs().max()      # dx is a difference of terms of this size
+        assert (dx.double() - want[0]).norm() < 2.0 ** -8 * want[0].norm() + (2e-3 if act else 1e-5) * scale
+        for got, term in ((db, gd[0]), (dw, (gd * (xd - mean) * rstd)[0].detach())):
+            assert (got.double() - term.sum((0, 1))).norm() <= (2e-3 if act else 1e-5) * term.abs().sum((0, 1)).norm()
+    assert int(ctrl[8]) == 8 and int(ctrl[9]) == 0 and ctrl[16:18].tolist() == [8, 8]      # every launch counted and signalled once
+    _ext.check_device_errors(dev)
+
+
+@pytest.mark.parametrize("b,c,h,w", [(1, 24, 10, 10), (8, 72, 80, 84), (1, 64, 180, 180), (2, 96, 30, 60), (8, 128, 1, 3601), (1, 192, 100, 181), (1, 8, 97, 192)])
+def test_instance_norm_rows_that_fill_no_whole_warps(b, c, h, w):
+    dev = _dev()
+    g = torch.Generator(dev).manual_seed(c + h)
+    x, dy = (torch.randn(b, h, w, c, device=dev, generator=g).bfloat16().permute(0, 3, 1, 2) for _ in range(2))
+    wt, bi = (torch.randn(c, device=dev, generator=g) for _ in range(2))
+    ext = _ext.require()
+    y, stats, wf, bf = ext.norm_forward(x, wt, bi, 1e-2, 0, float(h * w))
+    dx, dw, db = ext.norm_backward(x, dy, wf, bf, stats, True, 0, float(h * w))
+    xd, wd, bd = x.double().requires_grad_(), wt.double().requires_grad_(), bi.double().requires_grad_()
+    yd = torch.nn.functional.instance_norm(xd, None, None, wd, bd, True, 0.0, 1e-2)
+    want = torch.autograd.grad(yd, [xd, wd, bd], dy.double())
+    # half a unit of 2^-8 per value, sums of fp32
+    assert (y.double() - yd).norm() < 2.0 ** -8 * yd.norm()
+    assert (dx.double() - want[0]).norm() < 2.0 ** -8 * want[0].norm() + 1e-5 * dy.double().norm()
+    xh = torch.nn.functional.instance_norm(x.double(), eps=1e-2)
+    for got, ref, term in ((dw, want[1], dy.double() * xh), (db, want[2], dy.double())):
+        assert (got.double() - ref).norm() <= 1e-5 * term.abs().sum((0, 2, 3)).norm()
+    _ext.check_device_errors(dev)

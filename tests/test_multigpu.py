@@ -31,6 +31,12 @@ def test_peer_memory_instance_norm(sizes, world):
     _launch("peer_instance_norm", sizes, world, cuda=True)
 
 
+@pytest.mark.parametrize("sizes,world", [((2, 1, 1, 1), 2), ((2, 2, 1, 1), 4)])
+def test_peer_memory_instance_norm_widths(sizes, world):
+    _need(world)
+    _launch("peer_instance_norm_widths", sizes, world, cuda=True)
+
+
 @pytest.mark.parametrize("sizes,world", [((1, 1, 2, 1), 2), ((1, 1, 1, 2), 2), ((1, 1, 2, 2), 4)])
 def test_fused_channel_parallel_matmul(sizes, world):
     _need(world)
