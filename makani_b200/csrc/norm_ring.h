@@ -16,10 +16,11 @@ namespace mk {
 // (1, 8) 274, (2, 5) 285, (2, 3) 260; gradient with GELU (1, 8) 428, (2, 4) 387, (4, 2) 370, by four channels and 992 threads (4, 3) 389.
 // The backward sums wait for the fp32 pipe and the issue slots, not for rows: without a test per row 330 instead of 352, and by four channels of
 // a thread as by eight, but 51 us instead of 61 at 240 x 480.
-struct ClForwardSums { static constexpr int CH = 8, THREADS = 992, LAPS = 2, DEPTH = 5, TENSORS = 1; };
-struct ClForwardApply { static constexpr int CH = 8, THREADS = 992, LAPS = 2, DEPTH = 3, TENSORS = 1; };
-struct ClBackwardSums { static constexpr int CH = 4, THREADS = 992, LAPS = 4, DEPTH = 3, TENSORS = 2; };
-struct ClBackwardApply { static constexpr int CH = 8, THREADS = 608, LAPS = 4, DEPTH = 2, TENSORS = 2; };
+// START: stages that take as long as the start and the end of a CTA.
+struct ClForwardSums { static constexpr int CH = 8, THREADS = 992, LAPS = 2, DEPTH = 5, TENSORS = 1, START = 8; };
+struct ClForwardApply { static constexpr int CH = 8, THREADS = 992, LAPS = 2, DEPTH = 3, TENSORS = 1, START = 4; };
+struct ClBackwardSums { static constexpr int CH = 4, THREADS = 992, LAPS = 4, DEPTH = 3, TENSORS = 2, START = 3; };
+struct ClBackwardApply { static constexpr int CH = 8, THREADS = 608, LAPS = 4, DEPTH = 2, TENSORS = 2, START = 4; };
 
 constexpr int CL_CHANNELS = 1024;     // most channels
 constexpr int CL_BARRIERS = 128;      // bytes in front of all else
@@ -39,15 +40,34 @@ MK_HOST_DEVICE constexpr bool cl_sums_fit() { return P::DEPTH * P::LAPS * P::TEN
 struct ClGeometry {
   int rows, threads, ctas, bytes;
 };
-// One CTA per SM, all of them at once, and no more than there are stages.  Small fields spread over the SMs by smaller CTAs.
+// CTAs of an image.  One CTA per SM; all of them at once, and no more than there are stages, unless that leaves SMs idle (75 images, or
+// 149): further waves of smaller shares are taken where stages and starts together come out a tenth shorter.
+template <typename P>
+int cl_ctas(long long stages, int B, int sms) {
+  const int most = std::max(1, sms / B);
+  int best = static_cast<int>(std::min<long long>(most, stages));
+  if (10ll * most * B >= 9ll * sms && B <= sms) return best;
+  auto cost = [&](long long n) { return (B * n + sms - 1) / sms * ((stages + n - 1) / n + P::START); };
+  long long least = cost(best) * 9 / 10;
+  for (int n = best + 1; n <= std::min<long long>(stages, most + 16); ++n)
+    if (cost(n) < least) {
+      best = n;
+      least = cost(n);
+    }
+  return best;
+}
+// Small fields spread over the SMs by smaller CTAs.  With more images than SMs CTAs have half the size, so that one begins while the other ends.  Both
+// passes with GELU, us, one CTA of full size per image or more while they fit at once / now: 90 x 180 x 384, 75 images 2058 / 1378;
+// 149 4301 / 2523; 32 x 64 x 64, 149 images 137 / 123, 300 205 / 185; 50 images of 90 x 180 x 384 1077 / 934.
 template <typename P>
 ClGeometry cl_geometry(int C, long long T, int B, int sms, bool merged) {
   const int V = C / P::CH;
   const long long most = std::max(1, sms / B);
   const long long share = (T + P::LAPS * most - 1) / (P::LAPS * most);      // rows of threads that would give every CTA one stage
-  const int R = static_cast<int>(std::min<long long>(P::THREADS / V, std::max<long long>(share, (CL_FEWEST + V - 1) / V)));
-  const long long need = (T + P::LAPS * R - 1) / (P::LAPS * R);
-  return {R, (V * R + 31) / 32 * 32 + 32, static_cast<int>(std::min(most, need)), cl_ring_offset(C, merged) + cl_ring_bytes<P>(V * R)};
+  const int threads = B > sms ? (P::THREADS + 32) / 2 - 32 : P::THREADS;
+  const int R = static_cast<int>(std::min<long long>(threads / V, std::max<long long>(share, (CL_FEWEST + V - 1) / V)));
+  const long long stages = (T + P::LAPS * R - 1) / (P::LAPS * R);
+  return {R, (V * R + 31) / 32 * 32 + 32, cl_ctas<P>(stages, B, sms), cl_ring_offset(C, merged) + cl_ring_bytes<P>(V * R)};
 }
 
 }  // namespace mk

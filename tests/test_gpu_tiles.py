@@ -1035,7 +1035,7 @@ def test_triangular_rows_on_one_pair(l, m, h, n):
     _ext.check_device_errors(dev)
 
 
-@pytest.mark.parametrize("b,c,t", [(1, 24, 100), (1, 48, 100), (2, 72, 3360), (1, 64, 32400), (1, 96, 1800), (1, 128, 3601), (3, 192, 700), (1, 16, 18000),
+@pytest.mark.parametrize("b,c,t", [(75, 256, 3000), (1, 24, 100), (1, 48, 100), (2, 72, 3360), (1, 64, 32400), (1, 96, 1800), (1, 128, 3601), (3, 192, 700), (1, 16, 18000),
                                    (1, 1024, 333), (2, 384, 6720)])
 def test_instance_norm_with_statistics_of_two_devices(b, c, t):
     """The exchange form of the four kernels on one of two halves of a field, at rows of threads that fill no whole warps (and some that do): the other
@@ -1095,8 +1095,10 @@ def test_instance_norm_with_statistics_of_two_devices(b, c, t):
     _ext.check_device_errors(dev)
 
 
-@pytest.mark.parametrize("b,c,h,w", [(1, 24, 10, 10), (8, 72, 80, 84), (1, 64, 180, 180), (2, 96, 30, 60), (8, 128, 1, 3601), (1, 192, 100, 181), (1, 8, 97, 192)])
+@pytest.mark.parametrize("b,c,h,w", [(1, 24, 10, 10), (8, 72, 80, 84), (1, 64, 180, 180), (2, 96, 30, 60), (8, 128, 1, 3601), (1, 192, 100, 181), (1, 8, 97, 192),
+                                     (75, 384, 50, 60), (149, 128, 60, 128)])
 def test_instance_norm_rows_that_fill_no_whole_warps(b, c, h, w):
+    """The last two: shares of an image in several waves of CTAs."""
     dev = _dev()
     g = torch.Generator(dev).manual_seed(c + h)
     x, dy = (torch.randn(b, h, w, c, device=dev, generator=g).bfloat16().permute(0, 3, 1, 2) for _ in range(2))

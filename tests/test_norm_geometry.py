@@ -1,5 +1,5 @@
 """Launch geometry of the channels-last instance norm (csrc/norm_ring.h), without a GPU: every byte that the kernels address lies in the shared
-memory that their launch asks for, over all channel counts, field sizes and batches, alone and with statistics that cross devices."""
+memory that their launch asks for, over all channel counts, field sizes and batches, alone and with statistics that cross devices; and the CTAs of a launch share its work out evenly."""
 import os
 import shutil
 import subprocess
@@ -35,7 +35,22 @@ void check(const char* name, int C, long long T, int B, int sms, bool merged, bo
     std::printf("%s C %d T %lld B %d SMs %d merged %d: R %lld, %d threads, %d CTAs, %lld of %d bytes\n", name, C, T, B, sms, merged, R, g.threads, g.ctas,
                 end, g.bytes);
 }
+// Fields of many stages, any batch: the stages of the SMs that work longest, against an even share
+template <typename P>
+void balance(const char* name, int C, long long T, int B, int sms) {
+  const ClGeometry g = cl_geometry<P>(C, T, B, sms, false);
+  const long long stages = (T + P::LAPS * g.rows - 1) / (P::LAPS * g.rows), waves = (1ll * g.ctas * B + sms - 1) / sms;
+  const double over = static_cast<double>(waves * ((stages + g.ctas - 1) / g.ctas)) * sms / (static_cast<double>(B) * stages);
+  ++checked;
+  if (over > 1.25 && ++failed <= 10) std::printf("%s C %d T %lld B %d SMs %d: %d CTAs, %.2f of an even share\n", name, C, T, B, sms, g.ctas, over);
+}
 int main() {
+  for (int B = 1; B <= 600; ++B) {
+    balance<ClForwardSums>("forward sums", 384, 64800, B, 148);
+    balance<ClForwardApply>("forward output", 384, 64800, B, 148);
+    balance<ClBackwardSums>("backward sums", 384, 64800, B, 148);
+    balance<ClBackwardApply>("backward output", 384, 64800, B, 148);
+  }
   const long long fields[] = {1, 2, 3, 7, 31, 50, 64, 100, 255, 300, 719, 720, 1024, 1800, 2048, 2049, 3601, 5000, 6720, 8191, 16200, 18624, 20000, 32400, 57600, 64800, 115200, 259920, 1038240, 4147200, 50000000000};
   const int batches[] = {1, 2, 3, 4, 5, 7, 8, 16, 37, 50, 74, 75, 147, 148, 149, 300, 4096}, sm[] = {148, 132, 16};
   for (int sms : sm)
@@ -61,7 +76,7 @@ int main() {
 
 
 @pytest.mark.skipif(shutil.which("g++") is None, reason="no host compiler")
-def test_no_launch_addresses_more_shared_memory_than_it_asks_for(tmp_path):
+def test_launches_of_the_instance_norm(tmp_path):
     src, exe = tmp_path / "geometry.cpp", tmp_path / "geometry"
     src.write_text(PROGRAM)
     subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", "-Werror", "-I", CSRC, str(src), "-o", str(exe)], check=True)
