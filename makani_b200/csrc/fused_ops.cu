@@ -1419,9 +1419,8 @@ static inline bool cl_ok(int C) { return C % 8 == 0 && C >= 8 && C <= CL_CHANNEL
 namespace {
 template <typename P, typename Kernel>
 cudaError_t cl_allow(Kernel* kernel) {
-  static const cudaError_t allowed =
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, cl_ring_offset(CL_CHANNELS, true) + cl_ring_bytes<P>(P::THREADS));
-  return allowed;
+  static std::atomic<uint64_t> devices;      // (each of the kernels has parameters of its own)
+  return allow_shared_memory(devices, reinterpret_cast<const void*>(kernel), cl_ring_offset(CL_CHANNELS, true) + cl_ring_bytes<P>(P::THREADS));
 }
 }  // namespace
 

@@ -1391,12 +1391,9 @@ cudaError_t launch_t(const CUtensorMap& ma, const BMaps& mb, const CUtensorMap& 
   kp.stages = stages;
   const int smem = stages * STAGE + e_bytes + FIXED;
   const int threads = 32 * (3 + epi_warps(BN, EPI) + (kp.rowsum ? SUM_WARPS : (kp.e_tma ? 1 : 0)));
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_kernel<BN, EB, EPI, CG, RAGGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
+  static std::atomic<uint64_t> devices;
+  const cudaError_t allowed = allow_shared_memory(devices, reinterpret_cast<const void*>(&gemm_kernel<BN, EB, EPI, CG, RAGGED>), SMEM_LIMIT);
+  if (allowed != cudaSuccess) return allowed;
   const int num_sms = sm_count();
   const long long slabs = static_cast<long long>(kp.k_per_split) * (kp.cplx ? 2 : 1) * EB / 128;
   // tile order (MAKANI_B200_TILE_ORDER=m|n forces one order for A/B timing)

@@ -13,11 +13,26 @@
 // 99 -> 134 us; launched in the ordinary way).
 #pragma once
 #include <cuda_runtime.h>
+#include <stdint.h>
 #include <string.h>
 
+#include <atomic>
 #include <utility>
 
 namespace mk {
+
+// Lets `kernel` take up to `bytes` of dynamic shared memory on the current device.  The attribute belongs to kernel and device: `devices` (one per
+// kernel) holds those that have it, and none that refused.
+inline cudaError_t allow_shared_memory(std::atomic<uint64_t>& devices, const void* kernel, int bytes) {
+  int device = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  const uint64_t bit = device < 64 ? uint64_t{1} << device : 0;
+  if (devices.load(std::memory_order_relaxed) & bit) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess) devices.fetch_or(bit, std::memory_order_relaxed);
+  return e;
+}
 
 #ifdef __CUDACC__
 // `next` false: the next kernel does not begin before this one is complete.  `p`: pointers whose loads the compiler may take for constant during the kernel (const __restrict__) and could move in front of the wait; they

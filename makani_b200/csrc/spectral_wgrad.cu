@@ -229,7 +229,8 @@ cudaError_t spectral_wgrad(const __nv_bfloat16* dt, const __nv_bfloat16* t2, flo
       (reinterpret_cast<uintptr_t>(dw) & 31))
     return cudaErrorInvalidValue;
   bind_context(stream);
-  static const cudaError_t allowed = cudaFuncSetAttribute(spectral_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+  static std::atomic<uint64_t> devices;
+  const cudaError_t allowed = allow_shared_memory(devices, reinterpret_cast<const void*>(&spectral_wgrad_kernel), SMEM);
   if (allowed != cudaSuccess) return allowed;
   auto operand = [&](const __nv_bfloat16* t, int c) {
     GemmOperand op;
