@@ -7,10 +7,13 @@
 // devices are launched in the ordinary way, and the next one begins when they are complete: blocks that wait behind a wait would hold
 // shared memory that kernels of other streams may need.
 //
-// What it saves is the time between two launches (some 2 us) and the set-up: the AFNO filter of 90 x 180 tokens, 17 products of 10 - 20 us,
-// 256 -> 236 us a training pass, the token MLP (16200 x 768 -> 3072) 525 -> 511, the MLP of 240 x 480 tokens 600 -> 590.  For grids of one
-// wave: a block that begins later pays for the wait without need (the re-layout of the spectral weights, 18432 blocks, 70 -> 90 and
-// 99 -> 134 us; launched in the ordinary way).
+// What it saves is the time between two launches (some 2 us) and the set-up: the AFNO filter of 90 x 180 tokens, 14 products of 6 - 20 us, 256 -> 236 us
+// a training pass, the token MLP (16200 x 768 -> 3072) 525 -> 511, the MLP of 240 x 480 tokens 600 -> 590.  Kernels of several waves gain as well
+// (cast of 4096 x 4096 weights between two products, seven waves, 31.2 -> 30.9 us; weights of 8 x 512 AFNO channels, 3.5 waves, 29.7 -> 29.2).
+// Launched in the ordinary way:
+// - what spreads few blocks evenly, several to an SM: begun early these crowd on the SMs that are free (column sums, 127 us become 160);
+// - the re-layout of the spectral weights (18432 blocks, 70 -> 90 and 99 -> 134 us);
+// - long products (CHAINED_SLABS in gemm_tcgen05.cu).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>

@@ -1116,3 +1116,20 @@ def test_instance_norm_rows_that_fill_no_whole_warps(b, c, h, w):
     for got, ref, term in ((dw, want[1], dy.double() * xh), (db, want[2], dy.double())):
         assert (got.double() - ref).norm() <= 1e-5 * term.abs().sum((0, 2, 3)).norm()
     _ext.check_device_errors(dev)
+
+
+@pytest.mark.parametrize("co,ci", [(8, 8), (600, 1008), (1544, 1576), (2056, 1288)])
+def test_gradients_are_added_to_zero_at_any_size(co, ci):
+    """Cleared by blocks for four per SM (up to some 10 MB) and by four vectors of a thread: weight gradients that start in memory full of NaN."""
+    dev = _dev()
+    g = torch.Generator(dev).manual_seed(co)
+    ext = _ext.require()
+    x, dy = (torch.randn(2, 8, 16, c, device=dev, generator=g).bfloat16().permute(0, 3, 1, 2) for c in (ci, co))
+    wq = torch.randn(co, ci, device=dev, generator=g).bfloat16()
+    held = torch.full((co, ci), float("nan"), device=dev)
+    del held      # the gradient takes its place
+    _, dw, db = ext.conv_backward(dy, x, wq, ci, False, True, True)
+    rows = lambda t: t.double().permute(1, 0, 2, 3).flatten(1)  # noqa: E731
+    assert (dw.double() - rows(dy) @ rows(x).t()).norm() <= 1e-6 * (rows(dy) @ rows(x).t()).norm()
+    assert (db.double() - rows(dy).sum(1)).norm() <= 1e-6 * rows(dy).abs().sum(1).norm()
+    _ext.check_device_errors(dev)
