@@ -1368,7 +1368,10 @@ long long mixed_grid(long long grid, const KParams& kp, int bm, int bn) {
 // than the gap they save.  384 -> 384 channels over 721 x 1440 tokens (660 slabs) 342 us in the ordinary way, 354 chained; the decoder's training
 // pass, with the gradients of its weights (330 slabs and more) chained 1984, without 1969.  The products of 115200 tokens or 16200 x 768
 // -> 3072 have 110 to 150: 596 -> 582 and 518 -> 503 chained.
-constexpr long long CHAINED_SLABS = 256;
+// Products of several samples that add into one output lose more, from some 64 slabs on (a pass of 4 samples in the ordinary way / chained, us: 304 x 544
+// over 37888 tokens each, 144 slabs, 78 / 85; 272 x 888 over 22848, 116 slabs, 92 / 99; 264 x 848 over 17728, 90 slabs, 61 / 67; 296 x 208 over
+// 29184, 37 slabs, 39 / 39); of one sample they are even or gain (768 x 384 over 115200, 146 slabs, 73 / 71).
+constexpr long long CHAINED_SLABS = 256, CHAINED_SLABS_OF_SAMPLES = 64;
 
 template <int BN, int EB, int EPI, int CG, bool RAGGED = false>
 cudaError_t launch_t(const CUtensorMap& ma, const BMaps& mb, const CUtensorMap& me, const CUtensorMap& md,
@@ -1396,6 +1399,8 @@ cudaError_t launch_t(const CUtensorMap& ma, const BMaps& mb, const CUtensorMap& 
   if (allowed != cudaSuccess) return allowed;
   const int num_sms = sm_count();
   const long long slabs = static_cast<long long>(kp.k_per_split) * (kp.cplx ? 2 : 1) * EB / 128;
+  const bool samples = kp.accumulate && ((kp.zlo_n > 1 && kp.d_zlo == 0) || (kp.zhi_n > 1 && kp.d_zhi == 0));
+  const long long chained_slabs = samples ? CHAINED_SLABS_OF_SAMPLES : CHAINED_SLABS;
   // tile order (MAKANI_B200_TILE_ORDER=m|n forces one order for A/B timing)
   static const int forced_order = [] {
     const char* e = getenv("MAKANI_B200_TILE_ORDER");
@@ -1408,13 +1413,13 @@ cudaError_t launch_t(const CUtensorMap& ma, const BMaps& mb, const CUtensorMap& 
     if (clusters < 1) clusters = 1;
     if constexpr (EPI != 0 && EPI != 5) clusters = mixed_grid(clusters, kp, 2 * BM, BN);
     return launch_chained(gemm_kernel<BN, EB, EPI, CG, RAGGED>, dim3(static_cast<unsigned>(2 * clusters)), dim3(threads), smem, stream, 2,
-                          kp.total_tiles * slabs <= CHAINED_SLABS * clusters, ma, mb,
+                          kp.total_tiles * slabs <= chained_slabs * clusters, ma, mb,
                           me, md, mp, mdx, kp);
   }
   long long grid = kp.total_tiles < static_cast<uint32_t>(num_sms) ? kp.total_tiles : num_sms;
   if (grid < 1) grid = 1;
   if constexpr (EPI != 0 && EPI != 5) grid = mixed_grid(grid, kp, BM, BN);
-  const bool alone = kp.total_tiles * slabs <= CHAINED_SLABS * grid && kp.nseg <= 1 && kp.ndx == 0 && kp.sync.nwait == 0 && kp.sync.nsig == 0 && kp.sync.done_ctr == nullptr;
+  const bool alone = kp.total_tiles * slabs <= chained_slabs * grid && kp.nseg <= 1 && kp.ndx == 0 && kp.sync.nwait == 0 && kp.sync.nsig == 0 && kp.sync.done_ctr == nullptr;
   return launch_chained(gemm_kernel<BN, EB, EPI, CG, RAGGED>, dim3(static_cast<unsigned>(grid)), dim3(threads), smem, stream, 1, alone, ma, mb, me, md,
                         mp, mdx, kp);
 }
