@@ -24,6 +24,10 @@ struct ClBackwardApply { static constexpr int CH = 8, THREADS = 608, LAPS = 4, D
 
 constexpr int CL_CHANNELS = 1024;     // most channels
 constexpr int CL_BARRIERS = 128;      // bytes in front of all else
+// Bytes of which an SM has no second share, for CTAs of up to 512 threads (of more, two find no registers).  Where a launch of one CTA per SM begins while the
+// launch before it ends, these would crowd on the SMs that are free first.  Forward with GELU behind a product, us, without / with: 384 channels, 2048
+// tokens 24.3 / 20.9; 256, 4 images of 1024 24.2 / 19.7; 64, 4 of 4096 16.7 / 15.3; 64, 512 tokens 12.6 / 13.0.
+constexpr int CL_ALONE = 116 * 1024;
 constexpr int CL_FEWEST = 128;        // threads (2048 x 16, both passes: 28 us, from CTAs of full size 40, with rows in registers 34)
 
 // Shared memory: barriers, the merged sums of one image ([C][2] fp32, where the statistics cross devices), the ring.  The ring comes last: what
@@ -34,6 +38,10 @@ MK_HOST_DEVICE constexpr int cl_ring_bytes(int threads) { return P::DEPTH * P::L
 // the partial sums of all rows of threads (16 bytes for two channels) take the ring's place
 template <typename P>
 MK_HOST_DEVICE constexpr bool cl_sums_fit() { return P::DEPTH * P::LAPS * P::TENSORS * 2 >= 8; }
+
+// most bytes of a launch
+template <typename P>
+constexpr int cl_most_bytes() { return std::max(CL_ALONE, cl_ring_offset(CL_CHANNELS, true) + cl_ring_bytes<P>(P::THREADS)); }
 
 // Rows of threads (R: the kernels are told, they cannot derive it from a block of whole warps), threads of a CTA, CTAs per image, bytes of
 // shared memory
@@ -60,14 +68,16 @@ int cl_ctas(long long stages, int B, int sms) {
 // passes with GELU, us, one CTA of full size per image or more while they fit at once / now: 90 x 180 x 384, 75 images 2058 / 1378;
 // 149 4301 / 2523; 32 x 64 x 64, 149 images 137 / 123, 300 205 / 185; 50 images of 90 x 180 x 384 1077 / 934.
 template <typename P>
-ClGeometry cl_geometry(int C, long long T, int B, int sms, bool merged) {
+ClGeometry cl_geometry(int C, long long T, int B, int sms, bool merged, bool chained) {
   const int V = C / P::CH;
   const long long most = std::max(1, sms / B);
   const long long share = (T + P::LAPS * most - 1) / (P::LAPS * most);      // rows of threads that would give every CTA one stage
   const int threads = B > sms ? (P::THREADS + 32) / 2 - 32 : P::THREADS;
   const int R = static_cast<int>(std::min<long long>(threads / V, std::max<long long>(share, (CL_FEWEST + V - 1) / V)));
   const long long stages = (T + P::LAPS * R - 1) / (P::LAPS * R);
-  return {R, (V * R + 31) / 32 * 32 + 32, cl_ctas<P>(stages, B, sms), cl_ring_offset(C, merged) + cl_ring_bytes<P>(V * R)};
+  const int block = (V * R + 31) / 32 * 32 + 32, ctas = cl_ctas<P>(stages, B, sms), bytes = cl_ring_offset(C, merged) + cl_ring_bytes<P>(V * R);
+  const bool alone = chained && block <= 512 && static_cast<long long>(ctas) * B <= sms;
+  return {R, block, ctas, alone ? std::max(bytes, CL_ALONE) : bytes};
 }
 
 }  // namespace mk

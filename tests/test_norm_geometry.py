@@ -16,8 +16,8 @@ PROGRAM = r"""
 using namespace mk;
 static long long checked = 0, failed = 0;
 template <typename P>
-void check(const char* name, int C, long long T, int B, int sms, bool merged, bool sums) {
-  const ClGeometry g = cl_geometry<P>(C, T, B, sms, merged);
+void check(const char* name, int C, long long T, int B, int sms, bool merged, bool sums, bool chained) {
+  const ClGeometry g = cl_geometry<P>(C, T, B, sms, merged, chained);
   const long long V = C / P::CH, R = g.rows, rows = P::LAPS * R, row = 2ll * C;
   const long long ring = 128 + (merged ? 8ll * C : 0), stages = (T + rows - 1) / rows;
   long long end = ring;
@@ -28,8 +28,10 @@ void check(const char* name, int C, long long T, int B, int sms, bool merged, bo
     }
   if (sums) end = std::max(end, ring + 8 * ((R - 1) * C + C));
   const bool ok = R >= 1 && V * R <= g.threads - 32 && g.threads <= P::THREADS + 32 && g.threads % 32 == 0 && end <= g.bytes && g.bytes <= 232448 &&
-                  ring % 16 == 0 && g.bytes <= cl_ring_offset(CL_CHANNELS, true) + cl_ring_bytes<P>(P::THREADS) && g.ctas >= 1 && g.ctas <= stages &&
-                  16 * P::DEPTH <= 128;
+                  ring % 16 == 0 && g.bytes <= cl_most_bytes<P>() && g.ctas >= 1 && g.ctas <= stages &&
+                  16 * P::DEPTH <= 128 &&
+                  // a chained launch of one wave: 228 KB of an SM, 1 KB of each block, or its 65536 registers (57 and more a thread) have no room for two
+                  (!chained || 1ll * g.ctas * B > sms || 2ll * g.threads * 64 > 65536 || 2 * (g.bytes + 1024) > 228 * 1024);
   ++checked;
   if (!ok && ++failed <= 10)
     std::printf("%s C %d T %lld B %d SMs %d merged %d: R %lld, %d threads, %d CTAs, %lld of %d bytes\n", name, C, T, B, sms, merged, R, g.threads, g.ctas,
@@ -38,7 +40,7 @@ void check(const char* name, int C, long long T, int B, int sms, bool merged, bo
 // Fields of many stages, any batch: the stages of the SMs that work longest, against an even share
 template <typename P>
 void balance(const char* name, int C, long long T, int B, int sms) {
-  const ClGeometry g = cl_geometry<P>(C, T, B, sms, false);
+  const ClGeometry g = cl_geometry<P>(C, T, B, sms, false, true);
   const long long stages = (T + P::LAPS * g.rows - 1) / (P::LAPS * g.rows), waves = (1ll * g.ctas * B + sms - 1) / sms;
   const double over = static_cast<double>(waves * ((stages + g.ctas - 1) / g.ctas)) * sms / (static_cast<double>(B) * stages);
   ++checked;
@@ -57,17 +59,19 @@ int main() {
     for (int B : batches)
       for (int C = 8; C <= 1024; C += 8)
         for (long long T : fields) {
-          check<ClForwardSums>("forward sums", C, T, B, sms, false, true);
-          check<ClBackwardSums>("backward sums", C, T, B, sms, false, true);
+          check<ClForwardSums>("forward sums", C, T, B, sms, false, true, true);
+          check<ClForwardSums>("forward sums", C, T, B, sms, false, true, false);
+          check<ClBackwardSums>("backward sums", C, T, B, sms, false, true, true);
+          check<ClBackwardSums>("backward sums", C, T, B, sms, false, true, false);
           for (int merged = 0; merged < 2; ++merged) {
-            check<ClForwardApply>("forward output", C, T, B, sms, merged, false);
-            check<ClBackwardApply>("backward output", C, T, B, sms, merged, false);
+            check<ClForwardApply>("forward output", C, T, B, sms, merged, false, !merged);
+            check<ClBackwardApply>("backward output", C, T, B, sms, merged, false, !merged);
           }
         }
   for (long long T = 1; T <= 12000; ++T)
     for (int C : {8, 16, 24, 48, 64, 72, 96, 104, 128, 192, 232, 384}) {
-      check<ClForwardApply>("forward output", C, T, 1, 148, true, false);
-      check<ClBackwardApply>("backward output", C, T, 2, 148, true, false);
+      check<ClForwardApply>("forward output", C, T, 1, 148, true, false, false);
+      check<ClBackwardApply>("backward output", C, T, 2, 148, true, false, false);
     }
   std::printf("%lld checked, %lld failed\n", checked, failed);
   return failed != 0;
