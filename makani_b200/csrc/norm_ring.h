@@ -16,11 +16,11 @@ namespace mk {
 // (1, 8) 274, (2, 5) 285, (2, 3) 260; gradient with GELU (1, 8) 428, (2, 4) 387, (4, 2) 370, by four channels and 992 threads (4, 3) 389.
 // The backward sums wait for the fp32 pipe and the issue slots, not for rows: without a test per row 330 instead of 352, and by four channels of
 // a thread as by eight, but 51 us instead of 61 at 240 x 480.
-// START: stages that take as long as the start and the end of a CTA.
-struct ClForwardSums { static constexpr int CH = 8, THREADS = 992, LAPS = 2, DEPTH = 5, TENSORS = 1, START = 8; };
-struct ClForwardApply { static constexpr int CH = 8, THREADS = 992, LAPS = 2, DEPTH = 3, TENSORS = 1, START = 4; };
-struct ClBackwardSums { static constexpr int CH = 4, THREADS = 992, LAPS = 4, DEPTH = 3, TENSORS = 2, START = 3; };
-struct ClBackwardApply { static constexpr int CH = 8, THREADS = 608, LAPS = 4, DEPTH = 2, TENSORS = 2, START = 4; };
+// START: stages that take as long as the start and the end of a CTA.  NARROW: most threads where a row is 64 bytes at most.
+struct ClForwardSums { static constexpr int CH = 8, THREADS = 992, LAPS = 2, DEPTH = 5, TENSORS = 1, START = 8, NARROW = 480; };
+struct ClForwardApply { static constexpr int CH = 8, THREADS = 992, LAPS = 2, DEPTH = 3, TENSORS = 1, START = 4, NARROW = 480; };
+struct ClBackwardSums { static constexpr int CH = 4, THREADS = 992, LAPS = 4, DEPTH = 3, TENSORS = 2, START = 3, NARROW = 480; };
+struct ClBackwardApply { static constexpr int CH = 8, THREADS = 608, LAPS = 4, DEPTH = 2, TENSORS = 2, START = 4, NARROW = 608; };
 
 constexpr int CL_CHANNELS = 1024;     // most channels
 constexpr int CL_BARRIERS = 128;      // bytes in front of all else
@@ -67,12 +67,17 @@ int cl_ctas(long long stages, int B, int sms) {
 // Small fields spread over the SMs by smaller CTAs.  With more images than SMs CTAs have half the size, so that one begins while the other ends.  Both
 // passes with GELU, us, one CTA of full size per image or more while they fit at once / now: 90 x 180 x 384, 75 images 2058 / 1378;
 // 149 4301 / 2523; 32 x 64 x 64, 149 images 137 / 123, 300 205 / 185; 50 images of 90 x 180 x 384 1077 / 934.
+// Up to 32 channels over up to eight stages a CTA, smaller CTAs as well: one stage of a thousand rows keeps the CTA waiting for all of it, and its sums
+// are as many.  Forward with GELU, us, before the ring / full size / here: 8 channels, 12 images of 24840 12.3 / 13.6 / 11.1; 259200 tokens
+// 10.2 / 11.8 / 9.9; 16 channels, 2 of 76752 12.1 / 13.6 / 10.8; 32 channels, 4 of 16000 10.3 / 11.0 / 9.4; but 32 channels over 1038240 tokens
+// 36.7 at full size, 38.4 smaller.
 template <typename P>
 ClGeometry cl_geometry(int C, long long T, int B, int sms, bool merged, bool chained) {
   const int V = C / P::CH;
   const long long most = std::max(1, sms / B);
   const long long share = (T + P::LAPS * most - 1) / (P::LAPS * most);      // rows of threads that would give every CTA one stage
-  const int threads = B > sms ? (P::THREADS + 32) / 2 - 32 : P::THREADS;
+  const bool narrow = C <= 32 && T <= 8 * most * (P::THREADS / V * P::LAPS);
+  const int threads = B > sms ? (P::THREADS + 32) / 2 - 32 : narrow ? P::NARROW : P::THREADS;
   const int R = static_cast<int>(std::min<long long>(threads / V, std::max<long long>(share, (CL_FEWEST + V - 1) / V)));
   const long long stages = (T + P::LAPS * R - 1) / (P::LAPS * R);
   const int block = (V * R + 31) / 32 * 32 + 32, ctas = cl_ctas<P>(stages, B, sms), bytes = cl_ring_offset(C, merged) + cl_ring_bytes<P>(V * R);
