@@ -6,6 +6,7 @@
 #include "gemm_tcgen05.cuh"
 #include "launch.cuh"
 #include "norm_ring.h"
+#include "tcgen05.cuh"
 #include <cstring>
 #include <type_traits>
 
@@ -277,11 +278,6 @@ __device__ __forceinline__ unsigned int xch_ld_acquire(const unsigned int* ptr) 
   asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(ptr) : "memory");
   return v;
 }
-__device__ __forceinline__ unsigned long long xch_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
 // bounded wait (2 s) of one thread on the peers' flags; false + error word on expiry
 __device__ bool xch_wait(const StatExchange& xc, int code) {
   const unsigned int need = *xc.wait_exp + static_cast<unsigned int>(xc.wait_off);
@@ -290,7 +286,7 @@ __device__ bool xch_wait(const StatExchange& xc, int code) {
     for (unsigned int it = 0;; ++it) {
       if (static_cast<int>(xch_ld_acquire(xc.wait + peer) - need) >= 0) break;
       if ((it & 255u) == 255u) {
-        const unsigned long long now = xch_ns();
+        const unsigned long long now = global_ns();
         if (t0 == 0) t0 = now;
         else if (now - t0 > 2000000000ull) {
           atomicExch(xc.err, code);
@@ -317,28 +313,9 @@ __device__ void xch_signal(const StatExchange& xc) {
 // copied by every thread for itself (cp.async), 721 x 1440 tokens took 5 % longer than that, and with the stages of a CTA following one
 // another (here they are dealt out over the CTAs: all read one window of some MB that moves through the tensor) 8 %.
 __device__ __forceinline__ bool cl_wait(uint32_t bar, uint32_t parity, int* err) {
-  unsigned long long t0 = 0;
-  for (uint32_t it = 0;; ++it) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t"
-        ".reg .pred P1;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
-        "selp.b32 %0, 1, 0, P1;\n\t"
-        "}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (ok) return true;
-    if ((it & 63u) == 63u) {
-      const unsigned long long now = xch_ns();
-      if (t0 == 0) t0 = now;
-      else if (now - t0 > 2000000000ull) {
-        if (err) atomicExch(err, 58);
-        return false;
-      }
-    }
-  }
+  if (mbar_wait(bar, parity)) return true;
+  if (err) atomicExch(err, 58);
+  return false;
 }
 __device__ __forceinline__ void cl_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
@@ -347,10 +324,10 @@ __device__ __forceinline__ void cl_copy(uint32_t dst, const void* src, uint32_t 
 template <typename P>
 __device__ __forceinline__ void cl_init(uint4* smem) {      // (by all threads, once; a barrier of the CTA before cl_rows)
   if (threadIdx.x == 0) {
-    const uint32_t bars = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
+    const uint32_t bars = smem_u32(smem);
     for (int i = 0; i < P::DEPTH; ++i) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bars + 16 * i), "r"(1u));
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bars + 16 * i + 8), "r"(blockDim.x / 32 - 1));
+      mbar_init(bars + 16 * i, 1u);
+      mbar_init(bars + 16 * i + 8, blockDim.x / 32 - 1);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -360,7 +337,7 @@ __device__ __forceinline__ void cl_rows(uint4* smem, int offset, const __nv_bflo
                                         int* err, Use&& use) {
   using Word = ClWord<P::CH>;
   static_assert(P::DEPTH * 16 <= CL_BARRIERS, "two barriers a stage");
-  const uint32_t bars = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
+  const uint32_t bars = smem_u32(smem);
   const Word* const ring = reinterpret_cast<const Word*>(smem + offset / 16);
   const int rows = P::LAPS * R, half = rows * V;      // rows and words of one tensor in a stage
   const long long hop = static_cast<long long>(gridDim.x) * rows;
@@ -383,7 +360,7 @@ __device__ __forceinline__ void cl_rows(uint4* smem, int offset, const __nv_bflo
         if (!cl_wait(bars + 16 * s + 8, ph ^ 1u, err)) break;
         const uint32_t bytes = static_cast<uint32_t>(min(static_cast<long long>(rows), T - t)) * row;
         const uint32_t at = dst + s * P::TENSORS * rows * row;
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bars + 16 * s), "r"(P::TENSORS * bytes) : "memory");
+        mbar_expect_tx(bars + 16 * s, P::TENSORS * bytes);
         cl_copy(at, reinterpret_cast<const char*>(x) + t * row, bytes, bars + 16 * s);
         if (P::TENSORS == 2) cl_copy(at + rows * row, reinterpret_cast<const char*>(dy) + t * row, bytes, bars + 16 * s);
       }
@@ -403,7 +380,7 @@ __device__ __forceinline__ void cl_rows(uint4* smem, int offset, const __nv_bflo
       }
     }
     __syncwarp();
-    if ((threadIdx.x & 31) == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bars + 16 * s + 8) : "memory");
+    if ((threadIdx.x & 31) == 0) mbar_arrive(bars + 16 * s + 8);
   }
 }
 // bf16 channels of a thread as pairs of fp32

@@ -1287,7 +1287,8 @@ bool make_map(CUtensorMap* map, const GemmOperand& op, int K, int eb, int zlo_n,
   return true;
 }
 
-int max_pairs() {
+// CTA pairs that can be resident at once.  Every instance fills an SM with its shared memory, so one answers for all.
+static int max_pairs() {
   static const int n = [] {
     cudaLaunchConfig_t qc;
     memset(&qc, 0, sizeof(qc));
@@ -1331,7 +1332,9 @@ namespace {
 // neighbours.  It idles at the end, and on the way what two tiles share (the halves of 128-byte lines of a folded product's output, the rows of
 // activations of a plain one) is met so far apart in time that it leaves L2 in between.  A grid without a common factor mixes
 // them.  Synthesis of 1440 points, 64 orders, 136 channels 150 -> 88, 200 channels 187 -> 108; of 256 points, 129 orders, 384 channels
-// 35 -> 30 us.  Where a batch has many row tiles, all alike, the column tiles of one row take the place of a batch, and no wave may be added.
+// 35 -> 30 us.  Where a batch has many row tiles, all alike, the column tiles of one row take the place of a batch, and
+// at most one wave in sixteen may be added: what the rows cost twice is more than the waves (64 -> 264 channels over 720 x 1440 tokens, 110 waves of pairs
+// become 111, 259 -> 149 us; 128 -> 264 over 721 x 1440, 110 and 112, 187 -> 163; 384 -> 264 327 -> 291; 240 x 480 tokens, no wave more, 26.2 -> 26.1).
 long long mixed_grid(long long grid, const KParams& kp, int bm, int bn) {
   const bool columns = static_cast<long long>(kp.m_tiles) * kp.n_tiles > 256;
   if (columns && !kp.n_fast) return grid;
@@ -1426,8 +1429,11 @@ cudaError_t launch_t(const CUtensorMap& ma, const BMaps& mb, const CUtensorMap& 
 
 }  // namespace
 
-bool make_map_e(CUtensorMap* map, const void* ptr, int M, int N, int rd, long long rs_hi, long long rs_lo, long long zs_lo,
-                long long zs_hi, int zlo_n, int zhi_n, int box_rows, int ob, long long halves) {
+// Tensor map of an output or epilogue operand: [M rows][N contiguous] with two batch dimensions, 128-byte swizzle.  Rows
+// may be split, r = hi * rd + lo with rd a power of two that divides M and 32: a box is then 32 (or 128) / rd by rd rows.
+// With `halves` the second dimension is not part of the rows: two results `halves` elements apart (complex products).
+static bool make_map_e(CUtensorMap* map, const void* ptr, int M, int N, int rd, long long rs_hi, long long rs_lo, long long zs_lo,
+                       long long zs_hi, int zlo_n, int zhi_n, int box_rows = 128, int ob = 2, long long halves = 0) {
   EncodeTiledFn enc = get_encode();
   if (!enc) return false;
   const long long row_stride = rd > 1 ? rs_hi : rs_lo;

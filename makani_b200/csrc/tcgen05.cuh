@@ -11,13 +11,6 @@ namespace mk {
 // ---- host (gemm_tcgen05.cu)
 // tensor map of an operand: boxes of 128 bytes of the contiguous dimension by 64 (MN-major) or `box_rows_kmajor` rows
 bool make_map(CUtensorMap* map, const GemmOperand& op, int K, int eb, int zlo_n, int zhi_n, int box_rows_kmajor);
-// Tensor map of an output or epilogue operand: [M rows][N contiguous] with two batch dimensions, 128-byte swizzle.  Rows
-// may be split, r = hi * rd + lo with rd a power of two that divides M and 32: a box is then 32 (or 128) / rd by rd rows.
-// With `halves` the second dimension is not part of the rows: two results `halves` elements apart (complex products).
-bool make_map_e(CUtensorMap* map, const void* ptr, int M, int N, int rd, long long rs_hi, long long rs_lo, long long zs_lo,
-                long long zs_hi, int zlo_n, int zhi_n, int box_rows = 128, int ob = 2, long long halves = 0);
-// CTA pairs that can be resident at once.  Every kernel of them fills an SM with its shared memory, so one answers for all.
-int max_pairs();
 // cuTensorMapEncodeTiled is a driver call: binds the primary context to this host thread (not while `stream` is capturing)
 void bind_context(cudaStream_t stream);
 
