@@ -418,9 +418,9 @@ __global__ void __launch_bounds__(ClSums<MODE>::THREADS + 32, 1) inorm_cl_sums_k
   {
     // Pairs of channels in packed fp32 arithmetic: a packed instruction takes two cycles of a scheduler's fp32 pipe, three where it reads three
     // different register pairs, but one issue slot (GELU' with the polynomials by single instructions, whose coefficients need no
-    // registers: sums 330 us instead of 305).  721 x 1440 x 384 with GELU, rows in registers -> through the ring: forward 413 -> 393 us,
-    // backward 775 -> 657 (without GELU 413 -> 392, 650 -> 617); 240 x 480: 83 -> 64, 140 -> 101; 97 x 192: 48 -> 34, 67 -> 42.
-    // Both passes one after the other without a pause, under the power cap: 1222 -> 1107.
+    // registers: sums 330 us instead of 305).  With L2 flushed, us, rows in registers -> through the ring: 721 x 1440 x 384 with GELU forward
+    // 417 -> 388, backward 775 -> 656 (without GELU 421 -> 383, 660 -> 608); 240 x 480: 90 -> 66, 153 -> 108; 97 x 192: 48 -> 30, 70 -> 40.
+    // Both passes of the first looped without a pause, under the power cap: 1210 -> 1088.
     // Backward: pre = x ka + kb with ka = w rstd, kb = b - mean ka is the value the forward pass activated, and
     // sum g xhat = rstd sum g (x - mean).
     f32x2 nmean[PAIRS], ka[PAIRS], kb[PAIRS];

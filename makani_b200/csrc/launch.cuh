@@ -38,8 +38,8 @@ inline cudaError_t allow_shared_memory(std::atomic<uint64_t>& devices, const voi
 }
 
 #ifdef __CUDACC__
-// `next` false: the next kernel does not begin before this one is complete.  `p`: pointers whose loads the compiler may take for constant during the kernel (const __restrict__) and could move in front of the wait; they
-// come out of it as new values.
+// `next` false: the next kernel does not begin before this one is complete.  `p`: pointers whose loads the compiler may take for constant during the
+// kernel (const __restrict__) and could move in front of the wait; they come out of it as new values.
 template <typename... P>
 __device__ __forceinline__ void chain_begin(bool next, P&... p) {
   if (next) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

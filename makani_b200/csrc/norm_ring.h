@@ -12,10 +12,10 @@
 namespace mk {
 
 // The four kernels: channels of a thread, most threads that work on rows (whole rows of them are used, one more warp loads), rows per thread in
-// a stage of the ring and stages.  One CTA per SM.  721 x 1440 x 384, us, by (rows, stages): forward sums (1, 8) 147, (2, 5) 139; forward output
-// (1, 8) 274, (2, 5) 285, (2, 3) 260; gradient with GELU (1, 8) 428, (2, 4) 387, (4, 2) 370, by four channels and 992 threads (4, 3) 389.
-// The backward sums wait for the fp32 pipe and the issue slots, not for rows: without a test per row 330 instead of 352, and by four channels of
-// a thread as by eight, but 51 us instead of 61 at 240 x 480.
+// a stage of the ring and stages.  One CTA per SM.  721 x 1440 x 384 with GELU, each launch by itself with L2 flushed, us, by (rows, stages): forward
+// sums (1, 8) 147, (2, 5) 139; forward output (1, 8) 274, (2, 5) 285, (2, 3) 258; gradient (1, 8) 428, (2, 4) 387, (4, 2) 367, by four channels
+// and 992 threads (4, 3) 389.  The backward sums (303) wait for the fp32 pipe and the issue slots, not for rows: whole stages have no test per row,
+// and four channels of a thread are as fast as eight here, 51 us instead of 61 at 240 x 480.
 // START: stages that take as long as the start and the end of a CTA.  NARROW: most threads where a row is 64 bytes at most.
 struct ClForwardSums { static constexpr int CH = 8, THREADS = 992, LAPS = 2, DEPTH = 5, TENSORS = 1, START = 8, NARROW = 480; };
 struct ClForwardApply { static constexpr int CH = 8, THREADS = 992, LAPS = 2, DEPTH = 3, TENSORS = 1, START = 4, NARROW = 480; };
